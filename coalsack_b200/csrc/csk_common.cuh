@@ -1,5 +1,5 @@
-// Shared definitions of the MoE library: the repacked MXFP4 device layout, the
-// dequantisation helpers and the handle.  sm_100a only.
+// Shared definitions of the MoE library: code conversion, activations, barriers, launches and work lists.
+// sm_100a only.
 #pragma once
 
 #include <cuda_fp16.h>
@@ -15,57 +15,9 @@
 
 namespace csk {
 
-// ---------------------------------------------------------------------------
-// Device layout of one repacked MXFP4 matrix W[N, K] (K = contraction dim) for
-// the streaming kernel.
-//
-// The rows are cut into groups of 16; a group is stored as one contiguous run
-// of records along K: [group][k_tile][record], a record being 16 rows x 64
-// columns in 544 bytes:
-//
-//   bytes   0..511  codes, lane-major for a warp: lane l = 4*g + q owns 16 bytes
-//                   = four 32-bit words
-//                     word 0: row g,   columns 32*0 + 8q .. +7
-//                     word 1: row g,   columns 32*1 + 8q .. +7
-//                     word 2: row g+8, columns 32*0 + 8q .. +7
-//                     word 3: row g+8, columns 32*1 + 8q .. +7
-//                   nibble i of a word (bits 4i..4i+3) is the E2M1 code of
-//                   column 8q + i, i.e. the codes are in natural column order.
-//   bytes 512..543  E8M0 scales: for g = 0..7 four bytes
-//                     (row g blk 0, row g blk 1, row g+8 blk 0, row g+8 blk 1)
-//
-// One warp reads a record with a single 128-bit load per lane (plus one 32-bit
-// scale load).  For the fused gate/up matrix a group is 16 FEATURES and every
-// k-tile has two records, gate then up, so one warp sees both operands of the
-// gated activation.  Rows >= N and columns >= K are padded with zero codes.
-// ---------------------------------------------------------------------------
-constexpr int kSubBytes = 544;
-constexpr int kSubCodeBytes = 512;
-constexpr int kTileK = 64;
-
-struct MatLayout {
-  int N;        // logical rows (for gate/up: F features, stored as 2 x F rows)
-  int K;        // logical columns
-  int paired;   // 1 = fused gate/up
-  int groups;   // 16-row groups
-  int k_tiles;  // 64-column tiles along K
-  __host__ __device__ int recs() const { return paired ? 2 : 1; }
-  __host__ __device__ size_t group_bytes() const { return (size_t)k_tiles * recs() * kSubBytes; }
-  __host__ __device__ size_t bytes() const { return (size_t)groups * group_bytes(); }
-  __host__ __device__ int k_pad() const { return k_tiles * kTileK; }
-};
+constexpr int kTileK = 64;  // columns of K per step of the fp16 tensor-core kernels
 
 inline int ceil_div(int a, int b) { return (a + b - 1) / b; }
-
-inline MatLayout make_layout(int N, int K, bool paired) {
-  MatLayout L{};
-  L.N = N;
-  L.K = K;
-  L.paired = paired ? 1 : 0;
-  L.groups = ceil_div(N, 16);
-  L.k_tiles = ceil_div(K, kTileK);
-  return L;
-}
 
 // Two packed E2M1 codes (one byte) -> half2, low nibble in the low half.
 __device__ __forceinline__ uint32_t e2m1x2_to_h2(uint32_t byte) {
@@ -206,6 +158,11 @@ struct RowTile {
   int row0;    // first row of the tile in the grouped activation buffer
   int rows;    // rows in the tile (1 .. tile height)
   int pad;
+};
+
+// Where an expert's rows are among the row tiles: its first tile and the height of its tiles (the last may be shorter).
+struct ExpertTiles {
+  int tile0, height;
 };
 
 // Device-side status word values (or-ed).

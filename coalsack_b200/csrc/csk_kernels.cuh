@@ -1,92 +1,10 @@
-// The small kernels around the expert contractions: MXFP4 repack, router,
-// permutation by expert, gather to fp16 rows, weighted combine.
+// The small kernels around the expert contractions: router, permutation by
+// expert, gather to fp16 rows, weighted combine.
 #pragma once
 
 #include "csk_common.cuh"
 
 namespace csk {
-
-// ---------------------------------------------------------------------------
-// Repack: 17-byte MXFP4 blocks (row-major, [rows][K/32]) -> device tile layout.
-// src0 is the matrix itself, or the gate matrix of a fused gate/up pair whose
-// up matrix is src1.  One thread per destination word; the last 8 "words" of a
-// sub-tile record are its scale bytes.
-// ---------------------------------------------------------------------------
-__device__ __forceinline__ uint32_t raw_code(const uint8_t* src, int K, int row, int col) {
-  const uint8_t* blk = src + ((size_t)row * (K / 32) + col / 32) * 17;
-  const int j = col & 31;
-  const uint8_t byte = blk[1 + (j & 15)];
-  return j < 16 ? (byte & 0xF) : (byte >> 4);
-}
-
-__global__ void k_repack(const uint8_t* __restrict__ src0, const uint8_t* __restrict__ src1,
-                         uint8_t* __restrict__ dst, MatLayout L, int* __restrict__ emax_out) {
-  const size_t n_words = L.bytes() / 4;
-  for (size_t w = (size_t)blockIdx.x * blockDim.x + threadIdx.x; w < n_words;
-       w += (size_t)gridDim.x * blockDim.x) {
-    const size_t rec = w / (kSubBytes / 4);
-    const int wi = (int)(w % (kSubBytes / 4));
-    const int m = (int)(rec % L.recs());  // 0 = the matrix itself / gate, 1 = up
-    const int kt = (int)((rec / L.recs()) % L.k_tiles);
-    const int grp = (int)(rec / ((size_t)L.recs() * L.k_tiles));
-    const uint8_t* src = m ? src1 : src0;
-    uint32_t out = 0;
-    if (wi < kSubCodeBytes / 4) {
-      const int lane = wi >> 2, word = wi & 3;
-      const int g = lane >> 2, q = lane & 3;
-      const int row = grp * 16 + g + ((word & 2) ? 8 : 0);
-      const int col = kt * kTileK + (word & 1) * 32 + q * 8;
-      if (row < L.N && col < L.K) {
-#pragma unroll
-        for (int i = 0; i < 8; ++i) out |= raw_code(src, L.K, row, col + i) << (4 * i);
-      }
-    } else {
-      const int g = wi - kSubCodeBytes / 4;
-      int emax = -1;
-#pragma unroll
-      for (int slot = 0; slot < 4; ++slot) {
-        const int row = grp * 16 + g + ((slot & 2) ? 8 : 0);
-        const int col = kt * kTileK + (slot & 1) * 32;
-        uint32_t e = 0;  // padding: zero codes under the smallest scale
-        if (row < L.N && col < L.K) {
-          const uint8_t* blk = src + ((size_t)row * (L.K / 32) + col / 32) * 17;
-          e = min((uint32_t)blk[0], 254u);  // scale byte 255 is read as 254: stored that way, so the kernel need not clamp
-          // a block of zero codes is zero under any scale: it does not widen the matrix's exponent range
-          bool any = false;
-          for (int j = 1; j < 17; ++j) any = any || blk[j] != 0;
-          if (any) emax = max(emax, (int)e);
-        }
-        out |= e << (8 * slot);
-      }
-      if (emax >= 0) atomicMax(emax_out, emax);  // largest scale exponent among the matrix's non-zero blocks
-    }
-    reinterpret_cast<uint32_t*>(dst)[w] = out;
-  }
-}
-
-// Inverse of k_repack for one source matrix (which_half: 0 = the matrix itself
-// or the gate half, 1 = the up half).  One thread per 17-byte block.
-__global__ void k_unpack(const uint8_t* __restrict__ packed, uint8_t* __restrict__ out, MatLayout L,
-                         int which_half) {
-  const int kb = L.K / 32;
-  const size_t n_blocks = (size_t)L.N * kb;
-  for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n_blocks;
-       i += (size_t)gridDim.x * blockDim.x) {
-    const int row = (int)(i / kb), blk = (int)(i % kb);
-    const int grp = row / 16, r16 = row % 16;
-    const int g = r16 & 7, hi = r16 >> 3;
-    const int kt = blk / 2, b = blk & 1;
-    const uint8_t* rec = packed + (((size_t)grp * L.k_tiles + kt) * L.recs() + which_half) * kSubBytes;
-    uint8_t* o = out + i * 17;
-    o[0] = rec[kSubCodeBytes + g * 4 + hi * 2 + b];
-    uint32_t codes[32];
-    for (int q = 0; q < 4; ++q) {
-      const uint32_t w = reinterpret_cast<const uint32_t*>(rec)[(g * 4 + q) * 4 + hi * 2 + b];
-      for (int t = 0; t < 8; ++t) codes[q * 8 + t] = (w >> (4 * t)) & 0xF;
-    }
-    for (int j = 0; j < 16; ++j) o[1 + j] = (uint8_t)(codes[j] | (codes[j + 16] << 4));
-  }
-}
 
 // ---------------------------------------------------------------------------
 // Router (moe_router_node::compute_impl, moe_router_node.h:140-214).
@@ -835,7 +753,7 @@ k_router_topk(const float* __restrict__ logits, float* __restrict__ router_out, 
 // what lets every expert's weights be read once.
 //
 // meta layout (int32): [0] row tiles, [1] total rows, [2] distinct experts,
-//                      [3] device status word (or-ed kDevErr*), [4..7] spare.
+//                      [3] device status word (or-ed kDevErr*), [4] rows of the tallest row tile, [5..7] spare.
 // ---------------------------------------------------------------------------
 __global__ void k_hist(const float* __restrict__ router_out, int n_pairs, int E, int only_expert,
                        int* __restrict__ counts, int* __restrict__ meta) {
@@ -866,22 +784,21 @@ __global__ void k_hist(const float* __restrict__ router_out, int n_pairs, int E,
 // itself -- counts and the status word then need no clearing beforehand and the
 // whole plan is one launch.
 //
-// With row_of_pair / pair_of_row given as well (the streaming kernel then gathers its token
-// rows itself) the block also places every pair: row_of_pair[i] = its row in the grouped
-// order (-1: not placed), pair_of_row[row] = i.  Which row of its expert's segment a pair
-// gets depends on the order of the block's atomics; a row's value does not depend on it.
+// With row_of_pair given as well the block also places every pair: row_of_pair[i] = its row in
+// the grouped order (-1: not placed).  Which row of its expert's segment a pair gets depends on
+// the order of the block's atomics; a row's value does not depend on it.
 __global__ void __launch_bounds__(1024)
 k_scan(int* __restrict__ counts, int E, int e_begin, int e_count, int tile_rows, int max_rows,
        int max_tiles, const uint8_t* __restrict__ resident, int* __restrict__ offsets,
        int* __restrict__ cursor, RowTile* __restrict__ tiles, int* __restrict__ meta,
        const float* __restrict__ router_out, int n_pairs, int only_expert,
-       int* __restrict__ row_of_pair = nullptr, int* __restrict__ pair_of_row = nullptr) {
+       int* __restrict__ row_of_pair = nullptr, ExpertTiles* __restrict__ expert_tiles = nullptr) {
   __shared__ int s_row_off[1025];
   __shared__ int s_tile_off[1025];
   __shared__ int s_warp[2][32];
-  __shared__ int s_distinct;
+  __shared__ int s_distinct, s_tallest;
   const int e = threadIdx.x, lane = e & 31, warp = e >> 5;
-  if (e == 0) s_distinct = 0;
+  if (e == 0) s_distinct = s_tallest = 0;
   griddep_wait();
   griddep_launch();
   if (router_out) {
@@ -903,6 +820,17 @@ k_scan(int* __restrict__ counts, int E, int e_begin, int e_count, int tile_rows,
   __syncthreads();  // every thread holds its count before s_tile_off is reused
   const bool local = e >= e_begin && e < e_begin + e_count;
   const int nt = local ? (c + tile_rows - 1) / tile_rows : 0;
+  // An expert with several tiles gets them equally tall instead of full ones and a short rest: for the block-scaled
+  // kernel always (its time goes by the tile's rows), for the fp16 tensor-core kernel (rounded up to the MMA's 16-row
+  // step) with two to four tiles -- a tile's cost is nearly flat below ~175 rows, so 128 + 128 rows are cheaper than
+  // 192 + 64, and with more tiles only the last one would change.
+  auto tile_height = [&](int cnt) {
+    const int ntl = (cnt + tile_rows - 1) / tile_rows;
+    if (ntl < 2) return tile_rows;
+    const int even = (cnt + ntl - 1) / ntl;
+    if (expert_tiles) return even;
+    return tile_rows >= 64 && ntl <= 4 ? min(tile_rows, (even + 15) & ~15) : tile_rows;
+  };
   if (c > 0) {
     atomicAdd(&s_distinct, 1);
     if (local && resident && !resident[e - e_begin]) atomicOr(&meta[3], kDevErrNotResident);
@@ -941,6 +869,7 @@ k_scan(int* __restrict__ counts, int E, int e_begin, int e_count, int tile_rows,
   if (e < E) {
     offsets[e] = row_off;
     cursor[e] = 0;
+    if (expert_tiles) expert_tiles[e] = ExpertTiles{tile_off, tile_height(c)};
   }
   const int total_rows = s_warp[0][31], total_tiles = s_warp[1][31];
   if (e == 0) {
@@ -968,10 +897,12 @@ k_scan(int* __restrict__ counts, int E, int e_begin, int e_count, int tile_rows,
         if (pos >= max_rows) pos = -1;
       }
       row_of_pair[i] = pos;
-      if (pos >= 0) pair_of_row[pos] = i;
     }
   }
-  if (total_rows > max_rows || total_tiles > max_tiles) return;
+  if (total_rows > max_rows || total_tiles > max_tiles) {
+    if (e == 0) meta[4] = 0;
+    return;
+  }
   for (int i = threadIdx.x; i < total_tiles; i += blockDim.x) {
     // largest expert x with s_tile_off[x] <= i (experts without tiles repeat an offset)
     int lo = 0, hi = 1023;
@@ -982,12 +913,7 @@ k_scan(int* __restrict__ counts, int E, int e_begin, int e_count, int tile_rows,
     // step back over empty experts that share the offset: the owner is the last
     // expert with that offset that actually has tiles, i.e. the largest index.
     const int cnt = (lo < 1023 ? s_row_off[lo + 1] : s_row_off[1024]) - s_row_off[lo];
-    // An expert with two to four tensor-core tiles gets them equally tall (rounded up to the MMA's 16-row
-    // step) instead of full tiles and a short rest: a tile's cost is nearly flat below ~175 rows, so
-    // 128 + 128 rows are cheaper than 192 + 64.  (More tiles: only the last one would change.)
-    const int ntl = (cnt + tile_rows - 1) / tile_rows;
-    int per = tile_rows;
-    if (tile_rows >= 64 && ntl >= 2 && ntl <= 4) per = min(tile_rows, (((cnt + ntl - 1) / ntl) + 15) & ~15);
+    const int per = tile_height(cnt);
     const int r = (i - s_tile_off[lo]) * per;
     RowTile t;
     t.expert = lo - e_begin;
@@ -995,7 +921,10 @@ k_scan(int* __restrict__ counts, int E, int e_begin, int e_count, int tile_rows,
     t.rows = min(per, cnt - r);
     t.pad = 0;
     tiles[i] = t;
+    atomicMax(&s_tallest, t.rows);
   }
+  __syncthreads();
+  if (e == 0) meta[4] = s_tallest;
 }
 
 // One warp per (token, slot) pair: claim a row in the expert's segment, record

@@ -11,7 +11,7 @@
 #include "csk_common.cuh"
 #include "csk_kernels.cuh"
 #include "csk_kquant.cuh"
-#include "csk_stream.cuh"
+#include "csk_mx.cuh"
 #include "csk_tile.cuh"
 #include "csk_tile2.cuh"
 
@@ -25,7 +25,7 @@ std::string g_create_error;
 struct csk_moe_layer {
   csk_moe_config cfg{};
   int E = 0, k = 0, H = 0, F = 0, e0 = 0, Eloc = 0;
-  MatLayout Lgu{}, Ld{};    // streaming kernel's layout
+  MxLayout Lgu{}, Ld{};     // block-scaled kernel's layout
   TileLayout Tgu{}, Td{};   // tensor-core kernel's layout (a second copy of the codes)
   size_t off_gu = 0, off_d = 0, off_tgu = 0, off_td = 0, off_bias = 0, off_meta = 0, expert_stride = 0;
   uint8_t* d_weights = nullptr;
@@ -89,9 +89,10 @@ struct csk_moe_layer {
   int* d_offsets = nullptr;      // [E+1]
   int* d_cursor = nullptr;       // [E]
   int* d_row_of_pair = nullptr;  // [max_rows]
-  int* d_pair_of_row = nullptr;  // [max_rows] inverse map (small batches on the streaming kernel)
-  const float* gather_hidden = nullptr;  // transient: the streaming kernel's gate/up launch gathers rows from here
-  const float* gather_router = nullptr;
+  ExpertTiles* d_expert_tiles = nullptr;  // [E] where the experts' row tiles are (block-scaled kernel)
+  uint8_t* d_ximg = nullptr;     // the block-scaled kernel's operands: token rows and activated rows as digit images
+  uint8_t* d_aimg = nullptr;
+  int64_t mx_rows = 0;           // rows the images hold
   int* d_out_row_map = nullptr;  // [max_rows] (expert-parallel receive side)
   int* d_seg = nullptr;          // [2*1024+2] segment plan (expert-parallel receive side)
   RowTile* d_tiles = nullptr;
@@ -264,30 +265,22 @@ int launch_router(csk_moe_layer* L, const float* d_hidden, int64_t T, float* d_r
   return CSK_OK;
 }
 
-// histogram -> scan (+ row tiles of `tile_rows`) -> scatter rows as fp16 into x16
+// histogram -> scan (+ row tiles of `tile_rows`) -> token rows: as fp16 rows into x16, or (x16 null) as digits into
+// the block-scaled kernel's image
 constexpr int kOneBlockPairs = 8192;  // up to here histogram, scan and tile list are one single-block launch
 
-// place_only: no fp16 row buffer is written; the block that scans also places every pair
-// (row_of_pair, pair_of_row) and the streaming kernel gathers its token rows itself.
-int launch_permute(csk_moe_layer* L, const float* d_hidden, const float* d_router, int64_t T,
-                   int only_expert, int tile_rows, int e_begin, int e_count, __half* x16, int ldx,
-                   int64_t max_rows, cudaStream_t s, bool place_only = false) {
+int launch_permute(csk_moe_layer* L, const float* d_hidden, const float* d_router, int64_t T, int only_expert,
+                   int tile_rows, int e_begin, int e_count, __half* x16, int ldx, int64_t max_rows, cudaStream_t s) {
   const int n_pairs = (int)(T * L->k);
   const uint8_t* res = e_count ? L->d_resident : nullptr;
-  if (place_only) {
-    if (n_pairs > kOneBlockPairs) return fail(L, CSK_ERR_INVALID, "internal: too many pairs for the one-block plan");
+  const bool digits = x16 == nullptr;
+  const bool one_block = n_pairs <= kOneBlockPairs;
+  ExpertTiles* et = digits ? L->d_expert_tiles : nullptr;
+  if (one_block) {
+    // small batch: histogram, scan, tile list (and, for digits, the rows' places) in one single-block launch
     launch_k(k_scan, dim3(1), dim3(1024), 0, s, L->pdl, L->d_counts, L->E, e_begin, e_count, tile_rows, (int)max_rows,
              L->max_tiles, res, L->d_offsets, L->d_cursor, L->d_tiles, L->d_meta, d_router, n_pairs, only_expert,
-             L->d_row_of_pair, L->d_pair_of_row);
-    CSK_CUDA(L, cudaGetLastError());
-    L->last.launches += 1;
-    return CSK_OK;
-  }
-  if (n_pairs <= kOneBlockPairs) {
-    // small batch: histogram, scan and tile list in one single-block launch
-    launch_k(k_scan, dim3(1), dim3(1024), 0, s, L->pdl, L->d_counts, L->E, e_begin, e_count, tile_rows, (int)max_rows,
-             L->max_tiles, res, L->d_offsets, L->d_cursor, L->d_tiles, L->d_meta, d_router, n_pairs, only_expert,
-             (int*)nullptr, (int*)nullptr);
+             digits ? L->d_row_of_pair : (int*)nullptr, et);
     L->last.launches += 1;
   } else {
     CSK_CUDA(L, cudaMemsetAsync(L->d_counts, 0, sizeof(int) * L->E, s));
@@ -295,25 +288,75 @@ int launch_permute(csk_moe_layer* L, const float* d_hidden, const float* d_route
     k_hist<<<grid_for(n_pairs, 256, 2 * L->sm_count), 256, sizeof(int) * L->E, s>>>(
         d_router, n_pairs, L->E, only_expert, L->d_counts, L->d_meta);
     k_scan<<<1, 1024, 0, s>>>(L->d_counts, L->E, e_begin, e_count, tile_rows, (int)max_rows, L->max_tiles, res,
-                              L->d_offsets, L->d_cursor, L->d_tiles, L->d_meta, nullptr, 0, -1, nullptr, nullptr);
+                              L->d_offsets, L->d_cursor, L->d_tiles, L->d_meta, nullptr, 0, -1, nullptr, et);
     L->last.launches += 2;
   }
-  launch_k(k_scatter, dim3(grid_for(n_pairs, 8, 8 * L->sm_count)), dim3(256), 0, s, L->pdl, d_router, d_hidden,
-           n_pairs, L->k, L->H, L->E, only_expert, L->d_offsets, L->d_cursor, L->d_row_of_pair, x16, ldx, (int)max_rows,
-           L->cfg.weight_before_ffn);
+  if (digits) {
+    MxQuantArgs a{};
+    a.hidden = d_hidden;
+    a.router = d_router;
+    a.offsets = L->d_offsets;
+    a.et = L->d_expert_tiles;
+    a.cursor = one_block ? nullptr : L->d_cursor;
+    a.row_of_pair = L->d_row_of_pair;
+    a.tiles = L->d_tiles;
+    a.n_tiles_ptr = L->d_meta;
+    a.image = L->d_ximg;
+    a.T = (int)T;
+    a.H = L->H;
+    a.E = L->E;
+    a.k = L->k;
+    a.e_begin = e_begin;
+    a.e_count = e_count;
+    a.only_expert = only_expert;
+    a.max_rows = (int)max_rows;
+    a.weight_before_ffn = L->cfg.weight_before_ffn;
+    a.blocks = L->Lgu.blocks;
+    a.recs = L->Lgu.recs;
+    launch_k(k_mx_quant, dim3((unsigned)T), dim3(std::min(128, ceil_div(L->Lgu.blocks, 32) * 32)), 0, s, L->pdl, a);
+  } else {
+    launch_k(k_scatter, dim3(grid_for(n_pairs, 8, 8 * L->sm_count)), dim3(256), 0, s, L->pdl, d_router, d_hidden,
+             n_pairs, L->k, L->H, L->E, only_expert, L->d_offsets, L->d_cursor, L->d_row_of_pair, x16, ldx, (int)max_rows,
+             L->cfg.weight_before_ffn);
+  }
   CSK_CUDA(L, cudaGetLastError());
   L->last.launches += 1;
   return CSK_OK;
 }
 
-// Warps per CTA and ring stages of the streaming kernel (measured on B200): ten warps with
-// three-stage rings when every warp walks a whole contraction, eight warps with three stages
-// when the contraction is split over the warps.
-constexpr int kStreamWarps = 10, kStreamStages = 3, kStreamSplitStages = 3;
-template <int NT8, int KSPLIT, int W, int NSTG>
-void launch_stream_pair(csk_moe_layer* L, const __half* x16, float* y, int ldy, int x_rows, cudaStream_t s,
-                        StageTimer& tm) {
-  StreamArgs a{};
+// Images for `rows` grouped rows (row tiles of full height plus one shorter one per expert).
+int mx_reserve(csk_moe_layer* L, int64_t rows) {
+  if (L->w16 || rows <= L->mx_rows) return CSK_OK;
+  const size_t tiles = (size_t)rows / kMxTileRows + L->Eloc + 1;
+  const size_t xb = mx_image_bytes(rows, tiles, L->Lgu.recs), ab = mx_image_bytes(rows, tiles, L->Ld.recs);
+  uint8_t *x = nullptr, *a = nullptr;
+  cudaError_t e = cudaMalloc(&x, xb);
+  if (e == cudaSuccess) e = cudaMalloc(&a, ab);
+  if (e == cudaSuccess) e = cudaMemset(x, 0, xb);
+  if (e == cudaSuccess) e = cudaMemset(a, 0, ab);
+  if (e == cudaSuccess) e = cudaDeviceSynchronize();  // also: nothing reads the old images any more
+  if (e != cudaSuccess) {
+    cudaFree(x);
+    cudaFree(a);
+    cudaGetLastError();
+    return fail(L, e == cudaErrorMemoryAllocation ? CSK_ERR_NOMEM : CSK_ERR_CUDA, "row images: %s", cudaGetErrorString(e));
+  }
+  cudaFree(L->d_ximg);
+  cudaFree(L->d_aimg);
+  L->d_ximg = x;
+  L->d_aimg = a;
+  L->mx_rows = rows;
+  return CSK_OK;
+}
+
+// The grouped fp16 rows of the expert-parallel receive side as digits.
+void mx_quant_rows(csk_moe_layer* L, cudaStream_t s) {
+  k_mx_quant_rows<<<4 * L->sm_count, 128, 0, s>>>(L->d_x16, L->ldx, L->d_tiles, L->d_meta, L->d_ximg, L->H, L->Lgu.blocks,
+                                                  L->Lgu.recs);
+}
+
+void launch_mx_pair(csk_moe_layer* L, float* y, int ldy, cudaStream_t s, StageTimer& tm) {
+  MxArgs a{};
   a.weights = L->d_weights;
   a.expert_stride = L->expert_stride;
   a.bias_offset = L->off_bias;
@@ -323,88 +366,48 @@ void launch_stream_pair(csk_moe_layer* L, const __half* x16, float* y, int ldy, 
   a.act = L->cfg.activation;
   a.F = L->F;
   a.meta = L->d_meta;
-  a.x_rows = x_rows;
-  a.gather_hidden = L->gather_hidden;  // set by the caller for this launch only (null: rows come from x16)
-  a.pair_of_row = L->d_pair_of_row;
-  a.router = L->gather_router;
-  a.top_k = L->k;
-  a.H = L->H;
-  a.weight_before_ffn = L->cfg.weight_before_ffn;
-  // every CTA takes one contiguous range of work units; as many CTAs as fit at once
-  const size_t per_sm_limit = W > 8 ? 2 : 3;
-  auto grid_for_smem = [&](size_t smem) {
-    return L->sm_count * (int)std::max<size_t>(1, std::min<size_t>(per_sm_limit, (227 * 1024) / (smem + 1024)));
-  };
   // gate/up + activation
   a.mat_offset = L->off_gu;
   a.L = L->Lgu;
-  a.x = x16;
-  a.ldx = L->ldx;
-  a.a_out = L->d_a16;
-  a.lda = L->lda;
-  size_t smem = stream_smem_bytes(x_rows, NT8, L->Lgu.k_pad(), KSPLIT, true, W, NSTG);
-  launch_k(k_stream<NT8, true, KSPLIT, W, NSTG>, dim3(grid_for_smem(smem)), dim3(W * 32), smem, s, L->pdl, a);
+  a.x_img = L->d_ximg;
+  a.a_img = L->d_aimg;
+  a.a_blocks = L->Ld.blocks;
+  a.a_recs = L->Ld.recs;
+  launch_k(k_mx<true>, dim3(L->sm_count), dim3(kMxThreads), kMxSmem, s, L->pdl, a);
   tm.mark();
   // down
-  a.gather_hidden = nullptr;
   a.mat_offset = L->off_d;
   a.L = L->Ld;
-  a.x = L->d_a16;
-  a.ldx = L->lda;
-  a.y_out = y;
+  a.x_img = L->d_aimg;
+  a.y = y;
   a.ldy = ldy;
-  smem = stream_smem_bytes(x_rows, NT8, L->Ld.k_pad(), KSPLIT, false, W, NSTG);
-  launch_k(k_stream<NT8, false, KSPLIT, W, NSTG>, dim3(grid_for_smem(smem)), dim3(W * 32), smem, s, L->pdl, a);
+  launch_k(k_mx<false>, dim3(L->sm_count), dim3(kMxThreads), kMxSmem, s, L->pdl, a);
   tm.mark();
   L->last.launches += 2;
 }
 
-template <int NT8, int KSPLIT, int W, int NSTG>
-cudaError_t stream_prepare_one() {
-  cudaError_t e = cudaFuncSetAttribute(k_stream<NT8, true, KSPLIT, W, NSTG>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-  if (e == cudaSuccess)
-    e = cudaFuncSetAttribute(k_stream<NT8, false, KSPLIT, W, NSTG>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-  return e;
-}
-cudaError_t stream_prepare_device() {
-  cudaError_t e = stream_prepare_one<1, 1, kStreamWarps, kStreamStages>();
-  if (e == cudaSuccess) e = stream_prepare_one<1, 8, 8, kStreamSplitStages>();
-  if (e == cudaSuccess) e = stream_prepare_one<2, 1, 8, 3>();
-  return e;
-}
-
-int stream_tile_rows(const csk_moe_layer* L, int64_t rows) {
-  // 8-row tiles up to an average of twelve rows per expert: the 16-row variant of the streaming kernel is
-  // 1.8x slower per weight byte (558 vs 314 us per step at 64 tokens on the 128-expert layer), so it pays
-  // only when nearly every expert would otherwise stream its weights twice.  (Under CSK_PATH_AUTO the
-  // tensor-core kernel has taken over before that point.)
-  return rows <= 12 * (int64_t)std::max(1, L->Eloc) ? 8 : 16;
-}
+// Rows per resident expert from which the fp16 tensor-core kernel takes over.
+constexpr int64_t kMxRowsPerExpert = 48;
 
 int choose_path(const csk_moe_layer* L, int64_t rows) {
   if (L->w16) return CSK_PATH_TILE;  // fp16 weights exist in the tensor-core layout only
   if (L->path == CSK_PATH_STREAM) return CSK_PATH_STREAM;
   if (L->path == CSK_PATH_TILE || L->path == CSK_PATH_TILE_PAIR) return CSK_PATH_TILE;
-  // The tensor-core kernel's time is nearly flat in the rows per expert (600 us per step at 256 tokens,
-  // 700 at 1024 on the 128-expert layer), the streaming kernel's grows with the number of 8-row tiles
-  // (494 us at 256 tokens, 816 at 512): they cross at about ten rows per expert.
-  return (L->tile.available && rows >= 10 * (int64_t)std::max(1, L->Eloc)) ? CSK_PATH_TILE : CSK_PATH_STREAM;
+  return (L->tile.available && rows >= kMxRowsPerExpert * (int64_t)std::max(1, L->Eloc)) ? CSK_PATH_TILE : CSK_PATH_STREAM;
 }
 
 // the CTA-pair kernel runs only when asked for by name (and clusters of two can be launched)
 bool use_pairs(const csk_moe_layer* L) { return L->pair.available && L->path == CSK_PATH_TILE_PAIR; }
 
-int tile_rows_for(const csk_moe_layer* L, int path, int64_t rows) {
-  return path == CSK_PATH_TILE ? (use_pairs(L) ? kPairN : kTileM) : stream_tile_rows(L, rows);
+int tile_rows_for(const csk_moe_layer* L, int path) {
+  return path == CSK_PATH_TILE ? (use_pairs(L) ? kPairN : kTileM) : kMxTileRows;
 }
 
-// grouped gate/up + activation + down over the row tiles listed in d_tiles;
-// x16 holds the grouped rows; output rows go to y (through out_row_map if set)
-int launch_experts(csk_moe_layer* L, int path, int tile_rows, int64_t n_rows_hint, int64_t rows_per_expert_max,
-                   const __half* x16, float* y, int ldy, const int* out_row_map, cudaStream_t s, StageTimer& tm,
+// grouped gate/up + activation + down over the row tiles listed in d_tiles; the grouped rows are in d_x16 (tensor-core
+// path) or in d_ximg (streaming path); output rows go to y (through out_row_map or out_row_ptr if set)
+int launch_experts(csk_moe_layer* L, int path, float* y, int ldy, const int* out_row_map, cudaStream_t s, StageTimer& tm,
                    float* const* out_row_ptr = nullptr) {
   if (path == CSK_PATH_TILE) {
-    if (x16 != L->d_x16) return fail(L, CSK_ERR_INVALID, "the tile path reads the handle's own row buffer");
     int rc;
     if (use_pairs(L))
       rc = pair_launch(L->pair, L->tile, L->tile.tmap_xh, L->tile.tmap_ah, L->d_weights, L->expert_stride, L->off_tgu,
@@ -421,24 +424,7 @@ int launch_experts(csk_moe_layer* L, int path, int tile_rows, int64_t n_rows_hin
     L->last.launches += 2;
   } else {
     if (out_row_map || out_row_ptr) return fail(L, CSK_ERR_INVALID, "row maps need the tile path");
-    // no tile holds more rows than its expert received
-    const int x_rows = (int)std::max<int64_t>(1, std::min<int64_t>(tile_rows, rows_per_expert_max));
-    const int kp = std::max(L->Lgu.k_pad(), L->Ld.k_pad());
-    const size_t need = tile_rows == 8 ? std::max(stream_smem_bytes(x_rows, 1, kp, 8, true, 8, kStreamSplitStages),
-                                                  stream_smem_bytes(x_rows, 1, kp, 1, true, kStreamWarps, kStreamStages))
-                                       : stream_smem_bytes(x_rows, 2, kp, 1, true, 8, 3);
-    if (need > 200 * 1024)
-      return fail(L, CSK_ERR_NOMEM, "hidden/ffn dimension too large for the streaming kernel's row buffer");
-    if (tile_rows == 8) {
-      constexpr int64_t kSplitRows = 8;
-      if (n_rows_hint <= kSplitRows) {  // measured: the split pays only while the whole batch is a handful of rows
-        launch_stream_pair<1, 8, 8, kStreamSplitStages>(L, x16, y, ldy, x_rows, s, tm);  // a handful of rows: split the contraction over the warps
-      } else {
-        launch_stream_pair<1, 1, kStreamWarps, kStreamStages>(L, x16, y, ldy, x_rows, s, tm);
-      }
-    } else {
-      launch_stream_pair<2, 1, 8, 3>(L, x16, y, ldy, x_rows, s, tm);
-    }
+    launch_mx_pair(L, y, ldy, s, tm);
   }
   CSK_CUDA(L, cudaGetLastError());
   L->last.path = path;
@@ -517,21 +503,14 @@ int forward_dev(csk_moe_layer* L, const float* d_hidden, int64_t T, const float*
   }
   const int64_t rows = only_expert >= 0 ? T : T * L->k;
   const int path = choose_path(L, only_expert >= 0 ? rows * std::max(1, L->Eloc) : rows);
-  const int tile_rows = tile_rows_for(L, path, only_expert >= 0 ? rows * std::max(1, L->Eloc) : rows);
+  const int tile_rows = tile_rows_for(L, path);
   if (reinterpret_cast<uintptr_t>(d_hidden) % 16) return fail(L, CSK_ERR_INVALID, "hidden states must be 16-byte aligned");
-  // small batches on the streaming kernel: no fp16 row buffer in between, the kernel gathers its rows
-  // (up to 64 pairs: measured, the launch it saves is worth 2-3 us of a 50-190 us step there; with more rows per
-  // tile every work unit's copy of the gather costs more than the launch -- 7 % of the step at 32 tokens on 32 experts)
-  constexpr int64_t kGatherMaxPairs = 64;
-  const bool gather = path == CSK_PATH_STREAM && T * L->k <= kGatherMaxPairs;
-  int rc = launch_permute(L, d_hidden, router, T, only_expert, tile_rows, L->e0, L->Eloc, L->d_x16,
-                          L->ldx, L->max_rows, s, gather);
+  const bool mx = path == CSK_PATH_STREAM;
+  int rc = launch_permute(L, d_hidden, router, T, only_expert, tile_rows, L->e0, L->Eloc, mx ? nullptr : L->d_x16, L->ldx,
+                          mx ? L->mx_rows : L->max_rows, s);
   if (rc) return rc;
   tm.mark();
-  L->gather_hidden = gather ? d_hidden : nullptr;
-  L->gather_router = router;
-  rc = launch_experts(L, path, tile_rows, rows, T, L->d_x16, L->d_y, L->H, nullptr, s, tm);
-  L->gather_hidden = nullptr;
+  rc = launch_experts(L, path, L->d_y, L->H, nullptr, s, tm);
   if (rc) return rc;
   // the shared expert's rows come from another stream: the combine is the first kernel that reads them
   if (shared_ready) CSK_CUDA(L, cudaStreamWaitEvent(s, shared_ready, 0));
@@ -623,8 +602,8 @@ int csk_moe_create(const csk_moe_config* cfg, csk_moe_layer** out) {
   L->e0 = e0;
   L->Eloc = eloc;
   L->w16 = cfg->weight_format == CSK_WEIGHTS_F16;
-  L->Lgu = make_layout(L->F, L->H, true);
-  L->Ld = make_layout(L->H, L->F, false);
+  L->Lgu = make_mx_layout(L->F, L->H, true);
+  L->Ld = make_mx_layout(L->H, L->F, false);
   L->Tgu = make_tile_layout(L->F, L->H, true, L->w16);
   L->Td = make_tile_layout(L->H, L->F, false, L->w16);
   auto up256 = [](size_t v) { return (v + 255) / 256 * 256; };
@@ -638,8 +617,8 @@ int csk_moe_create(const csk_moe_config* cfg, csk_moe_layer** out) {
   L->resident.assign(eloc, 0);
   L->max_T = cfg->max_tokens;
   L->max_rows = cfg->max_tokens * cfg->top_k;
-  L->ldx = L->Lgu.k_pad();
-  L->lda = L->Ld.k_pad();
+  L->ldx = L->Tgu.k_pad();
+  L->lda = L->Td.k_pad();
   L->max_tiles = (int)(L->max_rows / 8 + eloc + 8);
 
 #define CK(call)                                                                              \
@@ -714,8 +693,12 @@ int csk_moe_create(const csk_moe_config* cfg, csk_moe_layer** out) {
   CK(cudaMalloc(&L->d_offsets, sizeof(int) * (L->E + 1)));
   CK(cudaMalloc(&L->d_cursor, sizeof(int) * L->E));
   CK(cudaMalloc(&L->d_row_of_pair, sizeof(int) * L->max_rows));
-  CK(cudaMalloc(&L->d_pair_of_row, sizeof(int) * L->max_rows));
-  CK(cudaMemset(L->d_pair_of_row, 0, sizeof(int) * L->max_rows));
+  CK(cudaMalloc(&L->d_expert_tiles, sizeof(ExpertTiles) * L->E));
+  if (mx_reserve(L, std::min(L->max_rows, kMxRowsPerExpert * eloc))) {
+    fail(nullptr, CSK_ERR_NOMEM, "%s", L->err.c_str());
+    csk_moe_destroy(L);
+    return CSK_ERR_NOMEM;
+  }
   CK(cudaMalloc(&L->d_out_row_map, sizeof(int) * L->max_rows));
   CK(cudaMalloc(&L->d_seg, sizeof(int) * (3 * 1024 + 8)));
   CK(cudaMalloc(&L->d_tiles, sizeof(RowTile) * L->max_tiles));
@@ -724,7 +707,7 @@ int csk_moe_create(const csk_moe_config* cfg, csk_moe_layer** out) {
   CK(cudaMallocHost(&L->h_meta, sizeof(int) * 16));
   CK(cudaMallocHost(&L->h_counts64, sizeof(int64_t) * L->E));
   CK(router_prepare_device());
-  CK(stream_prepare_device());
+  CK(mx_prepare_device());
   {
     int rc = tile_init(L->tile, cfg->device);
     if (!rc) rc = tile_set_buffers(L->tile, L->d_x16, L->ldx, L->d_a16, L->lda, (size_t)L->max_rows + pad_rows);
@@ -752,7 +735,7 @@ int csk_moe_destroy(csk_moe_layer* L) {
   void* dev[] = {L->d_shared_out, L->d_p2p_epoch, L->d_unit_router, L->d_stage2, L->d_norm_w, L->d_normed, L->d_part, L->d_hn2, L->d_wnorm, L->d_fb_list, L->d_fb, L->d_info, L->d_back, L->d_row_ptr, L->d_p2p_base, L->d_peer_x16, L->d_peer_info, L->d_peer_back,
                  L->d_router_phys, L->d_slot_map, L->d_weights, L->d_resident, L->d_stage, L->d_wg, L->d_wg_few, L->d_wg_many, L->d_route_cnt, L->d_logits, L->d_rbias, L->d_hidden,
                  L->d_router, L->d_out, L->d_x16, L->d_a16, L->d_y, L->d_counts, L->d_offsets,
-                 L->d_cursor, L->d_row_of_pair, L->d_pair_of_row, L->d_out_row_map, L->d_seg, L->d_tiles, L->d_meta};
+                 L->d_cursor, L->d_row_of_pair, L->d_expert_tiles, L->d_ximg, L->d_aimg, L->d_out_row_map, L->d_seg, L->d_tiles, L->d_meta};
   for (void* p : dev)
     if (p) cudaFree(p);
   if (L->h_meta) cudaFreeHost(L->h_meta);
@@ -817,8 +800,8 @@ int load_expert_enqueue(csk_moe_layer* L, int le, const uint8_t* w_up, const uin
     k_repack_tile_f16<<<grid_for(L->Tgu.bytes() / 16, 256, 4096), 256, 0, s>>>(h_gate, h_up, base + L->off_tgu, L->Tgu);
     k_repack_tile_f16<<<grid_for(L->Td.bytes() / 16, 256, 4096), 256, 0, s>>>(h_down, nullptr, base + L->off_td, L->Td);
   } else {
-  k_repack<<<grid_for(L->Lgu.bytes() / 4, 256, 4096), 256, 0, s>>>(s_gate, s_up, base + L->off_gu, L->Lgu, emeta);
-  k_repack<<<grid_for(L->Ld.bytes() / 4, 256, 4096), 256, 0, s>>>(s_down, nullptr, base + L->off_d, L->Ld, emeta + 1);
+  k_mx_repack<<<grid_for(L->Lgu.bytes() / 16, 256, 4096), 256, 0, s>>>(s_gate, s_up, base + L->off_gu, L->Lgu, emeta);
+  k_mx_repack<<<grid_for(L->Ld.bytes() / 16, 256, 4096), 256, 0, s>>>(s_down, nullptr, base + L->off_d, L->Ld, emeta + 1);
   k_repack_tile<<<grid_for(L->Tgu.bytes() / 4, 256, 4096), 256, 0, s>>>(s_gate, s_up, base + L->off_tgu, L->Tgu);
   k_repack_tile<<<grid_for(L->Td.bytes() / 4, 256, 4096), 256, 0, s>>>(s_down, nullptr, base + L->off_td, L->Td);
   }
@@ -1067,7 +1050,7 @@ struct ImageHeader {
 };
 ImageHeader image_header_of(const csk_moe_layer* L) {
   ImageHeader h{};
-  memcpy(h.magic, "CSKMOE02", 8);  // 02: the streaming layout stores scale byte 255 as 254
+  memcpy(h.magic, "CSKMOE03", 8);  // 03: the block-scaled kernel's layout; it stores scale byte 255 as 254
   h.E = L->E; h.k = L->k; h.H = L->H; h.F = L->F; h.has_bias = L->cfg.has_bias; h.e0 = L->e0; h.eloc = L->Eloc;
   h.expert_stride = L->expert_stride; h.off_gu = L->off_gu; h.off_d = L->off_d; h.off_tgu = L->off_tgu;
   h.off_td = L->off_td; h.off_bias = L->off_bias; h.off_meta = L->off_meta;
@@ -1129,9 +1112,9 @@ int csk_moe_unpack_expert_mxfp4(csk_moe_layer* L, int32_t expert_id, int32_t whi
   CSK_CUDA(L, cudaSetDevice(L->cfg.device));
   const uint8_t* base = L->d_weights + (size_t)(expert_id - L->e0) * L->expert_stride;
   if (which < 3) {
-    const MatLayout& lay = which == 2 ? L->Ld : L->Lgu;
+    const MxLayout& lay = which == 2 ? L->Ld : L->Lgu;
     const uint8_t* packed = base + (which == 2 ? L->off_d : L->off_gu);
-    k_unpack<<<grid_for((size_t)lay.N * (lay.K / 32), 128, 4096), 128, 0, L->stream>>>(
+    k_mx_unpack<<<grid_for((size_t)lay.N * (lay.K / 32), 128, 4096), 128, 0, L->stream>>>(
         packed, L->d_stage, lay, which == 0 ? 1 : 0);
   } else {
     const int w = which - 3;
@@ -1158,6 +1141,11 @@ int csk_moe_set_path(csk_moe_layer* L, int32_t path) {
     return fail(L, CSK_ERR_INVALID, "fp16 weights run on the one-CTA tensor-core kernel only");
   if (path == CSK_PATH_TILE_PAIR && !L->pair.available)
     return fail(L, CSK_ERR_INVALID, "the CTA-pair kernel is not available on this device: %s", L->pair.err.c_str());
+  CSK_CUDA(L, cudaSetDevice(L->cfg.device));
+  if (path == CSK_PATH_STREAM) {  // any batch may come: images for all of it
+    int rc = mx_reserve(L, L->max_rows);
+    if (rc) return rc;
+  }
   L->path = path;
   drop_graphs(L);
   return CSK_OK;
@@ -1874,11 +1862,17 @@ int csk_moe_ep_p2p_experts_dev(csk_moe_layer* L, const int32_t* d_all_counts, in
   cudaStream_t s = pick(L, stream);
   rows_hint = std::max<int64_t>(1, std::min<int64_t>(rows_hint, L->max_rows));
   const int path = choose_path(L, rows_hint);
-  const int tile_rows = tile_rows_for(L, path, rows_hint);
+  const int tile_rows = tile_rows_for(L, path);
+  const bool mx = path == CSK_PATH_STREAM;
+  if (mx) {  // the hint is no bound on the rows that arrive
+    int rc = mx_reserve(L, L->max_rows);
+    if (rc) return rc;
+  }
   // the status word of the dispatch stays; the tile list is rebuilt from the received counts
   k_ep_p2p_local_counts<<<(L->E + 255) / 256, 256, 0, s>>>(d_all_counts, L->p2p_world, L->E, L->e0, L->Eloc, L->d_counts);
   k_scan<<<1, 1024, 0, s>>>(L->d_counts, L->E, L->e0, L->Eloc, tile_rows, (int)L->max_rows, L->max_tiles,
-                            L->d_resident, L->d_offsets, L->d_cursor, L->d_tiles, L->d_meta, nullptr, 0, -1, nullptr, nullptr);
+                            L->d_resident, L->d_offsets, L->d_cursor, L->d_tiles, L->d_meta, nullptr, 0, -1, nullptr,
+                            mx ? L->d_expert_tiles : nullptr);
   k_ep_p2p_rowptr<<<4 * L->sm_count, 256, 0, s>>>(L->d_info, L->d_meta, L->d_peer_back, L->H, L->d_row_ptr,
                                                   (int)L->max_rows, L->p2p_world, (int)L->max_rows);
   CSK_CUDA(L, cudaGetLastError());
@@ -1886,9 +1880,10 @@ int csk_moe_ep_p2p_experts_dev(csk_moe_layer* L, const int32_t* d_all_counts, in
   tm.mark();
   int rc;
   if (path == CSK_PATH_TILE) {
-    rc = launch_experts(L, path, tile_rows, rows_hint, rows_hint, L->d_x16, nullptr, L->H, nullptr, s, tm, L->d_row_ptr);
+    rc = launch_experts(L, path, nullptr, L->H, nullptr, s, tm, L->d_row_ptr);
   } else {
-    rc = launch_experts(L, path, tile_rows, rows_hint, rows_hint, L->d_x16, L->d_y, L->H, nullptr, s, tm);
+    mx_quant_rows(L, s);
+    rc = launch_experts(L, path, L->d_y, L->H, nullptr, s, tm);
     if (!rc) {
       k_ep_p2p_return<<<8 * L->sm_count, 256, 0, s>>>(L->d_y, L->H, L->d_row_ptr, L->d_meta, (int)L->max_rows);
       CSK_CUDA(L, cudaGetLastError());
@@ -1918,12 +1913,18 @@ int csk_moe_ep_experts_dev(csk_moe_layer* L, const void* d_recv_f16, const int32
   cudaStream_t s = pick(L, stream);
   if (total_rows == 0) return CSK_OK;
   const int path = choose_path(L, total_rows);
-  const int tile_rows = tile_rows_for(L, path, total_rows);
+  const int tile_rows = tile_rows_for(L, path);
+  const bool mx = path == CSK_PATH_STREAM;
+  if (mx) {
+    int rc = mx_reserve(L, L->max_rows);
+    if (rc) return rc;
+  }
   CSK_CUDA(L, cudaMemsetAsync(L->d_meta, 0, sizeof(int) * 8, s));
   CSK_CUDA(L, cudaMemsetAsync(L->d_counts, 0, sizeof(int) * L->E, s));
   k_ep_plan<<<1, 1024, 0, s>>>(d_recv_counts, n_src, L->Eloc, L->e0, L->d_counts, L->d_seg);
   k_scan<<<1, 1024, 0, s>>>(L->d_counts, L->E, L->e0, L->Eloc, tile_rows, (int)L->max_rows, L->max_tiles,
-                            L->d_resident, L->d_offsets, L->d_cursor, L->d_tiles, L->d_meta, nullptr, 0, -1, nullptr, nullptr);
+                            L->d_resident, L->d_offsets, L->d_cursor, L->d_tiles, L->d_meta, nullptr, 0, -1, nullptr,
+                            mx ? L->d_expert_tiles : nullptr);
   k_ep_regroup<<<dim3((unsigned)(n_src * L->Eloc), (unsigned)std::max(1, 16 * L->sm_count / (n_src * L->Eloc))), 128, 0, s>>>((const __half*)d_recv_f16, L->d_x16, L->ldx, L->d_seg,
                                                L->d_offsets, n_src, L->Eloc, L->e0, L->d_out_row_map);
   CSK_CUDA(L, cudaGetLastError());
@@ -1931,9 +1932,10 @@ int csk_moe_ep_experts_dev(csk_moe_layer* L, const void* d_recv_f16, const int32
   tm.mark();
   int rc;
   if (path == CSK_PATH_TILE) {
-    rc = launch_experts(L, path, tile_rows, total_rows, total_rows, L->d_x16, d_ret, L->H, L->d_out_row_map, s, tm);
+    rc = launch_experts(L, path, d_ret, L->H, L->d_out_row_map, s, tm);
   } else {
-    rc = launch_experts(L, path, tile_rows, total_rows, total_rows, L->d_x16, L->d_y, L->H, nullptr, s, tm);
+    mx_quant_rows(L, s);
+    rc = launch_experts(L, path, L->d_y, L->H, nullptr, s, tm);
     if (!rc) {
       k_ep_ungroup<<<grid_for((size_t)total_rows, 8, 8 * L->sm_count), 256, 0, s>>>(
           L->d_y, d_ret, L->H, L->d_out_row_map, (int)total_rows);

@@ -1,0 +1,695 @@
+// Block-scaled grouped contraction over MXFP4 weights (the decode-side kernel), written for sm_100a.
+//
+// The weights go to the tensor cores AS THEY ARE: tcgen05.mma kind::mxf4 multiplies E2M1 codes under E8M0 block
+// scales, so no weight is ever converted, and the kernel's only bulk work is moving the packed bytes from HBM to
+// shared memory.  Its other operand has to be E2M1 codes under E8M0 scales too, so every activation row is written
+// as FIVE rows of such codes (the "digits" of a radix-8 expansion, below), which are five columns of the same MMA;
+// the accumulators of the five are added with weights 8^-p in the epilogue.  Tensor throughput is not what bounds
+// this kernel (an MXFP4 MMA runs four times as fast as the fp16 one), so five columns per row cost nothing until a
+// tile holds some 25 rows.
+//
+// Digits.  For a block of 32 values with largest magnitude m the scale is the power of two 2^e with m <= 4.5 * 2^e.
+// Digit 0 is v / 2^e rounded to E2M1 (0, 0.5, 1, 1.5, 2, 3, 4, 6): the remainder of a value of magnitude up to 4.5 is
+// at most 0.5, so eight times the remainder is again at most 4: digits 1 to 4 repeat the step.  What the fifth digit
+// leaves is at most 0.5 * 8^-4 * 2^e, i.e. 2^-14.2 of the block's largest value (fp16 operands keep 2^-12 of each
+// value; over a block the digits' error norm is the smaller one whatever the distribution: measured 2.9e-5 of the
+// norm for normal values and 5.5e-5 for fifth powers of normal values, fp16 2.1e-4 for both).  Products of codes are
+// exact and the sums are fp32.
+//
+//   * a work unit is (row tile of up to 48 grouped token rows of one expert) x (256 weight rows, as two halves of
+//     128: gate and up rows of the same 128 features, or 256 rows of a plain matrix); units are dealt to one
+//     persistent CTA per SM;
+//   * along K the unit is a run of records of 128 columns: 2 x 8192 bytes of codes and 2 x 512 bytes of scales,
+//     contiguous in memory, moved with ONE bulk copy each; a second bulk copy brings the same columns of the token
+//     rows' image.  A ring of 6 to 11 such stages keeps 100-190 KB per SM in flight;
+//   * the MMA warp copies the record's scales to tensor memory (tcgen05.cp) and issues two K=64 MMAs per half;
+//   * eight epilogue warps add up the digits' accumulators, add the bias and either apply the gated activation and
+//     write the result as digits again (a warp's 32 lanes are the 32 features of one block), in the image the down
+//     projection reads, or (plain matrix) store fp32 output rows.  Up to 22 rows the accumulators are doubled and
+//     the epilogue of one unit runs under the MMAs of the next.
+//
+// The producer asks for weights before griddepcontrol.wait: the tile list comes from a kernel two launches back.
+//
+// Every wait is bounded (csk_common.cuh); when one runs out the CTA records kDevErrWaitTimeout, all roles leave
+// their loops, copies and MMAs in flight are waited for (bounded again), tensor memory is freed.
+//
+// Follows the arithmetic of expert_mlp_node::compute_token_mxfp4
+// (include/coalsack/nn/nn_ops/expert_mlp_node.h:651-732): up/gate projections + bias, gated activation, down
+// projection + bias.
+#pragma once
+
+#include "csk_common.cuh"
+#include "csk_tc.cuh"
+
+namespace csk {
+
+constexpr int kMxDigits = 5;
+constexpr int kMxTileRows = 48;                    // token rows of a row tile: 5 * 48 = 240 <= 256 MMA columns
+constexpr int kMxMaxN = kMxDigits * kMxTileRows;
+constexpr int kMxRecBlocks = 4;                    // 32-column blocks per record
+constexpr int kMxSfAtom = 512;                     // scales of 128 rows x 4 blocks: [row % 32][row / 32][block]
+constexpr int kMxARecMax = kMxRecBlocks * 256 * 16 + 2 * kMxSfAtom;
+constexpr int kMxEpilogueWarps = 8;
+constexpr int kMxThreads = (2 + kMxEpilogueWarps) * 32;
+constexpr int kMxMaxStages = 12;
+constexpr int kMxSmem = 227 * 1024;
+constexpr int kMxCtrl = 512;
+constexpr int kMxSlack = 4096;      // a half of fewer than 128 rows lets the MMA read past its codes
+constexpr uint32_t kMxTmemCols = 512;
+constexpr uint32_t kMxTmemSf = 480;                // two sets of 16 columns: SF of half 0, of half 1, of the rows (8)
+
+// Device layout of a matrix for this kernel: units of 256 rows (paired: 128 gate + 128 up rows of the same features)
+// in order; a unit is `recs` records along K; a record of nb (4, the last one 2 or 4) 32-column blocks is
+//   for each pair of blocks: [half 0: 2 blocks x r0 rows x 16 bytes][half 1: 2 blocks x r1 rows x 16 bytes],
+//   then per half one 512-byte atom of scales.
+// 16 bytes are a row's 32 codes, column 2i in the low nibble of byte i.  r0, r1 are the half's real rows (the last
+// unit may have fewer than 128); columns past K are zero codes, scales of absent rows and columns 0.
+struct MxLayout {
+  int N, K, paired;
+  int n_units, blocks /* even */, recs;
+  __host__ __device__ int rows(int nt, int half) const {
+    const int left = paired ? N - nt * 128 : N - nt * 256 - half * 128;
+    return left < 0 ? 0 : left > 128 ? 128 : left;
+  }
+  __host__ __device__ int halves(int nt) const { return rows(nt, 1) > 0 ? 2 : 1; }
+  __host__ __device__ int rec_blocks(int rec) const { return blocks - rec * kMxRecBlocks < kMxRecBlocks ? blocks - rec * kMxRecBlocks : kMxRecBlocks; }
+  __host__ __device__ int rec_bytes(int nt, int nb) const {
+    return nb * (rows(nt, 0) + rows(nt, 1)) * 16 + halves(nt) * kMxSfAtom;
+  }
+  __host__ __device__ size_t unit_bytes(int nt) const {
+    return (size_t)blocks * (rows(nt, 0) + rows(nt, 1)) * 16 + (size_t)recs * halves(nt) * kMxSfAtom;
+  }
+  __host__ __device__ size_t bytes() const { return (size_t)(n_units - 1) * unit_bytes(0) + unit_bytes(n_units - 1); }
+};
+inline MxLayout make_mx_layout(int N, int K, bool paired) {
+  MxLayout L{};
+  L.N = N;
+  L.K = K;
+  L.paired = paired ? 1 : 0;
+  L.n_units = ceil_div(N, paired ? 128 : 256);
+  L.blocks = 2 * ceil_div(K, 64);
+  L.recs = ceil_div(L.blocks, kMxRecBlocks);
+  return L;
+}
+
+// The image of a row tile of `rows` token rows (5 * rows MMA columns, padded to a multiple of 16): per record
+// [scale atoms][4 blocks x npad x 16 bytes of codes]; column 5 r + p is digit p of row r.  Tiles lie one after the
+// other in row order; `col0` and `atom0` bound what the tiles before this one take.
+struct MxTileImage {
+  int npad, atoms;
+  size_t offset;      // of the tile's image
+  size_t rec_stride;
+};
+__host__ __device__ inline int mx_npad(int rows) { return (kMxDigits * rows + 15) / 16 * 16; }
+__host__ __device__ inline MxTileImage mx_tile_image(int tile, int row0, int rows, int recs) {
+  MxTileImage t;
+  t.npad = mx_npad(rows);
+  t.atoms = t.npad > 128 ? 2 : 1;
+  const size_t col0 = (size_t)kMxDigits * row0 + 16 * (size_t)tile;
+  const size_t atom0 = (size_t)kMxDigits * row0 / 128 + 2 * (size_t)tile;
+  t.offset = (size_t)recs * (col0 * (kMxRecBlocks * 16) + atom0 * kMxSfAtom);
+  t.rec_stride = (size_t)t.atoms * kMxSfAtom + (size_t)t.npad * (kMxRecBlocks * 16);
+  return t;
+}
+inline size_t mx_image_bytes(size_t rows, size_t tiles, int recs) {
+  return (size_t)recs * ((kMxDigits * rows + 16 * tiles) * (kMxRecBlocks * 16) +
+                         (kMxDigits * rows / 128 + 2 * tiles + 2) * kMxSfAtom);
+}
+__device__ __forceinline__ size_t mx_sf_pos(int n, int kb) {  // column n's scale of block kb inside a record's atoms
+  return (size_t)(n >> 7) * kMxSfAtom + (n & 31) * 16 + ((n & 127) >> 5) * 4 + (kb & 3);
+}
+
+// ---- repack and its inverse ---------------------------------------------------------------------------------------
+// One thread per (row, block): 17 raw bytes -> 16 bytes of codes and a scale byte; then one thread per absent row's
+// scale.  src1 = up matrix when paired.  A raw block holds column j in the low and column j + 16 in the high nibble
+// of byte j.  Scale byte 255 (NaN in the OCP MX specification) is stored as 254, so that a block of zero codes stays
+// zero under any scale byte, as in the reference.
+__global__ void k_mx_repack(const uint8_t* __restrict__ src0, const uint8_t* __restrict__ src1, uint8_t* __restrict__ dst,
+                            MxLayout L, int* __restrict__ emax_out) {
+  int emax = -1;
+  const int halves_all = 2 * L.n_units;
+  const size_t n = (size_t)halves_all * L.recs * kMxRecBlocks * 128;
+  const size_t unit0 = L.unit_bytes(0);
+  for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
+    const int kb = (int)(i % (L.recs * kMxRecBlocks));  // neighbouring threads: neighbouring raw blocks of one row
+    const size_t rest = i / (L.recs * kMxRecBlocks);
+    const int r = (int)(rest % 128), half = (int)((rest / 128) & 1), nt = (int)(rest / 256);
+    if (half >= L.halves(nt)) continue;
+    const int rec = kb / kMxRecBlocks, nb = L.rec_blocks(rec), kbl = kb % kMxRecBlocks;
+    const int r0 = L.rows(nt, 0), r1 = L.rows(nt, 1), rh = half ? r1 : r0;
+    uint8_t* record = dst + nt * unit0 + (size_t)rec * L.rec_bytes(nt, kMxRecBlocks);
+    const int row = L.paired ? nt * 128 + r : nt * 256 + half * 128 + r;
+    const bool real = r < rh && kb * 32 < L.K;
+    uint32_t e = 0;
+    uint32_t w[4] = {0u, 0u, 0u, 0u};
+    if (real) {
+      const uint8_t* b = (L.paired && half ? src1 : src0) + ((size_t)row * (L.K / 32) + kb) * 17;
+      e = min((uint32_t)b[0], 254u);
+      // a block of zero codes is zero under any scale: it does not widen the matrix's exponent range
+      uint32_t any = 0;
+#pragma unroll
+      for (int j = 1; j < 17; ++j) any |= b[j];
+      if (any) emax = max(emax, (int)e);
+#pragma unroll
+      for (int q = 0; q < 8; ++q) {
+        const uint32_t x = b[1 + 2 * q], y = b[2 + 2 * q];
+        const uint32_t lo = (x & 0xFu) | (y & 0xFu) << 4, hi = x >> 4 | (y >> 4) << 4;
+        w[q >> 2] |= lo << (8 * (q & 3));
+        w[2 + (q >> 2)] |= hi << (8 * (q & 3));
+      }
+    }
+    if (r < rh && kbl < nb)
+      *reinterpret_cast<uint4*>(record + (kbl >> 1) * 32 * (r0 + r1) + half * 32 * r0 + (size_t)(kbl & 1) * 16 * rh +
+                                (size_t)r * 16) = make_uint4(w[0], w[1], w[2], w[3]);
+    record[nb * (r0 + r1) * 16 + half * kMxSfAtom + (r & 31) * 16 + (r >> 5) * 4 + kbl] = (uint8_t)e;
+  }
+  emax = __reduce_max_sync(0xffffffffu, emax);
+  if ((threadIdx.x & 31) == 0 && emax >= 0) atomicMax(emax_out, emax);  // largest scale exponent of the non-zero blocks
+}
+// which_half: 0 = the matrix itself or the gate rows, 1 = the up rows.  One thread per 17-byte block.
+__global__ void k_mx_unpack(const uint8_t* __restrict__ packed, uint8_t* __restrict__ out, MxLayout L, int which_half) {
+  const int kbs = L.K / 32;
+  const size_t n = (size_t)L.N * kbs;
+  for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
+    const int row = (int)(i / kbs), kb = (int)(i % kbs);
+    const int nt = row / (L.paired ? 128 : 256), half = L.paired ? which_half : row / 128 % 2, r = row % 128;
+    const int rec = kb / kMxRecBlocks, nb = L.rec_blocks(rec), kbl = kb % kMxRecBlocks;
+    const int r0 = L.rows(nt, 0), r1 = L.rows(nt, 1), rh = half ? r1 : r0;
+    const uint8_t* record = packed + nt * L.unit_bytes(0) + (size_t)rec * L.rec_bytes(nt, kMxRecBlocks);
+    const uint8_t* c = record + (kbl >> 1) * 32 * (r0 + r1) + half * 32 * r0 + (kbl & 1) * 16 * rh + r * 16;
+    uint8_t* o = out + i * 17;
+    o[0] = record[nb * (r0 + r1) * 16 + half * kMxSfAtom + (r & 31) * 16 + (r >> 5) * 4 + kbl];
+    for (int j = 0; j < 16; ++j) {
+      const uint32_t lo = c[j / 2] >> (4 * (j & 1)) & 0xFu, hi = c[8 + j / 2] >> (4 * (j & 1)) & 0xFu;
+      o[1 + j] = (uint8_t)(lo | hi << 4);
+    }
+  }
+}
+
+// ---- digits ---------------------------------------------------------------------------------------------------------
+// Two values to a byte of E2M1 codes (a in the low nibble), round to nearest even.
+__device__ __forceinline__ uint32_t f32x2_to_e2m1(float a, float b) {
+  uint32_t r;
+  asm("{\n\t.reg .b8 t;\n\tcvt.rn.satfinite.e2m1x2.f32 t, %2, %1;\n\tcvt.u32.u8 %0, t;\n\t}" : "=r"(r) : "f"(a), "f"(b));
+  return r;
+}
+// The scale byte of a block whose largest magnitude has the bit pattern `amax`, and the factor that takes values to
+// digit units: 2^(sf - 127) is the smallest power of two with amax <= 4.5 of it.  A block that holds an infinity or
+// a NaN gets the NaN scale: its row's results are NaN, no other row's.
+__device__ __forceinline__ uint32_t mx_scale_of(uint32_t amax, float& inv) {
+  if (amax >= 0x7F800000u) {
+    inv = 0.f;
+    return 255u;
+  }
+  const uint32_t sf = (__float_as_uint(__uint_as_float(amax) * (1.0f / 4.5f)) + 0x7FFFFFu) >> 23;
+  inv = __uint_as_float((254u - sf) << 23);
+  return sf;
+}
+// One digit of two values; a and b become eight times the remainder.
+__device__ __forceinline__ uint32_t mx_digit(float& a, float& b) {
+  const uint32_t d = f32x2_to_e2m1(a, b);
+  const uint32_t h = e2m1x2_to_h2(d);
+  const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&h));
+  a = (a - f.x) * 8.0f;
+  b = (b - f.y) * 8.0f;
+  return d;
+}
+// A whole block by one thread: digit p's 32 codes in d[p].
+__device__ __forceinline__ uint32_t mx_encode_block(float (&v)[32], uint32_t (&d)[kMxDigits][4]) {
+  uint32_t amax = 0;
+#pragma unroll
+  for (int i = 0; i < 32; ++i) amax = max(amax, __float_as_uint(v[i]) & 0x7FFFFFFFu);
+  float inv;
+  const uint32_t sf = mx_scale_of(amax, inv);
+#pragma unroll
+  for (int i = 0; i < 32; ++i) v[i] *= inv;
+#pragma unroll
+  for (int p = 0; p < kMxDigits; ++p)
+#pragma unroll
+    for (int w = 0; w < 4; ++w) {
+      uint32_t x = 0;
+#pragma unroll
+      for (int q = 0; q < 4; ++q) x |= mx_digit(v[8 * w + 2 * q], v[8 * w + 2 * q + 1]) << (8 * q);
+      d[p][w] = x;
+    }
+  return sf;
+}
+__device__ __forceinline__ void mx_store_block(uint8_t* image, const MxTileImage& g, int r, int kb, const uint32_t (&d)[kMxDigits][4],
+                                               uint32_t sf) {
+  uint8_t* rec = image + g.offset + (size_t)(kb / kMxRecBlocks) * g.rec_stride;
+#pragma unroll
+  for (int p = 0; p < kMxDigits; ++p) {
+    const int n = kMxDigits * r + p;
+    *reinterpret_cast<uint4*>(rec + g.atoms * kMxSfAtom + ((size_t)(kb & 3) * g.npad + n) * 16) =
+        make_uint4(d[p][0], d[p][1], d[p][2], d[p][3]);
+    rec[mx_sf_pos(n, kb)] = (uint8_t)sf;
+  }
+}
+// Columns past K inside the last pair of blocks: the weights' codes are zero there, so any scale but NaN will do.
+__device__ __forceinline__ void mx_store_pad(uint8_t* image, const MxTileImage& g, int r, int kb) {
+  uint8_t* rec = image + g.offset + (size_t)(kb / kMxRecBlocks) * g.rec_stride;
+  for (int p = 0; p < kMxDigits; ++p) rec[mx_sf_pos(kMxDigits * r + p, kb)] = 0;
+}
+
+struct MxQuantArgs {
+  const float* hidden;       // [T,H]
+  const float* router;       // [T,k,2]
+  const int* offsets;        // [E+1] first row of each expert
+  const ExpertTiles* et;     // [E]
+  int* cursor;               // null: row_of_pair is given; else rows are claimed here and row_of_pair is written
+  int* row_of_pair;          // [T*k]
+  const RowTile* tiles;
+  const int* n_tiles_ptr;
+  uint8_t* image;
+  int T, H, E, k, e_begin, e_count, only_expert, max_rows, weight_before_ffn, blocks, recs;
+};
+// Token rows to digits, into the images of the row tiles they were placed in.  One CTA per token, one thread per
+// 32-column block: a token is encoded once and stored k times (with the routing weight applied before the expert
+// it is encoded per pair).  Bound by the latency of one thread's chain (about 900 instructions) for a few tokens.
+__global__ void __launch_bounds__(128) k_mx_quant(const MxQuantArgs A) {
+  __shared__ MxTileImage s_img[16];
+  __shared__ int s_r[16];
+  __shared__ float s_w[16];
+  const int t = blockIdx.x, kbs = A.H / 32;
+  float v[32];
+  uint32_t d[kMxDigits][4], sf = 0;
+  auto load = [&](int kb) {
+    const float4* src = reinterpret_cast<const float4*>(A.hidden + (size_t)t * A.H + kb * 32);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      const float4 x = __ldg(src + i);
+      v[4 * i] = x.x;
+      v[4 * i + 1] = x.y;
+      v[4 * i + 2] = x.z;
+      v[4 * i + 3] = x.w;
+    }
+  };
+  // the hidden states are older than the kernel before this one: encode while it is still placing rows
+  const bool early = !A.weight_before_ffn && (int)threadIdx.x < kbs;
+  if (early) {
+    load(threadIdx.x);
+    sf = mx_encode_block(v, d);
+  }
+  griddep_wait();
+  griddep_launch();
+  if ((int)threadIdx.x < A.k) {
+    const int j = threadIdx.x, pair = t * A.k + j;
+    const int e = (int)A.router[2 * (size_t)pair];
+    const bool mine = e >= 0 && e < A.E && (A.only_expert < 0 || e == A.only_expert);
+    int pos = -1;
+    if (A.cursor) {
+      if (mine) pos = A.offsets[e] + atomicAdd(&A.cursor[e], 1);
+      if (pos >= A.max_rows) pos = -1;
+      A.row_of_pair[pair] = pos;
+    } else {
+      pos = A.row_of_pair[pair];
+    }
+    s_r[j] = -1;
+    if (pos >= 0 && mine && e >= A.e_begin && e < A.e_begin + A.e_count && *A.n_tiles_ptr > 0) {
+      const ExpertTiles et = A.et[e];
+      const int r = pos - A.offsets[e], tile = et.tile0 + r / et.height;
+      const RowTile rt = A.tiles[tile];
+      s_img[j] = mx_tile_image(tile, rt.row0, rt.rows, A.recs);
+      s_r[j] = r % et.height;
+      s_w[j] = A.router[2 * (size_t)pair + 1];
+    }
+  }
+  __syncthreads();
+  for (int kb = threadIdx.x; kb < A.blocks; kb += blockDim.x) {
+    if (kb < kbs && !A.weight_before_ffn && kb != (int)threadIdx.x) {
+      load(kb);
+      sf = mx_encode_block(v, d);
+    }
+    for (int j = 0; j < A.k; ++j) {
+      if (s_r[j] < 0) continue;
+      if (kb >= kbs) {
+        mx_store_pad(A.image, s_img[j], s_r[j], kb);
+        continue;
+      }
+      if (A.weight_before_ffn) {
+        load(kb);
+#pragma unroll
+        for (int i = 0; i < 32; ++i) v[i] *= s_w[j];
+        sf = mx_encode_block(v, d);
+      }
+      mx_store_block(A.image, s_img[j], s_r[j], kb, d, sf);
+    }
+  }
+}
+// The same from grouped fp16 rows (the expert-parallel receive side): a CTA per row tile.
+__global__ void __launch_bounds__(128) k_mx_quant_rows(const __half* __restrict__ x16, int ldx, const RowTile* __restrict__ tiles,
+                                                       const int* __restrict__ n_tiles_ptr, uint8_t* __restrict__ image,
+                                                       int K, int blocks, int recs) {
+  const int n_tiles = *n_tiles_ptr, kbs = K / 32;
+  for (int tile = blockIdx.x; tile < n_tiles; tile += gridDim.x) {
+    const RowTile rt = tiles[tile];
+    const MxTileImage g = mx_tile_image(tile, rt.row0, rt.rows, recs);
+    for (int i = threadIdx.x; i < rt.rows * blocks; i += blockDim.x) {
+      const int r = i / blocks, kb = i % blocks;
+      if (kb >= kbs) {
+        mx_store_pad(image, g, r, kb);
+        continue;
+      }
+      const uint4* src = reinterpret_cast<const uint4*>(x16 + (size_t)(rt.row0 + r) * ldx + kb * 32);
+      float v[32];
+      uint32_t d[kMxDigits][4];
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        const uint4 x = src[q];
+        const uint32_t w[4] = {x.x, x.y, x.z, x.w};
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+          const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&w[c]));
+          v[8 * q + 2 * c] = f.x;
+          v[8 * q + 2 * c + 1] = f.y;
+        }
+      }
+      const uint32_t sf = mx_encode_block(v, d);
+      mx_store_block(image, g, r, kb, d, sf);
+    }
+  }
+}
+
+// ---- the contraction ------------------------------------------------------------------------------------------------
+struct MxArgs {
+  const uint8_t* weights;
+  size_t expert_stride, mat_offset, bias_offset;
+  MxLayout L;
+  const uint8_t* x_img;   // token rows' image, L.recs records
+  uint8_t* a_img;         // GATED: the activated rows' image for the down projection ...
+  int a_blocks, a_recs;   // ... and its blocks and records
+  float* y;               // !GATED: output rows [rows, ldy]
+  int ldy;
+  const RowTile* tiles;
+  const int* n_tiles_ptr;
+  int* meta;              // meta[3] = device status word
+  int has_bias, act, F;
+};
+
+__device__ __forceinline__ float mx_sum(const uint32_t* d) {  // the digits' accumulators, radix 8
+  float v = __uint_as_float(d[kMxDigits - 1]);
+#pragma unroll
+  for (int p = kMxDigits - 2; p >= 0; --p) v = fmaf(v, 0.125f, __uint_as_float(d[p]));
+  return v;
+}
+__device__ __forceinline__ void mx_ld40(uint32_t taddr, uint32_t (&r)[40]) {
+  tmem_ld32(taddr, *reinterpret_cast<uint32_t(*)[32]>(&r[0]));
+  tmem_ld8(taddr + 32, *reinterpret_cast<uint32_t(*)[8]>(&r[32]));
+}
+
+template <bool GATED>
+__global__ void __launch_bounds__(kMxThreads, 1) k_mx(const MxArgs A) {
+  extern __shared__ __align__(128) uint8_t mx_smem[];
+  const MxLayout& L = A.L;
+  // How many columns the launch's tallest row tile takes decides the stage size and whether two accumulator pairs fit:
+  // the tile list knows (meta[4]), the host does not.
+  const int n_max = mx_npad(max(1, A.meta[4]));
+  const uint32_t n_acc = 4 * n_max <= (int)kMxTmemSf ? 2u : 1u;
+  const int stage_bytes = kMxARecMax + (n_max > 128 ? 2 : 1) * kMxSfAtom + (n_max * kMxRecBlocks * 16 + 127) / 128 * 128;
+  const int NS = min(kMxMaxStages, (kMxSmem - kMxCtrl - kMxSlack) / stage_bytes);
+  uint8_t* ctrl = mx_smem + kMxSmem - kMxCtrl;
+  uint64_t* bars = reinterpret_cast<uint64_t*>(ctrl);
+  const uint32_t smem_base = smem_u32(mx_smem), bar_base = smem_u32(bars);
+  auto bar_full = [&](int s) { return bar_base + 8u * s; };
+  auto bar_empty = [&](int s) { return bar_base + 8u * (kMxMaxStages + s); };
+  auto bar_acc_full = [&](int b) { return bar_base + 8u * (2 * kMxMaxStages + b); };
+  auto bar_acc_empty = [&](int b) { return bar_base + 8u * (2 * kMxMaxStages + 2 + b); };
+  const uint32_t bar_drain = bar_base + 8u * (2 * kMxMaxStages + 4);
+  volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(ctrl + 8 * 32);
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(ctrl + 8 * 32 + 8);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < NS; ++s) {
+      mbar_init(bar_full(s), 1);
+      mbar_init(bar_empty(s), 1);
+    }
+    for (int b = 0; b < 2; ++b) {
+      mbar_init(bar_acc_full(b), 1);
+      mbar_init(bar_acc_empty(b), kMxEpilogueWarps);
+    }
+    mbar_init(bar_drain, 1);
+    *abort_flag = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  if (warp == 1) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32((const void*)tmem_slot)),
+                 "r"(kMxTmemCols)
+                 : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem_base = *tmem_slot;
+  // The tile list is two launches old: only the token rows' image has to be waited for.
+  const long n_items = (long)(*A.n_tiles_ptr) * L.n_units;
+
+  if (warp == 0) {
+    // ------------------------------ producer ------------------------------
+    if (lane == 0) {
+      const int n = (int)n_items;
+      bool ok = true;
+      // a stage's weights, and (separately) its token rows; both count on the stage's barrier
+      auto weights = [&](const RowTile& rt, int nt, const MxTileImage& g, int rec, int s) {
+        const int nb = L.rec_blocks(rec);
+        const uint32_t bytes = (uint32_t)L.rec_bytes(nt, nb);
+        mbar_expect_tx(bar_full(s), bytes + (uint32_t)(g.atoms * kMxSfAtom + nb * g.npad * 16));
+        bulk_load(smem_base + (uint32_t)s * stage_bytes,
+                  A.weights + (size_t)rt.expert * A.expert_stride + A.mat_offset + (size_t)nt * L.unit_bytes(0) +
+                      (size_t)rec * L.rec_bytes(nt, kMxRecBlocks),
+                  bytes, bar_full(s));
+      };
+      auto rows = [&](const MxTileImage& g, int rec, int s) {
+        bulk_load(smem_base + (uint32_t)s * stage_bytes + kMxARecMax, A.x_img + g.offset + (size_t)rec * g.rec_stride,
+                  (uint32_t)(g.atoms * kMxSfAtom + L.rec_blocks(rec) * g.npad * 16), bar_full(s));
+      };
+      // as many records of the first units as the ring holds are requested before the rows' image is complete
+      int first = 0;
+      for (int pass = 0; pass < 2; ++pass) {
+        first = 0;
+        for (int item = blockIdx.x; first < NS && item < n; item += gridDim.x) {
+          const int tile = item / L.n_units, nt = item % L.n_units;
+          const RowTile rt = A.tiles[tile];
+          const MxTileImage g = mx_tile_image(tile, rt.row0, rt.rows, L.recs);
+          for (int rec = 0; rec < L.recs && first < NS; ++rec, ++first) {
+            if (pass == 0) weights(rt, nt, g, rec, first);
+            else rows(g, rec, first);
+          }
+        }
+        if (pass == 0) {
+          griddep_wait();
+          asm volatile("fence.proxy.async.global;" ::: "memory");  // the image was written by ordinary stores
+        }
+      }
+      int s = 0, skip = first, issued = first;
+      uint32_t ph = 0;
+      for (int item = blockIdx.x; ok && item < n; item += gridDim.x) {
+        if (skip >= L.recs) {
+          skip -= L.recs;
+          continue;
+        }
+        const int tile = item / L.n_units, nt = item % L.n_units;
+        const RowTile rt = A.tiles[tile];
+        const MxTileImage g = mx_tile_image(tile, rt.row0, rt.rows, L.recs);
+        for (int rec = skip; rec < L.recs; ++rec) {
+          if (!mbar_wait(bar_empty(s), ph, abort_flag)) {
+            ok = false;
+            break;
+          }
+          weights(rt, nt, g, rec, s);
+          rows(g, rec, s);
+          ++issued;
+          if (++s == NS) {
+            s = 0;
+            ph ^= 1u;
+          }
+        }
+        skip = 0;
+      }
+      if (!ok) {
+        // let the copies still in flight land before the CTA goes away
+        for (int i = issued > NS ? issued - NS : 0; i < issued; ++i) {
+          const long long t0 = clock64();
+          while (!mbar_try(bar_full(i % NS), (uint32_t)((i / NS) & 1)) && clock64() - t0 < drain_budget()) {
+          }
+        }
+      }
+    }
+    __syncwarp();
+  } else if (warp == 1) {
+    // ------------------------------ MMA issuer (warp-wide loop, one elected lane issues) ------------------------------
+    const uint32_t tb = __shfl_sync(0xffffffffu, tmem_base, 0);
+    uint32_t c = 0, it = 0;
+    int s = 0;
+    uint32_t ph = 0;
+    bool ok = true;
+    griddep_wait();  // this kernel's successor may count on everything before this kernel's predecessor being complete
+    griddep_launch();
+    for (long item = blockIdx.x; ok && item < n_items; item += gridDim.x, ++it) {
+      const int tile = (int)(item / L.n_units), nt = (int)(item % L.n_units);
+      const int rows = A.tiles[tile].rows;
+      const int npad = mx_npad(rows), atoms = npad > 128 ? 2 : 1;
+      const int r0 = L.rows(nt, 0), r1 = L.rows(nt, 1), halves = L.halves(nt);
+      const uint32_t buf = n_acc == 2u ? it & 1u : 0u;
+      const uint32_t use = n_acc == 2u ? it >> 1 : it;
+      const uint32_t d0 = tb + buf * 2u * (uint32_t)n_max, d1 = d0 + (uint32_t)n_max;
+      ok = __all_sync(0xffffffffu, mbar_wait(bar_acc_empty(buf), (use & 1u) ^ 1u, abort_flag));
+      if (!ok) break;
+      tc_fence_after();
+      for (int rec = 0; rec < L.recs; ++rec, ++c) {
+        ok = __all_sync(0xffffffffu, mbar_wait(bar_full(s), ph, abort_flag));
+        if (!ok) break;
+        tc_fence_after();
+        const int nb = L.rec_blocks(rec);
+        const uint32_t a = smem_base + (uint32_t)s * stage_bytes, b = a + kMxARecMax;
+        const uint32_t sf = tb + kMxTmemSf + (c & 1u) * 16u;
+        const uint32_t a_sf = a + (uint32_t)(nb * (r0 + r1) * 16), b_codes = b + (uint32_t)(atoms * kMxSfAtom);
+        if (elect_one()) {
+          tmem_cp_scales(sf, umma_desc_plain(a_sf, 128, 128));
+          if (halves > 1) tmem_cp_scales(sf + 4, umma_desc_plain(a_sf + kMxSfAtom, 128, 128));
+          tmem_cp_scales(sf + 8, umma_desc_plain(b, 128, 128));
+          if (atoms > 1) tmem_cp_scales(sf + 12, umma_desc_plain(b + kMxSfAtom, 128, 128));
+#pragma unroll
+          for (int p = 0; p < 2; ++p) {
+            if (2 * p < nb) {
+              const uint32_t idesc = umma_idesc_mxf4(npad, 2 * p);
+              const uint64_t db = umma_desc_plain(b_codes + (uint32_t)(2 * p * npad * 16), (uint32_t)(npad * 16), 128);
+              const uint32_t ap = a + (uint32_t)(p * 32 * (r0 + r1));
+              umma_mxf4_ss(d0, umma_desc_plain(ap, (uint32_t)(r0 * 16), 128), db, idesc, sf, sf + 8, (rec | p) ? 1u : 0u);
+              if (halves > 1)
+                umma_mxf4_ss(d1, umma_desc_plain(ap + (uint32_t)(r0 * 32), (uint32_t)(r1 * 16), 128), db, idesc, sf + 4, sf + 8,
+                             (rec | p) ? 1u : 0u);
+            }
+          }
+          umma_commit(bar_empty(s));
+          if (rec == L.recs - 1) umma_commit(bar_acc_full(buf));
+        }
+        __syncwarp();
+        if (++s == NS) {
+          s = 0;
+          ph ^= 1u;
+        }
+      }
+    }
+    // everything issued has to retire before tensor memory is freed
+    if (lane == 0) {
+      umma_commit(bar_drain);
+      const long long t0 = clock64();
+      while (!mbar_try(bar_drain, 0) && clock64() - t0 < drain_budget()) {
+      }
+    }
+    __syncwarp();
+  } else {
+    // ------------------------------ epilogue ------------------------------
+    const int quarter = warp & 3, grp = (warp - 2) >> 2;  // tensor-memory lanes 32 * quarter ..; every second group of 8 rows
+    griddep_wait();  // output rows of an earlier launch of this step are read until then
+    uint32_t it = 0;
+    for (long item = blockIdx.x; item < n_items; item += gridDim.x, ++it) {
+      const int tile = (int)(item / L.n_units), nt = (int)(item % L.n_units);
+      const RowTile rt = A.tiles[tile];
+      const int halves = L.halves(nt);
+      const float* bias = reinterpret_cast<const float*>(A.weights + (size_t)rt.expert * A.expert_stride + A.bias_offset);
+      const uint32_t buf = n_acc == 2u ? it & 1u : 0u;
+      const uint32_t use = n_acc == 2u ? it >> 1 : it;
+      const uint32_t t_acc = tmem_base + ((uint32_t)(quarter * 32) << 16) + buf * 2u * (uint32_t)n_max;
+      const int groups = (rt.rows + 7) >> 3;
+      const int n = (GATED ? nt * 128 : nt * 256) + quarter * 32 + lane;
+      float b0 = 0.f, b1 = 0.f;
+      if (A.has_bias) {
+        if (GATED) {
+          if (n < L.N) {
+            b0 = bias[A.F + n];
+            b1 = bias[n];
+          }
+        } else {
+          if (n < L.N) b0 = bias[2 * A.F + n];
+          if (n + 128 < L.N) b1 = bias[2 * A.F + n + 128];
+        }
+      }
+      if (!mbar_wait(bar_acc_full(buf), use & 1u, abort_flag)) break;
+      tc_fence_after();
+      if (GATED) {
+        const bool live = nt * 128 + quarter * 32 < L.N;  // N is a multiple of 32: a warp's features are real or not as one
+        const MxTileImage g = mx_tile_image(tile, rt.row0, rt.rows, A.a_recs);
+        const int kb = nt * 4 + quarter;
+        uint8_t* rec = A.a_img + g.offset + (size_t)(kb / kMxRecBlocks) * g.rec_stride;
+        for (int gr = grp; gr < groups; gr += 2) {
+          uint32_t rg[40], ru[40];
+          mx_ld40(t_acc + (uint32_t)gr * 40, rg);
+          mx_ld40(t_acc + (uint32_t)n_max + (uint32_t)gr * 40, ru);
+          tmem_ld_wait();
+          if (!live) continue;
+#pragma unroll
+          for (int i = 0; i < 8; i += 2) {
+            const int r = gr * 8 + i;
+            if (r >= rt.rows) break;
+            float v[2];
+            uint32_t sf[2];
+#pragma unroll
+            for (int j = 0; j < 2; ++j) {
+              v[j] = gated_act(mx_sum(rg + 5 * (i + j)) + b0, mx_sum(ru + 5 * (i + j)) + b1, A.act);
+              float inv;
+              sf[j] = mx_scale_of(__reduce_max_sync(0xffffffffu, __float_as_uint(v[j]) & 0x7FFFFFFFu), inv);
+              v[j] *= inv;
+            }
+            uint32_t w = 0, w4;  // byte p: digit p of both rows (low nibble: the even one)
+#pragma unroll
+            for (int p = 0; p < 4; ++p) w |= mx_digit(v[0], v[1]) << (8 * p);
+            w4 = mx_digit(v[0], v[1]);
+            // neighbouring lanes hold neighbouring columns: the even one packs the even row's bytes, the odd one the odd row's
+            const uint32_t o = __shfl_xor_sync(0xffffffffu, w, 1), o4 = __shfl_xor_sync(0xffffffffu, w4, 1);
+            const bool odd = lane & 1;
+            w = odd ? ((o >> 4) & 0x0F0F0F0Fu) | (w & 0xF0F0F0F0u) : (w & 0x0F0F0F0Fu) | ((o & 0x0F0F0F0Fu) << 4);
+            w4 = odd ? (o4 >> 4) | (w4 & 0xF0u) : (w4 & 0x0Fu) | ((o4 & 0x0Fu) << 4);
+            const int my = r + (odd ? 1 : 0);
+            if (my < rt.rows) {
+              uint8_t* dst = rec + g.atoms * kMxSfAtom + ((size_t)(kb & 3) * g.npad + kMxDigits * my) * 16 + (lane >> 1);
+#pragma unroll
+              for (int p = 0; p < 4; ++p) dst[16 * p] = (uint8_t)(w >> (8 * p));
+              dst[64] = (uint8_t)w4;
+              if (lane < 2 * kMxDigits) {
+                const int col = kMxDigits * my + (lane >> 1);
+                rec[mx_sf_pos(col, kb)] = (uint8_t)(odd ? sf[1] : sf[0]);
+                if (kb + 1 < A.a_blocks && (kb + 1) * 32 >= A.F) rec[mx_sf_pos(col, kb + 1)] = 0;  // the padding block
+              }
+            }
+          }
+        }
+      } else {
+        for (int w = grp; w < halves * groups; w += 2) {
+          const int half = w >= groups ? 1 : 0, gr = w - half * groups;
+          uint32_t rd[40];
+          mx_ld40(t_acc + (uint32_t)(half * n_max) + (uint32_t)gr * 40, rd);
+          tmem_ld_wait();
+          const int col = n + 128 * half;
+          if (col >= L.N) continue;
+          float* out = A.y + (size_t)(rt.row0 + gr * 8) * A.ldy + col;
+#pragma unroll
+          for (int i = 0; i < 8; ++i)
+            if (gr * 8 + i < rt.rows) out[(size_t)i * A.ldy] = mx_sum(rd + 5 * i) + (half ? b1 : b0);
+        }
+      }
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(bar_acc_empty(buf));
+    }
+  }
+
+  // ------------------------------ teardown ------------------------------
+  tc_fence_before();
+  __syncthreads();
+  if (threadIdx.x == 0 && *abort_flag) atomicOr(&A.meta[3], kDevErrWaitTimeout);
+  if (warp == 1) {
+    tc_fence_after();
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(kMxTmemCols) : "memory");
+  }
+}
+
+inline cudaError_t mx_prepare_device() {
+  cudaError_t e = cudaFuncSetAttribute(k_mx<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMxSmem);
+  if (e == cudaSuccess) e = cudaFuncSetAttribute(k_mx<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMxSmem);
+  return e;
+}
+
+}  // namespace csk
