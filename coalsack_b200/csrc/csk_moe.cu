@@ -93,6 +93,7 @@ struct csk_moe_layer {
   uint8_t* d_ximg = nullptr;     // the block-scaled kernel's operands: token rows and activated rows as digit images
   uint8_t* d_aimg = nullptr;
   int64_t mx_rows = 0;           // rows the images hold
+  std::vector<uint8_t*> mx_outgrown;
   int* d_out_row_map = nullptr;  // [max_rows] (expert-parallel receive side)
   int* d_seg = nullptr;          // [2*1024+2] segment plan (expert-parallel receive side)
   RowTile* d_tiles = nullptr;
@@ -324,7 +325,9 @@ int launch_permute(csk_moe_layer* L, const float* d_hidden, const float* d_route
   return CSK_OK;
 }
 
-// Images for `rows` grouped rows (row tiles of full height plus one shorter one per expert).
+// Images for `rows` grouped rows (row tiles of full height plus one shorter one per expert).  Called when the layer is
+// created and when a path is chosen, never from a stage: those may run under a caller's capture.  Images that were
+// outgrown live as long as the layer, because graphs captured before (the handle's or a caller's) still name them.
 int mx_reserve(csk_moe_layer* L, int64_t rows) {
   if (L->w16 || rows <= L->mx_rows) return CSK_OK;
   const size_t tiles = (size_t)rows / kMxTileRows + L->Eloc + 1;
@@ -332,17 +335,19 @@ int mx_reserve(csk_moe_layer* L, int64_t rows) {
   uint8_t *x = nullptr, *a = nullptr;
   cudaError_t e = cudaMalloc(&x, xb);
   if (e == cudaSuccess) e = cudaMalloc(&a, ab);
-  if (e == cudaSuccess) e = cudaMemset(x, 0, xb);
-  if (e == cudaSuccess) e = cudaMemset(a, 0, ab);
-  if (e == cudaSuccess) e = cudaDeviceSynchronize();  // also: nothing reads the old images any more
+  if (e == cudaSuccess) e = cudaMemsetAsync(x, 0, xb, L->stream);
+  if (e == cudaSuccess) e = cudaMemsetAsync(a, 0, ab, L->stream);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(L->stream);
   if (e != cudaSuccess) {
     cudaFree(x);
     cudaFree(a);
     cudaGetLastError();
     return fail(L, e == cudaErrorMemoryAllocation ? CSK_ERR_NOMEM : CSK_ERR_CUDA, "row images: %s", cudaGetErrorString(e));
   }
-  cudaFree(L->d_ximg);
-  cudaFree(L->d_aimg);
+  if (L->d_ximg) {  // at most once: the images grow from their first size to max_rows
+    L->mx_outgrown.push_back(L->d_ximg);
+    L->mx_outgrown.push_back(L->d_aimg);
+  }
   L->d_ximg = x;
   L->d_aimg = a;
   L->mx_rows = rows;
@@ -394,6 +399,13 @@ int choose_path(const csk_moe_layer* L, int64_t rows) {
   if (L->path == CSK_PATH_STREAM) return CSK_PATH_STREAM;
   if (L->path == CSK_PATH_TILE || L->path == CSK_PATH_TILE_PAIR) return CSK_PATH_TILE;
   return (L->tile.available && rows >= kMxRowsPerExpert * (int64_t)std::max(1, L->Eloc)) ? CSK_PATH_TILE : CSK_PATH_STREAM;
+}
+
+// The expert-parallel receive side: the caller's row count is no bound on what one expert gets, so the block-scaled
+// kernel needs images for every row the handle may receive (a layer that holds part of the experts has them).
+int choose_path_received(const csk_moe_layer* L, int64_t rows) {
+  const int path = choose_path(L, rows);
+  return path == CSK_PATH_STREAM && L->mx_rows < L->max_rows ? CSK_PATH_TILE : path;
 }
 
 // the CTA-pair kernel runs only when asked for by name (and clusters of two can be launched)
@@ -694,11 +706,6 @@ int csk_moe_create(const csk_moe_config* cfg, csk_moe_layer** out) {
   CK(cudaMalloc(&L->d_cursor, sizeof(int) * L->E));
   CK(cudaMalloc(&L->d_row_of_pair, sizeof(int) * L->max_rows));
   CK(cudaMalloc(&L->d_expert_tiles, sizeof(ExpertTiles) * L->E));
-  if (mx_reserve(L, std::min(L->max_rows, kMxRowsPerExpert * eloc))) {
-    fail(nullptr, CSK_ERR_NOMEM, "%s", L->err.c_str());
-    csk_moe_destroy(L);
-    return CSK_ERR_NOMEM;
-  }
   CK(cudaMalloc(&L->d_out_row_map, sizeof(int) * L->max_rows));
   CK(cudaMalloc(&L->d_seg, sizeof(int) * (3 * 1024 + 8)));
   CK(cudaMalloc(&L->d_tiles, sizeof(RowTile) * L->max_tiles));
@@ -717,6 +724,12 @@ int csk_moe_create(const csk_moe_config* cfg, csk_moe_layer** out) {
       csk_moe_destroy(L);
       return rc;
     }
+  }
+  // images for the batches the block-scaled kernel takes by itself; for any, where rows come from other devices
+  if (mx_reserve(L, eloc < L->E ? L->max_rows : std::min(L->max_rows, kMxRowsPerExpert * eloc))) {
+    fail(nullptr, CSK_ERR_NOMEM, "%s", L->err.c_str());
+    csk_moe_destroy(L);
+    return CSK_ERR_NOMEM;
   }
   CK(cudaDeviceSynchronize());
 #undef CK
@@ -738,6 +751,7 @@ int csk_moe_destroy(csk_moe_layer* L) {
                  L->d_cursor, L->d_row_of_pair, L->d_expert_tiles, L->d_ximg, L->d_aimg, L->d_out_row_map, L->d_seg, L->d_tiles, L->d_meta};
   for (void* p : dev)
     if (p) cudaFree(p);
+  for (uint8_t* p : L->mx_outgrown) cudaFree(p);
   if (L->h_meta) cudaFreeHost(L->h_meta);
   if (L->h_counts64) cudaFreeHost(L->h_counts64);
   for (auto& e : L->ev)
@@ -1861,13 +1875,9 @@ int csk_moe_ep_p2p_experts_dev(csk_moe_layer* L, const int32_t* d_all_counts, in
   CSK_CUDA(L, cudaSetDevice(L->cfg.device));
   cudaStream_t s = pick(L, stream);
   rows_hint = std::max<int64_t>(1, std::min<int64_t>(rows_hint, L->max_rows));
-  const int path = choose_path(L, rows_hint);
+  const int path = choose_path_received(L, rows_hint);
   const int tile_rows = tile_rows_for(L, path);
   const bool mx = path == CSK_PATH_STREAM;
-  if (mx) {  // the hint is no bound on the rows that arrive
-    int rc = mx_reserve(L, L->max_rows);
-    if (rc) return rc;
-  }
   // the status word of the dispatch stays; the tile list is rebuilt from the received counts
   k_ep_p2p_local_counts<<<(L->E + 255) / 256, 256, 0, s>>>(d_all_counts, L->p2p_world, L->E, L->e0, L->Eloc, L->d_counts);
   k_scan<<<1, 1024, 0, s>>>(L->d_counts, L->E, L->e0, L->Eloc, tile_rows, (int)L->max_rows, L->max_tiles,
@@ -1912,13 +1922,9 @@ int csk_moe_ep_experts_dev(csk_moe_layer* L, const void* d_recv_f16, const int32
   CSK_CUDA(L, cudaSetDevice(L->cfg.device));
   cudaStream_t s = pick(L, stream);
   if (total_rows == 0) return CSK_OK;
-  const int path = choose_path(L, total_rows);
+  const int path = choose_path_received(L, total_rows);
   const int tile_rows = tile_rows_for(L, path);
   const bool mx = path == CSK_PATH_STREAM;
-  if (mx) {
-    int rc = mx_reserve(L, L->max_rows);
-    if (rc) return rc;
-  }
   CSK_CUDA(L, cudaMemsetAsync(L->d_meta, 0, sizeof(int) * 8, s));
   CSK_CUDA(L, cudaMemsetAsync(L->d_counts, 0, sizeof(int) * L->E, s));
   k_ep_plan<<<1, 1024, 0, s>>>(d_recv_counts, n_src, L->Eloc, L->e0, L->d_counts, L->d_seg);

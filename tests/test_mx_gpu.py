@@ -47,3 +47,53 @@ def test_edges(gpu_lib, port, E, k, H, F, T, bias, act, wbf):
     after, _ = lay.forward(h)
     assert np.array_equal(after, out)
     lay.close()
+
+
+def test_a_captured_step_outlives_larger_images(gpu_lib, port):
+    """The digit images grow when the streaming kernel is chosen for any batch; a step that a caller captured before
+    that still replays to the same result, on the images it was captured with."""
+    import torch
+    sh = synth.tiny(seed=351, E=2, k=1, H=256, F=192, T=160, has_bias=True)  # more rows than the first images hold
+    h, Wg, rb, ex = cases.layer_inputs(sh, router_scale=30.0)
+    lay = MoeLayer.from_shape(sh)
+    lay.set_router(Wg, rb)
+    lay.load_experts(ex)
+    n = 24
+    h_d, out = torch.from_numpy(h).cuda(), torch.empty((160, 256), device="cuda")
+    s = torch.cuda.Stream()
+    s.wait_stream(torch.cuda.current_stream())
+    lay.forward_dev(h_d, n, torch.empty_like(out), stream=s.cuda_stream)  # (a call's own graph cannot be replayed in a capture)
+    s.synchronize()
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g, stream=s):
+        lay.forward_dev(h_d, n, out, stream=s.cuda_stream)
+    g.replay()
+    torch.cuda.synchronize()
+    first = out[:n].cpu().numpy()
+    want, _ = port.moe_layer(h, Wg, rb, ex, 1, sh.act)
+    mx, mr = cases.err_stats(first, want[:n])
+    assert mx <= MX_MAX and mr <= MX_MEAN, (mx, mr)
+    lay.set_path(PATH_STREAM)
+    whole, _ = lay.forward(h)
+    mx, mr = cases.err_stats(whole, want)
+    assert mx <= MX_MAX and mr <= MX_MEAN, (mx, mr)
+    out.zero_()
+    torch.cuda.synchronize()
+    g.replay()
+    torch.cuda.synchronize()
+    assert np.array_equal(out[:n].cpu().numpy(), first)
+    lay.close()
+
+
+def test_received_rows_without_images_take_the_tensor_core_kernel(gpu_lib, port):
+    """A layer that holds every expert has images for its own small batches only; the expert-parallel receive side may
+    get more rows than those, allocates nothing, and takes the other kernel."""
+    import torch
+    from tests.test_ep_gpu import run_emulated_p2p
+    sh = synth.tiny(seed=353, E=2, k=1, H=256, F=192, T=1, has_bias=True)
+    _, Wg, rb, ex = cases.layer_inputs(sh, router_scale=30.0)
+    for out, ro, hs in run_emulated_p2p(torch, sh, 1, (150,), Wg, rb, ex, 0):
+        want, want_ro = port.moe_layer(hs, Wg, rb, ex, 1, sh.act)
+        assert np.array_equal(ro[..., 0], want_ro[..., 0])
+        mx, mr = cases.err_stats(out, want)
+        assert mx <= cases.MAX_ABS_OVER_RMS and mr <= cases.MEAN_REL, (mx, mr)
