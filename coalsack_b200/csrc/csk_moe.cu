@@ -12,6 +12,7 @@
 #include "csk_kernels.cuh"
 #include "csk_kquant.cuh"
 #include "csk_mx.cuh"
+#include "csk_router_tc.cuh"
 #include "csk_tile.cuh"
 #include "csk_tile2.cuh"
 
@@ -47,6 +48,9 @@ struct csk_moe_layer {
   float* d_wnorm = nullptr;    // [E] 2-norms of the gate rows
   int* d_fb_list = nullptr;    // [max_T] tokens the fast router could not certify
   int* d_fb = nullptr;         // [0] entries of d_fb_list, [1] ticket of its reset, [2..3] 64-bit running total
+  uint8_t* d_wg_tc = nullptr;      // gate rows as digits for the tensor-core router, their scales and norms
+  float* d_wg_tc_scale = nullptr;
+  float* d_wnorm_tc = nullptr;
   int router_mode = CSK_ROUTER_AUTO;
   int64_t routed_tokens = 0;   // tokens routed in certified mode since creation
   float* d_logits = nullptr;  // [max_T,E] router scratch
@@ -202,15 +206,56 @@ int launch_router(csk_moe_layer* L, const float* d_hidden, int64_t T, float* d_r
   // single 2880-step dependency on a few SMs: measured in graph replay on the 128-expert layer it is
   // 51 vs 53 us per step at T=1, level at T=4, and behind from T=16 on (361 vs 342 us at T=64).
   constexpr int64_t kCertifiedMaxTokens = 4;
-  if (L->router_mode == CSK_ROUTER_CHAIN || (L->router_mode == CSK_ROUTER_AUTO && T > kCertifiedMaxTokens)) {
+  // With many tokens the chain is held by its arithmetic, token x expert; the certified pass on the tensor cores costs
+  // little per token, but three launches and the chain of the few percent it cannot separate.  Chain / certified, us:
+  // 128 experts, 2880 columns: 1024 tokens 66 / 49, 2048 117 / 58, 8192 343 / 129; 128 x 2048: 2048 92 / 49; 32 x 2880: 1024
+  // 31 / 44, 4096 64 / 72, 8192 122 / 119 (a digit matrix has 128 rows whatever the experts).
+  constexpr int64_t kTensorMinWork = 4096;  // tokens x groups of 32 experts
+  const int groups = (L->E_router + 31) / 32;
+  const bool few = T <= kCertifiedMaxTokens, many = groups > 1 && T * groups >= kTensorMinWork;
+  if (L->router_mode == CSK_ROUTER_CHAIN || (L->router_mode == CSK_ROUTER_AUTO && !few && !many)) {
     launch_router_logits<true>(a, L->d_wg_few, L->d_wg_many, L->sm_count, s, L->pdl);
     CSK_CUDA(L, cudaGetLastError());
     L->last.launches += 1;
     return CSK_OK;
   }
   // fast logits with error bounds; tokens whose selection the bounds do not certify are listed ...
-  const int groups = (L->E_router + 31) / 32;
-  {
+  FinishRouterArgs g{};
+  g.part = L->d_part;
+  g.hn2 = L->d_hn2;
+  g.bias = a.bias;
+  g.router_out = d_router;
+  g.fb_list = L->d_fb_list;
+  g.fb_count = L->d_fb;
+  g.T = (int)T;
+  g.H = L->H;
+  g.E = L->E_router;
+  g.k = L->k;
+  g.sigmoid = L->cfg.sigmoid_gating;
+  if (many) {
+    RouterTcArgs f{};
+    f.hidden = d_hidden;
+    f.w = L->d_wg_tc;
+    f.w_scale = L->d_wg_tc_scale;
+    f.part = L->d_part;
+    f.hn2 = L->d_hn2;
+    f.status = a.status;
+    f.T = (int)T;
+    f.H = L->H;
+    f.E = L->E_router;
+    const int token_tiles = ceil_div((int)T, kRtTokens), rg = rt_groups(L->E_router);
+    // one CTA fits an SM: as many parts of the hidden dimension as one wave holds
+    int parts = std::min(std::min(rt_blocks(L->H), kFastMaxParts), std::max(1, L->sm_count / (token_tiles * rg)));
+    while (parts > 1 && T * parts > L->part_rows) --parts;
+    launch_k(k_router_tc, dim3((unsigned)token_tiles, (unsigned)rg, (unsigned)parts), dim3(kRtThreads), kRtSmem, s, L->pdl, f);
+    g.wnorm = L->d_wnorm_tc;
+    g.parts = parts;
+    g.slices = rt_blocks(L->H);
+    g.coef_prefix = kRtPrefixCoef;
+    g.coef_norm = kRtNormCoef;
+    launch_k(k_router_finish_many, dim3((unsigned)ceil_div((int)T, kFinishWarps)), dim3(32 * kFinishWarps),
+             sizeof(float) * 2 * kFinishWarps * L->E_router, s, L->pdl, g);
+  } else {
     FastRouterArgs f{};
     f.hidden = d_hidden;
     f.wg = L->d_wg;
@@ -235,19 +280,7 @@ int launch_router(csk_moe_layer* L, const float* d_hidden, int64_t T, float* d_r
       case 8: launch_k(k_router_fast<8>, grid, dim3(128), smem, s, L->pdl, f); break;
       default: launch_k(k_router_fast<16>, grid, dim3(128), smem, s, L->pdl, f); break;
     }
-    FinishRouterArgs g{};
-    g.part = L->d_part;
-    g.hn2 = L->d_hn2;
-    g.bias = a.bias;
     g.wnorm = L->d_wnorm;
-    g.router_out = d_router;
-    g.fb_list = L->d_fb_list;
-    g.fb_count = L->d_fb;
-    g.T = (int)T;
-    g.H = L->H;
-    g.E = L->E_router;
-    g.k = L->k;
-    g.sigmoid = L->cfg.sigmoid_gating;
     g.parts = parts;
     launch_k(k_router_finish, dim3((unsigned)T), dim3((unsigned)std::min(32 * groups, 256)), 0, s, L->pdl, g);
   }
@@ -258,7 +291,8 @@ int launch_router(csk_moe_layer* L, const float* d_hidden, int64_t T, float* d_r
   b.n_list = L->d_fb;
   b.fb_done = L->d_fb + 1;
   b.fb_total = reinterpret_cast<unsigned long long*>(L->d_fb + 2);
-  const int slots = (int)std::min<int64_t>(T, std::max(1, 4 * L->sm_count / groups));
+  // (one round of the grid holds 2 % of 8192 tokens)
+  const int slots = (int)std::min<int64_t>(T, std::max(1, (T > 6144 ? 8 : 4) * L->sm_count / groups));
   launch_router_logits<true>(b, L->d_wg_few, L->d_wg_many, L->sm_count, s, L->pdl, slots);
   CSK_CUDA(L, cudaGetLastError());
   L->last.launches += 3;
@@ -670,6 +704,9 @@ int csk_moe_create(const csk_moe_config* cfg, csk_moe_layer** out) {
   CK(cudaMemset(L->d_route_cnt, 0, sizeof(int) * L->max_T));
   CK(cudaMalloc(&L->d_logits, sizeof(float) * L->max_T * L->E));
   CK(cudaMalloc(&L->d_wnorm, sizeof(float) * L->E));
+  CK(cudaMalloc(&L->d_wg_tc, rt_weight_bytes(L->E, L->H)));
+  CK(cudaMalloc(&L->d_wg_tc_scale, sizeof(float) * rt_scale_floats(L->E, L->H)));
+  CK(cudaMalloc(&L->d_wnorm_tc, sizeof(float) * L->E));
   L->part_rows = L->max_T + 64 * (int64_t)(L->sm_count + fast_router_slices(L->H));
   CK(cudaMalloc(&L->d_part, sizeof(float2) * L->part_rows * L->E));
   CK(cudaMalloc(&L->d_hn2, sizeof(float) * L->part_rows));
@@ -715,6 +752,7 @@ int csk_moe_create(const csk_moe_config* cfg, csk_moe_layer** out) {
   CK(cudaMallocHost(&L->h_counts64, sizeof(int64_t) * L->E));
   CK(router_prepare_device());
   CK(mx_prepare_device());
+  CK(rt_prepare_device());
   {
     int rc = tile_init(L->tile, cfg->device);
     if (!rc) rc = tile_set_buffers(L->tile, L->d_x16, L->ldx, L->d_a16, L->lda, (size_t)L->max_rows + pad_rows);
@@ -745,7 +783,7 @@ int csk_moe_destroy(csk_moe_layer* L) {
     if (g.exec) cudaGraphExecDestroy(g.exec);
   tile_destroy(L->tile);
   for (void* p : L->ipc_opened) cudaIpcCloseMemHandle(p);
-  void* dev[] = {L->d_shared_out, L->d_p2p_epoch, L->d_unit_router, L->d_stage2, L->d_norm_w, L->d_normed, L->d_part, L->d_hn2, L->d_wnorm, L->d_fb_list, L->d_fb, L->d_info, L->d_back, L->d_row_ptr, L->d_p2p_base, L->d_peer_x16, L->d_peer_info, L->d_peer_back,
+  void* dev[] = {L->d_shared_out, L->d_p2p_epoch, L->d_unit_router, L->d_stage2, L->d_norm_w, L->d_normed, L->d_part, L->d_hn2, L->d_wnorm, L->d_wg_tc, L->d_wg_tc_scale, L->d_wnorm_tc, L->d_fb_list, L->d_fb, L->d_info, L->d_back, L->d_row_ptr, L->d_p2p_base, L->d_peer_x16, L->d_peer_info, L->d_peer_back,
                  L->d_router_phys, L->d_slot_map, L->d_weights, L->d_resident, L->d_stage, L->d_wg, L->d_wg_few, L->d_wg_many, L->d_route_cnt, L->d_logits, L->d_rbias, L->d_hidden,
                  L->d_router, L->d_out, L->d_x16, L->d_a16, L->d_y, L->d_counts, L->d_offsets,
                  L->d_cursor, L->d_row_of_pair, L->d_expert_tiles, L->d_ximg, L->d_aimg, L->d_out_row_map, L->d_seg, L->d_tiles, L->d_meta};
@@ -782,6 +820,9 @@ int csk_moe_set_router(csk_moe_layer* L, const float* gate_w, const float* gate_
   k_pack_router<<<grid_for(router_packed_floats(L->E_router, L->H, kRouterChunkMany), 256, 1024), 256, 0, L->stream>>>(
       L->d_wg, L->d_wg_many, L->E_router, L->H, kRouterChunkMany);
   k_router_wnorm<<<(L->E_router + 7) / 8, 256, 0, L->stream>>>(L->d_wg, L->d_wnorm, L->E_router, L->H);
+  k_rt_wnorm<<<(L->E_router + 7) / 8, 256, 0, L->stream>>>(L->d_wg, L->d_wnorm_tc, L->E_router, L->H);
+  k_rt_pack<<<grid_for(rt_scale_floats(L->E_router, L->H), 64, 1024), 64, 0, L->stream>>>(L->d_wg, L->d_wg_tc, L->d_wg_tc_scale,
+                                                                                       L->E_router, L->H);
   CSK_CUDA(L, cudaGetLastError());
   L->has_rbias = gate_bias != nullptr;
   if (gate_bias)

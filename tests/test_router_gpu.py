@@ -111,3 +111,53 @@ def test_near_ties_take_the_chain_and_still_match(gpu_lib, port):
     assert clean.sum() > T // 2
     assert np.array_equal(got[clean][..., 0], want[clean][..., 0])
     lay.close()
+
+
+@pytest.mark.parametrize("E,k,H,T,kind", [
+    (33, 4, 32, 2048, "normal"),     # one block of columns, half of it padding; two groups of 32, 95 of 128 rows padding
+    (128, 8, 96, 1025, "normal"),    # a tile of one token; the last block half full
+    (129, 2, 160, 1024, "heavy"),    # a second group of 128 experts with one row
+    (160, 16, 2080, 1100, "heavy"),  # more parts of the hidden dimension than tiles of one wave
+    (256, 1, 64, 4161, "tiny"),      # digits of blocks near the smallest scale
+    (64, 6, 2880, 8192, "normal"),   # one part, every stage of the ring many times over
+])
+def test_certified_router_on_the_tensor_cores(gpu_lib, port, E, k, H, T, kind):
+    """Large batches: the digits' logits and bounds, where tiles, groups and parts end.  Rows with an infinity or a NaN
+    certify nothing, touch no other row, and go through the chain."""
+    rng = np.random.default_rng(E + T)
+    Wg = (rng.standard_normal((E, H)) * 0.05).astype(np.float32)
+    h = rng.standard_normal((T, H)).astype(np.float32)
+    if kind == "heavy":
+        h, Wg = h ** 5, Wg * np.exp(rng.standard_normal((E, H))).astype(np.float32)
+    if kind == "tiny":
+        h[::3] *= np.float32(2.0 ** -100)
+        h[1::3, : H // 2] = 0
+    rb = None if kind == "heavy" else (rng.standard_normal(E) * 0.01).astype(np.float32)
+    lay = _router_layer(E, k, H, Wg, rb, T)
+    got = lay.route(h)
+    want, logits = port.router_logits(h, Wg, rb, k)
+    top = -np.sort(-logits, axis=1)[:, :k + 1]
+    clean = np.all(top[:, :-1] != top[:, 1:], axis=1)   # the reference leaves the order of equal logits open
+    assert clean.mean() > 0.6
+    assert np.array_equal(got[clean][..., 0], want[clean][..., 0])
+    # a softmax weight moves by at most the logits' errors: the chain's own (measured against 64 bits) and, of the
+    # digits' sums, a few roundings; against 64 bits they are no further off than the chain
+    exact = h.astype(np.float64) @ Wg.T.astype(np.float64) + (0 if rb is None else rb.astype(np.float64))
+    chain_err = np.abs(logits - exact).max(1)
+    tol = 2e-6 + 2 * chain_err
+    assert np.all(np.abs(got[..., 1] - want[..., 1]).max(1)[clean] <= tol[clean])
+    sel = np.take_along_axis(exact, want[..., 0].astype(np.int64), 1)
+    w64 = np.exp(sel - sel.max(1, keepdims=True))
+    w64 /= w64.sum(1, keepdims=True)
+    off_got, off_want = (np.abs(r[clean][..., 1] - w64[clean]).mean() for r in (got, want))
+    assert off_got <= 1.05 * off_want + 1e-9, (off_got, off_want)
+    routed, chained = lay.router_stats()
+    assert routed == T and chained < 0.8 * T
+    bad = h.copy()
+    bad[5, H - 1], bad[T - 1, 0] = np.inf, np.nan
+    other = lay.route(bad)
+    keep = clean.copy()
+    keep[[5, T - 1]] = False
+    assert np.array_equal(other[keep], got[keep])
+    assert lay.router_stats()[1] - chained >= 2
+    lay.close()
