@@ -477,6 +477,22 @@ def test_block_with_norm_and_residual(gpu_lib, port, shape):
     lay.close()
 
 
+@pytest.mark.parametrize("H,T", [(32, 1), (544, 2), (12800, 3), (64, 2500)])  # one batch of squares; ragged; the widest; two rounds
+def test_norm_rows_equal_the_reference_bit_for_bit(gpu_lib, port, H, T):
+    """The block's result against the plain layer on the checker's normed rows: equal in every bit (one summand)."""
+    sh = synth.tiny(seed=53, E=2, k=1, H=H, F=32, T=T, has_bias=True)
+    h, Wg, rb, ex = cases.layer_inputs(sh, router_scale=30.0)
+    nw = (1.0 + 0.1 * np.random.default_rng(530).standard_normal(H)).astype(np.float32)
+    lay = make_layer(sh, Wg, rb, ex, max_tokens=T)
+    lay.set_ffn_norm(nw, 1e-5)
+    x = (h * 3.0).astype(np.float32)
+    out, ro = lay.block_forward(x)
+    out2, ro2 = lay.forward(port.rmsnorm(x, nw, 1e-5))
+    assert np.array_equal(ro, ro2)
+    assert np.array_equal((x + out2).astype(np.float32), out)
+    lay.close()
+
+
 def test_block_with_shared_expert(gpu_lib, port):
     """The Llama-4 style block (llm_engine.cpp:714-777): x -> rmsnorm -> [routed experts -> merge] + [shared dense FFN]
     -> + x in one call.  Routing bit-exact after the fused norm; the result equals x + (layer + dense FFN) of the
