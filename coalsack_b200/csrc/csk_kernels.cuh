@@ -814,6 +814,18 @@ __global__ void k_hist(const float* __restrict__ router_out, int n_pairs, int E,
     if (sc[e]) atomicAdd(&counts[e], sc[e]);
 }
 
+// An expert with several tiles gets them equally tall instead of full ones and a short rest: for the block-scaled
+// kernel always (its time goes by the tile's rows), for the fp16 tensor-core kernel (rounded up to the MMA's 16-row
+// step) with two to four tiles -- a tile's cost is nearly flat below ~175 rows, so 128 + 128 rows are cheaper than
+// 192 + 64, and with more tiles only the last one would change.
+__device__ __forceinline__ int even_tile_height(int cnt, int tile_rows, bool block_scaled) {
+  const int ntl = (cnt + tile_rows - 1) / tile_rows;
+  if (ntl < 2) return tile_rows;
+  const int even = (cnt + ntl - 1) / ntl;
+  if (block_scaled) return even;
+  return tile_rows >= 64 && ntl <= 4 ? min(tile_rows, (even + 15) & ~15) : tile_rows;
+}
+
 // Exclusive scan of the per-expert row counts, row-tile list for tiles of
 // `tile_rows` rows, cursor reset.  One block of 1024 threads, E <= 1024.
 // counts are indexed by GLOBAL expert id; tiles carry the id local to this
@@ -860,17 +872,7 @@ k_scan(int* __restrict__ counts, int E, int e_begin, int e_count, int tile_rows,
   __syncthreads();  // every thread holds its count before s_tile_off is reused
   const bool local = e >= e_begin && e < e_begin + e_count;
   const int nt = local ? (c + tile_rows - 1) / tile_rows : 0;
-  // An expert with several tiles gets them equally tall instead of full ones and a short rest: for the block-scaled
-  // kernel always (its time goes by the tile's rows), for the fp16 tensor-core kernel (rounded up to the MMA's 16-row
-  // step) with two to four tiles -- a tile's cost is nearly flat below ~175 rows, so 128 + 128 rows are cheaper than
-  // 192 + 64, and with more tiles only the last one would change.
-  auto tile_height = [&](int cnt) {
-    const int ntl = (cnt + tile_rows - 1) / tile_rows;
-    if (ntl < 2) return tile_rows;
-    const int even = (cnt + ntl - 1) / ntl;
-    if (expert_tiles) return even;
-    return tile_rows >= 64 && ntl <= 4 ? min(tile_rows, (even + 15) & ~15) : tile_rows;
-  };
+  auto tile_height = [&](int cnt) { return even_tile_height(cnt, tile_rows, expert_tiles != nullptr); };
   if (c > 0) {
     atomicAdd(&s_distinct, 1);
     if (local && resident && !resident[e - e_begin]) atomicOr(&meta[3], kDevErrNotResident);
@@ -1003,6 +1005,35 @@ __global__ void k_scatter(const float* __restrict__ router_out, const float* __r
       o.y = *reinterpret_cast<uint32_t*>(&b);
       *reinterpret_cast<uint2*>(dst + d) = o;
     }
+  }
+}
+
+// The whole plan of a dense FFN (one expert, every token in order): rows to fp16, and by block 0 what k_scan leaves for
+// one expert.  The down projection's rows are the tokens' then, so no combine follows.
+__global__ void __launch_bounds__(256) k_dense_rows(const float* __restrict__ hidden, __half* __restrict__ x16, int ldx, int T, int H,
+                                                    int tile_rows, const uint8_t* __restrict__ resident, int* __restrict__ counts,
+                                                    int* __restrict__ offsets, RowTile* __restrict__ tiles, int* __restrict__ meta) {
+  griddep_wait();
+  griddep_launch();
+  if (blockIdx.x == 0) {
+    const int nt = (T + tile_rows - 1) / tile_rows;
+    const int per = even_tile_height(T, tile_rows, false);
+    for (int i = threadIdx.x; i < nt; i += blockDim.x) tiles[i] = RowTile{0, i * per, min(per, T - i * per), 0};
+    if (threadIdx.x == 0) {
+      counts[0] = offsets[1] = meta[1] = T;
+      offsets[0] = 0;
+      meta[0] = nt;
+      meta[2] = 1;
+      meta[3] = resident[0] ? 0 : kDevErrNotResident;
+      meta[4] = min(per, T);
+    }
+  }
+  const int per_row = H / 8;  // H is a multiple of 32, a row of x16 of 64
+  for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < (size_t)T * per_row; i += (size_t)gridDim.x * blockDim.x) {
+    const int t = (int)(i / per_row), d = (int)(i % per_row) * 8;
+    const float4 a = *reinterpret_cast<const float4*>(hidden + (size_t)t * H + d), b = *reinterpret_cast<const float4*>(hidden + (size_t)t * H + d + 4);
+    const __half2 h[4] = {__floats2half2_rn(a.x, a.y), __floats2half2_rn(a.z, a.w), __floats2half2_rn(b.x, b.y), __floats2half2_rn(b.z, b.w)};
+    *reinterpret_cast<uint4*>(x16 + (size_t)t * ldx + d) = *reinterpret_cast<const uint4*>(h);
   }
 }
 
