@@ -58,7 +58,6 @@ def measured_peaks():
 # Key = (workload name, tokens, kernel).  Other workloads report null.
 MEASURED_TRAFFIC = {
     ("c2_gptoss120b_prefill8192", 8192, "k_tile<gated>"): 1599.2e6,   # 1417.8 MB read + 181.4 MB written
-    ("c3_gptoss120b_decode", 64, "k_stream<gated>"): 954.3e6,        # 949.0 MB read + 5.3 MB written
 }
 
 
@@ -382,10 +381,9 @@ def run_ours(args):
                     "unit": "TFLOP/s", "frac": achieved / peaks["tflops"],
                     "peak_source": peaks["source"] + " (burst bf16 cuBLAS)"}
     else:
-        # weight streaming: algorithmic bytes = the packed gate/up records of every expert that received rows
-        # (544 bytes per 16 features x 64 columns, gate and up), read once per 8- or 16-row tile
-        recs = -(-sh.ffn // 16) * -(-H // 64) * 2
-        gu_bytes = stage.get("row_tiles", 0) * recs * 544.0
+        # weight streaming: algorithmic bytes = the packed gate and up matrices (17 bytes per 32 weights) of every expert
+        # that received rows, read once per 48-row tile
+        gu_bytes = stage.get("row_tiles", 0) * 2.0 * sh.ffn * H * 17 / 32
         achieved = gu_bytes / (gu_ms * 1e-3) / 1e9 if gu_ms > 0 else 0.0
         roofline = {"bound": "hbm", "kernel": stage["gate_up_kernel"], "achieved": achieved, "peak": peaks["hbm_gbs"],
                     "unit": "GB/s", "frac": achieved / peaks["hbm_gbs"],
@@ -464,9 +462,9 @@ class SingleGpu:
         out = {k: acc[k] / n for k in acc}
         out["path"] = {1: "stream", 2: "tile"}.get(int(round(out["path"])), "?")
         rows_per_expert, _, _ = self.layer.counters()
-        tr = 16 if self.T * self.sh.top_k > 8 * self.sh.num_experts else 8
+        tr = 48 if out["path"] == "stream" else 192
         out["row_tiles"] = int(sum(-(-int(r) // tr) for r in rows_per_expert))
-        out["gate_up_kernel"] = "k_stream<gated>" if out["path"] == "stream" else "k_tile<gated>"
+        out["gate_up_kernel"] = "k_mx<gated>" if out["path"] == "stream" else "k_tile<gated>"
         return out
 
     def time_e2e(self, steps, warmup):
