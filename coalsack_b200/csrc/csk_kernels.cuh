@@ -844,7 +844,8 @@ k_scan(int* __restrict__ counts, int E, int e_begin, int e_count, int tile_rows,
        int max_tiles, const uint8_t* __restrict__ resident, int* __restrict__ offsets,
        int* __restrict__ cursor, RowTile* __restrict__ tiles, int* __restrict__ meta,
        const float* __restrict__ router_out, int n_pairs, int only_expert,
-       int* __restrict__ row_of_pair = nullptr, ExpertTiles* __restrict__ expert_tiles = nullptr) {
+       int* __restrict__ row_of_pair = nullptr, ExpertTiles* __restrict__ expert_tiles = nullptr,
+       uint32_t* __restrict__ tile_masks = nullptr, int mask_words = 0) {
   __shared__ int s_row_off[1025];
   __shared__ int s_tile_off[1025];
   __shared__ int s_warp[2][32];
@@ -945,6 +946,8 @@ k_scan(int* __restrict__ counts, int E, int e_begin, int e_count, int tile_rows,
     if (e == 0) meta[4] = 0;
     return;
   }
+  if (tile_masks)  // the block-scaled kernel's record masks: nothing marked yet
+    for (int i = threadIdx.x; i < total_tiles * mask_words; i += blockDim.x) tile_masks[i] = 0;
   for (int i = threadIdx.x; i < total_tiles; i += blockDim.x) {
     // largest expert x with s_tile_off[x] <= i (experts without tiles repeat an offset)
     int lo = 0, hi = 1023;

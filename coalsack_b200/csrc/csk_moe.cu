@@ -96,7 +96,9 @@ struct csk_moe_layer {
   ExpertTiles* d_expert_tiles = nullptr;  // [E] where the experts' row tiles are (block-scaled kernel)
   uint8_t* d_ximg = nullptr;     // the block-scaled kernel's operands: token rows and activated rows as digit images
   uint8_t* d_aimg = nullptr;
+  size_t ximg_rest = 0, aimg_rest = 0;  // where the images of the digits after the first begin
   int64_t mx_rows = 0;           // rows the images hold
+  uint32_t* d_wide = nullptr;    // [max_tiles][mask words of token rows, of activated rows]
   std::vector<uint8_t*> mx_outgrown;
   int* d_out_row_map = nullptr;  // [max_rows] (expert-parallel receive side)
   int* d_seg = nullptr;          // [2*1024+2] segment plan (expert-parallel receive side)
@@ -141,6 +143,8 @@ struct csk_moe_layer {
 };
 
 namespace {
+
+int wide_stride(const csk_moe_layer* L) { return mx_mask_words(L->Lgu.recs) + mx_mask_words(L->Ld.recs); }
 
 int fail(csk_moe_layer* L, int code, const char* fmt, ...) {
   char buf[512];
@@ -315,7 +319,7 @@ int launch_permute(csk_moe_layer* L, const float* d_hidden, const float* d_route
     // small batch: histogram, scan, tile list (and, for digits, the rows' places) in one single-block launch
     launch_k(k_scan, dim3(1), dim3(1024), 0, s, L->pdl, L->d_counts, L->E, e_begin, e_count, tile_rows, (int)max_rows,
              L->max_tiles, res, L->d_offsets, L->d_cursor, L->d_tiles, L->d_meta, d_router, n_pairs, only_expert,
-             digits ? L->d_row_of_pair : (int*)nullptr, et);
+             digits ? L->d_row_of_pair : (int*)nullptr, et, digits ? L->d_wide : (uint32_t*)nullptr, wide_stride(L));
     L->last.launches += 1;
   } else {
     CSK_CUDA(L, cudaMemsetAsync(L->d_counts, 0, sizeof(int) * L->E, s));
@@ -323,7 +327,8 @@ int launch_permute(csk_moe_layer* L, const float* d_hidden, const float* d_route
     k_hist<<<grid_for(n_pairs, 256, 2 * L->sm_count), 256, sizeof(int) * L->E, s>>>(
         d_router, n_pairs, L->E, only_expert, L->d_counts, L->d_meta);
     k_scan<<<1, 1024, 0, s>>>(L->d_counts, L->E, e_begin, e_count, tile_rows, (int)max_rows, L->max_tiles, res,
-                              L->d_offsets, L->d_cursor, L->d_tiles, L->d_meta, nullptr, 0, -1, nullptr, et);
+                              L->d_offsets, L->d_cursor, L->d_tiles, L->d_meta, nullptr, 0, -1, nullptr, et,
+                              digits ? L->d_wide : nullptr, wide_stride(L));
     L->last.launches += 2;
   }
   if (digits) {
@@ -337,6 +342,9 @@ int launch_permute(csk_moe_layer* L, const float* d_hidden, const float* d_route
     a.tiles = L->d_tiles;
     a.n_tiles_ptr = L->d_meta;
     a.image = L->d_ximg;
+    a.rest = L->d_ximg + L->ximg_rest;
+    a.wide = L->d_wide;
+    a.wide_stride = wide_stride(L);
     a.T = (int)T;
     a.H = L->H;
     a.E = L->E;
@@ -348,7 +356,7 @@ int launch_permute(csk_moe_layer* L, const float* d_hidden, const float* d_route
     a.weight_before_ffn = L->cfg.weight_before_ffn;
     a.blocks = L->Lgu.blocks;
     a.recs = L->Lgu.recs;
-    launch_k(k_mx_quant, dim3((unsigned)T), dim3(std::min(128, ceil_div(L->Lgu.blocks, 32) * 32)), 0, s, L->pdl, a);
+    launch_k(k_mx_quant, dim3((unsigned)T), dim3(std::min(kMxQuantThreads, ceil_div(L->Lgu.blocks, 8) * 32)), 0, s, L->pdl, a);
   } else {
     launch_k(k_scatter, dim3(grid_for(n_pairs, 8, 8 * L->sm_count)), dim3(256), 0, s, L->pdl, d_router, d_hidden,
              n_pairs, L->k, L->H, L->E, only_expert, L->d_offsets, L->d_cursor, L->d_row_of_pair, x16, ldx, (int)max_rows,
@@ -365,7 +373,8 @@ int launch_permute(csk_moe_layer* L, const float* d_hidden, const float* d_route
 int mx_reserve(csk_moe_layer* L, int64_t rows) {
   if (L->w16 || rows <= L->mx_rows) return CSK_OK;
   const size_t tiles = (size_t)rows / kMxTileRows + L->Eloc + 1;
-  const size_t xb = mx_image_bytes(rows, tiles, L->Lgu.recs), ab = mx_image_bytes(rows, tiles, L->Ld.recs);
+  const size_t x1 = (mx_image_bytes(kMxDigitsX, rows, tiles, L->Lgu.recs) + 255) / 256 * 256, xb = 2 * x1;
+  const size_t a1 = (mx_image_bytes(kMxDigitsA, rows, tiles, L->Ld.recs) + 255) / 256 * 256, ab = 2 * a1;
   uint8_t *x = nullptr, *a = nullptr;
   cudaError_t e = cudaMalloc(&x, xb);
   if (e == cudaSuccess) e = cudaMalloc(&a, ab);
@@ -384,14 +393,16 @@ int mx_reserve(csk_moe_layer* L, int64_t rows) {
   }
   L->d_ximg = x;
   L->d_aimg = a;
+  L->ximg_rest = x1;
+  L->aimg_rest = a1;
   L->mx_rows = rows;
   return CSK_OK;
 }
 
 // The grouped fp16 rows of the expert-parallel receive side as digits.
 void mx_quant_rows(csk_moe_layer* L, cudaStream_t s) {
-  k_mx_quant_rows<<<4 * L->sm_count, 128, 0, s>>>(L->d_x16, L->ldx, L->d_tiles, L->d_meta, L->d_ximg, L->H, L->Lgu.blocks,
-                                                  L->Lgu.recs);
+  k_mx_quant_rows<<<4 * L->sm_count, 128, 0, s>>>(L->d_x16, L->ldx, L->d_tiles, L->d_meta, L->d_ximg, L->d_ximg + L->ximg_rest,
+                                                  L->d_wide, wide_stride(L), L->H, L->Lgu.blocks, L->Lgu.recs);
 }
 
 void launch_mx_pair(csk_moe_layer* L, float* y, int ldy, cudaStream_t s, StageTimer& tm) {
@@ -409,7 +420,12 @@ void launch_mx_pair(csk_moe_layer* L, float* y, int ldy, cudaStream_t s, StageTi
   a.mat_offset = L->off_gu;
   a.L = L->Lgu;
   a.x_img = L->d_ximg;
+  a.x_rest = L->d_ximg + L->ximg_rest;
+  a.x_wide = L->d_wide;
   a.a_img = L->d_aimg;
+  a.a_rest = L->d_aimg + L->aimg_rest;
+  a.a_wide = L->d_wide + mx_mask_words(L->Lgu.recs);
+  a.wide_stride = wide_stride(L);
   a.a_blocks = L->Ld.blocks;
   a.a_recs = L->Ld.recs;
   launch_k(k_mx<true>, dim3(L->sm_count), dim3(kMxThreads), kMxSmem, s, L->pdl, a);
@@ -417,7 +433,9 @@ void launch_mx_pair(csk_moe_layer* L, float* y, int ldy, cudaStream_t s, StageTi
   // down
   a.mat_offset = L->off_d;
   a.L = L->Ld;
-  a.x_img = L->d_aimg;
+  a.x_img = a.a_img;
+  a.x_rest = a.a_rest;
+  a.x_wide = a.a_wide;
   a.y = y;
   a.ldy = ldy;
   launch_k(k_mx<false>, dim3(L->sm_count), dim3(kMxThreads), kMxSmem, s, L->pdl, a);
@@ -426,7 +444,7 @@ void launch_mx_pair(csk_moe_layer* L, float* y, int ldy, cudaStream_t s, StageTi
 }
 
 // Rows per resident expert from which the fp16 tensor-core kernel takes over.
-constexpr int64_t kMxRowsPerExpert = 48;
+constexpr int64_t kMxRowsPerExpert = 40;
 
 int choose_path(const csk_moe_layer* L, int64_t rows) {
   if (L->w16) return CSK_PATH_TILE;  // fp16 weights exist in the tensor-core layout only
@@ -766,6 +784,7 @@ int csk_moe_create(const csk_moe_config* cfg, csk_moe_layer** out) {
   CK(cudaMalloc(&L->d_out_row_map, sizeof(int) * L->max_rows));
   CK(cudaMalloc(&L->d_seg, sizeof(int) * (3 * 1024 + 8)));
   CK(cudaMalloc(&L->d_tiles, sizeof(RowTile) * L->max_tiles));
+  CK(cudaMalloc(&L->d_wide, sizeof(uint32_t) * L->max_tiles * wide_stride(L)));
   CK(cudaMalloc(&L->d_meta, sizeof(int) * 16));
   CK(cudaMemset(L->d_meta, 0, sizeof(int) * 16));
   CK(cudaMallocHost(&L->h_meta, sizeof(int) * 16));
@@ -806,7 +825,7 @@ int csk_moe_destroy(csk_moe_layer* L) {
   void* dev[] = {L->d_shared_out, L->d_p2p_epoch, L->d_unit_router, L->d_stage2, L->d_norm_w, L->d_normed, L->d_part, L->d_hn2, L->d_wnorm, L->d_wg_tc, L->d_wg_tc_scale, L->d_wnorm_tc, L->d_fb_list, L->d_fb, L->d_info, L->d_back, L->d_row_ptr, L->d_p2p_base, L->d_peer_x16, L->d_peer_info, L->d_peer_back,
                  L->d_router_phys, L->d_slot_map, L->d_weights, L->d_resident, L->d_stage, L->d_wg, L->d_wg_few, L->d_wg_many, L->d_route_cnt, L->d_logits, L->d_rbias, L->d_hidden,
                  L->d_router, L->d_out, L->d_x16, L->d_a16, L->d_y, L->d_counts, L->d_offsets,
-                 L->d_cursor, L->d_row_of_pair, L->d_expert_tiles, L->d_ximg, L->d_aimg, L->d_out_row_map, L->d_seg, L->d_tiles, L->d_meta};
+                 L->d_cursor, L->d_row_of_pair, L->d_expert_tiles, L->d_ximg, L->d_aimg, L->d_wide, L->d_out_row_map, L->d_seg, L->d_tiles, L->d_meta};
   for (void* p : dev)
     if (p) cudaFree(p);
   for (uint8_t* p : L->mx_outgrown) cudaFree(p);
@@ -1943,7 +1962,7 @@ int csk_moe_ep_p2p_experts_dev(csk_moe_layer* L, const int32_t* d_all_counts, in
   k_ep_p2p_local_counts<<<(L->E + 255) / 256, 256, 0, s>>>(d_all_counts, L->p2p_world, L->E, L->e0, L->Eloc, L->d_counts);
   k_scan<<<1, 1024, 0, s>>>(L->d_counts, L->E, L->e0, L->Eloc, tile_rows, (int)L->max_rows, L->max_tiles,
                             L->d_resident, L->d_offsets, L->d_cursor, L->d_tiles, L->d_meta, nullptr, 0, -1, nullptr,
-                            mx ? L->d_expert_tiles : nullptr);
+                            mx ? L->d_expert_tiles : nullptr, mx ? L->d_wide : nullptr, wide_stride(L));
   k_ep_p2p_rowptr<<<4 * L->sm_count, 256, 0, s>>>(L->d_info, L->d_meta, L->d_peer_back, L->H, L->d_row_ptr,
                                                   (int)L->max_rows, L->p2p_world, (int)L->max_rows);
   CSK_CUDA(L, cudaGetLastError());
@@ -1991,7 +2010,7 @@ int csk_moe_ep_experts_dev(csk_moe_layer* L, const void* d_recv_f16, const int32
   k_ep_plan<<<1, 1024, 0, s>>>(d_recv_counts, n_src, L->Eloc, L->e0, L->d_counts, L->d_seg);
   k_scan<<<1, 1024, 0, s>>>(L->d_counts, L->E, L->e0, L->Eloc, tile_rows, (int)L->max_rows, L->max_tiles,
                             L->d_resident, L->d_offsets, L->d_cursor, L->d_tiles, L->d_meta, nullptr, 0, -1, nullptr,
-                            mx ? L->d_expert_tiles : nullptr);
+                            mx ? L->d_expert_tiles : nullptr, mx ? L->d_wide : nullptr, wide_stride(L));
   k_ep_regroup<<<dim3((unsigned)(n_src * L->Eloc), (unsigned)std::max(1, 16 * L->sm_count / (n_src * L->Eloc))), 128, 0, s>>>((const __half*)d_recv_f16, L->d_x16, L->ldx, L->d_seg,
                                                L->d_offsets, n_src, L->Eloc, L->e0, L->d_out_row_map);
   CSK_CUDA(L, cudaGetLastError());

@@ -3,30 +3,38 @@
 // The weights go to the tensor cores AS THEY ARE: tcgen05.mma kind::mxf4 multiplies E2M1 codes under E8M0 block
 // scales, so no weight is ever converted, and the kernel's only bulk work is moving the packed bytes from HBM to
 // shared memory.  Its other operand has to be E2M1 codes under E8M0 scales too, so every activation row is written
-// as FIVE rows of such codes (the "digits" of a radix-8 expansion, below), which are five columns of the same MMA;
-// the accumulators of the five are added with weights 8^-p in the epilogue.  Tensor throughput is not what bounds
-// this kernel (an MXFP4 MMA runs four times as fast as the fp16 one), so five columns per row cost nothing until a
-// tile holds some 25 rows.
+// as several rows of such codes (the "digits" of a radix-8 expansion, below), which are as many columns of the same
+// MMA; the accumulators of the digits are added with weights 8^-p in the epilogue.
 //
 // Digits.  For a block of 32 values with largest magnitude m the scale is the power of two 2^e with m <= 4.5 * 2^e.
 // Digit 0 is v / 2^e rounded to E2M1 (0, 0.5, 1, 1.5, 2, 3, 4, 6): the remainder of a value of magnitude up to 4.5 is
-// at most 0.5, so eight times the remainder is again at most 4: digits 1 to 4 repeat the step.  What the fifth digit
-// leaves is at most 0.5 * 8^-4 * 2^e, i.e. 2^-14.2 of the block's largest value (fp16 operands keep 2^-12 of each
-// value; over a block the digits' error norm is the smaller one whatever the distribution: measured 2.9e-5 of the
-// norm for normal values and 5.5e-5 for fifth powers of normal values, fp16 2.1e-4 for both).  Products of codes are
-// exact and the sums are fp32.
+// at most 0.5, so eight times the remainder is again at most 4: the other digits repeat the step.  n digits leave at
+// most 0.5 * 8^(1-n) * 2^e of every value (rms measured: 0.15 * 8^(1-n) * 2^e), the SAME amount of a large and of a small
+// one.  An fp16 operand leaves a share of each value (rms 2.07e-4 of it).  Token rows get five digits, activated rows,
+// whose values spread further, six: measured 2.9e-5 of the norm for normal values in five, 4.6e-6 to 5.8e-6 for gated
+// products of normal values in six, fp16 2.1e-4 for both.  Products of codes are exact and the sums are fp32.
 //
-//   * a work unit is (row tile of up to 48 grouped token rows of one expert) x (256 weight rows, as two halves of
+// Wide blocks.  Where a few values of a block are far above the others, the digits' absolute error may be more than fp16
+// would leave of those others, and the weights of the few may be zero.  Such a block gets as many digits again,
+// continuing the expansion (at most 2^-29 of the block's largest value is then left), in a second image of the same
+// geometry; the records of a row tile that hold any are run twice, once per image, into the same accumulators, and
+// everywhere else the second image holds zeros.  A block is taken as it is only if, WHICHEVER t of its values are left
+// out, the digits' error over the others is no larger than that of an fp16 operand (mx_wide_limit; t = 8 of 32 for
+// token rows, 4 for activated rows).  That costs nothing for normal values (none of 400,000 blocks is wide) and little for gated
+// products of them (7e-4 of the blocks and fewer).
+//
+//   * a work unit is (row tile of up to 40 grouped token rows of one expert) x (256 weight rows, as two halves of
 //     128: gate and up rows of the same 128 features, or 256 rows of a plain matrix); units are dealt to one
 //     persistent CTA per SM;
 //   * along K the unit is a run of records of 128 columns: 2 x 8192 bytes of codes and 2 x 512 bytes of scales,
 //     contiguous in memory, moved with ONE bulk copy each; a second bulk copy brings the same columns of the token
-//     rows' image.  A ring of 6 to 11 such stages keeps 100-190 KB per SM in flight;
+//     rows' image.  A ring of 6 (40 rows a tile) to 12 (3 rows) such stages keeps 105-210 KB of weights per SM in flight;
 //   * the MMA warp copies the record's scales to tensor memory (tcgen05.cp) and issues two K=64 MMAs per half;
 //   * eight epilogue warps add up the digits' accumulators, add the bias and either apply the gated activation and
-//     write the result as digits again (a warp's 32 lanes are the 32 features of one block), in the image the down
-//     projection reads, or (plain matrix) store fp32 output rows.  Up to 22 rows the accumulators are doubled and
-//     the epilogue of one unit runs under the MMAs of the next.
+//     write the result as digits again (a warp's 32 lanes are the 32 features of one block), in the images the down
+//     projection reads, or (plain matrix) store fp32 output rows.  Accumulators of even units grow from the bottom of
+//     tensor memory, those of odd units from the top: the epilogue of one unit runs under the MMAs of the next unless
+//     the two need more than 480 columns together (gate/up: two tiles of 22 rows fit; down: of 18).
 //
 // The producer asks for weights before griddepcontrol.wait: the tile list comes from a kernel two launches back.
 //
@@ -43,9 +51,8 @@
 
 namespace csk {
 
-constexpr int kMxDigits = 5;
-constexpr int kMxTileRows = 48;                    // token rows of a row tile: 5 * 48 = 240 <= 256 MMA columns
-constexpr int kMxMaxN = kMxDigits * kMxTileRows;
+constexpr int kMxDigitsX = 5, kMxDigitsA = 6;      // digits of a token row, of an activated row
+constexpr int kMxTileRows = 40;                    // token rows of a row tile: 6 * 40 = 240 MMA columns, twice in tensor memory
 constexpr int kMxRecBlocks = 4;                    // 32-column blocks per record
 constexpr int kMxSfAtom = 512;                     // scales of 128 rows x 4 blocks: [row % 32][row / 32][block]
 constexpr int kMxARecMax = kMxRecBlocks * 256 * 16 + 2 * kMxSfAtom;
@@ -92,29 +99,32 @@ inline MxLayout make_mx_layout(int N, int K, bool paired) {
   return L;
 }
 
-// The image of a row tile of `rows` token rows (5 * rows MMA columns, padded to a multiple of 16): per record
-// [scale atoms][4 blocks x npad x 16 bytes of codes]; column 5 r + p is digit p of row r.  Tiles lie one after the
+// The image of a row tile of `rows` rows of n digits (n * rows MMA columns, padded to a multiple of 16): per record
+// [scale atoms][4 blocks x npad x 16 bytes of codes]; column n r + p is digit p of row r.  Tiles lie one after the
 // other in row order; `col0` and `atom0` bound what the tiles before this one take.
 struct MxTileImage {
   int npad, atoms;
   size_t offset;      // of the tile's image
   size_t rec_stride;
 };
-__host__ __device__ inline int mx_npad(int rows) { return (kMxDigits * rows + 15) / 16 * 16; }
+template <int D>
+__host__ __device__ inline int mx_npad(int rows) { return (D * rows + 15) / 16 * 16; }
+template <int D>
 __host__ __device__ inline MxTileImage mx_tile_image(int tile, int row0, int rows, int recs) {
   MxTileImage t;
-  t.npad = mx_npad(rows);
+  t.npad = mx_npad<D>(rows);
   t.atoms = t.npad > 128 ? 2 : 1;
-  const size_t col0 = (size_t)kMxDigits * row0 + 16 * (size_t)tile;
-  const size_t atom0 = (size_t)kMxDigits * row0 / 128 + 2 * (size_t)tile;
+  const size_t col0 = (size_t)D * row0 + 16 * (size_t)tile;
+  const size_t atom0 = (size_t)D * row0 / 128 + 2 * (size_t)tile;
   t.offset = (size_t)recs * (col0 * (kMxRecBlocks * 16) + atom0 * kMxSfAtom);
   t.rec_stride = (size_t)t.atoms * kMxSfAtom + (size_t)t.npad * (kMxRecBlocks * 16);
   return t;
 }
-inline size_t mx_image_bytes(size_t rows, size_t tiles, int recs) {
-  return (size_t)recs * ((kMxDigits * rows + 16 * tiles) * (kMxRecBlocks * 16) +
-                         (kMxDigits * rows / 128 + 2 * tiles + 2) * kMxSfAtom);
+inline size_t mx_image_bytes(int digits, size_t rows, size_t tiles, int recs) {
+  return (size_t)recs * ((digits * rows + 16 * tiles) * (kMxRecBlocks * 16) + (digits * rows / 128 + 2 * tiles + 2) * kMxSfAtom);
 }
+// Words of a row tile's record mask (a bit per record: some row's block in it is wide).
+__host__ __device__ inline int mx_mask_words(int recs) { return (recs + 31) / 32; }
 __device__ __forceinline__ size_t mx_sf_pos(int n, int kb) {  // column n's scale of block kb inside a record's atoms
   return (size_t)(n >> 7) * kMxSfAtom + (n & 31) * 16 + ((n & 127) >> 5) * 4 + (kb & 3);
 }
@@ -214,41 +224,78 @@ __device__ __forceinline__ uint32_t mx_digit(float& a, float& b) {
   b = (b - f.y) * 8.0f;
   return d;
 }
-// A whole block by one thread: digit p's 32 codes in d[p].
-__device__ __forceinline__ uint32_t mx_encode_block(float (&v)[32], uint32_t (&d)[kMxDigits][4]) {
-  uint32_t amax = 0;
+// Clip and limit of the test for wide blocks.  With values in units of 2^e, digits leave an rms of 0.15 * 8^(1-n) of
+// each, fp16 2.07e-4 of each value: over any set of values whose rms is at least kappa = 0.15 * 8^(1-n) / 2.07e-4 (0.177 for
+// five digits, 0.0221 for six) the digits are the better operand.  The sum over the block of min(v^2, clip^2) loses at most
+// t clip^2 with any t of the values, so a sum of t clip^2 + (32 - t) kappa^2 leaves rms kappa for the rest.  Clip and t:
+// five digits 1/2 and 8 (2 + 0.752), six 1/8 and 4 (0.0625 + 0.0137); rounded up.
+template <int D>
+__host__ __device__ constexpr float mx_wide_clip2() { return D == kMxDigitsX ? 0.25f : 1.0f / 64.0f; }
+template <int D>
+__host__ __device__ constexpr float mx_wide_limit() { return D == kMxDigitsX ? 2.76f : 0.077f; }
+__host__ __device__ constexpr uint32_t mx_rest_shift(int digits) { return 3u * (uint32_t)digits; }  // the digits' scale over that of the digits after them
+
+// A block by four neighbouring lanes, eight values each: `d` the digits (a word of digit p's codes), `rest` the digits
+// after them (zeros unless the block is wide), the scale byte.  All lanes of the warp call it.
+struct MxEncoded {
+  uint32_t d[kMxDigitsX], rest[kMxDigitsX], sf;
+  bool wide;
+};
+__device__ __forceinline__ void mx_digits(float (&v)[8], uint32_t (&d)[kMxDigitsX]) {
 #pragma unroll
-  for (int i = 0; i < 32; ++i) amax = max(amax, __float_as_uint(v[i]) & 0x7FFFFFFFu);
-  float inv;
-  const uint32_t sf = mx_scale_of(amax, inv);
+  for (int p = 0; p < kMxDigitsX; ++p) {
+    d[p] = 0;
 #pragma unroll
-  for (int i = 0; i < 32; ++i) v[i] *= inv;
-#pragma unroll
-  for (int p = 0; p < kMxDigits; ++p)
-#pragma unroll
-    for (int w = 0; w < 4; ++w) {
-      uint32_t x = 0;
-#pragma unroll
-      for (int q = 0; q < 4; ++q) x |= mx_digit(v[8 * w + 2 * q], v[8 * w + 2 * q + 1]) << (8 * q);
-      d[p][w] = x;
-    }
-  return sf;
-}
-__device__ __forceinline__ void mx_store_block(uint8_t* image, const MxTileImage& g, int r, int kb, const uint32_t (&d)[kMxDigits][4],
-                                               uint32_t sf) {
-  uint8_t* rec = image + g.offset + (size_t)(kb / kMxRecBlocks) * g.rec_stride;
-#pragma unroll
-  for (int p = 0; p < kMxDigits; ++p) {
-    const int n = kMxDigits * r + p;
-    *reinterpret_cast<uint4*>(rec + g.atoms * kMxSfAtom + ((size_t)(kb & 3) * g.npad + n) * 16) =
-        make_uint4(d[p][0], d[p][1], d[p][2], d[p][3]);
-    rec[mx_sf_pos(n, kb)] = (uint8_t)sf;
+    for (int q = 0; q < 4; ++q) d[p] |= mx_digit(v[2 * q], v[2 * q + 1]) << (8 * q);
   }
 }
-// Columns past K inside the last pair of blocks: the weights' codes are zero there, so any scale but NaN will do.
-__device__ __forceinline__ void mx_store_pad(uint8_t* image, const MxTileImage& g, int r, int kb) {
+__device__ __forceinline__ MxEncoded mx_encode_block(float (&v)[8]) {
+  MxEncoded e;
+  uint32_t amax = 0;
+#pragma unroll
+  for (int i = 0; i < 8; ++i) amax = max(amax, __float_as_uint(v[i]) & 0x7FFFFFFFu);
+  amax = max(amax, __shfl_xor_sync(0xffffffffu, amax, 1));
+  amax = max(amax, __shfl_xor_sync(0xffffffffu, amax, 2));
+  float inv, q = 0.f;
+  e.sf = mx_scale_of(amax, inv);
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    v[i] *= inv;
+    q += fminf(v[i] * v[i], mx_wide_clip2<kMxDigitsX>());
+  }
+  q += __shfl_xor_sync(0xffffffffu, q, 1);  // (both sums are the same in every lane of the four)
+  q += __shfl_xor_sync(0xffffffffu, q, 2);
+  mx_digits(v, e.d);
+  e.wide = q < mx_wide_limit<kMxDigitsX>() && e.sf >= mx_rest_shift(kMxDigitsX) && e.sf != 255u;
+#pragma unroll
+  for (int p = 0; p < kMxDigitsX; ++p) e.rest[p] = 0;
+  if (e.wide) mx_digits(v, e.rest);
+  uint32_t left = 0;
+#pragma unroll
+  for (int p = 0; p < kMxDigitsX; ++p) left |= e.rest[p];
+  // a power of two among zeros: nothing is left (sign bits alone are digits of zero too)
+  e.wide = __ballot_sync(0xffffffffu, (left & 0x77777777u) != 0) >> (threadIdx.x & 28) & 0xFu;
+  return e;
+}
+// The four lanes' words of the digits to their columns of row r (word q = lane & 3 of each 16 bytes); the scale bytes
+// unless sf < 0: zeros are zero under any scale but NaN, and the second image never holds that.
+__device__ __forceinline__ void mx_store_block(uint8_t* image, const MxTileImage& g, int r, int kb, int q, const uint32_t (&d)[kMxDigitsX],
+                                               int sf) {
   uint8_t* rec = image + g.offset + (size_t)(kb / kMxRecBlocks) * g.rec_stride;
-  for (int p = 0; p < kMxDigits; ++p) rec[mx_sf_pos(kMxDigits * r + p, kb)] = 0;
+  const int n = kMxDigitsX * r;
+  uint8_t* codes = rec + g.atoms * kMxSfAtom + ((size_t)(kb & 3) * g.npad + n) * 16 + 4 * q;
+#pragma unroll
+  for (int p = 0; p < kMxDigitsX; ++p) *reinterpret_cast<uint32_t*>(codes + 16 * p) = d[p];
+  if (sf >= 0)
+    for (int p = q; p < kMxDigitsX; p += 4) rec[mx_sf_pos(n + p, kb)] = (uint8_t)sf;
+}
+// Columns past K inside the last pair of blocks: the weights' codes are zero there, so any scale but NaN will do.
+__device__ __forceinline__ void mx_store_pad(uint8_t* image, const MxTileImage& g, int r, int kb, int q) {
+  uint8_t* rec = image + g.offset + (size_t)(kb / kMxRecBlocks) * g.rec_stride;
+  for (int p = q; p < kMxDigitsX; p += 4) rec[mx_sf_pos(kMxDigitsX * r + p, kb)] = 0;
+}
+__device__ __forceinline__ void mx_mark_wide(uint32_t* tile_mask, int kb) {
+  atomicOr(tile_mask + kb / (32 * kMxRecBlocks), 1u << (kb / kMxRecBlocks & 31));
 }
 
 struct MxQuantArgs {
@@ -260,112 +307,113 @@ struct MxQuantArgs {
   int* row_of_pair;          // [T*k]
   const RowTile* tiles;
   const int* n_tiles_ptr;
-  uint8_t* image;
+  uint8_t *image, *rest;     // digits, and the digits after them
+  uint32_t* wide;            // record masks of the row tiles, wide_stride words each
+  int wide_stride;
   int T, H, E, k, e_begin, e_count, only_expert, max_rows, weight_before_ffn, blocks, recs;
 };
-// Token rows to digits, into the images of the row tiles they were placed in.  One CTA per token, one thread per
+// Token rows to digits, into the images of the row tiles they were placed in.  One CTA per token, four threads per
 // 32-column block: a token is encoded once and stored k times (with the routing weight applied before the expert
-// it is encoded per pair).  Bound by the latency of one thread's chain (about 900 instructions) for a few tokens.
-__global__ void __launch_bounds__(128) k_mx_quant(const MxQuantArgs A) {
+// it is encoded per pair).  Bound for a few tokens by its chain of dependent loads (8.8 us for one token of 2880 columns under
+// the profiler's cold caches; with one thread per block and the wide blocks' test 12.0; 333 tokens 14.8 and 20.0).
+constexpr int kMxQuantThreads = 384;  // 96 blocks at once
+__global__ void __launch_bounds__(kMxQuantThreads) k_mx_quant(const MxQuantArgs A) {
   __shared__ MxTileImage s_img[16];
-  __shared__ int s_r[16];
+  __shared__ int s_r[16], s_tile[16];
   __shared__ float s_w[16];
-  const int t = blockIdx.x, kbs = A.H / 32;
-  float v[32];
-  uint32_t d[kMxDigits][4], sf = 0;
-  auto load = [&](int kb) {
-    const float4* src = reinterpret_cast<const float4*>(A.hidden + (size_t)t * A.H + kb * 32);
-#pragma unroll
-    for (int i = 0; i < 8; ++i) {
-      const float4 x = __ldg(src + i);
-      v[4 * i] = x.x;
-      v[4 * i + 1] = x.y;
-      v[4 * i + 2] = x.z;
-      v[4 * i + 3] = x.w;
-    }
+  const int t = blockIdx.x, kbs = A.H / 32, q = threadIdx.x & 3, kb0 = threadIdx.x >> 2, step = blockDim.x >> 2;
+  float v[8];
+  MxEncoded e;
+  auto load = [&](int kb, float w) {  // the eight values of this thread times w (zeros past the row)
+    const float4* src = reinterpret_cast<const float4*>(A.hidden + (size_t)t * A.H + kb * 32 + q * 8);
+    const float4 x = kb < kbs ? __ldg(src) : make_float4(0.f, 0.f, 0.f, 0.f), y = kb < kbs ? __ldg(src + 1) : x;
+    v[0] = x.x * w, v[1] = x.y * w, v[2] = x.z * w, v[3] = x.w * w;
+    v[4] = y.x * w, v[5] = y.y * w, v[6] = y.z * w, v[7] = y.w * w;
   };
   // the hidden states are older than the kernel before this one: encode while it is still placing rows
-  const bool early = !A.weight_before_ffn && (int)threadIdx.x < kbs;
-  if (early) {
-    load(threadIdx.x);
-    sf = mx_encode_block(v, d);
+  if (!A.weight_before_ffn) {
+    load(kb0, 1.f);
+    e = mx_encode_block(v);
   }
   griddep_wait();
   griddep_launch();
   if ((int)threadIdx.x < A.k) {
     const int j = threadIdx.x, pair = t * A.k + j;
-    const int e = (int)A.router[2 * (size_t)pair];
-    const bool mine = e >= 0 && e < A.E && (A.only_expert < 0 || e == A.only_expert);
+    const int x = (int)A.router[2 * (size_t)pair];
+    const bool mine = x >= 0 && x < A.E && (A.only_expert < 0 || x == A.only_expert);
     int pos = -1;
     if (A.cursor) {
-      if (mine) pos = A.offsets[e] + atomicAdd(&A.cursor[e], 1);
+      if (mine) pos = A.offsets[x] + atomicAdd(&A.cursor[x], 1);
       if (pos >= A.max_rows) pos = -1;
       A.row_of_pair[pair] = pos;
     } else {
       pos = A.row_of_pair[pair];
     }
     s_r[j] = -1;
-    if (pos >= 0 && mine && e >= A.e_begin && e < A.e_begin + A.e_count && *A.n_tiles_ptr > 0) {
-      const ExpertTiles et = A.et[e];
-      const int r = pos - A.offsets[e], tile = et.tile0 + r / et.height;
+    if (pos >= 0 && mine && x >= A.e_begin && x < A.e_begin + A.e_count && *A.n_tiles_ptr > 0) {
+      const ExpertTiles et = A.et[x];
+      const int r = pos - A.offsets[x], tile = et.tile0 + r / et.height;
       const RowTile rt = A.tiles[tile];
-      s_img[j] = mx_tile_image(tile, rt.row0, rt.rows, A.recs);
+      s_img[j] = mx_tile_image<kMxDigitsX>(tile, rt.row0, rt.rows, A.recs);
+      s_tile[j] = tile;
       s_r[j] = r % et.height;
       s_w[j] = A.router[2 * (size_t)pair + 1];
     }
   }
   __syncthreads();
-  for (int kb = threadIdx.x; kb < A.blocks; kb += blockDim.x) {
-    if (kb < kbs && !A.weight_before_ffn && kb != (int)threadIdx.x) {
-      load(kb);
-      sf = mx_encode_block(v, d);
+  // (whole warps: the lanes of a block past the row's end take part in the exchanges)
+  for (int base = 0; base < A.blocks; base += step) {
+    const int kb = base + kb0;
+    if (base && !A.weight_before_ffn) {
+      load(kb, 1.f);
+      e = mx_encode_block(v);
     }
     for (int j = 0; j < A.k; ++j) {
       if (s_r[j] < 0) continue;
+      if (A.weight_before_ffn) {
+        load(kb, s_w[j]);
+        e = mx_encode_block(v);
+      }
       if (kb >= kbs) {
-        mx_store_pad(A.image, s_img[j], s_r[j], kb);
+        if (kb < A.blocks) mx_store_pad(A.image, s_img[j], s_r[j], kb, q);
         continue;
       }
-      if (A.weight_before_ffn) {
-        load(kb);
-#pragma unroll
-        for (int i = 0; i < 32; ++i) v[i] *= s_w[j];
-        sf = mx_encode_block(v, d);
-      }
-      mx_store_block(A.image, s_img[j], s_r[j], kb, d, sf);
+      mx_store_block(A.image, s_img[j], s_r[j], kb, q, e.d, (int)e.sf);
+      mx_store_block(A.rest, s_img[j], s_r[j], kb, q, e.rest, e.wide ? (int)(e.sf - mx_rest_shift(kMxDigitsX)) : -1);
+      if (e.wide && q == 0) mx_mark_wide(A.wide + (size_t)s_tile[j] * A.wide_stride, kb);
     }
   }
 }
 // The same from grouped fp16 rows (the expert-parallel receive side): a CTA per row tile.
 __global__ void __launch_bounds__(128) k_mx_quant_rows(const __half* __restrict__ x16, int ldx, const RowTile* __restrict__ tiles,
                                                        const int* __restrict__ n_tiles_ptr, uint8_t* __restrict__ image,
+                                                       uint8_t* __restrict__ rest_image, uint32_t* __restrict__ wide_masks, int wide_stride,
                                                        int K, int blocks, int recs) {
-  const int n_tiles = *n_tiles_ptr, kbs = K / 32;
+  const int n_tiles = *n_tiles_ptr, kbs = K / 32, q = threadIdx.x & 3;
   for (int tile = blockIdx.x; tile < n_tiles; tile += gridDim.x) {
     const RowTile rt = tiles[tile];
-    const MxTileImage g = mx_tile_image(tile, rt.row0, rt.rows, recs);
-    for (int i = threadIdx.x; i < rt.rows * blocks; i += blockDim.x) {
+    const MxTileImage g = mx_tile_image<kMxDigitsX>(tile, rt.row0, rt.rows, recs);
+    for (int base = 0; base < rt.rows * blocks; base += blockDim.x >> 2) {
+      const int i = base + (threadIdx.x >> 2);
       const int r = i / blocks, kb = i % blocks;
-      if (kb >= kbs) {
-        mx_store_pad(image, g, r, kb);
-        continue;
-      }
-      const uint4* src = reinterpret_cast<const uint4*>(x16 + (size_t)(rt.row0 + r) * ldx + kb * 32);
-      float v[32];
-      uint32_t d[kMxDigits][4];
+      const bool real = i < rt.rows * blocks && kb < kbs;
+      float v[8];
+      const uint4 x = real ? *reinterpret_cast<const uint4*>(x16 + (size_t)(rt.row0 + r) * ldx + kb * 32 + q * 8) : make_uint4(0, 0, 0, 0);
+      const uint32_t w[4] = {x.x, x.y, x.z, x.w};
 #pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        const uint4 x = src[q];
-        const uint32_t w[4] = {x.x, x.y, x.z, x.w};
-#pragma unroll
-        for (int c = 0; c < 4; ++c) {
-          const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&w[c]));
-          v[8 * q + 2 * c] = f.x;
-          v[8 * q + 2 * c + 1] = f.y;
-        }
+      for (int c = 0; c < 4; ++c) {
+        const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&w[c]));
+        v[2 * c] = f.x;
+        v[2 * c + 1] = f.y;
       }
-      const uint32_t sf = mx_encode_block(v, d);
-      mx_store_block(image, g, r, kb, d, sf);
+      const MxEncoded e = mx_encode_block(v);
+      if (real) {
+        mx_store_block(image, g, r, kb, q, e.d, (int)e.sf);
+        mx_store_block(rest_image, g, r, kb, q, e.rest, e.wide ? (int)(e.sf - mx_rest_shift(kMxDigitsX)) : -1);
+        if (e.wide && q == 0) mx_mark_wide(wide_masks + (size_t)tile * wide_stride, kb);
+      } else if (i < rt.rows * blocks) {
+        mx_store_pad(image, g, r, kb, q);
+      }
     }
   }
 }
@@ -375,9 +423,12 @@ struct MxArgs {
   const uint8_t* weights;
   size_t expert_stride, mat_offset, bias_offset;
   MxLayout L;
-  const uint8_t* x_img;   // token rows' image, L.recs records
-  uint8_t* a_img;         // GATED: the activated rows' image for the down projection ...
-  int a_blocks, a_recs;   // ... and its blocks and records
+  const uint8_t *x_img, *x_rest;  // the operand rows' images (digits, the digits after them), L.recs records
+  const uint32_t* x_wide;         // record masks, wide_stride words per row tile
+  uint8_t *a_img, *a_rest;        // GATED: the activated rows' images for the down projection ...
+  uint32_t* a_wide;
+  int a_blocks, a_recs;           // ... and its blocks and records
+  int wide_stride;
   float* y;               // !GATED: output rows [rows, ldy]
   int ldy;
   const RowTile* tiles;
@@ -386,25 +437,37 @@ struct MxArgs {
   int has_bias, act, F;
 };
 
+template <int D>
 __device__ __forceinline__ float mx_sum(const uint32_t* d) {  // the digits' accumulators, radix 8
-  float v = __uint_as_float(d[kMxDigits - 1]);
+  float v = __uint_as_float(d[D - 1]);
 #pragma unroll
-  for (int p = kMxDigits - 2; p >= 0; --p) v = fmaf(v, 0.125f, __uint_as_float(d[p]));
+  for (int p = D - 2; p >= 0; --p) v = fmaf(v, 0.125f, __uint_as_float(d[p]));
   return v;
 }
-__device__ __forceinline__ void mx_ld40(uint32_t taddr, uint32_t (&r)[40]) {
+// Eight rows' accumulators.  With a tile's last group of rows this reads up to 32 columns past the tile's own (of the other
+// accumulators, or of the scales: not used).
+template <int D>
+__device__ __forceinline__ void mx_ld_group(uint32_t taddr, uint32_t (&r)[8 * D]) {
   tmem_ld32(taddr, *reinterpret_cast<uint32_t(*)[32]>(&r[0]));
-  tmem_ld8(taddr + 32, *reinterpret_cast<uint32_t(*)[8]>(&r[32]));
+  if constexpr (D == 5) tmem_ld8(taddr + 32, *reinterpret_cast<uint32_t(*)[8]>(&r[32]));
+  else tmem_ld16(taddr + 32, *reinterpret_cast<uint32_t(*)[16]>(&r[32]));
+}
+
+// Is any record of the unit's row tile marked as holding wide blocks?  (After the kernel that writes the masks.)
+__device__ __forceinline__ uint32_t mx_any_wide(const MxArgs& A, int tile) {
+  uint32_t any = 0;
+  for (int w = 0; w < mx_mask_words(A.L.recs); ++w) any |= __ldcg(A.x_wide + (size_t)tile * A.wide_stride + w);
+  return any;
 }
 
 template <bool GATED>
 __global__ void __launch_bounds__(kMxThreads, 1) k_mx(const MxArgs A) {
   extern __shared__ __align__(128) uint8_t mx_smem[];
   const MxLayout& L = A.L;
-  // How many columns the launch's tallest row tile takes decides the stage size and whether two accumulator pairs fit:
-  // the tile list knows (meta[4]), the host does not.
-  const int n_max = mx_npad(max(1, A.meta[4]));
-  const uint32_t n_acc = 4 * n_max <= (int)kMxTmemSf ? 2u : 1u;
+  constexpr int D = GATED ? kMxDigitsX : kMxDigitsA;
+  // How many columns the launch's tallest row tile takes decides the stage size: the tile list knows (meta[4]), the host
+  // does not.
+  const int n_max = mx_npad<D>(max(1, A.meta[4]));
   const int stage_bytes = kMxARecMax + (n_max > 128 ? 2 : 1) * kMxSfAtom + (n_max * kMxRecBlocks * 16 + 127) / 128 * 128;
   const int NS = min(kMxMaxStages, (kMxSmem - kMxCtrl - kMxSlack) / stage_bytes);
   uint8_t* ctrl = mx_smem + kMxSmem - kMxCtrl;
@@ -460,52 +523,58 @@ __global__ void __launch_bounds__(kMxThreads, 1) k_mx(const MxArgs A) {
                       (size_t)rec * L.rec_bytes(nt, kMxRecBlocks),
                   bytes, bar_full(s));
       };
-      auto rows = [&](const MxTileImage& g, int rec, int s) {
-        bulk_load(smem_base + (uint32_t)s * stage_bytes + kMxARecMax, A.x_img + g.offset + (size_t)rec * g.rec_stride,
+      auto rows = [&](const uint8_t* image, const MxTileImage& g, int rec, int s) {
+        bulk_load(smem_base + (uint32_t)s * stage_bytes + kMxARecMax, image + g.offset + (size_t)rec * g.rec_stride,
                   (uint32_t)(g.atoms * kMxSfAtom + L.rec_blocks(rec) * g.npad * 16), bar_full(s));
       };
-      // as many records of the first units as the ring holds are requested before the rows' image is complete
+      // as many records of the first unit as the ring holds are requested before the rows' images are complete
       int first = 0;
-      for (int pass = 0; pass < 2; ++pass) {
-        first = 0;
-        for (int item = blockIdx.x; first < NS && item < n; item += gridDim.x) {
-          const int tile = item / L.n_units, nt = item % L.n_units;
-          const RowTile rt = A.tiles[tile];
-          const MxTileImage g = mx_tile_image(tile, rt.row0, rt.rows, L.recs);
-          for (int rec = 0; rec < L.recs && first < NS; ++rec, ++first) {
-            if (pass == 0) weights(rt, nt, g, rec, first);
-            else rows(g, rec, first);
-          }
-        }
-        if (pass == 0) {
-          griddep_wait();
-          asm volatile("fence.proxy.async.global;" ::: "memory");  // the image was written by ordinary stores
-        }
+      if ((int)blockIdx.x < n) {
+        const int tile = blockIdx.x / L.n_units, nt = blockIdx.x % L.n_units;
+        const RowTile rt = A.tiles[tile];
+        const MxTileImage g = mx_tile_image<D>(tile, rt.row0, rt.rows, L.recs);
+        for (; first < NS && first < L.recs; ++first) weights(rt, nt, g, first, first);
+        griddep_wait();
+        asm volatile("fence.proxy.async.global;" ::: "memory");  // the images were written by ordinary stores
+        for (int rec = 0; rec < first; ++rec) rows(A.x_img, g, rec, rec);
       }
-      int s = 0, skip = first, issued = first;
-      uint32_t ph = 0;
+      int s = first == NS ? 0 : first, issued = first;
+      uint32_t ph = first == NS ? 0u : 1u;  // a stage's first use waits for nothing
       for (int item = blockIdx.x; ok && item < n; item += gridDim.x) {
-        if (skip >= L.recs) {
-          skip -= L.recs;
-          continue;
-        }
         const int tile = item / L.n_units, nt = item % L.n_units;
         const RowTile rt = A.tiles[tile];
-        const MxTileImage g = mx_tile_image(tile, rt.row0, rt.rows, L.recs);
-        for (int rec = skip; rec < L.recs; ++rec) {
+        const MxTileImage g = mx_tile_image<D>(tile, rt.row0, rt.rows, L.recs);
+        for (int rec = first; rec < L.recs; ++rec) {
           if (!mbar_wait(bar_empty(s), ph, abort_flag)) {
             ok = false;
             break;
           }
           weights(rt, nt, g, rec, s);
-          rows(g, rec, s);
+          rows(A.x_img, g, rec, s);
           ++issued;
           if (++s == NS) {
             s = 0;
             ph ^= 1u;
           }
         }
-        skip = 0;
+        first = 0;
+        if (ok && mx_any_wide(A, tile)) {  // the records with wide blocks once more
+          for (int w = 0; ok && w < mx_mask_words(L.recs); ++w)
+            for (uint32_t bits = __ldcg(A.x_wide + (size_t)tile * A.wide_stride + w); bits; bits &= bits - 1) {
+              const int rec = 32 * w + __ffs((int)bits) - 1;
+              if (!mbar_wait(bar_empty(s), ph, abort_flag)) {
+                ok = false;
+                break;
+              }
+              weights(rt, nt, g, rec, s);
+              rows(A.x_rest, g, rec, s);
+              ++issued;
+              if (++s == NS) {
+                s = 0;
+                ph ^= 1u;
+              }
+            }
+        }
       }
       if (!ok) {
         // let the copies still in flight land before the CTA goes away
@@ -526,50 +595,83 @@ __global__ void __launch_bounds__(kMxThreads, 1) k_mx(const MxArgs A) {
     bool ok = true;
     griddep_wait();  // this kernel's successor may count on everything before this kernel's predecessor being complete
     griddep_launch();
+    int npad_before = 0, ahead_rows = 0;
+    uint32_t ahead_wide = 0;
     for (long item = blockIdx.x; ok && item < n_items; item += gridDim.x, ++it) {
       const int tile = (int)(item / L.n_units), nt = (int)(item % L.n_units);
-      const int rows = A.tiles[tile].rows;
-      const int npad = mx_npad(rows), atoms = npad > 128 ? 2 : 1;
+      if (!(it & 31u)) {
+        // what it needs to know of the next 32 units, one per lane (with a load in front of every unit, 16 tokens of the
+        // 128-expert 2048 x 768 layer took 81.8 us instead of 79.8)
+        const long ahead = item + (long)lane * gridDim.x;
+        if (ahead < n_items) {
+          ahead_rows = A.tiles[ahead / L.n_units].rows;
+          ahead_wide = mx_any_wide(A, (int)(ahead / L.n_units));
+        }
+      }
+      const int rows = __shfl_sync(0xffffffffu, ahead_rows, (int)(it & 31u));
+      const uint32_t any_wide = __shfl_sync(0xffffffffu, ahead_wide, (int)(it & 31u));
+      const int npad = mx_npad<D>(rows), atoms = npad > 128 ? 2 : 1;
       const int r0 = L.rows(nt, 0), r1 = L.rows(nt, 1), halves = L.halves(nt);
-      const uint32_t buf = n_acc == 2u ? it & 1u : 0u;
-      const uint32_t use = n_acc == 2u ? it >> 1 : it;
-      const uint32_t d0 = tb + buf * 2u * (uint32_t)n_max, d1 = d0 + (uint32_t)n_max;
+      const uint32_t buf = it & 1u, use = it >> 1;
+      const uint32_t d0 = tb + (buf ? kMxTmemSf - 2u * (uint32_t)npad : 0u), d1 = d0 + (uint32_t)npad;
       ok = __all_sync(0xffffffffu, mbar_wait(bar_acc_empty(buf), (use & 1u) ^ 1u, abort_flag));
+      if (ok && it && npad_before + npad > (int)kMxTmemSf / 2)  // the unit before this one lies in the way
+        ok = __all_sync(0xffffffffu, mbar_wait(bar_acc_empty(buf ^ 1u), ((it - 1u) >> 1) & 1u, abort_flag));
       if (!ok) break;
+      npad_before = npad;
       tc_fence_after();
-      for (int rec = 0; rec < L.recs; ++rec, ++c) {
-        ok = __all_sync(0xffffffffu, mbar_wait(bar_full(s), ph, abort_flag));
-        if (!ok) break;
-        tc_fence_after();
+      // the MMAs of the record in stage s (`add` 0: the accumulators start here), by the elected lane
+      auto issue = [&](int rec, uint32_t add) {
         const int nb = L.rec_blocks(rec);
         const uint32_t a = smem_base + (uint32_t)s * stage_bytes, b = a + kMxARecMax;
         const uint32_t sf = tb + kMxTmemSf + (c & 1u) * 16u;
         const uint32_t a_sf = a + (uint32_t)(nb * (r0 + r1) * 16), b_codes = b + (uint32_t)(atoms * kMxSfAtom);
-        if (elect_one()) {
-          tmem_cp_scales(sf, umma_desc_plain(a_sf, 128, 128));
-          if (halves > 1) tmem_cp_scales(sf + 4, umma_desc_plain(a_sf + kMxSfAtom, 128, 128));
-          tmem_cp_scales(sf + 8, umma_desc_plain(b, 128, 128));
-          if (atoms > 1) tmem_cp_scales(sf + 12, umma_desc_plain(b + kMxSfAtom, 128, 128));
+        tmem_cp_scales(sf, umma_desc_plain(a_sf, 128, 128));
+        if (halves > 1) tmem_cp_scales(sf + 4, umma_desc_plain(a_sf + kMxSfAtom, 128, 128));
+        tmem_cp_scales(sf + 8, umma_desc_plain(b, 128, 128));
+        if (atoms > 1) tmem_cp_scales(sf + 12, umma_desc_plain(b + kMxSfAtom, 128, 128));
 #pragma unroll
-          for (int p = 0; p < 2; ++p) {
-            if (2 * p < nb) {
-              const uint32_t idesc = umma_idesc_mxf4(npad, 2 * p);
-              const uint64_t db = umma_desc_plain(b_codes + (uint32_t)(2 * p * npad * 16), (uint32_t)(npad * 16), 128);
-              const uint32_t ap = a + (uint32_t)(p * 32 * (r0 + r1));
-              umma_mxf4_ss(d0, umma_desc_plain(ap, (uint32_t)(r0 * 16), 128), db, idesc, sf, sf + 8, (rec | p) ? 1u : 0u);
-              if (halves > 1)
-                umma_mxf4_ss(d1, umma_desc_plain(ap + (uint32_t)(r0 * 32), (uint32_t)(r1 * 16), 128), db, idesc, sf + 4, sf + 8,
-                             (rec | p) ? 1u : 0u);
-            }
+        for (int p = 0; p < 2; ++p) {
+          if (2 * p < nb) {
+            const uint32_t idesc = umma_idesc_mxf4(npad, 2 * p);
+            const uint64_t db = umma_desc_plain(b_codes + (uint32_t)(2 * p * npad * 16), (uint32_t)(npad * 16), 128);
+            const uint32_t ap = a + (uint32_t)(p * 32 * (r0 + r1));
+            umma_mxf4_ss(d0, umma_desc_plain(ap, (uint32_t)(r0 * 16), 128), db, idesc, sf, sf + 8, p ? 1u : add);
+            if (halves > 1)
+              umma_mxf4_ss(d1, umma_desc_plain(ap + (uint32_t)(r0 * 32), (uint32_t)(r1 * 16), 128), db, idesc, sf + 4, sf + 8, p ? 1u : add);
           }
-          umma_commit(bar_empty(s));
-          if (rec == L.recs - 1) umma_commit(bar_acc_full(buf));
+        }
+        umma_commit(bar_empty(s));
+      };
+      for (int rec = 0; rec < L.recs; ++rec, ++c) {
+        ok = __all_sync(0xffffffffu, mbar_wait(bar_full(s), ph, abort_flag));
+        if (!ok) break;
+        tc_fence_after();
+        if (elect_one()) {
+          issue(rec, rec ? 1u : 0u);
+          if (rec == L.recs - 1 && !any_wide) umma_commit(bar_acc_full(buf));
         }
         __syncwarp();
         if (++s == NS) {
           s = 0;
           ph ^= 1u;
         }
+      }
+      if (any_wide) {  // the records with wide blocks once more
+        for (int w = 0; ok && w < mx_mask_words(L.recs); ++w)
+          for (uint32_t bits = __ldcg(A.x_wide + (size_t)tile * A.wide_stride + w); bits; bits &= bits - 1, ++c) {
+            ok = __all_sync(0xffffffffu, mbar_wait(bar_full(s), ph, abort_flag));
+            if (!ok) break;
+            tc_fence_after();
+            if (elect_one()) issue(32 * w + __ffs((int)bits) - 1, 1u);
+            __syncwarp();
+            if (++s == NS) {
+              s = 0;
+              ph ^= 1u;
+            }
+          }
+        if (ok && elect_one()) umma_commit(bar_acc_full(buf));
+        __syncwarp();
       }
     }
     // everything issued has to retire before tensor memory is freed
@@ -590,9 +692,9 @@ __global__ void __launch_bounds__(kMxThreads, 1) k_mx(const MxArgs A) {
       const RowTile rt = A.tiles[tile];
       const int halves = L.halves(nt);
       const float* bias = reinterpret_cast<const float*>(A.weights + (size_t)rt.expert * A.expert_stride + A.bias_offset);
-      const uint32_t buf = n_acc == 2u ? it & 1u : 0u;
-      const uint32_t use = n_acc == 2u ? it >> 1 : it;
-      const uint32_t t_acc = tmem_base + ((uint32_t)(quarter * 32) << 16) + buf * 2u * (uint32_t)n_max;
+      const uint32_t buf = it & 1u, use = it >> 1;
+      const uint32_t npad = (uint32_t)mx_npad<D>(rt.rows);
+      const uint32_t t_acc = tmem_base + ((uint32_t)(quarter * 32) << 16) + (buf ? kMxTmemSf - 2u * npad : 0u);
       const int groups = (rt.rows + 7) >> 3;
       const int n = (GATED ? nt * 128 : nt * 256) + quarter * 32 + lane;
       float b0 = 0.f, b1 = 0.f;
@@ -611,13 +713,39 @@ __global__ void __launch_bounds__(kMxThreads, 1) k_mx(const MxArgs A) {
       tc_fence_after();
       if (GATED) {
         const bool live = nt * 128 + quarter * 32 < L.N;  // N is a multiple of 32: a warp's features are real or not as one
-        const MxTileImage g = mx_tile_image(tile, rt.row0, rt.rows, A.a_recs);
+        constexpr int DA = kMxDigitsA;
+        const MxTileImage g = mx_tile_image<DA>(tile, rt.row0, rt.rows, A.a_recs);
         const int kb = nt * 4 + quarter;
-        uint8_t* rec = A.a_img + g.offset + (size_t)(kb / kMxRecBlocks) * g.rec_stride;
+        const size_t rec_at = g.offset + (size_t)(kb / kMxRecBlocks) * g.rec_stride;
+        uint8_t *rec = A.a_img + rec_at, *rest = A.a_rest + rec_at;
+        const size_t codes_at = g.atoms * kMxSfAtom + (size_t)(kb & 3) * g.npad * 16;
+        const bool odd = lane & 1;
+        // neighbouring lanes hold neighbouring columns: the even one packs the even row's bytes, the odd one the odd row's
+        auto pack = [&](uint32_t w) {
+          const uint32_t o = __shfl_xor_sync(0xffffffffu, w, 1);
+          return odd ? ((o >> 4) & 0x0F0F0F0Fu) | (w & 0xF0F0F0F0u) : (w & 0x0F0F0F0Fu) | ((o & 0x0F0F0F0Fu) << 4);
+        };
+        // the next six digits of two rows, into the columns of row `to` (nothing when it is past the tile)
+        auto digits = [&](float (&v)[2], uint8_t* codes, int to) {
+          uint32_t w = 0, w2 = 0;  // byte p: digit p of both rows (low nibble: the even one)
+#pragma unroll
+          for (int p = 0; p < 4; ++p) w |= mx_digit(v[0], v[1]) << (8 * p);
+#pragma unroll
+          for (int p = 0; p < DA - 4; ++p) w2 |= mx_digit(v[0], v[1]) << (8 * p);
+          w = pack(w);
+          w2 = pack(w2);
+          if (to < rt.rows) {
+            uint8_t* dst = codes + (size_t)DA * to * 16 + (lane >> 1);
+#pragma unroll
+            for (int p = 0; p < 4; ++p) dst[16 * p] = (uint8_t)(w >> (8 * p));
+#pragma unroll
+            for (int p = 0; p < DA - 4; ++p) dst[16 * (4 + p)] = (uint8_t)(w2 >> (8 * p));
+          }
+        };
         for (int gr = grp; gr < groups; gr += 2) {
-          uint32_t rg[40], ru[40];
-          mx_ld40(t_acc + (uint32_t)gr * 40, rg);
-          mx_ld40(t_acc + (uint32_t)n_max + (uint32_t)gr * 40, ru);
+          uint32_t rg[8 * D], ru[8 * D];
+          mx_ld_group<D>(t_acc + (uint32_t)gr * 8 * D, rg);
+          mx_ld_group<D>(t_acc + npad + (uint32_t)gr * 8 * D, ru);
           tmem_ld_wait();
           if (!live) continue;
 #pragma unroll
@@ -626,48 +754,51 @@ __global__ void __launch_bounds__(kMxThreads, 1) k_mx(const MxArgs A) {
             if (r >= rt.rows) break;
             float v[2];
             uint32_t sf[2];
+            bool wide[2];
 #pragma unroll
             for (int j = 0; j < 2; ++j) {
-              v[j] = gated_act(mx_sum(rg + 5 * (i + j)) + b0, mx_sum(ru + 5 * (i + j)) + b1, A.act);
+              v[j] = gated_act(mx_sum<D>(rg + D * (i + j)) + b0, mx_sum<D>(ru + D * (i + j)) + b1, A.act);
               float inv;
               sf[j] = mx_scale_of(__reduce_max_sync(0xffffffffu, __float_as_uint(v[j]) & 0x7FFFFFFFu), inv);
               v[j] *= inv;
+              constexpr float kFixed = 1048576.f;  // the sum in fixed point: one instruction over the warp
+              const uint32_t q = (uint32_t)(fminf(v[j] * v[j], mx_wide_clip2<DA>()) * kFixed);
+              wide[j] = __reduce_add_sync(0xffffffffu, q) < (uint32_t)(mx_wide_limit<DA>() * kFixed) && r + j < rt.rows &&
+                        sf[j] >= mx_rest_shift(DA) && sf[j] != 255u;
             }
-            uint32_t w = 0, w4;  // byte p: digit p of both rows (low nibble: the even one)
-#pragma unroll
-            for (int p = 0; p < 4; ++p) w |= mx_digit(v[0], v[1]) << (8 * p);
-            w4 = mx_digit(v[0], v[1]);
-            // neighbouring lanes hold neighbouring columns: the even one packs the even row's bytes, the odd one the odd row's
-            const uint32_t o = __shfl_xor_sync(0xffffffffu, w, 1), o4 = __shfl_xor_sync(0xffffffffu, w4, 1);
-            const bool odd = lane & 1;
-            w = odd ? ((o >> 4) & 0x0F0F0F0Fu) | (w & 0xF0F0F0F0u) : (w & 0x0F0F0F0Fu) | ((o & 0x0F0F0F0Fu) << 4);
-            w4 = odd ? (o4 >> 4) | (w4 & 0xF0u) : (w4 & 0x0Fu) | ((o4 & 0x0Fu) << 4);
             const int my = r + (odd ? 1 : 0);
-            if (my < rt.rows) {
-              uint8_t* dst = rec + g.atoms * kMxSfAtom + ((size_t)(kb & 3) * g.npad + kMxDigits * my) * 16 + (lane >> 1);
+            digits(v, rec + codes_at, my);
+            if (my < rt.rows && lane < 2 * DA) {
+              const int col = DA * my + (lane >> 1);
+              rec[mx_sf_pos(col, kb)] = (uint8_t)(odd ? sf[1] : sf[0]);
+              if (kb + 1 < A.a_blocks && (kb + 1) * 32 >= A.F) rec[mx_sf_pos(col, kb + 1)] = 0;  // the padding block
+            }
 #pragma unroll
-              for (int p = 0; p < 4; ++p) dst[16 * p] = (uint8_t)(w >> (8 * p));
-              dst[64] = (uint8_t)w4;
-              if (lane < 2 * kMxDigits) {
-                const int col = kMxDigits * my + (lane >> 1);
-                rec[mx_sf_pos(col, kb)] = (uint8_t)(odd ? sf[1] : sf[0]);
-                if (kb + 1 < A.a_blocks && (kb + 1) * 32 >= A.F) rec[mx_sf_pos(col, kb + 1)] = 0;  // the padding block
-              }
+            for (int j = 0; j < 2; ++j)  // a power of two, zeros: nothing is left
+              wide[j] = wide[j] && __ballot_sync(0xffffffffu, (__float_as_uint(v[j]) & 0x7FFFFFFFu) != 0) != 0;
+            if (lane < 2 * DA && r + lane / DA < rt.rows)
+              *reinterpret_cast<uint4*>(rest + codes_at + (size_t)(DA * r + lane) * 16) = make_uint4(0, 0, 0, 0);
+            if (wide[0] || wide[1]) {
+              const bool mine = odd ? wide[1] : wide[0];
+              __syncwarp();
+              digits(v, rest + codes_at, mine ? my : rt.rows);
+              if (mine && lane < 2 * DA) rest[mx_sf_pos(DA * my + (lane >> 1), kb)] = (uint8_t)((odd ? sf[1] : sf[0]) - mx_rest_shift(DA));
+              if (lane == 0) mx_mark_wide(A.a_wide + (size_t)tile * A.wide_stride, kb);
             }
           }
         }
       } else {
         for (int w = grp; w < halves * groups; w += 2) {
           const int half = w >= groups ? 1 : 0, gr = w - half * groups;
-          uint32_t rd[40];
-          mx_ld40(t_acc + (uint32_t)(half * n_max) + (uint32_t)gr * 40, rd);
+          uint32_t rd[8 * D];
+          mx_ld_group<D>(t_acc + (half ? npad : 0u) + (uint32_t)gr * 8 * D, rd);
           tmem_ld_wait();
           const int col = n + 128 * half;
           if (col >= L.N) continue;
           float* out = A.y + (size_t)(rt.row0 + gr * 8) * A.ldy + col;
 #pragma unroll
           for (int i = 0; i < 8; ++i)
-            if (gr * 8 + i < rt.rows) out[(size_t)i * A.ldy] = mx_sum(rd + 5 * i) + (half ? b1 : b0);
+            if (gr * 8 + i < rt.rows) out[(size_t)i * A.ldy] = mx_sum<D>(rd + D * i) + (half ? b1 : b0);
         }
       }
       tc_fence_before();

@@ -3,7 +3,7 @@ padding end, against the CPU restatement of the reference."""
 import numpy as np
 import pytest
 
-from coalsack_b200 import MoeLayer, PATH_STREAM, synth
+from coalsack_b200 import MoeLayer, PATH_STREAM, PATH_TILE, synth
 from tests import cases
 
 pytestmark = pytest.mark.gpu
@@ -16,11 +16,16 @@ MX_MAX, MX_MEAN = 2e-3, 3e-4
 @pytest.mark.parametrize("E,k,H,F,T,bias,act,wbf", [
     (2, 1, 32, 32, 1, False, 0, False),      # one block: half of the K = 64 step is padding, 32 of 128 rows exist
     (2, 2, 96, 160, 3, True, 1, False),      # odd block counts either way; 15 of 16 columns
-    (1, 1, 128, 128, 48, True, 0, False),    # one full tile (240 columns), one whole record
+    (1, 1, 128, 128, 48, True, 0, False),    # two even tiles, one whole record
+    (1, 1, 128, 128, 40, False, 1, False),   # one full tile (200 and 240 columns)
     (1, 1, 160, 384, 49, True, 0, True),     # two even tiles; second half of a plain unit absent; routing weight first
-    (1, 1, 256, 288, 22, False, 0, False),   # the last height with two accumulator pairs ...
-    (1, 1, 256, 288, 23, False, 1, False),   # ... and the first with one
+    (1, 1, 256, 288, 18, False, 0, False),   # the last height at which two units' accumulators fit in the down projection ...
+    (1, 1, 256, 288, 19, False, 1, False),   # ... and the first at which they do not
+    (1, 1, 256, 288, 22, False, 0, False),   # the same of gate/up ...
+    (1, 1, 256, 288, 23, False, 1, False),   # ... and its first without
+    (2, 1, 64, 4224, 60, False, 1, False),   # more than 32 records of activated rows: two mask words
     (3, 2, 288, 352, 145, True, 0, False),   # several tiles per expert, uneven loads
+    (32, 2, 1536, 1536, 320, True, 0, False),  # several units per CTA, of tiles that do and that do not fit beside each other
     (4, 2, 2080, 1056, 65, True, 1, False),  # more records than ring stages
     (2, 1, 4128, 32, 5, False, 0, False),    # more than 128 blocks per row
 ])
@@ -97,3 +102,90 @@ def test_received_rows_without_images_take_the_tensor_core_kernel(gpu_lib, port)
         assert np.array_equal(ro[..., 0], want_ro[..., 0])
         mx, mr = cases.err_stats(out, want)
         assert mx <= cases.MAX_ABS_OVER_RMS and mr <= cases.MEAN_REL, (mx, mr)
+
+
+# ---- operand precision where a few values of a block are far above the others -----------------------------------------
+E2M1 = np.array([0, .5, 1, 1.5, 2, 3, 4, 6, 0, -.5, -1, -1.5, -2, -3, -4, -6])
+
+
+def _values(blocks, rows, cols):
+    """The numbers of an MXFP4 matrix in 64 bits."""
+    b = np.asarray(blocks).reshape(rows, cols // 32, 17)
+    codes = np.concatenate([b[:, :, 1:] & 15, b[:, :, 1:] >> 4], axis=2)
+    return (E2M1[codes] * 2.0 ** (b[:, :, :1].astype(np.float64) - 127)).reshape(rows, cols)
+
+
+def _zero_columns(blocks, rows, cols, which):
+    b = np.asarray(blocks).reshape(rows, cols // 32, 17).copy()
+    for c in which:
+        j = c % 32
+        b[:, c // 32, 1 + j % 16] &= 0xF0 if j < 16 else 0x0F
+    return b.reshape(-1)
+
+
+def _mlp64(h, ex, H, F, act):
+    up, gate, down = (_values(ex[n][0], *s) for n, s in (("w_up", (F, H)), ("w_gate", (F, H)), ("w_down", (H, F))))
+    u, g = h.astype(np.float64) @ up.T + ex["b_up"][0], h.astype(np.float64) @ gate.T + ex["b_gate"][0]
+    if act == 0:
+        g, u = np.minimum(g, 7), np.clip(u, -7, 7)
+        a = g / (1 + np.exp(np.minimum(-1.702 * g, 700))) * (u + 1)
+    else:
+        a = g / (1 + np.exp(-g)) * u
+    return a @ down.T + ex["b_down"][0]
+
+
+@pytest.mark.parametrize("times", [1, 30, 100, 1000, 10000])
+@pytest.mark.parametrize("where", ["dense", "unread", "activated"])
+def test_outliers_lose_no_precision(gpu_lib, where, times):
+    """Token rows with a few channels `times` above the others -- whose weights are ordinary, or zero, so that the others
+    decide -- and a few activated features above the others that the down projection does not read: the result is no
+    further from the 64-bit value than that of the kernel with fp16 operands (2e-6: fp32 sums of 1600 products)."""
+    H, F, T, act = 1600, 480, 50, 1 if where == "activated" else 0
+    sh = synth.tiny(seed=371, E=1, k=1, H=H, F=F, T=T, has_bias=True, act=act)
+    h, Wg, rb, ex = cases.layer_inputs(sh)
+    rng = np.random.default_rng(times)
+    ex["w_gate"], ex["w_up"] = ([_scaled(w[0], -4)] for w in (ex["w_gate"], ex["w_up"]))
+    if where == "activated":  # a handful of features at about `times` the others' values, their down columns zero
+        big = rng.choice(F, 5, replace=False)
+        ex["b_gate"][0][big], ex["b_up"][0][big] = 6.0, 0.5 * times
+        ex["w_down"][0] = _zero_columns(ex["w_down"][0], H, F, big)
+    else:
+        big = rng.choice(H, 9, replace=False)
+        h[:, big] = np.float32(times) * (1 + 0.1 * rng.standard_normal((T, 9))).astype(np.float32)
+        if times > 1:
+            h[:, big[0]] = times  # (an fp16 operand holds this one exactly)
+        for n in ("w_gate", "w_up"):
+            if where == "unread":
+                ex[n][0] = _zero_columns(ex[n][0], F, H, big)
+    want = _mlp64(h, ex, H, F, act)
+    err = {}
+    lay = MoeLayer.from_shape(sh)
+    lay.set_router(Wg, rb)
+    lay.load_experts(ex)
+    route = np.zeros((T, 1, 2), np.float32)
+    route[..., 1] = 1
+    for name, path in (("fp16", PATH_TILE), ("digits", PATH_STREAM)):
+        lay.set_path(path)
+        out, _ = lay.forward(h, router_out=route)
+        err[name] = np.linalg.norm(out - want) / np.linalg.norm(want)
+        again, _ = lay.forward(h, router_out=route)
+        assert np.array_equal(out, again)
+    print(f"{where} x{times}: relative error fp16 operands {err['fp16']:.2e}, digits {err['digits']:.2e}")
+    assert err["digits"] <= err["fp16"] + 2e-6, err
+    # rows without outliers beside rows with them: the same bits as without
+    if where != "activated":
+        plain = synth.hidden_states(sh)
+        alone, _ = lay.forward(plain, router_out=route)
+        mixed = plain.copy()
+        mixed[::3] = h[::3]
+        both, _ = lay.forward(mixed, router_out=route)
+        keep = np.arange(T) % 3 != 0
+        assert np.array_equal(both[keep], alone[keep])
+    lay.close()
+
+
+def _scaled(blocks, by):
+    """The matrix times 2^by."""
+    b = np.asarray(blocks).reshape(-1, 17).copy()
+    b[:, 0] = b[:, 0].astype(int) + by
+    return b.reshape(-1)
