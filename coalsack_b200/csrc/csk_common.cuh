@@ -38,6 +38,14 @@ __device__ __forceinline__ void dequant_word(uint32_t w, uint32_t (&h)[4]) {
       : "r"(w));
 }
 
+// x limited to [-lim, lim]; a NaN stays one, as the reference's comparisons leave it (fminf and fmaxf would make it a limit,
+// and a row that holds an infinity or a NaN would come out finite).
+__device__ __forceinline__ float limit_keep_nan(float x, float lim) {
+  float r;
+  asm("{\n\t.reg .f32 t;\n\tmax.NaN.f32 t, %1, %2;\n\tmin.NaN.f32 %0, t, %3;\n\t}" : "=f"(r) : "f"(x), "f"(-lim), "f"(lim));
+  return r;
+}
+
 // The same activations with the hardware's approximate exp2 and reciprocal (one MUFU
 // operation each, relative error around 2^-22, far below the fp16 rounding of the stored
 // result).  Used in the tensor-core kernel's epilogue, which sits on the critical path.
@@ -56,7 +64,7 @@ __device__ __forceinline__ float gated_act_fast(float gate, float up, int act) {
   if (act == CSK_ACT_MODIFIED_SWIGLU) {
     const float lim = 7.0f, alpha = 1.702f;
     const float g = fminf(gate, lim);
-    const float u = fminf(fmaxf(up, -lim), lim);
+    const float u = limit_keep_nan(up, lim);
     return g * rcp_approx(1.0f + ex2_approx(-alpha * kLog2e * g)) * (u + 1.0f);
   }
   return gate * rcp_approx(1.0f + ex2_approx(-kLog2e * gate)) * up;
@@ -67,7 +75,7 @@ __device__ __forceinline__ float gated_act(float gate, float up, int act) {
   if (act == CSK_ACT_MODIFIED_SWIGLU) {
     const float lim = 7.0f, alpha = 1.702f;
     float g = fminf(gate, lim);
-    float u = fminf(fmaxf(up, -lim), lim);
+    float u = limit_keep_nan(up, lim);
     float glu = g / (1.0f + expf(alpha * (-g)));
     return glu * (u + 1.0f);
   }

@@ -3,7 +3,7 @@ padding end, against the CPU restatement of the reference."""
 import numpy as np
 import pytest
 
-from coalsack_b200 import MoeLayer, PATH_STREAM, PATH_TILE, synth
+from coalsack_b200 import MoeLayer, PATH_STREAM, PATH_TILE, PATH_TILE_PAIR, synth
 from tests import cases
 
 pytestmark = pytest.mark.gpu
@@ -189,3 +189,28 @@ def _scaled(blocks, by):
     b = np.asarray(blocks).reshape(-1, 17).copy()
     b[:, 0] = b[:, 0].astype(int) + by
     return b.reshape(-1)
+
+
+@pytest.mark.parametrize("act", [0, 1])
+@pytest.mark.parametrize("path", [PATH_STREAM, PATH_TILE, PATH_TILE_PAIR])
+@pytest.mark.parametrize("bad", [np.inf, -np.inf, np.nan])
+def test_a_row_that_is_not_finite_does_not_come_out_finite(gpu_lib, port, act, path, bad):
+    """With the routing given by the caller nothing before the experts looks at the row: where the restatement's result is
+    not finite, neither is the kernels' (the clamped activation keeps a NaN of the up projection), and no other row changes."""
+    sh = synth.tiny(seed=361, E=2, k=1, H=160, F=96, T=9, has_bias=True, act=act)
+    h, Wg, rb, ex = cases.layer_inputs(sh)
+    lay = MoeLayer.from_shape(sh)
+    lay.set_router(Wg, rb)
+    lay.load_experts(ex)
+    lay.set_path(path)
+    route = np.ones((sh.tokens, 1, 2), np.float32)
+    route[:, 0, 0] = np.arange(sh.tokens) % 2
+    good, _ = lay.forward(h, router_out=route)
+    h[4, 77] = bad
+    out, _ = lay.forward(h, router_out=route)
+    want, _ = port.moe_layer(h, Wg, rb, ex, 1, act, router_out=route)
+    assert not np.isfinite(want[4]).any()
+    assert not np.isfinite(out[4]).any()
+    keep = np.arange(sh.tokens) != 4
+    assert np.array_equal(out[keep], good[keep])
+    lay.close()
