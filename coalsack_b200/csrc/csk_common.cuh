@@ -120,14 +120,19 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatil
   if (mbar_try(bar, parity)) return true;
   const long long t0 = clock64();
   for (;;) {
+    if (*abort_flag) return false;
     for (int i = 0; i < 32; ++i)
       if (mbar_try(bar, parity)) return true;
-    if (*abort_flag) return false;
     if (clock64() - t0 > wait_budget()) {
       *abort_flag = 1;
       return false;
     }
   }
+}
+// The same for a whole warp that goes on to warp-wide instructions: its lanes agree on whether the wait ran out (each lane
+// reads the clock and the flag for itself).
+__device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, volatile int* abort_flag) {
+  return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag));
 }
 __device__ __forceinline__ void bulk_load(uint32_t dst, const void* src, uint32_t bytes, uint32_t bar) {
   asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst),

@@ -69,7 +69,8 @@ struct csk_moe_layer {
   float** d_peer_back = nullptr;      // [world]
   std::vector<void*> ipc_opened;      // peer mappings to close
   bool pdl = false;  // launch the layer's kernels with programmatic dependent launch (small batches)
-  bool debug_stall = false;  // test hook: the next tensor-core launch's copy role issues nothing (one shot)
+  bool debug_stall = false;  // test hooks: the next expert (router) launch's copy role issues nothing (one shot)
+  bool debug_stall_router = false;
 
   float* d_norm_w = nullptr;   // [H] weight of the RMSNorm in front of the router (csk_moe_set_ffn_norm)
   float* d_normed = nullptr;   // [max_T,H] its output
@@ -247,6 +248,8 @@ int launch_router(csk_moe_layer* L, const float* d_hidden, int64_t T, float* d_r
     f.T = (int)T;
     f.H = L->H;
     f.E = L->E_router;
+    f.stall = L->debug_stall_router;
+    L->debug_stall_router = false;
     const int token_tiles = ceil_div((int)T, kRtTokens), rg = rt_groups(L->E_router);
     // one CTA fits an SM: as many parts of the hidden dimension as one wave holds
     int parts = std::min(std::min(rt_blocks(L->H), kFastMaxParts), std::max(1, L->sm_count / (token_tiles * rg)));
@@ -428,7 +431,10 @@ void launch_mx_pair(csk_moe_layer* L, float* y, int ldy, cudaStream_t s, StageTi
   a.wide_stride = wide_stride(L);
   a.a_blocks = L->Ld.blocks;
   a.a_recs = L->Ld.recs;
+  a.stall = L->debug_stall;
+  L->debug_stall = false;
   launch_k(k_mx<true>, dim3(L->sm_count), dim3(kMxThreads), kMxSmem, s, L->pdl, a);
+  a.stall = 0;
   tm.mark();
   // down
   a.mat_offset = L->off_d;
@@ -1333,7 +1339,7 @@ int csk_moe_forward_dev(csk_moe_layer* L, const float* d_hidden, int64_t T, cons
   CSK_CUDA(L, cudaSetDevice(L->cfg.device));
   cudaStream_t s = pick(L, stream);
   constexpr int64_t kGraphMaxTokens = 512;
-  if (!L->use_graphs || L->timing || L->debug_stall || T > kGraphMaxTokens || T <= 0 || T > L->max_T)
+  if (!L->use_graphs || L->timing || L->debug_stall || L->debug_stall_router || T > kGraphMaxTokens || T <= 0 || T > L->max_T)
     return forward_dev(L, d_hidden, T, d_router_in, d_router_out, d_out, -1, s, false);
   for (auto& g : L->graphs)
     if (g.T == T && g.hidden == d_hidden && g.router_in == d_router_in && g.router_out == d_router_out &&
@@ -2156,6 +2162,10 @@ int csk_moe_debug_set(csk_moe_layer* L, int32_t key, int64_t value) {
   }
   if (key == CSK_DEBUG_STALL_TILE_PRODUCER) {
     L->debug_stall = value != 0;
+    return CSK_OK;
+  }
+  if (key == CSK_DEBUG_STALL_ROUTER) {
+    L->debug_stall_router = value != 0;
     return CSK_OK;
   }
   return fail(L, CSK_ERR_INVALID, "debug: unknown key %d", key);

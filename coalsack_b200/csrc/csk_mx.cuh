@@ -435,6 +435,7 @@ struct MxArgs {
   const int* n_tiles_ptr;
   int* meta;              // meta[3] = device status word
   int has_bias, act, F;
+  int stall;              // test hook: the copy role issues nothing, every wait of the other roles runs out
 };
 
 template <int D>
@@ -511,7 +512,7 @@ __global__ void __launch_bounds__(kMxThreads, 1) k_mx(const MxArgs A) {
   if (warp == 0) {
     // ------------------------------ producer ------------------------------
     if (lane == 0) {
-      const int n = (int)n_items;
+      const int n = A.stall ? 0 : (int)n_items;
       bool ok = true;
       // a stage's weights, and (separately) its token rows; both count on the stage's barrier
       auto weights = [&](const RowTile& rt, int nt, const MxTileImage& g, int rec, int s) {
@@ -614,9 +615,9 @@ __global__ void __launch_bounds__(kMxThreads, 1) k_mx(const MxArgs A) {
       const int r0 = L.rows(nt, 0), r1 = L.rows(nt, 1), halves = L.halves(nt);
       const uint32_t buf = it & 1u, use = it >> 1;
       const uint32_t d0 = tb + (buf ? kMxTmemSf - 2u * (uint32_t)npad : 0u), d1 = d0 + (uint32_t)npad;
-      ok = __all_sync(0xffffffffu, mbar_wait(bar_acc_empty(buf), (use & 1u) ^ 1u, abort_flag));
+      ok = mbar_wait_warp(bar_acc_empty(buf), (use & 1u) ^ 1u, abort_flag);
       if (ok && it && npad_before + npad > (int)kMxTmemSf / 2)  // the unit before this one lies in the way
-        ok = __all_sync(0xffffffffu, mbar_wait(bar_acc_empty(buf ^ 1u), ((it - 1u) >> 1) & 1u, abort_flag));
+        ok = mbar_wait_warp(bar_acc_empty(buf ^ 1u), ((it - 1u) >> 1) & 1u, abort_flag);
       if (!ok) break;
       npad_before = npad;
       tc_fence_after();
@@ -644,7 +645,7 @@ __global__ void __launch_bounds__(kMxThreads, 1) k_mx(const MxArgs A) {
         umma_commit(bar_empty(s));
       };
       for (int rec = 0; rec < L.recs; ++rec, ++c) {
-        ok = __all_sync(0xffffffffu, mbar_wait(bar_full(s), ph, abort_flag));
+        ok = mbar_wait_warp(bar_full(s), ph, abort_flag);
         if (!ok) break;
         tc_fence_after();
         if (elect_one()) {
@@ -660,7 +661,7 @@ __global__ void __launch_bounds__(kMxThreads, 1) k_mx(const MxArgs A) {
       if (any_wide) {  // the records with wide blocks once more
         for (int w = 0; ok && w < mx_mask_words(L.recs); ++w)
           for (uint32_t bits = __ldcg(A.x_wide + (size_t)tile * A.wide_stride + w); bits; bits &= bits - 1, ++c) {
-            ok = __all_sync(0xffffffffu, mbar_wait(bar_full(s), ph, abort_flag));
+            ok = mbar_wait_warp(bar_full(s), ph, abort_flag);
             if (!ok) break;
             tc_fence_after();
             if (elect_one()) issue(32 * w + __ffs((int)bits) - 1, 1u);
@@ -709,7 +710,7 @@ __global__ void __launch_bounds__(kMxThreads, 1) k_mx(const MxArgs A) {
           if (n + 128 < L.N) b1 = bias[2 * A.F + n + 128];
         }
       }
-      if (!mbar_wait(bar_acc_full(buf), use & 1u, abort_flag)) break;
+      if (!mbar_wait_warp(bar_acc_full(buf), use & 1u, abort_flag)) break;
       tc_fence_after();
       if (GATED) {
         const bool live = nt * 128 + quarter * 32 < L.N;  // N is a multiple of 32: a warp's features are real or not as one

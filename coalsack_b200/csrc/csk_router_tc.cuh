@@ -139,6 +139,7 @@ struct RouterTcArgs {
   float* hn2;             // [T][parts]: the part's share of n^2
   int* status;
   int T, H, E;
+  int stall;              // test hook: the copy role issues nothing, every wait of the other roles runs out
 };
 
 __global__ void __launch_bounds__(kRtThreads, 1) k_router_tc(const RouterTcArgs A) {
@@ -190,7 +191,7 @@ __global__ void __launch_bounds__(kRtThreads, 1) k_router_tc(const RouterTcArgs 
     // ------------------------------ producer ------------------------------
     if (lane == 0) {
       int issued = 0;
-      for (int i = 0; i < n; ++i) {
+      for (int i = 0; i < (A.stall ? 0 : n); ++i) {
         const int s = i % kRtStages;
         if (i >= kRtStages && !mbar_wait(bar_empty(s), (uint32_t)((i / kRtStages - 1) & 1), abort_flag)) break;
         mbar_expect_tx(bar_w(s), kRtWBytes);
@@ -211,9 +212,9 @@ __global__ void __launch_bounds__(kRtThreads, 1) k_router_tc(const RouterTcArgs 
     bool ok = true;
     for (int i = 0; i < n; ++i) {
       const int s = i % kRtStages, buf = i & 1;
-      ok = __all_sync(0xffffffffu, mbar_wait(bar_acc_empty(buf), (uint32_t)((i >> 1) & 1) ^ 1u, abort_flag)) &&
-           __all_sync(0xffffffffu, mbar_wait(bar_w(s), (uint32_t)((i / kRtStages) & 1), abort_flag)) &&
-           __all_sync(0xffffffffu, mbar_wait(bar_x(s), (uint32_t)((i / kRtStages) & 1), abort_flag));
+      ok = mbar_wait_warp(bar_acc_empty(buf), (uint32_t)((i >> 1) & 1) ^ 1u, abort_flag) &&
+           mbar_wait_warp(bar_w(s), (uint32_t)((i / kRtStages) & 1), abort_flag) &&
+           mbar_wait_warp(bar_x(s), (uint32_t)((i / kRtStages) & 1), abort_flag);
       if (!ok) break;
       tc_fence_after();
       const uint32_t st = smem_base + (uint32_t)s * kRtStageBytes;
@@ -276,7 +277,9 @@ __global__ void __launch_bounds__(kRtThreads, 1) k_router_tc(const RouterTcArgs 
       if (q == 0) h2 = fmaf(__uint_as_float(amax), __uint_as_float(amax), h2);
       float inv;
       const float scale = rt_scale_of(amax, inv);
-      if (i >= kRtStages && !mbar_wait(bar_empty(s), (uint32_t)((i / kRtStages - 1) & 1), abort_flag)) return false;
+      // (a wait that ran out must not part the lanes in front of the shuffles: they go on, every further wait ends at once
+      // and nobody uses the digits)
+      if (i >= kRtStages) mbar_wait(bar_empty(s), (uint32_t)((i / kRtStages - 1) & 1), abort_flag);
       uint8_t* out = smem + (size_t)s * kRtStageBytes + kRtWBytes;
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
@@ -293,12 +296,13 @@ __global__ void __launch_bounds__(kRtThreads, 1) k_router_tc(const RouterTcArgs 
       asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
       __syncwarp();
       if (lane == 0) mbar_arrive(bar_x(s));
-      return true;
     };
     if (n > 0) load(0, next[0]);
     if (n > 1) load(1, next[1]);
-    for (int i = 0; i < n; i += 2)
-      if (!step(i, next[0]) || (i + 1 < n && !step(i + 1, next[1]))) break;
+    for (int i = 0; i < n; i += 2) {
+      step(i, next[0]);
+      if (i + 1 < n) step(i + 1, next[1]);
+    }
     __syncwarp();
     h2 += __shfl_xor_sync(0xffffffffu, h2, 1);
     h2 += __shfl_xor_sync(0xffffffffu, h2, 2);
@@ -316,7 +320,7 @@ __global__ void __launch_bounds__(kRtThreads, 1) k_router_tc(const RouterTcArgs 
     for (int i = 0; i < n; ++i) {
       const int buf = i & 1;
       const float sw = __ldg(ws + (size_t)i * kRtExperts);
-      ok = __all_sync(0xffffffffu, mbar_wait(bar_acc_full(buf), (uint32_t)((i >> 1) & 1), abort_flag));
+      ok = mbar_wait_warp(bar_acc_full(buf), (uint32_t)((i >> 1) & 1), abort_flag);
       if (!ok) break;
       tc_fence_after();
       const uint32_t acc = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)buf * 192u + (uint32_t)tok;

@@ -384,12 +384,12 @@ k_tile(const __grid_constant__ TileMaps maps, const TileArgs A) {
         const RowTile rt = A.tiles[item / L.n_tiles];
         const int n_mma = max(16, (rt.rows + 15) & ~15);
         const uint32_t idesc = umma_idesc_f16(n_mma);
-        ok = __all_sync(0xffffffffu, mbar_wait(bar_tmem_empty, (it & 1u) ^ 1u, abort_flag));
+        ok = mbar_wait_warp(bar_tmem_empty, (it & 1u) ^ 1u, abort_flag);
         if (!ok) break;
         tc_fence_after();
         for (int kt = 0; kt < KT; ++kt, ++c) {
           const uint32_t s = c % NR, sa = c % NA;
-          ok = __all_sync(0xffffffffu, mbar_wait(bar_full_a(sa), (c / NA) & 1u, abort_flag));
+          ok = mbar_wait_warp(bar_full_a(sa), (c / NA) & 1u, abort_flag);
           if (!ok) break;
           tc_fence_after();
           const uint64_t db = db0 + (uint64_t)((s * (uint32_t)RAW) >> 4);  // start-address field, 16-byte units
@@ -464,6 +464,10 @@ k_tile(const __grid_constant__ TileMaps maps, const TileArgs A) {
       const int halves = L.halves((int)(item % L.n_tiles));
       const int* emeta = reinterpret_cast<const int*>(A.weights + (size_t)rt.expert * A.expert_stride + A.meta_offset);
       const int emax = emeta[A.meta_slot];
+      // A wait that ran out in some lanes must not part them in front of the warp-wide stores: all of them go through the
+      // unit's remaining k-steps (the flag ends every further wait at once, nobody uses the tile) and agree afterwards.
+      // A vote per k-step costs 1 to 2 % of the kernel.
+      bool landed = true;
       for (int kt = 0; kt < KT; ++kt, ++c) {
         if ((int)(c & 1) != grp) continue;
         const int s = (int)(c % NR);
@@ -473,25 +477,16 @@ k_tile(const __grid_constant__ TileMaps maps, const TileArgs A) {
           // fill complete: were that fill still in flight (copies may complete out of order), the parity test
           // below would take the fill before it for the one awaited, and the conversion would read the
           // wrong k-step.  The stage's previous MMAs having retired implies its previous fill has landed.
-          if (!mbar_wait(bar_retired(s), (uint32_t)(((c - NR) / NR) & 1), abort_flag)) {
-            ok = false;
-            break;
-          }
+          landed = mbar_wait(bar_retired(s), (uint32_t)(((c - NR) / NR) & 1), abort_flag) && landed;
         }
-        if (!mbar_wait(bar_full_raw(s), ph, abort_flag)) {
-          ok = false;
-          break;
-        }
+        landed = mbar_wait(bar_full_raw(s), ph, abort_flag) && landed;
         const uint8_t* packed = smem + (size_t)s * RAW + kTileABytes;
         const int sa = (int)(c % NA);
         const uint32_t t_slot = tmem_base + ((uint32_t)(quarter * 32) << 16) + kTmemABase + (uint32_t)sa * 64;
         uint32_t h[2][16];
         convert(packed, emax, h);
         // the slot was last read by k-step c - NA
-        if (c >= NA && !mbar_wait(bar_retired((int)((c - NA) % NR)), (uint32_t)(((c - NA) / NR) & 1), abort_flag)) {
-          ok = false;
-          break;
-        }
+        if (c >= NA) landed = mbar_wait(bar_retired((int)((c - NA) % NR)), (uint32_t)(((c - NA) / NR) & 1), abort_flag) && landed;
         tc_fence_after();
         tmem_st16(t_slot, h[0]);
         tmem_st16(t_slot + 16, h[1]);
@@ -511,6 +506,7 @@ k_tile(const __grid_constant__ TileMaps maps, const TileArgs A) {
         __syncwarp();
         if (lane == 0) mbar_arrive(bar_full_a(sa));
       }
+      ok = __all_sync(0xffffffffu, landed);
     }
   } else {
     // ------------------------------ epilogue ------------------------------
@@ -534,7 +530,7 @@ k_tile(const __grid_constant__ TileMaps maps, const TileArgs A) {
       const float* bias = reinterpret_cast<const float*>(ebase + A.bias_offset);
       const int emax = reinterpret_cast<const int*>(ebase + A.meta_offset)[A.meta_slot];
       const float oscale = W16 ? 1.0f : ldexpf(1.0f, emax - 140);
-      if (!mbar_wait(bar_tmem_full, (uint32_t)(it & 1), abort_flag)) {
+      if (!mbar_wait_warp(bar_tmem_full, (uint32_t)(it & 1), abort_flag)) {
         ok = false;
         break;
       }

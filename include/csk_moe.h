@@ -417,11 +417,13 @@ int csk_moe_get_counters(csk_moe_layer* layer, int64_t* rows_per_expert, int64_t
  *   CSK_DEBUG_WAIT_BUDGET         clock cycles a device-side wait may take before it
  *                                 gives up (default 2e9, about a second); applies to
  *                                 every handle on the device
- *   CSK_DEBUG_STALL_TILE_PRODUCER non-zero: in the NEXT tensor-core expert launch the
- *                                 copy role issues nothing, so every other role's wait
- *                                 runs out, the kernel tears down and the call reports
- *                                 CSK_ERR_DEVICE (one shot) */
-enum { CSK_DEBUG_WAIT_BUDGET = 0, CSK_DEBUG_STALL_TILE_PRODUCER = 1 };
+ *   CSK_DEBUG_STALL_TILE_PRODUCER non-zero: in the NEXT expert launch (any of the three
+ *                                 kernels) the copy role issues nothing, so every other
+ *                                 role's wait runs out, the kernel tears down and the call
+ *                                 reports CSK_ERR_DEVICE (one shot)
+ *   CSK_DEBUG_STALL_ROUTER        the same in the NEXT tensor-core router launch (large
+ *                                 batches in certified mode) */
+enum { CSK_DEBUG_WAIT_BUDGET = 0, CSK_DEBUG_STALL_TILE_PRODUCER = 1, CSK_DEBUG_STALL_ROUTER = 2 };
 int csk_moe_debug_set(csk_moe_layer* layer, int32_t key, int64_t value);
 
 #ifdef __cplusplus

@@ -214,3 +214,30 @@ def test_a_row_that_is_not_finite_does_not_come_out_finite(gpu_lib, port, act, p
     keep = np.arange(sh.tokens) != 4
     assert np.array_equal(out[keep], good[keep])
     lay.close()
+
+
+@pytest.mark.parametrize("which", ["experts", "router"])
+def test_waits_run_out_and_the_handle_recovers(gpu_lib, port, which):
+    """The block-scaled kernel and the tensor-core router with a copy role that issues nothing, under a wait budget of 0.1 ms:
+    every role gives up, the call reports it, and the same handle then computes the layer as before."""
+    from coalsack_b200 import CskError
+    T = 70 if which == "experts" else 2048
+    sh = synth.tiny(seed=363, E=64, k=2, H=160, F=96, T=T, has_bias=True)
+    h, Wg, rb, ex = cases.layer_inputs(sh, router_scale=30.0)
+    lay = MoeLayer.from_shape(sh)
+    lay.set_router(Wg, rb)
+    lay.load_experts(ex)
+    lay.set_path(PATH_STREAM)
+    good, ro = lay.forward(h)
+    assert which == "experts" or lay.router_stats()[0] == T  # the certified pass ran
+    try:
+        lay.debug_set(lay.DEBUG_WAIT_BUDGET, 200_000)
+        lay.debug_set(lay.DEBUG_STALL_ROUTER if which == "router" else lay.DEBUG_STALL_TILE_PRODUCER, 1)
+        with pytest.raises(CskError) as err:
+            lay.forward(h)
+        assert err.value.code == -3 and "wait ran out" in str(err.value)
+    finally:
+        lay.debug_set(lay.DEBUG_WAIT_BUDGET, 2_000_000_000)
+    again, ro2 = lay.forward(h)
+    assert np.array_equal(ro, ro2) and np.array_equal(good, again)
+    lay.close()
