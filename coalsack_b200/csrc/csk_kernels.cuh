@@ -61,11 +61,12 @@ __global__ void k_pack_router(const float* __restrict__ wg, float* __restrict__ 
 // k rounds is an arg-max by shuffles (ties -> lower expert id; the reference
 // leaves ties unspecified).
 //
-// With `bounds` (the logits then come from the fast kernel, see k_router_logits)
-// one more round finds the runner-up, and the selection is CERTIFIED only if every
-// gap between neighbours of the k+1 best logits exceeds the sum of their error
-// bounds: the reference's own logits, which lie within those bounds, then order
-// the same experts the same way.  Returns false (warp-uniform) when a gap is too
+// With `bounds` (the logits then come from a fast kernel, see k_router_fast) the
+// selection is CERTIFIED only if every gap between neighbours of the k best logits
+// exceeds the sum of their error bounds, and the last of them less its bound exceeds
+// every other logit plus ITS bound (not only the runner-up's: a gate row of large
+// norm may have a larger bound than any).  The reference's own logits, which lie
+// within those bounds, then order the same experts the same way.  Returns false (warp-uniform) when a gap is too
 // small; the caller then sends the token through the order-faithful chain.
 // CG: logits and bounds are global memory written by other blocks (read through L2); else
 // they are the block's own shared memory.
@@ -79,10 +80,10 @@ __device__ __forceinline__ bool warp_topk_nv(const float* __restrict__ l, int E,
 #pragma unroll
   for (int i = 0; i < NV; ++i)
     v[i] = (i * 32 < E && i * 32 + lane < E) ? (CG ? __ldcg(l + i * 32 + lane) : l[i * 32 + lane]) : -INFINITY;
-  float sel_v[kMaxTopK + 1];
-  int sel_i[kMaxTopK + 1];
-  const int rounds = bounds ? min(k + 1, E) : k;
-  for (int j = 0; j < rounds; ++j) {
+  float sel_v[kMaxTopK];
+  int sel_i[kMaxTopK];
+  uint32_t gone = 0;
+  for (int j = 0; j < k; ++j) {
     float bv = -INFINITY;
     int bi = 0x7fffffff;
 #pragma unroll
@@ -108,15 +109,30 @@ __device__ __forceinline__ bool warp_topk_nv(const float* __restrict__ l, int E,
     // the winner leaves the pool: NaN never wins a '>' test again
 #pragma unroll
     for (int i = 0; i < NV; ++i)
-      if (i * 32 < E && bi == i * 32 + lane) v[i] = __int_as_float(0xffc00000);
+      if (i * 32 < E && bi == i * 32 + lane) {
+        v[i] = __int_as_float(0xffc00000);
+        gone |= 1u << i;
+      }
   }
   int certified = 1;
-  if (bounds && lane == 0) {
-    float b[kMaxTopK + 1];
-    for (int j = 0; j < rounds; ++j)
-      b[j] = (sel_i[j] >= 0 && sel_i[j] < E) ? (CG ? __ldcg(bounds + sel_i[j]) : bounds[sel_i[j]]) : INFINITY;
-    for (int j = 0; j + 1 < rounds; ++j)
-      if (!(sel_v[j] - sel_v[j + 1] > b[j] + b[j + 1])) certified = 0;  // also false for NaN
+  if (bounds) {
+    float above = -INFINITY;  // what no logit left out exceeds
+#pragma unroll
+    for (int i = 0; i < NV; ++i)
+      if (i * 32 < E && i * 32 + lane < E && !(gone >> i & 1u)) {
+        const float x = v[i] + (CG ? __ldcg(bounds + i * 32 + lane) : bounds[i * 32 + lane]);
+        above = x < INFINITY ? fmaxf(above, x) : INFINITY;  // (a NaN too)
+      }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) above = fmaxf(above, __shfl_xor_sync(0xffffffffu, above, o));
+    if (lane == 0) {
+      float b[kMaxTopK];
+      for (int j = 0; j < k; ++j)
+        b[j] = (sel_i[j] >= 0 && sel_i[j] < E) ? (CG ? __ldcg(bounds + sel_i[j]) : bounds[sel_i[j]]) : INFINITY;
+      for (int j = 0; j + 1 < k; ++j)
+        if (!(sel_v[j] - sel_v[j + 1] > b[j] + b[j + 1])) certified = 0;  // also false for NaN
+      if (!(sel_v[k - 1] - b[k - 1] > above)) certified = 0;
+    }
   }
   certified = __shfl_sync(0xffffffffu, certified, 0);
   if (lane == 0) {
@@ -524,8 +540,8 @@ inline void launch_router_logits(RouterArgs a, const float* wg_few, const float*
 //   A <= |h|_2 |w_e|_2 (Cauchy-Schwarz; |w_e|_2 precomputed, |h|_2 summed on the way).
 // bound = 1.05 u (33 sum_j |R_j| + 50 |h| |w_e|) + 4 u |logit| covers both, the two roundings
 // of the bias addition and the rounding of the bound's own arithmetic.  The top-k step accepts
-// a selection only when the gaps between neighbours of the k+1 best logits exceed the sum of
-// their bounds; every other token goes through the order-faithful chain (k_router_logits over
+// a selection only when the gaps between neighbours of the k best logits exceed the sum of
+// their bounds and no expert left out can reach the last of them; every other token goes through the order-faithful chain (k_router_logits over
 // the list of those tokens).  Expert indices are therefore the reference's in every case.
 //
 // k_router_fast: CTA = (block of 4*TPW tokens, group of 32 experts, part m of the hidden

@@ -161,3 +161,20 @@ def test_certified_router_on_the_tensor_cores(gpu_lib, port, E, k, H, T, kind):
     assert np.array_equal(other[keep], got[keep])
     assert lay.router_stats()[1] - chained >= 2
     lay.close()
+
+
+@pytest.mark.parametrize("T", [2, 2048])
+def test_an_expert_left_out_with_a_large_bound_is_not_overlooked(gpu_lib, port, T):
+    """One gate row's terms are rounded up next to a large entry that cancels at the end: its chain logit is twice the exact
+    one, the highest of all, while its exact logit is only the fourth, behind three with small error bounds."""
+    E, k, H = 40, 2, 64
+    Wg = np.zeros((E, H), np.float32)
+    Wg[0, 1], Wg[1, 1], Wg[2, 1] = 2.0, 1.9, 1.8
+    Wg[5, 0], Wg[5, 62] = 2.0 ** 20, -(2.0 ** 20)
+    Wg[5, np.r_[1:25:2, 33:57:2]] = 0.0626
+    h = np.ones((T, H), np.float32)
+    want, logits = port.router_logits(h, Wg, None, k)
+    assert np.argmax(logits[0]) == 5 and abs(Wg[5].astype(np.float64).sum() - 24 * 0.0626) < 1e-6
+    lay = _router_layer(E, k, H, Wg, None, T)
+    assert np.array_equal(lay.route(h)[..., 0], want[..., 0])
+    lay.close()
