@@ -698,6 +698,8 @@ struct FinishRouterArgs {
 };
 
 constexpr int kFastMaxParts = 32;
+// Squares of values under 2^-75 vanish in fp32: 2^16 columns of them have a norm of at most this.
+constexpr float kNormFloor = 0x1p-66f;
 
 // One block per token, one thread per expert (at most 256 threads; more experts take turns): a
 // thread's loads of its expert's parts are all in flight at once; logits and bounds meet in
@@ -713,7 +715,7 @@ __global__ void __launch_bounds__(256) k_router_finish(const FinishRouterArgs A)
   float h2 = lane < parts ? __ldcg(A.hn2 + (size_t)t * parts + lane) : 0.f;
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) h2 += __shfl_xor_sync(0xffffffffu, h2, o);  // every warp, all lanes
-  const float hn = sqrtf(h2) * 1.001f;
+  const float hn = sqrtf(h2) * 1.001f + kNormFloor;
   for (int e = threadIdx.x; e < E; e += blockDim.x) {
     float2 v[kFastMaxParts];
 #pragma unroll
@@ -756,7 +758,7 @@ __global__ void __launch_bounds__(32 * kFinishWarps) k_router_finish_many(const 
   float h2 = lane < parts ? __ldcg(A.hn2 + (size_t)t * parts + lane) : 0.f;
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) h2 += __shfl_xor_sync(0xffffffffu, h2, o);
-  const float hn = sqrtf(h2) * 1.001f;
+  const float hn = sqrtf(h2) * 1.001f + kNormFloor;
   for (int e = lane; e < E; e += 32) {
     float P = 0.f, sr = 0.f;
     for (int m = 0; m < parts; ++m) {
@@ -791,7 +793,7 @@ __global__ void k_router_wnorm(const float* __restrict__ wg, float* __restrict__
   float acc = 0.f;
   for (int d = lane; d < H; d += 32) acc = fmaf(wg[(size_t)e * H + d], wg[(size_t)e * H + d], acc);
   for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-  if (lane == 0) wnorm[e] = sqrtf(acc) * 1.001f;
+  if (lane == 0) wnorm[e] = sqrtf(acc) * 1.001f + kNormFloor;
 }
 
 __global__ void __launch_bounds__(128)

@@ -96,7 +96,7 @@ __global__ void k_rt_wnorm(const float* __restrict__ wg, float* __restrict__ wno
     if (lane == 0) acc = fmaf(m, m, acc);
   }
   for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-  if (lane == 0) wnorm[e] = sqrtf(acc) * 1.001f;
+  if (lane == 0) wnorm[e] = sqrtf(acc) * 1.001f + kNormFloor;
 }
 
 // Gate rows as digits: one thread per (group, block, expert).

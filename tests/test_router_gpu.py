@@ -178,3 +178,22 @@ def test_an_expert_left_out_with_a_large_bound_is_not_overlooked(gpu_lib, port, 
     lay = _router_layer(E, k, H, Wg, None, T)
     assert np.array_equal(lay.route(h)[..., 0], want[..., 0])
     lay.close()
+
+
+def test_tokens_whose_squares_underflow_are_not_certified_by_mistake(gpu_lib, port):
+    """Token rows near 2^-78 whose logits cancel down to the size of the chain's own rounding errors: their norms' squares
+    are below the smallest float, but the bounds must not be."""
+    E, k, H, T = 64, 2, 64, 2048
+    rng = np.random.default_rng(19)
+    g = rng.standard_normal(H).astype(np.float32)
+    Wg = rng.standard_normal((E, H)).astype(np.float32)
+    Wg[:, -1] = (2.0 ** -17 * rng.standard_normal(E) - Wg[:, :-1].astype(np.float64) @ g[:-1].astype(np.float64)) / g[-1]
+    h = (g * 2.0 ** -78 * rng.uniform(1, 2, (T, 1))).astype(np.float32)
+    want, logits = port.router_logits(h, Wg, None, k)
+    top = -np.sort(-logits, axis=1)[:, :k + 1]
+    clean = np.all(top[:, :-1] != top[:, 1:], axis=1)
+    exact = np.argsort(-(h.astype(np.float64) @ Wg.T.astype(np.float64)), axis=1)[:, :k]
+    assert np.any(exact[clean] != want[clean][..., 0])  # the chain orders some tokens otherwise than exact arithmetic
+    lay = _router_layer(E, k, H, Wg, None, T)
+    assert np.array_equal(lay.route(h)[clean][..., 0], want[clean][..., 0])
+    lay.close()
