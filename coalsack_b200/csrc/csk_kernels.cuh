@@ -183,6 +183,7 @@ struct RouterArgs {
   int* n_list;           // read at start; reset to zero, with fb_done, by the last block to finish
   int* fb_done;          // ticket of that reset
   unsigned long long* fb_total;  // running number of tokens that took the fall-back pass (statistics)
+  int list_over, list_max;       // the launch takes a list of list_over < entries <= list_max, and leaves any other alone
 };
 
 // A block is one producer warp (four with plain weights) plus TW consumer warps.  A
@@ -257,7 +258,8 @@ k_router_logits(const RouterArgs A) {
   griddep_launch();
   // tokens of this launch: all T, or the entries of a list built by an earlier kernel
   const int* const list = A.token_list;
-  const int n_tok = list ? min(*reinterpret_cast<volatile int*>(A.n_list), T) : T;
+  const int n_list = list ? min(*reinterpret_cast<volatile int*>(A.n_list), T) : 0;
+  const int n_tok = list ? (n_list > A.list_over && n_list <= A.list_max ? n_list : 0) : T;
   auto token_at = [&](int ti) { return ti < n_tok ? (list ? list[ti] : ti) : -1; };
 
   // A block takes the token blocks blockIdx.x, blockIdx.x + gridDim.x, ...  (one each unless the launch
@@ -462,8 +464,8 @@ k_router_logits(const RouterArgs A) {
   }  // token blocks of this block
 
   if (tid == 0 && *abort_flag && A.status) atomicOr(A.status, kDevErrWaitTimeout);
-  if (list && tid == 0) {
-    // every block of a list-driven launch, busy or idle, has read the list's length by now: the last
+  if (list && n_tok && tid == 0) {
+    // every block of the launch that takes the list, busy or idle, has read its length by now: the last
     // one to get here clears it for the next step
     __threadfence();
     if (atomicAdd(A.fb_done, 1) == (int)(gridDim.x * gridDim.y) - 1) {

@@ -212,9 +212,12 @@ int launch_router(csk_moe_layer* L, const float* d_hidden, int64_t T, float* d_r
   // 51 vs 53 us per step at T=1, level at T=4, and behind from T=16 on (361 vs 342 us at T=64).
   constexpr int64_t kCertifiedMaxTokens = 4;
   // With many tokens the chain is held by its arithmetic, token x expert; the certified pass on the tensor cores costs
-  // little per token, but three launches and the chain of the few percent it cannot separate.  Chain / certified, us:
-  // 128 experts, 2880 columns: 1024 tokens 66 / 49, 2048 117 / 58, 8192 343 / 129; 128 x 2048: 2048 92 / 49; 32 x 2880: 1024
-  // 31 / 44, 4096 64 / 72, 8192 122 / 119 (a digit matrix has 128 rows whatever the experts).
+  // little per token, but four launches and the chain of the few percent it cannot separate.  Chain / certified, us, normal
+  // rows: 128 experts, 2880 columns: 333 tokens 43 / (FMA pass) 75, 1024 66 / 51, 2048 119 / 57, 8192 343 / 138; 128 x 2048:
+  // 1024 49 / 44; 64 x 2880: 1024 43 / (FMA) 82, 2048 66 / 56; 256 x 2880: 512 68 / 57, 8192 664 / 259; 512 x 2880: 256
+  // 77 / 79, 512 131 / 75; 32 x 2880: 1024 31 / 44, 4096 64 / 72, 8192 122 / 119 (a digit matrix has 128 rows whatever the
+  // experts).  The line is where the two meet: at half as many pairs the FMA pass, which the certified mode then takes, is
+  // the slower one everywhere.
   constexpr int64_t kTensorMinWork = 4096;  // tokens x groups of 32 experts
   const int groups = (L->E_router + 31) / 32;
   const bool few = T <= kCertifiedMaxTokens, many = groups > 1 && T * groups >= kTensorMinWork;
@@ -224,6 +227,9 @@ int launch_router(csk_moe_layer* L, const float* d_hidden, int64_t T, float* d_r
     L->last.launches += 1;
     return CSK_OK;
   }
+  // (the kernels of a large batch's pass start while the one before them ends, too: the second launch for the list is then
+  // nearly free, 5 us otherwise)
+  const bool pdl = L->pdl || (many && !L->timing);
   // fast logits with error bounds; tokens whose selection the bounds do not certify are listed ...
   FinishRouterArgs g{};
   g.part = L->d_part;
@@ -254,14 +260,14 @@ int launch_router(csk_moe_layer* L, const float* d_hidden, int64_t T, float* d_r
     // one CTA fits an SM: as many parts of the hidden dimension as one wave holds
     int parts = std::min(std::min(rt_blocks(L->H), kFastMaxParts), std::max(1, L->sm_count / (token_tiles * rg)));
     while (parts > 1 && T * parts > L->part_rows) --parts;
-    launch_k(k_router_tc, dim3((unsigned)token_tiles, (unsigned)rg, (unsigned)parts), dim3(kRtThreads), kRtSmem, s, L->pdl, f);
+    launch_k(k_router_tc, dim3((unsigned)token_tiles, (unsigned)rg, (unsigned)parts), dim3(kRtThreads), kRtSmem, s, pdl, f);
     g.wnorm = L->d_wnorm_tc;
     g.parts = parts;
     g.slices = rt_blocks(L->H);
     g.coef_prefix = kRtPrefixCoef;
     g.coef_norm = kRtNormCoef;
     launch_k(k_router_finish_many, dim3((unsigned)ceil_div((int)T, kFinishWarps)), dim3(32 * kFinishWarps),
-             sizeof(float) * 2 * kFinishWarps * L->E_router, s, L->pdl, g);
+             sizeof(float) * 2 * kFinishWarps * L->E_router, s, pdl, g);
   } else {
     FastRouterArgs f{};
     f.hidden = d_hidden;
@@ -281,26 +287,43 @@ int launch_router(csk_moe_layer* L, const float* d_hidden, int64_t T, float* d_r
     const dim3 grid((unsigned)token_blocks, (unsigned)groups, (unsigned)parts);
     const size_t smem = fast_router_smem(tpw);
     switch (tpw) {
-      case 1: launch_k(k_router_fast<1>, grid, dim3(128), smem, s, L->pdl, f); break;
-      case 2: launch_k(k_router_fast<2>, grid, dim3(128), smem, s, L->pdl, f); break;
-      case 4: launch_k(k_router_fast<4>, grid, dim3(128), smem, s, L->pdl, f); break;
-      case 8: launch_k(k_router_fast<8>, grid, dim3(128), smem, s, L->pdl, f); break;
-      default: launch_k(k_router_fast<16>, grid, dim3(128), smem, s, L->pdl, f); break;
+      case 1: launch_k(k_router_fast<1>, grid, dim3(128), smem, s, pdl, f); break;
+      case 2: launch_k(k_router_fast<2>, grid, dim3(128), smem, s, pdl, f); break;
+      case 4: launch_k(k_router_fast<4>, grid, dim3(128), smem, s, pdl, f); break;
+      case 8: launch_k(k_router_fast<8>, grid, dim3(128), smem, s, pdl, f); break;
+      default: launch_k(k_router_fast<16>, grid, dim3(128), smem, s, pdl, f); break;
     }
     g.wnorm = L->d_wnorm;
     g.parts = parts;
-    launch_k(k_router_finish, dim3((unsigned)T), dim3((unsigned)std::min(32 * groups, 256)), 0, s, L->pdl, g);
+    launch_k(k_router_finish, dim3((unsigned)T), dim3((unsigned)std::min(32 * groups, 256)), 0, s, pdl, g);
   }
-  // ... and go through the order-faithful chain (a grid for a few percent of the tokens; its blocks
-  // walk the list however long it turned out, and leave at once when it is empty)
+  // ... and go through the order-faithful chain: its blocks walk the list and leave at once when it is empty
   RouterArgs b = a;
   b.token_list = L->d_fb_list;
   b.n_list = L->d_fb;
   b.fb_done = L->d_fb + 1;
   b.fb_total = reinterpret_cast<unsigned long long*>(L->d_fb + 2);
-  // (one round of the grid holds 2 % of 8192 tokens)
-  const int slots = (int)std::min<int64_t>(T, std::max(1, (T > 6144 ? 8 : 4) * L->sm_count / groups));
-  launch_router_logits<true>(b, L->d_wg_few, L->d_wg_many, L->sm_count, s, L->pdl, slots);
+  b.list_max = INT32_MAX;
+  const int64_t wave = std::max(1, 4 * L->sm_count / groups);  // tokens of one wave of four-token blocks
+  if (many) {
+    // How long the list is the data decide: 2 % of the tokens of normal rows, half of them with a few channels at 1000 times
+    // the others, all where rows repeat a value (padding).  Blocks of few tokens are quicker for a short list: the first
+    // launch has them for a 32nd of the tokens (at least one wave, at most two) and takes up to two rounds of that.
+    // The second has up to 16 tokens a block and takes any longer list; each leaves the other's lists alone.  128 experts,
+    // 2880 columns, one launch / two, us: 8192 normal rows 133 / 138, nine channels at 1000 times the others 569 / 399, every
+    // second row zero 513 / 351, every row 870 / 540 (the chain alone 343); 1024 tokens 51 / 51, every row zero 165 / 94 (66).
+    const int few_slots = (int)std::min(2 * wave, std::max(wave, T / 32));
+    b.list_max = 2 * few_slots;
+    launch_router_logits<true>(b, L->d_wg_few, L->d_wg_many, L->sm_count, s, pdl, few_slots);
+    if (T > b.list_max) {
+      b.list_over = b.list_max;
+      b.list_max = INT32_MAX;
+      launch_router_logits<true>(b, L->d_wg_few, L->d_wg_many, L->sm_count, s, pdl, (int)std::min(T, 8 * wave));
+      L->last.launches += 1;
+    }
+  } else {
+    launch_router_logits<true>(b, L->d_wg_few, L->d_wg_many, L->sm_count, s, pdl, (int)std::min(T, wave));
+  }
   CSK_CUDA(L, cudaGetLastError());
   L->last.launches += 3;
   L->routed_tokens += T;

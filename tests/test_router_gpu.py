@@ -197,3 +197,28 @@ def test_tokens_whose_squares_underflow_are_not_certified_by_mistake(gpu_lib, po
     lay = _router_layer(E, k, H, Wg, None, T)
     assert np.array_equal(lay.route(h)[clean][..., 0], want[clean][..., 0])
     lay.close()
+
+
+def test_lists_of_any_length_go_through_the_chain(gpu_lib, port):
+    """Tokens that the certified pass cannot separate: a few, more than one round of the launch for short lists holds, and
+    most of the batch (the other launch's), in turn on one handle; the experts are the reference's each time."""
+    E, k, H, T = 64, 4, 256, 2048
+    rng = np.random.default_rng(23)
+    Wg = (rng.standard_normal((E, H)) * 0.05).astype(np.float32)
+    Wg[E // 2:] = Wg[:E // 2]          # pairs of gate rows that differ in one column
+    Wg[E // 2:, 40] += np.float32(1e-3)
+    lay = _router_layer(E, k, H, Wg, None, T)
+    before = 0
+    for m in (30, 1500, 0, 500, T, 3):
+        h = rng.standard_normal((T, H)).astype(np.float32)
+        h[:, 40] = 4.0
+        h[rng.permutation(T)[:m], 40] = 0.002     # their pairs of logits differ by 2e-6
+        want, logits = port.router_logits(h, Wg, None, k)
+        top = -np.sort(-logits, axis=1)[:, :k + 1]
+        clean = np.all(top[:, :-1] != top[:, 1:], axis=1)
+        assert clean.mean() > 0.9
+        assert np.array_equal(lay.route(h)[clean][..., 0], want[clean][..., 0])
+        chained = lay.router_stats()[1]
+        assert m <= chained - before <= m + 0.1 * T, (m, chained - before)
+        before = chained
+    lay.close()
