@@ -394,7 +394,7 @@ int launch_permute(csk_moe_layer* L, const float* d_hidden, const float* d_route
 }
 
 // Images for `rows` grouped rows (row tiles of full height plus one shorter one per expert).  Called when the layer is
-// created and when a path is chosen, never from a stage: those may run under a caller's capture.  Images that were
+// created, when a path is chosen and when peers are set up, never from a stage: those may run under a caller's capture.  Images that were
 // outgrown live as long as the layer, because graphs captured before (the handle's or a caller's) still name them.
 int mx_reserve(csk_moe_layer* L, int64_t rows) {
   if (L->w16 || rows <= L->mx_rows) return CSK_OK;
@@ -482,11 +482,10 @@ int choose_path(const csk_moe_layer* L, int64_t rows) {
   return (L->tile.available && rows >= kMxRowsPerExpert * (int64_t)std::max(1, L->Eloc)) ? CSK_PATH_TILE : CSK_PATH_STREAM;
 }
 
-// The expert-parallel receive side: the caller's row count is no bound on what one expert gets, so the block-scaled
-// kernel needs images for every row the handle may receive (a layer that holds part of the experts has them).
-int choose_path_received(const csk_moe_layer* L, int64_t rows) {
+// The expert-parallel receive side: the block-scaled kernel needs images for every row that may come (`most`).
+int choose_path_received(const csk_moe_layer* L, int64_t rows, int64_t most) {
   const int path = choose_path(L, rows);
-  return path == CSK_PATH_STREAM && L->mx_rows < L->max_rows ? CSK_PATH_TILE : path;
+  return path == CSK_PATH_STREAM && L->mx_rows < most ? CSK_PATH_TILE : path;
 }
 
 // the CTA-pair kernel runs only when asked for by name (and clusters of two can be launched)
@@ -831,8 +830,8 @@ int csk_moe_create(const csk_moe_config* cfg, csk_moe_layer** out) {
       return rc;
     }
   }
-  // images for the batches the block-scaled kernel takes by itself; for any, where rows come from other devices
-  if (mx_reserve(L, eloc < L->E ? L->max_rows : std::min(L->max_rows, kMxRowsPerExpert * eloc))) {
+  // images for the batches the block-scaled kernel takes by itself
+  if (mx_reserve(L, std::min(L->max_rows, kMxRowsPerExpert * eloc))) {
     fail(nullptr, CSK_ERR_NOMEM, "%s", L->err.c_str());
     csk_moe_destroy(L);
     return CSK_ERR_NOMEM;
@@ -1784,6 +1783,8 @@ int ep_finish(csk_moe_layer* L, cudaStream_t s, int n_marks) {
 }
 int p2p_alloc_local(csk_moe_layer* L) {
   if (L->d_info) return CSK_OK;
+  int rc = mx_reserve(L, L->max_rows);  // how many rows the peers will send is not known on the host
+  if (rc) return rc;
   CSK_CUDA(L, cudaMalloc(&L->d_info, sizeof(RowOrigin) * (size_t)L->max_rows));
   // 0xFF bytes: (-1, -1), which no reader accepts as an origin (rows a sender had to skip stay that way)
   CSK_CUDA(L, cudaMemset(L->d_info, 0xFF, sizeof(RowOrigin) * (size_t)L->max_rows));
@@ -1984,12 +1985,12 @@ int csk_moe_ep_p2p_experts_dev(csk_moe_layer* L, const int32_t* d_all_counts, in
   CSK_CUDA(L, cudaSetDevice(L->cfg.device));
   cudaStream_t s = pick(L, stream);
   rows_hint = std::max<int64_t>(1, std::min<int64_t>(rows_hint, L->max_rows));
-  const int path = choose_path_received(L, rows_hint);
+  const int path = choose_path_received(L, rows_hint, L->max_rows);  // (a hint is no bound)
   const int tile_rows = tile_rows_for(L, path);
   const bool mx = path == CSK_PATH_STREAM;
   // the status word of the dispatch stays; the tile list is rebuilt from the received counts
   k_ep_p2p_local_counts<<<(L->E + 255) / 256, 256, 0, s>>>(d_all_counts, L->p2p_world, L->E, L->e0, L->Eloc, L->d_counts);
-  k_scan<<<1, 1024, 0, s>>>(L->d_counts, L->E, L->e0, L->Eloc, tile_rows, (int)L->max_rows, L->max_tiles,
+  k_scan<<<1, 1024, 0, s>>>(L->d_counts, L->E, L->e0, L->Eloc, tile_rows, (int)(mx ? L->mx_rows : L->max_rows), L->max_tiles,
                             L->d_resident, L->d_offsets, L->d_cursor, L->d_tiles, L->d_meta, nullptr, 0, -1, nullptr,
                             mx ? L->d_expert_tiles : nullptr, mx ? L->d_wide : nullptr, wide_stride(L));
   k_ep_p2p_rowptr<<<4 * L->sm_count, 256, 0, s>>>(L->d_info, L->d_meta, L->d_peer_back, L->H, L->d_row_ptr,
@@ -2031,13 +2032,13 @@ int csk_moe_ep_experts_dev(csk_moe_layer* L, const void* d_recv_f16, const int32
   CSK_CUDA(L, cudaSetDevice(L->cfg.device));
   cudaStream_t s = pick(L, stream);
   if (total_rows == 0) return CSK_OK;
-  const int path = choose_path_received(L, total_rows);
+  const int path = choose_path_received(L, total_rows, total_rows);
   const int tile_rows = tile_rows_for(L, path);
   const bool mx = path == CSK_PATH_STREAM;
   CSK_CUDA(L, cudaMemsetAsync(L->d_meta, 0, sizeof(int) * 8, s));
   CSK_CUDA(L, cudaMemsetAsync(L->d_counts, 0, sizeof(int) * L->E, s));
   k_ep_plan<<<1, 1024, 0, s>>>(d_recv_counts, n_src, L->Eloc, L->e0, L->d_counts, L->d_seg);
-  k_scan<<<1, 1024, 0, s>>>(L->d_counts, L->E, L->e0, L->Eloc, tile_rows, (int)L->max_rows, L->max_tiles,
+  k_scan<<<1, 1024, 0, s>>>(L->d_counts, L->E, L->e0, L->Eloc, tile_rows, (int)(mx ? L->mx_rows : L->max_rows), L->max_tiles,
                             L->d_resident, L->d_offsets, L->d_cursor, L->d_tiles, L->d_meta, nullptr, 0, -1, nullptr,
                             mx ? L->d_expert_tiles : nullptr, mx ? L->d_wide : nullptr, wide_stride(L));
   k_ep_regroup<<<dim3((unsigned)(n_src * L->Eloc), (unsigned)std::max(1, 16 * L->sm_count / (n_src * L->Eloc))), 128, 0, s>>>((const __half*)d_recv_f16, L->d_x16, L->ldx, L->d_seg,

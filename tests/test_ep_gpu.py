@@ -234,3 +234,18 @@ def test_emulated_p2p_overflow_is_a_status_not_a_fault(gpu_lib):
     assert codes == [-4, -4]
     for lay in layers:
         lay.close()
+
+
+def test_a_layer_with_part_of_the_experts_keeps_no_image_rows_it_cannot_use(gpu_lib):
+    """Digit images are for the batches the block-scaled kernel takes (40 rows per resident expert); images for every row
+    that peers may send come with the peer buffers.  Half a gigabyte here."""
+    import torch
+    torch.cuda.synchronize()
+    H, T, k = 2880, 8192, 4
+    free0 = torch.cuda.mem_get_info()[0]
+    lay = MoeLayer(8, k, H, H, max_tokens=T, expert_begin=2, expert_count=2)
+    used = free0 - torch.cuda.mem_get_info()[0]
+    rows = T * k * H * (2 + 2 + 4) + 2 * T * H * 4    # fp16 rows twice, output rows, hidden and result
+    weights = 2 * 2 * 3 * H * H * 17 // 32 + 3 * H * H * 17 // 32
+    assert used <= rows + weights + 150e6, (used, rows, weights)
+    lay.close()
