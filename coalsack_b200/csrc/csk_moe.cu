@@ -1178,6 +1178,37 @@ ImageHeader image_header_of(const csk_moe_layer* L) {
   h.off_td = L->off_td; h.off_bias = L->off_bias; h.off_meta = L->off_meta;
   return h;
 }
+// The header of an image of the layout before this one (02).  It differs in the first part of an expert's record only: the
+// decode kernel's copy of the codes was cut into records of 544 bytes, 16 rows x 64 columns.  What follows, from the other
+// kernel's tiles on, is the same.
+ImageHeader image_header_02(const csk_moe_layer* L) {
+  ImageHeader h = image_header_of(L);
+  memcpy(h.magic, "CSKMOE02", 8);
+  if (L->w16) return h;  // fp16 weights have no such copy
+  auto bytes = [](int N, int K, int parts) {
+    return ((size_t)ceil_div(N, 16) * ceil_div(K, 64) * parts * 544 + 255) / 256 * 256;
+  };
+  h.off_d = bytes(L->F, L->H, 2);
+  const uint64_t off_tgu = h.off_d + bytes(L->H, L->F, 1);
+  for (uint64_t* o : {&h.off_td, &h.off_bias, &h.off_meta}) *o = *o - h.off_tgu + off_tgu;
+  h.off_tgu = off_tgu;
+  h.expert_stride = (h.off_meta + 16 + 255) / 256 * 256;
+  return h;
+}
+// The decode kernel's copy of a resident expert's codes from the other kernel's tiles (which hold the blocks losslessly).
+int rebuild_mx_enqueue(csk_moe_layer* L, int le, cudaStream_t s) {
+  uint8_t* base = L->d_weights + (size_t)le * L->expert_stride;
+  uint8_t *s_up = L->d_stage, *s_gate = L->d_stage + L->stage_bytes, *s_down = L->d_stage + 2 * L->stage_bytes;
+  int* emeta = reinterpret_cast<int*>(base + L->off_meta);
+  const int grid = grid_for((size_t)L->F * (L->H / 32), 128, 4096);
+  k_unpack_tile<<<grid, 128, 0, s>>>(base + L->off_tgu, s_gate, L->Tgu, 0);
+  k_unpack_tile<<<grid, 128, 0, s>>>(base + L->off_tgu, s_up, L->Tgu, 1);
+  k_unpack_tile<<<grid, 128, 0, s>>>(base + L->off_td, s_down, L->Td, 0);
+  k_mx_repack<<<grid_for(L->Lgu.bytes() / 16, 256, 4096), 256, 0, s>>>(s_gate, s_up, base + L->off_gu, L->Lgu, emeta);
+  k_mx_repack<<<grid_for(L->Ld.bytes() / 16, 256, 4096), 256, 0, s>>>(s_down, nullptr, base + L->off_d, L->Ld, emeta + 1);
+  CSK_CUDA(L, cudaGetLastError());
+  return CSK_OK;
+}
 }  // namespace
 
 int csk_moe_save_image(csk_moe_layer* L, const char* path) {
@@ -1205,18 +1236,25 @@ int csk_moe_load_image(csk_moe_layer* L, const char* path) {
   FILE* f = fopen(path, "rb");
   if (!f) return fail(L, CSK_ERR_INVALID, "cannot open %s", path);
   ImageHeader h{};
-  const ImageHeader want = image_header_of(L);
+  const ImageHeader want = image_header_of(L), before = image_header_02(L);
   std::vector<uint8_t> res(L->Eloc);
   bool ok = fread(&h, sizeof h, 1, f) == 1;
-  if (ok && memcmp(&h, &want, sizeof h) != 0) {
+  const bool older = ok && memcmp(&h, &before, sizeof h) == 0;
+  if (ok && !older && memcmp(&h, &want, sizeof h) != 0) {
     fclose(f);
     return fail(L, CSK_ERR_INVALID, "%s was written for another layer shape, expert range or library layout", path);
   }
   ok = ok && fread(res.data(), 1, L->Eloc, f) == (size_t)L->Eloc;
-  std::vector<uint8_t> buf(L->expert_stride);
+  const bool rebuild = older && !L->w16;
+  const size_t from = rebuild ? h.off_tgu : 0, to = rebuild ? L->off_tgu : 0;
+  std::vector<uint8_t> buf(h.expert_stride);
   for (int e = 0; ok && e < L->Eloc; ++e) {
+    uint8_t* base = L->d_weights + (size_t)e * L->expert_stride;
     ok = fread(buf.data(), 1, buf.size(), f) == buf.size();
-    if (ok && cudaMemcpy(L->d_weights + (size_t)e * L->expert_stride, buf.data(), L->expert_stride, cudaMemcpyHostToDevice) != cudaSuccess) ok = false;
+    // (on the handle's stream, which does not wait for the default one: a plain copy may still be landing when it returns)
+    ok = ok && cudaMemcpyAsync(base + to, buf.data() + from, h.off_meta + 16 - from, cudaMemcpyHostToDevice, L->stream) == cudaSuccess;
+    if (ok && rebuild && res[e]) ok = rebuild_mx_enqueue(L, e, L->stream) == CSK_OK;
+    ok = cudaStreamSynchronize(L->stream) == cudaSuccess && ok;
   }
   fclose(f);
   if (!ok) return fail(L, CSK_ERR_CUDA, "reading the weight image from %s failed", path);

@@ -564,3 +564,56 @@ def test_bulk_load_and_weight_image(gpu_lib, port, tmp_path):
         other.load_image(img)
     for lay in (one, bulk, fresh, other):
         lay.close()
+
+
+@pytest.mark.parametrize("f16", [False, True])
+def test_weight_image_of_the_earlier_layout_still_loads(gpu_lib, tmp_path, f16):
+    """An image with the decode kernel's codes in the earlier layout (records of 16 rows x 64 columns, 544 bytes): that part
+    is rebuilt from the other kernel's tiles, which lie behind it; fp16 images had no such part."""
+    import struct
+    sh = synth.tiny(seed=57, E=3, k=1, H=160, F=96, T=8, has_bias=True)
+    h, Wg, rb, ex = cases.layer_inputs(sh, router_scale=40.0)
+    lay = MoeLayer.from_shape(sh, weights_f16=f16)
+    rng = np.random.default_rng(57)
+    for e in (0, 2):
+        if f16:
+            lay.load_expert_f16(e, *(rng.standard_normal(s).astype(np.float16) for s in ((96, 160), (96, 160), (160, 96))),
+                                ex["b_up"][e], ex["b_gate"][e], ex["b_down"][e])
+        else:
+            lay.load_expert(e, *cases.expert_args(ex, e))
+    img = tmp_path / "new.img"
+    lay.save_image(img)
+    raw = img.read_bytes()
+    head = struct.Struct("<8s8i7Q")
+    magic, *ints = head.unpack(raw[:head.size])
+    stride, off_gu, off_d, off_tgu, off_td, off_bias, off_meta = ints[8:]
+    part = lambda n, k, m: (-(-n // 16) * -(-k // 64) * m * 544 + 255) // 256 * 256
+    d2 = 0 if f16 else part(96, 160, 2)
+    move = (0 if f16 else d2 + part(160, 96, 1)) - off_tgu
+    stride2 = (off_meta + move + 16 + 255) // 256 * 256
+    out = head.pack(b"CSKMOE02", *ints[:8], stride2, 0, d2, off_tgu + move, off_td + move, off_bias + move, off_meta + move)
+    out += raw[head.size:head.size + 3]
+    for e in range(3):
+        rec = raw[head.size + 3 + e * stride:][:stride]
+        body = rng.integers(0, 256, off_tgu + move, dtype=np.uint8).tobytes() + rec[off_tgu:off_meta + 16]
+        out += body + bytes(stride2 - len(body))
+    older = tmp_path / "older.img"
+    older.write_bytes(out)
+    got = MoeLayer.from_shape(sh, weights_f16=f16)
+    got.load_image(older)
+    route = np.ones((8, 1, 2), np.float32)
+    route[:, 0, 0] = np.arange(8) % 2 * 2
+    assert not got.expert_resident(1)
+    for path in (PATH_TILE,) if f16 else (PATH_STREAM, PATH_TILE):
+        for x in (lay, got):
+            x.set_path(path)
+        assert np.array_equal(got.forward(h, router_out=route)[0], lay.forward(h, router_out=route)[0])
+    if not f16:
+        for e in (0, 2):
+            for which in range(6):
+                assert np.array_equal(got.unpack_expert(e, which), lay.unpack_expert(e, which))
+    older.write_bytes(out.replace(b"CSKMOE02", b"CSKMOE01", 1))
+    with pytest.raises(CskError):
+        got.load_image(older)
+    for x in (lay, got):
+        x.close()
