@@ -382,7 +382,7 @@ def run_ours(args):
                     "peak_source": peaks["source"] + " (burst bf16 cuBLAS)"}
     else:
         # weight streaming: algorithmic bytes = the packed gate and up matrices (17 bytes per 32 weights) of every expert
-        # that received rows, read once per 48-row tile
+        # that received rows, read once per 40-row tile
         gu_bytes = stage.get("row_tiles", 0) * 2.0 * sh.ffn * H * 17 / 32
         achieved = gu_bytes / (gu_ms * 1e-3) / 1e9 if gu_ms > 0 else 0.0
         roofline = {"bound": "hbm", "kernel": stage["gate_up_kernel"], "achieved": achieved, "peak": peaks["hbm_gbs"],
@@ -462,7 +462,7 @@ class SingleGpu:
         out = {k: acc[k] / n for k in acc}
         out["path"] = {1: "stream", 2: "tile"}.get(int(round(out["path"])), "?")
         rows_per_expert, _, _ = self.layer.counters()
-        tr = 48 if out["path"] == "stream" else 192
+        tr = 40 if out["path"] == "stream" else 192
         out["row_tiles"] = int(sum(-(-int(r) // tr) for r in rows_per_expert))
         out["gate_up_kernel"] = "k_mx<gated>" if out["path"] == "stream" else "k_tile<gated>"
         return out

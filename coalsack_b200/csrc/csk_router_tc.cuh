@@ -2,8 +2,8 @@
 //
 // The certified pass (csk_kernels.cuh, above k_router_fast) needs, per (token, expert), a value close to the exact
 // logit, the sum of the magnitudes of its prefixes, and a bound on its own error.  The FMA kernel is held by shared-
-// memory operand delivery; here the products are INTEGER products on tcgen05.mma kind::f16, so the bound needs no
-// assumption about how the tensor cores round:
+// memory operand delivery; here the products are INTEGER products on tcgen05.mma kind::f16, and the bound assumes of the
+// tensor cores only that sums of integers are exact in their fp32 accumulators while every partial sum is below 2^24:
 //   * per (row, block of 64 columns) x = 2^(e-8) (s0 + s1 2^-9 + s2 2^-18 + rest), 2^e the smallest power of two that
 //     the block's largest magnitude m does not exceed, s0, s1, s2 integers of magnitude <= 256 (fp16 holds them
 //     exactly), |rest| <= 2^-19: at most 2^-26 m is left out;

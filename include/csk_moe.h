@@ -375,14 +375,20 @@ int csk_moe_set_activation(csk_moe_layer* layer, int32_t activation /* CSK_ACT_*
  * logit a sequential fp32 multiply-then-add chain over the hidden dimension, top-k by
  * logit).  Every mode returns the same expert indices as the reference, bit for bit.
  *   CSK_ROUTER_CHAIN: every logit by the reference's own chain (one launch).
- *   CSK_ROUTER_CERTIFIED: logits by fused multiply-adds in 32-column blocks with a
- *     rigorous bound on their distance from the chain's value; a token whose k+1 best
- *     logits are further apart than the bounds keeps that selection, any other token is
- *     recomputed by the chain.  Routing WEIGHTS of certified tokens come from the fast
- *     logits and differ from the reference's by a few ulp (below 1e-6).
+ *   CSK_ROUTER_CERTIFIED: fast logits with a rigorous bound on their distance from the
+ *     chain's values -- fused multiply-adds in 32-column blocks, or, with more than 32
+ *     experts and at least 4096 (token, group of 32 experts) pairs, integer digits on the
+ *     tensor cores in 64-column blocks.  A token whose selection the bounds separate from
+ *     every other keeps it, any other token is recomputed by the chain.  Routing WEIGHTS of
+ *     certified tokens come from the fast logits and differ from the reference's by a few
+ *     ulp (below 1e-6).
  *   CSK_ROUTER_AUTO (default): certified for batches of up to 4 tokens, where the chain
- *     is one long dependency on a few SMs; the chain kernel for anything larger, where it
- *     is the faster of the two (measured). */
+ *     is one long dependency on a few SMs, and, with more than 32 experts, from 4096
+ *     (token, group of 32 experts) pairs on (1024 tokens of 128 experts), where it is held
+ *     by its arithmetic; the chain in between, where it is the faster of the two (measured).
+ *     So a token's weights may differ in their last bits between batch sizes, and within
+ *     a large batch between tokens that were certified and tokens that were not; the
+ *     experts never do.  CSK_ROUTER_CHAIN gives the reference's own at every size. */
 enum { CSK_ROUTER_AUTO = 0, CSK_ROUTER_CHAIN = 1, CSK_ROUTER_CERTIFIED = 2 };
 int csk_moe_set_router_mode(csk_moe_layer* layer, int32_t mode);
 /* Tokens routed in certified mode since the handle was created, and how many of them
