@@ -215,12 +215,12 @@ int launch_router(csk_moe_layer* L, const float* d_hidden, int64_t T, float* d_r
   // little per token, but four launches and the chain of the few percent it cannot separate.  Chain / certified, us, normal
   // rows: 128 experts, 2880 columns: 333 tokens 43 / (FMA pass) 75, 1024 66 / 51, 2048 119 / 57, 8192 343 / 138; 128 x 2048:
   // 1024 49 / 44; 64 x 2880: 1024 43 / (FMA) 82, 2048 66 / 56; 256 x 2880: 512 68 / 57, 8192 664 / 259; 512 x 2880: 256
-  // 77 / 79, 512 131 / 75; 32 x 2880: 1024 31 / 44, 4096 64 / 72, 8192 122 / 119 (a digit matrix has 128 rows whatever the
+  // 77 / 79, 512 131 / 75; 512 x 2048: 256 61 / 71, 512 98 / 63; 1024 x 2048: 128 61 / 97, 256 98 / 71; 32 x 2880: 1024 31 / 44, 4096 64 / 72, 8192 122 / 119 (a digit matrix has 128 rows whatever the
   // experts).  The line is where the two meet: at half as many pairs the FMA pass, which the certified mode then takes, is
-  // the slower one everywhere.
-  constexpr int64_t kTensorMinWork = 4096;  // tokens x groups of 32 experts
+  // the slower one everywhere; with 512 experts and more (few tokens, many digit matrices) they meet at twice as many.
   const int groups = (L->E_router + 31) / 32;
-  const bool few = T <= kCertifiedMaxTokens, many = groups > 1 && T * groups >= kTensorMinWork;
+  const int64_t tensor_min_work = groups >= 16 ? 8192 : 4096;  // tokens x groups of 32 experts
+  const bool few = T <= kCertifiedMaxTokens, many = groups > 1 && T * groups >= tensor_min_work;
   if (L->router_mode == CSK_ROUTER_CHAIN || (L->router_mode == CSK_ROUTER_AUTO && !few && !many)) {
     launch_router_logits<true>(a, L->d_wg_few, L->d_wg_many, L->sm_count, s, L->pdl);
     CSK_CUDA(L, cudaGetLastError());

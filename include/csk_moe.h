@@ -377,14 +377,15 @@ int csk_moe_set_activation(csk_moe_layer* layer, int32_t activation /* CSK_ACT_*
  *   CSK_ROUTER_CHAIN: every logit by the reference's own chain (one launch).
  *   CSK_ROUTER_CERTIFIED: fast logits with a rigorous bound on their distance from the
  *     chain's values -- fused multiply-adds in 32-column blocks, or, with more than 32
- *     experts and at least 4096 (token, group of 32 experts) pairs, integer digits on the
+ *     experts and at least 4096 (token, group of 32 experts) pairs (8192 from 512 experts
+ *     on), integer digits on the
  *     tensor cores in 64-column blocks.  A token whose selection the bounds separate from
  *     every other keeps it, any other token is recomputed by the chain.  Routing WEIGHTS of
  *     certified tokens come from the fast logits and differ from the reference's by a few
  *     ulp (below 1e-6).
  *   CSK_ROUTER_AUTO (default): certified for batches of up to 4 tokens, where the chain
- *     is one long dependency on a few SMs, and, with more than 32 experts, from 4096
- *     (token, group of 32 experts) pairs on (1024 tokens of 128 experts), where it is held
+ *     is one long dependency on a few SMs, and, with more than 32 experts, from as
+ *     many pairs on (1024 tokens of 128 experts), where it is held
  *     by its arithmetic; the chain in between, where it is the faster of the two (measured).
  *     So a token's weights may differ in their last bits between batch sizes, and within
  *     a large batch between tokens that were certified and tokens that were not; the

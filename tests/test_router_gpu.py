@@ -222,3 +222,20 @@ def test_lists_of_any_length_go_through_the_chain(gpu_lib, port):
         assert m <= chained - before <= m + 0.1 * T, (m, chained - before)
         before = chained
     lay.close()
+
+
+@pytest.mark.parametrize("E,T,certified", [(1024, 128, False), (1024, 256, True), (512, 511, False), (512, 512, True),
+                                           (128, 1023, False), (128, 1024, True), (32, 4096, False)])
+def test_which_batches_take_the_certified_pass_by_themselves(gpu_lib, port, E, T, certified):
+    """The default mode's rule, on both sides of its line: the pass is taken where it is the faster of the two."""
+    rng = np.random.default_rng(E + T)
+    Wg = (rng.standard_normal((E, 64)) * 0.05).astype(np.float32)
+    lay = _router_layer(E, 2, 64, Wg, None, T)
+    lay.set_router_mode(lay.ROUTER_AUTO)
+    h = rng.standard_normal((T, 64)).astype(np.float32)
+    want, logits = port.router_logits(h, Wg, None, 2)
+    top = -np.sort(-logits, axis=1)[:, :3]
+    clean = np.all(top[:, :-1] != top[:, 1:], axis=1)
+    assert np.array_equal(lay.route(h)[clean][..., 0], want[clean][..., 0])
+    assert (lay.router_stats()[0] == T) == certified
+    lay.close()
