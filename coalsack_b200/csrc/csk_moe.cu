@@ -472,14 +472,18 @@ void launch_mx_pair(csk_moe_layer* L, float* y, int ldy, cudaStream_t s, StageTi
   L->last.launches += 2;
 }
 
-// Rows per resident expert from which the fp16 tensor-core kernel takes over.
-constexpr int64_t kMxRowsPerExpert = 40;
+// Rows per resident expert from which the fp16 tensor-core kernel takes over: the block-scaled one's time goes by the rows
+// (digit columns; from 40 on it reads weights twice), the other's hardly, and short contractions leave its units' epilogues
+// exposed.  Whole layer, block-scaled / fp16 kernel, us: 128 experts of 2880 x 2880 at 32 rows 565 / 670, at 40 667 / 684, at 48
+// 826 / 705; 32 experts of 2880 x 2880 at 32 171 / 192, at 40 208 / 198 (Zipf load: 199 / 205); 8 experts of 1728 x 1728 at 32
+// 48 / 54, at 40 58 / 54; 128 experts of 2048 x 768 at 24 191 / 197, at 32 216 / 203.
+int64_t mx_rows_per_expert(const csk_moe_layer* L) { return std::min(kMxTileRows, 20 + std::min(L->H, L->F) / 128); }
 
 int choose_path(const csk_moe_layer* L, int64_t rows) {
   if (L->w16) return CSK_PATH_TILE;  // fp16 weights exist in the tensor-core layout only
   if (L->path == CSK_PATH_STREAM) return CSK_PATH_STREAM;
   if (L->path == CSK_PATH_TILE || L->path == CSK_PATH_TILE_PAIR) return CSK_PATH_TILE;
-  return (L->tile.available && rows >= kMxRowsPerExpert * (int64_t)std::max(1, L->Eloc)) ? CSK_PATH_TILE : CSK_PATH_STREAM;
+  return (L->tile.available && rows >= mx_rows_per_expert(L) * std::max(1, L->Eloc)) ? CSK_PATH_TILE : CSK_PATH_STREAM;
 }
 
 // The expert-parallel receive side: the block-scaled kernel needs images for every row that may come (`most`).
@@ -831,7 +835,7 @@ int csk_moe_create(const csk_moe_config* cfg, csk_moe_layer** out) {
     }
   }
   // images for the batches the block-scaled kernel takes by itself
-  if (mx_reserve(L, std::min(L->max_rows, kMxRowsPerExpert * eloc))) {
+  if (mx_reserve(L, std::min(L->max_rows, mx_rows_per_expert(L) * eloc))) {
     fail(nullptr, CSK_ERR_NOMEM, "%s", L->err.c_str());
     csk_moe_destroy(L);
     return CSK_ERR_NOMEM;

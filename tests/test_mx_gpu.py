@@ -241,3 +241,21 @@ def test_waits_run_out_and_the_handle_recovers(gpu_lib, port, which):
     again, ro2 = lay.forward(h)
     assert np.array_equal(ro, ro2) and np.array_equal(good, again)
     lay.close()
+
+
+@pytest.mark.parametrize("H,F,rows", [(256, 192, 21), (1728, 768, 26), (2880, 2880, 40)])
+def test_rows_per_expert_from_which_the_fp16_kernel_takes_over(gpu_lib, port, H, F, rows):
+    """The last batch of the block-scaled kernel and the first of the other, one expert: the images hold the one, and the
+    results of both are the checker's."""
+    sh = synth.tiny(seed=367, E=1, k=1, H=H, F=F, T=rows, has_bias=True)
+    h, Wg, rb, ex = cases.layer_inputs(sh)
+    lay = MoeLayer.from_shape(sh)
+    lay.set_router(Wg, rb)
+    lay.load_experts(ex)
+    for n, path in ((rows - 1, 1), (rows, 2)):
+        out, ro = lay.forward(h[:n])
+        assert lay.timings()["path"] == path
+        want, _ = port.moe_layer(h[:n], Wg, rb, ex, 1, sh.act, nthreads=8, router_out=ro)
+        mx, mr = cases.err_stats(out, want)
+        assert mx <= cases.MAX_ABS_OVER_RMS and mr <= cases.MEAN_REL, (mx, mr)
+    lay.close()
