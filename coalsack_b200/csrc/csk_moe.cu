@@ -483,7 +483,7 @@ int choose_path(const csk_moe_layer* L, int64_t rows) {
   if (L->w16) return CSK_PATH_TILE;  // fp16 weights exist in the tensor-core layout only
   if (L->path == CSK_PATH_STREAM) return CSK_PATH_STREAM;
   if (L->path == CSK_PATH_TILE || L->path == CSK_PATH_TILE_PAIR) return CSK_PATH_TILE;
-  return (L->tile.available && rows >= mx_rows_per_expert(L) * std::max(1, L->Eloc)) ? CSK_PATH_TILE : CSK_PATH_STREAM;
+  return (L->pair.available && rows >= mx_rows_per_expert(L) * std::max(1, L->Eloc)) ? CSK_PATH_TILE : CSK_PATH_STREAM;
 }
 
 // The expert-parallel receive side: the block-scaled kernel needs images for every row that may come (`most`).
@@ -492,8 +492,8 @@ int choose_path_received(const csk_moe_layer* L, int64_t rows, int64_t most) {
   return path == CSK_PATH_STREAM && L->mx_rows < most ? CSK_PATH_TILE : path;
 }
 
-// the CTA-pair kernel runs only when asked for by name (and clusters of two can be launched)
-bool use_pairs(const csk_moe_layer* L) { return L->pair.available && L->path == CSK_PATH_TILE_PAIR; }
+// MXFP4 runs on CTA pairs, fp16 weights on the one-CTA kernel
+bool use_pairs(const csk_moe_layer* L) { return !L->w16; }
 
 int tile_rows_for(const csk_moe_layer* L, int path) {
   return path == CSK_PATH_TILE ? (use_pairs(L) ? kPairN : kTileM) : kMxTileRows;
@@ -506,7 +506,7 @@ int launch_experts(csk_moe_layer* L, int path, float* y, int ldy, const int* out
   if (path == CSK_PATH_TILE) {
     int rc;
     if (use_pairs(L))
-      rc = pair_launch(L->pair, L->tile, L->tile.tmap_xh, L->tile.tmap_ah, L->d_weights, L->expert_stride, L->off_tgu,
+      rc = pair_launch(L->pair, L->tile, L->tile.pair_x, L->tile.pair_a, L->d_weights, L->expert_stride, L->off_tgu,
                        L->off_td, L->off_bias, L->off_meta, L->Tgu, L->Td, L->d_a16, L->lda, y, ldy, out_row_map,
                        out_row_ptr, L->d_tiles, L->d_meta, L->cfg.has_bias, L->cfg.activation, L->F, s,
                        [&]() { tm.mark(); }, L->debug_stall);
@@ -1199,6 +1199,28 @@ ImageHeader image_header_02(const csk_moe_layer* L) {
   h.expert_stride = (h.off_meta + 16 + 255) / 256 * 256;
   return h;
 }
+// An expert's tensor-core codes to the file's order (from the device into `dst`) or from it (from `src` to the device).
+int reorder_tiles_enqueue(csk_moe_layer* L, int le, uint8_t* part, bool to_file, cudaStream_t s) {
+  uint8_t* base = L->d_weights + (size_t)le * L->expert_stride + L->off_tgu;
+  for (const auto& [lay, at] : {std::pair{L->Tgu, (size_t)0}, std::pair{L->Td, L->off_td - L->off_tgu}})
+    k_reorder_tile<<<grid_for(lay.bytes() / 34, 256, 4096), 256, 0, s>>>(to_file ? base + at : part + at, to_file ? part + at : base + at, lay,
+                                                                       to_file);
+  CSK_CUDA(L, cudaGetLastError());
+  return CSK_OK;
+}
+// Device memory for one expert's tensor-core codes in the file's order, for the time of a save or a load.
+struct ImagePart {
+  uint8_t* p = nullptr;
+  size_t bytes = 0;
+  explicit ImagePart(const csk_moe_layer* L) : bytes(L->w16 ? 0 : L->off_bias - L->off_tgu) {
+    if (bytes && cudaMalloc(&p, bytes) != cudaSuccess) {
+      cudaGetLastError();
+      p = nullptr;
+    }
+  }
+  bool ok() const { return p || !bytes; }
+  ~ImagePart() { cudaFree(p); }
+};
 // The decode kernel's copy of a resident expert's codes from the other kernel's tiles (which hold the blocks losslessly).
 int rebuild_mx_enqueue(csk_moe_layer* L, int le, cudaStream_t s) {
   uint8_t* base = L->d_weights + (size_t)le * L->expert_stride;
@@ -1219,6 +1241,8 @@ int csk_moe_save_image(csk_moe_layer* L, const char* path) {
   if (check_layer(L)) return CSK_ERR_INVALID;
   if (!path) return fail(L, CSK_ERR_INVALID, "null path");
   CSK_CUDA(L, cudaSetDevice(L->cfg.device));
+  ImagePart part(L);
+  if (!part.ok()) return fail(L, CSK_ERR_NOMEM, "no device memory to write the weight image");
   FILE* f = fopen(path, "wb");
   if (!f) return fail(L, CSK_ERR_INVALID, "cannot open %s for writing", path);
   const ImageHeader h = image_header_of(L);
@@ -1226,6 +1250,10 @@ int csk_moe_save_image(csk_moe_layer* L, const char* path) {
   std::vector<uint8_t> buf(L->expert_stride);
   for (int e = 0; ok && e < L->Eloc; ++e) {
     if (cudaMemcpy(buf.data(), L->d_weights + (size_t)e * L->expert_stride, L->expert_stride, cudaMemcpyDeviceToHost) != cudaSuccess) ok = false;
+    if (ok && part.bytes) {
+      ok = reorder_tiles_enqueue(L, e, part.p, true, L->stream) == CSK_OK && cudaStreamSynchronize(L->stream) == cudaSuccess &&
+           cudaMemcpy(buf.data() + L->off_tgu, part.p, part.bytes, cudaMemcpyDeviceToHost) == cudaSuccess;
+    }
     ok = ok && fwrite(buf.data(), 1, buf.size(), f) == buf.size();
   }
   ok = fclose(f) == 0 && ok;
@@ -1237,6 +1265,8 @@ int csk_moe_load_image(csk_moe_layer* L, const char* path) {
   if (check_layer(L)) return CSK_ERR_INVALID;
   if (!path) return fail(L, CSK_ERR_INVALID, "null path");
   CSK_CUDA(L, cudaSetDevice(L->cfg.device));
+  ImagePart part(L);
+  if (!part.ok()) return fail(L, CSK_ERR_NOMEM, "no device memory to read the weight image");
   FILE* f = fopen(path, "rb");
   if (!f) return fail(L, CSK_ERR_INVALID, "cannot open %s", path);
   ImageHeader h{};
@@ -1257,6 +1287,9 @@ int csk_moe_load_image(csk_moe_layer* L, const char* path) {
     ok = fread(buf.data(), 1, buf.size(), f) == buf.size();
     // (on the handle's stream, which does not wait for the default one: a plain copy may still be landing when it returns)
     ok = ok && cudaMemcpyAsync(base + to, buf.data() + from, h.off_meta + 16 - from, cudaMemcpyHostToDevice, L->stream) == cudaSuccess;
+    if (ok && part.bytes)
+      ok = cudaMemcpyAsync(part.p, base + L->off_tgu, part.bytes, cudaMemcpyDeviceToDevice, L->stream) == cudaSuccess &&
+           reorder_tiles_enqueue(L, e, part.p, false, L->stream) == CSK_OK;
     if (ok && rebuild && res[e]) ok = rebuild_mx_enqueue(L, e, L->stream) == CSK_OK;
     ok = cudaStreamSynchronize(L->stream) == cudaSuccess && ok;
   }

@@ -1,5 +1,5 @@
-// Tensor-core grouped contraction over repacked MXFP4 weights (the prefill-side
-// kernel), written for sm_100a.
+// Tensor-core grouped contraction over fp16 weights (the dense FFN, fp16 expert slices), written for sm_100a, and the weight
+// layouts of both fp16-operand kernels.  (MXFP4 weights: csk_tile2.cuh.)
 //
 // The contraction is computed transposed, D[weight row, token] = W · Xᵀ, so that
 // the WEIGHTS are the tensor-memory operand of tcgen05.mma and only the token
@@ -10,36 +10,28 @@
 //     own row count rounded up to 16, so ragged expert sizes cost no padded
 //     tensor work, and every token tile fetched from L2 feeds 256 weight rows;
 //   * per 64-column k-step the producer warp issues one TMA tensor load of the
-//     192 x 64 fp16 token tile (128-byte swizzle) and one bulk copy of the packed
-//     weight tile (2 x 4352 bytes: codes + E8M0 scales, one contiguous span);
-//   * eight dequantiser warps in two groups of four turn the packed tile into fp16
-//     (cvt.e2m1x2 -> half2, times 2^(e - e_max + 13)) and write it straight into
+//     192 x 64 fp16 token tile (128-byte swizzle) and one bulk copy of the weight
+//     tile (2 x 16 KB);
+//   * eight copy warps in two groups of four write the weight tile into
 //     tensor memory with tcgen05.st: thread = one weight row x the 64 columns of
 //     the k-step, one half of the tile after the other.  The groups alternate
 //     k-steps and each owns one slot of the two-slot weight ring; the first half
-//     is converted before the slot is awaited.  The dequantised weights never
-//     touch shared memory.  (fp16 weights -- the dense FFN, fp16 expert slices --
-//     take the same route with a copy in place of the conversion.);
+//     is loaded before the slot is awaited;
 //   * the MMA warp runs its loop warp-wide with one elected lane issuing: per
 //     k-step ONE barrier test (the slot is full), then eight tcgen05.mma (kind::f16,
 //     A from tensor memory, B = the token tile via a shared-memory descriptor),
 //     four per half, into two fp32 accumulators in tensor memory, then one commit
 //     that releases both the shared-memory stage and the slot;
 //   * twelve epilogue warps (three per lane quarter) read the accumulators (lane =
-//     weight row, column = token), scale by the matrix's power of two, add the bias
+//     weight row, column = token), add the bias
 //     and either apply the gated activation (the gate and the up accumulator of a
 //     feature sit in the same lane, 192 columns apart; a warp finishes 64 token
 //     columns) and store fp16 rows, or (plain matrix: a warp finishes 128 of the
 //     two halves' 2 x 192 columns) store fp32 output rows.
 //
 // Tensor memory (512 columns): [0,384) the accumulators of the two halves, 192
-// columns each; [384,512) a ring of two dequantised weight tiles, 2 x 32 columns
+// columns each; [384,512) a ring of two weight tiles, 2 x 32 columns
 // (2 x 64 fp16 per row) each.
-//
-// fp16 operands: every MXFP4 value is value(E2M1) * 2^(e-127).  Within a matrix
-// the tile holds value * 2^(e - e_max + 13) (at most 6 * 2^13; exact in fp16
-// while e_max - e <= 36, smaller blocks lose bits below 2^-24 of that range) and
-// the accumulator is multiplied by 2^(e_max - 140) afterwards.
 //
 // Every wait on an mbarrier is bounded: past a clock budget the CTA records
 // kDevErrWaitTimeout in the status word, all roles leave their loops, copies in
@@ -59,9 +51,9 @@ namespace csk {
 
 constexpr int kTileM = 192;          // token rows of a row tile (TMA box height, MMA N <= 192)
 constexpr int kTileW = 128;          // weight rows of half a weight tile (tensor-memory lanes, MMA M)
-constexpr int kDequantWarps = 8;
+constexpr int kCopyWarps = 8;
 constexpr int kEpilogueWarps = 12;    // four lane quarters x three column ranges (sixteen measured no faster)
-constexpr int kTileThreads = (2 + kDequantWarps + kEpilogueWarps) * 32;  // producer, MMA, dequantisers, epilogue
+constexpr int kTileThreads = (2 + kCopyWarps + kEpilogueWarps) * 32;  // producer, MMA, weight copies, epilogue
 constexpr int kTileABytes = kTileM * 128;                   // token tile in shared memory
 constexpr int kTileBoxes = kTileM / 32;                     // TMA boxes of 32, 64, ... kTileM rows: a row tile is fetched
                                                             // with the smallest that holds it (a 128-row tile costs 16 KB
@@ -71,28 +63,35 @@ struct TileMaps {
 };
 constexpr int kHalfPacked = 4352;                           // packed half tile: 4096 codes + 256 scales
 constexpr int kTilePacked = 2 * kHalfPacked;                // packed weight tile (two halves)
-constexpr int kTileRawBytes = kTileABytes + 9216;           // one shared-memory stage (1024-byte multiple)
-constexpr int kTileStages = 6;
 // fp16 weights (dense FFN, fp16 expert slices): a half tile is 128 rows x 64 fp16 = 16 KB, rows of 128 bytes
 // whose eight 16-byte pieces are stored at piece ^ (row & 7) (a quarter-warp reading one piece of eight
 // neighbouring rows then hits eight different bank groups)
 constexpr int kHalf16 = 128 * 128;
 constexpr int kTile16 = 2 * kHalf16;
-constexpr int kTileRawBytes16 = kTileABytes + kTile16;      // 57344, a 1024-byte multiple
-constexpr int kTileStages16 = 3;
+constexpr int kTileRawBytes = kTileABytes + kTile16;        // one shared-memory stage: 57344, a 1024-byte multiple
+constexpr int kTileStages = 3;
 constexpr int kTileAStages = 2;                             // weight tiles resident in tensor memory
-constexpr int kPairBoxRows = 96;                            // TMA box height of the CTA-pair kernel's half tiles
+constexpr int kPairBoxes = 8;                               // the CTA-pair kernel's half tiles: boxes of 16, 32, ... 128 rows
+struct PairMaps {
+  CUtensorMap m[kPairBoxes];
+};
 constexpr uint32_t kTmemCols = 512;
 constexpr uint32_t kTmemABase = 2 * kTileM;                 // first column of the weight ring
 
-// Device layout of a matrix for this kernel: tiles of 256 rows x 64 columns,
-// stored [n_tile][k_tile]; a tile is two halves of 128 rows, 4352 bytes each:
+// Device layout of a matrix for the fp16 tensor-core kernels: tiles of 256 rows x 64 columns, as two halves of 128 rows.
+//
+// MXFP4 (the CTA-pair kernel, csk_tile2.cuh): [n_tile][half][k_tile], so that a CTA's half runs on along K; a half tile is
+// 4352 bytes,
 //   bytes    0..4095  codes: [column block 0/1][row 0..127][16 bytes = 32 codes, nibble i of
 //                     word w = column 8w + i]
 //   bytes 4096..4351  E8M0 scales: [column block][row]
-// For the fused gate/up matrix half 0 holds the gate rows and half 1 the up rows of the
-// SAME 128 features (128*n_tile ..), so a feature's two accumulators sit in one
+// Gate/up: half c holds the features 64c .. 64c+63 of the tile's 128, in groups of 16 gate and 16 up rows (a warp's lanes).
+//
+// fp16 (k_tile): [n_tile][k_tile][half], a half tile is 128 rows of 128 bytes.  Gate/up: half 0 holds the gate rows and half
+// 1 the up rows of the SAME 128 features (128*n_tile ..), so a feature's two accumulators sit in one
 // tensor-memory lane, 192 columns apart.
+//
+// In the file images MXFP4 codes keep fp16's order of tiles and rows (k_reorder_tile).
 struct TileLayout {
   int N, K, paired, n_tiles, k_tiles, w16;
   __host__ __device__ int half_bytes() const { return w16 ? kHalf16 : kHalfPacked; }
@@ -102,6 +101,13 @@ struct TileLayout {
   __host__ __device__ int halves(int nt) const { return paired || nt * 2 * kTileW + kTileW < N ? 2 : 1; }
   __host__ __device__ size_t bytes() const { return (size_t)n_tiles * k_tiles * tile_bytes(); }
   __host__ __device__ int k_pad() const { return k_tiles * kTileK; }
+  // where half tiles of MXFP4 codes lie, and which half and which of its rows row `feat` of the matrix (of its gate or,
+  // which = 1, its up matrix) is
+  __host__ __device__ size_t half_at(int nt, int half, int kt) const { return (((size_t)nt * 2 + half) * k_tiles + kt) * kHalfPacked; }
+  __host__ __device__ int half_of(int feat) const { return feat / (paired ? kTileW / 2 : kTileW) & 1; }
+  __host__ __device__ int row_of(int feat, int which) const {
+    return paired ? (feat % (kTileW / 2) & ~15) * 2 + which * 16 + (feat & 15) : feat % kTileW;
+  }
 };
 inline TileLayout make_tile_layout(int N, int K, bool paired, bool w16 = false) {
   TileLayout L{};
@@ -122,14 +128,12 @@ __global__ void k_repack_tile(const uint8_t* __restrict__ src0, const uint8_t* _
   for (size_t w = (size_t)blockIdx.x * blockDim.x + threadIdx.x; w < n_words; w += (size_t)gridDim.x * blockDim.x) {
     const size_t half_idx = w / WPT;
     const int wi = (int)(w % WPT);
-    const int half = (int)(half_idx & 1);
-    const size_t tile = half_idx >> 1;
-    const int kt = (int)(tile % L.k_tiles), nt = (int)(tile / L.k_tiles);
+    const int kt = (int)(half_idx % L.k_tiles), half = (int)(half_idx / L.k_tiles & 1), nt = (int)(half_idx / (2 * L.k_tiles));
     uint32_t out = 0;
     auto source = [&](int trow, const uint8_t*& src, int& feat) {
       if (L.paired) {
-        src = half ? src1 : src0;
-        feat = nt * kTileW + trow;
+        src = trow & 16 ? src1 : src0;
+        feat = nt * kTileW + half * (kTileW / 2) + (trow >> 5) * 16 + (trow & 15);
       } else {
         src = src0;
         feat = nt * 2 * kTileW + half * kTileW + trow;
@@ -204,11 +208,9 @@ __global__ void k_unpack_tile(const uint8_t* __restrict__ packed, uint8_t* __res
   const size_t n_blocks = (size_t)L.N * kb;
   for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n_blocks; i += (size_t)gridDim.x * blockDim.x) {
     const int feat = (int)(i / kb), blk_g = (int)(i % kb);
-    const int nt = feat / L.feats_per_tile();
-    const int half = L.paired ? which_half : (feat % (2 * kTileW)) / kTileW;
-    const int trow = feat % kTileW;
+    const int nt = feat / L.feats_per_tile(), trow = L.row_of(feat, which_half);
     const int kt = blk_g / 2, blk = blk_g & 1;
-    const uint8_t* tile = packed + ((size_t)nt * L.k_tiles + kt) * kTilePacked + (size_t)half * kHalfPacked;
+    const uint8_t* tile = packed + L.half_at(nt, L.half_of(feat), kt);
     uint8_t* o = out + i * 17;
     o[0] = tile[4096 + blk * 128 + trow];
     const uint32_t* words = reinterpret_cast<const uint32_t*>(tile + ((size_t)blk * 128 + trow) * 16);
@@ -219,13 +221,33 @@ __global__ void k_unpack_tile(const uint8_t* __restrict__ packed, uint8_t* __res
   }
 }
 
+// MXFP4 codes from the device's order of tiles and rows to that of the file images ([n_tile][k_tile][half]; gate/up: half 0 the
+// gate, half 1 the up rows of 128 features) or back.  One thread per row of a half tile.
+__global__ void k_reorder_tile(const uint8_t* __restrict__ src, uint8_t* __restrict__ dst, TileLayout L, int to_file) {
+  const size_t n = (size_t)L.n_tiles * 2 * L.k_tiles * kTileW;
+  for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
+    const int r = (int)(i % kTileW), kt = (int)(i / kTileW % L.k_tiles);
+    const int half = (int)(i / ((size_t)kTileW * L.k_tiles) & 1), nt = (int)(i / ((size_t)2 * kTileW * L.k_tiles));
+    const int file_half = L.paired ? r >> 4 & 1 : half, file_row = L.paired ? half * 64 + (r >> 5) * 16 + (r & 15) : r;
+    const size_t here = L.half_at(nt, half, kt), file = (((size_t)nt * L.k_tiles + kt) * 2 + file_half) * kHalfPacked;
+    const uint8_t* s = src + (to_file ? here : file);
+    uint8_t* d = dst + (to_file ? file : here);
+    const int sr = to_file ? r : file_row, dr = to_file ? file_row : r;
+#pragma unroll
+    for (int blk = 0; blk < 2; ++blk) {
+      *reinterpret_cast<uint4*>(d + (blk * 128 + dr) * 16) = *reinterpret_cast<const uint4*>(s + (blk * 128 + sr) * 16);
+      d[4096 + blk * 128 + dr] = s[4096 + blk * 128 + sr];
+    }
+  }
+}
+
 struct TileState {
   bool available = false;
   std::string err;
   TileMaps maps_x{};      // grouped input rows  [rows, ldx] fp16, one map per box height
   TileMaps maps_a{};      // activated rows      [rows, lda] fp16
-  CUtensorMap tmap_xh{};  // the same with boxes of half a row tile (the CTA-pair kernel's half tiles)
-  CUtensorMap tmap_ah{};
+  PairMaps pair_x{};      // the same for the CTA-pair kernel's half tiles
+  PairMaps pair_a{};
   bool maps_ready = false;
   void* encode_fn = nullptr;
 };
@@ -259,19 +281,17 @@ struct TileArgs {
   int stall;              // test hook: the copy role issues nothing, so every other role's wait runs out
 };
 
-inline size_t tile_smem_bytes(bool w16 = false) {
-  return (w16 ? (size_t)kTileStages16 * kTileRawBytes16 : (size_t)kTileStages * kTileRawBytes) + 1024 + 512;
-}
+inline size_t tile_smem_bytes() { return (size_t)kTileStages * kTileRawBytes + 1024 + 512; }
 
-template <bool GATED, bool W16>
+template <bool GATED>
 __global__ void __launch_bounds__(kTileThreads, 1)
 k_tile(const __grid_constant__ TileMaps maps, const TileArgs A) {
   extern __shared__ __align__(1024) uint8_t tile_smem[];
   const TileLayout& L = A.L;
   const int KT = L.k_tiles;
-  constexpr int NR = W16 ? kTileStages16 : kTileStages, NA = kTileAStages;
-  constexpr int RAW = W16 ? kTileRawBytes16 : kTileRawBytes;  // bytes of a shared-memory stage
-  constexpr int HALF_B = W16 ? kHalf16 : kHalfPacked, TILE_B = 2 * HALF_B;
+  constexpr int NR = kTileStages, NA = kTileAStages;
+  constexpr int RAW = kTileRawBytes;  // bytes of a shared-memory stage
+  constexpr int HALF_B = kHalf16, TILE_B = kTile16;
 
   uint8_t* smem = reinterpret_cast<uint8_t*>(((uintptr_t)tile_smem + 1023) & ~(uintptr_t)1023);
   const uint32_t smem_base = smem_u32(smem);  // ring of [token tile | packed weight tile]
@@ -279,7 +299,7 @@ k_tile(const __grid_constant__ TileMaps maps, const TileArgs A) {
   uint64_t* bars = reinterpret_cast<uint64_t*>(ctrl);
   const uint32_t bar_base = smem_u32(bars);
   // k-step c uses shared-memory stage c % NR and tensor-memory slot c % NA; one barrier per stage tells both the
-  // copy role (stage free) and the dequantisers (slot of k-step c - NA free) that its MMAs have retired
+  // copy role (stage free) and the weight copies (slot of k-step c - NA free) that its MMAs have retired
   auto bar_full_raw = [&](int s) { return bar_base + 8u * s; };               // TMA landed
   auto bar_retired = [&](int s) { return bar_base + 8u * (8 + s); };          // MMAs of the k-step in that stage retired
   auto bar_full_a = [&](int s) { return bar_base + 8u * (16 + s); };          // both halves of the slot are in tensor memory
@@ -296,7 +316,7 @@ k_tile(const __grid_constant__ TileMaps maps, const TileArgs A) {
       mbar_init(bar_full_raw(s), 1);
       mbar_init(bar_retired(s), 1);
     }
-    for (int s = 0; s < NA; ++s) mbar_init(bar_full_a(s), kDequantWarps / 2);
+    for (int s = 0; s < NA; ++s) mbar_init(bar_full_a(s), kCopyWarps / 2);
     mbar_init(bar_tmem_full, 1);
     mbar_init(bar_tmem_empty, kEpilogueWarps);
     mbar_init(bar_drain, 1);
@@ -334,7 +354,7 @@ k_tile(const __grid_constant__ TileMaps maps, const TileArgs A) {
         const CUtensorMap* tmap = &maps.m[box];
         const uint32_t box_bytes = (uint32_t)(box + 1) * 32u * 128u;
         for (int kt = 0; kt < KT; ++kt) {
-          if (!mbar_wait(bar_retired(s), ph ^ 1, abort_flag)) {
+          if (!mbar_wait_here(bar_retired(s), ph ^ 1, abort_flag)) {
             ok = false;
             break;
           }
@@ -371,7 +391,7 @@ k_tile(const __grid_constant__ TileMaps maps, const TileArgs A) {
     // branch) every descriptor and address has to be moved across for every instruction, and a K=16 MMA
     // then issues once per ~185 clocks whatever its shape (measured; the pipe needs 96 for 128 x 192 x 16).
     // The loop is also kept to ONE barrier test per k-step (a satisfied test still costs ~110 clocks): the
-    // token tile of a stage needs no test of its own, because the dequantisers waited for the same stage's
+    // token tile of a stage needs no test of its own, because the weight copies waited for the same stage's
     // copies before they wrote the slot this warp waits for.  Both halves' MMAs are always issued; a half
     // that is padding (the last weight tile of a plain matrix) accumulates into columns nobody reads.
     {
@@ -384,12 +404,12 @@ k_tile(const __grid_constant__ TileMaps maps, const TileArgs A) {
         const RowTile rt = A.tiles[item / L.n_tiles];
         const int n_mma = max(16, (rt.rows + 15) & ~15);
         const uint32_t idesc = umma_idesc_f16(n_mma);
-        ok = mbar_wait_warp(bar_tmem_empty, (it & 1u) ^ 1u, abort_flag);
+        ok = __all_sync(0xffffffffu, mbar_wait_here(bar_tmem_empty, (it & 1u) ^ 1u, abort_flag));
         if (!ok) break;
         tc_fence_after();
         for (int kt = 0; kt < KT; ++kt, ++c) {
           const uint32_t s = c % NR, sa = c % NA;
-          ok = mbar_wait_warp(bar_full_a(sa), (c / NA) & 1u, abort_flag);
+          ok = __all_sync(0xffffffffu, mbar_wait_here(bar_full_a(sa), (c / NA) & 1u, abort_flag));
           if (!ok) break;
           tc_fence_after();
           const uint64_t db = db0 + (uint64_t)((s * (uint32_t)RAW) >> 4);  // start-address field, 16-byte units
@@ -416,54 +436,29 @@ k_tile(const __grid_constant__ TileMaps maps, const TileArgs A) {
       }
       __syncwarp();
     }
-  } else if (warp < 2 + kDequantWarps) {
-    // ------------------------------ dequantisers ------------------------------
-    // Two groups of four warps; group g converts the k-steps whose running number is g mod 2
+  } else if (warp < 2 + kCopyWarps) {
+    // ------------------------------ weight copies ------------------------------
+    // Two groups of four warps; group g copies the k-steps whose running number is g mod 2
     // and owns slot g of the tensor-memory weight ring.  thread = weight row (tensor-memory
     // lane) x the 64 columns of the k-step, one half after the other: the first half is
-    // converted BEFORE the slot is awaited (so only the store is on the slot's critical path),
+    // loaded BEFORE the slot is awaited (so only the store is on the slot's critical path),
     // the second while the MMAs of the first run.
     const int quarter = warp & 3;            // lanes 32*quarter .. +31 are this warp's
     const int grp = (warp - 2) >> 2;         // which k-steps / which slot
     const int trow = quarter * 32 + lane;
     long c = 0;                              // running k-step number of this CTA
     bool ok = true;
-    auto convert = [&](const uint8_t* packed, int emax, uint32_t (&h)[2][16]) {
-      if (W16) {  // the row's 64 fp16 values as they are: eight 16-byte pieces, stored at piece ^ (row & 7)
-        const uint8_t* row = packed + trow * 128;
+    auto load = [&](const uint8_t* half, uint32_t (&h)[2][16]) {  // the row's 64 values: eight 16-byte pieces, stored at piece ^ (row & 7)
+      const uint8_t* row = half + trow * 128;
 #pragma unroll
-        for (int j = 0; j < 8; ++j) {
-          const uint4 v = *reinterpret_cast<const uint4*>(row + ((j ^ (trow & 7)) << 4));
-          h[j >> 2][(j & 3) * 4 + 0] = v.x;
-          h[j >> 2][(j & 3) * 4 + 1] = v.y;
-          h[j >> 2][(j & 3) * 4 + 2] = v.z;
-          h[j >> 2][(j & 3) * 4 + 3] = v.w;
-        }
-        return;
-      }
-#pragma unroll
-      for (int blk = 0; blk < 2; ++blk) {
-        const uint4 cw = *reinterpret_cast<const uint4*>(packed + (blk * 128 + trow) * 16);
-        const int e = min((int)packed[4096 + blk * 128 + trow], 254);  // scale byte 255 is read as 254
-        const uint32_t sh2 = h2_pow2(e - emax + 13);
-        uint32_t t[4];
-        dequant_word(cw.x, t);
-        h[blk][0] = t[0]; h[blk][1] = t[1]; h[blk][2] = t[2]; h[blk][3] = t[3];
-        dequant_word(cw.y, t);
-        h[blk][4] = t[0]; h[blk][5] = t[1]; h[blk][6] = t[2]; h[blk][7] = t[3];
-        dequant_word(cw.z, t);
-        h[blk][8] = t[0]; h[blk][9] = t[1]; h[blk][10] = t[2]; h[blk][11] = t[3];
-        dequant_word(cw.w, t);
-        h[blk][12] = t[0]; h[blk][13] = t[1]; h[blk][14] = t[2]; h[blk][15] = t[3];
-#pragma unroll
-        for (int i = 0; i < 16; ++i) h[blk][i] = hmul2_u32(h[blk][i], sh2);
+      for (int j = 0; j < 8; ++j) {
+        const uint4 v = *reinterpret_cast<const uint4*>(row + ((j ^ (trow & 7)) << 4));
+        uint32_t* d = &h[j >> 2][4 * (j & 3)];
+        d[0] = v.x; d[1] = v.y; d[2] = v.z; d[3] = v.w;
       }
     };
     for (long item = blockIdx.x; ok && item < n_items; item += gridDim.x) {
-      const RowTile rt = A.tiles[item / L.n_tiles];
       const int halves = L.halves((int)(item % L.n_tiles));
-      const int* emeta = reinterpret_cast<const int*>(A.weights + (size_t)rt.expert * A.expert_stride + A.meta_offset);
-      const int emax = emeta[A.meta_slot];
       // A wait that ran out in some lanes must not part them in front of the warp-wide stores: all of them go through the
       // unit's remaining k-steps (the flag ends every further wait at once, nobody uses the tile) and agree afterwards.
       // A vote per k-step costs 1 to 2 % of the kernel.
@@ -472,32 +467,30 @@ k_tile(const __grid_constant__ TileMaps maps, const TileArgs A) {
         if ((int)(c & 1) != grp) continue;
         const int s = (int)(c % NR);
         const uint32_t ph = (uint32_t)((c / NR) & 1);
-        if (NR % 2 != 0 && c >= NR) {
+        if (c >= NR) {
           // An odd ring hands a stage to the two groups in turn, so this group never saw the stage's previous
           // fill complete: were that fill still in flight (copies may complete out of order), the parity test
-          // below would take the fill before it for the one awaited, and the conversion would read the
+          // below would take the fill before it for the one awaited, and the loads would read the
           // wrong k-step.  The stage's previous MMAs having retired implies its previous fill has landed.
-          landed = mbar_wait(bar_retired(s), (uint32_t)(((c - NR) / NR) & 1), abort_flag) && landed;
+          landed = mbar_wait_here(bar_retired(s), (uint32_t)(((c - NR) / NR) & 1), abort_flag) && landed;
         }
-        landed = mbar_wait(bar_full_raw(s), ph, abort_flag) && landed;
+        landed = mbar_wait_here(bar_full_raw(s), ph, abort_flag) && landed;
         const uint8_t* packed = smem + (size_t)s * RAW + kTileABytes;
         const int sa = (int)(c % NA);
         const uint32_t t_slot = tmem_base + ((uint32_t)(quarter * 32) << 16) + kTmemABase + (uint32_t)sa * 64;
         uint32_t h[2][16];
-        convert(packed, emax, h);
+        load(packed, h);
         // the slot was last read by k-step c - NA
-        if (c >= NA) landed = mbar_wait(bar_retired((int)((c - NA) % NR)), (uint32_t)(((c - NA) / NR) & 1), abort_flag) && landed;
+        if (c >= NA) landed = mbar_wait_here(bar_retired((int)((c - NA) % NR)), (uint32_t)(((c - NA) / NR) & 1), abort_flag) && landed;
         tc_fence_after();
         tmem_st16(t_slot, h[0]);
         tmem_st16(t_slot + 16, h[1]);
         if (halves > 1) {
           // h is reused: the stores above read their registers asynchronously, so they have to be waited for
-          // before the registers change (with fp16 weights the second conversion is only eight loads, and
-          // without this wait rows of the first half were occasionally stored with the second half's values).
-          // Converting both halves ahead of the slot wait (64 registers), or giving each thread half a row
-          // of both halves (sixteen dequantiser warps), both measured slower than this.
+          // before the registers change (without this wait rows of the first half were occasionally stored with the
+          // second half's values).
           tmem_st_wait();
-          convert(packed + HALF_B, emax, h);
+          load(packed + HALF_B, h);
           tmem_st16(t_slot + 32, h[0]);
           tmem_st16(t_slot + 48, h[1]);
         }
@@ -511,7 +504,7 @@ k_tile(const __grid_constant__ TileMaps maps, const TileArgs A) {
   } else {
     // ------------------------------ epilogue ------------------------------
     const int quarter = warp & 3;  // tensor-memory lanes 32*quarter .. +31 belong to this warp
-    const int ew = warp - 2 - kDequantWarps;
+    const int ew = warp - 2 - kCopyWarps;
     // three warps per lane quarter.  gate/up: both halves (gate and up of its lane's feature) x one of three
     // 64-column ranges.  Plain matrix: the two halves' columns laid end to end (2 x 192) x one of three
     // 128-column ranges, walked in steps of 32 that never straddle the halves.
@@ -528,9 +521,7 @@ k_tile(const __grid_constant__ TileMaps maps, const TileArgs A) {
       const int halves = L.halves(nt);
       const uint8_t* ebase = A.weights + (size_t)rt.expert * A.expert_stride;
       const float* bias = reinterpret_cast<const float*>(ebase + A.bias_offset);
-      const int emax = reinterpret_cast<const int*>(ebase + A.meta_offset)[A.meta_slot];
-      const float oscale = W16 ? 1.0f : ldexpf(1.0f, emax - 140);
-      if (!mbar_wait_warp(bar_tmem_full, (uint32_t)(it & 1), abort_flag)) {
+      if (!__all_sync(0xffffffffu, mbar_wait_here(bar_tmem_full, (uint32_t)(it & 1), abort_flag))) {
         ok = false;
         break;
       }
@@ -554,8 +545,8 @@ k_tile(const __grid_constant__ TileMaps maps, const TileArgs A) {
           // two columns at a time: one packed conversion (an ALU instruction) instead of two single ones
 #pragma unroll
           for (int j = 0; j < 16; j += 2) {
-            const float g0 = fmaf(__uint_as_float(rg[j]), oscale, bg), u0 = fmaf(__uint_as_float(ru[j]), oscale, bu);
-            const float g1 = fmaf(__uint_as_float(rg[j + 1]), oscale, bg), u1 = fmaf(__uint_as_float(ru[j + 1]), oscale, bu);
+            const float g0 = __uint_as_float(rg[j]) + bg, u0 = __uint_as_float(ru[j]) + bu;
+            const float g1 = __uint_as_float(rg[j + 1]) + bg, u1 = __uint_as_float(ru[j + 1]) + bu;
             const __half2 a = __floats2half2_rn(gated_act_fast(g0, u0, A.act), gated_act_fast(g1, u1, A.act));
             if (feat_ok && c0 + j < rt.rows) out[(size_t)(c0 + j) * A.lda] = __low2half(a);
             if (feat_ok && c0 + j + 1 < rt.rows) out[(size_t)(c0 + j + 1) * A.lda] = __high2half(a);
@@ -582,7 +573,7 @@ k_tile(const __grid_constant__ TileMaps maps, const TileArgs A) {
 #pragma unroll
           for (int j = 0; j < 32; ++j) {
             float* row = reinterpret_cast<float*>(__shfl_sync(0xffffffffu, my_bits, j));
-            if (n_ok && row && c0 + j < rt.rows) row[n] = __uint_as_float(r[j]) * oscale + my_bias;
+            if (n_ok && row && c0 + j < rt.rows) row[n] = __uint_as_float(r[j]) + my_bias;
           }
         }
       }
@@ -619,14 +610,10 @@ inline int tile_init(TileState& st, int device) {
     return CSK_ERR_CUDA;
   }
   st.encode_fn = fn;
-  for (int w16 = 0; w16 < 2; ++w16) {
-    const void* fs[2] = {w16 ? (const void*)k_tile<true, true> : (const void*)k_tile<true, false>,
-                         w16 ? (const void*)k_tile<false, true> : (const void*)k_tile<false, false>};
-    for (const void* f : fs) {
-      if (cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tile_smem_bytes(w16 != 0)) != cudaSuccess) {
-        st.err = std::string("cudaFuncSetAttribute: ") + cudaGetErrorString(cudaGetLastError());
-        return CSK_ERR_CUDA;
-      }
+  for (const void* f : {(const void*)k_tile<true>, (const void*)k_tile<false>}) {
+    if (cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tile_smem_bytes()) != cudaSuccess) {
+      st.err = std::string("cudaFuncSetAttribute: ") + cudaGetErrorString(cudaGetLastError());
+      return CSK_ERR_CUDA;
     }
   }
   st.available = true;
@@ -657,8 +644,10 @@ inline int tile_set_buffers(TileState& st, const __half* x16, int ldx, const __h
     rc = tile_make_map(st, &st.maps_x.m[b], x16, rows_alloc, ldx, 32 * (b + 1));
     if (!rc) rc = tile_make_map(st, &st.maps_a.m[b], a16, rows_alloc, lda, 32 * (b + 1));
   }
-  if (!rc) rc = tile_make_map(st, &st.tmap_xh, x16, rows_alloc, ldx, kPairBoxRows);
-  if (!rc) rc = tile_make_map(st, &st.tmap_ah, a16, rows_alloc, lda, kPairBoxRows);
+  for (int b = 0; b < kPairBoxes && !rc; ++b) {
+    rc = tile_make_map(st, &st.pair_x.m[b], x16, rows_alloc, ldx, 16 * (b + 1));
+    if (!rc) rc = tile_make_map(st, &st.pair_a.m[b], a16, rows_alloc, lda, 16 * (b + 1));
+  }
   if (rc) return rc;
   st.maps_ready = true;
   return CSK_OK;
@@ -686,16 +675,14 @@ inline int tile_launch(TileState& st, const uint8_t* weights, size_t expert_stri
   a.act = act;
   a.F = F;
   a.stall = stall ? 1 : 0;
-  const bool w16 = Lgu.w16 != 0;
-  const size_t smem = tile_smem_bytes(w16);
+  const size_t smem = tile_smem_bytes();
   // gate/up + activation
   a.mat_offset = off_gu;
   a.L = Lgu;
   a.a_out = a16;
   a.lda = lda;
   a.meta_slot = 0;
-  if (w16) k_tile<true, true><<<sm_count, kTileThreads, smem, s>>>(st.maps_x, a);
-  else k_tile<true, false><<<sm_count, kTileThreads, smem, s>>>(st.maps_x, a);
+  k_tile<true><<<sm_count, kTileThreads, smem, s>>>(st.maps_x, a);
   mark();
   // down
   a.mat_offset = off_d;
@@ -705,8 +692,7 @@ inline int tile_launch(TileState& st, const uint8_t* weights, size_t expert_stri
   a.out_row_map = out_row_map;
   a.out_row_ptr = out_row_ptr;
   a.meta_slot = 1;
-  if (w16) k_tile<false, true><<<sm_count, kTileThreads, smem, s>>>(st.maps_a, a);
-  else k_tile<false, false><<<sm_count, kTileThreads, smem, s>>>(st.maps_a, a);
+  k_tile<false><<<sm_count, kTileThreads, smem, s>>>(st.maps_a, a);
   mark();
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) {

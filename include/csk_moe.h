@@ -49,8 +49,8 @@ enum { CSK_ACT_MODIFIED_SWIGLU = 0, CSK_ACT_STANDARD_SWIGLU = 1 };
 enum {
   CSK_PATH_AUTO = 0,
   CSK_PATH_STREAM = 1,      /* weight-streaming kernel (few rows per expert)                    */
-  CSK_PATH_TILE = 2,        /* tensor-core kernel, one CTA per work item                        */
-  CSK_PATH_TILE_PAIR = 3    /* tensor-core kernel on CTA pairs (cta_group::2); needs cluster launch */
+  CSK_PATH_TILE = 2,        /* fp16 tensor-core kernel: MXFP4 weights on CTA pairs, fp16 weights one CTA per work item */
+  CSK_PATH_TILE_PAIR = 3    /* the same, for MXFP4 layers only                                   */
 };
 
 /* Layer description: graph_builder::config num_experts / expert_top_k /
