@@ -10,6 +10,7 @@
 
 #include "csk_common.cuh"
 #include "csk_kernels.cuh"
+#include "csk_few16.cuh"
 #include "csk_kquant.cuh"
 #include "csk_mx.cuh"
 #include "csk_router_tc.cuh"
@@ -502,8 +503,41 @@ int tile_rows_for(const csk_moe_layer* L, int path) {
 // grouped gate/up + activation + down over the row tiles listed in d_tiles; the grouped rows are in d_x16 (tensor-core
 // path) or in d_ximg (streaming path); output rows go to y (through out_row_map or out_row_ptr if set)
 int launch_experts(csk_moe_layer* L, int path, float* y, int ldy, const int* out_row_map, cudaStream_t s, StageTimer& tm,
-                   float* const* out_row_ptr = nullptr) {
-  if (path == CSK_PATH_TILE) {
+                   float* const* out_row_ptr = nullptr, int64_t most_rows = INT64_MAX) {
+  // Few rows per expert: the weights' bytes are all that counts (csk_few16.cuh).  Step, k_tile / k_few16, us: dense FFN of 2880 x
+  // 2880 (weights in L2) 1 token 41 / 15, 16 43 / 17, 32 45 / 25, 48 48 / 39, 64 51 / 41; 16 experts of 2048 x 2048 beside a
+  // shared one 1 token 72 / 39, 5 85 / 62, 16 114 / 103, 32 120 / 145 (most experts are hit, by two rows each).
+  if (path == CSK_PATH_TILE && L->w16 && most_rows <= (L->Eloc == 1 ? kFewMaxRows : kFewMaxRowsRouted) && !L->debug_stall) {
+    FewArgs f{};
+    f.x = L->d_x16;
+    f.ldx = L->ldx;
+    f.one_expert = L->Eloc == 1;
+    TileArgs& a = f.t;
+    a.weights = L->d_weights;
+    a.expert_stride = L->expert_stride;
+    a.bias_offset = L->off_bias;
+    a.tiles = L->d_tiles;
+    a.n_tiles_ptr = a.meta = L->d_meta;
+    a.has_bias = L->cfg.has_bias;
+    a.act = L->cfg.activation;
+    a.F = L->F;
+    a.mat_offset = L->off_tgu;
+    a.L = L->Tgu;
+    a.a_out = L->d_a16;
+    a.lda = L->lda;
+    const int tiles = (int)std::min<int64_t>(L->Eloc, most_rows * L->k);
+    CSK_CUDA(L, few_launch_one<true>(f, L->F, tiles, (int)most_rows, s, L->pdl));
+    tm.mark();
+    f.x = L->d_a16;
+    f.ldx = L->lda;
+    a.mat_offset = L->off_td;
+    a.L = L->Td;
+    a.y_out = y;
+    a.ldy = ldy;
+    CSK_CUDA(L, few_launch_one<false>(f, L->H, tiles, (int)most_rows, s, L->pdl));
+    tm.mark();
+    L->last.launches += 2;
+  } else if (path == CSK_PATH_TILE) {
     int rc;
     if (use_pairs(L))
       rc = pair_launch(L->pair, L->tile, L->tile.pair_x, L->tile.pair_a, L->d_weights, L->expert_stride, L->off_tgu,
@@ -610,7 +644,7 @@ int forward_dev(csk_moe_layer* L, const float* d_hidden, int64_t T, const float*
     CSK_CUDA(L, cudaGetLastError());
     L->last.launches++;
     tm.mark();
-    int rc = launch_experts(L, path, d_out, L->H, nullptr, s, tm);
+    int rc = launch_experts(L, path, d_out, L->H, nullptr, s, tm, nullptr, T);
     if (rc) return rc;
     tm.mark();  // nothing to combine
     L->n_marks = tm.n;
@@ -626,7 +660,7 @@ int forward_dev(csk_moe_layer* L, const float* d_hidden, int64_t T, const float*
                           mx ? L->mx_rows : L->max_rows, s);
   if (rc) return rc;
   tm.mark();
-  rc = launch_experts(L, path, L->d_y, L->H, nullptr, s, tm);
+  rc = launch_experts(L, path, L->d_y, L->H, nullptr, s, tm, nullptr, T);
   if (rc) return rc;
   // the shared expert's rows come from another stream: the combine is the first kernel that reads them
   if (shared_ready) CSK_CUDA(L, cudaStreamWaitEvent(s, shared_ready, 0));
@@ -823,6 +857,7 @@ int csk_moe_create(const csk_moe_config* cfg, csk_moe_layer** out) {
   CK(cudaMallocHost(&L->h_counts64, sizeof(int64_t) * L->E));
   CK(router_prepare_device());
   CK(mx_prepare_device());
+  CK(few_prepare_device());
   CK(rt_prepare_device());
   {
     int rc = tile_init(L->tile, cfg->device);

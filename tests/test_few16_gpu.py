@@ -1,0 +1,52 @@
+"""fp16 weights on few token rows (the streaming kernel of the dense FFN and of fp16 experts) at the ends of its row groups,
+k-tiles and warps, against the CPU restatement of the reference; and the first batch of the kernel after it."""
+import numpy as np
+import pytest
+
+from coalsack_b200 import MoeLayer, dense_ffn_node, synth
+from tests import cases
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("T", [1, 8, 9, 16, 17, 32, 33, 64, 65])
+@pytest.mark.parametrize("H,F,bias", [
+    (32, 96, True),       # one k-tile of which half is padding: seven of eight warps idle
+    (544, 160, False),    # nine k-tiles (the warps' second turn) and three
+    (1088, 2080, True),   # seventeen and thirty-three: the third and fifth turn
+])
+def test_dense(gpu_lib, port, H, F, bias, T):
+    hidden, gw, uw, dw, bg, bu, bd = cases.dense_ffn_case(H=H, F=F, T=T, bias=True, seed=700 + T)
+    biases = [bg, bu, bd] if bias else []
+    node = dense_ffn_node()
+    out = node.compute([hidden[None], gw, uw, dw] + biases)[0]
+    mx, mr = cases.err_stats(out, port.dense_ffn(hidden, gw, uw, dw, *(biases or [None] * 3)))
+    assert mx <= cases.MAX_ABS_OVER_RMS and mr <= cases.MEAN_REL, (mx, mr)
+    assert np.array_equal(out, node.compute([hidden[None], gw, uw, dw] + biases)[0])
+    node.close()
+
+
+@pytest.mark.parametrize("E,k,T", [(5, 1, 3), (5, 2, 20), (40, 4, 64)])
+def test_experts(gpu_lib, port, E, k, T):
+    """Routed fp16 experts: more tiles than rows and fewer, experts without rows, a row that is not finite touches no other."""
+    H, F = 288, 160
+    rng = np.random.default_rng(E + T)
+    hidden = rng.standard_normal((T, H)).astype(np.float32)
+    experts = [cases.dense_ffn_case(H=H, F=F, T=1, bias=True, seed=900 + e)[1:] for e in range(E)]
+    lay = MoeLayer(E, k, H, F, activation=synth.STANDARD_SWIGLU, has_bias=True, max_tokens=T, weights_f16=True)
+    lay.set_router((rng.standard_normal((E, H)) * 0.3).astype(np.float32), None)
+    for e, (gw, uw, dw, bg, bu, bd) in enumerate(experts):
+        lay.load_expert_f16(e, uw, gw, dw, bu, bg, bd)
+    out, ro = lay.forward(hidden)
+    dense = [port.dense_ffn(hidden, *w) for w in experts]
+    want = np.zeros((T, H), np.float32)
+    for j in range(k):
+        want += ro[:, j, 1:] * np.stack([dense[int(e)][t] for t, e in enumerate(ro[:, j, 0])])
+    mx, mr = cases.err_stats(out, want)
+    assert mx <= cases.MAX_ABS_OVER_RMS and mr <= cases.MEAN_REL, (mx, mr)
+    bad = hidden.copy()
+    bad[T // 2, 5] = np.inf
+    got, _ = lay.forward(bad, router_out=ro)
+    keep = np.arange(T) != T // 2
+    assert np.array_equal(got[keep], out[keep]) and not np.isfinite(got[T // 2]).any()
+    lay.close()
