@@ -58,8 +58,9 @@ __global__ void k_pack_router(const float* __restrict__ wg, float* __restrict__ 
 // Top-k of one token's logits by one warp, then softmax over the selected
 // logits (or sigmoid) exactly as the reference (moe_router_node.h:165-214).
 // The logits sit in registers (lane l holds experts l, l+32, ...); each of the
-// k rounds is an arg-max by shuffles (ties -> lower expert id; the reference
-// leaves ties unspecified).
+// k rounds is an arg-max over the warp (ties -> lower expert id; the reference
+// leaves ties unspecified).  Lane j keeps the j-th selection: with all of them in one lane's arrays (local memory), ten
+// shuffles a round and the softmax in one lane a token took 3 us more.
 //
 // With `bounds` (the logits then come from a fast kernel, see k_router_fast) the
 // selection is CERTIFIED only if every gap between neighbours of the k best logits
@@ -80,9 +81,10 @@ __device__ __forceinline__ bool warp_topk_nv(const float* __restrict__ l, int E,
 #pragma unroll
   for (int i = 0; i < NV; ++i)
     v[i] = (i * 32 < E && i * 32 + lane < E) ? (CG ? __ldcg(l + i * 32 + lane) : l[i * 32 + lane]) : -INFINITY;
-  float sel_v[kMaxTopK];
-  int sel_i[kMaxTopK];
+  float my_v = -INFINITY;
+  int my_i = 0x7fffffff;
   uint32_t gone = 0;
+#pragma unroll 1
   for (int j = 0; j < k; ++j) {
     float bv = -INFINITY;
     int bi = 0x7fffffff;
@@ -96,16 +98,15 @@ __device__ __forceinline__ bool warp_topk_nv(const float* __restrict__ l, int E,
         }
       }
     }
-    for (int o = 16; o > 0; o >>= 1) {
-      const float ov = __shfl_xor_sync(0xffffffffu, bv, o);
-      const int oi = __shfl_xor_sync(0xffffffffu, bi, o);
-      if (ov > bv || (ov == bv && oi < bi)) {
-        bv = ov;
-        bi = oi;
-      }
+    // the lanes' bests as integers of the same order (both zeros alike), the lowest id of those that reach the maximum
+    const uint32_t bits = __float_as_uint(bv + 0.f), key = bits ^ ((int)bits < 0 ? 0xffffffffu : 0x80000000u);
+    const uint32_t top = __reduce_max_sync(0xffffffffu, key);
+    bi = (int)__reduce_min_sync(0xffffffffu, key == top ? (uint32_t)bi : 0x7fffffffu);
+    bv = __shfl_sync(0xffffffffu, bv, bi & 31);  // (nothing to choose from: -inf in every lane)
+    if (lane == j) {
+      my_v = bv;
+      my_i = bi;
     }
-    sel_v[j] = bv;
-    sel_i[j] = bi;
     // the winner leaves the pool: NaN never wins a '>' test again
 #pragma unroll
     for (int i = 0; i < NV; ++i)
@@ -114,7 +115,7 @@ __device__ __forceinline__ bool warp_topk_nv(const float* __restrict__ l, int E,
         gone |= 1u << i;
       }
   }
-  int certified = 1;
+  bool certified = true;
   if (bounds) {
     float above = -INFINITY;  // what no logit left out exceeds
 #pragma unroll
@@ -125,37 +126,28 @@ __device__ __forceinline__ bool warp_topk_nv(const float* __restrict__ l, int E,
       }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) above = fmaxf(above, __shfl_xor_sync(0xffffffffu, above, o));
-    if (lane == 0) {
-      float b[kMaxTopK];
-      for (int j = 0; j < k; ++j)
-        b[j] = (sel_i[j] >= 0 && sel_i[j] < E) ? (CG ? __ldcg(bounds + sel_i[j]) : bounds[sel_i[j]]) : INFINITY;
-      for (int j = 0; j + 1 < k; ++j)
-        if (!(sel_v[j] - sel_v[j + 1] > b[j] + b[j + 1])) certified = 0;  // also false for NaN
-      if (!(sel_v[k - 1] - b[k - 1] > above)) certified = 0;
-    }
+    const float b = lane < k && my_i >= 0 && my_i < E ? (CG ? __ldcg(bounds + my_i) : bounds[my_i]) : INFINITY;
+    const float next_v = __shfl_down_sync(0xffffffffu, my_v, 1), next_b = __shfl_down_sync(0xffffffffu, b, 1);
+    const bool apart = lane + 1 < k ? my_v - next_v > b + next_b : my_v - b > above;  // false for NaN
+    certified = __all_sync(0xffffffffu, lane >= k || apart);
   }
-  certified = __shfl_sync(0xffffffffu, certified, 0);
-  if (lane == 0) {
-    float w[kMaxTopK];
-    if (sigmoid) {
-      for (int j = 0; j < k; ++j) w[j] = 1.0f / (1.0f + expf(-sel_v[j]));
-    } else {
-      float mx = sel_v[0];
-      for (int j = 1; j < k; ++j) mx = fmaxf(mx, sel_v[j]);
-      float se = 0.f;
-      for (int j = 0; j < k; ++j) {
-        w[j] = expf(sel_v[j] - mx);
-        se += w[j];
-      }
-      const float inv = se > 0.f ? 1.0f / se : 0.f;
-      for (int j = 0; j < k; ++j) w[j] *= inv;
-    }
-    for (int j = 0; j < k; ++j) {
-      out[j * 2 + 0] = (float)sel_i[j];
-      out[j * 2 + 1] = w[j];
-    }
+  float w;
+  if (sigmoid) {
+    w = 1.0f / (1.0f + expf(-my_v));
+  } else {
+    // one lane per selection; the sum in order
+    float mx = __shfl_sync(0xffffffffu, my_v, 0);
+    for (int j = 1; j < k; ++j) mx = fmaxf(mx, __shfl_sync(0xffffffffu, my_v, j));
+    w = expf(my_v - mx);
+    float se = 0.f;
+    for (int j = 0; j < k; ++j) se += __shfl_sync(0xffffffffu, w, j);
+    w *= se > 0.f ? 1.0f / se : 0.f;
   }
-  return certified != 0;
+  if (lane < k) {
+    out[2 * lane] = (float)my_i;
+    out[2 * lane + 1] = w;
+  }
+  return certified;
 }
 
 template <bool CG = true>
@@ -712,6 +704,10 @@ __global__ void __launch_bounds__(256) k_router_finish(const FinishRouterArgs A)
   const int t = blockIdx.x;
   const int parts = A.parts, E = A.E;
   const int n_slices = (A.H / 32 + kFastSliceBlocks - 1) / kFastSliceBlocks;
+  // blocks of each part (with a division per part in every thread, and that selection, the kernel took 10.1 us, now 5.2)
+  __shared__ int s_blocks[kFastMaxParts];
+  if ((int)threadIdx.x < parts) s_blocks[threadIdx.x] = kFastSliceBlocks * (n_slices * ((int)threadIdx.x + 1) / parts - n_slices * (int)threadIdx.x / parts);
+  __syncthreads();
   griddep_wait();
   griddep_launch();
   float h2 = lane < parts ? __ldcg(A.hn2 + (size_t)t * parts + lane) : 0.f;
@@ -729,8 +725,7 @@ __global__ void __launch_bounds__(256) k_router_finish(const FinishRouterArgs A)
 #pragma unroll
     for (int m = 0; m < kFastMaxParts; ++m) {
       if (m < parts) {
-        const int blocks = kFastSliceBlocks * (n_slices * (m + 1) / parts - n_slices * m / parts);
-        sr += (float)blocks * fabsf(P) + v[m].y;
+        sr += (float)s_blocks[m] * fabsf(P) + v[m].y;
         P += v[m].x;
       }
     }
@@ -1146,9 +1141,9 @@ __global__ void __launch_bounds__(256) k_combine(const float* __restrict__ route
 // sequential fp32 chain of separate multiplies and adds, division, square root and products are the
 // IEEE round-to-nearest operations the reference's scalar code performs.
 //
-// A block per token: all its threads square the row into shared memory, one walks the squares (the next 32
-// in registers while 32 are added, so that it runs at the add latency), all of them scale the row.  Bound by
-// that chain, H x 4 cycles: 8 tokens x 2880 columns ~18 us less than one warp per token with the products in the chain.
+// A block per token: all its threads square the row into shared memory, one walks the squares (sixteen
+// in registers while the sixteen before are added), all of them scale the row.  Bound by that chain: 8 tokens x 2880 columns
+// 14.6 us with 32 copied from register to register, now 11.4 (4.4 cycles a column would be 6.5).
 // ---------------------------------------------------------------------------
 __global__ void __launch_bounds__(128) k_rmsnorm(const float* __restrict__ x, const float* __restrict__ w, float eps,
                                                  float* __restrict__ out, int T, int H) {
@@ -1166,20 +1161,22 @@ __global__ void __launch_bounds__(128) k_rmsnorm(const float* __restrict__ x, co
     if (threadIdx.x == 0) {
       const float4* q = reinterpret_cast<const float4*>(rms_sq);
       float s = 0.f;
-      float4 next[8];
+      auto add = [&](const float4 (&v)[4]) {
 #pragma unroll
-      for (int i = 0; i < 8; ++i) next[i] = q[i];
+        for (int i = 0; i < 4; ++i) s = __fadd_rn(__fadd_rn(__fadd_rn(__fadd_rn(s, v[i].x), v[i].y), v[i].z), v[i].w);
+      };
+      float4 u[4], v[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) u[i] = q[i];
+#pragma unroll 1
       for (int d = 0; d < H / 4; d += 8) {  // H is a multiple of 32
-        float4 at_hand[8];
 #pragma unroll
-        for (int i = 0; i < 8; ++i) at_hand[i] = next[i];
-        if (d + 8 < H / 4) {
+        for (int i = 0; i < 4; ++i) v[i] = q[d + 4 + i];
+        add(u);
+        const int after = d + 8 < H / 4 ? d + 8 : d;  // (the last ones are not used)
 #pragma unroll
-          for (int i = 0; i < 8; ++i) next[i] = q[d + 8 + i];
-        }
-#pragma unroll
-        for (int i = 0; i < 8; ++i)
-          s = __fadd_rn(__fadd_rn(__fadd_rn(__fadd_rn(s, at_hand[i].x), at_hand[i].y), at_hand[i].z), at_hand[i].w);
+        for (int i = 0; i < 4; ++i) u[i] = q[after + i];
+        add(v);
       }
       s_rms = __fsqrt_rn(__fadd_rn(__fdiv_rn(s, (float)H), eps));
     }
