@@ -1645,14 +1645,17 @@ int csk_moe_route(csk_moe_layer* L, const float* hidden, int64_t T, float* route
 }
 
 namespace {
-// How many passes the host entry point cuts a batch into so that the copies of one pass overlap
-// the kernels of another: as many as leave every expert about 128 rows per pass (the tensor-core
-// kernel's cost per row tile is nearly flat below that), at most two (measured: four passes cost more
-// in kernel time than they hide in copies); small batches take one.
+// How many equal passes the host entry point cuts a batch into so that the copies of one pass overlap the kernels of another.
+// What stays exposed is the first copy in and the last copy out; what passes cost is kernel time, the less the more rows an
+// expert has (a row tile's cost is nearly flat below 100 rows).  Page-locked buffers, 1 / 2 / 3 / 4 / 8 passes, ms: 128 experts of
+// 2880 x 2880, 4096 tokens (128 rows per expert) 2.59 / 2.27 / - / 2.73 / 3.22, 8192 4.97 / 3.58 / 3.64 / 3.67 / 5.12; 32 experts, 1500
+// (187) 0.97 / 0.84 / - / 1.01 / 1.29, 3000 (375) 1.84 / 1.32 / 1.26 / 1.34 / 1.82, 8192 (1024) 4.82 / 3.40 / 3.03 / 2.75 / 2.57.  (Shorter
+// first and last passes were up to 5 % quicker still, but the certified router adds a token's parts in an order that goes by
+// the pass's size: the low bits of its weights would depend on where in the batch it stands.)
 int host_passes(const csk_moe_layer* L, int64_t T) {
   if (L->timing || L->path == CSK_PATH_STREAM) return 1;
   const int64_t rows_per_expert = T * L->k / std::max(1, L->Eloc);
-  return (int)std::max<int64_t>(1, std::min<int64_t>(2, rows_per_expert / 128));
+  return rows_per_expert < 128 ? 1 : (int)std::max<int64_t>(2, std::min<int64_t>(csk_moe_layer::kMaxPasses, rows_per_expert / 120));
 }
 }  // namespace
 
