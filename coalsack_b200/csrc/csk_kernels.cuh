@@ -860,7 +860,7 @@ k_scan(int* __restrict__ counts, int E, int e_begin, int e_count, int tile_rows,
        int* __restrict__ cursor, RowTile* __restrict__ tiles, int* __restrict__ meta,
        const float* __restrict__ router_out, int n_pairs, int only_expert,
        int* __restrict__ row_of_pair = nullptr, ExpertTiles* __restrict__ expert_tiles = nullptr,
-       uint32_t* __restrict__ tile_masks = nullptr, int mask_words = 0) {
+       uint32_t* __restrict__ tile_masks = nullptr, int mask_words = 0, int4* __restrict__ places = nullptr) {
   __shared__ int s_row_off[1025];
   __shared__ int s_tile_off[1025];
   __shared__ int s_warp[2][32];
@@ -949,12 +949,23 @@ k_scan(int* __restrict__ counts, int E, int e_begin, int e_count, int tile_rows,
     const bool over = total_rows > max_rows || total_tiles > max_tiles;
     for (int i = e; i < n_pairs; i += 1024) {
       const int x = (int)router_out[2 * (size_t)i];
-      int pos = -1;
+      int pos = -1, r = -1;
       if (!over && x >= 0 && x < E && (only_expert < 0 || x == only_expert)) {
-        pos = s_row_off[x] + atomicAdd(&s_cur[x], 1);
+        r = atomicAdd(&s_cur[x], 1);
+        pos = s_row_off[x] + r;
         if (pos >= max_rows) pos = -1;
       }
       row_of_pair[i] = pos;
+      if (places) {
+        // the pair's row tile (number, first row, rows) and its row in it, or -1: one load for the kernel that writes the rows
+        // where it would chase expert, tile number and tile
+        int4 at = make_int4(0, 0, 0, -1);
+        if (pos >= 0 && x >= e_begin && x < e_begin + e_count) {
+          const int cnt = (x < 1023 ? s_row_off[x + 1] : s_row_off[1024]) - s_row_off[x], per = tile_height(cnt), q = r / per;
+          at = make_int4(s_tile_off[x] + q, s_row_off[x] + q * per, min(per, cnt - q * per), r - q * per);
+        }
+        places[i] = at;
+      }
     }
   }
   if (total_rows > max_rows || total_tiles > max_tiles) {

@@ -95,6 +95,7 @@ struct csk_moe_layer {
   int* d_offsets = nullptr;      // [E+1]
   int* d_cursor = nullptr;       // [E]
   int* d_row_of_pair = nullptr;  // [max_rows]
+  int4* d_places = nullptr;      // [min(max_rows, kOneBlockPairs)] where the pairs of a small batch go (block-scaled kernel)
   ExpertTiles* d_expert_tiles = nullptr;  // [E] where the experts' row tiles are (block-scaled kernel)
   uint8_t* d_ximg = nullptr;     // the block-scaled kernel's operands: token rows and activated rows as digit images
   uint8_t* d_aimg = nullptr;
@@ -346,7 +347,8 @@ int launch_permute(csk_moe_layer* L, const float* d_hidden, const float* d_route
     // small batch: histogram, scan, tile list (and, for digits, the rows' places) in one single-block launch
     launch_k(k_scan, dim3(1), dim3(1024), 0, s, L->pdl, L->d_counts, L->E, e_begin, e_count, tile_rows, (int)max_rows,
              L->max_tiles, res, L->d_offsets, L->d_cursor, L->d_tiles, L->d_meta, d_router, n_pairs, only_expert,
-             digits ? L->d_row_of_pair : (int*)nullptr, et, digits ? L->d_wide : (uint32_t*)nullptr, wide_stride(L));
+             digits ? L->d_row_of_pair : (int*)nullptr, et, digits ? L->d_wide : (uint32_t*)nullptr, wide_stride(L),
+             digits ? L->d_places : (int4*)nullptr);
     L->last.launches += 1;
   } else {
     CSK_CUDA(L, cudaMemsetAsync(L->d_counts, 0, sizeof(int) * L->E, s));
@@ -355,7 +357,7 @@ int launch_permute(csk_moe_layer* L, const float* d_hidden, const float* d_route
         d_router, n_pairs, L->E, only_expert, L->d_counts, L->d_meta);
     k_scan<<<1, 1024, 0, s>>>(L->d_counts, L->E, e_begin, e_count, tile_rows, (int)max_rows, L->max_tiles, res,
                               L->d_offsets, L->d_cursor, L->d_tiles, L->d_meta, nullptr, 0, -1, nullptr, et,
-                              digits ? L->d_wide : nullptr, wide_stride(L));
+                              digits ? L->d_wide : nullptr, wide_stride(L), nullptr);
     L->last.launches += 2;
   }
   if (digits) {
@@ -366,6 +368,7 @@ int launch_permute(csk_moe_layer* L, const float* d_hidden, const float* d_route
     a.et = L->d_expert_tiles;
     a.cursor = one_block ? nullptr : L->d_cursor;
     a.row_of_pair = L->d_row_of_pair;
+    a.places = L->d_places;
     a.tiles = L->d_tiles;
     a.n_tiles_ptr = L->d_meta;
     a.image = L->d_ximg;
@@ -846,6 +849,7 @@ int csk_moe_create(const csk_moe_config* cfg, csk_moe_layer** out) {
   CK(cudaMalloc(&L->d_offsets, sizeof(int) * (L->E + 1)));
   CK(cudaMalloc(&L->d_cursor, sizeof(int) * L->E));
   CK(cudaMalloc(&L->d_row_of_pair, sizeof(int) * L->max_rows));
+  CK(cudaMalloc(&L->d_places, sizeof(int4) * std::min<int64_t>(L->max_rows, kOneBlockPairs)));
   CK(cudaMalloc(&L->d_expert_tiles, sizeof(ExpertTiles) * L->E));
   CK(cudaMalloc(&L->d_out_row_map, sizeof(int) * L->max_rows));
   CK(cudaMalloc(&L->d_seg, sizeof(int) * (3 * 1024 + 8)));
@@ -892,7 +896,7 @@ int csk_moe_destroy(csk_moe_layer* L) {
   void* dev[] = {L->d_shared_out, L->d_p2p_epoch, L->d_unit_router, L->d_stage2, L->d_norm_w, L->d_normed, L->d_part, L->d_hn2, L->d_wnorm, L->d_wg_tc, L->d_wg_tc_scale, L->d_wnorm_tc, L->d_fb_list, L->d_fb, L->d_info, L->d_back, L->d_row_ptr, L->d_p2p_base, L->d_peer_x16, L->d_peer_info, L->d_peer_back,
                  L->d_router_phys, L->d_slot_map, L->d_weights, L->d_resident, L->d_stage, L->d_wg, L->d_wg_few, L->d_wg_many, L->d_route_cnt, L->d_logits, L->d_rbias, L->d_hidden,
                  L->d_router, L->d_out, L->d_x16, L->d_a16, L->d_y, L->d_counts, L->d_offsets,
-                 L->d_cursor, L->d_row_of_pair, L->d_expert_tiles, L->d_ximg, L->d_aimg, L->d_wide, L->d_out_row_map, L->d_seg, L->d_tiles, L->d_meta};
+                 L->d_cursor, L->d_row_of_pair, L->d_places, L->d_expert_tiles, L->d_ximg, L->d_aimg, L->d_wide, L->d_out_row_map, L->d_seg, L->d_tiles, L->d_meta};
   for (void* p : dev)
     if (p) cudaFree(p);
   for (uint8_t* p : L->mx_outgrown) cudaFree(p);

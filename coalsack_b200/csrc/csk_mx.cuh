@@ -303,8 +303,9 @@ struct MxQuantArgs {
   const float* router;       // [T,k,2]
   const int* offsets;        // [E+1] first row of each expert
   const ExpertTiles* et;     // [E]
-  int* cursor;               // null: row_of_pair is given; else rows are claimed here and row_of_pair is written
+  int* cursor;               // null: the places are given; else rows are claimed here and row_of_pair is written
   int* row_of_pair;          // [T*k]
+  const int4* places;        // [T*k] the pairs' places by k_scan (cursor null), see there
   const RowTile* tiles;
   const int* n_tiles_ptr;
   uint8_t *image, *rest;     // digits, and the digits after them
@@ -339,25 +340,28 @@ __global__ void __launch_bounds__(kMxQuantThreads) k_mx_quant(const MxQuantArgs 
   griddep_launch();
   if ((int)threadIdx.x < A.k) {
     const int j = threadIdx.x, pair = t * A.k + j;
-    const int x = (int)A.router[2 * (size_t)pair];
-    const bool mine = x >= 0 && x < A.E && (A.only_expert < 0 || x == A.only_expert);
-    int pos = -1;
-    if (A.cursor) {
-      if (mine) pos = A.offsets[x] + atomicAdd(&A.cursor[x], 1);
+    if (!A.cursor) {
+      const int4 at = A.places[pair];
+      s_img[j] = mx_tile_image<kMxDigitsX>(at.x, at.y, at.z, A.recs);
+      s_tile[j] = at.x;
+      s_r[j] = at.w;
+      s_w[j] = A.router[2 * (size_t)pair + 1];
+    } else {
+      const int x = (int)A.router[2 * (size_t)pair];
+      int pos = -1;
+      if (x >= 0 && x < A.E && (A.only_expert < 0 || x == A.only_expert)) pos = A.offsets[x] + atomicAdd(&A.cursor[x], 1);
       if (pos >= A.max_rows) pos = -1;
       A.row_of_pair[pair] = pos;
-    } else {
-      pos = A.row_of_pair[pair];
-    }
-    s_r[j] = -1;
-    if (pos >= 0 && mine && x >= A.e_begin && x < A.e_begin + A.e_count && *A.n_tiles_ptr > 0) {
-      const ExpertTiles et = A.et[x];
-      const int r = pos - A.offsets[x], tile = et.tile0 + r / et.height;
-      const RowTile rt = A.tiles[tile];
-      s_img[j] = mx_tile_image<kMxDigitsX>(tile, rt.row0, rt.rows, A.recs);
-      s_tile[j] = tile;
-      s_r[j] = r % et.height;
-      s_w[j] = A.router[2 * (size_t)pair + 1];
+      s_r[j] = -1;
+      if (pos >= 0 && x >= A.e_begin && x < A.e_begin + A.e_count && *A.n_tiles_ptr > 0) {
+        const ExpertTiles et = A.et[x];
+        const int r = pos - A.offsets[x], tile = et.tile0 + r / et.height;
+        const RowTile rt = A.tiles[tile];
+        s_img[j] = mx_tile_image<kMxDigitsX>(tile, rt.row0, rt.rows, A.recs);
+        s_tile[j] = tile;
+        s_r[j] = r % et.height;
+        s_w[j] = A.router[2 * (size_t)pair + 1];
+      }
     }
   }
   __syncthreads();
