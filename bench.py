@@ -462,9 +462,9 @@ class SingleGpu:
         out = {k: acc[k] / n for k in acc}
         out["path"] = {1: "stream", 2: "tile"}.get(int(round(out["path"])), "?")
         rows_per_expert, _, _ = self.layer.counters()
-        tr = 40 if out["path"] == "stream" else 192
+        tr = 40 if out["path"] == "stream" else 256
         out["row_tiles"] = int(sum(-(-int(r) // tr) for r in rows_per_expert))
-        out["gate_up_kernel"] = "k_mx<gated>" if out["path"] == "stream" else "k_tile<gated>"
+        out["gate_up_kernel"] = "k_mx<gated>" if out["path"] == "stream" else "k_tile2<gated>"
         return out
 
     def time_e2e(self, steps, warmup):
