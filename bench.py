@@ -56,9 +56,7 @@ def measured_peaks():
 # dram__bytes_read.sum + dram__bytes_write.sum of ONE launch of the dominant kernel, from an ncu capture
 # (--metrics dram__bytes_read.sum,dram__bytes_write.sum) of this program on the same workload, single GPU.
 # Key = (workload name, tokens, kernel).  Other workloads report null.
-MEASURED_TRAFFIC = {
-    ("c2_gptoss120b_prefill8192", 8192, "k_tile<gated>"): 1599.2e6,   # 1417.8 MB read + 181.4 MB written
-}
+MEASURED_TRAFFIC = {}
 
 
 def measured_traffic(sh, kernel, world):
