@@ -34,9 +34,11 @@ struct FewArgs {
   int one_expert;   // the layer holds a single expert: the tile list may be one launch old
 };
 
-// NT = groups of eight token rows.  blockIdx.x: 16 weight rows (features), blockIdx.y: row tile, blockIdx.z: its rows from 8 NT z on.
+// NT = groups of eight token rows.  blockIdx.x: 16 weight rows (features), blockIdx.y: row tile.  TURNS: the tile may have more
+// than 8 NT rows, which are taken 8 NT after another (the loop's registers cost the others up to 5 %: 128 experts of 2048 x 768, 16
+// tokens of eight slots 224 -> 236 us).
 // Two blocks an SM up to 32 rows (in 128 registers; three blocks of 80 were slower, 62 -> 70 us for a block of 5 tokens).
-template <bool GATED, int NT>
+template <bool GATED, int NT, bool TURNS>
 __global__ void __launch_bounds__(kFewWarps * 32, NT <= 4 ? 2 : 1) k_few16(const FewArgs F) {
   extern __shared__ float few_sums[];
   const TileArgs& A = F.t;
@@ -68,88 +70,102 @@ __global__ void __launch_bounds__(kFewWarps * 32, NT <= 4 ? 2 : 1) k_few16(const
   griddep_launch();
   if ((int)blockIdx.y >= *A.n_tiles_ptr) return;
   RowTile rt = A.tiles[blockIdx.y];
-  rt.row0 += 8 * NT * (int)blockIdx.z;
-  rt.rows -= 8 * NT * (int)blockIdx.z;
-  if (rt.rows <= 0) return;
-  float acc[M][NT][4];
+  for (;;) {
+    float acc[M][NT][4];
 #pragma unroll
-  for (int m = 0; m < M; ++m)
+    for (int m = 0; m < M; ++m)
 #pragma unroll
-    for (int t = 0; t < NT; ++t)
+      for (int t = 0; t < NT; ++t)
 #pragma unroll
-      for (int c = 0; c < 4; ++c) acc[m][t][c] = 0.f;
-  const __half* x = F.x + (size_t)(rt.row0 + g) * F.ldx + q * 8;
-  auto step = [&](int kt, const uint4 (&d)[M][2][2]) {
+        for (int c = 0; c < 4; ++c) acc[m][t][c] = 0.f;
+    const __half* x = F.x + (size_t)(rt.row0 + g) * F.ldx + q * 8;
+    auto step = [&](int kt, const uint4 (&d)[M][2][2]) {
 #pragma unroll
-    for (int t = 0; t < NT; ++t) {
-      if (t && 8 * t >= rt.rows) continue;
-      const uint4* xr = reinterpret_cast<const uint4*>(x + (size_t)(8 * t) * F.ldx + kt * kTileK);
+      for (int t = 0; t < NT; ++t) {
+        if (t && 8 * t >= rt.rows) continue;
+        const uint4* xr = reinterpret_cast<const uint4*>(x + (size_t)(8 * t) * F.ldx + kt * kTileK);
 #pragma unroll
-      for (int p = 0; p < 2; ++p) {
-        const uint4 b = xr[4 * p];
+        for (int p = 0; p < 2; ++p) {
+          const uint4 b = xr[4 * p];
 #pragma unroll
-        for (int m = 0; m < M; ++m) {
-          const uint4 lo = d[m][0][p], hi = d[m][1][p];
-          mma_16816(acc[m][t], lo.x, hi.x, lo.y, hi.y, b.x, b.y);
-          mma_16816(acc[m][t], lo.z, hi.z, lo.w, hi.w, b.z, b.w);
+          for (int m = 0; m < M; ++m) {
+            const uint4 lo = d[m][0][p], hi = d[m][1][p];
+            mma_16816(acc[m][t], lo.x, hi.x, lo.y, hi.y, b.x, b.y);
+            mma_16816(acc[m][t], lo.z, hi.z, lo.w, hi.w, b.z, b.w);
+          }
         }
       }
+    };
+    for (int kt = warp; kt < L.k_tiles; kt += 2 * kFewWarps) {
+      step(kt, w[0]);
+      if (kt + 2 * kFewWarps < L.k_tiles) load_w(kt + 2 * kFewWarps, w[0]);
+      if (kt + kFewWarps < L.k_tiles) {
+        step(kt + kFewWarps, w[1]);
+        if (kt + 3 * kFewWarps < L.k_tiles) load_w(kt + 3 * kFewWarps, w[1]);
+      }
     }
-  };
-  for (int kt = warp; kt < L.k_tiles; kt += 2 * kFewWarps) {
-    step(kt, w[0]);
-    if (kt + 2 * kFewWarps < L.k_tiles) load_w(kt + 2 * kFewWarps, w[0]);
-    if (kt + kFewWarps < L.k_tiles) {
-      step(kt + kFewWarps, w[1]);
-      if (kt + 3 * kFewWarps < L.k_tiles) load_w(kt + 3 * kFewWarps, w[1]);
+    // [warp][matrix][group][register][lane]
+    constexpr int kPer = M * NT * 4 * 32;
+#pragma unroll
+    for (int m = 0; m < M; ++m)
+#pragma unroll
+      for (int t = 0; t < NT; ++t)
+#pragma unroll
+        for (int c = 0; c < 4; ++c) few_sums[warp * kPer + ((m * NT + t) * 4 + c) * 32 + lane] = acc[m][t][c];
+    __syncthreads();
+    const float* bias = reinterpret_cast<const float*>(ebase + A.bias_offset);
+    for (int i = threadIdx.x; i < NT * 128; i += kFewWarps * 32) {
+      // sixteen neighbouring threads: sixteen features of one token
+      const int row = i & 15, token = i >> 4, n = n0 + row;
+      const int at = ((token >> 3) * 4 + (row >> 3) * 2 + (token & 1)) * 32 + (row & 7) * 4 + (token >> 1 & 3);
+      float s[M];
+#pragma unroll
+      for (int m = 0; m < M; ++m) {
+        s[m] = few_sums[m * NT * 128 + at];
+#pragma unroll
+        for (int v = 1; v < kFewWarps; ++v) s[m] += few_sums[v * kPer + m * NT * 128 + at];
+      }
+      if (token >= rt.rows) continue;
+      if (GATED) {
+        const float gate = s[0] + (A.has_bias ? bias[A.F + n] : 0.f), up = s[M - 1] + (A.has_bias ? bias[n] : 0.f);
+        A.a_out[(size_t)(rt.row0 + token) * A.lda + n] = __float2half_rn(gated_act_fast(gate, up, A.act));
+      } else {
+        A.y_out[(size_t)(rt.row0 + token) * A.ldy + n] = s[0] + (A.has_bias ? bias[2 * A.F + n] : 0.f);
+      }
     }
-  }
-  // [warp][matrix][group][register][lane]
-  constexpr int kPer = M * NT * 4 * 32;
-#pragma unroll
-  for (int m = 0; m < M; ++m)
-#pragma unroll
-    for (int t = 0; t < NT; ++t)
-#pragma unroll
-      for (int c = 0; c < 4; ++c) few_sums[warp * kPer + ((m * NT + t) * 4 + c) * 32 + lane] = acc[m][t][c];
-  __syncthreads();
-  const float* bias = reinterpret_cast<const float*>(ebase + A.bias_offset);
-  for (int i = threadIdx.x; i < NT * 128; i += kFewWarps * 32) {
-    // sixteen neighbouring threads: sixteen features of one token
-    const int row = i & 15, token = i >> 4, n = n0 + row;
-    const int at = ((token >> 3) * 4 + (row >> 3) * 2 + (token & 1)) * 32 + (row & 7) * 4 + (token >> 1 & 3);
-    float s[M];
-#pragma unroll
-    for (int m = 0; m < M; ++m) {
-      s[m] = few_sums[m * NT * 128 + at];
-#pragma unroll
-      for (int v = 1; v < kFewWarps; ++v) s[m] += few_sums[v * kPer + m * NT * 128 + at];
-    }
-    if (token >= rt.rows) continue;
-    if (GATED) {
-      const float gate = s[0] + (A.has_bias ? bias[A.F + n] : 0.f), up = s[M - 1] + (A.has_bias ? bias[n] : 0.f);
-      A.a_out[(size_t)(rt.row0 + token) * A.lda + n] = __float2half_rn(gated_act_fast(gate, up, A.act));
-    } else {
-      A.y_out[(size_t)(rt.row0 + token) * A.ldy + n] = s[0] + (A.has_bias ? bias[2 * A.F + n] : 0.f);
-    }
+    rt.row0 += 8 * NT;
+    rt.rows -= 8 * NT;
+    if (!TURNS || rt.rows <= 0) break;
+    __syncthreads();  // the sums have been read
+    if (warp < L.k_tiles) load_w(warp, w[0]);
+    if (warp + kFewWarps < L.k_tiles) load_w(warp + kFewWarps, w[1]);
   }
 }
 
-template <bool GATED>
-inline cudaError_t few_launch_one(const FewArgs& f, int features, int tiles, int rows, cudaStream_t s, bool pdl) {
+template <bool GATED, bool TURNS>
+inline cudaError_t few_launch_turns(const FewArgs& f, int features, int tiles, int rows, cudaStream_t s, bool pdl) {
   const int groups = rows <= 8 ? 1 : rows <= 16 ? 2 : rows <= 32 ? 4 : 8;
-  const dim3 grid((unsigned)(features / 16), (unsigned)tiles, (unsigned)ceil_div(rows, 8 * groups)), block(kFewWarps * 32);
+  const dim3 grid((unsigned)(features / 16), (unsigned)tiles), block(kFewWarps * 32);
   const size_t smem = few_smem_bytes(groups, GATED);
   switch (groups) {
-    case 1: return launch_k(k_few16<GATED, 1>, grid, block, smem, s, pdl, f);
-    case 2: return launch_k(k_few16<GATED, 2>, grid, block, smem, s, pdl, f);
-    case 4: return launch_k(k_few16<GATED, 4>, grid, block, smem, s, pdl, f);
-    default: return launch_k(k_few16<GATED, 8>, grid, block, smem, s, pdl, f);
+    case 1: return launch_k(k_few16<GATED, 1, TURNS>, grid, block, smem, s, pdl, f);
+    case 2: return launch_k(k_few16<GATED, 2, TURNS>, grid, block, smem, s, pdl, f);
+    case 4: return launch_k(k_few16<GATED, 4, TURNS>, grid, block, smem, s, pdl, f);
+    default: return launch_k(k_few16<GATED, 8, TURNS>, grid, block, smem, s, pdl, f);
   }
+}
+
+// `tiles`: no fewer than the list may have; `rows`: of an expert, unless the routing may name it twice in a token
+template <bool GATED>
+inline cudaError_t few_launch_one(const FewArgs& f, int features, int tiles, int rows, bool repeats, cudaStream_t s, bool pdl) {
+  return repeats ? few_launch_turns<GATED, true>(f, features, tiles, rows, s, pdl)
+                 : few_launch_turns<GATED, false>(f, features, tiles, rows, s, pdl);
 }
 
 inline cudaError_t few_prepare_device() {
-  return cudaFuncSetAttribute(k_few16<true, 8>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)few_smem_bytes(8, true));
+  const cudaError_t e = cudaFuncSetAttribute(k_few16<true, 8, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)few_smem_bytes(8, true));
+  if (e != cudaSuccess) return e;
+  return cudaFuncSetAttribute(k_few16<true, 8, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)few_smem_bytes(8, true));
 }
 
 }  // namespace csk

@@ -504,13 +504,14 @@ int tile_rows_for(const csk_moe_layer* L, int path) {
 }
 
 // grouped gate/up + activation + down over the row tiles listed in d_tiles; the grouped rows are in d_x16 (tensor-core
-// path) or in d_ximg (streaming path); output rows go to y (through out_row_map or out_row_ptr if set)
+// path) or in d_ximg (streaming path); output rows go to y (through out_row_map or out_row_ptr if set).  `tokens`: of the batch, where
+// its rows are known to come from one; `repeats`: a token's slots may name an expert more than once
 int launch_experts(csk_moe_layer* L, int path, float* y, int ldy, const int* out_row_map, cudaStream_t s, StageTimer& tm,
-                   float* const* out_row_ptr = nullptr, int64_t most_rows = INT64_MAX) {
+                   float* const* out_row_ptr = nullptr, int64_t tokens = INT64_MAX, bool repeats = false) {
   // Few rows per expert: the weights' bytes are all that counts (csk_few16.cuh).  Step, k_tile / k_few16, us: dense FFN of 2880 x
   // 2880 (weights in L2) 1 token 41 / 15, 16 43 / 17, 32 45 / 25, 48 48 / 39, 64 51 / 41; 16 experts of 2048 x 2048 beside a
   // shared one 1 token 72 / 39, 5 85 / 62, 16 114 / 103, 32 120 / 145 (most experts are hit, by two rows each).
-  if (path == CSK_PATH_TILE && L->w16 && most_rows <= (L->Eloc == 1 ? kFewMaxRows : kFewMaxRowsRouted) && !L->debug_stall) {
+  if (path == CSK_PATH_TILE && L->w16 && tokens <= (L->Eloc == 1 ? kFewMaxRows : kFewMaxRowsRouted) && !L->debug_stall) {
     FewArgs f{};
     f.x = L->d_x16;
     f.ldx = L->ldx;
@@ -528,8 +529,10 @@ int launch_experts(csk_moe_layer* L, int path, float* y, int ldy, const int* out
     a.L = L->Tgu;
     a.a_out = L->d_a16;
     a.lda = L->lda;
-    const int tiles = (int)std::min<int64_t>(L->Eloc, most_rows * L->k);
-    CSK_CUDA(L, few_launch_one<true>(f, L->F, tiles, (int)most_rows, s, L->pdl));
+    // (where a token's slots may all name one expert, its rows may need several tiles)
+    const int64_t pairs = tokens * L->k;
+    const int tiles = (int)std::min(pairs, repeats ? L->Eloc + pairs / kTileM : (int64_t)L->Eloc);
+    CSK_CUDA(L, few_launch_one<true>(f, L->F, tiles, (int)tokens, repeats, s, L->pdl));
     tm.mark();
     f.x = L->d_a16;
     f.ldx = L->lda;
@@ -537,7 +540,7 @@ int launch_experts(csk_moe_layer* L, int path, float* y, int ldy, const int* out
     a.L = L->Td;
     a.y_out = y;
     a.ldy = ldy;
-    CSK_CUDA(L, few_launch_one<false>(f, L->H, tiles, (int)most_rows, s, L->pdl));
+    CSK_CUDA(L, few_launch_one<false>(f, L->H, tiles, (int)tokens, repeats, s, L->pdl));
     tm.mark();
     L->last.launches += 2;
   } else if (path == CSK_PATH_TILE) {
@@ -663,7 +666,7 @@ int forward_dev(csk_moe_layer* L, const float* d_hidden, int64_t T, const float*
                           mx ? L->mx_rows : L->max_rows, s);
   if (rc) return rc;
   tm.mark();
-  rc = launch_experts(L, path, L->d_y, L->H, nullptr, s, tm, nullptr, T);
+  rc = launch_experts(L, path, L->d_y, L->H, nullptr, s, tm, nullptr, T, !routed && L->k > 1);
   if (rc) return rc;
   // the shared expert's rows come from another stream: the combine is the first kernel that reads them
   if (shared_ready) CSK_CUDA(L, cudaStreamWaitEvent(s, shared_ready, 0));

@@ -2,6 +2,7 @@
 k-tiles and warps, against the CPU restatement of the reference; and the first batch of the kernel after it."""
 import numpy as np
 import pytest
+import torch
 
 from coalsack_b200 import MoeLayer, dense_ffn_node, synth
 from tests import cases
@@ -49,4 +50,51 @@ def test_experts(gpu_lib, port, E, k, T):
     got, _ = lay.forward(bad, router_out=ro)
     keep = np.arange(T) != T // 2
     assert np.array_equal(got[keep], out[keep]) and not np.isfinite(got[T // 2]).any()
+    lay.close()
+
+
+@pytest.mark.parametrize("E,count,k,T", [
+    (5, 0, 2, 1), (5, 0, 2, 5), (5, 0, 2, 8), (5, 0, 2, 9), (5, 0, 4, 5), (5, 0, 4, 16),  # up to four turns of a tile's rows
+    (16, 0, 16, 16),                                                                      # 256 rows: two tiles of one expert
+    (4, 1, 2, 8), (4, 1, 4, 9), (4, 1, 4, 16), (4, 1, 4, 64),                             # a shard that holds one expert
+])
+@pytest.mark.parametrize("one", [True, False])
+def test_routing_that_names_an_expert_twice(gpu_lib, port, E, count, k, T, one):
+    """The caller's routing may fill several slots of a token with one expert (padding with expert 0 does): every such pair
+    is a row of its own, so an expert has up to k rows per token.  After a batch of other values, whose rows must not show."""
+    H, F = 288, 160
+    held = count or E
+    rng = np.random.default_rng(E + k + T)
+    experts = [cases.dense_ffn_case(H=H, F=F, T=1, bias=True, seed=950 + e)[1:] for e in range(held)]
+    lay = MoeLayer(E, k, H, F, activation=synth.STANDARD_SWIGLU, has_bias=True, max_tokens=80, weights_f16=True, expert_count=count)
+    for e, (gw, uw, dw, bg, bu, bd) in enumerate(experts):
+        lay.load_expert_f16(e, uw, gw, dw, bu, bg, bd)
+
+    def routing(n):
+        ro = rng.uniform(0.1, 1.0, (n, k, 2)).astype(np.float32)
+        ro[..., 0] = 0 if one else rng.integers(0, held, (n, k))
+        return ro
+
+    def forward(hidden, ro):  # (on device buffers: never cut into passes)
+        x, r, out = torch.from_numpy(hidden).cuda(), torch.from_numpy(ro).cuda(), torch.empty(hidden.shape, device="cuda")
+        torch.cuda.synchronize()
+        lay.forward_dev(x, len(hidden), out, d_router_in=r)
+        lay.sync()
+        return out.cpu().numpy()
+
+    forward((100 * rng.standard_normal((80, H))).astype(np.float32), routing(80))
+    hidden, ro = rng.standard_normal((T, H)).astype(np.float32), routing(T)
+    out = forward(hidden, ro)
+    dense = [port.dense_ffn(hidden, *w) for w in experts]
+    want = np.zeros((T, H), np.float32)
+    for j in range(k):
+        want += ro[:, j, 1:] * np.stack([dense[int(e)][t] for t, e in enumerate(ro[:, j, 0])])
+    mx, mr = cases.err_stats(out, want)
+    assert mx <= cases.MAX_ABS_OVER_RMS and mr <= cases.MEAN_REL, (mx, mr)
+    named = (ro[..., 0] == 0).any(axis=1)
+    if named.any():
+        alone = lay.expert_forward(0, hidden, ro)
+        mx, mr = cases.err_stats(alone[named], dense[0][named])
+        assert mx <= cases.MAX_ABS_OVER_RMS and mr <= cases.MEAN_REL, (mx, mr)
+        assert np.all(alone[~named] == 0)
     lay.close()
