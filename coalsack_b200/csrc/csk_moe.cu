@@ -3,6 +3,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <cmath>
 #include <cstdarg>
 #include <cstdio>
 #include <cstring>
@@ -503,15 +504,34 @@ int tile_rows_for(const csk_moe_layer* L, int path) {
   return path == CSK_PATH_TILE ? (use_pairs(L) ? kPairN : kTileM) : kMxTileRows;
 }
 
+// What is known of the tokens whose rows are listed (nothing of rows received from peers).
+struct Batch {
+  int64_t tokens = INT64_MAX;
+  bool repeats = false;     // a token's slots may name an expert more than once
+  bool one_expert = false;  // only one expert's rows are listed
+};
+
+// fp16 weights: the kernel for few rows (csk_few16.cuh) takes a batch of so many tokens.  The weights' bytes are all that counts
+// there.  Step, k_tile / k_few16, us: dense FFN of 2880 x 2880 (weights in L2) 1 token 41 / 15, 16 43 / 17, 32 45 / 25, 48 48 / 39, 64
+// 51 / 41; 16 experts of 2048 x 2048 beside a shared one 1 token 72 / 39, 5 85 / 62, 16 114 / 103, 32 120 / 145.
+// Of several experts its time goes by those that are hit, k_tile's by the rounds of their items (128 features of an expert) on
+// the SMs.  The line is 1.4 items per SM, for evenly spread routing: 2048 x 2048, 16 experts, top-1, 16 tokens (165 items) 88 / 85,
+// top-2 12 (202) 93 / 92, 16 (224) 95 / 100, top-4 16 (252) 99 / 108; 128 of 2048 x 768, top-8, 2 (91) 63 / 62, 4 (170) 92 / 93, 8 (303)
+// 123 / 147, 16 (487) 164 / 232; 64 of 512 x 512, top-8, 4 (101) 38 / 34, 16 (222) 40 / 47; 32 of 2880 x 2880, top-4, 3 (233) 123 / 130, 8
+// (470) 213 / 234; 12 of 2880 x 2880, top-2, 8 (207) 123 / 120, 16 (259) 130 / 142; 8 of 2048 x 2048, top-2, 16 (126) 74 / 71.
+bool few_rows(const csk_moe_layer* L, const Batch& b) {
+  if (L->Eloc == 1) return b.tokens <= kFewMaxRows;
+  if (b.tokens > kFewMaxRowsRouted) return false;
+  if (b.one_expert) return true;
+  const double hit = L->Eloc * (1.0 - std::pow(1.0 - 1.0 / L->E, (double)(b.tokens * L->k)));
+  return hit * L->Tgu.n_tiles <= 1.4 * L->sm_count;
+}
+
 // grouped gate/up + activation + down over the row tiles listed in d_tiles; the grouped rows are in d_x16 (tensor-core
-// path) or in d_ximg (streaming path); output rows go to y (through out_row_map or out_row_ptr if set).  `tokens`: of the batch, where
-// its rows are known to come from one; `repeats`: a token's slots may name an expert more than once
+// path) or in d_ximg (streaming path); output rows go to y (through out_row_map or out_row_ptr if set)
 int launch_experts(csk_moe_layer* L, int path, float* y, int ldy, const int* out_row_map, cudaStream_t s, StageTimer& tm,
-                   float* const* out_row_ptr = nullptr, int64_t tokens = INT64_MAX, bool repeats = false) {
-  // Few rows per expert: the weights' bytes are all that counts (csk_few16.cuh).  Step, k_tile / k_few16, us: dense FFN of 2880 x
-  // 2880 (weights in L2) 1 token 41 / 15, 16 43 / 17, 32 45 / 25, 48 48 / 39, 64 51 / 41; 16 experts of 2048 x 2048 beside a
-  // shared one 1 token 72 / 39, 5 85 / 62, 16 114 / 103, 32 120 / 145 (most experts are hit, by two rows each).
-  if (path == CSK_PATH_TILE && L->w16 && tokens <= (L->Eloc == 1 ? kFewMaxRows : kFewMaxRowsRouted) && !L->debug_stall) {
+                   float* const* out_row_ptr = nullptr, const Batch& batch = {}) {
+  if (path == CSK_PATH_TILE && L->w16 && few_rows(L, batch) && !L->debug_stall) {
     FewArgs f{};
     f.x = L->d_x16;
     f.ldx = L->ldx;
@@ -530,9 +550,9 @@ int launch_experts(csk_moe_layer* L, int path, float* y, int ldy, const int* out
     a.a_out = L->d_a16;
     a.lda = L->lda;
     // (where a token's slots may all name one expert, its rows may need several tiles)
-    const int64_t pairs = tokens * L->k;
-    const int tiles = (int)std::min(pairs, repeats ? L->Eloc + pairs / kTileM : (int64_t)L->Eloc);
-    CSK_CUDA(L, few_launch_one<true>(f, L->F, tiles, (int)tokens, repeats, s, L->pdl));
+    const int64_t pairs = batch.tokens * L->k;
+    const int tiles = (int)std::min(pairs, batch.repeats ? L->Eloc + pairs / kTileM : (int64_t)L->Eloc);
+    CSK_CUDA(L, few_launch_one<true>(f, L->F, tiles, (int)batch.tokens, batch.repeats, s, L->pdl));
     tm.mark();
     f.x = L->d_a16;
     f.ldx = L->lda;
@@ -540,7 +560,7 @@ int launch_experts(csk_moe_layer* L, int path, float* y, int ldy, const int* out
     a.L = L->Td;
     a.y_out = y;
     a.ldy = ldy;
-    CSK_CUDA(L, few_launch_one<false>(f, L->H, tiles, (int)tokens, repeats, s, L->pdl));
+    CSK_CUDA(L, few_launch_one<false>(f, L->H, tiles, (int)batch.tokens, batch.repeats, s, L->pdl));
     tm.mark();
     L->last.launches += 2;
   } else if (path == CSK_PATH_TILE) {
@@ -650,7 +670,7 @@ int forward_dev(csk_moe_layer* L, const float* d_hidden, int64_t T, const float*
     CSK_CUDA(L, cudaGetLastError());
     L->last.launches++;
     tm.mark();
-    int rc = launch_experts(L, path, d_out, L->H, nullptr, s, tm, nullptr, T);
+    int rc = launch_experts(L, path, d_out, L->H, nullptr, s, tm, nullptr, Batch{T});
     if (rc) return rc;
     tm.mark();  // nothing to combine
     L->n_marks = tm.n;
@@ -666,7 +686,7 @@ int forward_dev(csk_moe_layer* L, const float* d_hidden, int64_t T, const float*
                           mx ? L->mx_rows : L->max_rows, s);
   if (rc) return rc;
   tm.mark();
-  rc = launch_experts(L, path, L->d_y, L->H, nullptr, s, tm, nullptr, T, !routed && L->k > 1);
+  rc = launch_experts(L, path, L->d_y, L->H, nullptr, s, tm, nullptr, Batch{T, !routed && L->k > 1, only_expert >= 0});
   if (rc) return rc;
   // the shared expert's rows come from another stream: the combine is the first kernel that reads them
   if (shared_ready) CSK_CUDA(L, cudaStreamWaitEvent(s, shared_ready, 0));

@@ -98,3 +98,23 @@ def test_routing_that_names_an_expert_twice(gpu_lib, port, E, count, k, T, one):
         assert mx <= cases.MAX_ABS_OVER_RMS and mr <= cases.MEAN_REL, (mx, mr)
         assert np.all(alone[~named] == 0)
     lay.close()
+
+
+@pytest.mark.parametrize("E,k,T,few", [(64, 8, 4, True), (64, 8, 15, False), (8, 2, 15, True)])
+def test_many_hit_experts_go_to_the_tensor_core_kernel(gpu_lib, E, k, T, few):
+    """The streaming kernel is the slower one once a small batch hits many experts.  The tensor-core kernel serves 17 tokens in
+    any case, and a row's bits do not depend on its batch: so it has served the shorter batch if and only if the bits agree."""
+    H, F = 256, 512
+    rng = np.random.default_rng(E + T)
+    lay = MoeLayer(E, k, H, F, activation=synth.STANDARD_SWIGLU, has_bias=False, max_tokens=17, weights_f16=True)
+    for e in range(E):
+        _, gw, uw, dw, *_ = cases.dense_ffn_case(H=H, F=F, T=1, bias=False, seed=e)
+        lay.load_expert_f16(e, uw, gw, dw)
+    hidden = rng.standard_normal((17, H)).astype(np.float32)
+    ro = rng.uniform(0.1, 1.0, (17, k, 2)).astype(np.float32)
+    ro[..., 0] = [rng.permutation(E)[:k] for _ in range(17)]
+    out, _ = lay.forward(hidden, router_out=ro)
+    short, _ = lay.forward(hidden[:T], router_out=ro[:T])
+    assert np.allclose(short, out[:T], rtol=0, atol=2e-2 * out.std())
+    assert np.array_equal(short, out[:T]) == (not few)
+    lay.close()
