@@ -103,15 +103,27 @@ __device__ __forceinline__ void mbar_arrive(uint32_t bar) {
 __device__ __forceinline__ void mbar_expect_tx(uint32_t bar, uint32_t bytes) {
   asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
 }
+// CLUSTER: threads of the other CTA of a cluster arrive on this barrier, too (without a qualifier the wait acquires from its own CTA
+// only; no dearer in k_tile2: 8192 tokens of the 128-expert layer 1.58 ms either way)
+template <bool CLUSTER = false>
 __device__ __forceinline__ bool mbar_try(uint32_t bar, uint32_t parity) {
   uint32_t ok;
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-      "selp.u32 %0, 1, 0, p;\n\t}"
-      : "=r"(ok)
-      : "r"(bar), "r"(parity)
-      : "memory");
+  if (CLUSTER)
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(ok)
+        : "r"(bar), "r"(parity)
+        : "memory");
+  else
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(ok)
+        : "r"(bar), "r"(parity)
+        : "memory");
   return ok != 0;
 }
 // Bounded wait.  Returns false (and raises the CTA's abort flag) when the clock
@@ -132,6 +144,7 @@ __device__ __forceinline__ bool mbar_wait_here(uint32_t bar, uint32_t parity, vo
 // The same with all but the first test in one function that every wait of a kernel shares: kernels of many roles and waits
 // have the less code to fetch (k_tile2 on 2048 tokens of the 128-expert 2048 x 768 layer 97 -> 93 us, k_mx on 16 tokens of
 // it 81 -> 79 for the step), while k_tile, with few waits, loses by it (228 -> 235 us on 8192 tokens) and polls in place.
+template <bool CLUSTER = false>
 static __device__ __noinline__ bool mbar_wait_more(uint32_t bar, uint32_t parity, volatile int* abort_flag) {
   const long long t0 = clock64();
 #pragma unroll 1
@@ -139,15 +152,16 @@ static __device__ __noinline__ bool mbar_wait_more(uint32_t bar, uint32_t parity
     if (*abort_flag) return false;
 #pragma unroll 1
     for (int i = 0; i < 32; ++i)
-      if (mbar_try(bar, parity)) return true;
+      if (mbar_try<CLUSTER>(bar, parity)) return true;
     if (clock64() - t0 > wait_budget()) {
       *abort_flag = 1;
       return false;
     }
   }
 }
+template <bool CLUSTER = false>
 __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatile int* abort_flag) {
-  return mbar_try(bar, parity) || mbar_wait_more(bar, parity, abort_flag);
+  return mbar_try<CLUSTER>(bar, parity) || mbar_wait_more<CLUSTER>(bar, parity, abort_flag);
 }
 // The same for a whole warp that goes on to warp-wide instructions: its lanes agree on whether the wait ran out (each lane
 // reads the clock and the flag for itself).
