@@ -7,6 +7,7 @@
 #include <cstdarg>
 #include <cstdio>
 #include <cstring>
+#include <initializer_list>
 #include <new>
 
 #include "csk_common.cuh"
@@ -1672,17 +1673,43 @@ int csk_moe_route(csk_moe_layer* L, const float* hidden, int64_t T, float* route
 }
 
 namespace {
+// Whether every buffer of a call is page-locked (null: not given).  A copy to or from other memory returns when it is done.
+bool page_locked(std::initializer_list<const void*> buffers) {
+  for (const void* p : buffers) {
+    cudaPointerAttributes at{};
+    if (p && (cudaPointerGetAttributes(&at, p) != cudaSuccess || at.type != cudaMemoryTypeHost)) {
+      cudaGetLastError();
+      return false;
+    }
+  }
+  return true;
+}
+
 // How many equal passes the host entry point cuts a batch into so that the copies of one pass overlap the kernels of another.
-// What stays exposed is the first copy in and the last copy out; what passes cost is kernel time, the less the more rows an
-// expert has (a row tile's cost is nearly flat below 100 rows).  Page-locked buffers, 1 / 2 / 3 / 4 / 8 passes, ms: 128 experts of
-// 2880 x 2880, 4096 tokens (128 rows per expert) 2.59 / 2.27 / - / 2.73 / 3.22, 8192 4.97 / 3.58 / 3.64 / 3.67 / 5.12; 32 experts, 1500
-// (187) 0.97 / 0.84 / - / 1.01 / 1.29, 3000 (375) 1.84 / 1.32 / 1.26 / 1.34 / 1.82, 8192 (1024) 4.82 / 3.40 / 3.03 / 2.75 / 2.57.  (Shorter
-// first and last passes were up to 5 % quicker still, but the certified router adds a token's parts in an order that goes by
-// the pass's size: the low bits of its weights would depend on where in the batch it stands.)
-int host_passes(const csk_moe_layer* L, int64_t T) {
+// Pageable buffers: two from 256 rows per expert on.  Their copies block the caller, so a pass is enqueued only when the one before
+// it has been copied out.  1 / 2 / 4 / 8 passes, ms: 128 experts of 2880 x 2880, 4096 tokens (128 rows per expert) 6.49 / 7.31 /
+// 9.62 / 11.0, 8192 (256) 18.1 / 16.8 / 16.5 / 18.5; 32 experts, 1500 (187) 2.29 / 2.51 / 3.05 / 3.78, 3000 (375) 4.82 / 4.76 / 5.22 / 6.28, 8192
+// (1024) 15.5 / 15.6 / 16.7 / 16.9; 8 of 1728 x 1728, top-2, 2000 (500) 1.58 / 1.69 / 1.89 / 2.31; fp16, 32 of 2880 x 2880, 4096 (512) 8.33 / 8.77
+// / 8.85 / 10.3.
+// Page-locked buffers: two from 128 rows per expert on, one more for every 120.  What stays exposed is the first copy in and the last
+// copy out; what passes cost is kernel time, the less the more rows an expert has (a row tile's cost is nearly flat below 100 rows).
+// 1 / 2 / 3 / 4 / 8 passes, ms: 128 experts of 2880 x 2880, 4096 tokens 2.59 / 2.27 / - / 2.73 / 3.22, 8192 4.97 / 3.58 / 3.64 / 3.67 / 5.12;
+// 32 experts, 1500 0.97 / 0.84 / - / 1.01 / 1.29, 3000 1.84 / 1.32 / 1.26 / 1.34 / 1.82, 8192 4.82 / 3.40 / 3.03 / 2.75 / 2.57; fp16, 32
+// experts, 1500 1.20 / 1.11 / 1.26 / 1.50 / 2.59, 8192 5.41 / 3.84 / 3.57 / 3.56 / 3.77.  But no more than leave a pass items (a row
+// tile x 128 features) for a third of the SMs: below, its kernels take as long as the whole batch's (one fp16 expert of 2880 x 2880, 150
+// tokens 0.19 / 0.23 / 0.25 / 0.30 / 0.43, 1024 0.59 / 0.49 / 0.52 / 0.56 / 0.80).
+// (Shorter first and last passes were up to 5 % quicker still, but the certified router adds a token's parts in an order that goes
+// by the pass's size: the low bits of its weights would depend on where in the batch it stands.)
+int host_passes(const csk_moe_layer* L, int64_t T, std::initializer_list<const void*> buffers) {
   if (L->timing || L->path == CSK_PATH_STREAM) return 1;
-  const int64_t rows_per_expert = T * L->k / std::max(1, L->Eloc);
-  return rows_per_expert < 128 ? 1 : (int)std::max<int64_t>(2, std::min<int64_t>(csk_moe_layer::kMaxPasses, rows_per_expert / 120));
+  const int64_t rows = T * L->k / std::max(1, L->Eloc);  // per expert
+  const int least = rows < 256 ? 1 : 2;
+  if (rows < 128 || !page_locked(buffers)) return least;
+  const int tile_rows = tile_rows_for(L, CSK_PATH_TILE);
+  auto items = [&](int passes) { return (rows / passes + tile_rows - 1) / tile_rows * L->Eloc * L->Tgu.n_tiles; };
+  int passes = (int)std::max<int64_t>(2, std::min<int64_t>(csk_moe_layer::kMaxPasses, rows / 120));
+  while (passes > least && 3 * items(passes) < L->sm_count) --passes;
+  return passes;
 }
 }  // namespace
 
@@ -1693,7 +1720,7 @@ int csk_moe_forward(csk_moe_layer* L, const float* hidden, int64_t T, const floa
   if (T <= 0 || T > L->max_T) return fail(L, CSK_ERR_NOMEM, "T=%lld outside (0, max_tokens]", (long long)T);
   CSK_CUDA(L, cudaSetDevice(L->cfg.device));
   cudaStream_t s = L->stream;
-  const int passes = host_passes(L, T);
+  const int passes = host_passes(L, T, {hidden, router_in, router_out, out});
   if (passes == 1) {
     CSK_CUDA(L, cudaMemcpyAsync(L->d_hidden, hidden, sizeof(float) * T * L->H, cudaMemcpyHostToDevice, s));
     if (router_in)
