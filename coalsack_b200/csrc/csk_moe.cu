@@ -485,11 +485,17 @@ void launch_mx_pair(csk_moe_layer* L, float* y, int ldy, cudaStream_t s, StageTi
 // 48 / 54, at 40 58 / 54; 128 experts of 2048 x 768 at 24 191 / 197, at 32 216 / 203.
 int64_t mx_rows_per_expert(const csk_moe_layer* L) { return std::min(kMxTileRows, 20 + std::min(L->H, L->F) / 128); }
 
+// Rows the block-scaled kernel's images have to hold when a layer is created: the batches the kernel takes by itself, or every
+// batch where no cluster of two CTAs can be resident (an MXFP4 layer has no other kernel then, whatever path is asked for).
+int64_t mx_rows_own(const csk_moe_layer* L) {
+  return L->pair.available ? std::min(L->max_rows, mx_rows_per_expert(L) * L->Eloc) : L->max_rows;
+}
+
 int choose_path(const csk_moe_layer* L, int64_t rows) {
   if (L->w16) return CSK_PATH_TILE;  // fp16 weights exist in the tensor-core layout only
-  if (L->path == CSK_PATH_STREAM) return CSK_PATH_STREAM;
+  if (L->path == CSK_PATH_STREAM || !L->pair.available) return CSK_PATH_STREAM;
   if (L->path == CSK_PATH_TILE || L->path == CSK_PATH_TILE_PAIR) return CSK_PATH_TILE;
-  return (L->pair.available && rows >= mx_rows_per_expert(L) * std::max(1, L->Eloc)) ? CSK_PATH_TILE : CSK_PATH_STREAM;
+  return (rows >= mx_rows_per_expert(L) * std::max(1, L->Eloc)) ? CSK_PATH_TILE : CSK_PATH_STREAM;
 }
 
 // The expert-parallel receive side: the block-scaled kernel needs images for every row that may come (`most`).
@@ -897,8 +903,7 @@ int csk_moe_create(const csk_moe_config* cfg, csk_moe_layer** out) {
       return rc;
     }
   }
-  // images for the batches the block-scaled kernel takes by itself
-  if (mx_reserve(L, std::min(L->max_rows, mx_rows_per_expert(L) * eloc))) {
+  if (mx_reserve(L, mx_rows_own(L))) {
     fail(nullptr, CSK_ERR_NOMEM, "%s", L->err.c_str());
     csk_moe_destroy(L);
     return CSK_ERR_NOMEM;
@@ -2358,6 +2363,13 @@ int csk_moe_debug_set(csk_moe_layer* L, int32_t key, int64_t value) {
   if (key == CSK_DEBUG_STALL_ROUTER) {
     L->debug_stall_router = value != 0;
     return CSK_OK;
+  }
+  if (key == CSK_DEBUG_NO_CLUSTERS) {
+    if (!value) return fail(L, CSK_ERR_INVALID, "debug: clusters do not come back");
+    L->pair.available = false;
+    L->pair.err = "turned off by a test";
+    drop_graphs(L);
+    return mx_reserve(L, mx_rows_own(L));
   }
   return fail(L, CSK_ERR_INVALID, "debug: unknown key %d", key);
 }

@@ -373,7 +373,7 @@ class MoeLayer:
         self._check(self._lib.csk_moe_get_router_stats(self._h, C.byref(a), C.byref(b)))
         return a.value, b.value
 
-    DEBUG_WAIT_BUDGET, DEBUG_STALL_TILE_PRODUCER, DEBUG_STALL_ROUTER = 0, 1, 2
+    DEBUG_WAIT_BUDGET, DEBUG_STALL_TILE_PRODUCER, DEBUG_STALL_ROUTER, DEBUG_NO_CLUSTERS = 0, 1, 2, 3
 
     def debug_set(self, key, value):
         """Test hooks of the failure path (csk_moe_debug_set)."""

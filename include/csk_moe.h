@@ -50,7 +50,8 @@ enum {
   CSK_PATH_AUTO = 0,
   CSK_PATH_STREAM = 1,      /* weight-streaming kernel (few rows per expert)                    */
   CSK_PATH_TILE = 2,        /* fp16 tensor-core kernel: MXFP4 weights on CTA pairs, fp16 weights one CTA per work item */
-  CSK_PATH_TILE_PAIR = 3    /* the same, for MXFP4 layers only                                   */
+  CSK_PATH_TILE_PAIR = 3    /* the same, for MXFP4 layers only; refused where no cluster of two CTAs can be resident
+                               (the weight-streaming kernel serves every batch of MXFP4 layers there)        */
 };
 
 /* Layer description: graph_builder::config num_experts / expert_top_k /
@@ -429,8 +430,10 @@ int csk_moe_get_counters(csk_moe_layer* layer, int64_t* rows_per_expert, int64_t
  *                                 role's wait runs out, the kernel tears down and the call
  *                                 reports CSK_ERR_DEVICE (one shot)
  *   CSK_DEBUG_STALL_ROUTER        the same in the NEXT tensor-core router launch (large
- *                                 batches in certified mode) */
-enum { CSK_DEBUG_WAIT_BUDGET = 0, CSK_DEBUG_STALL_TILE_PRODUCER = 1, CSK_DEBUG_STALL_ROUTER = 2 };
+ *                                 batches in certified mode)
+ *   CSK_DEBUG_NO_CLUSTERS         non-zero: the handle goes on as on a device where no
+ *                                 cluster of two CTAs can be resident */
+enum { CSK_DEBUG_WAIT_BUDGET = 0, CSK_DEBUG_STALL_TILE_PRODUCER = 1, CSK_DEBUG_STALL_ROUTER = 2, CSK_DEBUG_NO_CLUSTERS = 3 };
 int csk_moe_debug_set(csk_moe_layer* layer, int32_t key, int64_t value);
 
 #ifdef __cplusplus

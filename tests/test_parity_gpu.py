@@ -4,7 +4,7 @@ inputs, and the reference itself where its compiled wrapper travelled along."""
 import numpy as np
 import pytest
 
-from coalsack_b200 import (CskError, MoeLayer, PATH_STREAM, PATH_TILE, PATH_TILE_PAIR, expert_merge_node, expert_mlp_node,
+from coalsack_b200 import (CskError, MoeLayer, PATH_AUTO, PATH_STREAM, PATH_TILE, PATH_TILE_PAIR, expert_merge_node, expert_mlp_node,
                            moe_router_node, synth)
 from tests import cases
 
@@ -617,3 +617,34 @@ def test_weight_image_of_the_earlier_layout_still_loads(gpu_lib, tmp_path, f16):
         got.load_image(older)
     for x in (lay, got):
         x.close()
+
+
+def test_layers_where_no_cluster_can_be_resident(gpu_lib, port):
+    """MXFP4 prefill runs on CTA pairs; without them the block-scaled kernel serves every batch, also one that asks for the
+    tensor-core kernel by name, and the pair kernel is refused."""
+    sh = synth.tiny(seed=63, E=4, k=2, H=256, F=192, T=300, has_bias=True)
+    h, Wg, rb, ex = cases.layer_inputs(sh, router_scale=40.0)
+    lay = make_layer(sh, Wg, rb, ex)
+    want, want_ro = port.moe_layer(h, Wg, rb, ex, 2, sh.act, nthreads=8)
+    lay.debug_set(lay.DEBUG_NO_CLUSTERS, 1)
+    with pytest.raises(CskError, match="CTA-pair kernel is not available"):
+        lay.set_path(PATH_TILE_PAIR)
+    for path in (PATH_AUTO, PATH_TILE):
+        lay.set_path(path)
+        out, ro = lay.forward(h)
+        assert same_experts(ro, want_ro)
+        assert_close(out, want, f"no clusters, path {path}")
+        assert lay.timings()["path"] == PATH_STREAM
+    # ... and rows received from peers (one rank that owns every expert)
+    import torch
+    T, k, H = h.shape[0], 2, sh.hidden
+    send = torch.zeros((T * k, lay.ep_row_pitch()), dtype=torch.float16, device="cuda")
+    counts = torch.zeros(4, dtype=torch.int32, device="cuda")
+    back, out = torch.zeros((T * k, H), device="cuda"), torch.empty((T, H), device="cuda")
+    torch.cuda.synchronize()
+    lay.ep_dispatch_dev(torch.from_numpy(h).cuda(), T, send, counts)
+    lay.ep_experts_dev(send, counts, 1, T * k, back)
+    lay.ep_combine_dev(back, T, out)
+    lay.sync()
+    assert_close(out.cpu().numpy(), want, "no clusters, received rows")
+    lay.close()
