@@ -174,6 +174,10 @@ int fail(csk_moe_layer* L, int code, const char* fmt, ...) {
                   __FILE__, __LINE__);                                                       \
   } while (0)
 
+// Bytes of an expert's tensor-core codes in the order of the file images (fp16 weights are in that order on the device, too).  The
+// first staging area holds them, so that images can be written and read when the device is full.
+size_t image_part_bytes(const csk_moe_layer* L) { return L->w16 ? 0 : L->off_bias - L->off_tgu; }
+
 int grid_for(size_t work_items, int threads, int cap) {
   size_t b = (work_items + threads - 1) / threads;
   return (int)std::max<size_t>(1, std::min<size_t>(b, (size_t)cap));
@@ -833,7 +837,7 @@ int csk_moe_create(const csk_moe_config* cfg, csk_moe_layer** out) {
   CK(cudaMalloc(&L->d_resident, eloc));
   CK(cudaMemset(L->d_resident, 0, eloc));
   L->stage_bytes = L->w16 ? (size_t)L->H * L->F * 2 : (size_t)L->H * L->F / 32 * 17;
-  CK(cudaMalloc(&L->d_stage, 3 * L->stage_bytes));
+  CK(cudaMalloc(&L->d_stage, std::max(3 * L->stage_bytes, image_part_bytes(L))));
   CK(cudaMalloc(&L->d_wg, sizeof(float) * L->E * L->H));
   CK(cudaMalloc(&L->d_wg_few, sizeof(float) * router_packed_floats(L->E, L->H, kRouterChunkFew)));
   CK(cudaMalloc(&L->d_wg_many, sizeof(float) * router_packed_floats(L->E, L->H, kRouterChunkMany)));
@@ -1267,28 +1271,16 @@ ImageHeader image_header_02(const csk_moe_layer* L) {
   h.expert_stride = (h.off_meta + 16 + 255) / 256 * 256;
   return h;
 }
-// An expert's tensor-core codes to the file's order (from the device into `dst`) or from it (from `src` to the device).
-int reorder_tiles_enqueue(csk_moe_layer* L, int le, uint8_t* part, bool to_file, cudaStream_t s) {
+// An expert's tensor-core codes to the file's order (from the device into the staging area) or from it (and back).
+int reorder_tiles_enqueue(csk_moe_layer* L, int le, bool to_file, cudaStream_t s) {
   uint8_t* base = L->d_weights + (size_t)le * L->expert_stride + L->off_tgu;
+  uint8_t* part = L->d_stage;
   for (const auto& [lay, at] : {std::pair{L->Tgu, (size_t)0}, std::pair{L->Td, L->off_td - L->off_tgu}})
     k_reorder_tile<<<grid_for(lay.bytes() / 34, 256, 4096), 256, 0, s>>>(to_file ? base + at : part + at, to_file ? part + at : base + at, lay,
                                                                        to_file);
   CSK_CUDA(L, cudaGetLastError());
   return CSK_OK;
 }
-// Device memory for one expert's tensor-core codes in the file's order, for the time of a save or a load.
-struct ImagePart {
-  uint8_t* p = nullptr;
-  size_t bytes = 0;
-  explicit ImagePart(const csk_moe_layer* L) : bytes(L->w16 ? 0 : L->off_bias - L->off_tgu) {
-    if (bytes && cudaMalloc(&p, bytes) != cudaSuccess) {
-      cudaGetLastError();
-      p = nullptr;
-    }
-  }
-  bool ok() const { return p || !bytes; }
-  ~ImagePart() { cudaFree(p); }
-};
 // The decode kernel's copy of a resident expert's codes from the other kernel's tiles (which hold the blocks losslessly).
 int rebuild_mx_enqueue(csk_moe_layer* L, int le, cudaStream_t s) {
   uint8_t* base = L->d_weights + (size_t)le * L->expert_stride;
@@ -1309,8 +1301,7 @@ int csk_moe_save_image(csk_moe_layer* L, const char* path) {
   if (check_layer(L)) return CSK_ERR_INVALID;
   if (!path) return fail(L, CSK_ERR_INVALID, "null path");
   CSK_CUDA(L, cudaSetDevice(L->cfg.device));
-  ImagePart part(L);
-  if (!part.ok()) return fail(L, CSK_ERR_NOMEM, "no device memory to write the weight image");
+  const size_t part = image_part_bytes(L);
   FILE* f = fopen(path, "wb");
   if (!f) return fail(L, CSK_ERR_INVALID, "cannot open %s for writing", path);
   const ImageHeader h = image_header_of(L);
@@ -1318,9 +1309,9 @@ int csk_moe_save_image(csk_moe_layer* L, const char* path) {
   std::vector<uint8_t> buf(L->expert_stride);
   for (int e = 0; ok && e < L->Eloc; ++e) {
     if (cudaMemcpy(buf.data(), L->d_weights + (size_t)e * L->expert_stride, L->expert_stride, cudaMemcpyDeviceToHost) != cudaSuccess) ok = false;
-    if (ok && part.bytes) {
-      ok = reorder_tiles_enqueue(L, e, part.p, true, L->stream) == CSK_OK && cudaStreamSynchronize(L->stream) == cudaSuccess &&
-           cudaMemcpy(buf.data() + L->off_tgu, part.p, part.bytes, cudaMemcpyDeviceToHost) == cudaSuccess;
+    if (ok && part) {
+      ok = reorder_tiles_enqueue(L, e, true, L->stream) == CSK_OK && cudaStreamSynchronize(L->stream) == cudaSuccess &&
+           cudaMemcpy(buf.data() + L->off_tgu, L->d_stage, part, cudaMemcpyDeviceToHost) == cudaSuccess;
     }
     ok = ok && fwrite(buf.data(), 1, buf.size(), f) == buf.size();
   }
@@ -1333,8 +1324,7 @@ int csk_moe_load_image(csk_moe_layer* L, const char* path) {
   if (check_layer(L)) return CSK_ERR_INVALID;
   if (!path) return fail(L, CSK_ERR_INVALID, "null path");
   CSK_CUDA(L, cudaSetDevice(L->cfg.device));
-  ImagePart part(L);
-  if (!part.ok()) return fail(L, CSK_ERR_NOMEM, "no device memory to read the weight image");
+  const size_t part = image_part_bytes(L);
   FILE* f = fopen(path, "rb");
   if (!f) return fail(L, CSK_ERR_INVALID, "cannot open %s", path);
   ImageHeader h{};
@@ -1355,9 +1345,9 @@ int csk_moe_load_image(csk_moe_layer* L, const char* path) {
     ok = fread(buf.data(), 1, buf.size(), f) == buf.size();
     // (on the handle's stream, which does not wait for the default one: a plain copy may still be landing when it returns)
     ok = ok && cudaMemcpyAsync(base + to, buf.data() + from, h.off_meta + 16 - from, cudaMemcpyHostToDevice, L->stream) == cudaSuccess;
-    if (ok && part.bytes)
-      ok = cudaMemcpyAsync(part.p, base + L->off_tgu, part.bytes, cudaMemcpyDeviceToDevice, L->stream) == cudaSuccess &&
-           reorder_tiles_enqueue(L, e, part.p, false, L->stream) == CSK_OK;
+    if (ok && part)
+      ok = cudaMemcpyAsync(L->d_stage, base + L->off_tgu, part, cudaMemcpyDeviceToDevice, L->stream) == cudaSuccess &&
+           reorder_tiles_enqueue(L, e, false, L->stream) == CSK_OK;
     if (ok && rebuild && res[e]) ok = rebuild_mx_enqueue(L, e, L->stream) == CSK_OK;
     ok = cudaStreamSynchronize(L->stream) == cudaSuccess && ok;
   }

@@ -648,3 +648,47 @@ def test_layers_where_no_cluster_can_be_resident(gpu_lib, port):
     lay.sync()
     assert_close(out.cpu().numpy(), want, "no clusters, received rows")
     lay.close()
+
+
+def test_weight_image_with_a_full_device(gpu_lib, tmp_path):
+    """Images are written and read without device memory of their own: a server's caches may hold all of it."""
+    import torch
+    sh = synth.tiny(seed=59, E=2, k=1, H=2880, F=2880, T=8, has_bias=True)
+    ex = synth.all_experts(sh)
+    lay, other = MoeLayer.from_shape(sh), MoeLayer.from_shape(sh)
+    lay.load_experts(ex)
+    a, b = tmp_path / "a.img", tmp_path / "b.img"
+    lay.save_image(a)
+    other.load_image(a)  # (every kernel of both is on the device now)
+    held, size = [], 1 << 34
+    while size >= 1 << 21:
+        try:
+            held.append(torch.empty(size, dtype=torch.uint8, device="cuda"))
+        except torch.OutOfMemoryError:
+            size >>= 1
+    try:
+        assert torch.cuda.mem_get_info()[0] < 12 << 20
+        lay.save_image(b)
+        other.load_image(b)
+    finally:
+        del held
+        torch.cuda.empty_cache()
+    assert a.read_bytes() == b.read_bytes()
+    for which in range(6):
+        assert np.array_equal(other.unpack_expert(1, which), lay.unpack_expert(1, which))
+    lay.close()
+    other.close()
+
+
+@pytest.mark.parametrize("H,F", [(32, 32), (32, 160), (96, 32), (64, 2080)])
+def test_weight_image_of_shapes_that_are_mostly_padding(gpu_lib, tmp_path, H, F):
+    sh = synth.tiny(seed=61, E=2, k=1, H=H, F=F, T=8, has_bias=True)
+    ex = synth.all_experts(sh)
+    lay, other = MoeLayer.from_shape(sh), MoeLayer.from_shape(sh)
+    lay.load_experts(ex)
+    lay.save_image(tmp_path / "a.img")
+    other.load_image(tmp_path / "a.img")
+    for which in range(6):
+        assert np.array_equal(other.unpack_expert(1, which), lay.unpack_expert(1, which))
+    lay.close()
+    other.close()
