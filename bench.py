@@ -172,6 +172,10 @@ def run_reference(args):
     rank = int(os.environ.get("RANK", "0"))
     if rank != 0:
         return
+    import oracle
+    if not oracle.have_ref():  # (its restatement is not the reference: it would be timed under the wrong name)
+        print(json.dumps({"impl": "reference", "unavailable": "the reference's sources are not here: oracle/_ref was never compiled"}))
+        return
     sh, total = per_rank_shape(args, args.gpus)
     cb, ms = time_reference(sh.with_(tokens=total), args.steps, args.warmup)
     line = {"impl": "reference", "metric": METRIC, "value": cb["value"], "unit": UNIT, "n_gpus": args.gpus,
