@@ -27,22 +27,27 @@ def test_dense(gpu_lib, port, H, F, bias, T):
     node.close()
 
 
-@pytest.mark.parametrize("E,k,T", [(5, 1, 3), (5, 2, 20), (40, 4, 64)])
-def test_experts(gpu_lib, port, E, k, T):
+@pytest.mark.parametrize("E,k,T,wbf", [
+    (5, 1, 3, False), (5, 2, 8, False), (5, 2, 9, True), (40, 2, 16, False), (40, 4, 16, True),  # the streaming kernel
+    (5, 2, 17, False), (5, 2, 20, False), (40, 4, 64, True),                                  # the tensor-core kernel
+])
+def test_experts(gpu_lib, port, E, k, T, wbf):
     """Routed fp16 experts: more tiles than rows and fewer, experts without rows, a row that is not finite touches no other."""
     H, F = 288, 160
     rng = np.random.default_rng(E + T)
     hidden = rng.standard_normal((T, H)).astype(np.float32)
     experts = [cases.dense_ffn_case(H=H, F=F, T=1, bias=True, seed=900 + e)[1:] for e in range(E)]
-    lay = MoeLayer(E, k, H, F, activation=synth.STANDARD_SWIGLU, has_bias=True, max_tokens=T, weights_f16=True)
+    lay = MoeLayer(E, k, H, F, activation=synth.STANDARD_SWIGLU, has_bias=True, max_tokens=T, weights_f16=True, weight_before_ffn=wbf)
     lay.set_router((rng.standard_normal((E, H)) * 0.3).astype(np.float32), None)
     for e, (gw, uw, dw, bg, bu, bd) in enumerate(experts):
         lay.load_expert_f16(e, uw, gw, dw, bu, bg, bd)
     out, ro = lay.forward(hidden)
-    dense = [port.dense_ffn(hidden, *w) for w in experts]
     want = np.zeros((T, H), np.float32)
     for j in range(k):
-        want += ro[:, j, 1:] * np.stack([dense[int(e)][t] for t, e in enumerate(ro[:, j, 0])])
+        w = ro[:, j, 1:]
+        for e in set(ro[:, j, 0].astype(int)):
+            on = ro[:, j, 0] == e
+            want[on] += port.dense_ffn(w[on] * hidden[on], *experts[e]) if wbf else w[on] * port.dense_ffn(hidden[on], *experts[e])
     mx, mr = cases.err_stats(out, want)
     assert mx <= cases.MAX_ABS_OVER_RMS and mr <= cases.MEAN_REL, (mx, mr)
     bad = hidden.copy()

@@ -3,7 +3,7 @@ padding end, against the CPU restatement of the reference."""
 import numpy as np
 import pytest
 
-from coalsack_b200 import MoeLayer, PATH_STREAM, PATH_TILE, PATH_TILE_PAIR, synth
+from coalsack_b200 import MoeLayer, PATH_STREAM, PATH_TILE, synth
 from tests import cases
 
 pytestmark = pytest.mark.gpu
@@ -192,7 +192,7 @@ def _scaled(blocks, by):
 
 
 @pytest.mark.parametrize("act", [0, 1])
-@pytest.mark.parametrize("path", [PATH_STREAM, PATH_TILE, PATH_TILE_PAIR])
+@pytest.mark.parametrize("path", [PATH_STREAM, PATH_TILE])
 @pytest.mark.parametrize("bad", [np.inf, -np.inf, np.nan])
 def test_a_row_that_is_not_finite_does_not_come_out_finite(gpu_lib, port, act, path, bad):
     """With the routing given by the caller nothing before the experts looks at the row: where the restatement's result is

@@ -254,7 +254,7 @@ def test_many_rows_one_expert_and_ragged(gpu_lib, port):
     assert rows[0] > 250 and rows[5:].sum() == 0 and rows.sum() == 600
     want, _ = port.moe_layer(h, Wg, rb, ex, 2, sh.act, nthreads=8, router_out=ro)
     assert_close(out, want, "skewed")
-    for path in (PATH_STREAM, PATH_TILE, PATH_TILE_PAIR):
+    for path in (PATH_STREAM, PATH_TILE):
         lay.set_path(path)
         out2, _ = lay.forward(h, router_out=ro)
         assert_close(out2, want, f"skewed path {path}")
@@ -326,15 +326,11 @@ def test_expert_node_empty_and_dense(gpu_lib, golden):
 
 
 # ---- the tensor-core (tcgen05) kernel, forced --------------------------------------
-TILE_KERNELS = [pytest.param(PATH_TILE, id="one_cta"), pytest.param(PATH_TILE_PAIR, id="cta_pair")]
-
-
-@pytest.mark.parametrize("tile", TILE_KERNELS)
 @pytest.mark.parametrize("tag", list(cases.TINY_CASES))
-def test_tile_path_tiny_layers(gpu_lib, golden, tag, tile):
+def test_tile_path_tiny_layers(gpu_lib, golden, tag):
     sh, h, Wg, rb, ex, wbf = cases.tiny_case(tag)
     lay = make_layer(sh, Wg, rb, ex, wbf)
-    lay.set_path(tile)
+    lay.set_path(PATH_TILE)
     out, ro = lay.forward(h)
     assert lay.timings()["path"] == PATH_TILE
     assert same_experts(ro, golden[f"{tag}_router"])
@@ -350,12 +346,11 @@ def test_tile_path_tiny_layers(gpu_lib, golden, tag, tile):
     lay.close()
 
 
-@pytest.mark.parametrize("tile", TILE_KERNELS)
-def test_tile_path_c0(gpu_lib, golden, port, tile):
+def test_tile_path_c0(gpu_lib, golden, port):
     sh = synth.C0
     h, Wg, rb, ex = cases.layer_inputs(sh, 32)
     lay = make_layer(sh, Wg, rb, ex, max_tokens=32)
-    lay.set_path(tile)
+    lay.set_path(PATH_TILE)
     out1, ro1 = lay.forward(h[:1])
     assert_close(out1, golden["c0_t1_out"], "c0 T=1 tile")
     out32, ro32 = lay.forward(h)
@@ -363,6 +358,8 @@ def test_tile_path_c0(gpu_lib, golden, port, tile):
     assert_close(out32[:4], golden["c0_t32_out_first4"], "c0 T=32 tile")
     want, _ = port.moe_layer(h, Wg, rb, ex, sh.top_k, sh.act, nthreads=8, router_out=ro32)
     assert_close(out32, want, "c0 T=32 tile, all rows")
+    lay.set_path(PATH_TILE_PAIR)  # the same kernel by its other name
+    assert np.array_equal(lay.forward(h)[0], out32)
     lay.close()
 
 
@@ -376,7 +373,7 @@ def test_tile_path_wide_exponents(gpu_lib, port):
         ex["w_down"][e] = synth.mxfp4_matrix(sh.seed, synth._T_WDOWN, e, 128, 128, 100, 136)
     lay = make_layer(sh, Wg, rb, ex, max_tokens=200)
     want = None
-    for path in (PATH_TILE, PATH_TILE_PAIR, PATH_STREAM):
+    for path in (PATH_TILE, PATH_STREAM):
         lay.set_path(path)
         out, ro = lay.forward(h)
         if want is None:
@@ -410,7 +407,7 @@ def test_edge_scale_bytes(gpu_lib, port):
             want_blocks[want_blocks[:, 0] == 255, 0] = 254   # the streaming layout stores 255 as what it is read as
         assert np.array_equal(lay.unpack_expert(1, which), want_blocks.reshape(-1)), which
     want = None
-    for path in (PATH_STREAM, PATH_TILE, PATH_TILE_PAIR):
+    for path in (PATH_STREAM, PATH_TILE):
         lay.set_path(path)
         out, ro = lay.forward(h)
         if want is None:
@@ -421,16 +418,23 @@ def test_edge_scale_bytes(gpu_lib, port):
     lay.close()
 
 
-@pytest.mark.parametrize("tile", TILE_KERNELS)
-def test_bounded_wait_runs_out_and_the_handle_recovers(gpu_lib, port, tile):
-    """The failure path of the tensor-core kernel, made to happen without any fault: the wait budget is
+@pytest.mark.parametrize("f16", [pytest.param(False, id="mxfp4"), pytest.param(True, id="fp16")])
+def test_bounded_wait_runs_out_and_the_handle_recovers(gpu_lib, port, f16):
+    """The failure path of the tensor-core kernels (CTA pairs for MXFP4 weights, one CTA for fp16 ones), made to happen without any fault: the wait budget is
     cut to 0.1 ms and the next launch's copy role is told to issue nothing, so the MMA, dequantiser and
     epilogue roles all wait on barriers that nothing arms, give up, tear down (tensor memory freed) and
     the call returns CSK_ERR_DEVICE.  The same handle then computes the layer correctly."""
-    sh = synth.tiny(seed=49, E=4, k=2, H=128, F=128, T=96, has_bias=True)
+    sh = synth.tiny(seed=49, E=4, k=2, H=128, F=128, T=96, has_bias=True, act=synth.STANDARD_SWIGLU if f16 else synth.MODIFIED_SWIGLU)
     h, Wg, rb, ex = cases.layer_inputs(sh, router_scale=50.0)
-    lay = make_layer(sh, Wg, rb, ex, max_tokens=sh.tokens)
-    lay.set_path(tile)
+    if f16:
+        w16 = [cases.dense_ffn_case(H=128, F=128, T=1, bias=True, seed=490 + e)[1:] for e in range(4)]
+        lay = MoeLayer.from_shape(sh, weights_f16=True)
+        lay.set_router(Wg, rb)
+        for e, (gw, uw, dw, bg, bu, bd) in enumerate(w16):
+            lay.load_expert_f16(e, uw, gw, dw, bu, bg, bd)
+    else:
+        lay = make_layer(sh, Wg, rb, ex, max_tokens=sh.tokens)
+        lay.set_path(PATH_TILE)
     good, ro = lay.forward(h)
     try:
         lay.debug_set(lay.DEBUG_WAIT_BUDGET, 200_000)
@@ -442,7 +446,11 @@ def test_bounded_wait_runs_out_and_the_handle_recovers(gpu_lib, port, tile):
         lay.debug_set(lay.DEBUG_WAIT_BUDGET, 2_000_000_000)
     again, ro2 = lay.forward(h)
     assert np.array_equal(ro, ro2) and np.array_equal(good, again)
-    want, _ = port.moe_layer(h, Wg, rb, ex, sh.top_k, sh.act, nthreads=8, router_out=ro)
+    if f16:
+        dense = [port.dense_ffn(h, *w) for w in w16]
+        want = sum(ro[:, j, 1:] * np.stack([dense[int(e)][t] for t, e in enumerate(ro[:, j, 0])]) for j in range(sh.top_k))
+    else:
+        want, _ = port.moe_layer(h, Wg, rb, ex, sh.top_k, sh.act, nthreads=8, router_out=ro)
     assert_close(again, want, "after the aborted call")
     lay.close()
 
