@@ -1393,7 +1393,7 @@ int csk_moe_set_path(csk_moe_layer* L, int32_t path) {
   if (check_layer(L)) return CSK_ERR_INVALID;
   if (path < CSK_PATH_AUTO || path > CSK_PATH_TILE_PAIR) return fail(L, CSK_ERR_INVALID, "unknown path %d", path);
   if (L->w16 && (path == CSK_PATH_STREAM || path == CSK_PATH_TILE_PAIR))
-    return fail(L, CSK_ERR_INVALID, "fp16 weights run on the one-CTA tensor-core kernel only");
+    return fail(L, CSK_ERR_INVALID, "fp16 weights have no weight-streaming and no CTA-pair kernel");
   if (path == CSK_PATH_TILE_PAIR && !L->pair.available)
     return fail(L, CSK_ERR_INVALID, "the CTA-pair kernel is not available on this device: %s", L->pair.err.c_str());
   CSK_CUDA(L, cudaSetDevice(L->cfg.device));

@@ -479,7 +479,7 @@ class EpBench:
         limiting = max(stage_max, key=stage_max.get) if stage_max else None
         out.update(route_ms=0.0, permute_ms=0.0, combine_ms=0.0, total_ms=out["gate_up_ms"] + out["down_ms"],
                    path={1: "stream", 2: "tile"}.get(int(path), "?"), launches=14, rows_received=int(rows))
-        out["gate_up_kernel"] = "k_mx<gated>" if out["path"] == "stream" else "k_tile<gated>"
+        out["gate_up_kernel"] = "k_mx<gated>" if out["path"] == "stream" else "k_tile2<gated>"
         out["ep"] = {"stages_ms_max_over_ranks": stage_max,
                      "stages_note": "max over ranks; the gather of the counts and the two barriers as the last "
                                     "rank to arrive saw them (min over ranks)",

@@ -49,7 +49,8 @@ enum { CSK_ACT_MODIFIED_SWIGLU = 0, CSK_ACT_STANDARD_SWIGLU = 1 };
 enum {
   CSK_PATH_AUTO = 0,
   CSK_PATH_STREAM = 1,      /* weight-streaming kernel (few rows per expert)                    */
-  CSK_PATH_TILE = 2,        /* fp16 tensor-core kernel: MXFP4 weights on CTA pairs, fp16 weights one CTA per work item */
+  CSK_PATH_TILE = 2,        /* fp16 operands: MXFP4 weights on CTA pairs; fp16 weights one CTA per work item, or the
+                               kernel for few token rows                                                       */
   CSK_PATH_TILE_PAIR = 3    /* the same, for MXFP4 layers only; refused where no cluster of two CTAs can be resident
                                (the weight-streaming kernel serves every batch of MXFP4 layers there)        */
 };
@@ -59,10 +60,12 @@ enum {
  * plus the per-node settings (moe_router_node.h:27-34, expert_mlp_node.h:44-52,
  * expert_merge_node.h:17-24). */
 /* How the experts' weight matrices arrive:
- *   CSK_WEIGHTS_MXFP4  17-byte MXFP4 blocks (csk_moe_load_expert_mxfp4); both expert kernels.
+ *   CSK_WEIGHTS_MXFP4  17-byte MXFP4 blocks (csk_moe_load_expert_mxfp4); the weight-streaming kernel and the
+ *                      tensor-core kernel on CTA pairs.
  *   CSK_WEIGHTS_F16    fp16 row-major matrices (csk_moe_load_expert_f16): the reference's fp16 expert
  *                      slices (expert_mlp_node.h:533-647) and, with num_experts = top_k = 1, its dense
- *                      shared-expert FFN (dense_ffn_node.h:28-219).  Tensor-core kernel only. */
+ *                      shared-expert FFN (dense_ffn_node.h:28-219).  The one-CTA tensor-core kernel and, for few
+ *                      token rows, a kernel of its own. */
 enum { CSK_WEIGHTS_MXFP4 = 0, CSK_WEIGHTS_F16 = 1 };
 
 typedef struct csk_moe_config {

@@ -99,7 +99,7 @@ def test_dense_ffn_errors(gpu_lib):
         node.compute([hidden[None], gw, uw[:-32], dw])
     with pytest.raises(RuntimeError, match="FLOAT16"):
         node.compute([hidden[None], gw.astype(np.float64), uw.astype(np.float64), dw.astype(np.float64)])
-    # the two weight formats do not mix, and fp16 layers have the one-CTA tensor-core kernel only
+    # the two weight formats do not mix, and fp16 layers have neither the weight-streaming nor the CTA-pair kernel
     lay = MoeLayer(1, 1, 256, 192, activation=1, has_bias=False, max_tokens=16, weights_f16=True)
     with pytest.raises(CskError, match="fp16 weights"):
         lay.load_expert(0, np.zeros(256 * 192 // 32 * 17, np.uint8), np.zeros(256 * 192 // 32 * 17, np.uint8),
