@@ -19,14 +19,16 @@ namespace csk {
 // softmax over the selected logits (or sigmoid) exactly as the reference.
 // ---------------------------------------------------------------------------
 constexpr int kRouterPad = 4;       // row stride 4 mod 32 words: a quarter-warp's 128-bit loads hit distinct banks
-// ring depth: four stages, three for the widest blocks (shared memory for two blocks per SM)
-__host__ __device__ constexpr int router_stages(int tokens_per_block) { return tokens_per_block >= 32 ? 3 : 4; }
+// Columns of a stage: few / many tokens, and the ring's stages.  A stage costs a lone chain some 250 cycles: 192 columns and four stages 12.0 us
+// (8 tokens, 32 experts, 2880 columns, back to back), 288 or 384 and three 11.2, 96 and six 13.9; of 256 two blocks fit an SM.
+constexpr int kRouterChunkFew = 256, kRouterChunkMany = 128;
+__host__ __device__ constexpr int router_stages(int ch) { return ch > 128 ? 3 : 4; }
 constexpr int kMaxTopK = 16;
 constexpr int kMaxExperts = 1024;
 
-// ch = columns of the hidden dimension per pipeline stage
-inline size_t router_smem_bytes(int tokens_per_block, int ch) {
-  return (size_t)router_stages(tokens_per_block) * (32 + tokens_per_block) * (ch + kRouterPad) * sizeof(float) + 128;
+// ch = columns of the hidden dimension per pipeline stage; experts: of the logits that the blocks of a cluster exchange (twice), 0 without one
+inline size_t router_smem_bytes(int tokens_per_block, int ch, int experts) {
+  return ((size_t)router_stages(ch) * (32 + tokens_per_block) * (ch + kRouterPad) + 2 * (size_t)tokens_per_block * experts) * sizeof(float) + 128;
 }
 
 __device__ __forceinline__ void cp_async16(uint32_t smem_dst, const void* gsrc) {
@@ -73,14 +75,9 @@ __global__ void k_pack_router(const float* __restrict__ wg, float* __restrict__ 
 // they are the block's own shared memory.
 // NV: logits per lane (E <= 32 * NV); the selection loops are unrolled over it.
 template <bool CG, int NV>
-__device__ __forceinline__ bool warp_topk_nv(const float* __restrict__ l, int E, int k, int sigmoid,
-                                             float* __restrict__ out /* [k][2] */,
-                                             const float* __restrict__ bounds) {
+__device__ __forceinline__ bool warp_topk_regs(float (&v)[NV], int E, int k, int sigmoid, float* __restrict__ out /* [k][2] */,
+                                               const float* __restrict__ bounds) {
   const int lane = threadIdx.x & 31;
-  float v[NV];
-#pragma unroll
-  for (int i = 0; i < NV; ++i)
-    v[i] = (i * 32 < E && i * 32 + lane < E) ? (CG ? __ldcg(l + i * 32 + lane) : l[i * 32 + lane]) : -INFINITY;
   float my_v = -INFINITY;
   int my_i = 0x7fffffff;
   uint32_t gone = 0;
@@ -150,6 +147,18 @@ __device__ __forceinline__ bool warp_topk_nv(const float* __restrict__ l, int E,
   return certified;
 }
 
+template <bool CG, int NV>
+__device__ __forceinline__ bool warp_topk_nv(const float* __restrict__ l, int E, int k, int sigmoid,
+                                             float* __restrict__ out /* [k][2] */,
+                                             const float* __restrict__ bounds) {
+  const int lane = threadIdx.x & 31;
+  float v[NV];
+#pragma unroll
+  for (int i = 0; i < NV; ++i)
+    v[i] = (i * 32 < E && i * 32 + lane < E) ? (CG ? __ldcg(l + i * 32 + lane) : l[i * 32 + lane]) : -INFINITY;
+  return warp_topk_regs<CG, NV>(v, E, k, sigmoid, out, bounds);
+}
+
 template <bool CG = true>
 __device__ __forceinline__ bool warp_topk(const float* __restrict__ l, int E, int k, int sigmoid,
                                           float* __restrict__ out /* [k][2] */,
@@ -170,6 +179,7 @@ struct RouterArgs {
   int* counters;         // one per token block, all zero between launches; null = logits only
   int* status;           // device status word or null
   int T, H, E, k, sigmoid;
+  int cluster;           // the blocks of a token block's groups of experts form a cluster
   // order-faithful kernel over a token list (the fall-back pass): token_list[0 .. *n_list)
   const int* token_list;
   int* n_list;           // read at start; reset to zero, with fb_done, by the last block to finish
@@ -180,23 +190,85 @@ struct RouterArgs {
 
 // A block is one producer warp (four with plain weights) plus TW consumer warps.  A
 // consumer warp owns TT tokens, its lanes 32 neighbouring experts: a thread runs TT chains.
-//   * expert rows: a four-stage ring of CH-column chunks filled by bulk copies
-//     (cp.async.bulk, completion counted on the stage's mbarrier).  An SM starts
-//     only about one bulk copy per 70-100 cycles, so with PACKED weights a stage
-//     is one copy issued by one thread; with plain [E,H] weights the producers'
-//     lanes issue one copy per row;
-//   * token rows: each consumer warp keeps its own TT rows in a ring of the same
-//     depth, filled with cp.async by the warp itself (nobody else reads them);
-//   * a lane reads its own expert row with 128-bit loads (conflict-free by the
-//     row padding) and the token rows by broadcast.  A chain costs one dependent
-//     add per column, so a logit takes about H x (add latency) cycles however
-//     many run at once: TT = 1 keeps two 32-column register blocks in flight to
-//     run one chain at that speed (few tokens), larger TT trades latency for
-//     fewer shared-memory reads per chain (many tokens);
-//   * with `counters`, the last block to finish a token block's logits (an
-//     atomic ticket after a fence) also selects the top-k for those tokens.
-// Waits are bounded; a wait that runs out sets kDevErrWaitTimeout in *status
-// (when given) and the block leaves.
+//   * a ring of three or four stages of CH columns, filled by the producer alone: the expert rows by
+//     bulk copies (cp.async.bulk; an SM starts only about one per 70-100 cycles, so with PACKED
+//     weights a stage is one copy issued by one thread, with plain [E,H] weights a copy per
+//     row), the token rows by cp.async; both count on the stage's mbarrier, the only thing a
+//     consumer waits for.  Packed weights of the first stages are requested before the kernel
+//     in front has ended;
+//   * a lane reads its own expert row with 128-bit loads (conflict-free by the row padding)
+//     and the token rows by broadcast, some groups of four columns ahead; the products of the
+//     next group are written between the additions of this one, two to an instruction
+//     (mul.rn.f32x2: the same rounding, half the issue slots);
+//   * a chain costs one dependent addition per column, 4.3 cycles: TT = 1 runs one chain at
+//     that speed (few tokens), larger TT has the additions of TT chains fill those cycles, up to
+//     the 2 cycles a column and chain that product and sum take of the fp32 pipe;
+//   * the logits of a token's other groups of 32 experts come from the blocks of the same
+//     cluster (A.cluster: gridDim.y of them, through distributed shared memory; the tokens'
+//     selections are dealt to its blocks), or, with more than eight groups, through global
+//     memory: the last block to finish a token block's logits (an atomic ticket after a fence)
+//     selects then.  With one group they are in the lanes already.  Without `counters` the
+//     logits are all there is.
+// Waits are bounded; a wait that runs out sets kDevErrWaitTimeout in *status (when given): every
+// further wait of the block ends at once, and it goes through the rest of its loops with
+// whatever it holds, so that the blocks of a cluster still meet.
+__device__ __forceinline__ void cp_async_arrive(uint32_t bar) {  // arrives once this thread's cp.asyncs so far have landed
+  asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(bar) : "memory");
+}
+__device__ __forceinline__ float4 lds128(uint32_t addr) {  // (volatile: it stays where the code asks for it, ahead of its use)
+  float4 v;
+  asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(addr));
+  return v;
+}
+// Four products with the rounding of single multiplications; PACKED2: two to an instruction (half the issue slots, which a lone
+// chain has to spare, while the pair's later result is in its way: 5.3 cycles a column, not 4.6).
+template <bool PACKED2>
+__device__ __forceinline__ float4 mul4_rn(const float4& a, const float4& b) {
+  if (!PACKED2) return make_float4(__fmul_rn(a.x, b.x), __fmul_rn(a.y, b.y), __fmul_rn(a.z, b.z), __fmul_rn(a.w, b.w));
+  float4 r;
+  asm("{\n\t.reg .b64 p, q;\n\tmov.b64 p, {%4, %5};\n\tmov.b64 q, {%8, %9};\n\tmul.rn.f32x2 p, p, q;\n\tmov.b64 {%0, %1}, p;\n\t"
+      "mov.b64 p, {%6, %7};\n\tmov.b64 q, {%10, %11};\n\tmul.rn.f32x2 p, p, q;\n\tmov.b64 {%2, %3}, p;\n\t}"
+      : "=f"(r.x), "=f"(r.y), "=f"(r.z), "=f"(r.w)
+      : "f"(a.x), "f"(a.y), "f"(a.z), "f"(a.w), "f"(b.x), "f"(b.y), "f"(b.z), "f"(b.w));
+  return r;
+}
+
+// N columns of TT chains; w, h: the lane's expert row and the warp's token rows (ld_bytes apart) in shared memory.  AHEAD groups of
+// four columns are in registers ahead.
+template <int TT, int N, int AHEAD>
+__device__ __forceinline__ void chain_columns(uint32_t w, uint32_t h, int ld_bytes, float (&acc)[TT]) {
+  constexpr int G = N / 4, A = AHEAD < G ? AHEAD : G;
+  float4 wv[A], hv[A][TT], now[TT], next[TT];
+  auto load = [&](int g) {
+    wv[g % A] = lds128(w + 16 * g);
+#pragma unroll
+    for (int i = 0; i < TT; ++i) hv[g % A][i] = lds128(h + i * ld_bytes + 16 * g);
+  };
+#pragma unroll
+  for (int g = 0; g < A; ++g) load(g);
+#pragma unroll
+  for (int i = 0; i < TT; ++i) now[i] = mul4_rn<(TT > 1)>(hv[0][i], wv[0]);
+#pragma unroll
+  for (int g = 0; g < G; ++g) {
+    if (g + A < G) load(g + A);  // the registers of group g, whose products have been made
+    if (g + 1 < G) {
+#pragma unroll
+      for (int i = 0; i < TT; ++i) next[i] = mul4_rn<(TT > 1)>(hv[(g + 1) % A][i], wv[(g + 1) % A]);
+    }
+#pragma unroll
+    for (int i = 0; i < TT; ++i) acc[i] = __fadd_rn(acc[i], now[i].x);
+#pragma unroll
+    for (int i = 0; i < TT; ++i) acc[i] = __fadd_rn(acc[i], now[i].y);
+#pragma unroll
+    for (int i = 0; i < TT; ++i) acc[i] = __fadd_rn(acc[i], now[i].z);
+#pragma unroll
+    for (int i = 0; i < TT; ++i) acc[i] = __fadd_rn(acc[i], now[i].w);
+#pragma unroll
+    for (int i = 0; i < TT; ++i) now[i] = next[i];
+  }
+}
+__host__ __device__ constexpr int router_ahead(int tt) { return tt == 1 ? 8 : tt == 2 ? 4 : tt <= 4 ? 3 : 2; }
+
 // Bounded wait that naps between polls, for a warp that shares its scheduler with a
 // warp doing the real work.
 __device__ __forceinline__ bool mbar_wait_nap(uint32_t bar, uint32_t parity, volatile int* abort_flag) {
@@ -216,20 +288,21 @@ __device__ __forceinline__ bool mbar_wait_nap(uint32_t bar, uint32_t parity, vol
 __host__ __device__ constexpr int router_producer_warps(bool packed) { return packed ? 1 : 4; }
 
 template <int TW, int TT, int CH, bool PACKED>
-__global__ void __launch_bounds__((TW + router_producer_warps(PACKED)) * 32)
+__global__ void __launch_bounds__((TW + router_producer_warps(PACKED)) * 32, 1)
 k_router_logits(const RouterArgs A) {
   extern __shared__ __align__(128) uint8_t router_smem_raw[];
   constexpr int LD = CH + kRouterPad;
-  constexpr int NS = router_stages(TW * TT), NP = router_producer_warps(PACKED);
+  constexpr int NS = router_stages(CH), NP = router_producer_warps(PACKED);
   constexpr int BT = TW * TT;                   // tokens of the block
   constexpr int stage_floats = (32 + BT) * LD;  // ws[32][LD] then hs[BT][LD]
-  float* stages = reinterpret_cast<float*>(router_smem_raw);
+  const uint32_t stages = smem_u32(router_smem_raw);
   uint64_t* bars = reinterpret_cast<uint64_t*>(router_smem_raw + (size_t)NS * stage_floats * sizeof(float));
   const uint32_t bar_base = smem_u32(bars);
   auto bar_full = [&](int s) { return bar_base + 8u * s; };
   auto bar_empty = [&](int s) { return bar_base + 8u * (NS + s); };
   volatile int* abort_flag = reinterpret_cast<volatile int*>(bars + 2 * NS);
   volatile int* ticket = abort_flag + 1;
+  float* const exchanged = reinterpret_cast<float*>(bars) + 32;  // two buffers of the block's tokens x E logits (with a cluster)
 
   const int T = A.T, H = A.H, E = A.E;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -238,223 +311,164 @@ k_router_logits(const RouterArgs A) {
 
   if (tid == 0) {
     for (int s = 0; s < NS; ++s) {
-      mbar_init(bar_full(s), PACKED ? 1 : NP);
+      mbar_init(bar_full(s), (PACKED ? 1 : NP) + 32 * NP);  // the copies' announcement, and every producer lane's token pieces
       mbar_init(bar_empty(s), TW);
     }
     *abort_flag = 0;
     *ticket = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
-  __syncthreads();
+  if (A.cluster) cluster_sync_all();  // (a block of the cluster may be written to only once it runs)
+  else __syncthreads();
+  const int* const list = A.token_list;
+  const float* const packed = A.wg + (size_t)blockIdx.y * n_chunks * 32 * LD;
+  auto packed_stage = [&](int ci, int st) {
+    mbar_expect_tx(bar_full(st), 32 * LD * 4);
+    bulk_load(stages + (uint32_t)st * stage_floats * 4, packed + (size_t)ci * 32 * LD, 32 * LD * 4, bar_full(st));
+  };
+  const int ahead = PACKED && !list ? min(NS, n_chunks) : 0;  // (a list may turn out empty; T is not)
+  if (warp == 0 && lane == 0)
+    for (int ci = 0; ci < ahead; ++ci) packed_stage(ci, ci);
   griddep_wait();
   griddep_launch();
   // tokens of this launch: all T, or the entries of a list built by an earlier kernel
-  const int* const list = A.token_list;
   const int n_list = list ? min(*reinterpret_cast<volatile int*>(A.n_list), T) : 0;
   const int n_tok = list ? (n_list > A.list_over && n_list <= A.list_max ? n_list : 0) : T;
   auto token_at = [&](int ti) { return ti < n_tok ? (list ? list[ti] : ti) : -1; };
 
   // A block takes the token blocks blockIdx.x, blockIdx.x + gridDim.x, ...  (one each unless the launch
   // is list-driven and the list turned out longer than the grid).  The ring's barriers carry on from
-  // one token block to the next: cg0 = chunks this block has moved so far.
+  // one token block to the next: cg = running number of the chunk.
+  bool ok = true;
+  int cg = 0;
   for (int tb = blockIdx.x, iter = 0; tb * BT < n_tok; tb += gridDim.x, ++iter) {
-  const int t0 = tb * BT;
-  const int cg0 = iter * n_chunks;
-  if (warp < NP) {
-    // ------------------------------ producers ------------------------------
-    const int n_e = min(32, E - e0);
-    const bool mine = PACKED ? (warp == 0 && lane == 0) : (warp + NP * lane < n_e);
-    const int row = warp + NP * lane;  // !PACKED: producer p moves expert rows p, p+NP, ...
-    const int n_mine = __popc(__ballot_sync(0xffffffffu, mine));  // !PACKED: may be 0, the warp still posts its arrival
-    const float* src = PACKED ? A.wg + (size_t)blockIdx.y * n_chunks * 32 * LD : A.wg + (size_t)(e0 + row) * H;
-    int issued = 0;
-    bool ok = true;
-    if (!PACKED || n_mine) {
-      for (int ci = 0; ci < n_chunks; ++ci) {
-        const int cg = cg0 + ci, st = cg % NS;
-        if (cg >= NS && !mbar_wait_nap(bar_empty(st), (uint32_t)((cg / NS - 1) & 1), abort_flag)) {
-          ok = false;
-          break;
-        }
-        const uint32_t dst = smem_u32(stages + (size_t)st * stage_floats);
+    const int t0 = tb * BT;
+    if (warp < NP) {
+      // ------------------------------ producers ------------------------------
+      const int n_e = min(32, E - e0);
+      const int row = warp + NP * lane;  // !PACKED: producer p moves expert rows p, p + NP, ...
+      const int n_mine = __popc(__ballot_sync(0xffffffffu, row < n_e));
+      constexpr int R = (BT + NP - 1) / NP;  // token rows p, p + NP, ... are a producer's
+      const float* src[R];
+#pragma unroll
+      for (int i = 0; i < R; ++i) {
+        const int r = warp + NP * i, t = r < BT ? token_at(t0 + r) : -1;
+        src[i] = t >= 0 ? A.hidden + (size_t)t * H + lane * 4 : nullptr;
+      }
+      for (int ci = 0; ci < n_chunks; ++ci, ++cg) {
+        const int st = cg % NS, d0 = ci * CH, dc = min(CH, H - d0);
+        if (ok && cg >= NS) ok = __all_sync(0xffffffffu, mbar_wait_nap(bar_empty(st), (uint32_t)((cg / NS - 1) & 1), abort_flag));
+        if (!ok) break;
+        const uint32_t dst = stages + (uint32_t)st * stage_floats * 4;
         if (PACKED) {
-          if (mine) {
-            mbar_expect_tx(bar_full(st), 32 * LD * 4);
-            bulk_load(dst, src + (size_t)ci * 32 * LD, 32 * LD * 4, bar_full(st));
-          }
+          if (lane == 0 && cg >= ahead) packed_stage(ci, st);
         } else {
-          const int d0 = ci * CH;
-          const uint32_t row_bytes = (uint32_t)min(CH, H - d0) * sizeof(float);  // H % 32 == 0: a multiple of 128
+          const uint32_t row_bytes = (uint32_t)dc * sizeof(float);  // H % 32 == 0: a multiple of 128
           if (lane == 0) mbar_expect_tx(bar_full(st), (uint32_t)n_mine * row_bytes);
           __syncwarp();
-          if (mine) bulk_load(dst + (uint32_t)row * LD * 4, src + d0, row_bytes, bar_full(st));
-        }
-        ++issued;
-      }
-    }
-    if (!ok) {
-      // let the copies still in flight land before the block goes away
-      for (int i = 0; i < NS && i < issued; ++i) {
-        const int cg = cg0 + issued - 1 - i;
-        const long long tc = clock64();
-        while (!mbar_try(bar_full(cg % NS), (uint32_t)((cg / NS) & 1)) && clock64() - tc < drain_budget()) {
-        }
-      }
-    }
-  } else {
-    // ------------------------------ consumers ------------------------------
-    const int w = warp - NP;
-    float acc[TT];
-    int tok[TT];
-#pragma unroll
-    for (int i = 0; i < TT; ++i) {
-      acc[i] = 0.f;
-      tok[i] = token_at(t0 + w * TT + i);
-    }
-    // this warp's token rows of chunk ci -> its rows of stage ci % NS
-    auto load_tokens = [&](int ci) {
-      const int d0 = ci * CH;
-      const int dc = min(CH, H - d0);
-      const uint32_t dst = smem_u32(stages + (size_t)((cg0 + ci) % NS) * stage_floats + (32 + w * TT) * LD);
-#pragma unroll
-      for (int i = 0; i < TT; ++i) {
-        const int t = tok[i];
-        if (t >= 0)
-          for (int c = lane * 4; c < dc; c += 128)
-            cp_async16(dst + (uint32_t)(i * LD + c) * 4, A.hidden + (size_t)t * H + d0 + c);
-      }
-    };
-    for (int i = 0; i < NS - 1; ++i) {
-      if (i < n_chunks) load_tokens(i);
-      cp_async_commit();
-    }
-    bool ok = true;
-    for (int ci = 0; ci < n_chunks; ++ci) {
-      const int cg = cg0 + ci, st = cg % NS;
-      cp_async_wait<NS - 2>();  // this lane's part of the token rows of chunk ci has landed ...
-      __syncwarp();             // ... and the other lanes'; the rows used in the last iteration are free
-      if (ci + NS - 1 < n_chunks) load_tokens(ci + NS - 1);
-      cp_async_commit();
-      if (!__all_sync(0xffffffffu, mbar_wait(bar_full(st), (uint32_t)((cg / NS) & 1), abort_flag))) {  // warp-uniform
-        ok = false;
-        break;
-      }
-      const float* wp = stages + (size_t)st * stage_floats + lane * LD;
-      const float* hp = stages + (size_t)st * stage_floats + (32 + w * TT) * LD;
-      const int dc = min(CH, H - ci * CH);
-      if (dc < CH) {
-        // last, partial chunk: the code below always walks CH columns, so the missing ones must
-        // multiply to zero.  Every lane clears the tail of its own expert row (stale but written
-        // only with zeros by anyone) and of the warp's token rows.
-        float* wrow = stages + (size_t)st * stage_floats + lane * LD;
-        for (int c = dc; c < CH; ++c) wrow[c] = 0.f;
-        float* hrow = stages + (size_t)st * stage_floats + (32 + w * TT) * LD;
-        for (int i = 0; i < TT; ++i)
-          for (int c = dc + lane; c < CH; c += 32) hrow[i * LD + c] = 0.f;
-        __syncwarp();
-      }
-      if (TT == 1) {
-        // 32-column blocks, straight-line code for the whole chunk.  The add chain issues one
-        // instruction per four cycles; the loads and the (independent) products of the NEXT block
-        // are written between its adds so they go into those idle issue slots.
-        constexpr int NBLK = CH / 32;
-        float p[2][32];
-        float a = acc[0];
-#pragma unroll
-        for (int i = 0; i < 8; ++i) {
-          const float4 wv = *reinterpret_cast<const float4*>(wp + i * 4);
-          const float4 hv = *reinterpret_cast<const float4*>(hp + i * 4);
-          p[0][4 * i] = __fmul_rn(hv.x, wv.x);
-          p[0][4 * i + 1] = __fmul_rn(hv.y, wv.y);
-          p[0][4 * i + 2] = __fmul_rn(hv.z, wv.z);
-          p[0][4 * i + 3] = __fmul_rn(hv.w, wv.w);
+          if (row < n_e) bulk_load(dst + (uint32_t)row * LD * 4, A.wg + (size_t)(e0 + row) * H + d0, row_bytes, bar_full(st));
         }
 #pragma unroll
-        for (int blk = 0; blk < NBLK; ++blk) {
-          const int cur = blk & 1, nxt = cur ^ 1;
-          float4 wv[8], hv[8];
-          if (blk + 1 < NBLK) {
+        for (int i = 0; i < R; ++i) {
+          if (src[i]) {
 #pragma unroll
-            for (int i = 0; i < 8; ++i) {
-              wv[i] = *reinterpret_cast<const float4*>(wp + (blk + 1) * 32 + i * 4);
-              hv[i] = *reinterpret_cast<const float4*>(hp + (blk + 1) * 32 + i * 4);
-            }
-          }
-#pragma unroll
-          for (int i = 0; i < 8; ++i) {
-            a = __fadd_rn(a, p[cur][4 * i]);
-            if (blk + 1 < NBLK) p[nxt][4 * i] = __fmul_rn(hv[i].x, wv[i].x);
-            a = __fadd_rn(a, p[cur][4 * i + 1]);
-            if (blk + 1 < NBLK) p[nxt][4 * i + 1] = __fmul_rn(hv[i].y, wv[i].y);
-            a = __fadd_rn(a, p[cur][4 * i + 2]);
-            if (blk + 1 < NBLK) p[nxt][4 * i + 2] = __fmul_rn(hv[i].z, wv[i].z);
-            a = __fadd_rn(a, p[cur][4 * i + 3]);
-            if (blk + 1 < NBLK) p[nxt][4 * i + 3] = __fmul_rn(hv[i].w, wv[i].w);
+            for (int c = 0; c < CH; c += 128)
+              if (c + lane * 4 < dc) cp_async16(dst + (uint32_t)((32 + warp + NP * i) * LD + c + lane * 4) * 4, src[i] + d0 + c);
           }
         }
-        acc[0] = a;
-      } else {
-#pragma unroll 4
-        for (int d = 0; d < CH; d += 4) {
-          const float4 wv = *reinterpret_cast<const float4*>(wp + d);
-          float4 hv[TT];
-#pragma unroll
-          for (int i = 0; i < TT; ++i) hv[i] = *reinterpret_cast<const float4*>(hp + i * LD + d);
-#pragma unroll
-          for (int i = 0; i < TT; ++i) {
-            float a = acc[i];
-            a = __fadd_rn(a, __fmul_rn(hv[i].x, wv.x));
-            a = __fadd_rn(a, __fmul_rn(hv[i].y, wv.y));
-            a = __fadd_rn(a, __fmul_rn(hv[i].z, wv.z));
-            a = __fadd_rn(a, __fmul_rn(hv[i].w, wv.w));
-            acc[i] = a;
-          }
-        }
+        cp_async_arrive(bar_full(st));
       }
       __syncwarp();
-      if (lane == 0) mbar_arrive(bar_empty(st));
-    }
-    cp_async_wait<0>();
-    if (ok) {
+    } else {
+      // ------------------------------ consumers ------------------------------
+      const int w = warp - NP;
+      float acc[TT];
+#pragma unroll
+      for (int i = 0; i < TT; ++i) acc[i] = 0.f;
+      bool here = mbar_try(bar_full(cg % NS), (uint32_t)((cg / NS) & 1));
+      for (int ci = 0; ci < n_chunks; ++ci) {
+        const int st = cg % NS, dc = min(CH, H - ci * CH);
+        if (!here) ok = mbar_wait(bar_full(st), (uint32_t)((cg / NS) & 1), abort_flag) && ok;
+        ++cg;
+        // (the answer is needed after this chunk only; the question alone costs 100 cycles in front of one)
+        here = ci + 1 < n_chunks && mbar_test(bar_full(cg % NS), (uint32_t)((cg / NS) & 1));
+        const uint32_t wp = stages + (uint32_t)(st * stage_floats + lane * LD) * 4;
+        const uint32_t hp = stages + (uint32_t)(st * stage_floats + (32 + w * TT) * LD) * 4;
+        if (dc == CH) {
+          chain_columns<TT, CH, router_ahead(TT)>(wp, hp, LD * 4, acc);
+        } else {
+#pragma unroll 1
+          for (int d = 0; d < dc; d += 32) chain_columns<TT, 32, router_ahead(TT)>(wp + d * 4, hp + d * 4, LD * 4, acc);
+        }
+        __syncwarp();
+        if (lane == 0 && ok) mbar_arrive(bar_empty(st));
+      }
+      __syncwarp();
       const int e = e0 + lane;
       const float b = (A.bias && e < E) ? A.bias[e] : 0.f;
 #pragma unroll
       for (int i = 0; i < TT; ++i) {
-        const int t = tok[i];
-        if (t >= 0 && e < E) A.logits[(size_t)t * E + e] = __fadd_rn(acc[i], b);
+        const int j = w * TT + i, t = token_at(t0 + j);
+        const float logit = e < E ? __fadd_rn(acc[i], b) : -INFINITY;
+        if (A.counters && gridDim.y == 1) {
+          float v[1] = {logit};
+          if (t >= 0) warp_topk_regs<false, 1>(v, E, A.k, A.sigmoid, A.router_out + (size_t)t * A.k * 2, nullptr);
+        } else if (t >= 0 && e < E) {
+          if (A.cluster) {
+            const uint32_t to = map_to_cta(smem_u32(exchanged + ((size_t)(iter & 1) * BT + j) * E + e), (uint32_t)j % gridDim.y);
+            asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(to), "f"(logit) : "memory");
+          } else {
+            A.logits[(size_t)t * E + e] = logit;
+          }
+        }
       }
-      __threadfence();  // the logits before the block's ticket below
+      if (A.counters && !A.cluster) __threadfence();  // the logits before the block's ticket below
     }
-  }
-  __syncthreads();
-  if (*abort_flag) break;  // a wait ran out: the ring's state is unknown, the block stops here
-
-  // ---- the last block of this token block selects the top-k ----
-  if (A.counters != nullptr) {
-    if (tid == 0) {
-      int last = 1;
-      if (gridDim.y > 1) {
+    if (A.counters == nullptr || gridDim.y == 1) continue;
+    int first = 0, step = 1;
+      if (A.cluster) {
+      // (a block writes the next token block's logits into the other buffer, and the one after that only when all have come
+      // past the next barrier, which is after they have read these)
+      cluster_sync_all();
+      first = blockIdx.y;
+      step = gridDim.y;
+    } else {
+      // ---- the last block of this token block selects the top-k ----
+      __syncthreads();
+      if (tid == 0) {
         __threadfence();  // this block's logits before its ticket
-        last = atomicAdd(&A.counters[tb], 1) == (int)gridDim.y - 1;
+        const int last = atomicAdd(&A.counters[tb], 1) == (int)gridDim.y - 1;
         if (last) {
           A.counters[tb] = 0;  // ready for the next launch
           __threadfence();     // the other blocks' logits after their tickets
         }
+        *ticket = last;
       }
-      *ticket = last;
+      __syncthreads();
+      if (!*ticket) first = BT;
     }
-    __syncthreads();
-    if (*ticket) {
-      for (int i = warp; i < BT; i += TW + NP) {
-        const int t = token_at(t0 + i);
-        if (t < 0) continue;
-        warp_topk(A.logits + (size_t)t * E, E, A.k, A.sigmoid, A.router_out + (size_t)t * A.k * 2);
-      }
+    for (int j = first + step * warp; j < BT; j += step * (TW + NP)) {
+      const int t = token_at(t0 + j);
+      if (t < 0) continue;
+      float* const to = A.router_out + (size_t)t * A.k * 2;
+      if (A.cluster) warp_topk<false>(exchanged + ((size_t)(iter & 1) * BT + j) * E, E, A.k, A.sigmoid, to);
+      else warp_topk(A.logits + (size_t)t * E, E, A.k, A.sigmoid, to);
     }
-    __syncthreads();  // `ticket` is rewritten by the next token block
-  }
+    if (!A.cluster) __syncthreads();  // `ticket` is rewritten by the next token block
   }  // token blocks of this block
 
+  if (warp < NP) {
+    // let the copies still in flight land before the block goes away (they have, unless a wait ran out)
+    const int issued = cg;
+    for (int i = 0; lane == 0 && *abort_flag && i < NS && i < issued; ++i) {
+      const int c = issued - 1 - i;
+      const long long tc = clock64();
+      while (!mbar_try(bar_full(c % NS), (uint32_t)((c / NS) & 1)) && clock64() - tc < drain_budget()) {
+      }
+    }
+    asm volatile("cp.async.wait_all;" ::: "memory");
+  }
+  __syncthreads();
   if (tid == 0 && *abort_flag && A.status) atomicOr(A.status, kDevErrWaitTimeout);
   if (list && n_tok && tid == 0) {
     // every block of the launch that takes the list, busy or idle, has read its length by now: the last
@@ -469,19 +483,21 @@ k_router_logits(const RouterArgs A) {
   }
 }
 
+constexpr int kRouterClusterGroups = 8;  // groups of 32 experts up to which their blocks form a cluster (the portable size)
 template <int TW, int TT, int CH, bool PACKED>
 cudaError_t router_prepare_one() {
   return cudaFuncSetAttribute(k_router_logits<TW, TT, CH, PACKED>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                              (int)router_smem_bytes(TW * TT, CH));
+                              (int)router_smem_bytes(TW * TT, CH, PACKED ? 32 * kRouterClusterGroups : 0));
 }
-constexpr int kRouterChunkFew = 256, kRouterChunkMany = 128;  // columns per stage: few / many tokens
 template <bool PACKED>
 cudaError_t router_prepare_set() {
   cudaError_t e = router_prepare_one<1, 1, kRouterChunkFew, PACKED>();
   if (e == cudaSuccess) e = router_prepare_one<2, 1, kRouterChunkFew, PACKED>();
   if (e == cudaSuccess) e = router_prepare_one<4, 1, kRouterChunkFew, PACKED>();
   if (e == cudaSuccess) e = router_prepare_one<4, 2, kRouterChunkMany, PACKED>();
+  if (e == cudaSuccess) e = router_prepare_one<4, 3, kRouterChunkMany, PACKED>();
   if (e == cudaSuccess) e = router_prepare_one<4, 4, kRouterChunkMany, PACKED>();
+  if (e == cudaSuccess) e = router_prepare_one<8, 3, kRouterChunkMany, PACKED>();
   if (e == cudaSuccess) e = router_prepare_one<8, 4, kRouterChunkMany, PACKED>();
   return e;
 }
@@ -490,33 +506,53 @@ cudaError_t router_prepare_set() {
 inline cudaError_t router_prepare_device();
 
 template <int TW, int TT, int CH, bool PACKED>
-void launch_router_one(const RouterArgs& a, int token_slots, cudaStream_t s, bool pdl) {
-  const dim3 grid((unsigned)((token_slots + TW * TT - 1) / (TW * TT)), (unsigned)((a.E + 31) / 32));
-  launch_k(k_router_logits<TW, TT, CH, PACKED>, grid, dim3((TW + router_producer_warps(PACKED)) * 32),
-           router_smem_bytes(TW * TT, CH), s, pdl, a);
+void launch_router_one(RouterArgs a, int token_slots, cudaStream_t s, bool pdl) {
+  const unsigned groups = (unsigned)((a.E + 31) / 32);
+  constexpr int BT = TW * TT;
+  a.cluster = PACKED && a.counters && groups > 1 && groups <= kRouterClusterGroups;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3((unsigned)((token_slots + BT - 1) / BT), groups);
+  cfg.blockDim = dim3((TW + router_producer_warps(PACKED)) * 32);
+  cfg.dynamicSmemBytes = router_smem_bytes(BT, CH, a.cluster ? a.E : 0);
+  cfg.stream = s;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = 1;
+  attr[0].val.clusterDim.y = a.cluster ? groups : 1;
+  attr[0].val.clusterDim.z = 1;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = pdl ? 2 : 1;
+  cudaLaunchKernelEx(&cfg, k_router_logits<TW, TT, CH, PACKED>, a);
 }
 
-// Few tokens per block while that still leaves SMs idle (a block's speed is bounded by its
-// shared-memory reads: one 16-byte word per lane per four columns and chain), more chains per
-// thread once the machine is full.  wg_few / wg_many: the weights packed for the two chunk
-// widths (PACKED) or both the plain [E,H] matrix.  token_slots: tokens the grid is sized for
-// (a.T, or for a list-driven launch the most entries the list can have).
+// The fewest tokens per block with which the blocks are one wave: a block's time goes by its chains per thread and, from four warps
+// on, by its shared-memory reads (a row of weights per lane costs 4 cycles per four columns, a token row 2), so that a second
+// wave is dearer than more chains in one.  Clusters leave some SMs of a GPC over: nine tenths count as a wave then.  One launch, us (6 of
+// them the events), 2880 columns, by warps x tokens of a warp: 128 experts, 64 tokens 1x1 21.5, 2x1 19.6; 128 tokens 2x1 21.7, 4x1 21.7;
+// 200 4x1 35.8, 4x2 24.0; 333 4x2 38.0, 4x3 30.9, 4x4 35.0; 512 4x3 44.1, 4x4 34.0; 700 4x4 60.6, 8x3 45.0, 8x4 52.4; 1024 8x3 83, 8x4 53;
+// 32 experts, 333 2x1 21.9, 4x1 19.9; 1024 4x1 28.1, 4x2 24.2; 2048 4x2 36.2, 4x4 34.8; 4096 4x4 52.6, 8x4 54.4; 8192 4x4 97, 8x4 101.
+// Before (a producer for the weights only, loads at their use, up to 16 tokens a block and no cluster): 8 tokens 20.8, 64 21.6, 333 46.9, 1024
+// 64; 32 experts, 4096 tokens 62.
+// wg_few / wg_many: the weights packed for the two chunk widths (PACKED) or both the plain [E,H] matrix.  token_slots: tokens the
+// grid is sized for (a.T, or for a list-driven launch the most entries the list can have).
 template <bool PACKED>
 inline void launch_router_logits(RouterArgs a, const float* wg_few, const float* wg_many, int sm_count,
                                  cudaStream_t s, bool pdl = false, int token_slots = -1) {
   if (token_slots < 0) token_slots = a.T;
-  const int64_t token_blocks = (int64_t)token_slots * ((a.E + 31) / 32);  // blocks if every block held one token
-  if (token_blocks <= 4 * (int64_t)sm_count) {
-    a.wg = wg_few;
-    if (token_blocks <= sm_count) launch_router_one<1, 1, kRouterChunkFew, PACKED>(a, token_slots, s, pdl);
-    else if (token_blocks <= 2 * (int64_t)sm_count) launch_router_one<2, 1, kRouterChunkFew, PACKED>(a, token_slots, s, pdl);
-    else launch_router_one<4, 1, kRouterChunkFew, PACKED>(a, token_slots, s, pdl);
-  } else {
-    a.wg = wg_many;
-    if (token_blocks <= 8 * (int64_t)sm_count) launch_router_one<4, 2, kRouterChunkMany, PACKED>(a, token_slots, s, pdl);
-    else if (token_blocks <= 64 * (int64_t)sm_count) launch_router_one<4, 4, kRouterChunkMany, PACKED>(a, token_slots, s, pdl);
-    else launch_router_one<8, 4, kRouterChunkMany, PACKED>(a, token_slots, s, pdl);
-  }
+  const int64_t groups = (a.E + 31) / 32, wave = groups == 1 ? sm_count : 9 * (int64_t)sm_count / 10;
+  auto one_wave = [&](int tokens) { return (token_slots + tokens - 1) / tokens * groups <= wave; };
+  a.wg = wg_few;
+  if (one_wave(1)) return launch_router_one<1, 1, kRouterChunkFew, PACKED>(a, token_slots, s, pdl);
+  if (one_wave(2)) return launch_router_one<2, 1, kRouterChunkFew, PACKED>(a, token_slots, s, pdl);
+  if (one_wave(4)) return launch_router_one<4, 1, kRouterChunkFew, PACKED>(a, token_slots, s, pdl);
+  a.wg = wg_many;
+  if (one_wave(8)) return launch_router_one<4, 2, kRouterChunkMany, PACKED>(a, token_slots, s, pdl);
+  if (one_wave(12)) return launch_router_one<4, 3, kRouterChunkMany, PACKED>(a, token_slots, s, pdl);
+  if (one_wave(16) || (!one_wave(32) && groups == 1)) return launch_router_one<4, 4, kRouterChunkMany, PACKED>(a, token_slots, s, pdl);
+  if (one_wave(24)) return launch_router_one<8, 3, kRouterChunkMany, PACKED>(a, token_slots, s, pdl);
+  launch_router_one<8, 4, kRouterChunkMany, PACKED>(a, token_slots, s, pdl);
 }
 
 // ---------------------------------------------------------------------------

@@ -1,0 +1,43 @@
+"""The order-faithful router kernel where its blocks, stages and clusters end, against the CPU restatement: the products and
+sums are the reference's one after the other, so the selections are equal and the routing weights are, too, but for the
+exponential's last bits."""
+import numpy as np
+import pytest
+
+from coalsack_b200 import MoeLayer
+
+pytestmark = pytest.mark.gpu
+
+
+def _waves():
+    """The last batch of each launch shape and the first of the next, for one group of 32 experts (148 blocks a wave) and
+    four (133 blocks in clusters)."""
+    for E, blocks in ((32, 148), (128, 33)):
+        for tokens in (1, 2, 4, 8, 12, 16, 24, 32):
+            yield E, 96, blocks * tokens
+            yield E, 96, blocks * tokens + 1
+
+
+@pytest.mark.parametrize("E,H,T", [
+    *_waves(),
+    (5, 32, 3), (33, 256, 7), (64, 288, 9),          # fewer columns than a stage, one stage, one more block of columns
+    (256, 1056, 5), (257, 544, 5), (1024, 160, 40),  # the widest cluster, the first without one, the most experts
+    (128, 2880, 8), (128, 2880, 333), (40, 4128, 150),
+])
+@pytest.mark.parametrize("sigmoid", [False, True])
+def test_chain_at_the_edges_of_its_launches(gpu_lib, port, E, H, T, sigmoid):
+    rng = np.random.default_rng(E + H + T)
+    k = min(4, E)
+    h = rng.standard_normal((T, H)).astype(np.float32)
+    Wg = (rng.standard_normal((E, H)) * 0.02).astype(np.float32)
+    rb = (rng.standard_normal(E) * 0.01).astype(np.float32)
+    lay = MoeLayer(E, k, H, 32, has_bias=False, sigmoid_gating=sigmoid, max_tokens=T)
+    lay.set_router(Wg, rb)
+    lay.set_router_mode(lay.ROUTER_CHAIN)
+    got = lay.route(h)
+    want = port.router(h, Wg, rb, k, sigmoid)
+    assert np.array_equal(got[..., 0], want[..., 0])
+    # expf: 2 ulp here, in its sum as much again, and the reciprocal's and the product's roundings: 2.4e-7 + 2.4e-7 + 1.2e-7 of a weight
+    assert np.allclose(got[..., 1], want[..., 1], rtol=0, atol=6e-7)
+    assert np.array_equal(lay.route(h), got)
+    lay.close()
