@@ -2,6 +2,8 @@
 // expert, gather to fp16 rows, weighted combine.
 #pragma once
 
+#include <algorithm>
+
 #include "csk_common.cuh"
 
 namespace csk {
@@ -527,9 +529,32 @@ void launch_router_one(RouterArgs a, int token_slots, cudaStream_t s, bool pdl) 
   cudaLaunchKernelEx(&cfg, k_router_logits<TW, TT, CH, PACKED>, a);
 }
 
+// Blocks of the widest launch that are resident at once, for `groups` groups of 32 experts: an SM each, but clusters leave some SMs of a
+// GPC over (with a fixed nine tenths of the SMs, 64 tokens of 256 experts took two waves of clusters of eight, 30.5 us).
+inline int router_wave(int groups, int sm_count) {
+  if (groups < 2 || groups > kRouterClusterGroups) return sm_count;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(1024, (unsigned)groups);
+  cfg.blockDim = dim3((8 + router_producer_warps(true)) * 32);
+  cfg.dynamicSmemBytes = router_smem_bytes(32, kRouterChunkMany, 32 * groups);
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = 1;
+  attr[0].val.clusterDim.y = (unsigned)groups;
+  attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  int clusters = 0;
+  if (cudaOccupancyMaxActiveClusters(&clusters, k_router_logits<8, 4, kRouterChunkMany, true>, &cfg) != cudaSuccess || clusters < 1) {
+    cudaGetLastError();
+    return 3 * sm_count / 4;
+  }
+  return std::min(clusters * groups, sm_count);
+}
+
 // The fewest tokens per block with which the blocks are one wave: a block's time goes by its chains per thread and, from four warps
 // on, by its shared-memory reads (a row of weights per lane costs 4 cycles per four columns, a token row 2), so that a second
-// wave is dearer than more chains in one.  Clusters leave some SMs of a GPC over: nine tenths count as a wave then.  One launch, us (6 of
+// wave is dearer than more chains in one.  `wave`: see router_wave.  One launch, us (6 of
 // them the events), 2880 columns, by warps x tokens of a warp: 128 experts, 64 tokens 1x1 21.5, 2x1 19.6; 128 tokens 2x1 21.7, 4x1 21.7;
 // 200 4x1 35.8, 4x2 24.0; 333 4x2 38.0, 4x3 30.9, 4x4 35.0; 512 4x3 44.1, 4x4 34.0; 700 4x4 60.6, 8x3 45.0, 8x4 52.4; 1024 8x3 83, 8x4 53;
 // 32 experts, 333 2x1 21.9, 4x1 19.9; 1024 4x1 28.1, 4x2 24.2; 2048 4x2 36.2, 4x4 34.8; 4096 4x4 52.6, 8x4 54.4; 8192 4x4 97, 8x4 101.
@@ -538,10 +563,10 @@ void launch_router_one(RouterArgs a, int token_slots, cudaStream_t s, bool pdl) 
 // wg_few / wg_many: the weights packed for the two chunk widths (PACKED) or both the plain [E,H] matrix.  token_slots: tokens the
 // grid is sized for (a.T, or for a list-driven launch the most entries the list can have).
 template <bool PACKED>
-inline void launch_router_logits(RouterArgs a, const float* wg_few, const float* wg_many, int sm_count,
-                                 cudaStream_t s, bool pdl = false, int token_slots = -1) {
+inline void launch_router_logits(RouterArgs a, const float* wg_few, const float* wg_many, int wave, cudaStream_t s, bool pdl = false,
+                                 int token_slots = -1) {
   if (token_slots < 0) token_slots = a.T;
-  const int64_t groups = (a.E + 31) / 32, wave = groups == 1 ? sm_count : 9 * (int64_t)sm_count / 10;
+  const int64_t groups = (a.E + 31) / 32;
   auto one_wave = [&](int tokens) { return (token_slots + tokens - 1) / tokens * groups <= wave; };
   a.wg = wg_few;
   if (one_wave(1)) return launch_router_one<1, 1, kRouterChunkFew, PACKED>(a, token_slots, s, pdl);

@@ -55,6 +55,7 @@ struct csk_moe_layer {
   float* d_wg_tc_scale = nullptr;
   float* d_wnorm_tc = nullptr;
   int router_mode = CSK_ROUTER_AUTO;
+  int router_waves[kMaxExperts / 32 + 1] = {};  // router_wave by groups of 32 experts
   int64_t routed_tokens = 0;   // tokens routed in certified mode since creation
   float* d_logits = nullptr;  // [max_T,E] router scratch
   float* d_rbias = nullptr;
@@ -214,23 +215,24 @@ int launch_router(csk_moe_layer* L, const float* d_hidden, int64_t T, float* d_r
   a.E = L->E_router;
   a.k = L->k;
   a.sigmoid = L->cfg.sigmoid_gating;
-  // The certified pass (three launches: sliced FMA logits, certification, chain over the few tokens it
-  // could not separate) beats the one-launch chain only for a handful of tokens, where the chain is a
-  // single 2880-step dependency on a few SMs: measured in graph replay on the 128-expert layer it is
-  // 51 vs 53 us per step at T=1, level at T=4, and behind from T=16 on (361 vs 342 us at T=64).
+  // Of a handful of tokens the certified pass (three launches: sliced FMA logits, certification, chain over the few tokens it
+  // could not separate) spreads the columns over the machine, where a chain is alone: the step of 1 token of the 128-expert layer 42.4 us,
+  // with the chain 46.8 (the router alone, without its neighbours' overlap, 15.6 and 14.6); of 8 tokens it is behind.
   constexpr int64_t kCertifiedMaxTokens = 4;
   // With many tokens the chain is held by its arithmetic, token x expert; the certified pass on the tensor cores costs
   // little per token, but four launches and the chain of the few percent it cannot separate.  Chain / certified, us, normal
-  // rows: 128 experts, 2880 columns: 333 tokens 43 / (FMA pass) 75, 1024 66 / 51, 2048 119 / 57, 8192 343 / 138; 128 x 2048:
-  // 1024 49 / 44; 64 x 2880: 1024 43 / (FMA) 82, 2048 66 / 56; 256 x 2880: 512 68 / 57, 8192 664 / 259; 512 x 2880: 256
-  // 77 / 79, 512 131 / 75; 512 x 2048: 256 61 / 71, 512 98 / 63; 1024 x 2048: 128 61 / 97, 256 98 / 71; 32 x 2880: 1024 31 / 44, 4096 64 / 72, 8192 122 / 119 (a digit matrix has 128 rows whatever the
-  // experts).  The line is where the two meet: at half as many pairs the FMA pass, which the certified mode then takes, is
-  // the slower one everywhere; with 512 experts and more (few tokens, many digit matrices) they meet at twice as many.
+  // rows: 128 experts, 2880 columns: 1 token 14.6 / (FMA pass) 15.6, 64 14.6 / (FMA) 25, 512 30 / (FMA) 77, 1024 49 / 44, 2048 95 / 62,
+  // 8192 369 / 121; 128 x 2048: 1024 37 / 38, 2048 71 / 48; 64 x 2880: 2048 49 / 48, 4096 96 / 73; 256 x 2880: 256 56 / (FMA) 79, 512
+  // 95 / 51; 512 x 2048: 256 54 / (FMA) 95, 512 86 / 63; 1024 x 2048: 128 54 / (FMA) 98, 256 86 / 72; 32 x 2880: 4096 50 / 104, 8192 92 / 146
+  // (a digit matrix has 128 rows whatever the experts).  The line is where the two meet: with half as many pairs the FMA pass, which
+  // the certified mode then takes, is the slower one everywhere; with 512 experts and more (few tokens, many digit matrices) they
+  // meet at twice as many.
   const int groups = (L->E_router + 31) / 32;
   const int64_t tensor_min_work = groups >= 16 ? 8192 : 4096;  // tokens x groups of 32 experts
   const bool few = T <= kCertifiedMaxTokens, many = groups > 1 && T * groups >= tensor_min_work;
+  const int router_wave = L->router_waves[groups];
   if (L->router_mode == CSK_ROUTER_CHAIN || (L->router_mode == CSK_ROUTER_AUTO && !few && !many)) {
-    launch_router_logits<true>(a, L->d_wg_few, L->d_wg_many, L->sm_count, s, L->pdl);
+    launch_router_logits<true>(a, L->d_wg_few, L->d_wg_many, router_wave, s, L->pdl);
     CSK_CUDA(L, cudaGetLastError());
     L->last.launches += 1;
     return CSK_OK;
@@ -312,25 +314,27 @@ int launch_router(csk_moe_layer* L, const float* d_hidden, int64_t T, float* d_r
   b.fb_done = L->d_fb + 1;
   b.fb_total = reinterpret_cast<unsigned long long*>(L->d_fb + 2);
   b.list_max = INT32_MAX;
-  const int64_t wave = std::max(1, 4 * L->sm_count / groups);  // tokens of one wave of four-token blocks
+  const int64_t wave = std::max(1, 4 * (router_wave / groups));  // tokens of one wave of four-token blocks
   if (many) {
     // How long the list is the data decide: 2 % of the tokens of normal rows, half of them with a few channels at 1000 times
     // the others, all where rows repeat a value (padding).  Blocks of few tokens are quicker for a short list: the first
-    // launch has them for a 32nd of the tokens (at least one wave, at most two) and takes up to two rounds of that.
-    // The second has up to 16 tokens a block and takes any longer list; each leaves the other's lists alone.  128 experts,
-    // 2880 columns, one launch / two, us: 8192 normal rows 133 / 138, nine channels at 1000 times the others 569 / 399, every
-    // second row zero 513 / 351, every row 870 / 540 (the chain alone 343); 1024 tokens 51 / 51, every row zero 165 / 94 (66).
+    // launch has them for a 32nd of the tokens (at least one wave of four-token blocks, at most two) and takes up to two rounds of
+    // that.  The second has up to 32 tokens a block and takes any longer list; each leaves the other's lists alone.  128 experts, 2880
+    // columns, one launch / two, us (before the chain's blocks were as they are): 8192 normal rows 133 / 138, nine channels at 1000
+    // times the others 569 / 399, every second row zero 513 / 351, every row 870 / 540 (the chain alone 343); 1024 tokens 51 / 51, every
+    // row zero 165 / 94 (66).  (With room for a quarter of a wave: 2048 tokens of eight slots, whose lists are longer, 284 -> 291 for
+    // the step.)
     const int few_slots = (int)std::min(2 * wave, std::max(wave, T / 32));
     b.list_max = 2 * few_slots;
-    launch_router_logits<true>(b, L->d_wg_few, L->d_wg_many, L->sm_count, s, pdl, few_slots);
+    launch_router_logits<true>(b, L->d_wg_few, L->d_wg_many, router_wave, s, pdl, few_slots);
     if (T > b.list_max) {
       b.list_over = b.list_max;
       b.list_max = INT32_MAX;
-      launch_router_logits<true>(b, L->d_wg_few, L->d_wg_many, L->sm_count, s, pdl, (int)std::min(T, 8 * wave));
+      launch_router_logits<true>(b, L->d_wg_few, L->d_wg_many, router_wave, s, pdl, (int)std::min(T, 8 * wave));
       L->last.launches += 1;
     }
   } else {
-    launch_router_logits<true>(b, L->d_wg_few, L->d_wg_many, L->sm_count, s, pdl, (int)std::min(T, wave));
+    launch_router_logits<true>(b, L->d_wg_few, L->d_wg_many, router_wave, s, pdl, (int)std::min(T, wave));
   }
   CSK_CUDA(L, cudaGetLastError());
   L->last.launches += 3;
@@ -894,6 +898,7 @@ int csk_moe_create(const csk_moe_config* cfg, csk_moe_layer** out) {
   CK(cudaMallocHost(&L->h_meta, sizeof(int) * 16));
   CK(cudaMallocHost(&L->h_counts64, sizeof(int64_t) * L->E));
   CK(router_prepare_device());
+  for (int g = 1; g <= kMaxExperts / 32; ++g) L->router_waves[g] = router_wave(g, L->sm_count);
   CK(mx_prepare_device());
   CK(few_prepare_device());
   CK(rt_prepare_device());
