@@ -871,23 +871,35 @@ k_router_topk(const float* __restrict__ logits, float* __restrict__ router_out, 
 // meta layout (int32): [0] row tiles, [1] total rows, [2] distinct experts,
 //                      [3] device status word (or-ed kDevErr*), [4] rows of the tallest row tile, [5..7] spare.
 // ---------------------------------------------------------------------------
+//
+// k_hist: rows per expert of a batch that is planned by two launches.  With `partial` every block leaves its own counts,
+// partial[block][E + 1], the last of them whether it met an id outside [0, E), and nothing has to be cleared beforehand;
+// else they are added to `counts` (zero at first) and the status word.
+constexpr int kHistBlocks = 32;
 __global__ void k_hist(const float* __restrict__ router_out, int n_pairs, int E, int only_expert,
-                       int* __restrict__ counts, int* __restrict__ meta) {
+                       int* __restrict__ counts, int* __restrict__ meta, int* __restrict__ partial = nullptr) {
   extern __shared__ int sc[];
-  for (int e = threadIdx.x; e < E; e += blockDim.x) sc[e] = 0;
+  for (int e = threadIdx.x; e <= E; e += blockDim.x) sc[e] = 0;
   __syncthreads();
+  griddep_wait();
+  griddep_launch();
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n_pairs; i += gridDim.x * blockDim.x) {
     const int e = (int)router_out[2 * (size_t)i];
     if (e < 0 || e >= E) {
-      atomicOr(&meta[3], kDevErrExpertRange);
+      sc[E] = 1;
       continue;
     }
     if (only_expert >= 0 && e != only_expert) continue;
     atomicAdd(&sc[e], 1);
   }
   __syncthreads();
+  if (partial) {
+    for (int e = threadIdx.x; e <= E; e += blockDim.x) partial[(size_t)blockIdx.x * (E + 1) + e] = sc[e];
+    return;
+  }
   for (int e = threadIdx.x; e < E; e += blockDim.x)
     if (sc[e]) atomicAdd(&counts[e], sc[e]);
+  if (threadIdx.x == 0 && sc[E]) atomicOr(&meta[3], kDevErrExpertRange);
 }
 
 // An expert with several tiles gets them equally tall instead of full ones and a short rest: for the block-scaled
@@ -903,56 +915,83 @@ __device__ __forceinline__ int even_tile_height(int cnt, int tile_rows, bool blo
 }
 
 // Exclusive scan of the per-expert row counts, row-tile list for tiles of
-// `tile_rows` rows, cursor reset.  One block of 1024 threads, E <= 1024.
+// `tile_rows` rows, cursor reset.  One block of whole warps, a thread for every expert.
 // counts are indexed by GLOBAL expert id; tiles carry the id local to this
 // device (e - e_begin); rows of experts outside [e_begin, e_begin+e_count) get
 // offsets but no tiles (under expert parallelism they belong to other devices).
 //
-// With router_out given (small batches) the block first builds the histogram
-// itself -- counts and the status word then need no clearing beforehand and the
-// whole plan is one launch.
+// The counts come from `counts` or, with `partial`, from k_hist's blocks; with router_out given (small batches: at most
+// kScanPairs pairs a thread) the block builds the histogram itself, and the whole plan is one launch.  In both cases counts
+// and the status word need no clearing beforehand.
 //
 // With row_of_pair given as well the block also places every pair: row_of_pair[i] = its row in
-// the grouped order (-1: not placed).  Which row of its expert's segment a pair gets depends on
-// the order of the block's atomics; a row's value does not depend on it.
-__global__ void __launch_bounds__(1024)
-k_scan(int* __restrict__ counts, int E, int e_begin, int e_count, int tile_rows, int max_rows,
-       int max_tiles, const uint8_t* __restrict__ resident, int* __restrict__ offsets,
-       int* __restrict__ cursor, RowTile* __restrict__ tiles, int* __restrict__ meta,
-       const float* __restrict__ router_out, int n_pairs, int only_expert,
-       int* __restrict__ row_of_pair = nullptr, ExpertTiles* __restrict__ expert_tiles = nullptr,
-       uint32_t* __restrict__ tile_masks = nullptr, int mask_words = 0, int4* __restrict__ places = nullptr) {
-  __shared__ int s_row_off[1025];
-  __shared__ int s_tile_off[1025];
+// the grouped order (-1: not placed).  Which row of its expert's segment a pair gets is what the histogram's atomic returned;
+// a row's value does not depend on it.
+//
+// Bound by its barriers and the latency of the routing's loads: 32 pairs, 128 experts 6.3 us with 1024 threads, a second
+// pass of loads and atomics for the places and a search of the offsets for every tile, now 5.3 (profiler, cold caches).
+constexpr int kScanPairs = 8;
+struct ScanArgs {
+  int *counts, *offsets, *cursor, *meta;
+  int E, e_begin, e_count, tile_rows, max_rows, max_tiles;
+  const uint8_t* resident;
+  RowTile* tiles;
+  const int* partial;           // or null
+  int n_partial;
+  const float* router_out;      // or null
+  int n_pairs, only_expert;
+  int* row_of_pair;             // or null
+  ExpertTiles* expert_tiles;    // block-scaled kernel: where the experts' tiles are, the tiles' words to clear, the pairs' places
+  uint32_t* tile_words;
+  int words_per_tile;
+  int4* places;
+};
+// Threads of the block.
+inline int scan_threads(int E, int n_pairs) { return std::min(1024, std::max(ceil_div(E, 32), ceil_div(n_pairs, 32)) * 32); }
+
+__global__ void __launch_bounds__(1024) k_scan(const ScanArgs A) {
+  __shared__ int s_row_off[1024], s_tile_off[1024], s_count[1024];
   __shared__ int s_warp[2][32];
-  __shared__ int s_distinct, s_tallest;
-  const int e = threadIdx.x, lane = e & 31, warp = e >> 5;
-  if (e == 0) s_distinct = s_tallest = 0;
+  __shared__ int s_distinct, s_tallest, s_status;
+  const int e = threadIdx.x, lane = e & 31, warp = e >> 5, B = blockDim.x, E = A.E;
+  if (e == 0) s_distinct = s_tallest = s_status = 0;
+  s_count[e] = 0;
+  __syncthreads();
   griddep_wait();
   griddep_launch();
-  if (router_out) {
-    s_tile_off[e] = 0;  // serves as the histogram until the scan below overwrites it
-    if (e == 0) meta[3] = 0;
-    __syncthreads();
-    for (int i = e; i < n_pairs; i += 1024) {
-      const int x = (int)router_out[2 * (size_t)i];
-      if (x < 0 || x >= E) {
-        atomicOr(&meta[3], kDevErrExpertRange);
-      } else if (only_expert < 0 || x == only_expert) {
-        atomicAdd(&s_tile_off[x], 1);
+  int x[kScanPairs], r[kScanPairs];  // the pairs of this thread: expert (-1: none, or not placed), row among the expert's
+  if (A.router_out) {
+#pragma unroll
+    for (int j = 0; j < kScanPairs; ++j) x[j] = e + j * B < A.n_pairs ? (int)A.router_out[2 * (size_t)(e + j * B)] : 0;
+#pragma unroll
+    for (int j = 0; j < kScanPairs; ++j) {
+      if (e + j * B >= A.n_pairs) {
+        x[j] = -1;
+      } else if (x[j] < 0 || x[j] >= E) {
+        x[j] = -1;
+        atomicOr(&s_status, kDevErrExpertRange);
+      } else if (A.only_expert >= 0 && x[j] != A.only_expert) {
+        x[j] = -1;
       }
+      if (x[j] >= 0) r[j] = atomicAdd(&s_count[x[j]], 1);
     }
+    __syncthreads();
+  } else if (e < E) {
+    int n = 0;
+    if (A.partial)
+      for (int b = 0; b < A.n_partial; ++b) n += A.partial[(size_t)b * (E + 1) + e];
+    else
+      n = A.counts[e];
+    s_count[e] = n;
   }
-  __syncthreads();
-  const int c = router_out ? s_tile_off[e] : (e < E ? counts[e] : 0);
-  if (router_out && e < E) counts[e] = c;
-  __syncthreads();  // every thread holds its count before s_tile_off is reused
-  const bool local = e >= e_begin && e < e_begin + e_count;
-  const int nt = local ? (c + tile_rows - 1) / tile_rows : 0;
-  auto tile_height = [&](int cnt) { return even_tile_height(cnt, tile_rows, expert_tiles != nullptr); };
+  if (A.partial && e < A.n_partial && A.partial[(size_t)e * (E + 1) + E]) atomicOr(&s_status, kDevErrExpertRange);
+  const int c = e < E ? s_count[e] : 0;
+  const bool local = e >= A.e_begin && e < A.e_begin + A.e_count;
+  const int nt = local ? (c + A.tile_rows - 1) / A.tile_rows : 0;
+  auto tile_height = [&](int cnt) { return even_tile_height(cnt, A.tile_rows, A.expert_tiles != nullptr); };
   if (c > 0) {
     atomicAdd(&s_distinct, 1);
-    if (local && resident && !resident[e - e_begin]) atomicOr(&meta[3], kDevErrNotResident);
+    if (local && A.resident && !A.resident[e - A.e_begin]) atomicOr(&s_status, kDevErrNotResident);
   }
   // block-wide inclusive scans of (c, nt)
   int rc = c, rt = nt;
@@ -968,134 +1007,122 @@ k_scan(int* __restrict__ counts, int E, int e_begin, int e_count, int tile_rows,
     s_warp[1][warp] = rt;
   }
   __syncthreads();
-  if (warp == 0) {
-    int a = s_warp[0][lane], b = s_warp[1][lane];
-    for (int o = 1; o < 32; o <<= 1) {
-      const int ua = __shfl_up_sync(0xffffffffu, a, o), ub = __shfl_up_sync(0xffffffffu, b, o);
-      if (lane >= o) {
-        a += ua;
-        b += ub;
-      }
-    }
-    s_warp[0][lane] = a;
-    s_warp[1][lane] = b;
-  }
-  __syncthreads();
-  const int base_c = warp ? s_warp[0][warp - 1] : 0, base_t = warp ? s_warp[1][warp - 1] : 0;
-  const int row_off = base_c + rc - c, tile_off = base_t + rt - nt;
+  // every warp adds up the warps before it and all of them
+  int wc = lane < B / 32 ? s_warp[0][lane] : 0, wt = lane < B / 32 ? s_warp[1][lane] : 0;
+  const int total_rows = __reduce_add_sync(0xffffffffu, wc), total_tiles = __reduce_add_sync(0xffffffffu, wt);
+  if (lane >= warp) wc = wt = 0;
+  const int row_off = __reduce_add_sync(0xffffffffu, wc) + rc - c, tile_off = __reduce_add_sync(0xffffffffu, wt) + rt - nt;
   s_row_off[e] = row_off;
   s_tile_off[e] = tile_off;
+  const bool over = total_rows > A.max_rows || total_tiles > A.max_tiles;
+  const int height = tile_height(c);
   if (e < E) {
-    offsets[e] = row_off;
-    cursor[e] = 0;
-    if (expert_tiles) expert_tiles[e] = ExpertTiles{tile_off, tile_height(c)};
+    if (A.router_out || A.partial) A.counts[e] = c;
+    A.offsets[e] = row_off;
+    A.cursor[e] = 0;
+    if (A.expert_tiles) A.expert_tiles[e] = ExpertTiles{tile_off, height};
   }
-  const int total_rows = s_warp[0][31], total_tiles = s_warp[1][31];
-  if (e == 0) {
-    s_row_off[1024] = total_rows;
-    s_tile_off[1024] = total_tiles;
-    offsets[E] = total_rows;
-    const bool over = total_rows > max_rows || total_tiles > max_tiles;
-    if (over) atomicOr(&meta[3], kDevErrCapacity);
-    meta[0] = over ? 0 : total_tiles;
-    meta[1] = total_rows;
+  if (nt && !over) {
+    for (int q = 0; q < nt; ++q) A.tiles[tile_off + q] = RowTile{e - A.e_begin, row_off + q * height, min(height, c - q * height), 0};
+    atomicMax(&s_tallest, min(height, c));
   }
   __syncthreads();
-  if (e == 0) meta[2] = s_distinct;
-  if (router_out && row_of_pair) {
-    // s_warp is free now: reuse nothing of it; the cursors live in s_cur
-    __shared__ int s_cur[1024];
-    s_cur[e] = 0;
-    __syncthreads();
-    const bool over = total_rows > max_rows || total_tiles > max_tiles;
-    for (int i = e; i < n_pairs; i += 1024) {
-      const int x = (int)router_out[2 * (size_t)i];
-      int pos = -1, r = -1;
-      if (!over && x >= 0 && x < E && (only_expert < 0 || x == only_expert)) {
-        r = atomicAdd(&s_cur[x], 1);
-        pos = s_row_off[x] + r;
-        if (pos >= max_rows) pos = -1;
+  if (e == 0) {
+    A.offsets[E] = total_rows;
+    A.meta[0] = over ? 0 : total_tiles;
+    A.meta[1] = total_rows;
+    A.meta[2] = s_distinct;
+    const int st = s_status | (over ? kDevErrCapacity : 0);
+    if (A.router_out || A.partial) A.meta[3] = st;
+    else if (st) atomicOr(&A.meta[3], st);
+    A.meta[4] = s_tallest;
+    A.meta[5] = A.meta[6] = 0;
+  }
+  if (A.router_out && A.row_of_pair) {
+#pragma unroll
+    for (int j = 0; j < kScanPairs; ++j) {
+      const int i = e + j * B;
+      if (i >= A.n_pairs) break;
+      int pos = -1;
+      if (!over && x[j] >= 0) {
+        pos = s_row_off[x[j]] + r[j];
+        if (pos >= A.max_rows) pos = -1;
       }
-      row_of_pair[i] = pos;
-      if (places) {
+      A.row_of_pair[i] = pos;
+      if (A.places) {
         // the pair's row tile (number, first row, rows) and its row in it, or -1: one load for the kernel that writes the rows
         // where it would chase expert, tile number and tile
         int4 at = make_int4(0, 0, 0, -1);
-        if (pos >= 0 && x >= e_begin && x < e_begin + e_count) {
-          const int cnt = (x < 1023 ? s_row_off[x + 1] : s_row_off[1024]) - s_row_off[x], per = tile_height(cnt), q = r / per;
-          at = make_int4(s_tile_off[x] + q, s_row_off[x] + q * per, min(per, cnt - q * per), r - q * per);
+        if (pos >= 0 && x[j] >= A.e_begin && x[j] < A.e_begin + A.e_count) {
+          const int cnt = s_count[x[j]], per = tile_height(cnt), q = r[j] / per;
+          at = make_int4(s_tile_off[x[j]] + q, s_row_off[x[j]] + q * per, min(per, cnt - q * per), r[j] - q * per);
         }
-        places[i] = at;
+        A.places[i] = at;
       }
     }
   }
-  if (total_rows > max_rows || total_tiles > max_tiles) {
-    if (e == 0) meta[4] = 0;
-    return;
-  }
-  if (tile_masks)  // the block-scaled kernel's record masks: nothing marked yet
-    for (int i = threadIdx.x; i < total_tiles * mask_words; i += blockDim.x) tile_masks[i] = 0;
-  for (int i = threadIdx.x; i < total_tiles; i += blockDim.x) {
-    // largest expert x with s_tile_off[x] <= i (experts without tiles repeat an offset)
-    int lo = 0, hi = 1023;
-    while (lo < hi) {
-      const int mid = (lo + hi + 1) >> 1;
-      if (s_tile_off[mid] <= i) lo = mid; else hi = mid - 1;
-    }
-    // step back over empty experts that share the offset: the owner is the last
-    // expert with that offset that actually has tiles, i.e. the largest index.
-    const int cnt = (lo < 1023 ? s_row_off[lo + 1] : s_row_off[1024]) - s_row_off[lo];
-    const int per = tile_height(cnt);
-    const int r = (i - s_tile_off[lo]) * per;
-    RowTile t;
-    t.expert = lo - e_begin;
-    t.row0 = s_row_off[lo] + r;
-    t.rows = min(per, cnt - r);
-    t.pad = 0;
-    tiles[i] = t;
-    atomicMax(&s_tallest, t.rows);
-  }
-  __syncthreads();
-  if (e == 0) meta[4] = s_tallest;
+  if (A.tile_words && !over)  // the block-scaled kernel's record masks and counts: nothing marked or done yet
+    for (int i = e; i < total_tiles * A.words_per_tile; i += B) A.tile_words[i] = 0;
 }
 
-// One warp per (token, slot) pair: claim a row in the expert's segment, record
-// the maps, and write the token's hidden row there as fp16 (times the routing
-// weight when it is applied before the expert).
-__global__ void k_scatter(const float* __restrict__ router_out, const float* __restrict__ hidden,
-                          int n_pairs, int k, int H, int E, int only_expert,
-                          const int* __restrict__ offsets, int* __restrict__ cursor,
-                          int* __restrict__ row_of_pair, __half* __restrict__ x16, int ldx,
-                          int max_rows, int weight_before_ffn) {
-  const int lane = threadIdx.x & 31;
-  const int warps_per_block = blockDim.x >> 5;
-  griddep_wait();
-  griddep_launch();
-  for (int i = blockIdx.x * warps_per_block + (threadIdx.x >> 5); i < n_pairs;
-       i += gridDim.x * warps_per_block) {
-    const int e = (int)router_out[2 * (size_t)i];
-    const float w = router_out[2 * (size_t)i + 1];
-    int pos = -1;
-    if (e >= 0 && e < E && (only_expert < 0 || e == only_expert)) {
-      if (lane == 0) pos = offsets[e] + atomicAdd(&cursor[e], 1);
-      pos = __shfl_sync(0xffffffffu, pos, 0);
-      if (pos >= max_rows) pos = -1;
-    }
-    if (lane == 0) row_of_pair[i] = pos;
-    if (pos < 0) continue;
-    const float* src = hidden + (size_t)(i / k) * H;
-    __half* dst = x16 + (size_t)pos * ldx;
-    const float mul = weight_before_ffn ? w : 1.0f;
-    for (int d = lane * 4; d < H; d += 128) {
-      const float4 v = *reinterpret_cast<const float4*>(src + d);
-      __half2 a = __floats2half2_rn(v.x * mul, v.y * mul);
-      __half2 b = __floats2half2_rn(v.z * mul, v.w * mul);
-      uint2 o;
-      o.x = *reinterpret_cast<uint32_t*>(&a);
-      o.y = *reinterpret_cast<uint32_t*>(&b);
-      *reinterpret_cast<uint2*>(dst + d) = o;
+// One block per token: its hidden row goes to the token's rows as fp16 (times the routing weight when it is applied before the
+// expert).  The rows are given (cursor null) or claimed here, in the experts' segments.  The hidden states are older than the
+// kernel before this one and are on their way while that ends; a row is read once and stored k times, 16 bytes a thread.
+// Bound by HBM (4 H bytes in, 2 k H out): 4096 tokens x 4 slots x 2880 columns, 141 MB, 19.5 us (a warp per pair,
+// eight bytes a lane: 38).
+constexpr int kScatterThreads = 128, kScatterKept = 3;  // columns of a row in registers: 8 x 128 x 3
+__global__ void __launch_bounds__(kScatterThreads) k_scatter(const float* __restrict__ router_out, const float* __restrict__ hidden,
+                                                             int k, int H, int E, int only_expert, const int* __restrict__ offsets,
+                                                             int* __restrict__ cursor, int* __restrict__ row_of_pair,
+                                                             __half* __restrict__ x16, int ldx, int max_rows, int weight_before_ffn) {
+  __shared__ int s_pos[kMaxTopK];
+  __shared__ float s_w[kMaxTopK];
+  const int t = blockIdx.x;
+  const float* src = hidden + (size_t)t * H;
+  float4 v[kScatterKept][2];
+#pragma unroll
+  for (int i = 0; i < kScatterKept; ++i) {
+    const int d = (threadIdx.x + i * kScatterThreads) * 8;
+    if (d < H) {
+      v[i][0] = __ldg(reinterpret_cast<const float4*>(src + d));
+      v[i][1] = __ldg(reinterpret_cast<const float4*>(src + d + 4));
     }
   }
+  griddep_wait();
+  griddep_launch();
+  if ((int)threadIdx.x < k) {
+    const size_t i = (size_t)t * k + threadIdx.x;
+    int pos = -1;
+    if (!cursor) {
+      pos = row_of_pair[i];
+    } else {
+      const int e = (int)router_out[2 * i];
+      if (e >= 0 && e < E && (only_expert < 0 || e == only_expert)) {
+        pos = offsets[e] + atomicAdd(&cursor[e], 1);
+        if (pos >= max_rows) pos = -1;
+      }
+      row_of_pair[i] = pos;
+    }
+    s_pos[threadIdx.x] = pos;
+    s_w[threadIdx.x] = weight_before_ffn ? router_out[2 * i + 1] : 1.0f;
+  }
+  __syncthreads();
+  auto store = [&](int d, const float4& a, const float4& b) {
+    for (int j = 0; j < k; ++j) {
+      if (s_pos[j] < 0) continue;
+      const float m = s_w[j];
+      const __half2 h[4] = {__floats2half2_rn(a.x * m, a.y * m), __floats2half2_rn(a.z * m, a.w * m),
+                            __floats2half2_rn(b.x * m, b.y * m), __floats2half2_rn(b.z * m, b.w * m)};
+      *reinterpret_cast<uint4*>(x16 + (size_t)s_pos[j] * ldx + d) = *reinterpret_cast<const uint4*>(h);
+    }
+  };
+#pragma unroll
+  for (int i = 0; i < kScatterKept; ++i) {
+    const int d = (threadIdx.x + i * kScatterThreads) * 8;
+    if (d < H) store(d, v[i][0], v[i][1]);
+  }
+  for (int d = (threadIdx.x + kScatterKept * kScatterThreads) * 8; d < H; d += 8 * kScatterThreads)
+    store(d, __ldg(reinterpret_cast<const float4*>(src + d)), __ldg(reinterpret_cast<const float4*>(src + d + 4)));
 }
 
 // The whole plan of a dense FFN (one expert, every token in order): rows to fp16, and by block 0 what k_scan leaves for
@@ -1136,7 +1163,9 @@ __global__ void __launch_bounds__(256) k_dense_rows(const float* __restrict__ hi
 // ---------------------------------------------------------------------------
 //
 // Bound by HBM (k rows of y in, one out).  Four slots' rows are requested at once: one at a time a
-// step of 8192 tokens took 2046 us, with four 2011; 2048 tokens of eight slots 318 and 306.
+// step of 8192 tokens took 2046 us, with four 2011; 2048 tokens of eight slots 318 and 306.  A few tokens are bound by the
+// latency of their loads: a row is then dealt to several blocks (gridDim.y), so that a thread has one round of them (8 tokens of
+// 2880 columns 7.9 -> 4.5 us, profiler).
 //
 // carry (optional; the host entry point that runs a batch in several passes): block 0 folds this
 // pass's status word into a sticky one and adds its per-expert row counts to running totals --
@@ -1153,7 +1182,7 @@ __global__ void __launch_bounds__(256) k_combine(const float* __restrict__ route
   const int t = blockIdx.x;
   griddep_wait();
   griddep_launch();
-  if (carry && t == 0) {
+  if (carry && t == 0 && blockIdx.y == 0) {
     if (threadIdx.x == 0 && meta[3]) atomicOr(&carry[0], meta[3]);
     for (int e = threadIdx.x; e < E; e += blockDim.x) carry[1 + e] += counts[e];
   }
@@ -1163,7 +1192,7 @@ __global__ void __launch_bounds__(256) k_combine(const float* __restrict__ route
     s_w[threadIdx.x] = unweighted ? 1.f : router_out[((size_t)t * k + threadIdx.x) * 2 + 1];  // 1 * v is v
   }
   __syncthreads();
-  for (int d = threadIdx.x * 4; d < H; d += blockDim.x * 4) {
+  for (int d = (blockIdx.y * blockDim.x + threadIdx.x) * 4; d < H; d += gridDim.y * blockDim.x * 4) {
     float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
     bool done = false;
     for (int j0 = 0; j0 < k && !done; j0 += kCombineAtOnce) {
@@ -1213,56 +1242,79 @@ __global__ void __launch_bounds__(256) k_combine(const float* __restrict__ route
 // sequential fp32 chain of separate multiplies and adds, division, square root and products are the
 // IEEE round-to-nearest operations the reference's scalar code performs.
 //
-// A block per token: all its threads square the row into shared memory, one walks the squares (sixteen
-// in registers while the sixteen before are added), all of them scale the row.  Bound by that chain: 8 tokens x 2880 columns
-// 14.6 us with 32 copied from register to register, now 11.4 (4.4 cycles a column would be 6.5).
+// A block per token: all its threads square the row into shared memory (and keep it, and its weights, in registers), one walks
+// the squares, 32 columns of them in registers ahead, all of them scale the row.  Bound by that chain, 4.3 cycles a column: 8
+// tokens x 2880 columns 14.1 -> 10.2 us (profiler, cold caches; 16 columns ahead and the row read twice before).
 // ---------------------------------------------------------------------------
-__global__ void __launch_bounds__(128) k_rmsnorm(const float* __restrict__ x, const float* __restrict__ w, float eps,
-                                                 float* __restrict__ out, int T, int H) {
+constexpr int kNormThreads = 256, kNormKept = 4;  // 4096 columns in registers; the rest of a longer row is read again
+template <int N>
+__device__ __forceinline__ float add_columns(float s, uint32_t at) {
+  constexpr int G = N / 4, A = 8;
+  float4 v[A];
+#pragma unroll
+  for (int g = 0; g < A; ++g) v[g] = lds128(at + 16 * g);
+#pragma unroll
+  for (int g = 0; g < G; ++g) {
+    const float4 u = v[g % A];
+    if (g + A < G) v[g % A] = lds128(at + 16 * (g + A));
+    s = __fadd_rn(__fadd_rn(__fadd_rn(__fadd_rn(s, u.x), u.y), u.z), u.w);
+  }
+  return s;
+}
+__global__ void __launch_bounds__(kNormThreads) k_rmsnorm(const float* __restrict__ x, const float* __restrict__ w, float eps,
+                                                          float* __restrict__ out, int T, int H) {
   extern __shared__ __align__(16) float rms_sq[];
   __shared__ float s_rms;
+  float4 g[kNormKept];
+#pragma unroll
+  for (int i = 0; i < kNormKept; ++i) {
+    const int d = (threadIdx.x + i * kNormThreads) * 4;
+    if (d < H) g[i] = __ldg(reinterpret_cast<const float4*>(w + d));
+  }
   griddep_wait();
   griddep_launch();
   for (int t = blockIdx.x; t < T; t += gridDim.x) {
     const float* src = x + (size_t)t * H;
-    for (int d = threadIdx.x * 4; d < H; d += 512) {
-      const float4 v = __ldg(reinterpret_cast<const float4*>(src + d));
+    auto square = [&](int d, const float4& v) {
       *reinterpret_cast<float4*>(rms_sq + d) = make_float4(__fmul_rn(v.x, v.x), __fmul_rn(v.y, v.y), __fmul_rn(v.z, v.z), __fmul_rn(v.w, v.w));
+    };
+    auto scale = [&](int d, const float4& v, const float4& f, float rms) {
+      *reinterpret_cast<float4*>(out + (size_t)t * H + d) =
+          make_float4(__fmul_rn(__fdiv_rn(v.x, rms), f.x), __fmul_rn(__fdiv_rn(v.y, rms), f.y), __fmul_rn(__fdiv_rn(v.z, rms), f.z),
+                      __fmul_rn(__fdiv_rn(v.w, rms), f.w));
+    };
+    float4 kept[kNormKept];
+#pragma unroll
+    for (int i = 0; i < kNormKept; ++i) {
+      const int d = (threadIdx.x + i * kNormThreads) * 4;
+      if (d < H) kept[i] = __ldg(reinterpret_cast<const float4*>(src + d));
     }
+#pragma unroll
+    for (int i = 0; i < kNormKept; ++i) {
+      const int d = (threadIdx.x + i * kNormThreads) * 4;
+      if (d < H) square(d, kept[i]);
+    }
+    for (int d = (threadIdx.x + kNormKept * kNormThreads) * 4; d < H; d += 4 * kNormThreads) square(d, __ldg(reinterpret_cast<const float4*>(src + d)));
     __syncthreads();
     if (threadIdx.x == 0) {
-      const float4* q = reinterpret_cast<const float4*>(rms_sq);
+      const uint32_t at = smem_u32(rms_sq);
       float s = 0.f;
-      auto add = [&](const float4 (&v)[4]) {
-#pragma unroll
-        for (int i = 0; i < 4; ++i) s = __fadd_rn(__fadd_rn(__fadd_rn(__fadd_rn(s, v[i].x), v[i].y), v[i].z), v[i].w);
-      };
-      float4 u[4], v[4];
-#pragma unroll
-      for (int i = 0; i < 4; ++i) u[i] = q[i];
+      int d = 0;
 #pragma unroll 1
-      for (int d = 0; d < H / 4; d += 8) {  // H is a multiple of 32
-#pragma unroll
-        for (int i = 0; i < 4; ++i) v[i] = q[d + 4 + i];
-        add(u);
-        const int after = d + 8 < H / 4 ? d + 8 : d;  // (the last ones are not used)
-#pragma unroll
-        for (int i = 0; i < 4; ++i) u[i] = q[after + i];
-        add(v);
-      }
+      for (; d + 192 <= H; d += 192) s = add_columns<192>(s, at + 4 * d);
+#pragma unroll 1
+      for (; d < H; d += 32) s = add_columns<32>(s, at + 4 * d);  // H is a multiple of 32
       s_rms = __fsqrt_rn(__fadd_rn(__fdiv_rn(s, (float)H), eps));
     }
     __syncthreads();
     const float rms = s_rms;
-    for (int d = threadIdx.x * 4; d < H; d += 512) {
-      const float4 v = __ldg(reinterpret_cast<const float4*>(src + d)), g = __ldg(reinterpret_cast<const float4*>(w + d));
-      float4 o;
-      o.x = __fmul_rn(__fdiv_rn(v.x, rms), g.x);
-      o.y = __fmul_rn(__fdiv_rn(v.y, rms), g.y);
-      o.z = __fmul_rn(__fdiv_rn(v.z, rms), g.z);
-      o.w = __fmul_rn(__fdiv_rn(v.w, rms), g.w);
-      *reinterpret_cast<float4*>(out + (size_t)t * H + d) = o;
+#pragma unroll
+    for (int i = 0; i < kNormKept; ++i) {
+      const int d = (threadIdx.x + i * kNormThreads) * 4;
+      if (d < H) scale(d, kept[i], g[i], rms);
     }
+    for (int d = (threadIdx.x + kNormKept * kNormThreads) * 4; d < H; d += 4 * kNormThreads)
+      scale(d, __ldg(reinterpret_cast<const float4*>(src + d)), __ldg(reinterpret_cast<const float4*>(w + d)), rms);
     __syncthreads();  // s_rms and the squares are rewritten for the block's next token
   }
 }

@@ -94,6 +94,7 @@ struct csk_moe_layer {
   __half* d_a16 = nullptr;    // [max_rows+pad, lda]
   float* d_y = nullptr;       // [max_rows, H]
   int ldx = 0, lda = 0;
+  int* d_hist = nullptr;       // [kHistBlocks][E + 1] row counts of a large batch's plan
   int* d_counts = nullptr;       // [E]
   int* d_offsets = nullptr;      // [E+1]
   int* d_cursor = nullptr;       // [E]
@@ -342,6 +343,29 @@ int launch_router(csk_moe_layer* L, const float* d_hidden, int64_t T, float* d_r
   return CSK_OK;
 }
 
+ScanArgs scan_args(csk_moe_layer* L, int tile_rows, int e_begin, int e_count, const uint8_t* resident, int64_t max_rows, bool digits) {
+  ScanArgs p{};
+  p.counts = L->d_counts;
+  p.offsets = L->d_offsets;
+  p.cursor = L->d_cursor;
+  p.meta = L->d_meta;
+  p.E = L->E;
+  p.e_begin = e_begin;
+  p.e_count = e_count;
+  p.tile_rows = tile_rows;
+  p.max_rows = (int)max_rows;
+  p.max_tiles = L->max_tiles;
+  p.resident = resident;
+  p.tiles = L->d_tiles;
+  p.only_expert = -1;
+  if (digits) {
+    p.expert_tiles = L->d_expert_tiles;
+    p.tile_words = L->d_wide;
+    p.words_per_tile = wide_stride(L);
+  }
+  return p;
+}
+
 // histogram -> scan (+ row tiles of `tile_rows`) -> token rows: as fp16 rows into x16, or (x16 null) as digits into
 // the block-scaled kernel's image
 constexpr int kOneBlockPairs = 8192;  // up to here histogram, scan and tile list are one single-block launch
@@ -352,24 +376,23 @@ int launch_permute(csk_moe_layer* L, const float* d_hidden, const float* d_route
   const uint8_t* res = e_count ? L->d_resident : nullptr;
   const bool digits = x16 == nullptr;
   const bool one_block = n_pairs <= kOneBlockPairs;
-  ExpertTiles* et = digits ? L->d_expert_tiles : nullptr;
+  ScanArgs p = scan_args(L, tile_rows, e_begin, e_count, res, max_rows, digits);
   if (one_block) {
     // small batch: histogram, scan, tile list (and, for digits, the rows' places) in one single-block launch
-    launch_k(k_scan, dim3(1), dim3(1024), 0, s, L->pdl, L->d_counts, L->E, e_begin, e_count, tile_rows, (int)max_rows,
-             L->max_tiles, res, L->d_offsets, L->d_cursor, L->d_tiles, L->d_meta, d_router, n_pairs, only_expert,
-             digits ? L->d_row_of_pair : (int*)nullptr, et, digits ? L->d_wide : (uint32_t*)nullptr, wide_stride(L),
-             digits ? L->d_places : (int4*)nullptr);
+    p.router_out = d_router;
+    p.n_pairs = n_pairs;
+    p.only_expert = only_expert;
+    p.row_of_pair = L->d_row_of_pair;
+    p.places = digits ? L->d_places : nullptr;
     L->last.launches += 1;
   } else {
-    CSK_CUDA(L, cudaMemsetAsync(L->d_counts, 0, sizeof(int) * L->E, s));
-    CSK_CUDA(L, cudaMemsetAsync(L->d_meta, 0, sizeof(int) * 8, s));
-    k_hist<<<grid_for(n_pairs, 256, 2 * L->sm_count), 256, sizeof(int) * L->E, s>>>(
-        d_router, n_pairs, L->E, only_expert, L->d_counts, L->d_meta);
-    k_scan<<<1, 1024, 0, s>>>(L->d_counts, L->E, e_begin, e_count, tile_rows, (int)max_rows, L->max_tiles, res,
-                              L->d_offsets, L->d_cursor, L->d_tiles, L->d_meta, nullptr, 0, -1, nullptr, et,
-                              digits ? L->d_wide : nullptr, wide_stride(L), nullptr);
+    launch_k(k_hist, dim3(kHistBlocks), dim3(512), sizeof(int) * (L->E + 1), s, L->pdl, d_router, n_pairs, L->E, only_expert, L->d_counts,
+             L->d_meta, L->d_hist);
+    p.partial = L->d_hist;
+    p.n_partial = kHistBlocks;
     L->last.launches += 2;
   }
+  launch_k(k_scan, dim3(1), dim3(scan_threads(L->E, one_block ? n_pairs : 0)), 0, s, L->pdl, p);
   if (digits) {
     MxQuantArgs a{};
     a.hidden = d_hidden;
@@ -398,9 +421,8 @@ int launch_permute(csk_moe_layer* L, const float* d_hidden, const float* d_route
     a.recs = L->Lgu.recs;
     launch_k(k_mx_quant, dim3((unsigned)T), dim3(std::min(kMxQuantThreads, ceil_div(L->Lgu.blocks, 8) * 32)), 0, s, L->pdl, a);
   } else {
-    launch_k(k_scatter, dim3(grid_for(n_pairs, 8, 8 * L->sm_count)), dim3(256), 0, s, L->pdl, d_router, d_hidden,
-             n_pairs, L->k, L->H, L->E, only_expert, L->d_offsets, L->d_cursor, L->d_row_of_pair, x16, ldx, (int)max_rows,
-             L->cfg.weight_before_ffn);
+    launch_k(k_scatter, dim3((unsigned)T), dim3(kScatterThreads), 0, s, L->pdl, d_router, d_hidden, L->k, L->H, L->E, only_expert, L->d_offsets,
+             one_block ? (int*)nullptr : L->d_cursor, L->d_row_of_pair, x16, ldx, (int)max_rows, L->cfg.weight_before_ffn);
   }
   CSK_CUDA(L, cudaGetLastError());
   L->last.launches += 1;
@@ -705,7 +727,9 @@ int forward_dev(csk_moe_layer* L, const float* d_hidden, int64_t T, const float*
   if (rc) return rc;
   // the shared expert's rows come from another stream: the combine is the first kernel that reads them
   if (shared_ready) CSK_CUDA(L, cudaStreamWaitEvent(s, shared_ready, 0));
-  launch_k(k_combine, dim3((unsigned)T), dim3(256), 0, s, L->pdl && !shared_ready, router, L->d_row_of_pair,
+  // (few tokens: a row dealt to several blocks)
+  const unsigned row_blocks = T < 4 * L->sm_count ? (unsigned)ceil_div(L->H, 1024) : 1u;
+  launch_k(k_combine, dim3((unsigned)T, row_blocks), dim3(256), 0, s, L->pdl && !shared_ready, router, L->d_row_of_pair,
            (const float*)L->d_y, L->H, d_out, (int)T, L->k, L->H, (int)L->cfg.weight_before_ffn, (int)(only_expert >= 0),
            (const int*)L->d_meta, (const int*)L->d_counts, L->carry_active ? L->d_carry : (int*)nullptr, L->E, d_residual,
            d_shared);
@@ -884,6 +908,7 @@ int csk_moe_create(const csk_moe_config* cfg, csk_moe_layer** out) {
   CK(cudaMemset(L->d_a16, 0, sizeof(__half) * (L->max_rows + pad_rows) * L->lda));
   CK(cudaMalloc(&L->d_y, sizeof(float) * L->max_rows * L->H));
   CK(cudaMalloc(&L->d_counts, sizeof(int) * L->E));
+  CK(cudaMalloc(&L->d_hist, sizeof(int) * kHistBlocks * (L->E + 1)));
   CK(cudaMalloc(&L->d_offsets, sizeof(int) * (L->E + 1)));
   CK(cudaMalloc(&L->d_cursor, sizeof(int) * L->E));
   CK(cudaMalloc(&L->d_row_of_pair, sizeof(int) * L->max_rows));
@@ -933,7 +958,7 @@ int csk_moe_destroy(csk_moe_layer* L) {
   for (void* p : L->ipc_opened) cudaIpcCloseMemHandle(p);
   void* dev[] = {L->d_shared_out, L->d_p2p_epoch, L->d_unit_router, L->d_stage2, L->d_norm_w, L->d_normed, L->d_part, L->d_hn2, L->d_wnorm, L->d_wg_tc, L->d_wg_tc_scale, L->d_wnorm_tc, L->d_fb_list, L->d_fb, L->d_info, L->d_back, L->d_row_ptr, L->d_p2p_base, L->d_peer_x16, L->d_peer_info, L->d_peer_back,
                  L->d_router_phys, L->d_slot_map, L->d_weights, L->d_resident, L->d_stage, L->d_wg, L->d_wg_few, L->d_wg_many, L->d_route_cnt, L->d_logits, L->d_rbias, L->d_hidden,
-                 L->d_router, L->d_out, L->d_x16, L->d_a16, L->d_y, L->d_counts, L->d_offsets,
+                 L->d_router, L->d_out, L->d_x16, L->d_a16, L->d_y, L->d_counts, L->d_hist, L->d_offsets,
                  L->d_cursor, L->d_row_of_pair, L->d_places, L->d_expert_tiles, L->d_ximg, L->d_aimg, L->d_wide, L->d_out_row_map, L->d_seg, L->d_tiles, L->d_meta};
   for (void* p : dev)
     if (p) cudaFree(p);
@@ -1576,7 +1601,7 @@ int csk_moe_block_forward_dev(csk_moe_layer* L, const float* d_x, int64_t T, flo
   CSK_CUDA(L, cudaSetDevice(L->cfg.device));
   cudaStream_t s = pick(L, stream);
   const int blocks = (int)std::min<int64_t>(T, 16 * (int64_t)L->sm_count);
-  k_rmsnorm<<<blocks, 128, sizeof(float) * L->H, s>>>(d_x, L->d_norm_w, L->norm_eps, L->d_normed, (int)T, L->H);
+  launch_k(k_rmsnorm, dim3((unsigned)blocks), dim3(kNormThreads), sizeof(float) * L->H, s, !L->timing, d_x, (const float*)L->d_norm_w, L->norm_eps, L->d_normed, (int)T, L->H);
   CSK_CUDA(L, cudaGetLastError());
   return forward_dev(L, L->d_normed, T, nullptr, d_router_out, d_out, -1, s, false, d_x);
 }
@@ -1605,7 +1630,7 @@ int csk_moe_block_forward_shared_dev(csk_moe_layer* L, csk_moe_layer* S, const f
   }
   cudaStream_t s = pick(L, stream);
   const int blocks = (int)std::min<int64_t>(T, 16 * (int64_t)L->sm_count);
-  k_rmsnorm<<<blocks, 128, sizeof(float) * L->H, s>>>(d_x, L->d_norm_w, L->norm_eps, L->d_normed, (int)T, L->H);
+  launch_k(k_rmsnorm, dim3((unsigned)blocks), dim3(kNormThreads), sizeof(float) * L->H, s, !L->timing, d_x, (const float*)L->d_norm_w, L->norm_eps, L->d_normed, (int)T, L->H);
   CSK_CUDA(L, cudaGetLastError());
   // the shared expert reads the normed rows on its own stream, next to the routed experts; the combine joins them
   CSK_CUDA(L, cudaEventRecord(L->ev_shared_fork, s));
@@ -2100,7 +2125,7 @@ int csk_moe_ep_p2p_counts_dev(csk_moe_layer* L, const float* d_hidden, int64_t T
   }
   CSK_CUDA(L, cudaMemsetAsync(L->d_counts, 0, sizeof(int) * L->E, s));
   CSK_CUDA(L, cudaMemsetAsync(L->d_meta, 0, sizeof(int) * 8, s));
-  k_hist<<<grid_for(n_pairs, 256, 2 * L->sm_count), 256, sizeof(int) * L->E, s>>>(router, n_pairs, L->E, -1, L->d_counts,
+  k_hist<<<grid_for(n_pairs, 256, 2 * L->sm_count), 256, sizeof(int) * (L->E + 1), s>>>(router, n_pairs, L->E, -1, L->d_counts,
                                                                                  L->d_meta);
   CSK_CUDA(L, cudaGetLastError());
   CSK_CUDA(L, cudaMemcpyAsync(d_counts, L->d_counts, sizeof(int) * L->E, cudaMemcpyDeviceToDevice, s));
@@ -2157,9 +2182,7 @@ int csk_moe_ep_p2p_experts_dev(csk_moe_layer* L, const int32_t* d_all_counts, in
   const bool mx = path == CSK_PATH_STREAM;
   // the status word of the dispatch stays; the tile list is rebuilt from the received counts
   k_ep_p2p_local_counts<<<(L->E + 255) / 256, 256, 0, s>>>(d_all_counts, L->p2p_world, L->E, L->e0, L->Eloc, L->d_counts);
-  k_scan<<<1, 1024, 0, s>>>(L->d_counts, L->E, L->e0, L->Eloc, tile_rows, (int)(mx ? L->mx_rows : L->max_rows), L->max_tiles,
-                            L->d_resident, L->d_offsets, L->d_cursor, L->d_tiles, L->d_meta, nullptr, 0, -1, nullptr,
-                            mx ? L->d_expert_tiles : nullptr, mx ? L->d_wide : nullptr, wide_stride(L));
+  k_scan<<<1, scan_threads(L->E, 0), 0, s>>>(scan_args(L, tile_rows, L->e0, L->Eloc, L->d_resident, mx ? L->mx_rows : L->max_rows, mx));
   k_ep_p2p_rowptr<<<4 * L->sm_count, 256, 0, s>>>(L->d_info, L->d_meta, L->d_peer_back, L->H, L->d_row_ptr,
                                                   (int)L->max_rows, L->p2p_world, (int)L->max_rows);
   CSK_CUDA(L, cudaGetLastError());
@@ -2205,9 +2228,7 @@ int csk_moe_ep_experts_dev(csk_moe_layer* L, const void* d_recv_f16, const int32
   CSK_CUDA(L, cudaMemsetAsync(L->d_meta, 0, sizeof(int) * 8, s));
   CSK_CUDA(L, cudaMemsetAsync(L->d_counts, 0, sizeof(int) * L->E, s));
   k_ep_plan<<<1, 1024, 0, s>>>(d_recv_counts, n_src, L->Eloc, L->e0, L->d_counts, L->d_seg);
-  k_scan<<<1, 1024, 0, s>>>(L->d_counts, L->E, L->e0, L->Eloc, tile_rows, (int)(mx ? L->mx_rows : L->max_rows), L->max_tiles,
-                            L->d_resident, L->d_offsets, L->d_cursor, L->d_tiles, L->d_meta, nullptr, 0, -1, nullptr,
-                            mx ? L->d_expert_tiles : nullptr, mx ? L->d_wide : nullptr, wide_stride(L));
+  k_scan<<<1, scan_threads(L->E, 0), 0, s>>>(scan_args(L, tile_rows, L->e0, L->Eloc, L->d_resident, mx ? L->mx_rows : L->max_rows, mx));
   k_ep_regroup<<<dim3((unsigned)(n_src * L->Eloc), (unsigned)std::max(1, 16 * L->sm_count / (n_src * L->Eloc))), 128, 0, s>>>((const __half*)d_recv_f16, L->d_x16, L->ldx, L->d_seg,
                                                L->d_offsets, n_src, L->Eloc, L->e0, L->d_out_row_map);
   CSK_CUDA(L, cudaGetLastError());

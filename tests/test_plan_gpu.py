@@ -1,0 +1,50 @@
+"""The plan of a batch (rows per expert, row tiles, places) where its block, its pairs per thread and its two forms end: the
+caller's routing, against the CPU restatement, and the counters."""
+import numpy as np
+import pytest
+import torch
+
+from coalsack_b200 import CskError, MoeLayer, PATH_STREAM, PATH_TILE, synth
+from tests import cases
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("E,k,T", [
+    (1, 1, 1), (33, 4, 9),                       # fewer pairs than threads; experts in two warps
+    (1024, 1, 3), (1024, 2, 700),                # a thread per expert, one and two pairs each
+    (3, 2, 4096), (3, 2, 4097), (40, 8, 1025),   # the most pairs of one launch and the fewest of two
+])
+@pytest.mark.parametrize("path", [PATH_STREAM, PATH_TILE])
+def test_plan_edges(gpu_lib, port, E, k, T, path):
+    sh = synth.tiny(seed=E + T, E=E, k=k, H=32, F=32, T=T, has_bias=True)
+    h, Wg, rb, ex = cases.layer_inputs(sh)
+    lay = MoeLayer.from_shape(sh)
+    lay.set_router(Wg, rb)
+    lay.load_experts(ex)
+    lay.set_path(path)
+    rng = np.random.default_rng(T)
+    ro = rng.uniform(0.1, 1.0, (T, k, 2)).astype(np.float32)
+    ro[..., 0] = [rng.permutation(E)[:k] for _ in range(T)]
+    h_d, out_d = torch.from_numpy(h).cuda(), torch.empty((T, 32), device="cuda")
+    torch.cuda.synchronize()
+
+    def forward(routing):  # (on device buffers: never cut into passes)
+        r = torch.from_numpy(routing).cuda()
+        torch.cuda.synchronize()
+        lay.forward_dev(h_d, T, out_d, d_router_in=r)
+        lay.sync()
+        return out_d.cpu().numpy()
+
+    out = forward(ro)
+    want, _ = port.moe_layer(h, Wg, rb, ex, k, sh.act, router_out=ro)
+    mx, mr = cases.err_stats(out, want)
+    assert mx <= cases.MAX_ABS_OVER_RMS and mr <= cases.MEAN_REL, (mx, mr)
+    rows, distinct, _ = lay.counters()
+    assert np.array_equal(rows, np.bincount(ro[..., 0].astype(int).ravel(), minlength=E)) and distinct == (rows > 0).sum()
+    bad = ro.copy()
+    bad[T - 1, k - 1, 0] = E
+    with pytest.raises(CskError, match="out of range"):
+        forward(bad)
+    assert np.array_equal(forward(ro), out)
+    lay.close()
