@@ -605,7 +605,7 @@ int launch_experts(csk_moe_layer* L, int path, float* y, int ldy, const int* out
     if (use_pairs(L))
       rc = pair_launch(L->pair, L->tile, L->tile.pair_x, L->tile.pair_a, L->d_weights, L->expert_stride, L->off_tgu,
                        L->off_td, L->off_bias, L->off_meta, L->Tgu, L->Td, L->d_a16, L->lda, y, ldy, out_row_map,
-                       out_row_ptr, L->d_tiles, L->d_meta, L->cfg.has_bias, L->cfg.activation, L->F, s,
+                       out_row_ptr, L->d_tiles, L->d_meta, L->cfg.has_bias, L->cfg.activation, L->F, s, L->pdl,
                        [&]() { tm.mark(); }, L->debug_stall);
     else
       rc = tile_launch(L->tile, L->d_weights, L->expert_stride, L->off_tgu, L->off_td, L->off_bias,
@@ -673,12 +673,12 @@ int forward_dev(csk_moe_layer* L, const float* d_hidden, int64_t T, const float*
   L->last = csk_moe_timings{};
   L->last_T = T;
   if (!L->carry_active) L->counts_in_carry = false;
-  // small batches are launch-bound: let each kernel become resident while its predecessor drains
+  // each kernel may become resident while its predecessor drains
   struct PdlScope {
     csk_moe_layer* l;
     ~PdlScope() { l->pdl = false; }
   } pdl_scope{L};
-  L->pdl = T <= 512 && !L->timing;
+  L->pdl = !L->timing;
   StageTimer tm(L, s);
   tm.mark();
   const float* router = d_router_in;
