@@ -138,24 +138,9 @@ __device__ __forceinline__ bool mbar_test(uint32_t bar, uint32_t parity) {
       : "memory");
   return ok != 0;
 }
-// Bounded wait.  Returns false (and raises the CTA's abort flag) when the clock
-// budget ran out or another role already aborted.
-__device__ __forceinline__ bool mbar_wait_here(uint32_t bar, uint32_t parity, volatile int* abort_flag) {
-  if (mbar_try(bar, parity)) return true;
-  const long long t0 = clock64();
-  for (;;) {
-    if (*abort_flag) return false;
-    for (int i = 0; i < 32; ++i)
-      if (mbar_try(bar, parity)) return true;
-    if (clock64() - t0 > wait_budget()) {
-      *abort_flag = 1;
-      return false;
-    }
-  }
-}
-// The same with all but the first test in one function that every wait of a kernel shares: kernels of many roles and waits
-// have the less code to fetch (k_tile2 on 2048 tokens of the 128-expert 2048 x 768 layer 97 -> 93 us, k_mx on 16 tokens of
-// it 81 -> 79 for the step), while k_tile, with few waits, loses by it (228 -> 235 us on 8192 tokens) and polls in place.
+// Bounded wait.  Returns false (and raises the CTA's abort flag) when the clock budget ran out or another role already aborted.  All but
+// the first test is in one function that every wait of a kernel shares: kernels of many roles and waits have the less code to fetch
+// (k_tile2 on 2048 tokens of the 128-expert 2048 x 768 layer 97 -> 93 us, k_mx on 16 tokens of it 81 -> 79 for the step).
 template <bool CLUSTER = false>
 static __device__ __noinline__ bool mbar_wait_more(uint32_t bar, uint32_t parity, volatile int* abort_flag) {
   const long long t0 = clock64();

@@ -1,7 +1,7 @@
 // Grouped contraction over fp16 weights for FEW token rows (the dense FFN and fp16 experts in decode), written for sm_100a.
 //
-// Every weight is read once and meets at most 64 token rows, so its bytes count.  k_tile gives a CTA 256 weight rows and all of K,
-// which leaves most SMs without work (a 2880 x 2880 matrix is 23 items) and each of the others with one stream.  Here a block
+// Every weight is read once and meets at most 32 token rows, so its bytes count.  k_pair16 gives a CTA pair 256 weight rows and all of
+// K, which leaves most SMs without work (a 2880 x 2880 matrix is 23 items) and each of the others with one stream.  Here a block
 // of eight warps has 16 weight rows (gate/up: 16 gate and the same features' 16 up rows); its warps take the k-tiles in turn
 // and their sums are added in warp order at the end, so a matrix is some hundred blocks that are all resident at once.
 //
@@ -20,7 +20,7 @@
 namespace csk {
 
 constexpr int kFewWarps = 8;
-constexpr int kFewMaxRows = 64;        // tokens of a batch: the layer holds one expert ...
+constexpr int kFewMaxRows = 32;        // tokens of a batch: the layer holds one expert ...
 constexpr int kFewMaxRowsRouted = 16;  // ... or several
 
 inline size_t few_smem_bytes(int groups, bool gated) { return (size_t)kFewWarps * 32 * 4 * groups * (gated ? 2 : 1) * sizeof(float); }
@@ -41,9 +41,9 @@ struct FewArgs {
 // NT = groups of eight token rows.  blockIdx.x: 16 weight rows (features), blockIdx.y: row tile.  TURNS: the tile may have more
 // than 8 NT rows, which are taken 8 NT after another (the loop's registers cost the others up to 5 %: 128 experts of 2048 x 768, 16
 // tokens of eight slots 224 -> 236 us).
-// Two blocks an SM up to 32 rows (in 128 registers; three blocks of 80 were slower, 62 -> 70 us for a block of 5 tokens).
+// Two blocks an SM (in 128 registers; three blocks of 80 were slower, 62 -> 70 us for a block of 5 tokens).
 template <bool GATED, int NT, bool TURNS>
-__global__ void __launch_bounds__(kFewWarps * 32, NT <= 4 ? 2 : 1) k_few16(const FewArgs F) {
+__global__ void __launch_bounds__(kFewWarps * 32, 2) k_few16(const FewArgs F) {
   extern __shared__ float few_sums[];
   const TileArgs& A = F.t;
   const TileLayout& L = A.L;
@@ -53,8 +53,9 @@ __global__ void __launch_bounds__(kFewWarps * 32, NT <= 4 ? 2 : 1) k_few16(const
   // (the tile list is two launches old, unless there is one expert only)
   const int expert = !F.one_expert && (int)blockIdx.y < *A.n_tiles_ptr ? A.tiles[blockIdx.y].expert : 0;
   const uint8_t* ebase = A.weights + (size_t)expert * A.expert_stride;
-  // row g of the block's 16 in the tile layout (gate/up: half 0 gate, half 1 up), its pieces stored at piece ^ (row & 7)
-  const int nt = n0 / L.feats_per_tile(), in_tile = n0 % L.feats_per_tile(), half = in_tile / kTileW, r0 = in_tile % kTileW;
+  // row g of the block's 16 in the tile layout (gate/up: the up rows 16 rows behind), its pieces stored at piece ^ (row & 7)
+  constexpr int kUp = 16 * 128;
+  const int nt = n0 / L.feats_per_tile(), half = L.half_of(n0), r0 = L.row_of(n0 % L.feats_per_tile(), 0);
   const uint8_t* wt = ebase + A.mat_offset + (size_t)nt * L.k_tiles * kTile16 + (size_t)half * kHalf16 + (size_t)(r0 + g) * 128;
   const int p0 = (q ^ g) << 4, p1 = ((q + 4) ^ g) << 4;  // (row & 7 = g for rows g and g + 8)
   uint4 w[2][M][2][2];  // [buffer][matrix][row g, g + 8][piece q, q + 4]
@@ -64,8 +65,8 @@ __global__ void __launch_bounds__(kFewWarps * 32, NT <= 4 ? 2 : 1) k_few16(const
     for (int m = 0; m < M; ++m)
 #pragma unroll
       for (int h = 0; h < 2; ++h) {
-        d[m][h][0] = __ldg(reinterpret_cast<const uint4*>(base + m * kHalf16 + h * 1024 + p0));
-        d[m][h][1] = __ldg(reinterpret_cast<const uint4*>(base + m * kHalf16 + h * 1024 + p1));
+        d[m][h][0] = __ldg(reinterpret_cast<const uint4*>(base + m * kUp + h * 1024 + p0));
+        d[m][h][1] = __ldg(reinterpret_cast<const uint4*>(base + m * kUp + h * 1024 + p1));
       }
   };
   if (warp < L.k_tiles) load_w(warp, w[0]);
@@ -134,7 +135,9 @@ __global__ void __launch_bounds__(kFewWarps * 32, NT <= 4 ? 2 : 1) k_few16(const
         const float gate = s[0] + (A.has_bias ? bias[A.F + n] : 0.f), up = s[M - 1] + (A.has_bias ? bias[n] : 0.f);
         A.a_out[(size_t)(rt.row0 + token) * A.lda + n] = __float2half_rn(gated_act_fast(gate, up, A.act));
       } else {
-        A.y_out[(size_t)(rt.row0 + token) * A.ldy + n] = s[0] + (A.has_bias ? bias[2 * A.F + n] : 0.f);
+        const int gr = rt.row0 + token;
+        float* out = A.out_row_ptr ? A.out_row_ptr[gr] : A.y_out + (size_t)(A.out_row_map ? A.out_row_map[gr] : gr) * A.ldy;
+        if (out) out[n] = s[0] + (A.has_bias ? bias[2 * A.F + n] : 0.f);
       }
     }
     rt.row0 += 8 * NT;
@@ -144,18 +147,18 @@ __global__ void __launch_bounds__(kFewWarps * 32, NT <= 4 ? 2 : 1) k_few16(const
     if (warp < L.k_tiles) load_w(warp, w[0]);
     if (warp + kFewWarps < L.k_tiles) load_w(warp + kFewWarps, w[1]);
   }
+  if (!GATED && A.out_row_ptr) __threadfence_system();  // rows written to other GPUs before the kernel is seen as done
 }
 
 template <bool GATED, bool TURNS>
 inline cudaError_t few_launch_turns(const FewArgs& f, int features, int tiles, int rows, cudaStream_t s, bool pdl) {
-  const int groups = rows <= 8 ? 1 : rows <= 16 ? 2 : rows <= 32 ? 4 : 8;
+  const int groups = rows <= 8 ? 1 : rows <= 16 ? 2 : 4;
   const dim3 grid((unsigned)(features / 16), (unsigned)tiles), block(kFewWarps * 32);
   const size_t smem = few_smem_bytes(groups, GATED);
   switch (groups) {
     case 1: return launch_k(k_few16<GATED, 1, TURNS>, grid, block, smem, s, pdl, f);
     case 2: return launch_k(k_few16<GATED, 2, TURNS>, grid, block, smem, s, pdl, f);
-    case 4: return launch_k(k_few16<GATED, 4, TURNS>, grid, block, smem, s, pdl, f);
-    default: return launch_k(k_few16<GATED, 8, TURNS>, grid, block, smem, s, pdl, f);
+    default: return launch_k(k_few16<GATED, 4, TURNS>, grid, block, smem, s, pdl, f);
   }
 }
 
@@ -164,12 +167,6 @@ template <bool GATED>
 inline cudaError_t few_launch_one(const FewArgs& f, int features, int tiles, int rows, bool repeats, cudaStream_t s, bool pdl) {
   return repeats ? few_launch_turns<GATED, true>(f, features, tiles, rows, s, pdl)
                  : few_launch_turns<GATED, false>(f, features, tiles, rows, s, pdl);
-}
-
-inline cudaError_t few_prepare_device() {
-  const cudaError_t e = cudaFuncSetAttribute(k_few16<true, 8, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)few_smem_bytes(8, true));
-  if (e != cudaSuccess) return e;
-  return cudaFuncSetAttribute(k_few16<true, 8, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)few_smem_bytes(8, true));
 }
 
 }  // namespace csk

@@ -18,6 +18,7 @@
 #include "csk_router_tc.cuh"
 #include "csk_tile.cuh"
 #include "csk_tile2.cuh"
+#include "csk_pair16.cuh"
 
 using namespace csk;
 
@@ -176,9 +177,9 @@ int fail(csk_moe_layer* L, int code, const char* fmt, ...) {
                   __FILE__, __LINE__);                                                       \
   } while (0)
 
-// Bytes of an expert's tensor-core codes in the order of the file images (fp16 weights are in that order on the device, too).  The
-// first staging area holds them, so that images can be written and read when the device is full.
-size_t image_part_bytes(const csk_moe_layer* L) { return L->w16 ? 0 : L->off_bias - L->off_tgu; }
+// Bytes of an expert's tensor-core tiles in the order of the file images.  The first staging area holds them, so that images can be
+// written and read when the device is full.
+size_t image_part_bytes(const csk_moe_layer* L) { return L->off_bias - L->off_tgu; }
 
 int grid_for(size_t work_items, int threads, int cap) {
   size_t b = (work_items + threads - 1) / threads;
@@ -534,12 +535,7 @@ int choose_path_received(const csk_moe_layer* L, int64_t rows, int64_t most) {
   return path == CSK_PATH_STREAM && L->mx_rows < most ? CSK_PATH_TILE : path;
 }
 
-// MXFP4 runs on CTA pairs, fp16 weights on the one-CTA kernel
-bool use_pairs(const csk_moe_layer* L) { return !L->w16; }
-
-int tile_rows_for(const csk_moe_layer* L, int path) {
-  return path == CSK_PATH_TILE ? (use_pairs(L) ? kPairN : kTileM) : kMxTileRows;
-}
+int tile_rows_for(int path) { return path == CSK_PATH_TILE ? kPairN : kMxTileRows; }
 
 // What is known of the tokens whose rows are listed (nothing of rows received from peers).
 struct Batch {
@@ -549,19 +545,22 @@ struct Batch {
 };
 
 // fp16 weights: the kernel for few rows (csk_few16.cuh) takes a batch of so many tokens.  The weights' bytes are all that counts
-// there.  Step, k_tile / k_few16, us: dense FFN of 2880 x 2880 (weights in L2) 1 token 41 / 15, 16 43 / 17, 32 45 / 25, 48 48 / 39, 64
-// 51 / 41; 16 experts of 2048 x 2048 beside a shared one 1 token 72 / 39, 5 85 / 62, 16 114 / 103, 32 120 / 145.
-// Of several experts its time goes by those that are hit, k_tile's by the rounds of their items (128 features of an expert) on
-// the SMs.  The line is 1.4 items per SM, for evenly spread routing: 2048 x 2048, 16 experts, top-1, 16 tokens (165 items) 88 / 85,
-// top-2 12 (202) 93 / 92, 16 (224) 95 / 100, top-4 16 (252) 99 / 108; 128 of 2048 x 768, top-8, 2 (91) 63 / 62, 4 (170) 92 / 93, 8 (303)
-// 123 / 147, 16 (487) 164 / 232; 64 of 512 x 512, top-8, 4 (101) 38 / 34, 16 (222) 40 / 47; 32 of 2880 x 2880, top-4, 3 (233) 123 / 130, 8
-// (470) 213 / 234; 12 of 2880 x 2880, top-2, 8 (207) 123 / 120, 16 (259) 130 / 142; 8 of 2048 x 2048, top-2, 16 (126) 74 / 71.
+// there.  Step, k_pair16 / k_few16, us: dense FFN of 2880 x 2880 (weights in L2) 1 token 26.8 / 14.4, 16 27.8 / 16.5, 32 28.4 / 24.7, 48 28.8 /
+// 40.1; 2048 x 8192 16 43.4 / 29.3, 24 44.7 / 43.7, 32 45.0 / 46.9; 512 x 512 32 12.5 / 10.4.
+// Of several experts its time goes by the row tiles, most of which hold a row or two, k_pair16's by the rounds of its items (128
+// features of an expert) on the SMs.  The line is half an item per SM, for evenly spread routing (in brackets): 16 of 2048 x 2048, top-1, 1 token
+// (0.11) 36.0 / 25.6, 5 (0.47) 51.3 / 51.3, 16 (1.1) 70.8 / 81.5; top-2, 1 (0.22) 37.0 / 28.3, 4 (0.70) 55.2 / 61.7; top-4, 1 (0.39) 42.0 / 41.6;
+// 2 of 2880 x 2880, 1 (0.16) 40.7 / 26.9, 8 (0.31) 47.6 / 43.3; 4, top-2, 1 (0.27) 45.2 / 44.7; 128 of 2048 x 768, top-8, 1 (0.32) 39.0 / 43.1, 2 (0.61)
+// 53.5 / 58.6; 64 of 512 x 512, top-8, 1 (0.21) 25.8 / 21.0, 4 (0.69) 32.2 / 35.0; beside a shared expert 16 of 2048 x 2048, top-1, 5 tokens 60.4 / 59.2.  And 24 MB of
+// weights, where launches and latencies are what is left: 64 of 256 x 512, top-8, 2 (0.37, 11 MB) 22.7 / 20.6, 4 (0.68, 20 MB) 24.2 / 24.7, 8 (1.1, 32 MB)
+// 24.8 / 30.9.
 bool few_rows(const csk_moe_layer* L, const Batch& b) {
+  if (!L->pair.available) return true;  // (in turns of a tile's rows: fp16 layers have no other kernel then)
   if (L->Eloc == 1) return b.tokens <= kFewMaxRows;
   if (b.tokens > kFewMaxRowsRouted) return false;
   if (b.one_expert) return true;
   const double hit = L->Eloc * (1.0 - std::pow(1.0 - 1.0 / L->E, (double)(b.tokens * L->k)));
-  return hit * L->Tgu.n_tiles <= 1.4 * L->sm_count;
+  return hit * L->Tgu.n_tiles <= 0.5 * L->sm_count || hit * (3.0 * sizeof(__half) * L->H * L->F) <= 24e6;
 }
 
 // grouped gate/up + activation + down over the row tiles listed in d_tiles; the grouped rows are in d_x16 (tensor-core
@@ -587,9 +586,14 @@ int launch_experts(csk_moe_layer* L, int path, float* y, int ldy, const int* out
     a.a_out = L->d_a16;
     a.lda = L->lda;
     // (where a token's slots may all name one expert, its rows may need several tiles)
-    const int64_t pairs = batch.tokens * L->k;
-    const int tiles = (int)std::min(pairs, batch.repeats ? L->Eloc + pairs / kTileM : (int64_t)L->Eloc);
-    CSK_CUDA(L, few_launch_one<true>(f, L->F, tiles, (int)batch.tokens, batch.repeats, s, L->pdl));
+    const int64_t pairs = std::min(L->max_rows, batch.tokens < L->max_rows ? batch.tokens * L->k : L->max_rows);
+    const bool turns = batch.repeats || batch.tokens > (L->Eloc == 1 ? kFewMaxRows : kFewMaxRowsRouted);
+    const int64_t tiles = std::min(pairs, turns ? L->Eloc + pairs / kPairN : (int64_t)L->Eloc);
+    if (tiles > 65535) return fail(L, CSK_ERR_NOMEM, "more row tiles than a launch takes");
+    const int rows = (int)std::min<int64_t>(batch.tokens, kFewMaxRows);
+    a.out_row_map = out_row_map;
+    a.out_row_ptr = out_row_ptr;
+    CSK_CUDA(L, few_launch_one<true>(f, L->F, (int)tiles, rows, turns, s, L->pdl));
     tm.mark();
     f.x = L->d_a16;
     f.ldx = L->lda;
@@ -597,20 +601,14 @@ int launch_experts(csk_moe_layer* L, int path, float* y, int ldy, const int* out
     a.L = L->Td;
     a.y_out = y;
     a.ldy = ldy;
-    CSK_CUDA(L, few_launch_one<false>(f, L->H, tiles, (int)batch.tokens, batch.repeats, s, L->pdl));
+    CSK_CUDA(L, few_launch_one<false>(f, L->H, (int)tiles, rows, turns, s, L->pdl));
     tm.mark();
     L->last.launches += 2;
   } else if (path == CSK_PATH_TILE) {
-    int rc;
-    if (use_pairs(L))
-      rc = pair_launch(L->pair, L->tile, L->tile.pair_x, L->tile.pair_a, L->d_weights, L->expert_stride, L->off_tgu,
+    const int rc =
+        pair_launch(L->pair, L->tile, L->tile.pair_x, L->tile.pair_a, L->d_weights, L->expert_stride, L->off_tgu,
                        L->off_td, L->off_bias, L->off_meta, L->Tgu, L->Td, L->d_a16, L->lda, y, ldy, out_row_map,
                        out_row_ptr, L->d_tiles, L->d_meta, L->cfg.has_bias, L->cfg.activation, L->F, s, L->pdl,
-                       [&]() { tm.mark(); }, L->debug_stall);
-    else
-      rc = tile_launch(L->tile, L->d_weights, L->expert_stride, L->off_tgu, L->off_td, L->off_bias,
-                       L->off_meta, L->Tgu, L->Td, L->d_a16, L->lda, y, ldy, out_row_map, out_row_ptr, L->d_tiles,
-                       L->d_meta, L->cfg.has_bias, L->cfg.activation, L->F, L->sm_count, s,
                        [&]() { tm.mark(); }, L->debug_stall);
     L->debug_stall = false;
     if (rc) return fail(L, rc, "tensor-core path: %s", L->tile.err.c_str());
@@ -696,7 +694,7 @@ int forward_dev(csk_moe_layer* L, const float* d_hidden, int64_t T, const float*
   }
   const int64_t rows = only_expert >= 0 ? T : T * L->k;
   const int path = choose_path(L, only_expert >= 0 ? rows * std::max(1, L->Eloc) : rows);
-  const int tile_rows = tile_rows_for(L, path);
+  const int tile_rows = tile_rows_for(path);
   if (reinterpret_cast<uintptr_t>(d_hidden) % 16) return fail(L, CSK_ERR_INVALID, "hidden states must be 16-byte aligned");
   const bool mx = path == CSK_PATH_STREAM;
   if (router == L->d_unit_router && router && !mx && only_expert < 0 && !d_router_out && !d_residual && !d_shared && !L->carry_active) {
@@ -901,7 +899,7 @@ int csk_moe_create(const csk_moe_config* cfg, csk_moe_layer** out) {
   CK(cudaMalloc(&L->d_p2p_base, sizeof(int) * L->E));
   L->E_router = L->E;
   CK(cudaMalloc(&L->d_out, sizeof(float) * L->max_T * L->H));
-  const size_t pad_rows = std::max(kTileM, kPairN);  // a row tile's loads may reach this far past the last row
+  const size_t pad_rows = kPairN;  // a row tile's loads may reach this far past the last row
   CK(cudaMalloc(&L->d_x16, sizeof(__half) * (L->max_rows + pad_rows) * L->ldx));
   CK(cudaMemset(L->d_x16, 0, sizeof(__half) * (L->max_rows + pad_rows) * L->ldx));
   CK(cudaMalloc(&L->d_a16, sizeof(__half) * (L->max_rows + pad_rows) * L->lda));
@@ -925,11 +923,12 @@ int csk_moe_create(const csk_moe_config* cfg, csk_moe_layer** out) {
   CK(router_prepare_device());
   for (int g = 1; g <= kMaxExperts / 32; ++g) L->router_waves[g] = router_wave(g, L->sm_count);
   CK(mx_prepare_device());
-  CK(few_prepare_device());
   CK(rt_prepare_device());
   {
     int rc = tile_init(L->tile, cfg->device);
-    if (!rc) rc = tile_set_buffers(L->tile, L->d_x16, L->ldx, L->d_a16, L->lda, (size_t)L->max_rows + pad_rows);
+    if (!rc)
+      rc = tile_set_buffers(L->tile, L->d_x16, L->ldx, L->d_a16, L->lda, (size_t)L->max_rows + pad_rows, L->w16 ? L->d_weights : nullptr,
+                            L->expert_stride * L->Eloc);
     if (!rc) rc = pair_init(L->pair, L->tile, L->sm_count);
     if (rc) {
       rc = fail(nullptr, rc, "tensor-core path setup: %s", L->tile.err.c_str());
@@ -1306,7 +1305,7 @@ int reorder_tiles_enqueue(csk_moe_layer* L, int le, bool to_file, cudaStream_t s
   uint8_t* base = L->d_weights + (size_t)le * L->expert_stride + L->off_tgu;
   uint8_t* part = L->d_stage;
   for (const auto& [lay, at] : {std::pair{L->Tgu, (size_t)0}, std::pair{L->Td, L->off_td - L->off_tgu}})
-    k_reorder_tile<<<grid_for(lay.bytes() / 34, 256, 4096), 256, 0, s>>>(to_file ? base + at : part + at, to_file ? part + at : base + at, lay,
+    k_reorder_tile<<<grid_for(lay.bytes() / (lay.w16 ? 128 : 34), 256, 4096), 256, 0, s>>>(to_file ? base + at : part + at, to_file ? part + at : base + at, lay,
                                                                        to_file);
   CSK_CUDA(L, cudaGetLastError());
   return CSK_OK;
@@ -1423,7 +1422,7 @@ int csk_moe_set_path(csk_moe_layer* L, int32_t path) {
   if (check_layer(L)) return CSK_ERR_INVALID;
   if (path < CSK_PATH_AUTO || path > CSK_PATH_TILE_PAIR) return fail(L, CSK_ERR_INVALID, "unknown path %d", path);
   if (L->w16 && (path == CSK_PATH_STREAM || path == CSK_PATH_TILE_PAIR))
-    return fail(L, CSK_ERR_INVALID, "fp16 weights have no weight-streaming and no CTA-pair kernel");
+    return fail(L, CSK_ERR_INVALID, "fp16 weights have no weight-streaming kernel, and their CTA-pair kernel is not chosen by name");
   if (path == CSK_PATH_TILE_PAIR && !L->pair.available)
     return fail(L, CSK_ERR_INVALID, "the CTA-pair kernel is not available on this device: %s", L->pair.err.c_str());
   CSK_CUDA(L, cudaSetDevice(L->cfg.device));
@@ -1730,7 +1729,7 @@ int host_passes(const csk_moe_layer* L, int64_t T, std::initializer_list<const v
   const int64_t rows = T * L->k / std::max(1, L->Eloc);  // per expert
   const int least = rows < 256 ? 1 : 2;
   if (rows < 128 || !page_locked(buffers)) return least;
-  const int tile_rows = tile_rows_for(L, CSK_PATH_TILE);
+  const int tile_rows = tile_rows_for(CSK_PATH_TILE);
   auto items = [&](int passes) { return (rows / passes + tile_rows - 1) / tile_rows * L->Eloc * L->Tgu.n_tiles; };
   int passes = (int)std::max<int64_t>(2, std::min<int64_t>(csk_moe_layer::kMaxPasses, rows / 120));
   while (passes > least && 3 * items(passes) < L->sm_count) --passes;
@@ -2178,7 +2177,7 @@ int csk_moe_ep_p2p_experts_dev(csk_moe_layer* L, const int32_t* d_all_counts, in
   cudaStream_t s = pick(L, stream);
   rows_hint = std::max<int64_t>(1, std::min<int64_t>(rows_hint, L->max_rows));
   const int path = choose_path_received(L, rows_hint, L->max_rows);  // (a hint is no bound)
-  const int tile_rows = tile_rows_for(L, path);
+  const int tile_rows = tile_rows_for(path);
   const bool mx = path == CSK_PATH_STREAM;
   // the status word of the dispatch stays; the tile list is rebuilt from the received counts
   k_ep_p2p_local_counts<<<(L->E + 255) / 256, 256, 0, s>>>(d_all_counts, L->p2p_world, L->E, L->e0, L->Eloc, L->d_counts);
@@ -2223,7 +2222,7 @@ int csk_moe_ep_experts_dev(csk_moe_layer* L, const void* d_recv_f16, const int32
   cudaStream_t s = pick(L, stream);
   if (total_rows == 0) return CSK_OK;
   const int path = choose_path_received(L, total_rows, total_rows);
-  const int tile_rows = tile_rows_for(L, path);
+  const int tile_rows = tile_rows_for(path);
   const bool mx = path == CSK_PATH_STREAM;
   CSK_CUDA(L, cudaMemsetAsync(L->d_meta, 0, sizeof(int) * 8, s));
   CSK_CUDA(L, cudaMemsetAsync(L->d_counts, 0, sizeof(int) * L->E, s));

@@ -64,8 +64,8 @@ enum {
  *                      tensor-core kernel on CTA pairs.
  *   CSK_WEIGHTS_F16    fp16 row-major matrices (csk_moe_load_expert_f16): the reference's fp16 expert
  *                      slices (expert_mlp_node.h:533-647) and, with num_experts = top_k = 1, its dense
- *                      shared-expert FFN (dense_ffn_node.h:28-219).  The one-CTA tensor-core kernel and, for few
- *                      token rows, a kernel of its own. */
+ *                      shared-expert FFN (dense_ffn_node.h:28-219).  A tensor-core kernel on CTA pairs of
+ *                      their own and, for few token rows, another. */
 enum { CSK_WEIGHTS_MXFP4 = 0, CSK_WEIGHTS_F16 = 1 };
 
 typedef struct csk_moe_config {
