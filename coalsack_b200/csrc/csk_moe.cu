@@ -114,6 +114,8 @@ struct csk_moe_layer {
   int* d_meta = nullptr;  // 16 ints: [0..7] rewritten by every permutation, [8] the router's status word
   int* h_meta = nullptr;  // pinned mirror
   int64_t* h_counts64 = nullptr;
+  float* h_staged = nullptr;       // page-locked staging of small host batches: h_staged_bytes in, as many out
+  size_t h_staged_bytes = 0;
 
   cudaStream_t stream = nullptr;
   // the host entry point's pipeline: copy-in and copy-out streams beside `stream`, one event pair per pass
@@ -151,6 +153,10 @@ struct csk_moe_layer {
 };
 
 namespace {
+
+// Host buffers of at most so many bytes each way go through page-locked staging of the handle's own.  32 tokens of
+// the 32-expert layer, pageable: 200 -> 191 us a call (copies of pageable memory wait for the device, and the status had a wait of its own).
+constexpr size_t kStagedMax = 1 << 20;
 
 int wide_stride(const csk_moe_layer* L) { return mx_mask_words(L->Lgu.recs) + mx_mask_words(L->Ld.recs); }
 
@@ -920,6 +926,8 @@ int csk_moe_create(const csk_moe_config* cfg, csk_moe_layer** out) {
   CK(cudaMemset(L->d_meta, 0, sizeof(int) * 16));
   CK(cudaMallocHost(&L->h_meta, sizeof(int) * 16));
   CK(cudaMallocHost(&L->h_counts64, sizeof(int64_t) * L->E));
+  L->h_staged_bytes = std::min<size_t>(kStagedMax, sizeof(float) * L->max_T * (L->H + 2 * L->k));
+  CK(cudaMallocHost(&L->h_staged, 2 * L->h_staged_bytes));
   CK(router_prepare_device());
   for (int g = 1; g <= kMaxExperts / 32; ++g) L->router_waves[g] = router_wave(g, L->sm_count);
   CK(mx_prepare_device());
@@ -964,6 +972,7 @@ int csk_moe_destroy(csk_moe_layer* L) {
   for (uint8_t* p : L->mx_outgrown) cudaFree(p);
   if (L->h_meta) cudaFreeHost(L->h_meta);
   if (L->h_counts64) cudaFreeHost(L->h_counts64);
+  if (L->h_staged) cudaFreeHost(L->h_staged);
   for (auto& e : L->ev)
     if (e) cudaEventDestroy(e);
   for (auto& e : L->ev_in)
@@ -1710,28 +1719,29 @@ bool page_locked(std::initializer_list<const void*> buffers) {
 }
 
 // How many equal passes the host entry point cuts a batch into so that the copies of one pass overlap the kernels of another.
-// Pageable buffers: two from 256 rows per expert on.  Their copies block the caller, so a pass is enqueued only when the one before
-// it has been copied out.  1 / 2 / 4 / 8 passes, ms: 128 experts of 2880 x 2880, 4096 tokens (128 rows per expert) 6.49 / 7.31 /
-// 9.62 / 11.0, 8192 (256) 18.1 / 16.8 / 16.5 / 18.5; 32 experts, 1500 (187) 2.29 / 2.51 / 3.05 / 3.78, 3000 (375) 4.82 / 4.76 / 5.22 / 6.28, 8192
-// (1024) 15.5 / 15.6 / 16.7 / 16.9; 8 of 1728 x 1728, top-2, 2000 (500) 1.58 / 1.69 / 1.89 / 2.31; fp16, 32 of 2880 x 2880, 4096 (512) 8.33 / 8.77
-// / 8.85 / 10.3.
-// Page-locked buffers: two from 128 rows per expert on, one more for every 120.  What stays exposed is the first copy in and the last
-// copy out; what passes cost is kernel time, the less the more rows an expert has (a row tile's cost is nearly flat below 100 rows).
-// 1 / 2 / 3 / 4 / 8 passes, ms: 128 experts of 2880 x 2880, 4096 tokens 2.59 / 2.27 / - / 2.73 / 3.22, 8192 4.97 / 3.58 / 3.64 / 3.67 / 5.12;
-// 32 experts, 1500 0.97 / 0.84 / - / 1.01 / 1.29, 3000 1.84 / 1.32 / 1.26 / 1.34 / 1.82, 8192 4.82 / 3.40 / 3.03 / 2.75 / 2.57; fp16, 32
-// experts, 1500 1.20 / 1.11 / 1.26 / 1.50 / 2.59, 8192 5.41 / 3.84 / 3.57 / 3.56 / 3.77.  But no more than leave a pass items (a row
+// Pageable buffers: two from 600 rows per expert on.  Their copies block the caller, so a pass is enqueued only when the one before
+// it has been copied out.  1 / 2 / 4 / 8 passes, ms: 128 experts of 2880 x 2880, 4096 tokens (128 rows per expert) 7.57 / 7.59 / 7.91 / 8.99, 8192
+// (256) 14.7 / 15.4 / 15.9 / 18.0; 32 experts, 2048 (256) 2.92 / 3.12 / 3.67 / 4.56, 3000 (375) 4.46 / 4.41 / 5.09 / 5.95, 8192 (1024) 13.5 / 13.4 /
+// 15.2 / 15.3; 8 of 1728 x 1728, top-2, 2000 (500) 1.68 / 1.80 / 2.02 / 2.39; fp16, 32 of 2880 x 2880, 4096 (512) 6.10 / 6.32 / 6.88 / 8.35.
+// Page-locked buffers: two from 128 rows per expert on, three from 240, and one for every 120.  What stays exposed is the first copy in and
+// the last copy out; what passes cost is kernel time, the less the more rows an expert has (a row tile's cost is nearly flat below 100
+// rows).  1 / 2 / 3 / 4 / 8 passes, ms: 128 experts of 2880 x 2880, 4096 tokens 2.58 / 2.20 / 2.46 / 2.74 / 3.18, 8192 4.96 / 3.47 / 3.30 / 3.54 / 5.02;
+// 32 experts, 1500 (187) 0.95 / 0.77 / 0.82 / 0.93 / 1.29, 2048 1.29 / 0.90 / 0.93 / 1.01 / 1.48, 3000 1.80 / 1.30 / 1.14 / 1.18 / 1.66, 8192 4.76 / 3.39 /
+// 2.97 / 2.76 / 2.49; 128 of 2048 x 768, top-8, 4096 (256) 1.70 / 1.25 / 1.14 / 1.13 / 1.47; fp16, 16 of 2048 x 2048, 4096 (256) 1.42 / 1.15 / 1.09 / 1.10 /
+// 1.02; 32 of 2880 x 2880, 1500 1.03 / 1.01 / 1.16 / 1.39 / 2.44, 8192 4.98 / 3.47 / 3.02 / 2.80 / 3.14.  But no more than leave a pass items (a row
 // tile x 128 features) for a third of the SMs: below, its kernels take as long as the whole batch's (one fp16 expert of 2880 x 2880, 150
-// tokens 0.19 / 0.23 / 0.25 / 0.30 / 0.43, 1024 0.59 / 0.49 / 0.52 / 0.56 / 0.80).
+// tokens 0.15 / 0.16 / 0.20 / 0.24 / 0.37, 1024 0.56 / 0.46 / 0.42 / 0.43 / 0.50).
 // (Shorter first and last passes were up to 5 % quicker still, but the certified router adds a token's parts in an order that goes
 // by the pass's size: the low bits of its weights would depend on where in the batch it stands.)
 int host_passes(const csk_moe_layer* L, int64_t T, std::initializer_list<const void*> buffers) {
   if (L->timing || L->path == CSK_PATH_STREAM) return 1;
   const int64_t rows = T * L->k / std::max(1, L->Eloc);  // per expert
+  if (rows < 128) return 1;
+  if (!page_locked(buffers)) return rows < 600 ? 1 : 2;
   const int least = rows < 256 ? 1 : 2;
-  if (rows < 128 || !page_locked(buffers)) return least;
   const int tile_rows = tile_rows_for(CSK_PATH_TILE);
   auto items = [&](int passes) { return (rows / passes + tile_rows - 1) / tile_rows * L->Eloc * L->Tgu.n_tiles; };
-  int passes = (int)std::max<int64_t>(2, std::min<int64_t>(csk_moe_layer::kMaxPasses, rows / 120));
+  int passes = (int)std::max<int64_t>(rows < 240 ? 2 : 3, std::min<int64_t>(csk_moe_layer::kMaxPasses, rows / 120));
   while (passes > least && 3 * items(passes) < L->sm_count) --passes;
   return passes;
 }
@@ -1745,6 +1755,35 @@ int csk_moe_forward(csk_moe_layer* L, const float* hidden, int64_t T, const floa
   CSK_CUDA(L, cudaSetDevice(L->cfg.device));
   cudaStream_t s = L->stream;
   const int passes = host_passes(L, T, {hidden, router_in, router_out, out});
+  const size_t row_bytes = sizeof(float) * T * L->H, route_bytes = sizeof(float) * T * L->k * 2;
+  if (passes == 1 && row_bytes + route_bytes <= L->h_staged_bytes) {
+    // A small batch goes through page-locked staging, in two pieces on the way in, and its status word comes back with its results:
+    // one wait a call, and no copy that the driver has to stage itself.
+    const int64_t half = T / 2 * L->H;
+    for (const auto& [at, n] : {std::pair{(int64_t)0, half}, std::pair{half, T * L->H - half}}) {
+      if (!n) continue;
+      memcpy(L->h_staged + at, hidden + at, sizeof(float) * n);
+      CSK_CUDA(L, cudaMemcpyAsync(L->d_hidden + at, L->h_staged + at, sizeof(float) * n, cudaMemcpyHostToDevice, s));
+    }
+    float *staged_out = L->h_staged + L->h_staged_bytes / sizeof(float), *staged_route = staged_out + T * L->H;
+    if (router_in) {
+      memcpy(L->h_staged + T * L->H, router_in, route_bytes);
+      CSK_CUDA(L, cudaMemcpyAsync(L->d_router, L->h_staged + T * L->H, route_bytes, cudaMemcpyHostToDevice, s));
+    }
+    int rc = csk_moe_forward_dev(L, L->d_hidden, T, router_in ? L->d_router : nullptr, nullptr, L->d_out, s);
+    if (rc) {
+      cudaStreamSynchronize(s);  // the copies in have left the staging area
+      return rc;
+    }
+    CSK_CUDA(L, cudaMemcpyAsync(staged_out, L->d_out, row_bytes, cudaMemcpyDeviceToHost, s));
+    if (router_out) CSK_CUDA(L, cudaMemcpyAsync(staged_route, L->d_router, route_bytes, cudaMemcpyDeviceToHost, s));
+    rc = check_device_status(L, s);
+    if (rc) return rc;
+    if (L->timing && L->n_marks > 1) finish_timings(L, L->n_marks, L->last_routed);
+    memcpy(out, staged_out, row_bytes);
+    if (router_out) memcpy(router_out, staged_route, route_bytes);
+    return CSK_OK;
+  }
   if (passes == 1) {
     CSK_CUDA(L, cudaMemcpyAsync(L->d_hidden, hidden, sizeof(float) * T * L->H, cudaMemcpyHostToDevice, s));
     if (router_in)
