@@ -905,7 +905,7 @@ int csk_moe_create(const csk_moe_config* cfg, csk_moe_layer** out) {
   CK(cudaMalloc(&L->d_p2p_base, sizeof(int) * L->E));
   L->E_router = L->E;
   CK(cudaMalloc(&L->d_out, sizeof(float) * L->max_T * L->H));
-  const size_t pad_rows = kPairN;  // a row tile's loads may reach this far past the last row
+  const size_t pad_rows = 32;  // a row tile's loads may reach this far past the last row (its MMAs' rows are a multiple of 32)
   CK(cudaMalloc(&L->d_x16, sizeof(__half) * (L->max_rows + pad_rows) * L->ldx));
   CK(cudaMemset(L->d_x16, 0, sizeof(__half) * (L->max_rows + pad_rows) * L->ldx));
   CK(cudaMalloc(&L->d_a16, sizeof(__half) * (L->max_rows + pad_rows) * L->lda));
