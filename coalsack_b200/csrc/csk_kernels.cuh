@@ -817,17 +817,38 @@ __global__ void __launch_bounds__(32 * kFinishWarps) k_router_finish_many(const 
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) h2 += __shfl_xor_sync(0xffffffffu, h2, o);
   const float hn = sqrtf(h2) * 1.001f + kNormFloor;
-  for (int e = lane; e < E; e += 32) {
-    float P = 0.f, sr = 0.f;
-    for (int m = 0; m < parts; ++m) {
-      const float2 v = __ldcg(A.part + ((size_t)t * parts + m) * E + e);
-      const int blocks = A.slices * (m + 1) / parts - A.slices * m / parts;
-      sr += (float)blocks * fabsf(P) + v.y;
-      P += v.x;
+  // four experts of a lane at a time, their loads in flight together (one after the other: 8192 tokens of 128 experts 24 us, now 15)
+  constexpr int N = 4;
+  for (int e0 = lane; e0 < E; e0 += 32 * N) {
+    float P[N], sr[N], bias[N], wn[N];
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+      const int e = e0 + 32 * i;
+      P[i] = sr[i] = 0.f;
+      bias[i] = A.bias && e < E ? A.bias[e] : 0.f;
+      wn[i] = e < E ? A.wnorm[e] : 0.f;
     }
-    const float logit = __fadd_rn(P, A.bias ? A.bias[e] : 0.f);
-    s_logit[e] = logit;
-    s_bound[e] = 6.3e-8f * (A.coef_prefix * sr + A.coef_norm * hn * A.wnorm[e]) + 2.4e-7f * fabsf(logit) + 1e-30f;
+    for (int m = 0; m < parts; ++m) {
+      float2 v[N];
+#pragma unroll
+      for (int i = 0; i < N; ++i)
+        if (e0 + 32 * i < E) v[i] = __ldcg(A.part + ((size_t)t * parts + m) * E + e0 + 32 * i);
+      const float blocks = (float)(A.slices * (m + 1) / parts - A.slices * m / parts);
+#pragma unroll
+      for (int i = 0; i < N; ++i) {
+        if (e0 + 32 * i >= E) continue;
+        sr[i] += blocks * fabsf(P[i]) + v[i].y;
+        P[i] += v[i].x;
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+      const int e = e0 + 32 * i;
+      if (e >= E) continue;
+      const float logit = __fadd_rn(P[i], bias[i]);
+      s_logit[e] = logit;
+      s_bound[e] = 6.3e-8f * (A.coef_prefix * sr[i] + A.coef_norm * hn * wn[i]) + 2.4e-7f * fabsf(logit) + 1e-30f;
+    }
   }
   __syncwarp();
   const bool sure = warp_topk<false>(s_logit, E, A.k, A.sigmoid, A.router_out + (size_t)t * A.k * 2, s_bound);

@@ -41,3 +41,30 @@ def test_chain_at_the_edges_of_its_launches(gpu_lib, port, E, H, T, sigmoid):
     assert np.allclose(got[..., 1], want[..., 1], rtol=0, atol=6e-7)
     assert np.array_equal(lay.route(h), got)
     lay.close()
+
+
+@pytest.mark.parametrize("E,H,T", [(2, 128, 1), (64, 1024, 4), (300, 160, 3), (1024, 96, 2)])
+def test_a_handful_of_tokens_that_cannot_be_separated(gpu_lib, port, E, H, T):
+    """Gate rows in pairs that differ in a few low bits: the bounds cannot tell them apart, and the tokens of a batch this small
+    take the certified pass and then the chain.  (Tokens whose logits tie among the k + 1 best are left out.)"""
+    rng = np.random.default_rng(E)
+    k = min(4, E // 2)
+    base = (rng.standard_normal((E // 2, H)) * 0.05).astype(np.float32)
+    twin = base.copy()
+    move = rng.random(base.shape) < 0.1
+    twin[move] *= np.float32(1.0 + 2.0 ** -14)
+    Wg = np.ascontiguousarray(np.stack([base, twin], axis=1).reshape(E, H))
+    lay = MoeLayer(E, k, H, 32, has_bias=False, max_tokens=T)
+    lay.set_router(Wg, None)
+    seen = 0
+    for rep in range(8):
+        h = rng.standard_normal((T, H)).astype(np.float32)
+        got = lay.route(h)
+        want, logits = port.router_logits(h, Wg, None, k)
+        top = -np.sort(-logits, axis=1)[:, :k + 1]
+        clean = np.all(top[:, :-1] != top[:, 1:], axis=1)
+        seen += int(clean.sum())
+        assert np.array_equal(got[clean][..., 0], want[clean][..., 0])
+    routed, chained = lay.router_stats()
+    assert routed == 8 * T and chained >= T and seen >= T, (routed, chained, seen)
+    lay.close()
