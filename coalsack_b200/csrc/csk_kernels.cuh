@@ -977,6 +977,8 @@ __global__ void __launch_bounds__(1024) k_scan(const ScanArgs A) {
   const int e = threadIdx.x, lane = e & 31, warp = e >> 5, B = blockDim.x, E = A.E;
   if (e == 0) s_distinct = s_tallest = s_status = 0;
   s_count[e] = 0;
+  const bool local = e >= A.e_begin && e < A.e_begin + A.e_count;
+  const bool missing = local && A.resident && !A.resident[e - A.e_begin];  // (older than the kernel in front)
   __syncthreads();
   griddep_wait();
   griddep_launch();
@@ -1007,12 +1009,11 @@ __global__ void __launch_bounds__(1024) k_scan(const ScanArgs A) {
   }
   if (A.partial && e < A.n_partial && A.partial[(size_t)e * (E + 1) + E]) atomicOr(&s_status, kDevErrExpertRange);
   const int c = e < E ? s_count[e] : 0;
-  const bool local = e >= A.e_begin && e < A.e_begin + A.e_count;
   const int nt = local ? (c + A.tile_rows - 1) / A.tile_rows : 0;
   auto tile_height = [&](int cnt) { return even_tile_height(cnt, A.tile_rows, A.expert_tiles != nullptr); };
   if (c > 0) {
     atomicAdd(&s_distinct, 1);
-    if (local && A.resident && !A.resident[e - A.e_begin]) atomicOr(&s_status, kDevErrNotResident);
+    if (missing) atomicOr(&s_status, kDevErrNotResident);
   }
   // block-wide inclusive scans of (c, nt)
   int rc = c, rt = nt;
@@ -1201,6 +1202,11 @@ __global__ void __launch_bounds__(256) k_combine(const float* __restrict__ route
   __shared__ int s_row[kMaxTopK];
   __shared__ float s_w[kMaxTopK];
   const int t = blockIdx.x;
+  // (the routing and the rows' places are older than the kernel in front)
+  if (t < T && (int)threadIdx.x < k) {
+    s_row[threadIdx.x] = row_of_pair[(size_t)t * k + threadIdx.x];
+    s_w[threadIdx.x] = unweighted ? 1.f : router_out[((size_t)t * k + threadIdx.x) * 2 + 1];  // 1 * v is v
+  }
   griddep_wait();
   griddep_launch();
   if (carry && t == 0 && blockIdx.y == 0) {
@@ -1208,10 +1214,6 @@ __global__ void __launch_bounds__(256) k_combine(const float* __restrict__ route
     for (int e = threadIdx.x; e < E; e += blockDim.x) carry[1 + e] += counts[e];
   }
   if (t >= T) return;
-  if ((int)threadIdx.x < k) {
-    s_row[threadIdx.x] = row_of_pair[(size_t)t * k + threadIdx.x];
-    s_w[threadIdx.x] = unweighted ? 1.f : router_out[((size_t)t * k + threadIdx.x) * 2 + 1];  // 1 * v is v
-  }
   __syncthreads();
   for (int d = (blockIdx.y * blockDim.x + threadIdx.x) * 4; d < H; d += gridDim.y * blockDim.x * 4) {
     float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);

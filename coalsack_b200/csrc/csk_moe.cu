@@ -481,6 +481,7 @@ void launch_mx_pair(csk_moe_layer* L, float* y, int ldy, cudaStream_t s, StageTi
   a.bias_offset = L->off_bias;
   a.tiles = L->d_tiles;
   a.n_tiles_ptr = L->d_meta;
+  a.max_tiles = L->max_tiles;
   a.has_bias = L->cfg.has_bias;
   a.act = L->cfg.activation;
   a.F = L->F;
