@@ -73,7 +73,7 @@ struct csk_moe_layer {
   RowOrigin** d_peer_info = nullptr;  // [world]
   float** d_peer_back = nullptr;      // [world]
   std::vector<void*> ipc_opened;      // peer mappings to close
-  bool pdl = false;  // launch the layer's kernels with programmatic dependent launch (small batches)
+  bool pdl = false;  // launch the kernels with programmatic dependent launch (unless they are timed one by one)
   bool debug_stall = false;  // test hooks: the next expert (router) launch's copy role issues nothing (one shot)
   bool debug_stall_router = false;
 
