@@ -188,6 +188,10 @@ __device__ __forceinline__ uint32_t map_to_cta(uint32_t local_addr, uint32_t ran
 // successor start early.
 __device__ __forceinline__ void griddep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void griddep_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+// Bulk and tensor copies read global memory through the async proxy.  A kernel that is already running when its predecessor ends has
+// no kernel boundary in front of what that wrote with ordinary stores: the threads that issue such copies of it call this after
+// griddep_wait().
+__device__ __forceinline__ void fence_async_global() { asm volatile("fence.proxy.async.global;" ::: "memory"); }
 
 template <typename... P, typename... A>
 inline cudaError_t launch_k(void (*kern)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, bool pdl,

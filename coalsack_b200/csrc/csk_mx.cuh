@@ -545,7 +545,7 @@ __global__ void __launch_bounds__(kMxThreads, 1) k_mx(const MxArgs A) {
         const MxTileImage g = mx_tile_image<D>(tile, rt.row0, rt.rows, L.recs);
         for (; first < NS && first < L.recs; ++first) weights(rt, nt, g, first, first);
         griddep_wait();
-        asm volatile("fence.proxy.async.global;" ::: "memory");  // the images were written by ordinary stores
+        fence_async_global();  // the images were written by ordinary stores
         for (int rec = 0; rec < first; ++rec) rows(A.x_img, g, rec, rec);
       }
       int s = first == NS ? 0 : first, issued = first;
