@@ -1092,7 +1092,9 @@ __global__ void __launch_bounds__(1024) k_scan(const ScanArgs A) {
 // kernel before this one and are on their way while that ends; a row is read once and stored k times, 16 bytes a thread.
 // Bound by HBM (4 H bytes in, 2 k H out): 4096 tokens x 4 slots x 2880 columns, 141 MB, 19.5 us (a warp per pair,
 // eight bytes a lane: 38).
+// V: what a store moves, uint4, or uint2 where the rows (a caller's, who sends them) lie at a multiple of 8 bytes only.
 constexpr int kScatterThreads = 128, kScatterKept = 3;  // columns of a row in registers: 8 x 128 x 3
+template <typename V>
 __global__ void __launch_bounds__(kScatterThreads) k_scatter(const float* __restrict__ router_out, const float* __restrict__ hidden,
                                                              int k, int H, int E, int only_expert, const int* __restrict__ offsets,
                                                              int* __restrict__ cursor, int* __restrict__ row_of_pair,
@@ -1133,9 +1135,11 @@ __global__ void __launch_bounds__(kScatterThreads) k_scatter(const float* __rest
     for (int j = 0; j < k; ++j) {
       if (s_pos[j] < 0) continue;
       const float m = s_w[j];
-      const __half2 h[4] = {__floats2half2_rn(a.x * m, a.y * m), __floats2half2_rn(a.z * m, a.w * m),
-                            __floats2half2_rn(b.x * m, b.y * m), __floats2half2_rn(b.z * m, b.w * m)};
-      *reinterpret_cast<uint4*>(x16 + (size_t)s_pos[j] * ldx + d) = *reinterpret_cast<const uint4*>(h);
+      const __align__(16) __half2 h[4] = {__floats2half2_rn(a.x * m, a.y * m), __floats2half2_rn(a.z * m, a.w * m),
+                                          __floats2half2_rn(b.x * m, b.y * m), __floats2half2_rn(b.z * m, b.w * m)};
+#pragma unroll
+      for (int i = 0; i < (int)(16 / sizeof(V)); ++i)
+        reinterpret_cast<V*>(x16 + (size_t)s_pos[j] * ldx + d)[i] = reinterpret_cast<const V*>(h)[i];
     }
   };
 #pragma unroll

@@ -429,8 +429,9 @@ int launch_permute(csk_moe_layer* L, const float* d_hidden, const float* d_route
     a.recs = L->Lgu.recs;
     launch_k(k_mx_quant, dim3((unsigned)T), dim3(std::min(kMxQuantThreads, ceil_div(L->Lgu.blocks, 8) * 32)), 0, s, L->pdl, a);
   } else {
-    launch_k(k_scatter, dim3((unsigned)T), dim3(kScatterThreads), 0, s, L->pdl, d_router, d_hidden, L->k, L->H, L->E, only_expert, L->d_offsets,
-             one_block ? (int*)nullptr : L->d_cursor, L->d_row_of_pair, x16, ldx, (int)max_rows, L->cfg.weight_before_ffn);
+    launch_k(reinterpret_cast<uintptr_t>(x16) % 16 ? k_scatter<uint2> : k_scatter<uint4>, dim3((unsigned)T), dim3(kScatterThreads), 0, s, L->pdl,
+             d_router, d_hidden, L->k, L->H, L->E, only_expert, L->d_offsets, one_block ? (int*)nullptr : L->d_cursor, L->d_row_of_pair, x16, ldx,
+             (int)max_rows, L->cfg.weight_before_ffn);
   }
   CSK_CUDA(L, cudaGetLastError());
   L->last.launches += 1;
@@ -1939,6 +1940,8 @@ int csk_moe_ep_dispatch_dev(csk_moe_layer* L, const float* d_hidden, int64_t T, 
   if (check_layer(L)) return CSK_ERR_INVALID;
   if (!d_hidden || !d_send_f16 || !d_counts) return fail(L, CSK_ERR_INVALID, "null argument");
   if (T <= 0 || T > L->max_T) return fail(L, CSK_ERR_NOMEM, "T=%lld outside (0, max_tokens]", (long long)T);
+  if (reinterpret_cast<uintptr_t>(d_hidden) % 16) return fail(L, CSK_ERR_INVALID, "hidden states must be 16-byte aligned");
+  if (reinterpret_cast<uintptr_t>(d_send_f16) % 8) return fail(L, CSK_ERR_INVALID, "the rows to send must be 8-byte aligned");
   CSK_CUDA(L, cudaSetDevice(L->cfg.device));
   cudaStream_t s = pick(L, stream);
   L->last = csk_moe_timings{};

@@ -281,7 +281,9 @@ int csk_moe_route_static_status(void);
  *   dispatch_dev  : route local tokens, group their (token, expert) rows by
  *                   global expert id (which is by destination rank, then
  *                   expert), write them as fp16 rows into d_send and the
- *                   per-expert row counts into d_counts [E] (int32)
+ *                   per-expert row counts into d_counts [E] (int32).
+ *                   d_hidden lies at a multiple of 16 bytes, d_send of 8
+ *                   (of 16: wider stores)
  *   <all-to-all of counts, then of rows: the caller's NCCL>
  *   experts_dev   : run the resident experts over received rows.  d_recv holds
  *                   n_src segments (one per source rank), each ordered by local

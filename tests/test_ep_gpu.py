@@ -249,3 +249,37 @@ def test_a_layer_with_part_of_the_experts_keeps_no_image_rows_it_cannot_use(gpu_
     weights = 2 * 2 * 3 * H * H * 17 // 32 + 3 * H * H * 17 // 32
     assert used <= rows + weights + 150e6, (used, rows, weights)
     lay.close()
+
+
+@pytest.mark.parametrize("T,k", [(5, 2), (700, 2), (1100, 8)])  # (rows placed by the plan's one block, and claimed by the kernel)
+def test_rows_to_send_at_a_multiple_of_8_bytes(gpu_lib, T, k):
+    """The buffer of the rows to send may lie 8 bytes off a multiple of 16; what lies around it stays."""
+    import torch
+    from coalsack_b200 import CskError
+    sh = synth.tiny(seed=T, E=16, k=k, H=96, F=64, T=T, has_bias=True)
+    h, Wg, rb, ex = cases.layer_inputs(sh)
+    lay = MoeLayer.from_shape(sh)
+    lay.set_router(Wg, rb)
+    lay.load_experts(ex)
+    pitch, n = lay.ep_row_pitch(), T * k
+    x = torch.from_numpy(h).cuda()
+    outs = []
+    for off in (0, 4, 12):  # fp16 elements
+        store = torch.full((n * pitch + 32,), 7.0, dtype=torch.float16, device="cuda")
+        send = store[off:off + n * pitch]
+        send.zero_()
+        counts = torch.zeros(16, dtype=torch.int32, device="cuda")
+        back, out = torch.zeros((n, 96), device="cuda"), torch.empty((T, 96), device="cuda")
+        torch.cuda.synchronize()
+        lay.ep_dispatch_dev(x, T, send, counts)
+        torch.cuda.synchronize()
+        assert (store[:off] == 7).all() and (store[off + n * pitch:] == 7).all()
+        assert (send.view(n, pitch)[:, 96:] == 0).all()
+        lay.ep_experts_dev(send.clone(), counts, 1, n, back)
+        lay.ep_combine_dev(back, T, out)
+        lay.sync()
+        outs.append(out)
+    assert torch.equal(outs[0], outs[1]) and torch.equal(outs[0], outs[2])
+    with pytest.raises(CskError, match="aligned"):
+        lay.ep_dispatch_dev(x, T, store[2:2 + n * pitch], counts)
+    lay.close()
