@@ -507,11 +507,18 @@ cudaError_t router_prepare_set() {
 // memory.  Once per device.
 inline cudaError_t router_prepare_device();
 
+// How the chain is launched for a number of groups of 32 experts: the blocks that are resident at once, and whether the blocks of a
+// token block form a cluster (else they meet in global memory).
+struct RouterWave {
+  int blocks;
+  bool clusters;
+};
+
 template <int TW, int TT, int CH, bool PACKED>
-void launch_router_one(RouterArgs a, int token_slots, cudaStream_t s, bool pdl) {
+void launch_router_one(RouterArgs a, int token_slots, RouterWave wave, cudaStream_t s, bool pdl) {
   const unsigned groups = (unsigned)((a.E + 31) / 32);
   constexpr int BT = TW * TT;
-  a.cluster = PACKED && a.counters && groups > 1 && groups <= kRouterClusterGroups;
+  a.cluster = PACKED && a.counters && wave.clusters;
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3((unsigned)((token_slots + BT - 1) / BT), groups);
   cfg.blockDim = dim3((TW + router_producer_warps(PACKED)) * 32);
@@ -529,10 +536,12 @@ void launch_router_one(RouterArgs a, int token_slots, cudaStream_t s, bool pdl) 
   cudaLaunchKernelEx(&cfg, k_router_logits<TW, TT, CH, PACKED>, a);
 }
 
-// Blocks of the widest launch that are resident at once, for `groups` groups of 32 experts: an SM each, but clusters leave some SMs of a
-// GPC over (with a fixed nine tenths of the SMs, 64 tokens of 256 experts took two waves of clusters of eight, 30.5 us).
-inline int router_wave(int groups, int sm_count) {
-  if (groups < 2 || groups > kRouterClusterGroups) return sm_count;
+// An SM each, but clusters leave some SMs of a GPC over (with a fixed nine tenths of the SMs, 64 tokens of 256 experts took two waves
+// of clusters of eight, 30.5 us): the runtime is asked about the widest launch.  One group needs no cluster, more than
+// kRouterClusterGroups of them can have none, and where no such cluster can be resident (a part of a device) there is none either.
+// (Through global memory, with clusters / without, us: 128 experts of 2880 columns 8 tokens 14.5 / 15.7, 333 25.4 / 28.8; 64 experts 333 20.6 / 23.0.)
+inline RouterWave router_wave(int groups, int sm_count) {
+  if (groups < 2 || groups > kRouterClusterGroups) return {sm_count, false};
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3(1024, (unsigned)groups);
   cfg.blockDim = dim3((8 + router_producer_warps(true)) * 32);
@@ -547,9 +556,9 @@ inline int router_wave(int groups, int sm_count) {
   int clusters = 0;
   if (cudaOccupancyMaxActiveClusters(&clusters, k_router_logits<8, 4, kRouterChunkMany, true>, &cfg) != cudaSuccess || clusters < 1) {
     cudaGetLastError();
-    return 3 * sm_count / 4;
+    return {sm_count, false};
   }
-  return std::min(clusters * groups, sm_count);
+  return {std::min(clusters * groups, sm_count), true};
 }
 
 // The fewest tokens per block with which the blocks are one wave: a block's time goes by its chains per thread and, from four warps
@@ -563,21 +572,21 @@ inline int router_wave(int groups, int sm_count) {
 // wg_few / wg_many: the weights packed for the two chunk widths (PACKED) or both the plain [E,H] matrix.  token_slots: tokens the
 // grid is sized for (a.T, or for a list-driven launch the most entries the list can have).
 template <bool PACKED>
-inline void launch_router_logits(RouterArgs a, const float* wg_few, const float* wg_many, int wave, cudaStream_t s, bool pdl = false,
-                                 int token_slots = -1) {
+inline void launch_router_logits(RouterArgs a, const float* wg_few, const float* wg_many, RouterWave wave, cudaStream_t s,
+                                 bool pdl = false, int token_slots = -1) {
   if (token_slots < 0) token_slots = a.T;
   const int64_t groups = (a.E + 31) / 32;
-  auto one_wave = [&](int tokens) { return (token_slots + tokens - 1) / tokens * groups <= wave; };
+  auto one_wave = [&](int tokens) { return (token_slots + tokens - 1) / tokens * groups <= wave.blocks; };
   a.wg = wg_few;
-  if (one_wave(1)) return launch_router_one<1, 1, kRouterChunkFew, PACKED>(a, token_slots, s, pdl);
-  if (one_wave(2)) return launch_router_one<2, 1, kRouterChunkFew, PACKED>(a, token_slots, s, pdl);
-  if (one_wave(4)) return launch_router_one<4, 1, kRouterChunkFew, PACKED>(a, token_slots, s, pdl);
+  if (one_wave(1)) return launch_router_one<1, 1, kRouterChunkFew, PACKED>(a, token_slots, wave, s, pdl);
+  if (one_wave(2)) return launch_router_one<2, 1, kRouterChunkFew, PACKED>(a, token_slots, wave, s, pdl);
+  if (one_wave(4)) return launch_router_one<4, 1, kRouterChunkFew, PACKED>(a, token_slots, wave, s, pdl);
   a.wg = wg_many;
-  if (one_wave(8)) return launch_router_one<4, 2, kRouterChunkMany, PACKED>(a, token_slots, s, pdl);
-  if (one_wave(12)) return launch_router_one<4, 3, kRouterChunkMany, PACKED>(a, token_slots, s, pdl);
-  if (one_wave(16) || (!one_wave(32) && groups == 1)) return launch_router_one<4, 4, kRouterChunkMany, PACKED>(a, token_slots, s, pdl);
-  if (one_wave(24)) return launch_router_one<8, 3, kRouterChunkMany, PACKED>(a, token_slots, s, pdl);
-  launch_router_one<8, 4, kRouterChunkMany, PACKED>(a, token_slots, s, pdl);
+  if (one_wave(8)) return launch_router_one<4, 2, kRouterChunkMany, PACKED>(a, token_slots, wave, s, pdl);
+  if (one_wave(12)) return launch_router_one<4, 3, kRouterChunkMany, PACKED>(a, token_slots, wave, s, pdl);
+  if (one_wave(16) || (!one_wave(32) && groups == 1)) return launch_router_one<4, 4, kRouterChunkMany, PACKED>(a, token_slots, wave, s, pdl);
+  if (one_wave(24)) return launch_router_one<8, 3, kRouterChunkMany, PACKED>(a, token_slots, wave, s, pdl);
+  launch_router_one<8, 4, kRouterChunkMany, PACKED>(a, token_slots, wave, s, pdl);
 }
 
 // ---------------------------------------------------------------------------

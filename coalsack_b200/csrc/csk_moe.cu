@@ -56,7 +56,7 @@ struct csk_moe_layer {
   float* d_wg_tc_scale = nullptr;
   float* d_wnorm_tc = nullptr;
   int router_mode = CSK_ROUTER_AUTO;
-  int router_waves[kMaxExperts / 32 + 1] = {};  // router_wave by groups of 32 experts
+  RouterWave router_waves[kMaxExperts / 32 + 1] = {};  // by groups of 32 experts
   int64_t routed_tokens = 0;   // tokens routed in certified mode since creation
   float* d_logits = nullptr;  // [max_T,E] router scratch
   float* d_rbias = nullptr;
@@ -239,7 +239,7 @@ int launch_router(csk_moe_layer* L, const float* d_hidden, int64_t T, float* d_r
   const int groups = (L->E_router + 31) / 32;
   const int64_t tensor_min_work = groups >= 16 ? 8192 : 4096;  // tokens x groups of 32 experts
   const bool few = T <= kCertifiedMaxTokens, many = groups > 1 && T * groups >= tensor_min_work;
-  const int router_wave = L->router_waves[groups];
+  const RouterWave router_wave = L->router_waves[groups];
   if (L->router_mode == CSK_ROUTER_CHAIN || (L->router_mode == CSK_ROUTER_AUTO && !few && !many)) {
     launch_router_logits<true>(a, L->d_wg_few, L->d_wg_many, router_wave, s, L->pdl);
     CSK_CUDA(L, cudaGetLastError());
@@ -323,7 +323,7 @@ int launch_router(csk_moe_layer* L, const float* d_hidden, int64_t T, float* d_r
   b.fb_done = L->d_fb + 1;
   b.fb_total = reinterpret_cast<unsigned long long*>(L->d_fb + 2);
   b.list_max = INT32_MAX;
-  const int64_t wave = std::max(1, 4 * (router_wave / groups));  // tokens of one wave of four-token blocks
+  const int64_t wave = std::max(1, 4 * (router_wave.blocks / groups));  // tokens of one wave of four-token blocks
   if (many) {
     // How long the list is the data decide: 2 % of the tokens of normal rows, half of them with a few channels at 1000 times
     // the others, all where rows repeat a value (padding).  Blocks of few tokens are quicker for a short list: the first
@@ -2379,7 +2379,7 @@ int csk_moe_route_static(const float* d_hidden, int64_t T, int32_t H, const floa
   a.T = (int)T;
   a.H = H;
   a.E = E;
-  launch_router_logits<false>(a, d_gate_w, d_gate_w, sms, s);
+  launch_router_logits<false>(a, d_gate_w, d_gate_w, RouterWave{sms, false}, s);
   k_router_topk<<<(unsigned)((T + 3) / 4), 128, 0, s>>>(logits, d_router_out, (int)T, E, k, sigmoid_gating);
   ce = cudaGetLastError();
   if (ce != cudaSuccess) return fail(nullptr, CSK_ERR_CUDA, "route_static: launch failed: %s", cudaGetErrorString(ce));
@@ -2428,8 +2428,24 @@ int csk_moe_debug_set(csk_moe_layer* L, int32_t key, int64_t value) {
     if (!value) return fail(L, CSK_ERR_INVALID, "debug: clusters do not come back");
     L->pair.available = false;
     L->pair.err = "turned off by a test";
+    for (RouterWave& w : L->router_waves) w = RouterWave{L->sm_count, false};
     drop_graphs(L);
     return mx_reserve(L, mx_rows_own(L));
+  }
+  return fail(L, CSK_ERR_INVALID, "debug: unknown key %d", key);
+}
+
+int csk_moe_debug_get(csk_moe_layer* L, int32_t key, int64_t* value) {
+  if (check_layer(L)) return CSK_ERR_INVALID;
+  if (!value) return fail(L, CSK_ERR_INVALID, "null argument");
+  const RouterWave w = L->router_waves[(L->E_router + 31) / 32];
+  if (key == CSK_DEBUG_ROUTER_WAVE) {
+    *value = w.blocks;
+    return CSK_OK;
+  }
+  if (key == CSK_DEBUG_ROUTER_CLUSTERS) {
+    *value = w.clusters ? 1 : 0;
+    return CSK_OK;
   }
   return fail(L, CSK_ERR_INVALID, "debug: unknown key %d", key);
 }

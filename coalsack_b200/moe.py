@@ -374,10 +374,17 @@ class MoeLayer:
         return a.value, b.value
 
     DEBUG_WAIT_BUDGET, DEBUG_STALL_TILE_PRODUCER, DEBUG_STALL_ROUTER, DEBUG_NO_CLUSTERS = 0, 1, 2, 3
+    DEBUG_ROUTER_WAVE, DEBUG_ROUTER_CLUSTERS = 4, 5
 
     def debug_set(self, key, value):
         """Test hooks of the failure path (csk_moe_debug_set)."""
         self._check(self._lib.csk_moe_debug_set(self._h, int(key), int(value)))
+
+    def debug_get(self, key):
+        """What can be asked for beside them (csk_moe_debug_get)."""
+        v = C.c_int64(0)
+        self._check(self._lib.csk_moe_debug_get(self._h, int(key), C.byref(v)))
+        return v.value
 
     def enable_timing(self, on=True):
         self._check(self._lib.csk_moe_enable_timing(self._h, int(on)))

@@ -437,9 +437,21 @@ int csk_moe_get_counters(csk_moe_layer* layer, int64_t* rows_per_expert, int64_t
  *   CSK_DEBUG_STALL_ROUTER        the same in the NEXT tensor-core router launch (large
  *                                 batches in certified mode)
  *   CSK_DEBUG_NO_CLUSTERS         non-zero: the handle goes on as on a device where no
- *                                 cluster of two CTAs can be resident */
-enum { CSK_DEBUG_WAIT_BUDGET = 0, CSK_DEBUG_STALL_TILE_PRODUCER = 1, CSK_DEBUG_STALL_ROUTER = 2, CSK_DEBUG_NO_CLUSTERS = 3 };
+ *                                 cluster of CTAs can be resident
+ * and what can be asked for:
+ *   CSK_DEBUG_ROUTER_WAVE         blocks of the router's chain that are resident at once (a
+ *                                 block has 32 experts and some tokens)
+ *   CSK_DEBUG_ROUTER_CLUSTERS     whether the blocks of its groups of experts form clusters */
+enum {
+  CSK_DEBUG_WAIT_BUDGET = 0,
+  CSK_DEBUG_STALL_TILE_PRODUCER = 1,
+  CSK_DEBUG_STALL_ROUTER = 2,
+  CSK_DEBUG_NO_CLUSTERS = 3,
+  CSK_DEBUG_ROUTER_WAVE = 4,
+  CSK_DEBUG_ROUTER_CLUSTERS = 5
+};
 int csk_moe_debug_set(csk_moe_layer* layer, int32_t key, int64_t value);
+int csk_moe_debug_get(csk_moe_layer* layer, int32_t key, int64_t* value);
 
 #ifdef __cplusplus
 }

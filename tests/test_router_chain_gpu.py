@@ -68,3 +68,29 @@ def test_a_handful_of_tokens_that_cannot_be_separated(gpu_lib, port, E, H, T):
     routed, chained = lay.router_stats()
     assert routed == 8 * T and chained >= T and seen >= T, (routed, chained, seen)
     lay.close()
+
+
+@pytest.mark.parametrize("E,H,T", [(33, 256, 3), (64, 288, 64), (128, 2880, 1), (128, 256, 333), (128, 160, 1100), (256, 1056, 40), (256, 96, 2000)])
+def test_the_same_without_clusters(gpu_lib, E, H, T):
+    """Where no cluster can be resident the groups of experts of a token block meet in global memory: the same routing bit for bit, of the
+    chain and of the certified pass with its list."""
+    rng = np.random.default_rng(E + T)
+    h = rng.standard_normal((T, H)).astype(np.float32)
+    h[::3] = h[0]  # (rows that repeat ...
+    h[T - 1] = 0.0     # ... and one that no bound can certify)
+    Wg = (rng.standard_normal((E, H)) * 0.02).astype(np.float32)
+    lay = MoeLayer(E, 4, H, 32, has_bias=False, max_tokens=T)
+    lay.set_router(Wg, None)
+    assert lay.debug_get(lay.DEBUG_ROUTER_CLUSTERS) == 1
+    modes = (lay.ROUTER_CHAIN, lay.ROUTER_CERTIFIED, lay.ROUTER_AUTO)
+    want = []
+    for mode in modes:
+        lay.set_router_mode(mode)
+        want.append(lay.route(h))
+    lay.debug_set(lay.DEBUG_NO_CLUSTERS, 1)
+    assert lay.debug_get(lay.DEBUG_ROUTER_CLUSTERS) == 0
+    for mode, w in zip(modes, want):
+        lay.set_router_mode(mode)
+        for _ in range(2):
+            assert np.array_equal(lay.route(h), w), mode
+    lay.close()
