@@ -512,6 +512,7 @@ inline cudaError_t router_prepare_device();
 struct RouterWave {
   int blocks;
   bool clusters;
+  int alone;  // blocks resident at once without clusters
 };
 
 template <int TW, int TT, int CH, bool PACKED>
@@ -541,7 +542,7 @@ void launch_router_one(RouterArgs a, int token_slots, RouterWave wave, cudaStrea
 // kRouterClusterGroups of them can have none, and where no such cluster can be resident (a part of a device) there is none either.
 // (Through global memory, with clusters / without, us: 128 experts of 2880 columns 8 tokens 14.5 / 15.7, 333 25.4 / 28.8; 64 experts 333 20.6 / 23.0.)
 inline RouterWave router_wave(int groups, int sm_count) {
-  if (groups < 2 || groups > kRouterClusterGroups) return {sm_count, false};
+  if (groups < 2 || groups > kRouterClusterGroups) return {sm_count, false, sm_count};
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3(1024, (unsigned)groups);
   cfg.blockDim = dim3((8 + router_producer_warps(true)) * 32);
@@ -556,9 +557,9 @@ inline RouterWave router_wave(int groups, int sm_count) {
   int clusters = 0;
   if (cudaOccupancyMaxActiveClusters(&clusters, k_router_logits<8, 4, kRouterChunkMany, true>, &cfg) != cudaSuccess || clusters < 1) {
     cudaGetLastError();
-    return {sm_count, false};
+    return {sm_count, false, sm_count};
   }
-  return {std::min(clusters * groups, sm_count), true};
+  return {std::min(clusters * groups, sm_count), true, sm_count};
 }
 
 // The fewest tokens per block with which the blocks are one wave: a block's time goes by its chains per thread and, from four warps
@@ -577,6 +578,12 @@ inline void launch_router_logits(RouterArgs a, const float* wg_few, const float*
   if (token_slots < 0) token_slots = a.T;
   const int64_t groups = (a.E + 31) / 32;
   auto one_wave = [&](int tokens) { return (token_slots + tokens - 1) / tokens * groups <= wave.blocks; };
+  if (wave.clusters && !one_wave(32)) {
+    // The SMs that clusters leave over may be what the last wave needs: without clusters then.  2880 columns, with / without: 256 experts
+    // (120 blocks at once / 148), 511 tokens 94.3 / 54.5 us, 1000 139.5 / 99.0; 224 experts, 560 tokens 94.3 / 55.0.
+    const int64_t blocks = (token_slots + 31) / 32 * groups;
+    if ((blocks + wave.alone - 1) / wave.alone < (blocks + wave.blocks - 1) / wave.blocks) wave = {wave.alone, false, wave.alone};
+  }
   a.wg = wg_few;
   if (one_wave(1)) return launch_router_one<1, 1, kRouterChunkFew, PACKED>(a, token_slots, wave, s, pdl);
   if (one_wave(2)) return launch_router_one<2, 1, kRouterChunkFew, PACKED>(a, token_slots, wave, s, pdl);

@@ -2379,7 +2379,7 @@ int csk_moe_route_static(const float* d_hidden, int64_t T, int32_t H, const floa
   a.T = (int)T;
   a.H = H;
   a.E = E;
-  launch_router_logits<false>(a, d_gate_w, d_gate_w, RouterWave{sms, false}, s);
+  launch_router_logits<false>(a, d_gate_w, d_gate_w, RouterWave{sms, false, sms}, s);
   k_router_topk<<<(unsigned)((T + 3) / 4), 128, 0, s>>>(logits, d_router_out, (int)T, E, k, sigmoid_gating);
   ce = cudaGetLastError();
   if (ce != cudaSuccess) return fail(nullptr, CSK_ERR_CUDA, "route_static: launch failed: %s", cudaGetErrorString(ce));
@@ -2428,7 +2428,7 @@ int csk_moe_debug_set(csk_moe_layer* L, int32_t key, int64_t value) {
     if (!value) return fail(L, CSK_ERR_INVALID, "debug: clusters do not come back");
     L->pair.available = false;
     L->pair.err = "turned off by a test";
-    for (RouterWave& w : L->router_waves) w = RouterWave{L->sm_count, false};
+    for (RouterWave& w : L->router_waves) w = RouterWave{L->sm_count, false, L->sm_count};
     drop_graphs(L);
     return mx_reserve(L, mx_rows_own(L));
   }
