@@ -154,10 +154,20 @@ struct csk_moe_layer {
 
 namespace {
 
-// Host buffers of at most so many bytes each way go through page-locked staging of the handle's own.  32 tokens of
-// the 32-expert layer, pageable: 200 -> 191 us a call (copies of pageable memory wait for the device, and the status had a wait of its own).
-// One area for both ways: with two, creating a layer of 8192 tokens took 13.5 ms, with one 11.1.
+// Host buffers of at most so many bytes each way go through page-locked staging of the handle's own if they are pageable.  32
+// tokens of the 32-expert layer: 200 -> 169 us a call, 80 (0.9 MB) 277 -> 268 (copies of pageable memory wait for the device, and the status had a
+// wait of its own).  One area for both ways: with two, creating a layer of 8192 tokens took 13.5 ms, with one 11.1.
 constexpr size_t kStagedMax = 1 << 20;
+// On the way in the driver takes up to 64 KB itself without a wait, and a second piece, whose host copy runs beside the first one's way
+// to the device, costs a launch.  By the driver / one piece / two, us: 2 tokens of that layer (22 KB) 76 / 78 / 89, 4 (45 KB) 97.5 / 103 / 107, 8 (90
+// KB) 134 / 129 / 131, 16 (180 KB) 155 / 148 / 151, 32 (360 KB) 176 / 173 / 169; 8 experts of 512 x 512, 8 tokens (16 KB) 51 / 51 / 63, 32 (64 KB)
+// 60 / 65 / 67, 80 (160 KB) 80 / 73 / 77, 200 (400 KB) 101 / 99 / 92.
+constexpr size_t kStagedInMin = 64 << 10, kStagedTwoPieces = 256 << 10;
+// Page-locked buffers need none on the way in.  On the way out a copy into them has to wait for the status word, so that a call that
+// fails leaves them alone: up to so many bytes that wait is dearer than a host copy.  The layer above, direct / staged, us: 1 token (11 KB)
+// 70.3 / 64.4, 2 81.7 / 76.6, 8 (90 KB) 121.9 / 118.7, 16 (180 KB) 145.3 / 147.4, 32 160.5 / 168.6, 80 186 / 216; 8 experts of 512 x 512, 32 tokens
+// (64 KB) 68.3 / 65.2, 80 (160 KB) 70.7 / 71.7.  (Staged on the way in, too: 32 tokens 173, 80 268.)
+constexpr size_t kStagedLockedMax = 128 << 10;
 
 int wide_stride(const csk_moe_layer* L) { return mx_mask_words(L->Lgu.recs) + mx_mask_words(L->Ld.recs); }
 
@@ -1709,11 +1719,11 @@ int csk_moe_route(csk_moe_layer* L, const float* hidden, int64_t T, float* route
 }
 
 namespace {
-// Whether every buffer of a call is page-locked (null: not given).  A copy to or from other memory returns when it is done.
-bool page_locked(std::initializer_list<const void*> buffers) {
+// Whether every buffer of a call (null: not given) is in memory of a type: page-locked (Host) or pageable (Unregistered).
+bool all_in(cudaMemoryType type, std::initializer_list<const void*> buffers) {
   for (const void* p : buffers) {
     cudaPointerAttributes at{};
-    if (p && (cudaPointerGetAttributes(&at, p) != cudaSuccess || at.type != cudaMemoryTypeHost)) {
+    if (p && (cudaPointerGetAttributes(&at, p) != cudaSuccess || at.type != type)) {
       cudaGetLastError();
       return false;
     }
@@ -1740,7 +1750,8 @@ int host_passes(const csk_moe_layer* L, int64_t T, std::initializer_list<const v
   if (L->timing || L->path == CSK_PATH_STREAM) return 1;
   const int64_t rows = T * L->k / std::max(1, L->Eloc);  // per expert
   if (rows < 128) return 1;
-  if (!page_locked(buffers)) return rows < 600 ? 1 : 2;
+  // (a copy to or from other than page-locked memory returns when it is done)
+  if (!all_in(cudaMemoryTypeHost, buffers)) return rows < 600 ? 1 : 2;
   const int least = rows < 256 ? 1 : 2;
   const int tile_rows = tile_rows_for(CSK_PATH_TILE);
   auto items = [&](int passes) { return (rows / passes + tile_rows - 1) / tile_rows * L->Eloc * L->Tgu.n_tiles; };
@@ -1759,47 +1770,46 @@ int csk_moe_forward(csk_moe_layer* L, const float* hidden, int64_t T, const floa
   cudaStream_t s = L->stream;
   const int passes = host_passes(L, T, {hidden, router_in, router_out, out});
   const size_t row_bytes = sizeof(float) * T * L->H, route_bytes = sizeof(float) * T * L->k * 2;
-  if (passes == 1 && row_bytes + route_bytes <= L->h_staged_bytes) {
-    // A small batch goes through page-locked staging, in two pieces on the way in, and its status word comes back with its results:
-    // one wait a call, and no copy that the driver has to stage itself.
-    const int64_t half = T / 2 * L->H;
-    for (const auto& [at, n] : {std::pair{(int64_t)0, half}, std::pair{half, T * L->H - half}}) {
-      if (!n) continue;
-      memcpy(L->h_staged + at, hidden + at, sizeof(float) * n);
-      CSK_CUDA(L, cudaMemcpyAsync(L->d_hidden + at, L->h_staged + at, sizeof(float) * n, cudaMemcpyHostToDevice, s));
-    }
+  if (passes == 1) {
+    // Through the handle's staging area a batch's status word comes back with its results, and nothing waits for a copy that the driver stages.
+    const size_t bytes = row_bytes + route_bytes;
+    const bool fits = bytes <= L->h_staged_bytes;
+    const bool staged_in = fits && row_bytes > kStagedInMin && all_in(cudaMemoryTypeUnregistered, {hidden, router_in});
+    const bool staged_out = fits && (all_in(cudaMemoryTypeUnregistered, {out, router_out}) ||
+                                     (bytes <= kStagedLockedMax && all_in(cudaMemoryTypeHost, {out, router_out})));
     float* staged_route = L->h_staged + T * L->H;
-    if (router_in) {
-      memcpy(staged_route, router_in, route_bytes);
-      CSK_CUDA(L, cudaMemcpyAsync(L->d_router, staged_route, route_bytes, cudaMemcpyHostToDevice, s));
+    if (staged_in) {
+      const int64_t half = row_bytes < kStagedTwoPieces ? 0 : T / 2 * L->H;
+      for (const auto& [at, n] : {std::pair{(int64_t)0, half}, std::pair{half, T * L->H - half}}) {
+        if (!n) continue;
+        memcpy(L->h_staged + at, hidden + at, sizeof(float) * n);
+        CSK_CUDA(L, cudaMemcpyAsync(L->d_hidden + at, L->h_staged + at, sizeof(float) * n, cudaMemcpyHostToDevice, s));
+      }
+      if (router_in) memcpy(staged_route, router_in, route_bytes);
+    } else {
+      CSK_CUDA(L, cudaMemcpyAsync(L->d_hidden, hidden, row_bytes, cudaMemcpyHostToDevice, s));
     }
+    if (router_in) CSK_CUDA(L, cudaMemcpyAsync(L->d_router, staged_in ? staged_route : router_in, route_bytes, cudaMemcpyHostToDevice, s));
     int rc = csk_moe_forward_dev(L, L->d_hidden, T, router_in ? L->d_router : nullptr, nullptr, L->d_out, s);
     if (rc) {
-      cudaStreamSynchronize(s);  // the copies in have left the staging area
+      if (staged_in) cudaStreamSynchronize(s);  // the copies in have left the staging area
       return rc;
     }
-    // The results come back to where the inputs went out from: the stream has taken those first.
-    CSK_CUDA(L, cudaMemcpyAsync(L->h_staged, L->d_out, row_bytes, cudaMemcpyDeviceToHost, s));
-    if (router_out) CSK_CUDA(L, cudaMemcpyAsync(staged_route, L->d_router, route_bytes, cudaMemcpyDeviceToHost, s));
+    if (staged_out) {
+      // (where the inputs went out from, too: the stream has taken those first)
+      CSK_CUDA(L, cudaMemcpyAsync(L->h_staged, L->d_out, row_bytes, cudaMemcpyDeviceToHost, s));
+      if (router_out) CSK_CUDA(L, cudaMemcpyAsync(staged_route, L->d_router, route_bytes, cudaMemcpyDeviceToHost, s));
+    }
     rc = check_device_status(L, s);
     if (rc) return rc;
     if (L->timing && L->n_marks > 1) finish_timings(L, L->n_marks, L->last_routed);
-    memcpy(out, L->h_staged, row_bytes);
-    if (router_out) memcpy(router_out, staged_route, route_bytes);
-    return CSK_OK;
-  }
-  if (passes == 1) {
-    CSK_CUDA(L, cudaMemcpyAsync(L->d_hidden, hidden, sizeof(float) * T * L->H, cudaMemcpyHostToDevice, s));
-    if (router_in)
-      CSK_CUDA(L, cudaMemcpyAsync(L->d_router, router_in, sizeof(float) * T * L->k * 2, cudaMemcpyHostToDevice, s));
-    int rc = csk_moe_forward_dev(L, L->d_hidden, T, router_in ? L->d_router : nullptr, nullptr, L->d_out, s);
-    if (rc) return rc;
-    rc = check_device_status(L, s);
-    if (rc) return rc;
-    if (L->timing && L->n_marks > 1) finish_timings(L, L->n_marks, L->last_routed);
-    CSK_CUDA(L, cudaMemcpyAsync(out, L->d_out, sizeof(float) * T * L->H, cudaMemcpyDeviceToHost, s));
-    if (router_out)
-      CSK_CUDA(L, cudaMemcpyAsync(router_out, L->d_router, sizeof(float) * T * L->k * 2, cudaMemcpyDeviceToHost, s));
+    if (staged_out) {
+      memcpy(out, L->h_staged, row_bytes);
+      if (router_out) memcpy(router_out, staged_route, route_bytes);
+      return CSK_OK;
+    }
+    CSK_CUDA(L, cudaMemcpyAsync(out, L->d_out, row_bytes, cudaMemcpyDeviceToHost, s));
+    if (router_out) CSK_CUDA(L, cudaMemcpyAsync(router_out, L->d_router, route_bytes, cudaMemcpyDeviceToHost, s));
     CSK_CUDA(L, cudaStreamSynchronize(s));
     return CSK_OK;
   }

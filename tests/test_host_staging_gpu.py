@@ -40,3 +40,35 @@ def test_results_and_errors(gpu_lib, T, routed):
     lay.forward(h, router_out=given, out=out, router_out_buf=ro)
     assert np.array_equal(out, kept_out) and np.array_equal(ro, kept_ro)
     lay.close()
+
+
+# (64 KB are 16 rows of 1024 columns, 128 KB 31 with two slots each, 256 KB 64)
+@pytest.mark.parametrize("T", [1, 16, 17, 31, 32, 63, 64, 200, 256])
+@pytest.mark.parametrize("locked_in,locked_out", [(True, True), (True, False), (False, True)])
+def test_page_locked_buffers(gpu_lib, T, locked_in, locked_out):
+    """Page-locked buffers are copied without staging (small results with it), in any mixture: the same results, and nothing written
+    by a call that fails."""
+    sh = synth.tiny(seed=70 + T, E=8, k=2, H=1024, F=64, T=T, has_bias=True)
+    h, Wg, rb, ex = cases.layer_inputs(sh)
+    lay = MoeLayer.from_shape(sh)
+    lay.set_router(Wg, rb)
+    lay.load_experts(ex)
+    out, ro = np.full((T, 1024), 7, np.float32), np.full((T, 2, 2), 7, np.float32)
+    lay.forward(h, out=out, router_out_buf=ro)
+
+    def host(shape, locked):
+        return torch.full(shape, 5.0, pin_memory=locked).numpy()
+
+    x, x_route = host((T, 1024), locked_in), host((T, 2, 2), locked_in)
+    got, got_ro = host((T, 1024), locked_out), host((T, 2, 2), locked_out)
+    x[:], x_route[:] = h, ro
+    for given in (None, x_route):
+        for _ in range(2):
+            got[:], got_ro[:] = 5, 5
+            lay.forward(x, router_out=given, out=got, router_out_buf=got_ro)
+            assert np.array_equal(got, out) and np.array_equal(got_ro, ro)
+    x_route[T - 1, 1, 0] = 8
+    with pytest.raises(CskError, match="out of range"):
+        lay.forward(x, router_out=x_route, out=got, router_out_buf=got_ro)
+    assert np.array_equal(got, out) and np.array_equal(got_ro, ro)
+    lay.close()
