@@ -1775,8 +1775,6 @@ int csk_moe_forward(csk_moe_layer* L, const float* hidden, int64_t T, const floa
     const size_t bytes = row_bytes + route_bytes;
     const bool fits = bytes <= L->h_staged_bytes;
     const bool staged_in = fits && row_bytes > kStagedInMin && all_in(cudaMemoryTypeUnregistered, {hidden, router_in});
-    const bool staged_out = fits && (all_in(cudaMemoryTypeUnregistered, {out, router_out}) ||
-                                     (bytes <= kStagedLockedMax && all_in(cudaMemoryTypeHost, {out, router_out})));
     float* staged_route = L->h_staged + T * L->H;
     if (staged_in) {
       const int64_t half = row_bytes < kStagedTwoPieces ? 0 : T / 2 * L->H;
@@ -1795,6 +1793,9 @@ int csk_moe_forward(csk_moe_layer* L, const float* hidden, int64_t T, const floa
       if (staged_in) cudaStreamSynchronize(s);  // the copies in have left the staging area
       return rc;
     }
+    // (asked while the kernels run)
+    const bool staged_out = fits && (all_in(cudaMemoryTypeUnregistered, {out, router_out}) ||
+                                     (bytes <= kStagedLockedMax && all_in(cudaMemoryTypeHost, {out, router_out})));
     if (staged_out) {
       // (where the inputs went out from, too: the stream has taken those first)
       CSK_CUDA(L, cudaMemcpyAsync(L->h_staged, L->d_out, row_bytes, cudaMemcpyDeviceToHost, s));
