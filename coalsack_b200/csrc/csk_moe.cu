@@ -1736,12 +1736,16 @@ bool all_in(cudaMemoryType type, std::initializer_list<const void*> buffers) {
 // it has been copied out.  1 / 2 / 4 / 8 passes, ms: 128 experts of 2880 x 2880, 4096 tokens (128 rows per expert) 7.57 / 7.59 / 7.91 / 8.99, 8192
 // (256) 14.7 / 15.4 / 15.9 / 18.0; 32 experts, 2048 (256) 2.92 / 3.12 / 3.67 / 4.56, 3000 (375) 4.46 / 4.41 / 5.09 / 5.95, 8192 (1024) 13.5 / 13.4 /
 // 15.2 / 15.3; 8 of 1728 x 1728, top-2, 2000 (500) 1.68 / 1.80 / 2.02 / 2.39; fp16, 32 of 2880 x 2880, 4096 (512) 6.10 / 6.32 / 6.88 / 8.35.
-// Page-locked buffers: two from 128 rows per expert on, three from 240, and one for every 120.  What stays exposed is the first copy in and
-// the last copy out; what passes cost is kernel time, the less the more rows an expert has (a row tile's cost is nearly flat below 100
-// rows).  1 / 2 / 3 / 4 / 8 passes, ms: 128 experts of 2880 x 2880, 4096 tokens 2.58 / 2.20 / 2.46 / 2.74 / 3.18, 8192 4.96 / 3.47 / 3.30 / 3.54 / 5.02;
-// 32 experts, 1500 (187) 0.95 / 0.77 / 0.82 / 0.93 / 1.29, 2048 1.29 / 0.90 / 0.93 / 1.01 / 1.48, 3000 1.80 / 1.30 / 1.14 / 1.18 / 1.66, 8192 4.76 / 3.39 /
-// 2.97 / 2.76 / 2.49; 128 of 2048 x 768, top-8, 4096 (256) 1.70 / 1.25 / 1.14 / 1.13 / 1.47; fp16, 16 of 2048 x 2048, 4096 (256) 1.42 / 1.15 / 1.09 / 1.10 /
-// 1.02; 32 of 2880 x 2880, 1500 1.03 / 1.01 / 1.16 / 1.39 / 2.44, 8192 4.98 / 3.47 / 3.02 / 2.80 / 3.14.  But no more than leave a pass items (a row
+// Page-locked buffers: two from 128 rows per expert on, and one for every 120.  What stays exposed is the first copy in and the last
+// copy out; what passes cost is kernel time, the less the more rows an expert has (a row tile's cost is nearly flat below 100
+// rows).  1 / 2 / 3 / 4 / 8 passes, ms: 128 experts of 2880 x 2880, 4096 tokens 2.58 / 2.20 / 2.46 / 2.74 / 3.18; 32 experts, 1500 (187) 0.95 / 0.77 /
+// 0.82 / 0.93 / 1.29, 3000 1.80 / 1.30 / 1.14 / 1.18 / 1.66, 8192 4.76 / 3.39 / 2.97 / 2.76 / 2.49; fp16, 32 of 2880 x 2880, 1500 1.03 / 1.01 / 1.16 / 1.39 /
+// 2.44, 8192 4.98 / 3.47 / 3.02 / 2.80 / 3.14.  From 240 rows on three may be quicker already: the third hides a sixth of both copies and
+// reads the weights once more, with 30 us of launches; the two meet where a copy has 6 MB and a 21st of the weights' bytes.  2 / 3 passes, ms
+// (copy of that sum): 128 of 2880 x 2880, 240 rows 3.32 / 3.23 (1.02), 256 3.47 / 3.33 (1.09); 64, 240 1.69 / 1.69 (0.95), 256 1.78 / 1.75 (1.02), 320
+// 2.17 / 1.97 (1.27); 32, 240 0.87 / 0.91 (0.85), 256 0.91 / 0.94 (0.90), 290 1.02 / 0.98 (1.02), 359 1.24 / 1.11; 8 of 1728 x 1728, 240 0.281 / 0.279 (0.85), 300
+// 0.36 / 0.33 (1.06); 128 of 2048 x 768, top-8, 256 1.23 / 1.10 (1.58); 16 of 2048 x 2880, top-8, 240 0.30 / 0.34 (0.30), 300 0.33 / 0.37; 32 of 1024 x 1024, 240 0.32 /
+// 0.32 (0.92), 300 0.40 / 0.35 (1.15); fp16, 16 of 2048 x 2048, 256 1.12 / 1.07 (1.33); 32 of 2880 x 2880, 300 1.23 / 1.36 (0.34); 1 of 2880 x 2880, 240 0.18 / 0.22 (0.33).  But no more than leave a pass items (a row
 // tile x 128 features) for a third of the SMs: below, its kernels take as long as the whole batch's (one fp16 expert of 2880 x 2880, 150
 // tokens 0.15 / 0.16 / 0.20 / 0.24 / 0.37, 1024 0.56 / 0.46 / 0.42 / 0.43 / 0.50).
 // (Shorter first and last passes were up to 5 % quicker still, but the certified router adds a token's parts in an order that goes
@@ -1755,7 +1759,9 @@ int host_passes(const csk_moe_layer* L, int64_t T, std::initializer_list<const v
   const int least = rows < 256 ? 1 : 2;
   const int tile_rows = tile_rows_for(CSK_PATH_TILE);
   auto items = [&](int passes) { return (rows / passes + tile_rows - 1) / tile_rows * L->Eloc * L->Tgu.n_tiles; };
-  int passes = (int)std::max<int64_t>(rows < 240 ? 2 : 3, std::min<int64_t>(csk_moe_layer::kMaxPasses, rows / 120));
+  int passes = (int)std::max<int64_t>(2, std::min<int64_t>(csk_moe_layer::kMaxPasses, rows / 120));
+  const double weights = (L->w16 ? 2.0 : 17.0 / 32) * 3 * L->H * L->F * L->Eloc;
+  if (rows >= 240 && passes == 2 && (double)sizeof(float) * T * L->H >= 6e6 + weights / 21) passes = 3;
   while (passes > least && 3 * items(passes) < L->sm_count) --passes;
   return passes;
 }

@@ -15,6 +15,8 @@ pytestmark = pytest.mark.gpu
     (64, 64, 12800, False, True, 6400),    # page-locked: two
     (32, 256, 20000, False, False, 10000),  # pageable, 625: two
     (32, 256, 20000, False, True, 4000),   # page-locked: five
+    (80, 64, 20000, False, True, 10000),   # 250 rows, copies of 5 MB: still two ...
+    (96, 64, 24500, False, True, 8167),    # ... and of 6.3 MB: three
     (1, 64, 20000, True, True, 10000),     # one expert without work for more than two
 ])
 def test_passes(gpu_lib, E, F, T, f16, pinned, most):
