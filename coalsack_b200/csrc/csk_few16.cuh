@@ -135,9 +135,7 @@ __global__ void __launch_bounds__(kFewWarps * 32, 2) k_few16(const FewArgs F) {
         const float gate = s[0] + (A.has_bias ? bias[A.F + n] : 0.f), up = s[M - 1] + (A.has_bias ? bias[n] : 0.f);
         A.a_out[(size_t)(rt.row0 + token) * A.lda + n] = __float2half_rn(gated_act_fast(gate, up, A.act));
       } else {
-        const int gr = rt.row0 + token;
-        float* out = A.out_row_ptr ? A.out_row_ptr[gr] : A.y_out + (size_t)(A.out_row_map ? A.out_row_map[gr] : gr) * A.ldy;
-        if (out) out[n] = s[0] + (A.has_bias ? bias[2 * A.F + n] : 0.f);
+        A.y_out[(size_t)(rt.row0 + token) * A.ldy + n] = s[0] + (A.has_bias ? bias[2 * A.F + n] : 0.f);
       }
     }
     rt.row0 += 8 * NT;
@@ -147,7 +145,6 @@ __global__ void __launch_bounds__(kFewWarps * 32, 2) k_few16(const FewArgs F) {
     if (warp < L.k_tiles) load_w(warp, w[0]);
     if (warp + kFewWarps < L.k_tiles) load_w(warp + kFewWarps, w[1]);
   }
-  if (!GATED && A.out_row_ptr) __threadfence_system();  // rows written to other GPUs before the kernel is seen as done
 }
 
 template <bool GATED, bool TURNS>

@@ -574,7 +574,6 @@ struct Batch {
 // weights, where launches and latencies are what is left: 64 of 256 x 512, top-8, 2 (0.37, 11 MB) 22.7 / 20.6, 4 (0.68, 20 MB) 24.2 / 24.7, 8 (1.1, 32 MB)
 // 24.8 / 30.9.
 bool few_rows(const csk_moe_layer* L, const Batch& b) {
-  if (!L->pair.available) return true;  // (in turns of a tile's rows: fp16 layers have no other kernel then)
   if (L->Eloc == 1) return b.tokens <= kFewMaxRows;
   if (b.tokens > kFewMaxRowsRouted) return false;
   if (b.one_expert) return true;
@@ -605,14 +604,9 @@ int launch_experts(csk_moe_layer* L, int path, float* y, int ldy, const int* out
     a.a_out = L->d_a16;
     a.lda = L->lda;
     // (where a token's slots may all name one expert, its rows may need several tiles)
-    const int64_t pairs = std::min(L->max_rows, batch.tokens < L->max_rows ? batch.tokens * L->k : L->max_rows);
-    const bool turns = batch.repeats || batch.tokens > (L->Eloc == 1 ? kFewMaxRows : kFewMaxRowsRouted);
-    const int64_t tiles = std::min(pairs, turns ? L->Eloc + pairs / kPairN : (int64_t)L->Eloc);
-    if (tiles > 65535) return fail(L, CSK_ERR_NOMEM, "more row tiles than a launch takes");
-    const int rows = (int)std::min<int64_t>(batch.tokens, kFewMaxRows);
-    a.out_row_map = out_row_map;
-    a.out_row_ptr = out_row_ptr;
-    CSK_CUDA(L, few_launch_one<true>(f, L->F, (int)tiles, rows, turns, s, L->pdl));
+    const int64_t pairs = batch.tokens * L->k;
+    const int tiles = (int)std::min(pairs, batch.repeats ? L->Eloc + pairs / kPairN : (int64_t)L->Eloc);
+    CSK_CUDA(L, few_launch_one<true>(f, L->F, tiles, (int)batch.tokens, batch.repeats, s, L->pdl));
     tm.mark();
     f.x = L->d_a16;
     f.ldx = L->lda;
@@ -620,7 +614,7 @@ int launch_experts(csk_moe_layer* L, int path, float* y, int ldy, const int* out
     a.L = L->Td;
     a.y_out = y;
     a.ldy = ldy;
-    CSK_CUDA(L, few_launch_one<false>(f, L->H, (int)tiles, rows, turns, s, L->pdl));
+    CSK_CUDA(L, few_launch_one<false>(f, L->H, tiles, (int)batch.tokens, batch.repeats, s, L->pdl));
     tm.mark();
     L->last.launches += 2;
   } else if (path == CSK_PATH_TILE) {

@@ -122,15 +122,6 @@ __global__ void k_rt_pack(const float* __restrict__ wg, uint8_t* __restrict__ ds
   }
 }
 
-// D[tmem] (+)= A[smem] * B[smem]^T, kind::f16
-__device__ __forceinline__ void umma_f16_ss(uint32_t tmem_d, uint64_t da, uint64_t db, uint32_t idesc, uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(tmem_d),
-      "l"(da), "l"(db), "r"(idesc), "r"(accumulate)
-      : "memory");
-}
-
 struct RouterTcArgs {
   const float* hidden;    // [T,H], 16-byte aligned
   const uint8_t* w;       // k_rt_pack's digits
