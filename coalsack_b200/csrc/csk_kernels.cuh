@@ -1285,11 +1285,18 @@ __global__ void __launch_bounds__(256) k_combine(const float* __restrict__ route
 // sequential fp32 chain of separate multiplies and adds, division, square root and products are the
 // IEEE round-to-nearest operations the reference's scalar code performs.
 //
-// A block per token: all its threads square the row into shared memory (and keep it, and its weights, in registers), one walks
-// the squares, 32 columns of them in registers ahead, all of them scale the row.  Bound by that chain, 4.3 cycles a column: 8
-// tokens x 2880 columns 14.1 -> 10.2 us (profiler, cold caches; 16 columns ahead and the row read twice before).
+// A block per token: all its threads square the row into shared memory, one walks the squares, 32 columns of them in registers
+// ahead, all of them scale the row.  Bound by that chain, 4.3 cycles a column.
+//
+// A few tokens: 256 threads, which keep the row and its weights in registers (the rest of a row of more than 4096 columns is
+// read again); 8 tokens x 2880 columns 14.1 -> 10.2 us (profiler, cold caches; 16 columns ahead and the row read twice before).  An SM
+// holds three such blocks, and of many tokens the other chains wait: then 128 threads that read the row twice, twelve blocks.
+// The line is where a fourth block an SM would have to wait, and a little beyond.  256 / 128 threads, what the norm adds to a step, us: 2880
+// columns, 333 tokens 16.4 / 18.8, 444 16.1 / 18.0, 480 22.4 / 17.7, 1200 39 / 29, 2048 52 / 35, 8192 183 / 110; 512, 444 4.8 / 5.1, 480 7.1 / 6.1, 8192
+// 43 / 18; 4096, 444 19.1 / 24.3, 480 31.9 / 24.2, 8192 250 / 143; 8192, 333 47.5 / 44.9, 8192 507 / 348.
 // ---------------------------------------------------------------------------
-constexpr int kNormThreads = 256, kNormKept = 4;  // 4096 columns in registers; the rest of a longer row is read again
+constexpr int kNormThreadsFew = 256, kNormKeptFew = 4, kNormThreadsMany = 128;
+inline bool norm_few(int64_t T, int sm_count) { return 5 * T <= 16 * (int64_t)sm_count; }
 template <int N>
 __device__ __forceinline__ float add_columns(float s, uint32_t at) {
   constexpr int G = N / 4, A = 8;
@@ -1304,14 +1311,16 @@ __device__ __forceinline__ float add_columns(float s, uint32_t at) {
   }
   return s;
 }
-__global__ void __launch_bounds__(kNormThreads) k_rmsnorm(const float* __restrict__ x, const float* __restrict__ w, float eps,
-                                                          float* __restrict__ out, int T, int H) {
+// THREADS of a block, of whose columns KEPT runs of four are in registers
+template <int THREADS, int KEPT>
+__global__ void __launch_bounds__(THREADS) k_rmsnorm(const float* __restrict__ x, const float* __restrict__ w, float eps,
+                                                     float* __restrict__ out, int T, int H) {
   extern __shared__ __align__(16) float rms_sq[];
   __shared__ float s_rms;
-  float4 g[kNormKept];
+  float4 g[KEPT + 1];
 #pragma unroll
-  for (int i = 0; i < kNormKept; ++i) {
-    const int d = (threadIdx.x + i * kNormThreads) * 4;
+  for (int i = 0; i < KEPT; ++i) {
+    const int d = (threadIdx.x + i * THREADS) * 4;
     if (d < H) g[i] = __ldg(reinterpret_cast<const float4*>(w + d));
   }
   griddep_wait();
@@ -1326,18 +1335,18 @@ __global__ void __launch_bounds__(kNormThreads) k_rmsnorm(const float* __restric
           make_float4(__fmul_rn(__fdiv_rn(v.x, rms), f.x), __fmul_rn(__fdiv_rn(v.y, rms), f.y), __fmul_rn(__fdiv_rn(v.z, rms), f.z),
                       __fmul_rn(__fdiv_rn(v.w, rms), f.w));
     };
-    float4 kept[kNormKept];
+    float4 kept[KEPT + 1];
 #pragma unroll
-    for (int i = 0; i < kNormKept; ++i) {
-      const int d = (threadIdx.x + i * kNormThreads) * 4;
+    for (int i = 0; i < KEPT; ++i) {
+      const int d = (threadIdx.x + i * THREADS) * 4;
       if (d < H) kept[i] = __ldg(reinterpret_cast<const float4*>(src + d));
     }
 #pragma unroll
-    for (int i = 0; i < kNormKept; ++i) {
-      const int d = (threadIdx.x + i * kNormThreads) * 4;
+    for (int i = 0; i < KEPT; ++i) {
+      const int d = (threadIdx.x + i * THREADS) * 4;
       if (d < H) square(d, kept[i]);
     }
-    for (int d = (threadIdx.x + kNormKept * kNormThreads) * 4; d < H; d += 4 * kNormThreads) square(d, __ldg(reinterpret_cast<const float4*>(src + d)));
+    for (int d = (threadIdx.x + KEPT * THREADS) * 4; d < H; d += 4 * THREADS) square(d, __ldg(reinterpret_cast<const float4*>(src + d)));
     __syncthreads();
     if (threadIdx.x == 0) {
       const uint32_t at = smem_u32(rms_sq);
@@ -1352,11 +1361,11 @@ __global__ void __launch_bounds__(kNormThreads) k_rmsnorm(const float* __restric
     __syncthreads();
     const float rms = s_rms;
 #pragma unroll
-    for (int i = 0; i < kNormKept; ++i) {
-      const int d = (threadIdx.x + i * kNormThreads) * 4;
+    for (int i = 0; i < KEPT; ++i) {
+      const int d = (threadIdx.x + i * THREADS) * 4;
       if (d < H) scale(d, kept[i], g[i], rms);
     }
-    for (int d = (threadIdx.x + kNormKept * kNormThreads) * 4; d < H; d += 4 * kNormThreads)
+    for (int d = (threadIdx.x + KEPT * THREADS) * 4; d < H; d += 4 * THREADS)
       scale(d, __ldg(reinterpret_cast<const float4*>(src + d)), __ldg(reinterpret_cast<const float4*>(w + d)), rms);
     __syncthreads();  // s_rms and the squares are rewritten for the block's next token
   }

@@ -1596,12 +1596,21 @@ int csk_moe_set_ffn_norm(csk_moe_layer* L, const float* weight, float eps) {
     cudaError_t e = cudaMalloc(&L->d_norm_w, sizeof(float) * L->H);
     if (e == cudaSuccess) e = cudaMalloc(&L->d_normed, sizeof(float) * L->max_T * L->H);
     if (e != cudaSuccess) return fail(L, CSK_ERR_NOMEM, "cudaMalloc failed: %s", cudaGetErrorString(e));
-    CSK_CUDA(L, cudaFuncSetAttribute(k_rmsnorm, cudaFuncAttributeMaxDynamicSharedMemorySize, 50 * 1024));  // any layer's row: the attribute is the function's, not the layer's
+    // any layer's row: the attribute is the function's, not the layer's
+    CSK_CUDA(L, cudaFuncSetAttribute(k_rmsnorm<kNormThreadsFew, kNormKeptFew>, cudaFuncAttributeMaxDynamicSharedMemorySize, 50 * 1024));
+    CSK_CUDA(L, cudaFuncSetAttribute(k_rmsnorm<kNormThreadsMany, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, 50 * 1024));
   }
   CSK_CUDA(L, cudaMemcpyAsync(L->d_norm_w, weight, sizeof(float) * L->H, cudaMemcpyHostToDevice, L->stream));
   CSK_CUDA(L, cudaStreamSynchronize(L->stream));
   L->norm_eps = eps;
   return CSK_OK;
+}
+
+static cudaError_t launch_norm(csk_moe_layer* L, const float* d_x, int64_t T, cudaStream_t s) {
+  const bool few = norm_few(T, L->sm_count);
+  return launch_k(few ? k_rmsnorm<kNormThreadsFew, kNormKeptFew> : k_rmsnorm<kNormThreadsMany, 0>,
+                  dim3((unsigned)std::min<int64_t>(T, 16 * (int64_t)L->sm_count)), dim3(few ? kNormThreadsFew : kNormThreadsMany),
+                  sizeof(float) * L->H, s, !L->timing, d_x, (const float*)L->d_norm_w, L->norm_eps, L->d_normed, (int)T, L->H);
 }
 
 int csk_moe_block_forward_dev(csk_moe_layer* L, const float* d_x, int64_t T, float* d_router_out, float* d_out,
@@ -1615,9 +1624,7 @@ int csk_moe_block_forward_dev(csk_moe_layer* L, const float* d_x, int64_t T, flo
   if ((size_t)L->H * sizeof(float) * 4 > 200 * 1024) return fail(L, CSK_ERR_NOMEM, "hidden dimension too large for the norm kernel's row buffer");
   CSK_CUDA(L, cudaSetDevice(L->cfg.device));
   cudaStream_t s = pick(L, stream);
-  const int blocks = (int)std::min<int64_t>(T, 16 * (int64_t)L->sm_count);
-  launch_k(k_rmsnorm, dim3((unsigned)blocks), dim3(kNormThreads), sizeof(float) * L->H, s, !L->timing, d_x, (const float*)L->d_norm_w, L->norm_eps, L->d_normed, (int)T, L->H);
-  CSK_CUDA(L, cudaGetLastError());
+  CSK_CUDA(L, launch_norm(L, d_x, T, s));
   return forward_dev(L, L->d_normed, T, nullptr, d_router_out, d_out, -1, s, false, d_x);
 }
 
@@ -1644,9 +1651,7 @@ int csk_moe_block_forward_shared_dev(csk_moe_layer* L, csk_moe_layer* S, const f
     if (e != cudaSuccess) return fail(L, CSK_ERR_NOMEM, "shared-expert buffers: %s", cudaGetErrorString(e));
   }
   cudaStream_t s = pick(L, stream);
-  const int blocks = (int)std::min<int64_t>(T, 16 * (int64_t)L->sm_count);
-  launch_k(k_rmsnorm, dim3((unsigned)blocks), dim3(kNormThreads), sizeof(float) * L->H, s, !L->timing, d_x, (const float*)L->d_norm_w, L->norm_eps, L->d_normed, (int)T, L->H);
-  CSK_CUDA(L, cudaGetLastError());
+  CSK_CUDA(L, launch_norm(L, d_x, T, s));
   // the shared expert reads the normed rows on its own stream, next to the routed experts; the combine joins them
   CSK_CUDA(L, cudaEventRecord(L->ev_shared_fork, s));
   CSK_CUDA(L, cudaStreamWaitEvent(S->stream, L->ev_shared_fork, 0));

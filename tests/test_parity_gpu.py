@@ -485,7 +485,8 @@ def test_block_with_norm_and_residual(gpu_lib, port, shape):
     lay.close()
 
 
-@pytest.mark.parametrize("H,T", [(32, 1), (544, 2), (12800, 3), (64, 2500)])  # one batch of squares; ragged; the widest; two rounds
+@pytest.mark.parametrize("H,T", [(32, 1), (544, 2), (12800, 3), (64, 2500),  # one batch of squares; ragged; the widest; two rounds
+                                 (544, 473), (544, 474), (12800, 474)])             # the last batch of large blocks, the first of small ones
 def test_norm_rows_equal_the_reference_bit_for_bit(gpu_lib, port, H, T):
     """The block's result against the plain layer on the checker's normed rows: equal in every bit (one summand)."""
     sh = synth.tiny(seed=53, E=2, k=1, H=H, F=32, T=T, has_bias=True)
