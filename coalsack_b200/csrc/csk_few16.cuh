@@ -1,6 +1,6 @@
 // Grouped contraction over fp16 weights for FEW token rows (the dense FFN and fp16 experts in decode), written for sm_100a.
 //
-// Every weight is read once and meets at most 32 token rows, so its bytes count.  k_pair16 gives a CTA pair 256 weight rows and all of
+// Every weight is read once and meets at most 64 token rows, so its bytes count.  k_pair16 gives a CTA pair 256 weight rows and all of
 // K, which leaves most SMs without work (a 2880 x 2880 matrix is 23 items) and each of the others with one stream.  Here a block
 // of eight warps has 16 weight rows (gate/up: 16 gate and the same features' 16 up rows); its warps take the k-tiles in turn
 // and their sums are added in warp order at the end, so a matrix is some hundred blocks that are all resident at once.
@@ -21,7 +21,8 @@ namespace csk {
 
 constexpr int kFewWarps = 8;
 constexpr int kFewMaxRows = 32;        // tokens of a batch: the layer holds one expert ...
-constexpr int kFewMaxRowsRouted = 16;  // ... or several
+constexpr int kFewMaxRowsWave = 64;    // ... of which all blocks are resident at once, one an SM ...
+constexpr int kFewMaxRowsRouted = 16;  // ... or several experts
 
 inline size_t few_smem_bytes(int groups, bool gated) { return (size_t)kFewWarps * 32 * 4 * groups * (gated ? 2 : 1) * sizeof(float); }
 
@@ -41,9 +42,9 @@ struct FewArgs {
 // NT = groups of eight token rows.  blockIdx.x: 16 weight rows (features), blockIdx.y: row tile.  TURNS: the tile may have more
 // than 8 NT rows, which are taken 8 NT after another (the loop's registers cost the others up to 5 %: 128 experts of 2048 x 768, 16
 // tokens of eight slots 224 -> 236 us).
-// Two blocks an SM (in 128 registers; three blocks of 80 were slower, 62 -> 70 us for a block of 5 tokens).
+// Two blocks an SM up to 32 rows (in 128 registers; three blocks of 80 were slower, 62 -> 70 us for a block of 5 tokens).
 template <bool GATED, int NT, bool TURNS>
-__global__ void __launch_bounds__(kFewWarps * 32, 2) k_few16(const FewArgs F) {
+__global__ void __launch_bounds__(kFewWarps * 32, NT <= 4 ? 2 : 1) k_few16(const FewArgs F) {
   extern __shared__ float few_sums[];
   const TileArgs& A = F.t;
   const TileLayout& L = A.L;
@@ -149,13 +150,14 @@ __global__ void __launch_bounds__(kFewWarps * 32, 2) k_few16(const FewArgs F) {
 
 template <bool GATED, bool TURNS>
 inline cudaError_t few_launch_turns(const FewArgs& f, int features, int tiles, int rows, cudaStream_t s, bool pdl) {
-  const int groups = rows <= 8 ? 1 : rows <= 16 ? 2 : 4;
+  const int groups = rows <= 8 ? 1 : rows <= 16 ? 2 : rows <= 32 || TURNS ? 4 : 8;
   const dim3 grid((unsigned)(features / 16), (unsigned)tiles), block(kFewWarps * 32);
   const size_t smem = few_smem_bytes(groups, GATED);
   switch (groups) {
     case 1: return launch_k(k_few16<GATED, 1, TURNS>, grid, block, smem, s, pdl, f);
     case 2: return launch_k(k_few16<GATED, 2, TURNS>, grid, block, smem, s, pdl, f);
-    default: return launch_k(k_few16<GATED, 4, TURNS>, grid, block, smem, s, pdl, f);
+    case 4: return launch_k(k_few16<GATED, 4, TURNS>, grid, block, smem, s, pdl, f);
+    default: return launch_k(k_few16<GATED, TURNS ? 4 : 8, TURNS>, grid, block, smem, s, pdl, f);
   }
 }
 
@@ -164,6 +166,10 @@ template <bool GATED>
 inline cudaError_t few_launch_one(const FewArgs& f, int features, int tiles, int rows, bool repeats, cudaStream_t s, bool pdl) {
   return repeats ? few_launch_turns<GATED, true>(f, features, tiles, rows, s, pdl)
                  : few_launch_turns<GATED, false>(f, features, tiles, rows, s, pdl);
+}
+
+inline cudaError_t few_prepare_device() {
+  return cudaFuncSetAttribute(k_few16<true, 8, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)few_smem_bytes(8, true));
 }
 
 }  // namespace csk

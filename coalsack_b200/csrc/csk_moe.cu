@@ -565,7 +565,9 @@ struct Batch {
 
 // fp16 weights: the kernel for few rows (csk_few16.cuh) takes a batch of so many tokens.  The weights' bytes are all that counts
 // there.  Step, k_pair16 / k_few16, us: dense FFN of 2880 x 2880 (weights in L2) 1 token 26.8 / 14.4, 16 27.8 / 16.5, 32 28.4 / 24.7, 48 28.8 /
-// 40.1; 2048 x 8192 16 43.4 / 29.3, 24 44.7 / 43.7, 32 45.0 / 46.9; 512 x 512 32 12.5 / 10.4.
+// 40.1; 2048 x 8192 16 43.4 / 29.3, 24 44.7 / 43.7, 32 45.0 / 46.9; 512 x 512 32 12.5 / 10.4.  Of 33 to 64 rows a block has an SM to itself, and a
+// second round of blocks costs more than it saves: 33 and 64 rows, 256 x 256 12.4 / 10.3 and 12.4 / 10.3, 1024 x 1024 16.5 / 14.4 and 16.5 / 14.8, 2368 x
+// 2368 (148 blocks) 26.7 / 20.6 and 26.4 / 22.7, 2400 x 2400 24.7 / 32.9 and 26.3 / 36.1, 2048 x 2880 26.7 / 27.2 and 26.7 / 29.8.
 // Of several experts its time goes by the row tiles, most of which hold a row or two, k_pair16's by the rounds of its items (128
 // features of an expert) on the SMs.  The line is half an item per SM, for evenly spread routing (in brackets): 16 of 2048 x 2048, top-1, 1 token
 // (0.11) 36.0 / 25.6, 5 (0.47) 51.3 / 51.3, 16 (1.1) 70.8 / 81.5; top-2, 1 (0.22) 37.0 / 28.3, 4 (0.70) 55.2 / 61.7; top-4, 1 (0.39) 42.0 / 41.6;
@@ -574,7 +576,7 @@ struct Batch {
 // weights, where launches and latencies are what is left: 64 of 256 x 512, top-8, 2 (0.37, 11 MB) 22.7 / 20.6, 4 (0.68, 20 MB) 24.2 / 24.7, 8 (1.1, 32 MB)
 // 24.8 / 30.9.
 bool few_rows(const csk_moe_layer* L, const Batch& b) {
-  if (L->Eloc == 1) return b.tokens <= kFewMaxRows;
+  if (L->Eloc == 1) return b.tokens <= (std::max(L->F, L->H) / 16 <= L->sm_count ? kFewMaxRowsWave : kFewMaxRows);
   if (b.tokens > kFewMaxRowsRouted) return false;
   if (b.one_expert) return true;
   const double hit = L->Eloc * (1.0 - std::pow(1.0 - 1.0 / L->E, (double)(b.tokens * L->k)));
@@ -938,6 +940,7 @@ int csk_moe_create(const csk_moe_config* cfg, csk_moe_layer** out) {
   CK(router_prepare_device());
   for (int g = 1; g <= kMaxExperts / 32; ++g) L->router_waves[g] = router_wave(g, L->sm_count);
   CK(mx_prepare_device());
+  CK(few_prepare_device());
   CK(rt_prepare_device());
   {
     int rc = tile_init(L->tile, cfg->device);

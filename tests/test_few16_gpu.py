@@ -15,6 +15,7 @@ pytestmark = pytest.mark.gpu
     (32, 96, True),       # one k-tile of which half is padding: seven of eight warps idle
     (544, 160, False),    # nine k-tiles (the warps' second turn) and three
     (1088, 2080, True),   # seventeen and thirty-three: the third and fifth turn
+    (96, 2368, True), (2400, 64, False),  # the most blocks that are resident at once with more than 32 rows, and too many
 ])
 def test_dense(gpu_lib, port, H, F, bias, T):
     hidden, gw, uw, dw, bg, bu, bd = cases.dense_ffn_case(H=H, F=F, T=T, bias=True, seed=700 + T)
