@@ -83,34 +83,47 @@ __device__ __forceinline__ bool warp_topk_regs(float (&v)[NV], int E, int k, int
   float my_v = -INFINITY;
   int my_i = 0x7fffffff;
   uint32_t gone = 0;
+  // With many logits a lane, its best is looked for again only when it was selected (1024 experts of 512 columns, 100 tokens 44.3 -> 37.1 us, 511
+  // 78.0 -> 69.9; with eight a lane the branch costs as much).
+  constexpr bool kKeepBest = NV > 16;
+  float lane_v = -INFINITY;
+  int lane_i = 0x7fffffff;
+  bool look = true;
 #pragma unroll 1
   for (int j = 0; j < k; ++j) {
-    float bv = -INFINITY;
-    int bi = 0x7fffffff;
+    if (!kKeepBest || look) {
+      lane_v = -INFINITY;
+      lane_i = 0x7fffffff;
 #pragma unroll
-    for (int i = 0; i < NV; ++i) {
-      if (i * 32 < E) {  // warp-uniform
-        const float x = v[i];
-        if (x > bv) {  // ascending expert id within the lane: '>' keeps the lowest on ties
-          bv = x;
-          bi = i * 32 + lane;
+      for (int i = 0; i < NV; ++i) {
+        if (i * 32 < E) {  // warp-uniform
+          const float x = v[i];
+          if (x > lane_v && !(kKeepBest && (gone >> i & 1u))) {  // ascending expert id within the lane: '>' keeps the lowest on ties
+            lane_v = x;
+            lane_i = i * 32 + lane;
+          }
         }
       }
     }
     // the lanes' bests as integers of the same order (both zeros alike), the lowest id of those that reach the maximum
-    const uint32_t bits = __float_as_uint(bv + 0.f), key = bits ^ ((int)bits < 0 ? 0xffffffffu : 0x80000000u);
+    const uint32_t bits = __float_as_uint(lane_v + 0.f), key = bits ^ ((int)bits < 0 ? 0xffffffffu : 0x80000000u);
     const uint32_t top = __reduce_max_sync(0xffffffffu, key);
-    bi = (int)__reduce_min_sync(0xffffffffu, key == top ? (uint32_t)bi : 0x7fffffffu);
-    bv = __shfl_sync(0xffffffffu, bv, bi & 31);  // (nothing to choose from: -inf in every lane)
+    const int bi = (int)__reduce_min_sync(0xffffffffu, key == top ? (uint32_t)lane_i : 0x7fffffffu);
+    const float bv = __shfl_sync(0xffffffffu, lane_v, bi & 31);  // (nothing to choose from: -inf in every lane)
     if (lane == j) {
       my_v = bv;
       my_i = bi;
     }
-    // the winner leaves the pool: NaN never wins a '>' test again
+    // the winner leaves the pool
+    look = bi == lane_i && bi != 0x7fffffff;
+    if (kKeepBest) {
+      if (look) gone |= 1u << (bi >> 5);
+      continue;
+    }
 #pragma unroll
     for (int i = 0; i < NV; ++i)
       if (i * 32 < E && bi == i * 32 + lane) {
-        v[i] = __int_as_float(0xffc00000);
+        v[i] = __int_as_float(0xffc00000);  // NaN never wins a '>' test again
         gone |= 1u << i;
       }
   }
@@ -169,6 +182,7 @@ __device__ __forceinline__ bool warp_topk(const float* __restrict__ l, int E, in
   if (E <= 64) return warp_topk_nv<CG, 2>(l, E, k, sigmoid, out, bounds);
   if (E <= 128) return warp_topk_nv<CG, 4>(l, E, k, sigmoid, out, bounds);
   if (E <= 256) return warp_topk_nv<CG, 8>(l, E, k, sigmoid, out, bounds);
+  if (E <= 512) return warp_topk_nv<CG, 16>(l, E, k, sigmoid, out, bounds);
   return warp_topk_nv<CG, kMaxExperts / 32>(l, E, k, sigmoid, out, bounds);
 }
 
