@@ -592,9 +592,11 @@ inline void launch_router_logits(RouterArgs a, const float* wg_few, const float*
   if (token_slots < 0) token_slots = a.T;
   const int64_t groups = (a.E + 31) / 32;
   auto one_wave = [&](int tokens) { return (token_slots + tokens - 1) / tokens * groups <= wave.blocks; };
-  if (wave.clusters && !one_wave(32)) {
-    // The SMs that clusters leave over may be what the last wave needs: without clusters then.  2880 columns, with / without: 256 experts
-    // (120 blocks at once / 148), 511 tokens 94.3 / 54.5 us, 1000 139.5 / 99.0; 224 experts, 560 tokens 94.3 / 55.0.
+  if (wave.clusters && !one_wave(32) && a.H > 256) {
+    // The SMs that clusters leave over may be what the last wave needs: without clusters then, unless a chain is so short that the
+    // selection in one block per token block takes as long.  With / without, us: 2880 columns, 256 experts (120 blocks at once / 148), 511 tokens
+    // 94.3 / 54.5, 1000 139.5 / 99.0; 224 experts, 560 tokens 94.3 / 55.0; 256 experts, 511 tokens, 1024 columns 43.2 / 30.9, 512 28.9 / 24.8, 128
+    // 16.7 / 18.6.
     const int64_t blocks = (token_slots + 31) / 32 * groups;
     if ((blocks + wave.alone - 1) / wave.alone < (blocks + wave.blocks - 1) / wave.blocks) wave = {wave.alone, false, wave.alone};
   }

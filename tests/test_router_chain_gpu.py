@@ -71,7 +71,7 @@ def test_a_handful_of_tokens_that_cannot_be_separated(gpu_lib, port, E, H, T):
 
 
 @pytest.mark.parametrize("E,H,T", [(33, 256, 3), (64, 288, 64), (128, 2880, 1), (128, 256, 333), (128, 160, 1100), (256, 1056, 40), (256, 96, 2000),
-                                   (256, 160, 480), (256, 160, 481), (224, 96, 585)])  # (the last batches of one wave of clusters, the first of one without)
+                                   (256, 288, 480), (256, 288, 481), (256, 256, 481), (224, 288, 585)])  # (the last batches of one wave of clusters, the first of one without)
 def test_the_same_without_clusters(gpu_lib, E, H, T):
     """Where no cluster can be resident the groups of experts of a token block meet in global memory: the same routing bit for bit, of the
     chain and of the certified pass with its list."""
