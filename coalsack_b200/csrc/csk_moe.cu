@@ -205,6 +205,13 @@ int grid_for(size_t work_items, int threads, int cap) {
 
 cudaStream_t pick(csk_moe_layer* L, void* s) { return s ? (cudaStream_t)s : L->stream; }
 
+// Launches of the handle are programmatic dependents for as long as this lives (unless they are timed one by one).
+struct PdlScope {
+  csk_moe_layer* L;
+  explicit PdlScope(csk_moe_layer* l) : L(l) { L->pdl = !L->timing; }
+  ~PdlScope() { L->pdl = false; }
+};
+
 struct StageTimer {
   csk_moe_layer* L;
   cudaStream_t s;
@@ -687,11 +694,7 @@ int forward_dev(csk_moe_layer* L, const float* d_hidden, int64_t T, const float*
   L->last_T = T;
   if (!L->carry_active) L->counts_in_carry = false;
   // each kernel may become resident while its predecessor drains
-  struct PdlScope {
-    csk_moe_layer* l;
-    ~PdlScope() { l->pdl = false; }
-  } pdl_scope{L};
-  L->pdl = !L->timing;
+  const PdlScope pdl_scope(L);
   StageTimer tm(L, s);
   tm.mark();
   const float* router = d_router_in;
@@ -1963,6 +1966,7 @@ int csk_moe_ep_dispatch_dev(csk_moe_layer* L, const float* d_hidden, int64_t T, 
   if (reinterpret_cast<uintptr_t>(d_send_f16) % 8) return fail(L, CSK_ERR_INVALID, "the rows to send must be 8-byte aligned");
   CSK_CUDA(L, cudaSetDevice(L->cfg.device));
   cudaStream_t s = pick(L, stream);
+  const PdlScope pdl_scope(L);  // (the kernels are those of a layer's plan)
   L->last = csk_moe_timings{};
   L->last_T = T;
   if (!d_router_in) {

@@ -39,7 +39,7 @@ def _f16(E, k, H, F, T):
     (_f16, 4, 2, 700),       # fp16 weights on CTA pairs
     (_f16, 1, 1, 600),
 ])
-@pytest.mark.parametrize("entry", ["layer", "given", "block", "dense"])
+@pytest.mark.parametrize("entry", ["layer", "given", "block", "dense", "sent"])
 def test_calls_behind_one_another(gpu_lib, make, E, k, T, entry):
     if entry == "dense" and E > 1:
         pytest.skip("the dense entry takes layers of one expert")
@@ -53,6 +53,8 @@ def test_calls_behind_one_another(gpu_lib, make, E, k, T, entry):
     for r in routes:
         r[..., 0] = torch.rand(T, E, device="cuda", generator=g).argsort(1)[:, :k].float()
     ro = torch.empty(T, k, 2, device="cuda")
+    send, back = torch.zeros(T * k, lay.ep_row_pitch(), dtype=torch.float16, device="cuda"), torch.empty(T * k, H, device="cuda")
+    counts = torch.empty(E, dtype=torch.int32, device="cuda")
     tokens = [T, T - 1, T, T // 2 + 200, T, T - 33]
 
     def call(i, x, out):
@@ -62,8 +64,12 @@ def test_calls_behind_one_another(gpu_lib, make, E, k, T, entry):
             lay.forward_dev(x, tokens[i], out, d_router_in=routes[i])
         elif entry == "block":
             lay.block_forward_dev(x, tokens[i], ro, out)
-        else:
+        elif entry == "dense":
             lay.dense_forward_dev(x, tokens[i], out)
+        else:  # the expert-parallel stages of one rank
+            lay.ep_dispatch_dev(x, tokens[i], send, counts, d_router_in=routes[i] if i % 2 else None)
+            lay.ep_experts_dev(send, counts, 1, tokens[i] * k, back)
+            lay.ep_combine_dev(back, tokens[i], out)
 
     def run(wait, chained):
         outs = [torch.zeros(T, H, device="cuda") for _ in range(CALLS)]
