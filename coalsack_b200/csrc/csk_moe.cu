@@ -1770,6 +1770,18 @@ int host_passes(const csk_moe_layer* L, int64_t T, std::initializer_list<const v
   while (passes > least && 3 * items(passes) < L->sm_count) --passes;
   return passes;
 }
+// Whether a pass's results start on their way with the copy in of the pass after next (all copies in are enqueued in front then).  A copy
+// out that starts in the middle of a copy in leaves the two some 65 GB/s between them, where both starting together have 80: in passes of 4
+// to 12 MB that is worth the wait (smaller ones are over too soon, larger ones wait too long) if the kernels take less than a third of a
+// copy's time (they take about 7.5e-5 k F of it).  At once / in step, ms (MB of a pass, k F): 8 experts of 1728 x 1024, top-4, 8192 tokens in 8 passes 1.69 / 1.48
+// (7.1, 4096); 8 of 2048 x 1024, top-1, 8192 in 8 1.87 / 1.71 (8.4, 1024), 4096 in 4 1.02 / 1.00; 8 of 1024 x 2048, top-1, 8192 in 8 1.13 / 0.95 (4.2, 2048),
+// 4096 in 4 0.61 / 0.54; 16 of 2048 x 2048, top-2, 4096 in 4 1.06 / 1.02 (8.4, 4096); fp16, 1 of 2880 x 2880, 4096 in 7 1.43 / 1.31 (6.7, 2880); but 8 of 512 x 512, 8192 in
+// 8 0.53 / 0.59 (2.1); 16 of 2880 x 1024, top-1, 8192 in 4 2.51 / 2.69 (23.6); 16 of 2880 x 768, top-8, 4096 in 8 1.26 / 1.29 (5.9, 6144); 32 of 2880 x 2880, top-4, 8192
+// in 8 2.39 / 2.44 (11.8, 11520).
+bool copies_in_step(const csk_moe_layer* L, int64_t T, int passes) {
+  const double mb = 1e-6 * sizeof(float) * T * L->H / passes;
+  return passes >= 4 && mb >= 4 && mb <= 12 && (int64_t)L->k * L->F <= 4096;
+}
 }  // namespace
 
 int csk_moe_forward(csk_moe_layer* L, const float* hidden, int64_t T, const float* router_in,
@@ -1838,16 +1850,23 @@ int csk_moe_forward(csk_moe_layer* L, const float* hidden, int64_t T, const floa
   } carry_scope{L};
   L->carry_active = true;
   const int k2 = L->k * 2;
-  int rc = CSK_OK;
-  for (int p = 0; p < passes && !rc; ++p) {
-    const int64_t t0 = T * p / passes, t1 = T * (p + 1) / passes, n = t1 - t0;
-
+  auto copy_in = [&](int p) -> int {
+    const int64_t t0 = T * p / passes, n = T * (p + 1) / passes - t0;
     CSK_CUDA(L, cudaMemcpyAsync(L->d_hidden + t0 * L->H, hidden + t0 * L->H, sizeof(float) * n * L->H,
                                 cudaMemcpyHostToDevice, L->stream_in));
     if (router_in)
       CSK_CUDA(L, cudaMemcpyAsync(L->d_router + t0 * k2, router_in + t0 * k2, sizeof(float) * n * k2,
                                   cudaMemcpyHostToDevice, L->stream_in));
     CSK_CUDA(L, cudaEventRecord(L->ev_in[p], L->stream_in));
+    return CSK_OK;
+  };
+  const bool in_step = copies_in_step(L, T, passes);
+  int rc = CSK_OK;
+  for (int p = 0; in_step && p < passes && !rc; ++p) rc = copy_in(p);
+  for (int p = 0; p < passes && !rc; ++p) {
+    const int64_t t0 = T * p / passes, t1 = T * (p + 1) / passes, n = t1 - t0;
+    if (!in_step) rc = copy_in(p);
+    if (rc) break;
     CSK_CUDA(L, cudaStreamWaitEvent(s, L->ev_in[p], 0));
     // the router writes the pass's routing to its place in d_router (kept for router_out and for the counters)
     rc = forward_dev(L, L->d_hidden + t0 * L->H, n, router_in ? L->d_router + t0 * k2 : nullptr,
@@ -1855,6 +1874,7 @@ int csk_moe_forward(csk_moe_layer* L, const float* hidden, int64_t T, const floa
     if (rc) break;
     CSK_CUDA(L, cudaEventRecord(L->ev_done[p], s));
     CSK_CUDA(L, cudaStreamWaitEvent(L->stream_out, L->ev_done[p], 0));
+    if (in_step && p + 1 < passes) CSK_CUDA(L, cudaStreamWaitEvent(L->stream_out, L->ev_in[p + 1], 0));
     CSK_CUDA(L, cudaMemcpyAsync(out + t0 * L->H, L->d_out + t0 * L->H, sizeof(float) * n * L->H,
                                 cudaMemcpyDeviceToHost, L->stream_out));
     if (router_out)

@@ -5,7 +5,7 @@ import numpy as np
 import pytest
 import torch
 
-from coalsack_b200 import MoeLayer
+from coalsack_b200 import CskError, MoeLayer
 
 pytestmark = pytest.mark.gpu
 
@@ -52,4 +52,35 @@ def test_passes(gpu_lib, E, F, T, f16, pinned, most):
     lay.forward_dev(hidden.cuda(), T, got, d_router_in=route.cuda())
     lay.sync()
     assert torch.equal(got.cpu(), o)
+    lay.close()
+
+
+def test_copies_in_step(gpu_lib):
+    """Eight passes of 4.2 MB of a layer whose copies are all there is: the copies in go first, and every copy out waits for one of them."""
+    E, k, H, F, T = 8, 2, 512, 64, 16384
+    rng = np.random.default_rng(3)
+    lay = MoeLayer(E, k, H, F, activation=1, has_bias=False, max_tokens=T)
+    for e in range(E):
+        b = [np.full((F * H // 32, 17), 120, np.uint8) for _ in range(3)]
+        for m in b:
+            m[:, 1:] = rng.integers(0, 256, m[:, 1:].shape)
+        lay.load_expert(e, *(m.reshape(-1) for m in b))
+    hidden = torch.from_numpy(rng.standard_normal((T, H)).astype(np.float32)).pin_memory()
+    route = torch.rand(T, k, 2)
+    route[..., 0] = torch.rand(T, E).argsort(1)[:, :k].float()
+    route = route.pin_memory()
+    want = torch.empty(T, H, device="cuda")
+    lay.forward_dev(hidden.cuda(), T, want, d_router_in=route.cuda())
+    lay.sync()
+    out, routed = torch.zeros(T, H).pin_memory(), torch.zeros(T, k, 2).pin_memory()
+    for _ in range(2):
+        out.zero_()
+        lay.forward(hidden.numpy(), router_out=route.numpy(), out=out.numpy(), router_out_buf=routed.numpy())
+        assert torch.equal(out, want.cpu()) and torch.equal(routed, route)
+    bad = route.clone().pin_memory()
+    bad[T - 1, 1, 0] = E
+    with pytest.raises(CskError, match="out of range"):
+        lay.forward(hidden.numpy(), router_out=bad.numpy(), out=out.numpy(), router_out_buf=routed.numpy())
+    lay.forward(hidden.numpy(), router_out=route.numpy(), out=out.numpy(), router_out_buf=routed.numpy())
+    assert torch.equal(out, want.cpu())
     lay.close()
