@@ -174,7 +174,9 @@ __device__ __forceinline__ bool warp_topk_nv(const float* __restrict__ l, int E,
   return warp_topk_regs<CG, NV>(v, E, k, sigmoid, out, bounds);
 }
 
-template <bool CG = true>
+// SHORT: a kernel of a few microseconds, whose code counts: 257 to 512 experts take the form of 1024 (the router of one token of 64 and
+// 128 experts 16.5 -> 15.6 us, cold code)
+template <bool CG = true, bool SHORT = false>
 __device__ __forceinline__ bool warp_topk(const float* __restrict__ l, int E, int k, int sigmoid,
                                           float* __restrict__ out /* [k][2] */,
                                           const float* __restrict__ bounds = nullptr) {
@@ -182,7 +184,7 @@ __device__ __forceinline__ bool warp_topk(const float* __restrict__ l, int E, in
   if (E <= 64) return warp_topk_nv<CG, 2>(l, E, k, sigmoid, out, bounds);
   if (E <= 128) return warp_topk_nv<CG, 4>(l, E, k, sigmoid, out, bounds);
   if (E <= 256) return warp_topk_nv<CG, 8>(l, E, k, sigmoid, out, bounds);
-  if (E <= 512) return warp_topk_nv<CG, 16>(l, E, k, sigmoid, out, bounds);
+  if (!SHORT && E <= 512) return warp_topk_nv<CG, 16>(l, E, k, sigmoid, out, bounds);
   return warp_topk_nv<CG, kMaxExperts / 32>(l, E, k, sigmoid, out, bounds);
 }
 
@@ -828,7 +830,7 @@ __global__ void __launch_bounds__(256) k_router_finish(const FinishRouterArgs A)
   }
   __syncthreads();
   if (threadIdx.x >= 32) return;
-  const bool sure = warp_topk<false>(s_logit, E, A.k, A.sigmoid, A.router_out + (size_t)t * A.k * 2, s_bound);
+  const bool sure = warp_topk<false, true>(s_logit, E, A.k, A.sigmoid, A.router_out + (size_t)t * A.k * 2, s_bound);
   if (!sure && lane == 0) A.fb_list[atomicAdd(A.fb_count, 1)] = t;  // at most one entry per token
 }
 
