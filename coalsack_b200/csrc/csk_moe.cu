@@ -1535,6 +1535,7 @@ int csk_moe_route_dev(csk_moe_layer* L, const float* d_hidden, int64_t T, float*
   if (T <= 0 || T > L->max_T) return fail(L, CSK_ERR_NOMEM, "T=%lld outside (0, max_tokens]", (long long)T);
   CSK_CUDA(L, cudaSetDevice(L->cfg.device));
   L->last = csk_moe_timings{};
+  const PdlScope pdl_scope(L);
   return launch_router(L, d_hidden, T, d_router_out, pick(L, stream));
 }
 
@@ -1716,6 +1717,7 @@ int csk_moe_route(csk_moe_layer* L, const float* hidden, int64_t T, float* route
   cudaStream_t s = L->stream;
   L->last = csk_moe_timings{};
   CSK_CUDA(L, cudaMemcpyAsync(L->d_hidden, hidden, sizeof(float) * T * L->H, cudaMemcpyHostToDevice, s));
+  const PdlScope pdl_scope(L);
   int rc = launch_router(L, L->d_hidden, T, L->d_router, s);
   if (rc) return rc;
   CSK_CUDA(L, cudaMemcpyAsync(router_out, L->d_router, sizeof(float) * T * L->k * 2, cudaMemcpyDeviceToHost, s));

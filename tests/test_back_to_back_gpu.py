@@ -88,3 +88,24 @@ def test_calls_behind_one_another(gpu_lib, make, E, k, T, entry):
             for i, (a, b) in enumerate(zip(run(False, chained), want)):
                 assert torch.equal(a, b), (chained, i, (a != b).any(1).sum().item())
     lay.close()
+
+
+@pytest.mark.parametrize("E,T", [(8, 3), (128, 4), (128, 64), (64, 2100), (300, 40)])
+def test_routings_behind_one_another(gpu_lib, E, T):
+    lay = MoeLayer(E, 4, 256, 32, has_bias=False, max_tokens=T)
+    rng = np.random.default_rng(E + T)
+    lay.set_router((rng.standard_normal((E, 256)) * 0.1).astype(np.float32), None)
+    xs = [torch.from_numpy(rng.standard_normal((T, 256)).astype(np.float32)).cuda() for _ in range(CALLS)]
+    for x in xs:
+        x[::2] = x[0]  # (and rows that repeat)
+    want, got = ([torch.zeros(T, 4, 2, device="cuda") for _ in range(CALLS)] for _ in range(2))
+    torch.cuda.synchronize()
+    for x, r in zip(xs, want):
+        lay.route_dev(x, T, r)
+        torch.cuda.synchronize()
+    for _ in range(3):
+        for x, r in zip(xs, got):
+            lay.route_dev(x, T, r)
+        torch.cuda.synchronize()
+        assert all(torch.equal(a, b) for a, b in zip(got, want))
+    lay.close()
