@@ -27,6 +27,7 @@ constexpr int kRouterChunkFew = 256, kRouterChunkMany = 128;
 __host__ __device__ constexpr int router_stages(int ch) { return ch > 128 ? 3 : 4; }
 constexpr int kMaxTopK = 16;
 constexpr int kMaxExperts = 1024;
+constexpr int kRouterClusterGroups = 8;  // groups of 32 experts up to which their blocks form a cluster (the portable size)
 
 // ch = columns of the hidden dimension per pipeline stage; experts: of the logits that the blocks of a cluster exchange (twice), 0 without one
 inline size_t router_smem_bytes(int tokens_per_block, int ch, int experts) {
@@ -174,17 +175,17 @@ __device__ __forceinline__ bool warp_topk_nv(const float* __restrict__ l, int E,
   return warp_topk_regs<CG, NV>(v, E, k, sigmoid, out, bounds);
 }
 
-// SHORT: a kernel of a few microseconds, whose code counts: 257 to 512 experts take the form of 1024 (the router of one token of 64 and
-// 128 experts 16.5 -> 15.6 us, cold code)
-template <bool CG = true, bool SHORT = false>
+// MAX_E: of the experts there may be.  Code that is never run makes kernels of a few microseconds longer: with the forms of 512 and 1024 experts the
+// router of one token of 64 experts took 16.5 us, not 15.6 (cold code).
+template <bool CG = true, int MAX_E = kMaxExperts, bool FORM_512 = true>
 __device__ __forceinline__ bool warp_topk(const float* __restrict__ l, int E, int k, int sigmoid,
                                           float* __restrict__ out /* [k][2] */,
                                           const float* __restrict__ bounds = nullptr) {
   if (E <= 32) return warp_topk_nv<CG, 1>(l, E, k, sigmoid, out, bounds);
   if (E <= 64) return warp_topk_nv<CG, 2>(l, E, k, sigmoid, out, bounds);
   if (E <= 128) return warp_topk_nv<CG, 4>(l, E, k, sigmoid, out, bounds);
-  if (E <= 256) return warp_topk_nv<CG, 8>(l, E, k, sigmoid, out, bounds);
-  if (!SHORT && E <= 512) return warp_topk_nv<CG, 16>(l, E, k, sigmoid, out, bounds);
+  if (MAX_E <= 256 || E <= 256) return warp_topk_nv<CG, 8>(l, E, k, sigmoid, out, bounds);
+  if (FORM_512 && E <= 512) return warp_topk_nv<CG, 16>(l, E, k, sigmoid, out, bounds);
   return warp_topk_nv<CG, kMaxExperts / 32>(l, E, k, sigmoid, out, bounds);
 }
 
@@ -469,7 +470,7 @@ k_router_logits(const RouterArgs A) {
       const int t = token_at(t0 + j);
       if (t < 0) continue;
       float* const to = A.router_out + (size_t)t * A.k * 2;
-      if (A.cluster) warp_topk<false>(exchanged + ((size_t)(iter & 1) * BT + j) * E, E, A.k, A.sigmoid, to);
+      if (A.cluster) warp_topk<false, 32 * kRouterClusterGroups>(exchanged + ((size_t)(iter & 1) * BT + j) * E, E, A.k, A.sigmoid, to);
       else warp_topk(A.logits + (size_t)t * E, E, A.k, A.sigmoid, to);
     }
     if (!A.cluster) __syncthreads();  // `ticket` is rewritten by the next token block
@@ -501,7 +502,6 @@ k_router_logits(const RouterArgs A) {
   }
 }
 
-constexpr int kRouterClusterGroups = 8;  // groups of 32 experts up to which their blocks form a cluster (the portable size)
 template <int TW, int TT, int CH, bool PACKED>
 cudaError_t router_prepare_one() {
   return cudaFuncSetAttribute(k_router_logits<TW, TT, CH, PACKED>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -830,7 +830,7 @@ __global__ void __launch_bounds__(256) k_router_finish(const FinishRouterArgs A)
   }
   __syncthreads();
   if (threadIdx.x >= 32) return;
-  const bool sure = warp_topk<false, true>(s_logit, E, A.k, A.sigmoid, A.router_out + (size_t)t * A.k * 2, s_bound);
+  const bool sure = warp_topk<false, kMaxExperts, false>(s_logit, E, A.k, A.sigmoid, A.router_out + (size_t)t * A.k * 2, s_bound);
   if (!sure && lane == 0) A.fb_list[atomicAdd(A.fb_count, 1)] = t;  // at most one entry per token
 }
 
