@@ -957,16 +957,17 @@ __global__ void k_hist(const float* __restrict__ router_out, int n_pairs, int E,
   if (threadIdx.x == 0 && sc[E]) atomicOr(&meta[3], kDevErrExpertRange);
 }
 
-// An expert with several tiles gets them equally tall instead of full ones and a short rest: for the block-scaled
-// kernel always (its time goes by the tile's rows), for the fp16 tensor-core kernel (rounded up to the MMA's 16-row
-// step) with two to four tiles -- a tile's cost is nearly flat below ~175 rows, so 128 + 128 rows are cheaper than
-// 192 + 64, and with more tiles only the last one would change.
+// An expert with several tiles gets them equally tall instead of full ones and a short rest: for the block-scaled kernel always (its
+// time goes by the tile's rows), for the CTA-pair kernels, whose tiles of 256 rows take MMAs of a multiple of 32, with two to four
+// tiles (with more only the last one would change).  Full and rest / even, us: 8 experts of 2880 x 2880 (MXFP4) with 257 rows each 141 / 111, 330
+// 147 / 127, 480 166 / 166, 513 224 / 184, 800 292 / 269, 1000 326 / 326; 32 experts 257 rows 452 / 397, 480 617 / 616 (637 with heights of a multiple of
+// 16), 700 892 / 897 (955); fp16, one of 2880 x 2880, 257 43.8 / 33.5, 480 45.0 / 45.0, 800 54.0 / 51.5.
 __device__ __forceinline__ int even_tile_height(int cnt, int tile_rows, bool block_scaled) {
   const int ntl = (cnt + tile_rows - 1) / tile_rows;
   if (ntl < 2) return tile_rows;
   const int even = (cnt + ntl - 1) / ntl;
   if (block_scaled) return even;
-  return tile_rows >= 64 && ntl <= 4 ? min(tile_rows, (even + 15) & ~15) : tile_rows;
+  return tile_rows >= 64 && ntl <= 4 ? min(tile_rows, (even + 31) & ~31) : tile_rows;
 }
 
 // Exclusive scan of the per-expert row counts, row-tile list for tiles of

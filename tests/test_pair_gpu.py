@@ -17,7 +17,7 @@ def row_tiles(rows):
     out = []
     for r in rows:
         n = -(-r // 256)
-        per = min(256, (-(-r // n) + 15) // 16 * 16) if 2 <= n <= 4 else 256
+        per = min(256, (-(-r // n) + 31) // 32 * 32) if 2 <= n <= 4 else 256
         out += [min(per, r - at) for at in range(0, r, per)]
     return out
 
