@@ -10,12 +10,22 @@ pytestmark = pytest.mark.gpu
 
 
 def _waves():
-    """The last batch of each launch shape and the first of the next, for one group of 32 experts (148 blocks a wave) and
-    four (133 blocks in clusters)."""
-    for E, blocks in ((32, 148), (128, 33)):
+    """The last batch of each launch shape and the first of the next: of `tokens` a block, one wave of blocks (as many as the handle
+    says are resident at once), and a token more."""
+    for E in (32, 64, 128, 256):
         for tokens in (1, 2, 4, 8, 12, 16, 24, 32):
-            yield E, 96, blocks * tokens
-            yield E, 96, blocks * tokens + 1
+            yield E, 96, (tokens, 0)
+            yield E, 96, (tokens, 1)
+
+
+def _batch(E, H, T):
+    """T, or the batch that a wave of `tokens` a block and `more` tokens make."""
+    if not isinstance(T, tuple):
+        return T
+    lay = MoeLayer(E, 1, H, 32, has_bias=False, max_tokens=1)
+    blocks = lay.debug_get(lay.DEBUG_ROUTER_WAVE)
+    lay.close()
+    return blocks // (-(-E // 32)) * T[0] + T[1]
 
 
 @pytest.mark.parametrize("E,H,T", [
@@ -23,9 +33,11 @@ def _waves():
     (5, 32, 3), (33, 256, 7), (64, 288, 9),          # fewer columns than a stage, one stage, one more block of columns
     (256, 1056, 5), (257, 544, 5), (1024, 160, 40),  # the widest cluster, the first without one, the most experts
     (128, 2880, 8), (128, 2880, 333), (40, 4128, 150),
+    (512, 96, 40), (513, 96, 40), (1000, 64, 700),   # the selection's forms for 512 and 1024 experts
 ])
 @pytest.mark.parametrize("sigmoid", [False, True])
 def test_chain_at_the_edges_of_its_launches(gpu_lib, port, E, H, T, sigmoid):
+    T = _batch(E, H, T)
     rng = np.random.default_rng(E + H + T)
     k = min(4, E)
     h = rng.standard_normal((T, H)).astype(np.float32)
@@ -94,4 +106,24 @@ def test_the_same_without_clusters(gpu_lib, E, H, T):
         lay.set_router_mode(mode)
         for _ in range(2):
             assert np.array_equal(lay.route(h), w), mode
+    lay.close()
+
+
+@pytest.mark.parametrize("E,step", [(512, 256), (1024, 256), (1024, 255), (1024, 511)])
+def test_equal_logits_go_to_the_lower_expert(gpu_lib, port, E, step):
+    """Experts that repeat every `step` gate rows (in one lane of the selection, or in others): the lowest of the best one's copies first."""
+    rng = np.random.default_rng(E + step)
+    H, T, k = 64, 50, 5
+    base = (rng.standard_normal((step, H)) * 0.1).astype(np.float32)
+    Wg = np.ascontiguousarray(base[np.arange(E) % step])
+    lay = MoeLayer(E, k, H, 32, has_bias=False, max_tokens=T)
+    lay.set_router(Wg, None)
+    lay.set_router_mode(lay.ROUTER_CHAIN)
+    h = rng.standard_normal((T, H)).astype(np.float32)
+    got = lay.route(h)[..., 0].astype(int)
+    logits = port.router_logits(h, base, None, 1)[1]
+    order = np.argsort(-logits, axis=1, kind="stable")
+    for t in range(T):
+        want = [e for b in order[t, :k] for e in range(b, E, step)][:k]
+        assert got[t].tolist() == want, t
     lay.close()
