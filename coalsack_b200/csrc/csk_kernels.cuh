@@ -445,7 +445,7 @@ k_router_logits(const RouterArgs A) {
     }
     if (A.counters == nullptr || gridDim.y == 1) continue;
     int first = 0, step = 1;
-      if (A.cluster) {
+    if (A.cluster) {
       // (a block writes the next token block's logits into the other buffer, and the one after that only when all have come
       // past the next barrier, which is after they have read these)
       cluster_sync_all();

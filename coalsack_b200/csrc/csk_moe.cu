@@ -345,11 +345,11 @@ int launch_router(csk_moe_layer* L, const float* d_hidden, int64_t T, float* d_r
     // How long the list is the data decide: 2 % of the tokens of normal rows, half of them with a few channels at 1000 times
     // the others, all where rows repeat a value (padding).  Blocks of few tokens are quicker for a short list: the first
     // launch has them for a 32nd of the tokens (at least one wave of four-token blocks, at most two) and takes up to two rounds of
-    // that.  The second has up to 32 tokens a block and takes any longer list; each leaves the other's lists alone.  128 experts, 2880
-    // columns, one launch / two, us (before the chain's blocks were as they are): 8192 normal rows 133 / 138, nine channels at 1000
-    // times the others 569 / 399, every second row zero 513 / 351, every row 870 / 540 (the chain alone 343); 1024 tokens 51 / 51, every
-    // row zero 165 / 94 (66).  (With room for a quarter of a wave: 2048 tokens of eight slots, whose lists are longer, 284 -> 291 for
-    // the step.)
+    // that.  The second has up to 32 tokens a block and takes any longer list; each leaves the other's lists alone.  2880 columns, one
+    // launch / two (the chain of all tokens), us: 128 experts, 8192 normal rows 105 / 107 (326), nine channels at 1000 times the others 120 / 123,
+    // every tenth row zero 197 / 138, every second 564 / 277, every row 990 / 463; 2048 normal rows 43.6 / 46.5 (92), every row zero 241 / 126;
+    // 1024 35.5 / 39.0 (47), every row zero 128 / 72; 256 experts, 2048 normal rows 73 / 75 (185), every tenth zero 161 / 96, every row 965 / 281.  (With room
+    // for a quarter of a wave: 2048 tokens of eight slots, whose lists are longer, 284 -> 291 for the step.)
     const int few_slots = (int)std::min(2 * wave, std::max(wave, T / 32));
     b.list_max = 2 * few_slots;
     launch_router_logits<true>(b, L->d_wg_few, L->d_wg_many, router_wave, s, pdl, few_slots);
