@@ -837,7 +837,8 @@ __global__ void __launch_bounds__(256) k_router_finish(const FinishRouterArgs A)
 // The same for many tokens: a warp per token, so that no warp waits while another selects (a block per token took 91 us
 // of 8192 tokens).  Shared memory: logits and bounds of kFinishWarps tokens.
 constexpr int kFinishWarps = 8;
-__global__ void __launch_bounds__(32 * kFinishWarps) k_router_finish_many(const FinishRouterArgs A) {
+// (two blocks an SM: left alone, the compiler takes 80 registers for three and spills in the loop over the parts, 256 experts of 1024 columns, 2048 tokens 50.5 -> 53.9 us)
+__global__ void __launch_bounds__(32 * kFinishWarps, 2) k_router_finish_many(const FinishRouterArgs A) {
   extern __shared__ float finish_smem[];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int t = blockIdx.x * kFinishWarps + warp;
