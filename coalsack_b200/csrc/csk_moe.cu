@@ -1726,15 +1726,17 @@ int csk_moe_route(csk_moe_layer* L, const float* hidden, int64_t T, float* route
 }
 
 namespace {
-// Whether every buffer of a call (null: not given) is in memory of a type: page-locked (Host) or pageable (Unregistered).
-bool all_in(cudaMemoryType type, std::initializer_list<const void*> buffers) {
-  for (const void* p : buffers) {
-    cudaPointerAttributes at{};
-    if (p && (cudaPointerGetAttributes(&at, p) != cudaSuccess || at.type != type)) {
-      cudaGetLastError();
-      return false;
-    }
-  }
+// What memory a buffer is in: page-locked (Host), pageable (Unregistered), or the device's or managed.
+cudaMemoryType memory_of(const void* p) {
+  cudaPointerAttributes at{};
+  if (cudaPointerGetAttributes(&at, p) == cudaSuccess) return at.type;
+  cudaGetLastError();
+  return cudaMemoryTypeManaged;
+}
+// Whether every buffer of a call (null: not given) is page-locked.
+bool page_locked(std::initializer_list<const void*> buffers) {
+  for (const void* p : buffers)
+    if (p && memory_of(p) != cudaMemoryTypeHost) return false;
   return true;
 }
 
@@ -1762,7 +1764,7 @@ int host_passes(const csk_moe_layer* L, int64_t T, std::initializer_list<const v
   const int64_t rows = T * L->k / std::max(1, L->Eloc);  // per expert
   if (rows < 128) return 1;
   // (a copy to or from other than page-locked memory returns when it is done)
-  if (!all_in(cudaMemoryTypeHost, buffers)) return rows < 600 ? 1 : 2;
+  if (!page_locked(buffers)) return rows < 600 ? 1 : 2;
   const int least = rows < 256 ? 1 : 2;
   const int tile_rows = tile_rows_for(CSK_PATH_TILE);
   auto items = [&](int passes) { return (rows / passes + tile_rows - 1) / tile_rows * L->Eloc * L->Tgu.n_tiles; };
@@ -1799,7 +1801,12 @@ int csk_moe_forward(csk_moe_layer* L, const float* hidden, int64_t T, const floa
     // Through the handle's staging area a batch's status word comes back with its results, and nothing waits for a copy that the driver stages.
     const size_t bytes = row_bytes + route_bytes;
     const bool fits = bytes <= L->h_staged_bytes;
-    const bool staged_in = fits && row_bytes > kStagedInMin && all_in(cudaMemoryTypeUnregistered, {hidden, router_in});
+    // (a buffer that the host may copy: pageable, or page-locked where asked for; null: not given)
+    auto to_copy = [](const void* p, bool locked) {
+      const cudaMemoryType m = p ? memory_of(p) : cudaMemoryTypeUnregistered;
+      return m == cudaMemoryTypeUnregistered || (locked && m == cudaMemoryTypeHost);
+    };
+    const bool staged_in = fits && row_bytes > kStagedInMin && to_copy(hidden, false) && to_copy(router_in, true);
     float* staged_route = L->h_staged + T * L->H;
     if (staged_in) {
       const int64_t half = row_bytes < kStagedTwoPieces ? 0 : T / 2 * L->H;
@@ -1819,8 +1826,8 @@ int csk_moe_forward(csk_moe_layer* L, const float* hidden, int64_t T, const floa
       return rc;
     }
     // (asked while the kernels run)
-    const bool staged_out = fits && (all_in(cudaMemoryTypeUnregistered, {out, router_out}) ||
-                                     (bytes <= kStagedLockedMax && all_in(cudaMemoryTypeHost, {out, router_out})));
+    const bool locked = bytes <= kStagedLockedMax;
+    const bool staged_out = fits && to_copy(out, locked) && to_copy(router_out, true);
     if (staged_out) {
       // (where the inputs went out from, too: the stream has taken those first)
       CSK_CUDA(L, cudaMemcpyAsync(L->h_staged, L->d_out, row_bytes, cudaMemcpyDeviceToHost, s));

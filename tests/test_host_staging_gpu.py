@@ -45,7 +45,8 @@ def test_results_and_errors(gpu_lib, T, routed):
 # (64 KB are 16 rows of 1024 columns, 128 KB 31 with two slots each, 256 KB 64)
 @pytest.mark.parametrize("T", [1, 16, 17, 31, 32, 63, 64, 200, 256])
 @pytest.mark.parametrize("locked_in,locked_out", [(True, True), (True, False), (False, True)])
-def test_page_locked_buffers(gpu_lib, T, locked_in, locked_out):
+@pytest.mark.parametrize("mixed", [False, True])
+def test_page_locked_buffers(gpu_lib, T, locked_in, locked_out, mixed):
     """Page-locked buffers are copied without staging (small results with it), in any mixture: the same results, and nothing written
     by a call that fails."""
     sh = synth.tiny(seed=70 + T, E=8, k=2, H=1024, F=64, T=T, has_bias=True)
@@ -59,8 +60,9 @@ def test_page_locked_buffers(gpu_lib, T, locked_in, locked_out):
     def host(shape, locked):
         return torch.full(shape, 5.0, pin_memory=locked).numpy()
 
-    x, x_route = host((T, 1024), locked_in), host((T, 2, 2), locked_in)
-    got, got_ro = host((T, 1024), locked_out), host((T, 2, 2), locked_out)
+    # mixed: the routing is in the other kind of memory than the rows
+    x, x_route = host((T, 1024), locked_in), host((T, 2, 2), locked_in != mixed)
+    got, got_ro = host((T, 1024), locked_out), host((T, 2, 2), locked_out != mixed)
     x[:], x_route[:] = h, ro
     for given in (None, x_route):
         for _ in range(2):
