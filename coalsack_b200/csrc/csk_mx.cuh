@@ -523,67 +523,66 @@ __global__ void __launch_bounds__(kMxThreads, 1) k_mx(const MxArgs A) {
     if (lane == 0) {
       const int n = A.stall ? 0 : (int)n_items;
       bool ok = true;
-      // a stage's weights, and (separately) its token rows; both count on the stage's barrier
-      auto weights = [&](const RowTile& rt, int nt, const MxTileImage& g, int rec, int s) {
-        const int nb = L.rec_blocks(rec);
-        const uint32_t bytes = (uint32_t)L.rec_bytes(nt, nb);
-        mbar_expect_tx(bar_full(s), bytes + (uint32_t)(g.atoms * kMxSfAtom + nb * g.npad * 16));
-        bulk_load(smem_base + (uint32_t)s * stage_bytes,
-                  A.weights + (size_t)rt.expert * A.expert_stride + A.mat_offset + (size_t)nt * L.unit_bytes(0) +
-                      (size_t)rec * L.rec_bytes(nt, kMxRecBlocks),
-                  bytes, bar_full(s));
+      // What does not change over a unit's records is worked out once: a record then takes some 270 clocks to ask for, two
+      // thirds of them the two copies' own.
+      const int last = L.recs - 1, nb_last = L.rec_blocks(last);
+      const uint8_t *w_src = nullptr, *x_src = nullptr;
+      uint32_t w_full = 0, w_last = 0, x_full = 0, x_last = 0;
+      MxTileImage g{};
+      auto unit = [&](int item, const RowTile& rt) {
+        const int tile = item / L.n_units, nt = item % L.n_units;
+        g = mx_tile_image<D>(tile, rt.row0, rt.rows, L.recs);
+        w_src = A.weights + (size_t)rt.expert * A.expert_stride + A.mat_offset + (size_t)nt * L.unit_bytes(0);
+        w_full = (uint32_t)L.rec_bytes(nt, kMxRecBlocks);
+        w_last = (uint32_t)L.rec_bytes(nt, nb_last);
+        x_src = A.x_img + g.offset;
+        x_full = (uint32_t)g.rec_stride;
+        x_last = (uint32_t)(g.atoms * kMxSfAtom + nb_last * g.npad * 16);
       };
-      auto rows = [&](const uint8_t* image, const MxTileImage& g, int rec, int s) {
-        bulk_load(smem_base + (uint32_t)s * stage_bytes + kMxARecMax, image + g.offset + (size_t)rec * g.rec_stride,
-                  (uint32_t)(g.atoms * kMxSfAtom + L.rec_blocks(rec) * g.npad * 16), bar_full(s));
+      // a stage's weights, and (separately) its token rows; both count on the stage's barrier
+      auto weights = [&](int rec, int s) {
+        const uint32_t bytes = rec == last ? w_last : w_full;
+        mbar_expect_tx(bar_full(s), bytes + (rec == last ? x_last : x_full));
+        bulk_load(smem_base + (uint32_t)s * stage_bytes, w_src + (size_t)rec * w_full, bytes, bar_full(s));
+      };
+      auto rows = [&](const uint8_t* image, int rec, int s) {
+        bulk_load(smem_base + (uint32_t)s * stage_bytes + kMxARecMax, image + (size_t)rec * x_full, rec == last ? x_last : x_full, bar_full(s));
       };
       // as many records of the first unit as the ring holds are requested before the rows' images are complete
       int first = 0;
       if ((int)blockIdx.x < n) {
-        const int tile = blockIdx.x / L.n_units, nt = blockIdx.x % L.n_units;
-        const RowTile rt = first_tile;
-        const MxTileImage g = mx_tile_image<D>(tile, rt.row0, rt.rows, L.recs);
-        for (; first < NS && first < L.recs; ++first) weights(rt, nt, g, first, first);
+        unit(blockIdx.x, first_tile);
+        for (; first < NS && first < L.recs; ++first) weights(first, first);
         griddep_wait();
         fence_async_global();  // the images were written by ordinary stores
-        for (int rec = 0; rec < first; ++rec) rows(A.x_img, g, rec, rec);
+        for (int rec = 0; rec < first; ++rec) rows(x_src, rec, rec);
       }
       int s = first == NS ? 0 : first, issued = first;
       uint32_t ph = first == NS ? 0u : 1u;  // a stage's first use waits for nothing
-      for (int item = blockIdx.x; ok && item < n; item += gridDim.x) {
-        const int tile = item / L.n_units, nt = item % L.n_units;
-        const RowTile rt = item == (int)blockIdx.x ? first_tile : A.tiles[tile];
-        const MxTileImage g = mx_tile_image<D>(tile, rt.row0, rt.rows, L.recs);
-        for (int rec = first; rec < L.recs; ++rec) {
-          if (!mbar_wait(bar_empty(s), ph, abort_flag)) {
-            ok = false;
-            break;
-          }
-          weights(rt, nt, g, rec, s);
-          rows(A.x_img, g, rec, s);
-          ++issued;
-          if (++s == NS) {
-            s = 0;
-            ph ^= 1u;
-          }
+      auto put = [&](const uint8_t* image, int rec) {
+        if (!mbar_wait(bar_empty(s), ph, abort_flag)) return false;
+        weights(rec, s);
+        rows(image, rec, s);
+        ++issued;
+        if (++s == NS) {
+          s = 0;
+          ph ^= 1u;
         }
+        return true;
+      };
+      RowTile next = first_tile;
+      for (int item = blockIdx.x; ok && item < n; item += gridDim.x) {
+        if (item != (int)blockIdx.x) unit(item, next);
+        // (on their way while this unit's records are asked for: the next unit's tile, this one's marks)
+        if (item + (int)gridDim.x < n) next = A.tiles[(item + (int)gridDim.x) / L.n_units];
+        const int tile = item / L.n_units;
+        const uint32_t any_wide = mx_any_wide(A, tile);
+        for (int rec = first; ok && rec < L.recs; ++rec) ok = put(x_src, rec);
         first = 0;
-        if (ok && mx_any_wide(A, tile)) {  // the records with wide blocks once more
+        if (any_wide) {  // the records with wide blocks once more
           for (int w = 0; ok && w < mx_mask_words(L.recs); ++w)
-            for (uint32_t bits = __ldcg(A.x_wide + (size_t)tile * A.wide_stride + w); bits; bits &= bits - 1) {
-              const int rec = 32 * w + __ffs((int)bits) - 1;
-              if (!mbar_wait(bar_empty(s), ph, abort_flag)) {
-                ok = false;
-                break;
-              }
-              weights(rt, nt, g, rec, s);
-              rows(A.x_rest, g, rec, s);
-              ++issued;
-              if (++s == NS) {
-                s = 0;
-                ph ^= 1u;
-              }
-            }
+            for (uint32_t bits = __ldcg(A.x_wide + (size_t)tile * A.wide_stride + w); ok && bits; bits &= bits - 1)
+              ok = put(A.x_rest + g.offset, 32 * w + __ffs((int)bits) - 1);
         }
       }
       if (!ok) {
@@ -599,14 +598,13 @@ __global__ void __launch_bounds__(kMxThreads, 1) k_mx(const MxArgs A) {
   } else if (warp == 1) {
     // ------------------------------ MMA issuer (warp-wide loop, one elected lane issues) ------------------------------
     const uint32_t tb = __shfl_sync(0xffffffffu, tmem_base, 0);
-    uint32_t c = 0, it = 0;
-    int s = 0;
-    uint32_t ph = 0;
+    uint32_t c = 0, it = 0;  // records, units so far
     bool ok = true;
     griddep_wait();  // this kernel's successor may count on everything before this kernel's predecessor being complete
     griddep_launch();
     int npad_before = 0, ahead_rows = 0;
     uint32_t ahead_wide = 0;
+    const uint32_t stage16 = (uint32_t)stage_bytes >> 4, base16 = smem_base >> 4;
     for (long item = blockIdx.x; ok && item < n_items; item += gridDim.x, ++it) {
       const int tile = (int)(item / L.n_units), nt = (int)(item % L.n_units);
       if (!(it & 31u)) {
@@ -621,7 +619,7 @@ __global__ void __launch_bounds__(kMxThreads, 1) k_mx(const MxArgs A) {
       const int rows = __shfl_sync(0xffffffffu, ahead_rows, (int)(it & 31u));
       const uint32_t any_wide = __shfl_sync(0xffffffffu, ahead_wide, (int)(it & 31u));
       const int npad = mx_npad<D>(rows), atoms = npad > 128 ? 2 : 1;
-      const int r0 = L.rows(nt, 0), r1 = L.rows(nt, 1), halves = L.halves(nt);
+      const int r0 = L.rows(nt, 0), r1 = L.rows(nt, 1);
       const uint32_t buf = it & 1u, use = it >> 1;
       const uint32_t d0 = tb + (buf ? kMxTmemSf - 2u * (uint32_t)npad : 0u), d1 = d0 + (uint32_t)npad;
       ok = mbar_wait_warp(bar_acc_empty(buf), (use & 1u) ^ 1u, abort_flag);
@@ -630,59 +628,55 @@ __global__ void __launch_bounds__(kMxThreads, 1) k_mx(const MxArgs A) {
       if (!ok) break;
       npad_before = npad;
       tc_fence_after();
-      // the MMAs of the record in stage s (`add` 0: the accumulators start here), by the elected lane
-      auto issue = [&](int rec, uint32_t add) {
-        const int nb = L.rec_blocks(rec);
-        const uint32_t a = smem_base + (uint32_t)s * stage_bytes, b = a + kMxARecMax;
-        const uint32_t sf = tb + kMxTmemSf + (c & 1u) * 16u;
-        const uint32_t a_sf = a + (uint32_t)(nb * (r0 + r1) * 16), b_codes = b + (uint32_t)(atoms * kMxSfAtom);
-        tmem_cp_scales(sf, umma_desc_plain(a_sf, 128, 128));
-        if (halves > 1) tmem_cp_scales(sf + 4, umma_desc_plain(a_sf + kMxSfAtom, 128, 128));
-        tmem_cp_scales(sf + 8, umma_desc_plain(b, 128, 128));
-        if (atoms > 1) tmem_cp_scales(sf + 12, umma_desc_plain(b + kMxSfAtom, 128, 128));
-#pragma unroll
-        for (int p = 0; p < 2; ++p) {
-          if (2 * p < nb) {
-            const uint32_t idesc = umma_idesc_mxf4(npad, 2 * p);
-            const uint64_t db = umma_desc_plain(b_codes + (uint32_t)(2 * p * npad * 16), (uint32_t)(npad * 16), 128);
-            const uint32_t ap = a + (uint32_t)(p * 32 * (r0 + r1));
-            umma_mxf4_ss(d0, umma_desc_plain(ap, (uint32_t)(r0 * 16), 128), db, idesc, sf, sf + 8, p ? 1u : add);
-            if (halves > 1)
-              umma_mxf4_ss(d1, umma_desc_plain(ap + (uint32_t)(r0 * 32), (uint32_t)(r1 * 16), 128), db, idesc, sf + 4, sf + 8, p ? 1u : add);
+      int s = (int)(c % (uint32_t)NS);
+      uint32_t ph = c / (uint32_t)NS & 1u;
+      // One lane takes the unit's records by itself.  Its instructions are what a record takes once the stages are full (nothing waits for the
+      // tensor cores), so the operands' descriptors are worked out per unit and a record adds its stage's address, which is their low bits.
+      if (elect_one()) {
+        const uint32_t all = (uint32_t)(r0 + r1), idesc0 = umma_idesc_mxf4(npad, 0), idesc1 = umma_idesc_mxf4(npad, 2);
+        const uint32_t a0 = (uint32_t)r0 << 16, a1 = (uint32_t)(2 * r0) | (uint32_t)r1 << 16;
+        const uint32_t b0 = (uint32_t)(kMxARecMax / 16 + atoms * (kMxSfAtom / 16)) | (uint32_t)npad << 16;
+        constexpr uint32_t kSf = 8u << 16, kHi = 8u | 1u << 14;  // groups of 8 rows 128 bytes apart; descriptor version
+        auto desc = [](uint32_t lo) { return (uint64_t)kHi << 32 | lo; };
+        uint32_t at = base16 + (uint32_t)s * stage16, sf = tb + kMxTmemSf + (c & 1u) * 16u;
+        // the MMAs of a record in stage s (`add` 0: the accumulators start here)
+        auto record = [&](int rec, uint32_t add) {
+          if (!mbar_wait(bar_full(s), ph, abort_flag)) return false;
+          tc_fence_after();
+          const int nb = L.rec_blocks(rec);
+          const uint32_t a_sf = at + (uint32_t)nb * all + kSf, b_sf = at + kMxARecMax / 16 + kSf;
+          tmem_cp_scales(sf, desc(a_sf));
+          if (r1) tmem_cp_scales(sf + 4, desc(a_sf + kMxSfAtom / 16));
+          tmem_cp_scales(sf + 8, desc(b_sf));
+          if (atoms > 1) tmem_cp_scales(sf + 12, desc(b_sf + kMxSfAtom / 16));
+          umma_mxf4_ss(d0, desc(at + a0), desc(at + b0), idesc0, sf, sf + 8, add);
+          if (r1) umma_mxf4_ss(d1, desc(at + a1), desc(at + b0), idesc0, sf + 4, sf + 8, add);
+          if (nb > 2) {
+            const uint32_t a = at + 2 * all, b = at + b0 + 2 * (uint32_t)npad;
+            umma_mxf4_ss(d0, desc(a + a0), desc(b), idesc1, sf, sf + 8, 1u);
+            if (r1) umma_mxf4_ss(d1, desc(a + a1), desc(b), idesc1, sf + 4, sf + 8, 1u);
           }
-        }
-        umma_commit(bar_empty(s));
-      };
-      for (int rec = 0; rec < L.recs; ++rec, ++c) {
-        ok = mbar_wait_warp(bar_full(s), ph, abort_flag);
-        if (!ok) break;
-        tc_fence_after();
-        if (elect_one()) {
-          issue(rec, rec ? 1u : 0u);
-          if (rec == L.recs - 1 && !any_wide) umma_commit(bar_acc_full(buf));
-        }
-        __syncwarp();
-        if (++s == NS) {
-          s = 0;
-          ph ^= 1u;
-        }
-      }
-      if (any_wide) {  // the records with wide blocks once more
-        for (int w = 0; ok && w < mx_mask_words(L.recs); ++w)
-          for (uint32_t bits = __ldcg(A.x_wide + (size_t)tile * A.wide_stride + w); bits; bits &= bits - 1, ++c) {
-            ok = mbar_wait_warp(bar_full(s), ph, abort_flag);
-            if (!ok) break;
-            tc_fence_after();
-            if (elect_one()) issue(32 * w + __ffs((int)bits) - 1, 1u);
-            __syncwarp();
-            if (++s == NS) {
-              s = 0;
-              ph ^= 1u;
-            }
+          umma_commit(bar_empty(s));
+          at += stage16;
+          if (++s == NS) {
+            s = 0;
+            ph ^= 1u;
+            at = base16;
           }
-        if (ok && elect_one()) umma_commit(bar_acc_full(buf));
-        __syncwarp();
+          sf ^= 16u;
+          return true;
+        };
+        for (int rec = 0; ok && rec < L.recs; ++rec) ok = record(rec, rec ? 1u : 0u);
+        if (any_wide)  // the records with wide blocks once more
+          for (int w = 0; ok && w < mx_mask_words(L.recs); ++w)
+            for (uint32_t bits = __ldcg(A.x_wide + (size_t)tile * A.wide_stride + w); ok && bits; bits &= bits - 1)
+              ok = record(32 * w + __ffs((int)bits) - 1, 1u);
+        if (ok) umma_commit(bar_acc_full(buf));
       }
+      ok = __all_sync(0xffffffffu, ok);
+      c += (uint32_t)L.recs;
+      if (any_wide)
+        for (int w = 0; w < mx_mask_words(L.recs); ++w) c += (uint32_t)__popc(__ldcg(A.x_wide + (size_t)tile * A.wide_stride + w));
     }
     // everything issued has to retire before tensor memory is freed
     if (lane == 0) {
