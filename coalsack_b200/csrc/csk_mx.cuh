@@ -577,7 +577,30 @@ __global__ void __launch_bounds__(kMxThreads, 1) k_mx(const MxArgs A) {
         if (item + (int)gridDim.x < n) next = A.tiles[(item + (int)gridDim.x) / L.n_units];
         const int tile = item / L.n_units;
         const uint32_t any_wide = mx_any_wide(A, tile);
-        for (int rec = first; ok && rec < L.recs; ++rec) ok = put(x_src, rec);
+        int rec = first;
+        {
+          // full records in a loop without a branch but the wait's
+          bool here = false;
+          const uint32_t bytes = w_full + x_full;
+#pragma unroll 2
+          for (; rec < last; ++rec) {
+            if (!here && !mbar_wait(bar_empty(s), ph, abort_flag)) {
+              ok = false;
+              break;
+            }
+            const uint32_t bar = bar_full(s), dst = smem_base + (uint32_t)s * stage_bytes;
+            ++s;
+            ++issued;
+            const bool wrap = s == NS;
+            s = wrap ? 0 : s;
+            ph ^= wrap ? 1u : 0u;
+            here = mbar_test(bar_empty(s), ph);
+            mbar_expect_tx(bar, bytes);
+            bulk_load(dst, w_src + (size_t)rec * w_full, w_full, bar);
+            bulk_load(dst + kMxARecMax, x_src + (size_t)rec * x_full, x_full, bar);
+          }
+        }
+        for (; ok && rec < L.recs; ++rec) ok = put(x_src, rec);
         first = 0;
         if (any_wide) {  // the records with wide blocks once more
           for (int w = 0; ok && w < mx_mask_words(L.recs); ++w)
@@ -630,8 +653,10 @@ __global__ void __launch_bounds__(kMxThreads, 1) k_mx(const MxArgs A) {
       tc_fence_after();
       int s = (int)(c % (uint32_t)NS);
       uint32_t ph = c / (uint32_t)NS & 1u;
-      // One lane takes the unit's records by itself.  Its instructions are what a record takes once the stages are full (nothing waits for the
-      // tensor cores), so the operands' descriptors are worked out per unit and a record adds its stage's address, which is their low bits.
+      // One lane takes the unit's records by itself.  Its instructions are what a record takes once the stages are full (the tensor cores
+      // wait for it), so the operands' descriptors are worked out per unit and a record adds its stage's address, which is their
+      // low bits.  Branches cost it some 30 clocks each even where they are not taken: records of the ordinary form (both halves,
+      // one atom of row scales, four blocks) have a loop without any but the wait's, which asks for the next stage beforehand.
       if (elect_one()) {
         const uint32_t all = (uint32_t)(r0 + r1), idesc0 = umma_idesc_mxf4(npad, 0), idesc1 = umma_idesc_mxf4(npad, 2);
         const uint32_t a0 = (uint32_t)r0 << 16, a1 = (uint32_t)(2 * r0) | (uint32_t)r1 << 16;
@@ -639,6 +664,15 @@ __global__ void __launch_bounds__(kMxThreads, 1) k_mx(const MxArgs A) {
         constexpr uint32_t kSf = 8u << 16, kHi = 8u | 1u << 14;  // groups of 8 rows 128 bytes apart; descriptor version
         auto desc = [](uint32_t lo) { return (uint64_t)kHi << 32 | lo; };
         uint32_t at = base16 + (uint32_t)s * stage16, sf = tb + kMxTmemSf + (c & 1u) * 16u;
+        auto advance = [&]() {
+          at += stage16;
+          ++s;
+          const bool wrap = s == NS;
+          s = wrap ? 0 : s;
+          at = wrap ? base16 : at;
+          ph ^= wrap ? 1u : 0u;
+          sf ^= 16u;
+        };
         // the MMAs of a record in stage s (`add` 0: the accumulators start here)
         auto record = [&](int rec, uint32_t add) {
           if (!mbar_wait(bar_full(s), ph, abort_flag)) return false;
@@ -657,16 +691,36 @@ __global__ void __launch_bounds__(kMxThreads, 1) k_mx(const MxArgs A) {
             if (r1) umma_mxf4_ss(d1, desc(a + a1), desc(b), idesc1, sf + 4, sf + 8, 1u);
           }
           umma_commit(bar_empty(s));
-          at += stage16;
-          if (++s == NS) {
-            s = 0;
-            ph ^= 1u;
-            at = base16;
-          }
-          sf ^= 16u;
+          advance();
           return true;
         };
-        for (int rec = 0; ok && rec < L.recs; ++rec) ok = record(rec, rec ? 1u : 0u);
+        int rec = 0;
+        if (r1 && atoms == 1) {
+          const int ordinary = L.rec_blocks(L.recs - 1) == kMxRecBlocks ? L.recs : L.recs - 1;
+          const uint32_t a_sf = kMxRecBlocks * all + kSf, b_sf = kMxARecMax / 16 + kSf;
+          const uint32_t a2 = a0 + 2 * all, a3 = a1 + 2 * all, b2 = b0 + 2 * (uint32_t)npad;
+          bool here = false;
+#pragma unroll 2
+          for (; rec < ordinary; ++rec) {
+            if (!here && !mbar_wait(bar_full(s), ph, abort_flag)) {
+              ok = false;
+              break;
+            }
+            tc_fence_after();
+            const uint32_t now = at, sf_now = sf, bar_now = bar_empty(s);
+            advance();
+            here = mbar_test(bar_full(s), ph);  // (of a stage that nobody fills any more: not used)
+            tmem_cp_scales(sf_now, desc(now + a_sf));
+            tmem_cp_scales(sf_now + 4, desc(now + a_sf + kMxSfAtom / 16));
+            tmem_cp_scales(sf_now + 8, desc(now + b_sf));
+            umma_mxf4_ss(d0, desc(now + a0), desc(now + b0), idesc0, sf_now, sf_now + 8, rec ? 1u : 0u);
+            umma_mxf4_ss(d1, desc(now + a1), desc(now + b0), idesc0, sf_now + 4, sf_now + 8, rec ? 1u : 0u);
+            umma_mxf4_ss(d0, desc(now + a2), desc(now + b2), idesc1, sf_now, sf_now + 8, 1u);
+            umma_mxf4_ss(d1, desc(now + a3), desc(now + b2), idesc1, sf_now + 4, sf_now + 8, 1u);
+            umma_commit(bar_now);
+          }
+        }
+        for (; ok && rec < L.recs; ++rec) ok = record(rec, rec ? 1u : 0u);
         if (any_wide)  // the records with wide blocks once more
           for (int w = 0; ok && w < mx_mask_words(L.recs); ++w)
             for (uint32_t bits = __ldcg(A.x_wide + (size_t)tile * A.wide_stride + w); ok && bits; bits &= bits - 1)
