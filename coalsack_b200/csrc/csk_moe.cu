@@ -319,7 +319,7 @@ int launch_router(csk_moe_layer* L, const float* d_hidden, int64_t T, float* d_r
     // the token blocks alone fill the machine
     int parts = std::min(std::min(fast_router_slices(L->H), kFastMaxParts),
                          std::max(1, (L->sm_count + token_blocks * groups - 1) / (token_blocks * groups)));
-    while (parts > 1 && T * parts > L->part_rows) --parts;
+    while (parts > 1 && (T * parts > L->part_rows || finish_smem_bytes(parts, L->E_router) > kFinishMaxSmem)) --parts;
     const dim3 grid((unsigned)token_blocks, (unsigned)groups, (unsigned)parts);
     const size_t smem = fast_router_smem(tpw);
     switch (tpw) {
@@ -331,7 +331,7 @@ int launch_router(csk_moe_layer* L, const float* d_hidden, int64_t T, float* d_r
     }
     g.wnorm = L->d_wnorm;
     g.parts = parts;
-    launch_k(k_router_finish, dim3((unsigned)T), dim3((unsigned)std::min(32 * groups, 256)), 0, s, pdl, g);
+    launch_k(k_router_finish, dim3((unsigned)T), dim3(kFinishThreads), finish_smem_bytes(parts, L->E_router), s, pdl, g);
   }
   // ... and go through the order-faithful chain: its blocks walk the list and leave at once when it is empty
   RouterArgs b = a;
