@@ -444,7 +444,8 @@ int launch_permute(csk_moe_layer* L, const float* d_hidden, const float* d_route
     a.weight_before_ffn = L->cfg.weight_before_ffn;
     a.blocks = L->Lgu.blocks;
     a.recs = L->Lgu.recs;
-    launch_k(k_mx_quant, dim3((unsigned)T), dim3(std::min(kMxQuantThreads, ceil_div(L->Lgu.blocks, 8) * 32)), 0, s, L->pdl, a);
+    const int threads = ceil_div(L->Lgu.blocks, 8) * 32, part = one_block ? kMxQuantPart : kMxQuantThreads;
+    launch_k(k_mx_quant, dim3((unsigned)T, one_block ? ceil_div(threads, part) : 1), dim3(std::min(part, threads)), 0, s, L->pdl, a);
   } else {
     launch_k(reinterpret_cast<uintptr_t>(x16) % 16 ? k_scatter<uint2> : k_scatter<uint4>, dim3((unsigned)T), dim3(kScatterThreads), 0, s, L->pdl,
              d_router, d_hidden, L->k, L->H, L->E, only_expert, L->d_offsets, one_block ? (int*)nullptr : L->d_cursor, L->d_row_of_pair, x16, ldx,

@@ -313,29 +313,61 @@ struct MxQuantArgs {
   int wide_stride;
   int T, H, E, k, e_begin, e_count, only_expert, max_rows, weight_before_ffn, blocks, recs;
 };
-// Token rows to digits, into the images of the row tiles they were placed in.  One CTA per token, four threads per
-// 32-column block: a token is encoded once and stored k times (with the routing weight applied before the expert
-// it is encoded per pair).  Bound for a few tokens by its chain of dependent loads (8.8 us for one token of 2880 columns under
-// the profiler's cold caches; with one thread per block and the wide blocks' test 12.0; 333 tokens 14.8 and 20.0).
-constexpr int kMxQuantThreads = 384;  // 96 blocks at once
+// What four neighbouring lanes hold of a block, a word of each digit, as whole digits: lane q has digit q in `own` and all have the fifth.
+struct MxColumns {
+  uint4 own, fifth;
+};
+__device__ __forceinline__ MxColumns mx_columns(const uint32_t (&d)[kMxDigitsX], int q) {
+  const bool odd = q & 1, high = q & 2;
+  const uint32_t a = __shfl_xor_sync(0xffffffffu, odd ? d[0] : d[1], 1), b = __shfl_xor_sync(0xffffffffu, odd ? d[2] : d[3], 1);
+  const uint32_t l0 = odd ? a : d[0], l1 = odd ? d[1] : a, h0 = odd ? b : d[2], h1 = odd ? d[3] : b;  // two words of digits q & 1, 2 + (q & 1)
+  const uint32_t r0 = __shfl_xor_sync(0xffffffffu, high ? l0 : h0, 2), r1 = __shfl_xor_sync(0xffffffffu, high ? l1 : h1, 2);
+  MxColumns c;
+  c.own = high ? make_uint4(r0, r1, h0, h1) : make_uint4(l0, l1, r0, r1);
+  const int first = threadIdx.x & 28;
+  c.fifth = make_uint4(__shfl_sync(0xffffffffu, d[4], first), __shfl_sync(0xffffffffu, d[4], first + 1),
+                       __shfl_sync(0xffffffffu, d[4], first + 2), __shfl_sync(0xffffffffu, d[4], first + 3));
+  return c;
+}
+
+// Token rows to digits, into the images of the row tiles they were placed in.  A CTA per token and 32 of its 32-column blocks, four threads
+// per block: a token is encoded once and stored k times (with the routing weight applied before the expert it is
+// encoded per pair).  What a token costs is its stores (one CTA a token and a word a store: 1 token of 2880 columns 5500 of the
+// kernel's 6100 clocks after the wait): a lane stores whole digits, 16 bytes, sixteen lanes a record's scales as words, and
+// the blocks of a token are on several SMs (one CTA where the rows are claimed here).
+constexpr int kMxQuantThreads = 384, kMxQuantPart = 128;
+static_assert(kMxDigitsX == 5, "four lanes' digits and a fifth");
 __global__ void __launch_bounds__(kMxQuantThreads) k_mx_quant(const MxQuantArgs A) {
   __shared__ MxTileImage s_img[16];
   __shared__ int s_r[16], s_tile[16];
   __shared__ float s_w[16];
-  const int t = blockIdx.x, kbs = A.H / 32, q = threadIdx.x & 3, kb0 = threadIdx.x >> 2, step = blockDim.x >> 2;
+  const int t = blockIdx.x, kbs = A.H / 32, q = threadIdx.x & 3, step = (gridDim.y * blockDim.x) >> 2;
+  int kb = (blockIdx.y * blockDim.x + threadIdx.x) >> 2;
   float v[8];
   MxEncoded e;
-  auto load = [&](int kb, float w) {  // the eight values of this thread times w (zeros past the row)
+  auto load = [&](float w) {  // the eight values of this thread times w (zeros past the row)
     const float4* src = reinterpret_cast<const float4*>(A.hidden + (size_t)t * A.H + kb * 32 + q * 8);
     const float4 x = kb < kbs ? __ldg(src) : make_float4(0.f, 0.f, 0.f, 0.f), y = kb < kbs ? __ldg(src + 1) : x;
     v[0] = x.x * w, v[1] = x.y * w, v[2] = x.z * w, v[3] = x.w * w;
     v[4] = y.x * w, v[5] = y.y * w, v[6] = y.z * w, v[7] = y.w * w;
   };
-  // the hidden states are older than the kernel before this one: encode while it is still placing rows
-  if (!A.weight_before_ffn) {
-    load(kb0, 1.f);
+  MxColumns c, rest;
+  uint32_t scales = 0;  // of the record's four blocks
+  bool any_wide = false;
+  auto encode = [&](float w) {
+    load(w);
     e = mx_encode_block(v);
-  }
+    c = mx_columns(e.d, q);
+    any_wide = __any_sync(0xffffffffu, e.wide);
+    if (any_wide) rest = mx_columns(e.rest, q);
+    else rest.own = rest.fifth = make_uint4(0, 0, 0, 0);
+    // (columns past K inside the last blocks: the weights' codes are zero there, so any scale but NaN will do)
+    scales = kb < kbs ? e.sf << (8 * (kb & 3)) : 0u;
+    scales |= __shfl_xor_sync(0xffffffffu, scales, 4);
+    scales |= __shfl_xor_sync(0xffffffffu, scales, 8);
+  };
+  // the hidden states are older than the kernel before this one: encode while it is still placing rows
+  if (!A.weight_before_ffn) encode(1.f);
   griddep_wait();
   griddep_launch();
   if ((int)threadIdx.x < A.k) {
@@ -366,25 +398,31 @@ __global__ void __launch_bounds__(kMxQuantThreads) k_mx_quant(const MxQuantArgs 
   }
   __syncthreads();
   // (whole warps: the lanes of a block past the row's end take part in the exchanges)
-  for (int base = 0; base < A.blocks; base += step) {
-    const int kb = base + kb0;
-    if (base && !A.weight_before_ffn) {
-      load(kb, 1.f);
-      e = mx_encode_block(v);
-    }
+  for (bool first = true; (kb & ~7) < A.blocks; kb += step, first = false) {
+    if (!first && !A.weight_before_ffn) encode(1.f);
     for (int j = 0; j < A.k; ++j) {
       if (s_r[j] < 0) continue;
-      if (A.weight_before_ffn) {
-        load(kb, s_w[j]);
-        e = mx_encode_block(v);
+      if (A.weight_before_ffn) encode(s_w[j]);
+      if ((kb & ~3) >= A.blocks) continue;
+      const MxTileImage& g = s_img[j];
+      const int n = kMxDigitsX * s_r[j];
+      const size_t rec = g.offset + (size_t)(kb / kMxRecBlocks) * g.rec_stride;
+      const size_t codes = rec + g.atoms * kMxSfAtom + ((size_t)(kb & 3) * g.npad + n) * 16;
+      if (kb < kbs) {
+        *reinterpret_cast<uint4*>(A.image + codes + 16 * q) = c.own;
+        *reinterpret_cast<uint4*>(A.rest + codes + 16 * q) = rest.own;
+        if (q == (j & 3)) {
+          *reinterpret_cast<uint4*>(A.image + codes + 64) = c.fifth;
+          *reinterpret_cast<uint4*>(A.rest + codes + 64) = rest.fifth;
+        }
       }
-      if (kb >= kbs) {
-        if (kb < A.blocks) mx_store_pad(A.image, s_img[j], s_r[j], kb, q);
-        continue;
+      const int l = threadIdx.x & 15;
+      if (l < kMxDigitsX) *reinterpret_cast<uint32_t*>(A.image + rec + mx_sf_pos(n + l, 0)) = scales;
+      if (any_wide && e.wide && kb < kbs) {
+        // (zeros are zero under any scale but NaN, and the second image never holds that)
+        for (int p = q; p < kMxDigitsX; p += 4) A.rest[rec + mx_sf_pos(n + p, kb)] = (uint8_t)(e.sf - mx_rest_shift(kMxDigitsX));
+        if (q == 0) mx_mark_wide(A.wide + (size_t)s_tile[j] * A.wide_stride, kb);
       }
-      mx_store_block(A.image, s_img[j], s_r[j], kb, q, e.d, (int)e.sf);
-      mx_store_block(A.rest, s_img[j], s_r[j], kb, q, e.rest, e.wide ? (int)(e.sf - mx_rest_shift(kMxDigitsX)) : -1);
-      if (e.wide && q == 0) mx_mark_wide(A.wide + (size_t)s_tile[j] * A.wide_stride, kb);
     }
   }
 }
