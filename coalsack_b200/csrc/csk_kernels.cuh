@@ -216,8 +216,8 @@ struct RouterArgs {
 //     consumer waits for.  Packed weights of the first stages are requested before the kernel
 //     in front has ended;
 //   * a lane reads its own expert row with 128-bit loads (conflict-free by the row padding)
-//     and the token rows by broadcast, some groups of four columns ahead; the products of the
-//     next group are written between the additions of this one, two to an instruction
+//     and the token rows by broadcast, a batch of columns ahead; the products of the next four
+//     columns are written between the additions of these, two to an instruction
 //     (mul.rn.f32x2: the same rounding, half the issue slots);
 //   * a chain costs one dependent addition per column, 4.3 cycles: TT = 1 runs one chain at
 //     that speed (few tokens), larger TT has the additions of TT chains fill those cycles, up to
@@ -252,28 +252,36 @@ __device__ __forceinline__ float4 mul4_rn(const float4& a, const float4& b) {
   return r;
 }
 
-// N columns of TT chains; w, h: the lane's expert row and the warp's token rows (ld_bytes apart) in shared memory.  AHEAD groups of
-// four columns are in registers ahead.
-template <int TT, int N, int AHEAD>
-__device__ __forceinline__ void chain_columns(uint32_t w, uint32_t h, int ld_bytes, float (&acc)[TT]) {
-  constexpr int G = N / 4, A = AHEAD < G ? AHEAD : G;
-  float4 wv[A], hv[A][TT], now[TT], next[TT];
-  auto load = [&](int g) {
-    wv[g % A] = lds128(w + 16 * g);
+// A batch of 4 G columns in registers: the lane's expert row and the warp's token rows.
+__host__ __device__ constexpr int router_groups(int tt) { return tt == 1 ? 8 : 4; }
+template <int TT, int G>
+struct ChainBatch {
+  float4 w[G], h[G][TT];
+  // w, h: where the rows' columns are in shared memory, the token rows ld_bytes apart
+  __device__ __forceinline__ void load(int g, uint32_t wp, uint32_t hp, int ld_bytes) {
+    w[g] = lds128(wp + 16 * g);
 #pragma unroll
-    for (int i = 0; i < TT; ++i) hv[g % A][i] = lds128(h + i * ld_bytes + 16 * g);
-  };
+    for (int i = 0; i < TT; ++i) h[g][i] = lds128(hp + i * ld_bytes + 16 * g);
+  }
+  __device__ __forceinline__ void products(int g, float4 (&p)[TT]) const {
 #pragma unroll
-  for (int g = 0; g < A; ++g) load(g);
-#pragma unroll
-  for (int i = 0; i < TT; ++i) now[i] = mul4_rn<(TT > 1)>(hv[0][i], wv[0]);
+    for (int i = 0; i < TT; ++i) p[i] = mul4_rn<(TT > 1)>(h[g][i], w[g]);
+  }
+};
+// Adds the batch's columns to the chains and loads the next batch, a group between each two groups' additions.  `now`: the products of
+// the batch's first group; on return those of the next one's.
+// Batches alternate between two sets of registers, across the chunks' borders too, so that a load is waited for a whole batch
+// after it was asked for.  (With one ring of registers, refilled a group at a time, the additions of three chains waited for the
+// latest loads: 2750 clocks per 128 columns, 333 tokens of 128 experts; now 1480.  One chain: 1445 per 256 columns, now 1355.)
+template <int TT, int G>
+__device__ __forceinline__ void chain_batch(const ChainBatch<TT, G>& b, ChainBatch<TT, G>& next_batch, uint32_t wp, uint32_t hp, int ld_bytes,
+                                            float4 (&now)[TT], float (&acc)[TT]) {
 #pragma unroll
   for (int g = 0; g < G; ++g) {
-    if (g + A < G) load(g + A);  // the registers of group g, whose products have been made
-    if (g + 1 < G) {
-#pragma unroll
-      for (int i = 0; i < TT; ++i) next[i] = mul4_rn<(TT > 1)>(hv[(g + 1) % A][i], wv[(g + 1) % A]);
-    }
+    next_batch.load(g, wp, hp, ld_bytes);
+    float4 next[TT];
+    if (g + 1 < G) b.products(g + 1, next);
+    else next_batch.products(0, next);
 #pragma unroll
     for (int i = 0; i < TT; ++i) acc[i] = __fadd_rn(acc[i], now[i].x);
 #pragma unroll
@@ -286,7 +294,6 @@ __device__ __forceinline__ void chain_columns(uint32_t w, uint32_t h, int ld_byt
     for (int i = 0; i < TT; ++i) now[i] = next[i];
   }
 }
-__host__ __device__ constexpr int router_ahead(int tt) { return tt == 1 ? 8 : tt == 2 ? 4 : tt <= 4 ? 3 : 2; }
 
 // Bounded wait that naps between polls, for a warp that shares its scheduler with a
 // warp doing the real work.
@@ -345,6 +352,8 @@ k_router_logits(const RouterArgs A) {
     mbar_expect_tx(bar_full(st), 32 * LD * 4);
     bulk_load(stages + (uint32_t)st * stage_floats * 4, packed + (size_t)ci * 32 * LD, 32 * LD * 4, bar_full(st));
   };
+  const int e = e0 + lane;
+  const float bias = A.bias && warp >= NP && e < E ? __ldg(A.bias + e) : 0.f;  // (the router's own, older than any kernel of the step)
   const int ahead = PACKED && !list ? min(NS, n_chunks) : 0;  // (a list may turn out empty; T is not)
   if (warp == 0 && lane == 0)
     for (int ci = 0; ci < ahead; ++ci) packed_stage(ci, ci);
@@ -404,31 +413,59 @@ k_router_logits(const RouterArgs A) {
       float acc[TT];
 #pragma unroll
       for (int i = 0; i < TT; ++i) acc[i] = 0.f;
-      bool here = mbar_try(bar_full(cg % NS), (uint32_t)((cg / NS) & 1));
-      for (int ci = 0; ci < n_chunks; ++ci) {
-        const int st = cg % NS, dc = min(CH, H - ci * CH);
-        if (!here) ok = mbar_wait(bar_full(st), (uint32_t)((cg / NS) & 1), abort_flag) && ok;
-        ++cg;
-        // (the answer is needed after this chunk only; the question alone costs 100 cycles in front of one)
-        here = ci + 1 < n_chunks && mbar_test(bar_full(cg % NS), (uint32_t)((cg / NS) & 1));
-        const uint32_t wp = stages + (uint32_t)(st * stage_floats + lane * LD) * 4;
-        const uint32_t hp = stages + (uint32_t)(st * stage_floats + (32 + w * TT) * LD) * 4;
-        if (dc == CH) {
-          chain_columns<TT, CH, router_ahead(TT)>(wp, hp, LD * 4, acc);
-        } else {
+      constexpr int G = router_groups(TT), BC = 4 * G, NB = CH / BC;  // columns of a batch, batches of a chunk
+      static_assert(NB % 2 == 0 && 32 % BC == 0, "batches");
+      ChainBatch<TT, G> even, odd;
+      float4 now[TT];
+      auto w_at = [&](int c) { return stages + (uint32_t)((c % NS) * stage_floats + lane * LD) * 4; };
+      auto h_at = [&](int c) { return stages + (uint32_t)((c % NS) * stage_floats + (32 + w * TT) * LD) * 4; };
+      ok = mbar_wait(bar_full(cg % NS), (uint32_t)((cg / NS) & 1), abort_flag) && ok;
+      uint32_t wp = w_at(cg), hp = h_at(cg);
+#pragma unroll
+      for (int g = 0; g < G; ++g) even.load(g, wp, hp, LD * 4);
+      even.products(0, now);
+      const int full = H / CH;
 #pragma unroll 1
-          for (int d = 0; d < dc; d += 32) chain_columns<TT, 32, router_ahead(TT)>(wp + d * 4, hp + d * 4, LD * 4, acc);
+      for (int ci = 0; ci < full; ++ci) {
+        const int st = cg % NS;
+        ++cg;
+        const uint32_t parity = (uint32_t)((cg / NS) & 1);
+        const bool more = ci + 1 < n_chunks;
+        bool here = false;
+#pragma unroll
+        for (int b = 0; b < NB; b += 2) {
+          chain_batch<TT, G>(even, odd, wp + (b + 1) * BC * 4, hp + (b + 1) * BC * 4, LD * 4, now, acc);
+          if (b + 2 == NB && more) {  // the next chunk's first batch
+            if (!here) ok = mbar_wait(bar_full(cg % NS), parity, abort_flag) && ok;
+            wp = w_at(cg);
+            hp = h_at(cg);
+          }
+          // (the answer is needed two batches on; the question alone costs 100 cycles in front of a chunk)
+          if (b + 4 == NB) here = more && mbar_test(bar_full(cg % NS), parity);
+          const int ahead_columns = b + 2 < NB ? (b + 2) * BC : 0;  // (without a next chunk: anything, not used)
+          chain_batch<TT, G>(odd, even, wp + ahead_columns * 4, hp + ahead_columns * 4, LD * 4, now, acc);
         }
         __syncwarp();
         if (lane == 0 && ok) mbar_arrive(bar_empty(st));
       }
+      if (full < n_chunks) {  // the rest of a row
+        const int batches = (H - full * CH) / BC;
+#pragma unroll 1
+        for (int b = 0; b < batches; b += 2) {
+          // (a batch past the row's end is in the stage too: anything, not used)
+          chain_batch<TT, G>(even, odd, wp + (b + 1) * BC * 4, hp + (b + 1) * BC * 4, LD * 4, now, acc);
+          if (b + 1 == batches) break;
+          chain_batch<TT, G>(odd, even, wp + (b + 2) * BC * 4, hp + (b + 2) * BC * 4, LD * 4, now, acc);
+        }
+        const int st = cg++ % NS;
+        __syncwarp();
+        if (lane == 0 && ok) mbar_arrive(bar_empty(st));
+      }
       __syncwarp();
-      const int e = e0 + lane;
-      const float b = (A.bias && e < E) ? A.bias[e] : 0.f;
 #pragma unroll
       for (int i = 0; i < TT; ++i) {
         const int j = w * TT + i, t = token_at(t0 + j);
-        const float logit = e < E ? __fadd_rn(acc[i], b) : -INFINITY;
+        const float logit = e < E ? __fadd_rn(acc[i], bias) : -INFINITY;
         if (A.counters && gridDim.y == 1) {
           float v[1] = {logit};
           if (t >= 0) warp_topk_regs<false, 1>(v, E, A.k, A.sigmoid, A.router_out + (size_t)t * A.k * 2, nullptr);
