@@ -1276,21 +1276,24 @@ __global__ void __launch_bounds__(256) k_dense_rows(const float* __restrict__ hi
 // the token's row unweighted, or zeros.
 // ---------------------------------------------------------------------------
 //
-// Bound by HBM (k rows of y in, one out).  Four slots' rows are requested at once: one at a time a
+// Bound by HBM (k rows of y in, one out).  AT_ONCE slots' rows are requested at once: one at a time a
 // step of 8192 tokens took 2046 us, with four 2011; 2048 tokens of eight slots 318 and 306.  A few tokens are bound by the
 // latency of their loads: a row is then dealt to several blocks (gridDim.y), so that a thread has one round of them (8 tokens of
-// 2880 columns 7.9 -> 4.5 us, profiler).
+// 2880 columns 7.9 -> 4.5 us, profiler), the shared expert's and the residual row with it (16 tokens of eight slots, a step: four
+// slots at once and those two rows after them 64.0 us, now 62.5).
+// The rows are read for the last time, so they are the first to leave L2 (a step of 2048 tokens of eight slots 244.5 -> 240.6, of 4096
+// of four 768.5 -> 766.1).
 //
 // carry (optional; the host entry point that runs a batch in several passes): block 0 folds this
 // pass's status word into a sticky one and adds its per-expert row counts to running totals --
 // layout: carry[0] = sticky status, carry[1 .. E] = rows per expert.
-constexpr int kCombineAtOnce = 4;
+template <int AT_ONCE>
 __global__ void __launch_bounds__(256) k_combine(const float* __restrict__ router_out, const int* __restrict__ row_of_pair,
                           const float* __restrict__ y, int ldy, float* __restrict__ out, int T,
                           int k, int H, int unweighted, int dense_single,
                           const int* __restrict__ meta = nullptr, const int* __restrict__ counts = nullptr,
-                          int* __restrict__ carry = nullptr, int E = 0, const float* __restrict__ residual = nullptr,
-                          const float* __restrict__ shared_out = nullptr) {
+                          int* __restrict__ carry = nullptr, int E = 0, const float* residual = nullptr,
+                          const float* shared_out = nullptr) {
   __shared__ int s_row[kMaxTopK];
   __shared__ float s_w[kMaxTopK];
   const int t = blockIdx.x;
@@ -1299,6 +1302,7 @@ __global__ void __launch_bounds__(256) k_combine(const float* __restrict__ route
     s_row[threadIdx.x] = row_of_pair[(size_t)t * k + threadIdx.x];
     s_w[threadIdx.x] = unweighted ? 1.f : router_out[((size_t)t * k + threadIdx.x) * 2 + 1];  // 1 * v is v
   }
+  __syncthreads();
   griddep_wait();
   griddep_launch();
   if (carry && t == 0 && blockIdx.y == 0) {
@@ -1306,17 +1310,20 @@ __global__ void __launch_bounds__(256) k_combine(const float* __restrict__ route
     for (int e = threadIdx.x; e < E; e += blockDim.x) carry[1 + e] += counts[e];
   }
   if (t >= T) return;
-  __syncthreads();
   for (int d = (blockIdx.y * blockDim.x + threadIdx.x) * 4; d < H; d += gridDim.y * blockDim.x * 4) {
     float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+    // (on their way with the rows)
+    float4 sh, r;
+    if (shared_out) sh = *reinterpret_cast<const float4*>(shared_out + (size_t)t * H + d);
+    if (residual) r = *reinterpret_cast<const float4*>(residual + (size_t)t * H + d);
     bool done = false;
-    for (int j0 = 0; j0 < k && !done; j0 += kCombineAtOnce) {
-      float4 v[kCombineAtOnce];
+    for (int j0 = 0; j0 < k && !done; j0 += AT_ONCE) {
+      float4 v[AT_ONCE];
 #pragma unroll
-      for (int j = 0; j < kCombineAtOnce; ++j)
-        if (j0 + j < k && s_row[j0 + j] >= 0) v[j] = *reinterpret_cast<const float4*>(y + (size_t)s_row[j0 + j] * ldy + d);
+      for (int j = 0; j < AT_ONCE; ++j)
+        if (j0 + j < k && s_row[j0 + j] >= 0) v[j] = __ldcs(reinterpret_cast<const float4*>(y + (size_t)s_row[j0 + j] * ldy + d));
 #pragma unroll
-      for (int j = 0; j < kCombineAtOnce; ++j) {
+      for (int j = 0; j < AT_ONCE; ++j) {
         if (j0 + j >= k || s_row[j0 + j] < 0 || done) continue;
         if (dense_single) {
           acc = v[j];
@@ -1332,7 +1339,6 @@ __global__ void __launch_bounds__(256) k_combine(const float* __restrict__ route
     }
     if (shared_out) {
       // the shared expert's dense FFN on the same rows: add(merge output, shared output), llm_engine.cpp:766-769
-      const float4 sh = *reinterpret_cast<const float4*>(shared_out + (size_t)t * H + d);
       acc.x = __fadd_rn(acc.x, sh.x);
       acc.y = __fadd_rn(acc.y, sh.y);
       acc.z = __fadd_rn(acc.z, sh.z);
@@ -1340,7 +1346,6 @@ __global__ void __launch_bounds__(256) k_combine(const float* __restrict__ route
     }
     if (residual) {
       // the residual connection around the layer: add(residual, merge output), llm_engine.cpp:773-777
-      const float4 r = *reinterpret_cast<const float4*>(residual + (size_t)t * H + d);
       acc.x = __fadd_rn(r.x, acc.x);
       acc.y = __fadd_rn(r.y, acc.y);
       acc.z = __fadd_rn(r.z, acc.z);

@@ -746,7 +746,7 @@ int forward_dev(csk_moe_layer* L, const float* d_hidden, int64_t T, const float*
   if (shared_ready) CSK_CUDA(L, cudaStreamWaitEvent(s, shared_ready, 0));
   // (few tokens: a row dealt to several blocks)
   const unsigned row_blocks = T < 4 * L->sm_count ? (unsigned)ceil_div(L->H, 1024) : 1u;
-  launch_k(k_combine, dim3((unsigned)T, row_blocks), dim3(256), 0, s, L->pdl && !shared_ready, router, L->d_row_of_pair,
+  launch_k(L->k > 4 ? k_combine<8> : k_combine<4>, dim3((unsigned)T, row_blocks), dim3(256), 0, s, L->pdl && !shared_ready, router, L->d_row_of_pair,
            (const float*)L->d_y, L->H, d_out, (int)T, L->k, L->H, (int)L->cfg.weight_before_ffn, (int)(only_expert >= 0),
            (const int*)L->d_meta, (const int*)L->d_counts, L->carry_active ? L->d_carry : (int*)nullptr, L->E, d_residual,
            d_shared);
@@ -1976,7 +1976,7 @@ int csk_moe_merge(csk_moe_layer* L, const float* router_out, int64_t T, const fl
   CSK_CUDA(L, cudaMemcpyAsync(L->d_y, packed.data(), sizeof(float) * packed.size(), cudaMemcpyHostToDevice, s));
   CSK_CUDA(L, cudaMemcpyAsync(L->d_row_of_pair, rows.data(), sizeof(int) * rows.size(), cudaMemcpyHostToDevice, s));
   CSK_CUDA(L, cudaMemcpyAsync(L->d_router, router_out, sizeof(float) * T * L->k * 2, cudaMemcpyHostToDevice, s));
-  k_combine<<<(unsigned)T, 256, 0, s>>>(L->d_router, L->d_row_of_pair, L->d_y, L->H, L->d_out, (int)T,
+  k_combine<4><<<(unsigned)T, 256, 0, s>>>(L->d_router, L->d_row_of_pair, L->d_y, L->H, L->d_out, (int)T,
                                         L->k, L->H, L->cfg.weight_before_ffn, 0, nullptr, nullptr, nullptr, 0);
   CSK_CUDA(L, cudaGetLastError());
   CSK_CUDA(L, cudaMemcpyAsync(out, L->d_out, sizeof(float) * T * L->H, cudaMemcpyDeviceToHost, s));
@@ -2355,7 +2355,7 @@ int csk_moe_ep_combine_dev(csk_moe_layer* L, const float* d_back, int64_t T, flo
                                   (long long)T, (long long)L->last_T);
   CSK_CUDA(L, cudaSetDevice(L->cfg.device));
   cudaStream_t s = pick(L, stream);
-  k_combine<<<(unsigned)T, 256, 0, s>>>(L->d_router, L->d_row_of_pair, d_back, L->H, d_out, (int)T, L->k,
+  k_combine<4><<<(unsigned)T, 256, 0, s>>>(L->d_router, L->d_row_of_pair, d_back, L->H, d_out, (int)T, L->k,
                                         L->H, L->cfg.weight_before_ffn, 0, nullptr, nullptr, nullptr, 0);
   CSK_CUDA(L, cudaGetLastError());
   if (d_router_out)
