@@ -417,7 +417,10 @@ int launch_permute(csk_moe_layer* L, const float* d_hidden, const float* d_route
     p.n_partial = kHistBlocks;
     L->last.launches += 2;
   }
-  launch_k(k_scan, dim3(1), dim3(scan_threads(L->E, one_block ? n_pairs : 0)), 0, s, L->pdl, p);
+  if (e_count && n_pairs <= kPlanPairs)  // (rows to send have to be in the order of the slots)
+    launch_k(k_plan, dim3(1), dim3(ceil_div(n_pairs, 32) * 32), 0, s, L->pdl, p);
+  else
+    launch_k(k_scan, dim3(1), dim3(scan_threads(L->E, one_block ? n_pairs : 0)), 0, s, L->pdl, p);
   if (digits) {
     MxQuantArgs a{};
     a.hidden = d_hidden;

@@ -48,3 +48,43 @@ def test_plan_edges(gpu_lib, port, E, k, T, path):
         forward(bad)
     assert np.array_equal(forward(ro), out)
     lay.close()
+
+
+@pytest.mark.parametrize("E,k,T", [
+    (4, 1, 31), (64, 8, 128), (64, 8, 129),      # one warp and a lane less; the most pairs with a thread each, and one token more
+    (2, 1, 1000), (1024, 1, 1024),               # many tiles of an expert; as many experts as pairs
+])
+@pytest.mark.parametrize("path", [PATH_STREAM, PATH_TILE])
+def test_plan_of_a_thread_per_pair(gpu_lib, port, E, k, T, path):
+    """Rows that share an expert unevenly, some of it not loaded: outputs against the restatement, counters, and the error."""
+    sh = synth.tiny(seed=E + T, E=E, k=k, H=64, F=32, T=T, has_bias=True)
+    h, Wg, rb, ex = cases.layer_inputs(sh)
+    lay = MoeLayer.from_shape(sh)
+    lay.set_router(Wg, rb)
+    lay.load_experts(ex, range(E - 1))
+    lay.set_path(path)
+    rng = np.random.default_rng(T)
+    ro = rng.uniform(0.1, 1.0, (T, k, 2)).astype(np.float32)
+    p = 1.0 / (1.0 + np.arange(E - 1)) if E > 2 else np.ones(1)
+    ro[..., 0] = [rng.choice(E - 1, k, replace=False, p=p / p.sum()) for _ in range(T)]
+    h_d, out_d = torch.from_numpy(h).cuda(), torch.empty((T, 64), device="cuda")
+
+    def forward(routing):
+        r = torch.from_numpy(routing).cuda()
+        torch.cuda.synchronize()
+        lay.forward_dev(h_d, T, out_d, d_router_in=r)
+        lay.sync()
+        return out_d.cpu().numpy()
+
+    out = forward(ro)
+    want, _ = port.moe_layer(h, Wg, rb, ex, k, sh.act, router_out=ro)
+    mx, mr = cases.err_stats(out, want)
+    assert mx <= cases.MAX_ABS_OVER_RMS and mr <= cases.MEAN_REL, (mx, mr)
+    rows, distinct, _ = lay.counters()
+    assert np.array_equal(rows, np.bincount(ro[..., 0].astype(int).ravel(), minlength=E)) and distinct == (rows > 0).sum()
+    absent = ro.copy()
+    absent[0, 0, 0] = E - 1
+    with pytest.raises(CskError, match="not loaded"):
+        forward(absent)
+    assert np.array_equal(forward(ro), out)
+    lay.close()
