@@ -1373,13 +1373,16 @@ __global__ void __launch_bounds__(256) k_dense_rows(const float* __restrict__ hi
 // carry (optional; the host entry point that runs a batch in several passes): block 0 folds this
 // pass's status word into a sticky one and adds its per-expert row counts to running totals --
 // layout: carry[0] = sticky status, carry[1 .. E] = rows per expert.
+//
+// host_router, host_meta (optional): page-locked memory that the routing and the 16 words of `meta` go to beside the results, which
+// `out` may be in then, too.
 template <int AT_ONCE>
 __global__ void __launch_bounds__(256) k_combine(const float* __restrict__ router_out, const int* __restrict__ row_of_pair,
                           const float* __restrict__ y, int ldy, float* __restrict__ out, int T,
                           int k, int H, int unweighted, int dense_single,
                           const int* __restrict__ meta = nullptr, const int* __restrict__ counts = nullptr,
                           int* __restrict__ carry = nullptr, int E = 0, const float* residual = nullptr,
-                          const float* shared_out = nullptr) {
+                          const float* shared_out = nullptr, float* host_router = nullptr, int* host_meta = nullptr) {
   __shared__ int s_row[kMaxTopK];
   __shared__ float s_w[kMaxTopK];
   const int t = blockIdx.x;
@@ -1396,6 +1399,10 @@ __global__ void __launch_bounds__(256) k_combine(const float* __restrict__ route
     for (int e = threadIdx.x; e < E; e += blockDim.x) carry[1 + e] += counts[e];
   }
   if (t >= T) return;
+  if (blockIdx.y == 0) {
+    if (host_router && (int)threadIdx.x < 2 * k) host_router[(size_t)t * k * 2 + threadIdx.x] = router_out[(size_t)t * k * 2 + threadIdx.x];
+    if (host_meta && t == 0 && threadIdx.x < 16) host_meta[threadIdx.x] = meta[threadIdx.x];
+  }
   for (int d = (blockIdx.y * blockDim.x + threadIdx.x) * 4; d < H; d += gridDim.y * blockDim.x * 4) {
     float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
     // (on their way with the rows)

@@ -139,6 +139,7 @@ struct csk_moe_layer {
     int64_t T;
     const void *hidden, *router_in;
     void *router_out, *out;
+    const void* host_router;
     cudaStream_t stream;
     cudaGraphExec_t exec;
   };
@@ -157,17 +158,19 @@ namespace {
 // Host buffers of at most so many bytes each way go through page-locked staging of the handle's own if they are pageable.  32
 // tokens of the 32-expert layer: 200 -> 169 us a call, 80 (0.9 MB) 277 -> 268 (copies of pageable memory wait for the device, and the status had a
 // wait of its own).  One area for both ways: with two, creating a layer of 8192 tokens took 13.5 ms, with one 11.1.
+// The last kernel writes results, routing and status word there itself: copies by the driver, three of them behind the kernels, cost 13 to
+// 18 us more (1 token of that layer 72 -> 56, 4 95 -> 78, 16 140 -> 127, 32 182 -> 167, 80 280 -> 262).
 constexpr size_t kStagedMax = 1 << 20;
 // On the way in the driver takes up to 64 KB itself without a wait, and a second piece, whose host copy runs beside the first one's way
 // to the device, costs a launch.  By the driver / one piece / two, us: 2 tokens of that layer (22 KB) 76 / 78 / 89, 4 (45 KB) 97.5 / 103 / 107, 8 (90
 // KB) 134 / 129 / 131, 16 (180 KB) 155 / 148 / 151, 32 (360 KB) 176 / 173 / 169; 8 experts of 512 x 512, 8 tokens (16 KB) 51 / 51 / 63, 32 (64 KB)
 // 60 / 65 / 67, 80 (160 KB) 80 / 73 / 77, 200 (400 KB) 101 / 99 / 92.
 constexpr size_t kStagedInMin = 64 << 10, kStagedTwoPieces = 256 << 10;
-// Page-locked buffers need none on the way in.  On the way out a copy into them has to wait for the status word, so that a call that
-// fails leaves them alone: up to so many bytes that wait is dearer than a host copy.  The layer above, direct / staged, us: 1 token (11 KB)
-// 70.3 / 64.4, 2 81.7 / 76.6, 8 (90 KB) 121.9 / 118.7, 16 (180 KB) 145.3 / 147.4, 32 160.5 / 168.6, 80 186 / 216; 8 experts of 512 x 512, 32 tokens
-// (64 KB) 68.3 / 65.2, 80 (160 KB) 70.7 / 71.7.  (Staged on the way in, too: 32 tokens 173, 80 268.)
-constexpr size_t kStagedLockedMax = 128 << 10;
+// Page-locked buffers need none on the way in (32 tokens 160 without, 173 with).  On the way out a copy into them has to wait for the status
+// word, so that a call that fails leaves them alone: up to so many bytes that wait, and the copies, are dearer than a host copy.
+// The layer above, direct / staged, us: 1 token (11 KB) 62.6 / 47.0, 8 (90 KB) 114.7 / 101.1, 16 (180 KB) 134.0 / 121.9, 24 (270 KB) 139.0 / 130.9, 32
+// (361 KB) 145.5 / 139.5, 50 (564 KB) 155 / 166, 80 175 / 206; 128 experts of 2048 x 768, 30 tokens (240 KB) 122.4 / 111.0, 100 (800 KB) 159 / 186.
+constexpr size_t kStagedLockedMax = 384 << 10;
 
 int wide_stride(const csk_moe_layer* L) { return mx_mask_words(L->Lgu.recs) + mx_mask_words(L->Ld.recs); }
 
@@ -685,11 +688,17 @@ void finish_timings(csk_moe_layer* L, int n_marks, bool routed) {
   cudaEventElapsedTime(&L->last.total_ms, L->ev[0], L->ev[n_marks - 1]);
 }
 
+// Page-locked memory that the last kernel writes the routing (or null) and the words of d_meta to.
+struct HostResult {
+  float* router = nullptr;
+  int* meta = nullptr;
+};
+
 // The whole layer on device buffers.  only_expert >= 0 gives the dense output
 // of that single expert node.
 int forward_dev(csk_moe_layer* L, const float* d_hidden, int64_t T, const float* d_router_in,
                 float* d_router_out, float* d_out, int only_expert, cudaStream_t s, bool sync_check,
-                const float* d_residual = nullptr, const float* d_shared = nullptr, cudaEvent_t shared_ready = nullptr) {
+                const float* d_residual = nullptr, const float* d_shared = nullptr, cudaEvent_t shared_ready = nullptr, const HostResult& host = {}) {
   if (T <= 0 || T > L->max_T) return fail(L, CSK_ERR_NOMEM, "T=%lld outside (0, max_tokens=%lld]",
                                           (long long)T, (long long)L->max_T);
   if (L->has_slot_map)
@@ -752,7 +761,7 @@ int forward_dev(csk_moe_layer* L, const float* d_hidden, int64_t T, const float*
   launch_k(L->k > 4 ? k_combine<8> : k_combine<4>, dim3((unsigned)T, row_blocks), dim3(256), 0, s, L->pdl && !shared_ready, router, L->d_row_of_pair,
            (const float*)L->d_y, L->H, d_out, (int)T, L->k, L->H, (int)L->cfg.weight_before_ffn, (int)(only_expert >= 0),
            (const int*)L->d_meta, (const int*)L->d_counts, L->carry_active ? L->d_carry : (int*)nullptr, L->E, d_residual,
-           d_shared);
+           d_shared, host.router, host.meta);
   CSK_CUDA(L, cudaGetLastError());
   L->last.launches++;
   tm.mark();
@@ -1543,18 +1552,16 @@ int csk_moe_route_dev(csk_moe_layer* L, const float* d_hidden, int64_t T, float*
   return launch_router(L, d_hidden, T, d_router_out, pick(L, stream));
 }
 
-int csk_moe_forward_dev(csk_moe_layer* L, const float* d_hidden, int64_t T, const float* d_router_in,
-                        float* d_router_out, float* d_out, void* stream) {
-  if (check_layer(L)) return CSK_ERR_INVALID;
-  if (!d_hidden || !d_out) return fail(L, CSK_ERR_INVALID, "null argument");
-  CSK_CUDA(L, cudaSetDevice(L->cfg.device));
-  cudaStream_t s = pick(L, stream);
+// forward_dev, small batches as captured sequences
+static int forward_replayed(csk_moe_layer* L, const float* d_hidden, int64_t T, const float* d_router_in, float* d_router_out, float* d_out,
+                            cudaStream_t s, const HostResult& host = {}) {
+  auto enqueue = [&]() { return forward_dev(L, d_hidden, T, d_router_in, d_router_out, d_out, -1, s, false, nullptr, nullptr, nullptr, host); };
   constexpr int64_t kGraphMaxTokens = 512;
   if (!L->use_graphs || L->timing || L->debug_stall || L->debug_stall_router || T > kGraphMaxTokens || T <= 0 || T > L->max_T)
-    return forward_dev(L, d_hidden, T, d_router_in, d_router_out, d_out, -1, s, false);
+    return enqueue();
   for (auto& g : L->graphs)
     if (g.T == T && g.hidden == d_hidden && g.router_in == d_router_in && g.router_out == d_router_out &&
-        g.out == d_out && g.stream == s) {
+        g.out == d_out && g.host_router == host.router && g.stream == s) {
       CSK_CUDA(L, cudaGraphLaunch(g.exec, s));
       L->last_T = T;
       L->last_stream = s;
@@ -1565,13 +1572,13 @@ int csk_moe_forward_dev(csk_moe_layer* L, const float* d_hidden, int64_t T, cons
   cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
   if (cudaStreamIsCapturing(s, &st) != cudaSuccess || st != cudaStreamCaptureStatusNone) {
     cudaGetLastError();  // the caller is capturing this stream itself: just enqueue
-    return forward_dev(L, d_hidden, T, d_router_in, d_router_out, d_out, -1, s, false);
+    return enqueue();
   }
   if (cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal) != cudaSuccess) {
     cudaGetLastError();
-    return forward_dev(L, d_hidden, T, d_router_in, d_router_out, d_out, -1, s, false);
+    return enqueue();
   }
-  int rc = forward_dev(L, d_hidden, T, d_router_in, d_router_out, d_out, -1, s, false);
+  int rc = enqueue();
   cudaGraph_t graph = nullptr;
   cudaError_t ce = cudaStreamEndCapture(s, &graph);
   if (rc || ce != cudaSuccess || !graph) {
@@ -1579,7 +1586,7 @@ int csk_moe_forward_dev(csk_moe_layer* L, const float* d_hidden, int64_t T, cons
     if (graph) cudaGraphDestroy(graph);
     if (rc) return rc;
     L->use_graphs = false;  // capture is not possible here: fall back to plain launches for good
-    return forward_dev(L, d_hidden, T, d_router_in, d_router_out, d_out, -1, s, false);
+    return enqueue();
   }
   cudaGraphExec_t exec = nullptr;
   ce = cudaGraphInstantiate(&exec, graph, 0);
@@ -1587,15 +1594,23 @@ int csk_moe_forward_dev(csk_moe_layer* L, const float* d_hidden, int64_t T, cons
   if (ce != cudaSuccess || !exec) {
     cudaGetLastError();
     L->use_graphs = false;
-    return forward_dev(L, d_hidden, T, d_router_in, d_router_out, d_out, -1, s, false);
+    return enqueue();
   }
   if (L->graphs.size() >= 32) {
     cudaGraphExecDestroy(L->graphs.front().exec);
     L->graphs.erase(L->graphs.begin());
   }
-  L->graphs.push_back({T, d_hidden, d_router_in, d_router_out, d_out, s, exec});
+  L->graphs.push_back({T, d_hidden, d_router_in, d_router_out, d_out, host.router, s, exec});
   CSK_CUDA(L, cudaGraphLaunch(exec, s));
   return CSK_OK;
+}
+
+int csk_moe_forward_dev(csk_moe_layer* L, const float* d_hidden, int64_t T, const float* d_router_in,
+                        float* d_router_out, float* d_out, void* stream) {
+  if (check_layer(L)) return CSK_ERR_INVALID;
+  if (!d_hidden || !d_out) return fail(L, CSK_ERR_INVALID, "null argument");
+  CSK_CUDA(L, cudaSetDevice(L->cfg.device));
+  return forward_replayed(L, d_hidden, T, d_router_in, d_router_out, d_out, pick(L, stream));
 }
 
 // ---- the layer with the steps either side of it ------------------------------
@@ -1824,20 +1839,23 @@ int csk_moe_forward(csk_moe_layer* L, const float* hidden, int64_t T, const floa
       CSK_CUDA(L, cudaMemcpyAsync(L->d_hidden, hidden, row_bytes, cudaMemcpyHostToDevice, s));
     }
     if (router_in) CSK_CUDA(L, cudaMemcpyAsync(L->d_router, staged_in ? staged_route : router_in, route_bytes, cudaMemcpyHostToDevice, s));
-    int rc = csk_moe_forward_dev(L, L->d_hidden, T, router_in ? L->d_router : nullptr, nullptr, L->d_out, s);
+    // Results that the host copies are written to the staging area by the last kernel (where the inputs went out from, too: the stream has
+    // taken those first), with the routing and the status word.
+    const bool locked = bytes <= kStagedLockedMax;
+    const bool staged_out = fits && to_copy(out, locked) && to_copy(router_out, true);
+    HostResult host;
+    if (staged_out) host = {router_out ? staged_route : nullptr, L->h_meta};
+    int rc = forward_replayed(L, L->d_hidden, T, router_in ? L->d_router : nullptr, nullptr, staged_out ? L->h_staged : L->d_out, s, host);
     if (rc) {
       if (staged_in) cudaStreamSynchronize(s);  // the copies in have left the staging area
       return rc;
     }
-    // (asked while the kernels run)
-    const bool locked = bytes <= kStagedLockedMax;
-    const bool staged_out = fits && to_copy(out, locked) && to_copy(router_out, true);
     if (staged_out) {
-      // (where the inputs went out from, too: the stream has taken those first)
-      CSK_CUDA(L, cudaMemcpyAsync(L->h_staged, L->d_out, row_bytes, cudaMemcpyDeviceToHost, s));
-      if (router_out) CSK_CUDA(L, cudaMemcpyAsync(staged_route, L->d_router, route_bytes, cudaMemcpyDeviceToHost, s));
+      CSK_CUDA(L, cudaStreamSynchronize(s));
+      rc = report_status(L, L->h_meta[3] | L->h_meta[8], s);
+    } else {
+      rc = check_device_status(L, s);
     }
-    rc = check_device_status(L, s);
     if (rc) return rc;
     if (L->timing && L->n_marks > 1) finish_timings(L, L->n_marks, L->last_routed);
     if (staged_out) {

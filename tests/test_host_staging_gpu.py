@@ -74,3 +74,8 @@ def test_page_locked_buffers(gpu_lib, T, locked_in, locked_out, mixed):
         lay.forward(x, router_out=x_route, out=got, router_out_buf=got_ro)
     assert np.array_equal(got, out) and np.array_equal(got_ro, ro)
     lay.close()
+
+
+@pytest.mark.parametrize("T", [95, 96])  # 384 KB of results and routing are 95 rows
+def test_page_locked_results_at_the_line(gpu_lib, T):
+    test_page_locked_buffers(gpu_lib, T, True, True, False)
