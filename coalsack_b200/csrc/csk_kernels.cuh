@@ -253,7 +253,8 @@ __device__ __forceinline__ float4 mul4_rn(const float4& a, const float4& b) {
 }
 
 // A batch of 4 G columns in registers: the lane's expert row and the warp's token rows.
-__host__ __device__ constexpr int router_groups(int tt) { return tt == 1 ? 8 : 4; }
+// (two warps a scheduler hide the loads by themselves: 850 tokens of 128 experts 46.2 us with batches of eight columns, 47.5 with sixteen)
+__host__ __device__ constexpr int router_groups(int tw, int tt) { return tw > 4 ? 2 : tt == 1 ? 8 : 4; }
 template <int TT, int G>
 struct ChainBatch {
   float4 w[G], h[G][TT];
@@ -313,8 +314,10 @@ __device__ __forceinline__ bool mbar_wait_nap(uint32_t bar, uint32_t parity, vol
 
 __host__ __device__ constexpr int router_producer_warps(bool packed) { return packed ? 1 : 4; }
 
+// (Blocks of 4 x 4 tokens, which large batches of one group of experts take, are two an SM: left alone, the compiler takes registers for one, 32
+// experts of 2880 columns, 8192 tokens 89 -> 107 us.)
 template <int TW, int TT, int CH, bool PACKED>
-__global__ void __launch_bounds__((TW + router_producer_warps(PACKED)) * 32, 1)
+__global__ void __launch_bounds__((TW + router_producer_warps(PACKED)) * 32, TW * TT == 16 ? 2 : 1)
 k_router_logits(const RouterArgs A) {
   extern __shared__ __align__(128) uint8_t router_smem_raw[];
   constexpr int LD = CH + kRouterPad;
@@ -413,7 +416,7 @@ k_router_logits(const RouterArgs A) {
       float acc[TT];
 #pragma unroll
       for (int i = 0; i < TT; ++i) acc[i] = 0.f;
-      constexpr int G = router_groups(TT), BC = 4 * G, NB = CH / BC;  // columns of a batch, batches of a chunk
+      constexpr int G = router_groups(TW, TT), BC = 4 * G, NB = CH / BC;  // columns of a batch, batches of a chunk
       static_assert(NB % 2 == 0 && 32 % BC == 0, "batches");
       ChainBatch<TT, G> even, odd;
       float4 now[TT];
@@ -617,12 +620,10 @@ inline RouterWave router_wave(int groups, int sm_count) {
 
 // The fewest tokens per block with which the blocks are one wave: a block's time goes by its chains per thread and, from four warps
 // on, by its shared-memory reads (a row of weights per lane costs 4 cycles per four columns, a token row 2), so that a second
-// wave is dearer than more chains in one.  `wave`: see router_wave.  One launch, us (6 of
-// them the events), 2880 columns, by warps x tokens of a warp: 128 experts, 64 tokens 1x1 21.5, 2x1 19.6; 128 tokens 2x1 21.7, 4x1 21.7;
-// 200 4x1 35.8, 4x2 24.0; 333 4x2 38.0, 4x3 30.9, 4x4 35.0; 512 4x3 44.1, 4x4 34.0; 700 4x4 60.6, 8x3 45.0, 8x4 52.4; 1024 8x3 83, 8x4 53;
-// 32 experts, 333 2x1 21.9, 4x1 19.9; 1024 4x1 28.1, 4x2 24.2; 2048 4x2 36.2, 4x4 34.8; 4096 4x4 52.6, 8x4 54.4; 8192 4x4 97, 8x4 101.
-// Before (a producer for the weights only, loads at their use, up to 16 tokens a block and no cluster): 8 tokens 20.8, 64 21.6, 333 46.9, 1024
-// 64; 32 experts, 4096 tokens 62.
+// wave is dearer than more chains in one.  `wave`: see router_wave.  A launch among others, us, 2880 columns, by the shape taken (warps x tokens
+// of a warp): 128 experts, 8 tokens 1x1 11.1; 50 2x1 13.1; 100 4x1 13.6; 200 4x2 17.6; 333 4x3 21.4; 512 4x4 26.2; 700 8x3 37.9; 1000 8x4 46.1;
+// 32 experts, 333 4x1 13.1; 1024 4x2 17.7; 2048 4x4 28.4; 4096 8x4 47.0; 6000 4x4 71.2 and 8192 4x4 89.7, two blocks an SM (8x4 95).  Other shapes: 100
+// tokens 2x2 17.8; 592 8x2 38.3; 700 4x6 44.2; 1000 4x8 53.6.
 // wg_few / wg_many: the weights packed for the two chunk widths (PACKED) or both the plain [E,H] matrix.  token_slots: tokens the
 // grid is sized for (a.T, or for a list-driven launch the most entries the list can have).
 template <bool PACKED>

@@ -250,9 +250,9 @@ int launch_router(csk_moe_layer* L, const float* d_hidden, int64_t T, float* d_r
   constexpr int64_t kCertifiedMaxTokens = 4;
   // With many tokens the chain is held by its arithmetic, token x expert; the certified pass on the tensor cores costs
   // little per token, but four launches and the chain of the few percent it cannot separate.  Chain / certified, us, normal
-  // rows: 128 experts, 2880 columns: 1 token 14.6 / (FMA pass) 15.6, 64 14.6 / (FMA) 25, 512 30 / (FMA) 77, 1024 49 / 44, 2048 95 / 62,
-  // 8192 369 / 121; 128 x 2048: 1024 37 / 38, 2048 71 / 48; 64 x 2880: 2048 49 / 48, 4096 96 / 73; 256 x 2880: 256 56 / (FMA) 79, 512
-  // 95 / 51; 512 x 2048: 256 54 / (FMA) 95, 512 86 / 63; 1024 x 2048: 128 54 / (FMA) 98, 256 86 / 72; 32 x 2880: 4096 50 / 104, 8192 92 / 146
+  // rows: 128 experts, 2880 columns: 64 tokens 13 / (FMA pass) 25, 512 26 / 34, 1024 47 / 35, 2048 95 / 43; 128 x 2048: 600 29 / 32, 1000 36 / 32; 64 x 2880:
+  // 1024 26 / 34, 2048 48 / 44, 3000 96 / 49; 256 x 2880: 256 38 / 39, 512 54 / 39; 512 x 2048: 256 45 / (FMA) 95, 512 79 / 44; 128 x 512: 1000 14 /
+  // 21; 32 x 2880: 4096 47 / 104, 8192 90 / 146
   // (a digit matrix has 128 rows whatever the experts).  The line is where the two meet: with half as many pairs the FMA pass, which
   // the certified mode then takes, is the slower one everywhere; with 512 experts and more (few tokens, many digit matrices) they
   // meet at twice as many.
