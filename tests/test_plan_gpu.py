@@ -88,3 +88,23 @@ def test_plan_of_a_thread_per_pair(gpu_lib, port, E, k, T, path):
         forward(absent)
     assert np.array_equal(forward(ro), out)
     lay.close()
+
+
+@pytest.mark.parametrize("k", [4, 5, 8, 9, 16])  # slots asked for at once, and one more
+def test_combine_adds_the_slots_in_order(gpu_lib, port, k):
+    """Block calls (with a residual) and plain ones: the routed sum in router order, then the residual, bit for bit from one another."""
+    sh = synth.tiny(seed=k, E=20, k=k, H=96, F=32, T=11, has_bias=True)
+    h, Wg, rb, ex = cases.layer_inputs(sh, router_scale=30.0)
+    lay = MoeLayer.from_shape(sh)
+    lay.set_router(Wg, rb)
+    lay.load_experts(ex)
+    nw = np.ones(96, np.float32)
+    lay.set_ffn_norm(nw, 1e-5)
+    n = port.rmsnorm(h, nw, 1e-5)
+    out, ro = lay.forward(n)
+    want, _ = port.moe_layer(n, Wg, rb, ex, k, sh.act, router_out=ro)
+    mx, mr = cases.err_stats(out, want)
+    assert mx <= cases.MAX_ABS_OVER_RMS and mr <= cases.MEAN_REL, (mx, mr)
+    block, ro2 = lay.block_forward(h)
+    assert np.array_equal(ro, ro2) and np.array_equal((h + out).astype(np.float32), block)
+    lay.close()

@@ -239,3 +239,29 @@ def test_which_batches_take_the_certified_pass_by_themselves(gpu_lib, port, E, T
     assert np.array_equal(lay.route(h)[clean][..., 0], want[clean][..., 0])
     assert (lay.router_stats()[0] == T) == certified
     lay.close()
+
+
+@pytest.mark.parametrize("E,k,H,T", [
+    (5, 2, 2880, 3), (33, 4, 96, 1),         # an odd number of experts: their parts are copied one by one; one part
+    (129, 8, 2880, 4), (1023, 16, 64, 2),    # a second and an eighth turn of a thread's experts
+    (1024, 3, 4096, 4), (128, 16, 2880, 70), # the most parts x experts of a token; more tokens than one block of the logits
+])
+def test_certified_finish_edges(gpu_lib, port, E, k, H, T):
+    """The certified pass of a few tokens where its loops over parts and experts end; a row of zeros goes through the chain."""
+    rng = np.random.default_rng(E + H + T)
+    Wg = (rng.standard_normal((E, H)) * 0.05).astype(np.float32)
+    rb = (rng.standard_normal(E) * 0.01).astype(np.float32)
+    h = rng.standard_normal((T, H)).astype(np.float32)
+    h[T - 1] = 0
+    for bias in (rb, None):
+        lay = _router_layer(E, k, H, Wg, bias, T)
+        got = lay.route(h)
+        want = port.router(h, Wg, bias, k)
+        rows = slice(None) if bias is not None else slice(0, T - 1)  # (without a bias the last row's logits are all equal: any order)
+        assert np.array_equal(got[rows, :, 0], want[rows, :, 0])
+        # A logit of either kind is within b = 2^-24 (sum of |partial sums| + sum of |terms|) of the exact one, so the difference of two logits
+        # moves by no more than 4 b and a weight by that share of it (and by the rounding of exp and the division).
+        terms = h[:, None].astype(np.float64) * Wg[got[..., 0].astype(int) % E]
+        b = 2.0 ** -24 * (np.abs(np.cumsum(terms, -1)).sum(-1) + np.abs(terms).sum(-1)).max(-1, keepdims=True)
+        assert (np.abs(got[..., 1] - want[..., 1])[rows] <= (want[..., 1] * (4 * b + 2e-6))[rows]).all()
+        lay.close()
