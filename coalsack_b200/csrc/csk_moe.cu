@@ -245,8 +245,9 @@ int launch_router(csk_moe_layer* L, const float* d_hidden, int64_t T, float* d_r
   a.k = L->k;
   a.sigmoid = L->cfg.sigmoid_gating;
   // Of a handful of tokens the certified pass (three launches: sliced FMA logits, certification, chain over the few tokens it
-  // could not separate) spreads the columns over the machine, where a chain is alone: the step of 1 token of the 128-expert layer 42.4 us,
-  // with the chain 46.8 (the router alone, without its neighbours' overlap, 15.6 and 14.6); of 8 tokens it is behind.
+  // could not separate) spreads the columns over the machine, where a chain is alone.  A layer's step over fresh inputs, chain / certified, us: 128
+  // experts, 2880 columns, 1 token 35.4 / 30.9, 2 43.3 / 38.9, 4 59.1 / 55.9, 8 84.8 / 83.6, 16 126.8 / 127.3; 128 x 2048, 1 26.8 / 24.2, 4 35.9 / 36.3, 6
+  // 40.0 / 41.1.  (Rows that it cannot separate, like rows of zeros without a bias, cost both.)
   constexpr int64_t kCertifiedMaxTokens = 4;
   // With many tokens the chain is held by its arithmetic, token x expert; the certified pass on the tensor cores costs
   // little per token, but four launches and the chain of the few percent it cannot separate.  Chain / certified, us, normal
