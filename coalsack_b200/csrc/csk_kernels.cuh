@@ -314,10 +314,11 @@ __device__ __forceinline__ bool mbar_wait_nap(uint32_t bar, uint32_t parity, vol
 
 __host__ __device__ constexpr int router_producer_warps(bool packed) { return packed ? 1 : 4; }
 
-// (Blocks of 4 x 4 tokens, which large batches of one group of experts take, are two an SM: left alone, the compiler takes registers for one, 32
-// experts of 2880 columns, 8192 tokens 89 -> 107 us.)
-template <int TW, int TT, int CH, bool PACKED>
-__global__ void __launch_bounds__((TW + router_producer_warps(PACKED)) * 32, TW * TT == 16 ? 2 : 1)
+// PER_SM: blocks that an SM has to have registers for.  Two for blocks of 4 x 4 tokens in more than one wave (32 experts of 2880 columns, 8192 tokens
+// 107 us with registers for one, 90 with two; plain weights 107 and 95).  In one wave an SM has one block anyhow, and registers for two take the
+// second set of loads from it: 2000 tokens 29.3 us with two, 28.1 with one, plain weights 33.5 and 31.6; 512 tokens of 128 experts 28.2 and 27.0.
+template <int TW, int TT, int CH, bool PACKED, int PER_SM = 1>
+__global__ void __launch_bounds__((TW + router_producer_warps(PACKED)) * 32, PER_SM)
 k_router_logits(const RouterArgs A) {
   extern __shared__ __align__(128) uint8_t router_smem_raw[];
   constexpr int LD = CH + kRouterPad;
@@ -542,9 +543,9 @@ k_router_logits(const RouterArgs A) {
   }
 }
 
-template <int TW, int TT, int CH, bool PACKED>
+template <int TW, int TT, int CH, bool PACKED, int PER_SM = 1>
 cudaError_t router_prepare_one() {
-  return cudaFuncSetAttribute(k_router_logits<TW, TT, CH, PACKED>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+  return cudaFuncSetAttribute(k_router_logits<TW, TT, CH, PACKED, PER_SM>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                               (int)router_smem_bytes(TW * TT, CH, PACKED ? 32 * kRouterClusterGroups : 0));
 }
 template <bool PACKED>
@@ -555,6 +556,7 @@ cudaError_t router_prepare_set() {
   if (e == cudaSuccess) e = router_prepare_one<4, 2, kRouterChunkMany, PACKED>();
   if (e == cudaSuccess) e = router_prepare_one<4, 3, kRouterChunkMany, PACKED>();
   if (e == cudaSuccess) e = router_prepare_one<4, 4, kRouterChunkMany, PACKED>();
+  if (e == cudaSuccess) e = router_prepare_one<4, 4, kRouterChunkMany, PACKED, 2>();
   if (e == cudaSuccess) e = router_prepare_one<8, 3, kRouterChunkMany, PACKED>();
   if (e == cudaSuccess) e = router_prepare_one<8, 4, kRouterChunkMany, PACKED>();
   return e;
@@ -571,7 +573,7 @@ struct RouterWave {
   int alone;  // blocks resident at once without clusters
 };
 
-template <int TW, int TT, int CH, bool PACKED>
+template <int TW, int TT, int CH, bool PACKED, int PER_SM = 1>
 void launch_router_one(RouterArgs a, int token_slots, RouterWave wave, cudaStream_t s, bool pdl) {
   const unsigned groups = (unsigned)((a.E + 31) / 32);
   constexpr int BT = TW * TT;
@@ -590,7 +592,7 @@ void launch_router_one(RouterArgs a, int token_slots, RouterWave wave, cudaStrea
   attr[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = pdl ? 2 : 1;
-  cudaLaunchKernelEx(&cfg, k_router_logits<TW, TT, CH, PACKED>, a);
+  cudaLaunchKernelEx(&cfg, k_router_logits<TW, TT, CH, PACKED, PER_SM>, a);
 }
 
 // An SM each, but clusters leave some SMs of a GPC over (with a fixed nine tenths of the SMs, 64 tokens of 256 experts took two waves
@@ -647,7 +649,8 @@ inline void launch_router_logits(RouterArgs a, const float* wg_few, const float*
   a.wg = wg_many;
   if (one_wave(8)) return launch_router_one<4, 2, kRouterChunkMany, PACKED>(a, token_slots, wave, s, pdl);
   if (one_wave(12)) return launch_router_one<4, 3, kRouterChunkMany, PACKED>(a, token_slots, wave, s, pdl);
-  if (one_wave(16) || (!one_wave(32) && groups == 1)) return launch_router_one<4, 4, kRouterChunkMany, PACKED>(a, token_slots, wave, s, pdl);
+  if (one_wave(16)) return launch_router_one<4, 4, kRouterChunkMany, PACKED>(a, token_slots, wave, s, pdl);
+  if (!one_wave(32) && groups == 1) return launch_router_one<4, 4, kRouterChunkMany, PACKED, 2>(a, token_slots, wave, s, pdl);
   if (one_wave(24)) return launch_router_one<8, 3, kRouterChunkMany, PACKED>(a, token_slots, wave, s, pdl);
   launch_router_one<8, 4, kRouterChunkMany, PACKED>(a, token_slots, wave, s, pdl);
 }

@@ -127,3 +127,28 @@ def test_equal_logits_go_to_the_lower_expert(gpu_lib, port, E, step):
         want = [e for b in order[t, :k] for e in range(b, E, step)][:k]
         assert got[t].tolist() == want, t
     lay.close()
+
+
+@pytest.mark.parametrize("E", [5, 32, 64])
+@pytest.mark.parametrize("tokens", [1, 2, 4, 8, 12, 16, 24, 32])
+@pytest.mark.parametrize("more", [0, 1])
+def test_plain_weights_at_the_edges_of_their_launches(gpu_lib, port, E, tokens, more):
+    """The entry point without a handle: the last batch of each launch shape (one wave of blocks of so many tokens) and the first of the
+    next.  Blocks of 16 tokens have one form for one wave and another for more."""
+    import torch
+    lib = gpu_lib
+    blocks = torch.cuda.get_device_properties(0).multi_processor_count
+    T, H, k = blocks // (-(-E // 32)) * tokens + more, 160, 4
+    rng = np.random.default_rng(E + T)
+    h = rng.standard_normal((T, H)).astype(np.float32)
+    Wg = (rng.standard_normal((E, H)) * 0.02).astype(np.float32)
+    rb = (rng.standard_normal(E) * 0.01).astype(np.float32)
+    h_d, w_d, b_d = (torch.from_numpy(x).cuda() for x in (h, Wg, rb))
+    out = torch.full((T, k, 2), -1.0, device="cuda")
+    torch.cuda.synchronize()
+    assert lib.csk_moe_route_static(h_d.data_ptr(), T, H, w_d.data_ptr(), b_d.data_ptr(), E, k, 0, out.data_ptr(), None) == 0
+    torch.cuda.synchronize()
+    assert lib.csk_moe_route_static_status() == 0
+    got, want = out.cpu().numpy(), port.router(h, Wg, rb, k, False)
+    assert np.array_equal(got[..., 0], want[..., 0])
+    assert np.allclose(got[..., 1], want[..., 1], rtol=0, atol=6e-7)  # (as above)
