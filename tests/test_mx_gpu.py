@@ -184,6 +184,38 @@ def test_outliers_lose_no_precision(gpu_lib, where, times):
     lay.close()
 
 
+@pytest.mark.parametrize("where", ["rows", "activated"])
+def test_wide_blocks_past_the_first_word_of_marks(gpu_lib, where):
+    """33 records: only the last one, marked in the second word, holds wide blocks (channels at 10^4 times the others that nothing reads).
+    Without its second run those blocks' other values would be off by 10 %."""
+    H, F, T = (4224, 64, 9) if where == "rows" else (64, 4224, 9)
+    act = 0 if where == "rows" else 1
+    sh = synth.tiny(seed=377, E=1, k=1, H=H, F=F, T=T, has_bias=True, act=act)
+    h, Wg, rb, ex = cases.layer_inputs(sh)
+    ex["w_gate"], ex["w_up"] = ([_scaled(w[0], -4)] for w in (ex["w_gate"], ex["w_up"]))
+    big = np.array([4100, 4133, 4170, 4200])
+    if where == "rows":
+        h[:, big] = 1e4
+        for n in ("w_gate", "w_up"):
+            ex[n][0] = _zero_columns(ex[n][0], F, H, big)
+    else:
+        ex["b_gate"][0][big], ex["b_up"][0][big] = 6.0, 5e3
+        ex["w_down"][0] = _zero_columns(ex["w_down"][0], H, F, big)
+    want = _mlp64(h, ex, H, F, act)
+    lay = MoeLayer.from_shape(sh)
+    lay.set_router(Wg, rb)
+    lay.load_experts(ex)
+    route = np.zeros((T, 1, 2), np.float32)
+    route[..., 1] = 1
+    err = {}
+    for name, path in (("fp16", PATH_TILE), ("digits", PATH_STREAM)):
+        lay.set_path(path)
+        out, _ = lay.forward(h, router_out=route)
+        err[name] = np.linalg.norm(out - want) / np.linalg.norm(want)
+    assert err["digits"] <= err["fp16"] + 2e-6, err  # (as above)
+    lay.close()
+
+
 def _scaled(blocks, by):
     """The matrix times 2^by."""
     b = np.asarray(blocks).reshape(-1, 17).copy()
