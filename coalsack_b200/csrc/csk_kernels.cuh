@@ -1372,12 +1372,15 @@ __global__ void __launch_bounds__(256) k_dense_rows(const float* __restrict__ hi
 // ---------------------------------------------------------------------------
 //
 // Bound by HBM (k rows of y in, one out).  AT_ONCE slots' rows are requested at once: one at a time a
-// step of 8192 tokens took 2046 us, with four 2011; 2048 tokens of eight slots 318 and 306.  A few tokens are bound by the
-// latency of their loads: a row is then dealt to several blocks (gridDim.y), so that a thread has one round of them (8 tokens of
-// 2880 columns 7.9 -> 4.5 us, profiler), the shared expert's and the residual row with it (16 tokens of eight slots, a step: four
-// slots at once and those two rows after them 64.0 us, now 62.5).
+// step of 8192 tokens took 2046 us, with four 2011; 2048 tokens of eight slots 318 and 306.
+// Few tokens (FEW) are bound by the latency of their loads: up to eight slots' rows are requested at once, and the shared expert's and the
+// residual row with them (16 tokens of eight slots, a step: four at once and those two rows after them 64.0 us, now 62.5); of fewer than four an
+// SM a row is dealt to several blocks (gridDim.y), so that a thread has one round of loads (8 tokens of 2880 columns 7.9 -> 4.5 us, profiler).
+// Many tokens need blocks on an SM more than loads of a block: eight of them, with 32 registers a thread (profiler, cold caches; in
+// brackets with the few tokens' form, whose registers leave room for six or four): 8192 tokens, four slots of 512 columns 16.5 us (18.5); 4096, two
+// of 1024 11.2 (12.5); 2048, one of 2048 8.5 (9.7); 2048, eight of 2048 23.9 (25.1).
 // The rows are read for the last time, so they are the first to leave L2 (a step of 2048 tokens of eight slots 244.5 -> 240.6, of 4096
-// of four 768.5 -> 766.1).
+// of four level; this kernel alone, 4096 tokens, eight slots of 2048 columns 57 -> 47, 8192 tokens, four of 2880 82 -> 76).
 //
 // carry (optional; the host entry point that runs a batch in several passes): block 0 folds this
 // pass's status word into a sticky one and adds its per-expert row counts to running totals --
@@ -1385,13 +1388,12 @@ __global__ void __launch_bounds__(256) k_dense_rows(const float* __restrict__ hi
 //
 // host_router, host_meta (optional): page-locked memory that the routing and the 16 words of `meta` go to beside the results, which
 // `out` may be in then, too.
-template <int AT_ONCE>
-__global__ void __launch_bounds__(256) k_combine(const float* __restrict__ router_out, const int* __restrict__ row_of_pair,
+template <int AT_ONCE, bool FEW>
+__global__ void __launch_bounds__(256, !FEW ? 8 : AT_ONCE > 4 ? 4 : 6) k_combine(const float* __restrict__ router_out, const int* __restrict__ row_of_pair,
                           const float* __restrict__ y, int ldy, float* __restrict__ out, int T,
                           int k, int H, int unweighted, int dense_single,
-                          const int* __restrict__ meta = nullptr, const int* __restrict__ counts = nullptr,
-                          int* __restrict__ carry = nullptr, int E = 0, const float* residual = nullptr,
-                          const float* shared_out = nullptr, float* host_router = nullptr, int* host_meta = nullptr) {
+                          const int* __restrict__ meta, const int* __restrict__ counts, int* __restrict__ carry, int E,
+                          const float* residual, const float* shared_out, float* host_router, int* host_meta) {
   __shared__ int s_row[kMaxTopK];
   __shared__ float s_w[kMaxTopK];
   const int t = blockIdx.x;
@@ -1414,10 +1416,10 @@ __global__ void __launch_bounds__(256) k_combine(const float* __restrict__ route
   }
   for (int d = (blockIdx.y * blockDim.x + threadIdx.x) * 4; d < H; d += gridDim.y * blockDim.x * 4) {
     float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
-    // (on their way with the rows)
+    // (FEW: on their way with the rows)
     float4 sh, r;
-    if (shared_out) sh = *reinterpret_cast<const float4*>(shared_out + (size_t)t * H + d);
-    if (residual) r = *reinterpret_cast<const float4*>(residual + (size_t)t * H + d);
+    if (FEW && shared_out) sh = *reinterpret_cast<const float4*>(shared_out + (size_t)t * H + d);
+    if (FEW && residual) r = *reinterpret_cast<const float4*>(residual + (size_t)t * H + d);
     bool done = false;
     for (int j0 = 0; j0 < k && !done; j0 += AT_ONCE) {
       float4 v[AT_ONCE];
@@ -1440,6 +1442,7 @@ __global__ void __launch_bounds__(256) k_combine(const float* __restrict__ route
       }
     }
     if (shared_out) {
+      if (!FEW) sh = *reinterpret_cast<const float4*>(shared_out + (size_t)t * H + d);
       // the shared expert's dense FFN on the same rows: add(merge output, shared output), llm_engine.cpp:766-769
       acc.x = __fadd_rn(acc.x, sh.x);
       acc.y = __fadd_rn(acc.y, sh.y);
@@ -1447,6 +1450,7 @@ __global__ void __launch_bounds__(256) k_combine(const float* __restrict__ route
       acc.w = __fadd_rn(acc.w, sh.w);
     }
     if (residual) {
+      if (!FEW) r = *reinterpret_cast<const float4*>(residual + (size_t)t * H + d);
       // the residual connection around the layer: add(residual, merge output), llm_engine.cpp:773-777
       acc.x = __fadd_rn(r.x, acc.x);
       acc.y = __fadd_rn(r.y, acc.y);

@@ -695,6 +695,28 @@ struct HostResult {
   int* meta = nullptr;
 };
 
+// What k_combine does beside the sums, see there.
+struct CombineArgs {
+  bool dense_single = false;
+  const int *meta = nullptr, *counts = nullptr;
+  int* carry = nullptr;
+  const float *residual = nullptr, *shared = nullptr;
+  HostResult host;
+};
+
+// The rows of y (places in d_row_of_pair) to the tokens' results: of the layer, of the merge node, of expert parallelism.
+void launch_combine(csk_moe_layer* L, const float* router, const float* y, int64_t T, float* out, cudaStream_t s, bool pdl,
+                    const CombineArgs& c = {}) {
+  const unsigned row_blocks = T < 4 * L->sm_count ? (unsigned)ceil_div(L->H, 1024) : 1u;
+  // As long as its blocks are resident at once (of eight slots a little longer) the form for few tokens is the quicker one.  Few / many, a step, us:
+  // four slots of 2880 columns, 600 tokens 60.2 / 62.3, 740 63.9 / 66.1, 820 67.9 / 69.3, 1000 74.4 / 74.2; eight of 2048, 600 60.1 / 61.6, 740 65.4 / 66.1,
+  // 900 71.8 / 71.7, 1000 72.9 / 72.4; eight of 512, 740 36.1 / 35.5.
+  const bool few = T <= (L->k > 4 ? 5 : 6) * L->sm_count;
+  launch_k(!few ? k_combine<4, false> : L->k > 4 ? k_combine<8, true> : k_combine<4, true>, dim3((unsigned)T, row_blocks), dim3(256), 0, s, pdl, router,
+           L->d_row_of_pair, y, L->H, out, (int)T, L->k, L->H, (int)L->cfg.weight_before_ffn, (int)c.dense_single, c.meta, c.counts, c.carry,
+           L->E, c.residual, c.shared, c.host.router, c.host.meta);
+}
+
 // The whole layer on device buffers.  only_expert >= 0 gives the dense output
 // of that single expert node.
 int forward_dev(csk_moe_layer* L, const float* d_hidden, int64_t T, const float* d_router_in,
@@ -757,12 +779,15 @@ int forward_dev(csk_moe_layer* L, const float* d_hidden, int64_t T, const float*
   if (rc) return rc;
   // the shared expert's rows come from another stream: the combine is the first kernel that reads them
   if (shared_ready) CSK_CUDA(L, cudaStreamWaitEvent(s, shared_ready, 0));
-  // (few tokens: a row dealt to several blocks)
-  const unsigned row_blocks = T < 4 * L->sm_count ? (unsigned)ceil_div(L->H, 1024) : 1u;
-  launch_k(L->k > 4 ? k_combine<8> : k_combine<4>, dim3((unsigned)T, row_blocks), dim3(256), 0, s, L->pdl && !shared_ready, router, L->d_row_of_pair,
-           (const float*)L->d_y, L->H, d_out, (int)T, L->k, L->H, (int)L->cfg.weight_before_ffn, (int)(only_expert >= 0),
-           (const int*)L->d_meta, (const int*)L->d_counts, L->carry_active ? L->d_carry : (int*)nullptr, L->E, d_residual,
-           d_shared, host.router, host.meta);
+  CombineArgs c;
+  c.dense_single = only_expert >= 0;
+  c.meta = L->d_meta;
+  c.counts = L->d_counts;
+  c.carry = L->carry_active ? L->d_carry : nullptr;
+  c.residual = d_residual;
+  c.shared = d_shared;
+  c.host = host;
+  launch_combine(L, router, L->d_y, T, d_out, s, L->pdl && !shared_ready, c);
   CSK_CUDA(L, cudaGetLastError());
   L->last.launches++;
   tm.mark();
@@ -1998,8 +2023,7 @@ int csk_moe_merge(csk_moe_layer* L, const float* router_out, int64_t T, const fl
   CSK_CUDA(L, cudaMemcpyAsync(L->d_y, packed.data(), sizeof(float) * packed.size(), cudaMemcpyHostToDevice, s));
   CSK_CUDA(L, cudaMemcpyAsync(L->d_row_of_pair, rows.data(), sizeof(int) * rows.size(), cudaMemcpyHostToDevice, s));
   CSK_CUDA(L, cudaMemcpyAsync(L->d_router, router_out, sizeof(float) * T * L->k * 2, cudaMemcpyHostToDevice, s));
-  k_combine<4><<<(unsigned)T, 256, 0, s>>>(L->d_router, L->d_row_of_pair, L->d_y, L->H, L->d_out, (int)T,
-                                        L->k, L->H, L->cfg.weight_before_ffn, 0, nullptr, nullptr, nullptr, 0);
+  launch_combine(L, L->d_router, L->d_y, T, L->d_out, s, false);
   CSK_CUDA(L, cudaGetLastError());
   CSK_CUDA(L, cudaMemcpyAsync(out, L->d_out, sizeof(float) * T * L->H, cudaMemcpyDeviceToHost, s));
   CSK_CUDA(L, cudaStreamSynchronize(s));
@@ -2377,8 +2401,7 @@ int csk_moe_ep_combine_dev(csk_moe_layer* L, const float* d_back, int64_t T, flo
                                   (long long)T, (long long)L->last_T);
   CSK_CUDA(L, cudaSetDevice(L->cfg.device));
   cudaStream_t s = pick(L, stream);
-  k_combine<4><<<(unsigned)T, 256, 0, s>>>(L->d_router, L->d_row_of_pair, d_back, L->H, d_out, (int)T, L->k,
-                                        L->H, L->cfg.weight_before_ffn, 0, nullptr, nullptr, nullptr, 0);
+  launch_combine(L, L->d_router, d_back, T, d_out, s, false);
   CSK_CUDA(L, cudaGetLastError());
   if (d_router_out)
     CSK_CUDA(L, cudaMemcpyAsync(d_router_out, L->d_router, sizeof(float) * T * L->k * 2,

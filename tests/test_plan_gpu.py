@@ -108,3 +108,63 @@ def test_combine_adds_the_slots_in_order(gpu_lib, port, k):
     block, ro2 = lay.block_forward(h)
     assert np.array_equal(ro, ro2) and np.array_equal((h + out).astype(np.float32), block)
     lay.close()
+
+
+@pytest.mark.parametrize("k", [1, 2, 3, 4, 5, 8, 9, 16])
+@pytest.mark.parametrize("T", [7, 700, 1500])  # fewer tokens than four an SM, than five, and more than six: two forms of the combine
+def test_merge_adds_the_slots_one_after_the_other(gpu_lib, k, T):
+    """Rows of very different size, so that another order gives other bits: equal to products and sums in fp32, slot by slot."""
+    E, H = k + 3, 96
+    rng = np.random.default_rng(100 * k + T)
+    y = (rng.standard_normal((E, T, H)) * 10.0 ** rng.uniform(-3, 3, (E, T, 1))).astype(np.float32)
+    ro = rng.uniform(0.1, 1.0, (T, k, 2)).astype(np.float32)
+    ro[..., 0] = [rng.permutation(E)[:k] for _ in range(T)]
+    absent = int(ro[0, k - 1, 0]) if k > 1 else E - 1  # an expert without output adds nothing
+    lay = MoeLayer(E, k, H, 32, has_bias=False, max_tokens=T)
+    got = lay.merge(ro, [None if e == absent else y[e] for e in range(E)])
+
+    def in_order(slots):
+        acc = np.zeros((T, H), np.float32)
+        for j in slots:
+            e = ro[:, j, 0].astype(int)
+            term = ro[:, j, 1:] * y[e, np.arange(T)]
+            acc = np.where((e != absent)[:, None], acc + term, acc)
+        return acc
+
+    assert np.array_equal(got, in_order(range(k)))
+    assert k < 4 or not np.array_equal(got, in_order(reversed(range(k))))
+    lay.close()
+
+
+@pytest.mark.parametrize("k", [1, 4, 5, 8, 16])
+@pytest.mark.parametrize("T", [11, 700, 1500])
+def test_shared_and_residual_rows_come_last(gpu_lib, port, k, T):
+    """A block call with a shared expert: x + (routed sum + shared expert's row), bit for bit from the parts."""
+    H = 96
+    sh = synth.tiny(seed=40 + k, E=20, k=k, H=H, F=32, T=T, has_bias=True)
+    h, Wg, rb, ex = cases.layer_inputs(sh, router_scale=30.0)
+    lay = MoeLayer.from_shape(sh)
+    lay.set_router(Wg, rb)
+    lay.load_experts(ex)
+    nw = (1.0 + 0.1 * np.random.default_rng(k).standard_normal(H)).astype(np.float32)
+    lay.set_ffn_norm(nw, 1e-5)
+    _, gw, uw, dw, bg, bu, bd = cases.dense_ffn_case(H=H, F=64, T=1, bias=True, seed=k)
+    shared = MoeLayer(1, 1, H, 64, activation=synth.STANDARD_SWIGLU, has_bias=True, max_tokens=T, weights_f16=True)
+    shared.load_expert_f16(0, uw, gw, dw, bu, bg, bd)
+    n = port.rmsnorm(h, nw, 1e-5)
+    x_d, n_d = torch.from_numpy(h).cuda(), torch.from_numpy(n).cuda()
+    block, moe, dense = (torch.empty((T, H), device="cuda") for _ in range(3))
+    ro, ro2 = (torch.empty((T, k, 2), device="cuda") for _ in range(2))
+    torch.cuda.synchronize()
+    for with_shared in (shared, None):
+        lay.block_forward_dev(x_d, T, ro, block, shared=with_shared)
+        lay.sync()
+        lay.forward_dev(n_d, T, moe, d_router_out=ro2)
+        lay.sync()
+        shared.dense_forward_dev(n_d, T, dense)
+        shared.sync()
+        assert torch.equal(ro, ro2)
+        want = moe + dense if with_shared else moe
+        assert torch.equal(block, x_d + want)
+    shared.close()
+    lay.close()
