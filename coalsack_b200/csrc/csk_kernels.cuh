@@ -1378,7 +1378,8 @@ __global__ void __launch_bounds__(256) k_dense_rows(const float* __restrict__ hi
 // SM a row is dealt to several blocks (gridDim.y), so that a thread has one round of loads (8 tokens of 2880 columns 7.9 -> 4.5 us, profiler).
 // Many tokens need blocks on an SM more than loads of a block: eight of them, with 32 registers a thread (profiler, cold caches; in
 // brackets with the few tokens' form, whose registers leave room for six or four): 8192 tokens, four slots of 512 columns 16.5 us (18.5); 4096, two
-// of 1024 11.2 (12.5); 2048, one of 2048 8.5 (9.7); 2048, eight of 2048 23.9 (25.1).
+// of 1024 11.2 (12.5); 2048, one of 2048 8.5 (9.7); 2048, eight of 2048 23.9 (25.1).  Their barrier stands behind the wait, where the next kernel has been let in already (in front, with the
+// test for page-locked results: 16 experts of 2048 x 2048, top-1, 2048 tokens 92.8 -> 98.5 for the step, 64 of 1024 x 512, top-2, 77.6 -> 80.3).
 // The rows are read for the last time, so they are the first to leave L2 (a step of 2048 tokens of eight slots 244.5 -> 240.6, of 4096
 // of four level; this kernel alone, 4096 tokens, eight slots of 2048 columns 57 -> 47, 8192 tokens, four of 2880 82 -> 76).
 //
@@ -1386,7 +1387,7 @@ __global__ void __launch_bounds__(256) k_dense_rows(const float* __restrict__ hi
 // pass's status word into a sticky one and adds its per-expert row counts to running totals --
 // layout: carry[0] = sticky status, carry[1 .. E] = rows per expert.
 //
-// host_router, host_meta (optional): page-locked memory that the routing and the 16 words of `meta` go to beside the results, which
+// host_router, host_meta (optional, FEW only): page-locked memory that the routing and the 16 words of `meta` go to beside the results, which
 // `out` may be in then, too.
 template <int AT_ONCE, bool FEW>
 __global__ void __launch_bounds__(256, !FEW ? 8 : AT_ONCE > 4 ? 4 : 6) k_combine(const float* __restrict__ router_out, const int* __restrict__ row_of_pair,
@@ -1402,7 +1403,7 @@ __global__ void __launch_bounds__(256, !FEW ? 8 : AT_ONCE > 4 ? 4 : 6) k_combine
     s_row[threadIdx.x] = row_of_pair[(size_t)t * k + threadIdx.x];
     s_w[threadIdx.x] = unweighted ? 1.f : router_out[((size_t)t * k + threadIdx.x) * 2 + 1];  // 1 * v is v
   }
-  __syncthreads();
+  if (FEW) __syncthreads();
   griddep_wait();
   griddep_launch();
   if (carry && t == 0 && blockIdx.y == 0) {
@@ -1410,7 +1411,8 @@ __global__ void __launch_bounds__(256, !FEW ? 8 : AT_ONCE > 4 ? 4 : 6) k_combine
     for (int e = threadIdx.x; e < E; e += blockDim.x) carry[1 + e] += counts[e];
   }
   if (t >= T) return;
-  if (blockIdx.y == 0) {
+  if (!FEW) __syncthreads();
+  if (FEW && blockIdx.y == 0) {
     if (host_router && (int)threadIdx.x < 2 * k) host_router[(size_t)t * k * 2 + threadIdx.x] = router_out[(size_t)t * k * 2 + threadIdx.x];
     if (host_meta && t == 0 && threadIdx.x < 16) host_meta[threadIdx.x] = meta[threadIdx.x];
   }

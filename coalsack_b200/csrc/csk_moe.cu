@@ -711,7 +711,7 @@ void launch_combine(csk_moe_layer* L, const float* router, const float* y, int64
   // As long as its blocks are resident at once (of eight slots a little longer) the form for few tokens is the quicker one.  Few / many, a step, us:
   // four slots of 2880 columns, 600 tokens 60.2 / 62.3, 740 63.9 / 66.1, 820 67.9 / 69.3, 1000 74.4 / 74.2; eight of 2048, 600 60.1 / 61.6, 740 65.4 / 66.1,
   // 900 71.8 / 71.7, 1000 72.9 / 72.4; eight of 512, 740 36.1 / 35.5.
-  const bool few = T <= (L->k > 4 ? 5 : 6) * L->sm_count;
+  const bool few = c.host.meta || T <= (L->k > 4 ? 5 : 6) * L->sm_count;  // (page-locked results are small ones)
   launch_k(!few ? k_combine<4, false> : L->k > 4 ? k_combine<8, true> : k_combine<4, true>, dim3((unsigned)T, row_blocks), dim3(256), 0, s, pdl, router,
            L->d_row_of_pair, y, L->H, out, (int)T, L->k, L->H, (int)L->cfg.weight_before_ffn, (int)c.dense_single, c.meta, c.counts, c.carry,
            L->E, c.residual, c.shared, c.host.router, c.host.meta);

@@ -79,3 +79,22 @@ def test_page_locked_buffers(gpu_lib, T, locked_in, locked_out, mixed):
 @pytest.mark.parametrize("T", [95, 96])  # 384 KB of results and routing are 95 rows
 def test_page_locked_results_at_the_line(gpu_lib, T):
     test_page_locked_buffers(gpu_lib, T, True, True, False)
+
+
+@pytest.mark.parametrize("T", [900, 2000])  # more tokens than six an SM, in results that still fit the staging area
+def test_short_rows_of_many_tokens(gpu_lib, T):
+    sh = synth.tiny(seed=T, E=8, k=2, H=64, F=64, T=T, has_bias=True)
+    h, Wg, rb, ex = cases.layer_inputs(sh)
+    lay = MoeLayer.from_shape(sh)
+    lay.set_router(Wg, rb)
+    lay.load_experts(ex)
+    out, ro = np.full((T, 64), 7, np.float32), np.full((T, 2, 2), 7, np.float32)
+    x, got, got_ro = torch.from_numpy(h).cuda(), torch.empty((T, 64), device="cuda"), torch.empty((T, 2, 2), device="cuda")
+    torch.cuda.synchronize()
+    for _ in range(2):
+        out[:], ro[:] = 7, 7
+        lay.forward(h, out=out, router_out_buf=ro)
+        lay.forward_dev(x, T, got, d_router_out=got_ro)
+        lay.sync()
+        assert np.array_equal(out, got.cpu().numpy()) and np.array_equal(ro, got_ro.cpu().numpy())
+    lay.close()
