@@ -751,7 +751,8 @@ int forward_dev(csk_moe_layer* L, const float* d_hidden, int64_t T, const float*
   const int tile_rows = tile_rows_for(path);
   if (reinterpret_cast<uintptr_t>(d_hidden) % 16) return fail(L, CSK_ERR_INVALID, "hidden states must be 16-byte aligned");
   const bool mx = path == CSK_PATH_STREAM;
-  if (router == L->d_unit_router && router && !mx && only_expert < 0 && !d_router_out && !d_residual && !d_shared && !L->carry_active) {
+  if (router == L->d_unit_router && router && !mx && only_expert < 0 && !d_router_out && !d_residual && !d_shared && !L->carry_active &&
+      !host.meta) {
     // a dense FFN on the tensor-core kernel: the token rows are the grouped rows, and the down projection's the result
     // (8192 tokens, 2880 x 2880: 498 -> 450 us for a scan, a scatter and a combine less)
     launch_k(k_dense_rows, dim3(grid_for((size_t)T * (L->H / 8), 256, 8 * L->sm_count)), dim3(256), 0, s, L->pdl, d_hidden, L->d_x16, L->ldx,
