@@ -685,7 +685,7 @@ inline void launch_router_logits(RouterArgs a, const float* wg_few, const float*
 // weights into registers and runs its warp's TPW tokens against them (token values by
 // broadcast loads: one shared-memory wavefront per four FMAs).  Per (token, expert, part) it
 // leaves c = the part's sum and a = sum over the part's blocks of |prefix inside the part|.
-// k_router_finish: one warp per token adds the parts in order (prefix P_m before part m:
+// k_router_finish: a block per token, a thread per expert adds the parts in order (prefix P_m before part m:
 // sum_j |R_j| <= sum_m (blocks_m |P_m| + a_m)), forms logits and bounds, selects and certifies.
 // ---------------------------------------------------------------------------
 constexpr int kFastSliceBlocks = 3;                     // 32-column blocks per slice
@@ -850,7 +850,7 @@ __global__ void __launch_bounds__(kFinishThreads) k_router_finish(const FinishRo
   const int t = blockIdx.x;
   const int parts = A.parts, E = A.E;
   const int n_slices = (A.H / 32 + kFastSliceBlocks - 1) / kFastSliceBlocks;
-  // blocks of each part (with a division per part in every thread, and that selection, the kernel took 10.1 us, now 5.2)
+  // blocks of each part (a division each: by one thread)
   if (tid < parts) s_blocks[tid] = (float)(kFastSliceBlocks * (n_slices * (tid + 1) / parts - n_slices * tid / parts));
   // (the router's own, older than any kernel of the step)
   float bias = A.bias && tid < E ? __ldg(A.bias + tid) : 0.f, wn = tid < E ? __ldg(A.wnorm + tid) : 0.f;
@@ -954,7 +954,8 @@ inline cudaError_t router_prepare_device() {
   if (e == cudaSuccess) e = router_prepare_set<false>();
   if (e == cudaSuccess)
     e = cudaFuncSetAttribute(k_router_finish_many, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(2 * kFinishWarps * kMaxExperts * sizeof(float)));
-  // (parts x groups of 32 experts fill the SMs once, so parts x experts is bounded; of a larger device too)
+  // (Parts times groups of 32 experts are fewer than the SMs and the groups together, so the parts take at most 256 bytes an SM and 8 KB:
+  // 45 KB on 148 SMs, with the arrays more than the 48 KB that need no leave; this is enough for 350.)
   if (e == cudaSuccess) e = cudaFuncSetAttribute(k_router_finish, cudaFuncAttributeMaxDynamicSharedMemorySize, kFinishMaxSmem);
   if (e == cudaSuccess) e = cudaFuncSetAttribute(k_router_fast<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fast_router_smem(8));
   if (e == cudaSuccess) e = cudaFuncSetAttribute(k_router_fast<16>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fast_router_smem(16));

@@ -323,7 +323,7 @@ int launch_router(csk_moe_layer* L, const float* d_hidden, int64_t T, float* d_r
     // the token blocks alone fill the machine
     int parts = std::min(std::min(fast_router_slices(L->H), kFastMaxParts),
                          std::max(1, (L->sm_count + token_blocks * groups - 1) / (token_blocks * groups)));
-    while (parts > 1 && (T * parts > L->part_rows || finish_smem_bytes(parts, L->E_router) > kFinishMaxSmem)) --parts;
+    while (parts > 1 && T * parts > L->part_rows) --parts;
     const dim3 grid((unsigned)token_blocks, (unsigned)groups, (unsigned)parts);
     const size_t smem = fast_router_smem(tpw);
     switch (tpw) {
