@@ -54,6 +54,64 @@ def test_edges(gpu_lib, port, E, k, H, F, T, bias, act, wbf):
     lay.close()
 
 
+@pytest.mark.parametrize("H", [384, 2080])  # the down projection's last unit has 128 rows, or 32, and no second half
+@pytest.mark.parametrize("rows", [21, 22, 25, 26])  # the last with one atom of row scales and the first with two: down, gate/up
+def test_units_without_a_second_half_beside_ordinary_ones(gpu_lib, port, H, rows):
+    """Every expert has the same rows, so all tiles are alike; more units than CTAs, so that one CTA takes units of either kind."""
+    E, F = 80 if H == 384 else 40, 192
+    sh = synth.tiny(seed=rows, E=E, k=1, H=H, F=F, T=E * rows, has_bias=True)
+    h, Wg, rb, ex = cases.layer_inputs(sh)
+    ro = np.ones((E * rows, 1, 2), np.float32)
+    ro[:, 0, 0] = np.random.default_rng(rows).permutation(np.repeat(np.arange(E), rows))
+    ro[:, 0, 1] = 0.7
+    lay = MoeLayer.from_shape(sh)
+    lay.set_router(Wg, rb)
+    lay.load_experts(ex)
+    lay.set_path(PATH_STREAM)
+    out, _ = lay.forward(h, router_out=ro)
+    want, _ = port.moe_layer(h, Wg, rb, ex, 1, sh.act, router_out=ro, nthreads=16)
+    mx, mr = cases.err_stats(out, want)
+    assert mx <= MX_MAX and mr <= MX_MEAN, (mx, mr)
+    lay.close()
+
+
+@pytest.mark.parametrize("H,T", [(1056, 7), (2080, 7), (2880, 7),  # two and three CTAs a token, tails inside a warp
+                                 (1056, 2800)])                    # rows that are claimed, one CTA a token
+def test_routing_weight_before_the_expert(gpu_lib, H, T):
+    """Rows encoded per pair, wide blocks among them: bit for bit the sum, slot by slot, of the results for rows that were weighted
+    beforehand; of one expert alone, which leaves other slots' rows unplaced, its own."""
+    E, k, F = 6, 3, 64
+    sh = synth.tiny(seed=T + H, E=E, k=k, H=H, F=F, T=T, has_bias=True)
+    h, _, _, ex = cases.layer_inputs(sh)
+    h[T // 2, [5, H // 2, H - 3]] = 1000.0  # wide blocks, one of them the last
+    rng = np.random.default_rng(H)
+    ro = rng.uniform(0.1, 1.0, (T, k, 2)).astype(np.float32)
+    ro[..., 0] = [rng.permutation(E)[:k] for _ in range(T)]
+
+    def layer(k, before):
+        lay = MoeLayer(E, k, H, F, activation=sh.act, has_bias=True, max_tokens=T, weight_before_ffn=before)
+        lay.load_experts(ex)
+        lay.set_path(PATH_STREAM)
+        return lay
+
+    first, plain = layer(k, True), layer(1, False)
+    out, _ = first.forward(h, router_out=ro)
+    want, parts = np.zeros_like(out), []
+    for j in range(k):
+        one = np.ones((T, 1, 2), np.float32)
+        one[:, 0, 0] = ro[:, j, 0]
+        parts.append(plain.forward(h * ro[:, j, 1:], router_out=one)[0])
+        want = want + parts[-1]
+    assert np.array_equal(out, want)
+    if T < 100:
+        e = int(ro[T // 2, 1, 0])
+        alone = first.expert_forward(e, h, ro)
+        for t, j in np.argwhere(ro[..., 0] == e):
+            assert np.array_equal(alone[t], parts[j][t]), t
+    first.close()
+    plain.close()
+
+
 def test_a_captured_step_outlives_larger_images(gpu_lib, port):
     """The digit images grow when the streaming kernel is chosen for any batch; a step that a caller captured before
     that still replays to the same result, on the images it was captured with."""

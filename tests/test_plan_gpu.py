@@ -168,3 +168,59 @@ def test_shared_and_residual_rows_come_last(gpu_lib, port, k, T):
         assert torch.equal(block, x_d + want)
     shared.close()
     lay.close()
+
+
+@pytest.mark.parametrize("T", [1, 9, 200, 256, 257])  # up to 1024 pairs a thread each, then one block's histogram
+@pytest.mark.parametrize("path", [PATH_STREAM, PATH_TILE])
+def test_plan_of_a_shard(gpu_lib, T, path):
+    """A handle that holds experts 8 to 15 of 24: rows of the others, on both sides, are counted and take no tiles.  Tokens whose experts are
+    all here have the whole layer's results bit for bit."""
+    E, k, H, first, held = 24, 4, 64, 8, 8
+    sh = synth.tiny(seed=T, E=E, k=k, H=H, F=32, T=T, has_bias=True)
+    h, Wg, rb, ex = cases.layer_inputs(sh)
+    rng = np.random.default_rng(T)
+    ro = rng.uniform(0.1, 1.0, (T, k, 2)).astype(np.float32)
+    here = np.arange(T) % 2 == 0
+    ro[..., 0] = [first + rng.permutation(held)[:k] if x else rng.permutation(E)[:k] for x in here]
+    h_d, r_d = torch.from_numpy(h).cuda(), torch.from_numpy(ro).cuda()
+    outs, rows = [], []
+    for shard in (False, True):
+        lay = MoeLayer.from_shape(sh, expert_begin=first, expert_count=held) if shard else MoeLayer.from_shape(sh)
+        lay.set_router(Wg, rb)
+        if shard:
+            lay.load_experts({n: w[first:first + held] for n, w in ex.items()}, range(first, first + held))
+        else:
+            lay.load_experts(ex)
+        lay.set_path(path)
+        out = torch.empty((T, H), device="cuda")
+        torch.cuda.synchronize()
+        lay.forward_dev(h_d, T, out, d_router_in=r_d)
+        lay.sync()
+        outs.append(out.cpu().numpy())
+        rows.append(lay.counters()[0])
+        lay.close()
+    assert np.array_equal(outs[1][here], outs[0][here])
+    want = np.bincount(ro[..., 0].astype(int).ravel(), minlength=E)
+    assert np.array_equal(rows[0], want) and np.array_equal(rows[1], want)
+
+
+def test_more_rows_than_the_images_hold(gpu_lib):
+    """An expert node's routing may name its expert in every slot, which makes more rows than a shard of one expert has images
+    for: an error, and the handle goes on."""
+    E, k, H, e = 8, 8, 64, 3
+    sh = synth.tiny(seed=5, E=E, k=k, H=H, F=64, T=64, has_bias=True)
+    h, _, _, ex = cases.layer_inputs(sh)
+    lay = MoeLayer.from_shape(sh, expert_begin=e, expert_count=1)
+    lay.load_experts(ex, [e])
+
+    def routing(T, slots):
+        ro = np.ones((T, k, 2), np.float32)
+        ro[..., 0] = np.where(np.arange(k) < slots, e, 0)
+        return ro
+
+    once = lay.expert_forward(e, h[:10], routing(10, 1))  # 10 rows
+    assert np.array_equal(lay.expert_forward(e, h[:2], routing(2, k)), once[:2])  # 16 rows
+    with pytest.raises(CskError):
+        lay.expert_forward(e, h[:10], routing(10, k))  # 80 rows
+    assert np.array_equal(lay.expert_forward(e, h[:10], routing(10, 1)), once)
+    lay.close()
