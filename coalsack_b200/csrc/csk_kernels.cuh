@@ -628,8 +628,8 @@ inline RouterWave router_wave(int groups, int sm_count) {
 // The fewest tokens per block with which the blocks are one wave: a block's time goes by its chains per thread and, from four warps
 // on, by its shared-memory reads (a row of weights per lane costs 4 cycles per four columns, a token row 2), so that a second
 // wave is dearer than more chains in one.  `wave`: see router_wave.  A launch among others, us, 2880 columns, by the shape taken (warps x tokens
-// of a warp): 128 experts, 8 tokens 1x1 11.1; 50 2x1 13.1; 100 4x1 13.6; 200 4x2 17.6; 333 4x3 21.4; 512 4x4 26.2; 700 8x3 37.9; 1000 8x4 46.1;
-// 32 experts, 333 4x1 13.1; 1024 4x2 17.7; 2048 4x4 28.4; 4096 8x4 47.0; 6000 4x4 71.2 and 8192 4x4 89.7, two blocks an SM (8x4 95).  Other shapes: 100
+// of a warp): 128 experts, 8 tokens 1x1 11.8; 50 2x1 13.9; 100 4x1 14.4; 200 4x2 18.5; 333 4x3 22.3; 512 4x4 27.0; 700 8x3 38.3; 1000 8x4 46.1;
+// 32 experts, 333 4x1 13.9; 1024 4x2 18.5; 2000 4x4 28.1; 4096 8x4 47.2; 6000 4x4 72.0 and 8192 4x4 90.2, two blocks an SM (8x4 95).  Other shapes: 100
 // tokens 2x2 17.8; 592 8x2 38.3; 700 4x6 44.2; 1000 4x8 53.6.
 // wg_few / wg_many: the weights packed for the two chunk widths (PACKED) or both the plain [E,H] matrix.  token_slots: tokens the
 // grid is sized for (a.T, or for a list-driven launch the most entries the list can have).

@@ -170,6 +170,8 @@ constexpr size_t kStagedInMin = 64 << 10, kStagedTwoPieces = 256 << 10;
 // word, so that a call that fails leaves them alone: up to so many bytes that wait, and the copies, are dearer than a host copy.
 // The layer above, direct / staged, us: 1 token (11 KB) 62.6 / 47.0, 8 (90 KB) 114.7 / 101.1, 16 (180 KB) 134.0 / 121.9, 24 (270 KB) 139.0 / 130.9, 32
 // (361 KB) 145.5 / 139.5, 50 (564 KB) 155 / 166, 80 175 / 206; 128 experts of 2048 x 768, 30 tokens (240 KB) 122.4 / 111.0, 100 (800 KB) 159 / 186.
+// A row of 24 handles called in turn, whose staging areas are cold, as a model's layers are: 8 experts of 2880 x 2880, top-4, 16 tokens 97 / 89, 24 100 / 97, 28
+// (324 KB) 101 / 101, 32 102 and 111 / 107 (two runs); 32 of 2048 x 768, top-8, 32 tokens (266 KB) 92 / 89, 42 (350 KB) 101 / 95.5, 47 (392 KB) 104 / 106.
 constexpr size_t kStagedLockedMax = 384 << 10;
 
 int wide_stride(const csk_moe_layer* L) { return mx_mask_words(L->Lgu.recs) + mx_mask_words(L->Ld.recs); }
@@ -254,9 +256,11 @@ int launch_router(csk_moe_layer* L, const float* d_hidden, int64_t T, float* d_r
   // rows: 128 experts, 2880 columns: 64 tokens 13 / (FMA pass) 25, 512 26 / 34, 1024 47 / 35, 2048 95 / 43; 128 x 2048: 600 29 / 32, 1000 36 / 32; 64 x 2880:
   // 1024 26 / 34, 2048 48 / 44, 3000 96 / 49; 256 x 2880: 256 38 / 39, 512 54 / 39; 512 x 2048: 256 45 / (FMA) 95, 512 79 / 44; 128 x 512: 1000 14 /
   // 21; 32 x 2880: 4096 47 / 104, 8192 90 / 146
-  // (a digit matrix has 128 rows whatever the experts).  The line is where the two meet: with half as many pairs the FMA pass, which
-  // the certified mode then takes, is the slower one everywhere; with 512 experts and more (few tokens, many digit matrices) they
-  // meet at twice as many.
+  // (a digit matrix has 128 rows whatever the experts).  The line is a compromise over the columns, by which a chain goes and the certified pass hardly:
+  // at 1024 tokens of 128 experts the chain costs 12 us more of 2880 columns, 4 of 2048, and 7 less of 512, so that the two meet below the line (700
+  // tokens) for wide layers and beyond it for narrow ones; with 256 experts of 2880 columns they meet at half of it.  From 512 experts on (few
+  // tokens, many digit matrices) it is at twice as many pairs, where the chain is 35 us behind (512 x 2048, 512 tokens).  Below the line the certified
+  // mode takes the FMA pass, which is slower than the chain everywhere.
   const int groups = (L->E_router + 31) / 32;
   const int64_t tensor_min_work = groups >= 16 ? 8192 : 4096;  // tokens x groups of 32 experts
   const bool few = T <= kCertifiedMaxTokens, many = groups > 1 && T * groups >= tensor_min_work;
@@ -587,7 +591,7 @@ struct Batch {
 // features of an expert) on the SMs.  The line is half an item per SM, for evenly spread routing (in brackets): 16 of 2048 x 2048, top-1, 1 token
 // (0.11) 36.0 / 25.6, 5 (0.47) 51.3 / 51.3, 16 (1.1) 70.8 / 81.5; top-2, 1 (0.22) 37.0 / 28.3, 4 (0.70) 55.2 / 61.7; top-4, 1 (0.39) 42.0 / 41.6;
 // 2 of 2880 x 2880, 1 (0.16) 40.7 / 26.9, 8 (0.31) 47.6 / 43.3; 4, top-2, 1 (0.27) 45.2 / 44.7; 128 of 2048 x 768, top-8, 1 (0.32) 39.0 / 43.1, 2 (0.61)
-// 53.5 / 58.6; 64 of 512 x 512, top-8, 1 (0.21) 25.8 / 21.0, 4 (0.69) 32.2 / 35.0; beside a shared expert 16 of 2048 x 2048, top-1, 5 tokens 60.4 / 59.2.  And 24 MB of
+// 53.5 / 58.6; 64 of 512 x 512, top-8, 1 (0.21) 25.8 / 21.0, 4 (0.69) 32.2 / 35.0; beside a shared expert 16 of 2048 x 2048, top-1, 5 tokens level (60.4 / 59.2 of a block that takes 55 now).  And 24 MB of
 // weights, where launches and latencies are what is left: 64 of 256 x 512, top-8, 2 (0.37, 11 MB) 22.7 / 20.6, 4 (0.68, 20 MB) 24.2 / 24.7, 8 (1.1, 32 MB)
 // 24.8 / 30.9.
 bool few_rows(const csk_moe_layer* L, const Batch& b) {
